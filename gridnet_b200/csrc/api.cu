@@ -189,6 +189,8 @@ struct OuterWs {
     double2 *partials;  // [Bpad][blocks * 4]
     float2 *stats;      // [Bpad]
     float *packed;      // block 8 only: pair64_packed_floats(M, N, K) floats (weights in the large-batch kernel's order)
+    float *qpacked;     // weights in the quad kernel's order
+    float2 *gbt;        // (gamma, beta) per tile cell of every 8^3 region, for the quad kernel
     int *error_flag;
     size_t bytes;
 };
@@ -201,7 +203,8 @@ static OuterWs carve_outer(void *base, int B, int M, int N, int K, int block)
     const size_t P = (size_t)M * N * K;
     const size_t nb = (size_t)(M / block) * (N / block) * (K / block);
     const bool pair = block == 8 && M % 8 == 0 && N % 8 == 0 && K % 8 == 0;
-    const size_t Bp = pair ? (size_t)round_up64(B) : (size_t)B;
+    const bool regions = M % 8 == 0 && N % 8 == 0 && K % 8 == 0;
+    const size_t Bp = pair ? (size_t)round_up64(B) : (size_t)((B + 3) / 4 * 4);
     size_t off = 0;
     unsigned char *p = (unsigned char *)base;
     for (int i = 0; i < 2; ++i) {
@@ -214,21 +217,24 @@ static OuterWs carve_outer(void *base, int B, int M, int N, int K, int block)
     off = align_up(off + sizeof(float2) * Bp, 256);
     w.packed = (float *)(p + off);
     if (pair) off = align_up(off + sizeof(float) * pair64_packed_floats(M, N, K), 256);
+    w.qpacked = (float *)(p + off);
+    if (regions) off = align_up(off + sizeof(float) * quad_packed_floats(M, N, K), 256);
+    w.gbt = (float2 *)(p + off);
+    if (regions) off = align_up(off + sizeof(float2) * (size_t)(M / 8) * (N / 8) * (K / 8) * quad_tile_cells(block), 256);
     w.error_flag = (int *)(p + off);
     off = align_up(off + sizeof(int), 256);
     w.bytes = off;
     return w;
 }
 
-// 0 = choose automatically (the one persistent kernel of outer_small.cu for problems so small that launches are
-// what they cost; the large-batch kernel of step_pair64.cu when the batch fills its groups of 64 samples well; else
-// the register-patch kernel of step_fast.cu, one launch per outer step), 1 = always the register-patch kernel,
-// 2 = always the large-batch kernel, 3 = always the persistent kernel
+// 0 = choose automatically: the one persistent kernel of outer_small.cu for problems so small that launches are what
+// they cost; else the quad kernel of step_quad.cu from two samples up (64^3, 4 x 12 iterations, ms per loop,
+// register-patch / large-batch / quad, the latter two with the parameters re-ordered before: batch 1 0.265 / - / 0.257,
+// 4 0.445 / - / 0.261, 16 0.97 / - / 0.60, 64 2.92 / 1.87 / 1.76; 128^3, 2 x 16, batch 32: 9.85 / - / 6.06; 64^3 block 4,
+// 8 x 4, batch 128: 3.50 / - / 1.80; for one sample the re-ordering, 0.03 ms, costs more than the kernel gains); else the register-patch kernel of step_fast.cu. 1 = always the register-patch kernel, 2 = always the
+// large-batch kernel of step_pair64.cu, 3 = always the persistent kernel, 4 = always the quad kernel.
 static int g_outer_kernel = 0;
-
-// The large-batch kernel computes whole groups of 64 samples: worth it when at most a quarter of the
-// last group is padding.
-static bool pair64_fills_groups(int B) { return round_up64(B) * 3 <= B * 4; }
+constexpr int kQuadMinBatch = 2;
 
 static int check_ws(const void *ws, size_t have, size_t need)
 {
@@ -277,7 +283,7 @@ GN_API int gn_config_set(const char *key, int value)
 {
     if (!key) return GN_ERR_NULL_POINTER;
     if (!strcmp(key, "outer_kernel")) {
-        if (value < 0 || value > 3) return GN_ERR_UNSUPPORTED;
+        if (value < 0 || value > 4) return GN_ERR_UNSUPPORTED;
         g_outer_kernel = value;
         return GN_OK;
     }
@@ -924,9 +930,9 @@ GN_API int gn_outer_forward_plan(int B, int M, int N, int K, int inner, int oute
     if ((g_outer_kernel == 0 || g_outer_kernel == 3) && outer_small_spc(B, M, N, K, block, inner, outer, a, a, a, a, a, a, a) > 0)
         return 3;
     if (g_outer_kernel == 3) return 0;
-    if (pair64_applicable(M, N, K, block, inner) && (g_outer_kernel == 2 || (g_outer_kernel == 0 && pair64_fills_groups(B))))
-        return 2;
-    if (g_outer_kernel == 2) return 0;
+    if (((g_outer_kernel == 0 && B >= kQuadMinBatch) || g_outer_kernel == 4) && quad_applicable(M, N, K, block, inner)) return 5;
+    if (g_outer_kernel == 4) return 0;
+    if (g_outer_kernel == 2) return pair64_applicable(M, N, K, block, inner) ? 2 : 0;
     FastFwdParams p{};
     p.w = p.b = p.s = p.x = reinterpret_cast<const float *>(a);
     p.B = B; p.M = M; p.N = N; p.K = K; p.inner = inner; p.sub = block;
@@ -1008,8 +1014,41 @@ static int outer_forward_impl(const float *w, const float *b, const float *s, co
         }
         if (g_outer_kernel == 3) return GN_ERR_UNSUPPORTED;
     }
+    const bool quad_ok = quad_applicable(M, N, K, block, inner);
+    if (quad_ok && ((g_outer_kernel == 0 && B >= kQuadMinBatch) || g_outer_kernel == 4)) {
+        const int Q = (B + 3) / 4, regions = (M / 8) * (N / 8) * (K / 8);
+        if (cudaMemsetAsync(ws.error_flag, 0, sizeof(int), st) != cudaSuccess) {
+            record_cuda_error(cudaGetLastError(), "cudaMemsetAsync");
+            return GN_ERR_CUDA;
+        }
+        if (!(flags & GN_OUTER_PARAMS_UNCHANGED)) {
+            rc = launch_quad_pack(w, b, s, ws.qpacked, M, N, K, block, false, st);
+            if (rc != GN_OK) return rc;
+            rc = launch_quad_table(gamma, beta, ws.gbt, M, N, K, block, st);
+            if (rc != GN_OK) return rc;
+        }
+        rc = launch_to_il4(x, ws.buf[0], B, P, st);
+        if (rc != GN_OK) return rc;
+        for (int o = 0; o < outer; ++o) {
+            QuadStep a{};
+            a.packed = ws.qpacked; a.gbt = ws.gbt;
+            a.in_il4 = ws.buf[o & 1];
+            a.out_il4 = ws.buf[(o + 1) & 1];
+            a.in_stats = o > 0 ? ws.stats : nullptr;
+            a.out_partials = ws.partials;
+            a.nparts = regions;
+            a.error_flag = ws.error_flag;
+            a.M = M; a.N = N; a.K = K; a.Q = Q; a.inner = inner; a.block = block;
+            rc = launch_step_fwd_quad(a, act, st);
+            if (rc != GN_OK) return rc;
+            rc = launch_norm_finalize(ws.partials, regions, ws.stats, 4 * Q, P, ln_eps, st);
+            if (rc != GN_OK) return rc;
+        }
+        return launch_from_il4(ws.buf[outer & 1], ws.stats, gamma, beta, y, B, P, st);
+    }
+    if (g_outer_kernel == 4) return GN_ERR_UNSUPPORTED;
     const bool pair_ok = pair64_applicable(M, N, K, block, inner);
-    if (pair_ok && (g_outer_kernel == 2 || (g_outer_kernel == 0 && pair64_fills_groups(B)))) {
+    if (pair_ok && g_outer_kernel == 2) {
         const int Bp = round_up64(B), G = Bp / 64;
         const int nblocks = (M / 8) * (N / 8) * (K / 8);
         cudaError_t e = cudaMemsetAsync(ws.error_flag, 0, sizeof(int), st);

@@ -133,6 +133,31 @@ int launch_to_il64(const float *x, float *il, int B, int G, long long P, cudaStr
 int launch_from_il64(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, int G,
                      long long P, cudaStream_t st);
 
+// ---- step_quad.cu (weights in tensor memory, four samples per lane; activations in the IL4 layout [quad][z][y][x][4
+// samples], blocks of 8 and 4; B need not be a multiple of 4, the missing samples are zeros)
+struct QuadStep {
+    const float *packed;      // from launch_quad_pack
+    const float2 *gbt;        // from launch_quad_table; used when in_stats is set
+    const float *in_il4;
+    float *out_il4;           // or nullptr
+    const float2 *in_stats;   // [4 Q] or nullptr
+    double2 *out_partials;    // [4 Q][nparts] or nullptr; slots 0 .. regions-1 of every row are written
+    int nparts;
+    float *save_h, *save_x;   // replay (IL4 tensors, [inner] and [inner - 1] of them) or nullptr
+    int *error_flag;
+    int M, N, K, Q, inner, block;
+};
+bool quad_applicable(int M, int N, int K, int block, int inner);
+size_t quad_packed_floats(int M, int N, int K);
+int launch_quad_pack(const float *w, const float *b, const float *s, float *packed, int M, int N, int K, int block, bool transposed,
+                     cudaStream_t st);
+int quad_tile_cells(int block);  // float2 entries per region of the (gamma, beta) table
+int launch_quad_table(const float *gamma, const float *beta, float2 *gbt, int M, int N, int K, int block, cudaStream_t st);
+int launch_to_il4(const float *x, float *il, int B, long long P, cudaStream_t st);
+int launch_from_il4(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, long long P,
+                    cudaStream_t st);
+int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st);
+
 // ---- status.cu: device address of the per-device status word that kernels set when a bounded wait gives up
 // and the caller passed no flag of its own (nullptr if it cannot be resolved)
 int *device_status_ptr();

@@ -50,14 +50,17 @@ __global__ void __launch_bounds__(256) norm_partial_stats_k(const float *__restr
     if (threadIdx.x == 0) partials[(size_t)b * parts + part] = make_double2(s, q);
 }
 
-// grid B; adds nparts partials in a fixed order
-__global__ void __launch_bounds__(256) norm_finalize_k(const double2 *__restrict__ partials, int nparts,
+// grid B; adds nparts partials in a fixed order. One CTA reads a whole row, so what bounds a long row is how many of
+// its loads are in flight: 1024 threads with four each (256 threads with one each took 241 us for 32 rows of 32768 to
+// 131072 partials)
+__global__ void __launch_bounds__(1024) norm_finalize_k(const double2 *__restrict__ partials, int nparts,
                                                        float2 *__restrict__ stats, long long P, float eps)
 {
     __shared__ double red[33];
     const int b = blockIdx.x;
     const double2 *ps = partials + (size_t)b * nparts;
     double s = 0.0, q = 0.0;
+#pragma unroll 4
     for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
         const double2 v = ps[i];
         s += v.x;
@@ -265,7 +268,7 @@ int launch_norm_partial_stats(const float *x, double2 *partials, int B, long lon
 int launch_norm_finalize(const double2 *partials, int nparts, float2 *stats, int B, long long P, float eps,
                          cudaStream_t st)
 {
-    norm_finalize_k<<<B, 256, 0, st>>>(partials, nparts, stats, P, eps);
+    norm_finalize_k<<<B, nparts >= 2048 ? 1024 : 256, 0, st>>>(partials, nparts, stats, P, eps);
     return check_launch("norm_finalize");
 }
 

@@ -1,0 +1,232 @@
+// Geometry and building blocks shared by the quad kernels (step_quad.cu): how the 32 lanes of a warp split an 8^3
+// region of the grid, where a lane's window lies in the tile, the order of the weights in tensor memory, and the
+// 27-tap sum itself.
+#pragma once
+#include "packed.cuh"
+#include "tmem.cuh"
+
+namespace gn {
+
+namespace quad {
+constexpr int QUARTERS = 4;
+constexpr unsigned kSpinLimit = 1u << 20;
+// columns of tensor memory: 36 uses of 12 weights, then 16 biases, 16 scales
+constexpr int COL_BIAS = 432, COL_SCALE = 448;
+}  // namespace quad
+
+// A region's tile buffer, in cells of 16 bytes (four samples).
+template <int SUB>
+struct QuadGeo;
+
+// TEAM: warps per quarter of tensor memory; NBUF: tile buffers per team. Block 8: the region is one block, its tile
+// 10 x 10 x 10 cells.
+template <>
+struct QuadGeo<8> {
+    static constexpr int SIDE = 10, ROW = 10, PLANE = 100, CELLS = 1000, BUF_BYTES = 16000, TEAM = 2, NBUF = 3;
+    __device__ static void cell(int c, int &cz, int &cy, int &cx)
+    {
+        cx = c % 10, cy = (c / 10) % 10, cz = c / 100;
+    }
+};
+
+// Block 4: eight blocks, each with its own 6^3 tile (no room for a third buffer)
+template <>
+struct QuadGeo<4> {
+    static constexpr int SIDE = 6, ROW = 6, PLANE = 36, SUBCELLS = 216, CELLS = 8 * SUBCELLS, BUF_BYTES = CELLS * 16, TEAM = 2, NBUF = 2;
+    __device__ static void cell(int c, int &cz, int &cy, int &cx)
+    {
+        const int sub = c / SUBCELLS, l = c % SUBCELLS;
+        cx = (sub & 1) * 4 + l % 6, cy = ((sub >> 1) & 1) * 4 + (l / 6) % 6, cz = (sub >> 2) * 4 + l / 36;
+    }
+};
+
+// What a lane owns: the 2 x 2 x 4 patch at z = z0 + dz, y = y0 + ysgn * dy, x = 4 h + (h ? 3 - o : o) of the region,
+// and the tile cell of its window's corner, from which the window extends by + PLANE per z, ysgn * ROW per y and
+// xsgn per x. The upper x half and the upper y half walk inwards from the far end: with dense rows of 10 (or 6)
+// cells the 8 lanes of a quarter-warp then hit 8 different 16-byte banks in every load and store of a cell.
+template <int SUB>
+struct QuadLane {
+    int h, z0, y0, ysgn, xsgn, cell0;
+    __device__ __forceinline__ explicit QuadLane(int lane)
+    {
+        using G = QuadGeo<SUB>;
+        h = lane & 1;
+        const int yp = (lane >> 1) & 3, zp = lane >> 3, my = yp >> 1, e = yp & 1;
+        z0 = 2 * zp;
+        xsgn = h ? -1 : 1;
+        y0 = my ? 7 - 2 * e : 2 * e;
+        ysgn = my ? -1 : 1;
+        const int row = my ? G::SIDE - 1 - 2 * e : 2 * e, col = h ? G::SIDE - 1 : 0;
+        if (SUB == 8) cell0 = 2 * zp * G::PLANE + row * G::ROW + col;
+        else cell0 = (((zp >> 1) * 2 + my) * 2 + h) * 216 + 2 * (zp & 1) * G::PLANE + row * G::ROW + col;
+    }
+};
+
+__device__ __forceinline__ float4 lds128(unsigned a)
+{
+    float4 v;
+    asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a));
+    return v;
+}
+__device__ __forceinline__ void sts128(unsigned a, float4 v)
+{
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(a), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w) : "memory");
+}
+__device__ __forceinline__ void sts128u(unsigned a, u64 lo, u64 hi)
+{
+    asm volatile("st.shared.v2.u64 [%0], {%1, %2};" ::"r"(a), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ void lds128u(unsigned a, u64 &lo, u64 &hi)
+{
+    asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];" : "=l"(lo), "=l"(hi) : "r"(a));
+}
+__device__ __forceinline__ void stg128(float *p, u64 lo, u64 hi)
+{
+    asm volatile("st.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(lo), "l"(hi) : "memory");
+}
+__device__ __forceinline__ void st_release_shared(unsigned a, int v)
+{
+    asm volatile("st.release.cta.shared::cta.s32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ int ld_acquire_shared(unsigned a)
+{
+    int v;
+    asm volatile("ld.acquire.cta.shared::cta.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+// 16 bytes to shared memory, asynchronously
+__device__ __forceinline__ void cp_async16(unsigned dst, const void *src)
+{
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// the warps of a team
+template <int TEAM>
+__device__ __forceinline__ void team_sync(int quarter)
+{
+    asm volatile("bar.sync %0, %1;" ::"r"(quarter + 1), "n"(32 * TEAM) : "memory");
+}
+
+// Parameters of a region, packed in the order quad_stencil uses them (quad_pack_k): 116 vectors of four words per
+// lane, lane-contiguous (512 bytes per vector and warp).
+namespace quad {
+constexpr int VECS = 116, PACK_F = VECS * 128;  // floats per region
+}
+template <int N>
+__device__ __forceinline__ void quad_move(const float4 *src, unsigned col)
+{
+    float r[4 * N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const float4 v = __ldg(src + k * 32);
+        r[4 * k + 0] = v.x, r[4 * k + 1] = v.y, r[4 * k + 2] = v.z, r[4 * k + 3] = v.w;
+    }
+    int k = 0;
+#pragma unroll
+    for (; k + 4 <= N; k += 4) tmem_st16(col + 4 * k, r + 4 * k);
+    if (N & 2) {
+        tmem_st8(col + 4 * k, r + 4 * k);
+        k += 2;
+    }
+    if (N & 1) tmem_st4(col + 4 * k, r + 4 * k);
+}
+// -> tensor memory. Each warp of a team moves half of the vectors, 29 loads in flight per lane.
+__device__ __forceinline__ void quad_load_params(const float *packed, int role, int lane, unsigned tm)
+{
+    const float4 *src = reinterpret_cast<const float4 *>(packed) + role * 58 * 32 + lane;
+    quad_move<29>(src, tm + role * 232);
+    quad_move<29>(src + 29 * 32, tm + role * 232 + 116);
+}
+
+// The 27-tap sums of the lane's 16 neurons for four samples, acc[n = (dz, dy)][o][sample pair] += sum.
+//   FWD: acc starts at the bias, and done(n, o, scale, centre) is called when a sum is complete - for the neurons of
+//   dy = 0 between the FMAs of the last window rows, so that their activation functions (MUFU) run under them.
+//   Otherwise acc is added to, and done is not called.
+template <int SUB, bool FWD, typename Done>
+__device__ __forceinline__ void quad_stencil(unsigned win, unsigned tm, const QuadLane<SUB> &L, u64 (&acc)[4][4][2], Done done)
+{
+    using G = QuadGeo<SUB>;
+    const int dx = L.xsgn * 16, dy_ = L.ysgn * G::ROW * 16;
+    float wb[2][12], sc[2][4];
+    auto finish = [&](int n, int o, float s) {
+        u64 c0, c1;
+        lds128u(win + (unsigned)((1 + (n & 1)) * dy_ + (1 + o) * dx) + (1 + (n >> 1)) * G::PLANE * 16u, c0, c1);
+        done(n, o, s, c0, c1);
+    };
+    if (FWD) {
+        float bias[16];
+        tmem_ld16(tm + quad::COL_BIAS, bias);
+        tmem_wait_ld16(bias);
+#pragma unroll
+        for (int n = 0; n < 4; ++n)
+#pragma unroll
+            for (int o = 0; o < 4; ++o) acc[n][o][0] = acc[n][o][1] = pack2(bias[n * 4 + o], bias[n * 4 + o]);
+    }
+    tmem_ld8(tm, wb[0]);
+    tmem_ld4(tm + 8, wb[0] + 8);
+    int use = 0, fin = 0;
+#pragma unroll
+    for (int ry = 0; ry < 4; ++ry) {
+        unsigned a6[6];
+#pragma unroll
+        for (int j = 0; j < 6; ++j) a6[j] = win + (unsigned)(ry * dy_ + j * dx);
+#pragma unroll
+        for (int rz = 0; rz < 4; ++rz) {
+            u64 v[6][2];
+#pragma unroll
+            for (int j = 0; j < 6; ++j) lds128u(a6[j] + rz * G::PLANE * 16u, v[j][0], v[j][1]);
+#pragma unroll
+            for (int n = 0; n < 4; ++n) {
+                const int a = rz - (n >> 1), b = ry - (n & 1);
+                if (a < 0 || a > 2 || b < 0 || b > 2) continue;
+                float *wp = wb[use & 1];
+                tmem_wait_ld12(wp);
+                if (FWD && use == 30) tmem_use8(sc[0]);  // asked for before: that wait covered it
+                if (use + 1 < 36) {
+                    tmem_ld8(tm + (use + 1) * 12, wb[(use & 1) ^ 1]);
+                    tmem_ld4(tm + (use + 1) * 12 + 8, wb[(use & 1) ^ 1] + 8);
+                }
+                if (FWD && use == 29) {
+                    tmem_ld4(tm + quad::COL_SCALE, sc[0]);
+                    tmem_ld4(tm + quad::COL_SCALE + 8, sc[1]);
+                }
+#pragma unroll
+                for (int c = 0; c < 3; ++c)
+#pragma unroll
+                    for (int o = 0; o < 4; ++o) {
+                        const u64 ww = pack2(wp[c * 4 + o], wp[c * 4 + o]);
+                        ffma2(acc[n][o][0], v[o + c][0], ww);
+                        ffma2(acc[n][o][1], v[o + c][1], ww);
+                    }
+                ++use;
+                if (FWD && ry == 3)
+#pragma unroll
+                    for (int e = (use - 30) * 8 / 6; fin < e; ++fin) finish((fin >> 2) * 2, fin & 3, sc[fin >> 2][fin & 3]);
+            }
+        }
+    }
+    if (FWD) {
+        tmem_ld4(tm + quad::COL_SCALE + 4, sc[0]);
+        tmem_ld4(tm + quad::COL_SCALE + 12, sc[1]);
+        tmem_wait_ld8(sc[0]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) finish((e >> 2) * 2 + 1, e & 3, sc[e >> 2][e & 3]);
+    }
+}
+
+// Adds eight values over the warp; afterwards lanes 4 j .. 4 j + 3 all hold the sum of value j.
+__device__ __forceinline__ float quad_reduce8(const float (&v)[8], int lane)
+{
+    float a[4], b[2], c;
+    const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) a[k] = (h16 ? v[k + 4] : v[k]) + __shfl_xor_sync(0xffffffffu, h16 ? v[k] : v[k + 4], 16);
+#pragma unroll
+    for (int k = 0; k < 2; ++k) b[k] = (h8 ? a[k + 2] : a[k]) + __shfl_xor_sync(0xffffffffu, h8 ? a[k] : a[k + 2], 8);
+    c = (h4 ? b[1] : b[0]) + __shfl_xor_sync(0xffffffffu, h4 ? b[0] : b[1], 4);
+    c += __shfl_xor_sync(0xffffffffu, c, 2);
+    c += __shfl_xor_sync(0xffffffffu, c, 1);
+    return c;
+}
+
+}  // namespace gn

@@ -43,6 +43,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "packed.cuh"
 #include "tma.cuh"
 
 namespace gn {
@@ -91,67 +92,10 @@ struct Pair64Params {
     int nblocks, nitems;
 };
 
-typedef unsigned long long u64;
 struct Quad {
     u64 lo, hi;  // samples (0,1) and (2,3) of the lane
 };
 
-__device__ __forceinline__ u64 pack2(float a, float b)
-{
-    u64 r;
-    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-    return r;
-}
-__device__ __forceinline__ void unpack2(u64 v, float &a, float &b)
-{
-    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ void ffma2(u64 &acc, u64 a, u64 w)
-{
-    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(w));
-}
-__device__ __forceinline__ u64 fmul2(u64 a, u64 b)
-{
-    u64 r;
-    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 fadd2(u64 a, u64 b)
-{
-    u64 r;
-    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-    return r;
-}
-__device__ __forceinline__ u64 ffma2r(u64 a, u64 b, u64 c)
-{
-    u64 r;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
-    return r;
-}
-// cen + sc * act(h) for a pair of samples. silu is done on the pair: the multiplies and adds are packed, only the
-// two MUFU operations per value are scalar. 2^t overflows to +inf for very negative h; the reciprocal is then 0
-// and h * 0 = -0, the right limit, so no clamp is needed.
-template <int ACT>
-__device__ __forceinline__ u64 act_residual2(u64 h, float sc, u64 cen)
-{
-    const u64 sc2 = pack2(sc, sc);
-    if (ACT == GN_ACT_SILU) {
-        const u64 t = fmul2(h, pack2(-1.4426950408889634f, -1.4426950408889634f));
-        float t0, t1, e0, e1, r0, r1;
-        unpack2(t, t0, t1);
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(t0));
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(t1));
-        const u64 d = fadd2(pack2(e0, e1), pack2(1.0f, 1.0f));
-        float d0, d1;
-        unpack2(d, d0, d1);
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d0));
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d1));
-        return ffma2r(fmul2(h, pack2(r0, r1)), sc2, cen);
-    }
-    float h0, h1;
-    unpack2(h, h0, h1);
-    return ffma2r(pack2(Act<ACT, float>::fwd(h0), Act<ACT, float>::fwd(h1)), sc2, cen);
-}
 __device__ __forceinline__ Quad lds_quad(const float *p)
 {
     const ulonglong2 t = *reinterpret_cast<const ulonglong2 *>(p);

@@ -70,10 +70,9 @@ GN_API int gn_version(void);
 /* Process-wide tuning switches (not needed for normal use). Keys:
  *   "outer_kernel": which kernel gn_outer_forward_f32 uses: 0 = automatic (default: the whole
  *                   loop as one persistent kernel when the problem is so small that launches are
- *                   what it costs; the large-batch kernel when at most a quarter of the last group
- *                   of 64 samples would be padding; else the register-patch kernel), 1 = the
- *                   register-patch kernel, 2 = the large-batch kernel, 3 = the persistent kernel
- *                   (GN_ERR_UNSUPPORTED from gn_outer_forward_f32 when the forced one does not apply).
+ *                   what it costs; else the quad kernel; the register-patch kernel where neither
+ *                   applies), 1 = the register-patch kernel, 2 = the large-batch kernel, 3 = the
+ *                   persistent kernel, 4 = the quad kernel (GN_ERR_UNSUPPORTED from gn_outer_forward_f32 when the forced one does not apply).
  *   "forward_samples_per_cta": samples one CTA of the tuned float forward kernel walks through;
  *                   0 = chosen from the grid and batch size (default). */
 GN_API int gn_config_set(const char *key, int value);
@@ -432,14 +431,15 @@ GN_API int gn_norm_apply_f32(const float *x, const float *gamma, const float *be
  * per-sample statistics of what it writes, and the next step applies
  * (x - mean) * rstd * gamma + beta while it loads its tiles; only the last
  * step's output is normalised by a separate kernel into y.
- * workspace: two [B rounded up to 64, M,N,K] float buffers, the statistics partials and, for
- * block 8, the weights re-ordered for the large-batch kernel (29/27 of the weight tensor).
- * With the large-batch kernel (see gn_step_forward_pair64_f32 below) the activations stay
- * interleaved by groups of 64 samples between steps, [group][M][N][K][64], and are read by TMA. */
+ * workspace: two [B rounded up to 64 (block 4: 4), M,N,K] float buffers, the statistics partials, the weights
+ * re-ordered for the quad kernel (29/27 of the weight tensor) and for the large-batch kernel (block 8), and a
+ * (gamma, beta) table.
+ * With the quad kernel the activations stay interleaved by four samples between steps, [quad][M][N][K][4]; with the
+ * large-batch kernel (see gn_step_forward_pair64_f32 below) by groups of 64, [group][M][N][K][64]. */
 /* Which kernel gn_outer_forward_f32 would take for this problem with suitably aligned buffers: 3 = the whole loop
- * as one persistent kernel (1 launch), 2 = the large-batch kernel (2 launches per outer step + 3), 1 = the
- * register-patch kernel (2 per outer step + 1), 4 = the step-by-step composition of the generic kernels,
- * 0 = bad arguments or the kernel forced with gn_config_set does not apply. */
+ * as one persistent kernel (1 launch), 5 = the quad kernel (2 launches per outer step + 4), 2 = the large-batch
+ * kernel (2 per outer step + 3), 1 = the register-patch kernel (2 per outer step + 1), 4 = the step-by-step
+ * composition of the generic kernels, 0 = bad arguments or the kernel forced with gn_config_set does not apply. */
 GN_API int gn_outer_forward_plan(int B, int M, int N, int K, int inner, int outer, int block);
 GN_API size_t gn_outer_forward_workspace_bytes(int B, int M, int N, int K, int block);
 /* Byte offset, inside the workspace, of an int that gn_outer_forward_f32 sets to 1 when a bounded
@@ -453,7 +453,7 @@ GN_API int gn_outer_forward_f32(const float *weight, const float *bias, const fl
                          size_t workspace_bytes, void *stream);
 /* gn_outer_forward_f32 with flags. GN_OUTER_PARAMS_UNCHANGED: the previous call with this workspace had the same
  * weight, bias, scale, gamma and beta (same values, same shape) and nothing else has written to the workspace
- * since, so the re-ordered copy of the parameters that the large-batch kernel keeps there is still good and is
+ * since, so the re-ordered copy of the parameters that the quad and large-batch kernels keep there is still good and is
  * not rebuilt (an inference server calls the loop many times between weight updates). */
 #define GN_OUTER_PARAMS_UNCHANGED 1
 GN_API int gn_outer_forward_flags_f32(const float *weight, const float *bias, const float *scale,

@@ -224,6 +224,40 @@ def test_persistent_kernel_matches_step_by_step_loop_and_oracle(B, shape, inner,
     assert_close(got.cpu().numpy(), orc.outer_forward(*a64, inner, outer, 8, activation=act), None, f"persistent kernel B={B}")
 
 
+@pytest.mark.parametrize("B,shape,block,inner,outer,act", [
+    (1, (8, 8, 8), 8, 1, 1, "relu"),        # one region, one sample of a quad
+    (5, (8, 16, 24), 8, 3, 2, "tanh"),      # a ragged second quad, non-cubic grid
+    (9, (24, 8, 16), 4, 2, 3, "silu"),      # block 4: eight tiles per region; an odd number of quads
+    (44, (32, 24, 16), 8, 2, 2, "leaky_relu"),  # more items than workers: regions shared between them
+])
+def test_quad_kernel_matches_patch_kernel_and_oracle(B, shape, block, inner, outer, act):
+    """The quad step kernel (weights in tensor memory, four samples per lane) against the register-patch kernel and
+    the oracle; two runs give the same bits."""
+    from gridnet_b200 import outer_forward, outer_forward_failed, outer_forward_workspace
+    from gridnet_b200._lib import lib
+
+    w, b, s, gamma, beta = model_params(91, shape)
+    x = face_input(92, B, shape)
+    x[:, ::3, 1::2, 1:] = 0.3 * np.random.default_rng(93).standard_normal(x[:, ::3, 1::2, 1:].shape)
+    args = [dev(a) for a in (w, b, s, gamma, beta, x)]
+    ws = outer_forward_workspace(B, shape, block, args[0].device)
+    try:
+        assert lib.gn_config_set(b"outer_kernel", 1) == 0
+        base = outer_forward(*args, inner, outer, block, act)
+        assert lib.gn_config_set(b"outer_kernel", 4) == 0
+        got = outer_forward(*args, inner, outer, block, act, workspace=ws)
+        again = outer_forward(*args, inner, outer, block, act, workspace=ws)
+    finally:
+        lib.gn_config_set(b"outer_kernel", 0)
+    assert not outer_forward_failed(ws, B, shape, block)
+    assert torch.equal(got, again), "two runs differ"
+    assert torch.allclose(got, base, rtol=2e-5, atol=5e-6), (got - base).abs().max().item()
+    a64 = [a.astype(np.float64) for a in (w, b, s, gamma, beta, x)]
+    a32 = [a.astype(np.float32) for a in (w, b, s, gamma, beta, x)]
+    assert_close(got.cpu().numpy(), orc.outer_forward(*a64, inner, outer, block, activation=act),
+                 orc.outer_forward(*a32, inner, outer, block, activation=act), f"quad kernel B={B}")
+
+
 def test_packed_parameters_are_rebuilt_when_parameters_change():
     """A reused workspace keeps the re-ordered parameters of the large-batch kernel; changing a parameter in place,
     passing another parameter tensor, or scribbling over the workspace must all lead to a rebuild."""
