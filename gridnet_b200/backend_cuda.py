@@ -14,6 +14,8 @@ models run between steps (gridnet/scripts/train_mnist.py:54,62-64):
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import gridnet_cuda
@@ -67,24 +69,6 @@ def _stash_wanted(weight, init_activations, inner_iters: int, block_size: int) -
     # what torch's caching allocator holds but has not handed out counts as free too
     free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
     return need * 10 <= free
-
-
-def _stash_steps(weight, x, inner_iters: int, block_size: int, steps: int) -> int:
-    """How many of the ``steps`` outer steps of a fused training loop keep their inner iterations: all or none when
-    :func:`keep_forward_stash` forces it; otherwise as many as fit into 70 % of the device memory that is free when
-    the loop starts (a step costs its stash plus the raw output that is saved anyway). Asked once per loop: the
-    driver's memory query is not free, and a loop should not change its mind half-way for a few megabytes."""
-    if _keep_forward_stash is not None:
-        return steps if _keep_forward_stash else 0
-    B, M, N, K = x.shape
-    need = int(lib.gn_step_stash_bytes(B, M, N, K, int(inner_iters), int(block_size)))
-    if need <= 0 or steps <= 0:
-        return 0
-    dev = weight.device
-    free, _ = torch.cuda.mem_get_info(dev)
-    free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
-    per_step = need + x.numel() * 4
-    return max(0, min(steps, int(0.7 * free) // per_step))
 
 
 class GridnetCudaOp(torch.autograd.Function):
@@ -208,6 +192,138 @@ class GridNormOp(torch.autograd.Function):
         return gx, gg, gb, None
 
 
+_STAGGER = 4352  # bytes: 17 x 256, keeps 256-byte alignment
+_BIG = 1 << 30
+
+
+def _staggered(nbytes: int, device, k: int) -> torch.Tensor:
+    """``nbytes`` of device memory; from a GiB up starting ``(k % 7 + 1) * 4352`` bytes into its allocation. The tensors a
+    training step streams side by side (input, output, kept iterations) are each an exact power of two in size at the
+    benchmark's shapes, so fresh allocations start at the same offset inside every 2 MB page; depending on where
+    the driver put the pages, the forward pass of C3 then took anything from 79 to 105 ms. Different offsets make
+    the streams fall on different memory channels whatever the placement."""
+    if nbytes < _BIG:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
+    off = (k % 7 + 1) * _STAGGER
+    return torch.empty(nbytes + 8 * _STAGGER, dtype=torch.uint8, device=device)[off:off + nbytes]
+
+
+def _pointers(tensors):
+    return (ctypes.c_void_p * len(tensors))(*[None if t is None else t.data_ptr() for t in tensors])
+
+
+def _kept_steps(nbytes_out: int, nbytes_stash: int, outer: int, device) -> int:
+    """How many of the ``outer`` steps of a differentiated loop keep their inner iterations (the LAST ones: their
+    backward comes first): all or none when :func:`keep_forward_stash` forces it; otherwise as many as fit into 70 % of the
+    device memory that is free when the loop starts. A loop that needs less than a GiB in all does not ask (the driver's
+    answer takes longer than a small model's forward pass)."""
+    if _keep_forward_stash is not None:
+        return outer if _keep_forward_stash else 0
+    per_step = nbytes_out + nbytes_stash
+    if per_step * outer < _BIG:
+        return outer
+    free, _ = torch.cuda.mem_get_info(device)
+    # what torch's caching allocator holds but has not handed out counts as free too
+    free += torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+    return max(0, min(outer, int(0.7 * free) // per_step))
+
+
+def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, block: int, activation: str, ln_eps: float,
+                  residual: bool, need_grad: bool):
+    """The loop forward through ``gn_loop_forward_f32``; ``plist``: one (weight, bias, residual_scale) for all steps, or one
+    per step. Returns the output and the tensors the backward pass needs: (x_il4, stats, outs, stashes)."""
+    B, M, N, K = x.shape
+    for params in plist:
+        _assert_step_args(*params, x, block, False)
+        assert norm_weight.shape == params[1].shape == norm_bias.shape, f"{norm_weight.shape=} invalid for {params[1].shape=}"
+        _require_f32_cuda(weight=params[0], bias=params[1], residual_scale=params[2])
+    _require_f32_cuda(norm_weight=norm_weight, norm_bias=norm_bias, x=x)
+    dev = x.device
+    one = int(lib.gn_loop_tensor_bytes(B, M, N, K))
+    stat = outer * 4 * ((B + 3) // 4) * 8
+    stat = (stat + 255) // 256 * 256
+    y = torch.empty_like(x)
+    with torch.cuda.device(dev):
+        wbytes = int(lib.gn_loop_forward_workspace_bytes(B, M, N, K, inner, outer, block, int(residual)))
+        if wbytes == 0:
+            raise RuntimeError(f"the fused loop does not cover {tuple(x.shape)}, block {block}, {inner} inner iterations")
+        ws = torch.empty(wbytes, dtype=torch.uint8, device=dev)
+        stashes = [None] * outer
+        if need_grad:
+            stash_bytes = inner * one
+            keep = _kept_steps(one, stash_bytes, outer, dev)
+            total = (outer + 1) * one + stat + keep * stash_bytes
+            if total < _BIG:  # one allocation, cut up
+                try:
+                    pool = torch.empty(total, dtype=torch.uint8, device=dev)
+                except torch.cuda.OutOfMemoryError:
+                    keep = 0
+                    pool = torch.empty((outer + 1) * one + stat, dtype=torch.uint8, device=dev)
+                sizes = [stat] + [one] * (outer + 1) + [stash_bytes] * keep
+                parts, off = [], 0
+                for nb in sizes:
+                    parts.append(pool[off:off + nb])
+                    off += nb
+                stats, x_il4, outs = parts[0], parts[1], parts[2:2 + outer]
+                stashes[outer - keep:] = parts[2 + outer:]
+            else:
+                stats = torch.empty(stat, dtype=torch.uint8, device=dev)
+                x_il4 = _staggered(one, dev, 6)
+                outs = []
+                for k in range(outer):
+                    outs.append(_staggered(one, dev, k))
+                    if k >= outer - keep:
+                        stashes[k] = _staggered(stash_bytes, dev, k + 3)
+        else:
+            stats = torch.empty(stat, dtype=torch.uint8, device=dev)
+            x_il4 = torch.empty(one, dtype=torch.uint8, device=dev)
+            pair = [torch.empty(one, dtype=torch.uint8, device=dev) for _ in range(min(2, outer))]
+            outs = [pair[k & 1] for k in range(outer)]
+        weights, biases, scales = ([p[i] for p in plist] for i in range(3))
+        check(lib.gn_loop_forward_f32(_pointers(weights), _pointers(biases), _pointers(scales), len(plist),
+                                      norm_weight.data_ptr(), norm_bias.data_ptr(), x.data_ptr(), y.data_ptr(),
+                                      x_il4.data_ptr(), _pointers(outs), stats.data_ptr(), _pointers(stashes), B, M, N, K,
+                                      inner, outer, block, ln_eps, activation_id(activation), int(residual), ws.data_ptr(),
+                                      ws.numel(), torch.cuda.current_stream().cuda_stream))
+    return y, (x_il4, stats, outs, stashes)
+
+
+def _loop_backward(plist, norm_weight, norm_bias, saved, grad_y, inner: int, outer: int, block: int, activation: str,
+                   residual: bool):
+    """The gradients of :func:`_loop_forward` through ``gn_loop_backward_f32``: one (weight, bias, residual_scale) triple per
+    entry of ``plist``, then those of the norm's weight and bias and of x."""
+    x_il4, stats, outs, stashes = saved
+    g = grad_y.contiguous()
+    B, M, N, K = g.shape
+    dev = g.device
+    grads = [tuple(torch.empty_like(t) for t in params) for params in plist]
+    gg, gb, gx = torch.empty_like(norm_weight), torch.empty_like(norm_bias), torch.empty_like(g)
+    with torch.cuda.device(dev):
+        replay = int(any(t is None for t in stashes))
+        ws = torch.empty(int(lib.gn_loop_backward_workspace_bytes(B, M, N, K, inner, outer, block, int(residual), replay)),
+                         dtype=torch.uint8, device=dev)
+        columns = [_pointers([p[i] for p in plist]) for i in range(3)] + [_pointers([p[i] for p in grads]) for i in range(3)]
+        check(lib.gn_loop_backward_f32(*columns[:3], len(plist), norm_weight.data_ptr(), norm_bias.data_ptr(), x_il4.data_ptr(),
+                                       _pointers(outs), stats.data_ptr(), _pointers(stashes), g.data_ptr(), *columns[3:],
+                                       gg.data_ptr(), gb.data_ptr(), gx.data_ptr(), B, M, N, K, inner, outer, block,
+                                       activation_id(activation), int(residual), ws.data_ptr(), ws.numel(),
+                                       torch.cuda.current_stream().cuda_stream))
+    return grads, gg, gb, gx
+
+
+def _save_loop(ctx, params, saved):
+    x_il4, stats, outs, stashes = saved
+    ctx.kept = [t is not None for t in stashes]
+    ctx.save_for_backward(*params, x_il4, stats, *outs, *[t for t in stashes if t is not None])
+
+
+def _restore_loop(ctx, nparams: int, outer: int):
+    t = ctx.saved_tensors
+    params, rest = t[:nparams], t[nparams:]
+    outs, kept = rest[2:2 + outer], iter(rest[2 + outer:])
+    return params, (rest[0], rest[1], outs, [next(kept) if k else None for k in ctx.kept])
+
+
 class FusedLoopTrainOp(torch.autograd.Function):
     """The model loop of the reference's scripts with gradients:
 
@@ -215,14 +331,11 @@ class FusedLoopTrainOp(torch.autograd.Function):
         for _ in range(outer_iters):
             h = layer_norm(gridnet_step(weight, bias, residual_scale, h, ..., normalize=False), norm_weight, norm_bias)
 
-    (gridnet/scripts/train_mnist.py:62-64) as ONE autograd node, float32, shared parameters. The forward pass is the
-    fused loop of :func:`outer_forward`: every step kernel reduces the statistics of what it writes and normalises
-    its input while loading it, so between steps only the RAW step outputs (and [B, 2] statistics) exist and are
-    saved - half the activations that the step-by-step composition saves, and two passes over the grid fewer per
-    outer step. The backward pass walks the steps in reverse with the library's LayerNorm backward (reusing the
-    saved statistics) and the tuned step backward, whose normalised input is rebuilt from the saved raw tensor.
-    With the memory-for-time setting (:func:`keep_forward_stash`) the step kernels also keep their inner
-    iterations for the backward, as :class:`GridnetCudaOp` does.
+    (gridnet/scripts/train_mnist.py:62-64) as ONE autograd node, float32, shared parameters, on the quad kernels
+    (``gn_loop_forward_f32`` / ``gn_loop_backward_f32``): every step kernel reduces the statistics of what it writes and
+    normalises its input while loading it, so between steps only the RAW step outputs (and their statistics) exist and are
+    saved - half the activations that the step-by-step composition saves. The last steps also keep their inner iterations
+    for the backward pass, as many as the memory allows (:func:`keep_forward_stash`).
 
     ``FusedLoopTrainOp.apply(weight, bias, residual_scale, norm_weight, norm_bias, x, inner_iters, outer_iters,
     block_size, activation, ln_eps)``."""
@@ -231,46 +344,28 @@ class FusedLoopTrainOp(torch.autograd.Function):
     def supported(weight, x, inner_iters: int, block_size: int) -> bool:
         if weight.dtype != torch.float32 or not weight.is_cuda or inner_iters < 1 or x.shape[0] == 0:
             return False
-        B, M, N, K = x.shape
-        # the tuned forward (needed for the fusion) and the tuned backward both want whole 8^3 regions
-        return block_size in (4, 8) and M % 8 == 0 and N % 8 == 0 and K % 8 == 0 and \
-            int(lib.gn_step_backward_workspace_bytes(B, M, N, K, int(inner_iters), int(block_size), 0, 4)) > 0
+        return bool(lib.gn_loop_train_supported(*x.shape, int(inner_iters), int(block_size)))
 
     @staticmethod
     def forward(ctx, weight, bias, residual_scale, norm_weight, norm_bias, x, inner_iters: int, outer_iters: int,
                 block_size: int, activation: str, ln_eps: float):
-        need_grad = any(ctx.needs_input_grad[:6])
-        x = x.contiguous()
-        y, raws, stats, stashes = _fused_loop_forward([(weight, bias, residual_scale)] * int(outer_iters), norm_weight,
-                                                      norm_bias, x, int(inner_iters), int(block_size), activation,
-                                                      float(ln_eps), need_grad)
-        ctx.save_for_backward(weight, bias, residual_scale, norm_weight, norm_bias, x, *raws, *stats)
-        ctx.stashes = stashes
-        ctx.cfg = (int(inner_iters), int(outer_iters), int(block_size), activation, float(ln_eps))
+        ctx.cfg = (int(inner_iters), int(outer_iters), int(block_size), activation)
+        if not ctx.cfg[1]:
+            ctx.save_for_backward(weight, bias, residual_scale, norm_weight, norm_bias)
+            return x.clone()
+        y, saved = _loop_forward([(weight, bias, residual_scale)], norm_weight, norm_bias, x.contiguous(), *ctx.cfg,
+                                 float(ln_eps), False, any(ctx.needs_input_grad[:6]))
+        _save_loop(ctx, (weight, bias, residual_scale, norm_weight, norm_bias), saved)
         return y
 
     @staticmethod
     def backward(ctx, grad_y):
-        inner, outer, block, activation, ln_eps = ctx.cfg
-        saved = ctx.saved_tensors
-        weight, bias, scale, gamma, beta, x = saved[:6]
-        raws, stats = saved[6:6 + outer], saved[6 + outer:6 + 2 * outer]
-        stashes, ctx.stashes = ctx.stashes, None
-        total = []
-
-        def add(k, grads):  # the steps share one parameter set: their gradients are summed as they appear
-            if not total:
-                total.extend(grads)
-            else:
-                for acc, g in zip(total, grads):
-                    acc += g
-
-        gg, gbt, g = _fused_loop_backward([(weight, bias, scale)] * outer, gamma, beta, x, raws, stats, stashes,
-                                          grad_y, inner, block, activation, add)
-        if outer == 0:
-            z = torch.zeros_like
-            return z(weight), z(bias), z(scale), z(gamma), z(beta), g, None, None, None, None, None
-        return total[0], total[1], total[2], gg, gbt, g, None, None, None, None, None
+        outer = ctx.cfg[1]
+        if not outer:
+            return (*(torch.zeros_like(t) for t in ctx.saved_tensors), grad_y, None, None, None, None, None)
+        params, saved = _restore_loop(ctx, 5, outer)
+        grads, gg, gb, gx = _loop_backward([params[:3]], *params[3:], saved, grad_y, *ctx.cfg, False)
+        return (*grads[0], gg, gb, gx, None, None, None, None, None)
 
 
 class FusedLoopSeparateTrainOp(torch.autograd.Function):
@@ -286,34 +381,24 @@ class FusedLoopSeparateTrainOp(torch.autograd.Function):
                 *step_params):
         assert len(step_params) % 3 == 0, "three tensors (weight, bias, residual_scale) per outer step"
         plist = [tuple(step_params[i:i + 3]) for i in range(0, len(step_params), 3)]
-        need_grad = any(ctx.needs_input_grad)
-        x = x.contiguous()
-        y, raws, stats, stashes = _fused_loop_forward(plist, norm_weight, norm_bias, x, int(inner_iters),
-                                                      int(block_size), activation, float(ln_eps), need_grad)
-        ctx.save_for_backward(norm_weight, norm_bias, x, *step_params, *raws, *stats)
-        ctx.stashes = stashes
         ctx.cfg = (int(inner_iters), len(plist), int(block_size), activation)
+        if not plist:
+            ctx.save_for_backward(norm_weight, norm_bias)
+            return x.clone()
+        y, saved = _loop_forward(plist, norm_weight, norm_bias, x.contiguous(), *ctx.cfg, float(ln_eps), False,
+                                 any(ctx.needs_input_grad))
+        _save_loop(ctx, (norm_weight, norm_bias, *step_params), saved)
         return y
 
     @staticmethod
     def backward(ctx, grad_y):
-        inner, outer, block, activation = ctx.cfg
-        saved = ctx.saved_tensors
-        gamma, beta, x = saved[:3]
-        flat = saved[3:3 + 3 * outer]
-        plist = [tuple(flat[i:i + 3]) for i in range(0, 3 * outer, 3)]
-        raws, stats = saved[3 + 3 * outer:3 + 4 * outer], saved[3 + 4 * outer:3 + 5 * outer]
-        stashes, ctx.stashes = ctx.stashes, None
-        per_step = [None] * outer
-
-        def keep(k, grads):
-            per_step[k] = grads
-
-        gg, gbt, g = _fused_loop_backward(plist, gamma, beta, x, raws, stats, stashes, grad_y, inner, block, activation,
-                                          keep)
-        if outer == 0:
-            return torch.zeros_like(gamma), torch.zeros_like(beta), g, None, None, None, None
-        return (gg, gbt, g, None, None, None, None) + tuple(t for grads in per_step for t in grads)
+        outer = ctx.cfg[1]
+        if not outer:
+            return (*(torch.zeros_like(t) for t in ctx.saved_tensors), grad_y, None, None, None, None)
+        params, saved = _restore_loop(ctx, 2 + 3 * outer, outer)
+        plist = [params[i:i + 3] for i in range(2, 2 + 3 * outer, 3)]
+        grads, gg, gb, gx = _loop_backward(plist, *params[:2], saved, grad_y, *ctx.cfg, False)
+        return (gg, gb, gx, None, None, None, None) + tuple(t for triple in grads for t in triple)
 
 
 class FusedLoopResidualTrainOp(torch.autograd.Function):
@@ -322,10 +407,10 @@ class FusedLoopResidualTrainOp(torch.autograd.Function):
         for net in nets:  n = layer_norm(h);  h = h + (net(n) - n)
 
     as one autograd node. Forward: the step kernel normalises h while loading it, one pass writes
-    ``h + (y - layer_norm(h))`` and reduces the statistics of the result (``gn_norm_residual_combine_f32``); saved
-    are the step inputs h_k and their statistics (and the inner iterations of the last steps, memory permitting).
-    Backward, per step in reverse: the tuned step backward on the rebuilt ``n``, ``grad_n = grad_step - grad``,
-    the library's LayerNorm backward with the saved statistics, ``grad = grad + grad_h``.
+    ``h + (y - layer_norm(h))`` and reduces the statistics of the result; saved are the step inputs h_k and their
+    statistics (and the inner iterations of the last steps, memory permitting). Backward, per step in reverse: the step
+    backward on the rebuilt ``n``, then one pass for the sums of the LayerNorm gradient of ``grad_step - grad`` and one
+    that adds it to ``grad``.
 
     ``FusedLoopResidualTrainOp.apply(norm_weight, norm_bias, x, inner_iters, block_size, activation, ln_eps,
     outer_iters, *params)`` with ``params`` either one (weight, bias, residual_scale) shared by all outer steps or
@@ -336,281 +421,27 @@ class FusedLoopResidualTrainOp(torch.autograd.Function):
                 outer_iters: int, *params):
         outer = int(outer_iters)
         assert len(params) in (3, 3 * outer), "one (weight, bias, residual_scale), or one per outer step"
-        shared = len(params) == 3 and outer != 1
-        plist = [tuple(params[:3])] * outer if len(params) == 3 else [tuple(params[i:i + 3]) for i in range(0, 3 * outer, 3)]
-        x = x.contiguous()
-        B, M, N, K = x.shape
-        P = M * N * K
-        act = activation_id(activation)
-        dev = x.device
-        _require_f32_cuda(norm_weight=norm_weight, norm_bias=norm_bias, x=x)
-        need_grad = any(ctx.needs_input_grad)
-        inputs, stats, stashes = [], [], []
-        with torch.cuda.device(dev):
-            st = torch.cuda.current_stream().cuda_stream
-            nws = _workspace(lib.gn_norm_workspace_bytes(B, P), dev)
-            sums = torch.empty(B, 2, dtype=torch.float64, device=dev)
-            mr = torch.empty(B, 2, dtype=torch.float32, device=dev)
-            h = x
-            if outer:
-                check(lib.gn_norm_local_sums_f32(h.data_ptr(), sums.data_ptr(), B, P, nws.data_ptr(), nws.numel(), st))
-                check(lib.gn_norm_finalize_f32(sums.data_ptr(), 1, mr.data_ptr(), B, P, float(ln_eps), st))
-            keep = _stash_steps(plist[0][0], x, inner_iters, block_size, outer) if need_grad and outer else 0
-            y = torch.empty_like(x)
-            for k, (weight, bias, residual_scale) in enumerate(plist):
-                _assert_step_args(weight, bias, residual_scale, x, block_size, False)
-                _require_f32_cuda(weight=weight, bias=bias, residual_scale=residual_scale)
-                stash = None
-                if need_grad and k >= outer - keep:
-                    stash = _staggered_bytes(int(lib.gn_step_stash_bytes(B, M, N, K, int(inner_iters), int(block_size))),
-                                             dev, k + 3)
-                check(lib.gn_step_forward_train_f32(
-                    weight.data_ptr(), bias.data_ptr(), residual_scale.data_ptr(), h.data_ptr(), y.data_ptr(),
-                    norm_weight.data_ptr(), norm_bias.data_ptr(), mr.data_ptr(), None, B, M, N, K, int(inner_iters),
-                    int(block_size), act, None if stash is None else stash.data_ptr(),
-                    0 if stash is None else stash.numel(), st))
-                nxt = _staggered_like(x, k) if need_grad else torch.empty_like(x)
-                mr_next = torch.empty(B, 2, dtype=torch.float32, device=dev)
-                check(lib.gn_norm_residual_combine_f32(h.data_ptr(), y.data_ptr(), norm_weight.data_ptr(),
-                                                       norm_bias.data_ptr(), mr.data_ptr(), nxt.data_ptr(),
-                                                       mr_next.data_ptr(), B, P, float(ln_eps), nws.data_ptr(),
-                                                       nws.numel(), st))
-                if need_grad:
-                    inputs.append(h)
-                    stats.append(mr)
-                    stashes.append(stash)
-                h, mr = nxt, mr_next
-            out = h if outer else x.clone()
-        ctx.save_for_backward(norm_weight, norm_bias, *params, *inputs, *stats)
-        ctx.stashes = stashes
-        ctx.cfg = (int(inner_iters), outer, int(block_size), activation, len(params), shared)
-        return out
+        ctx.cfg = (int(inner_iters), outer, int(block_size), activation)
+        if not outer:
+            ctx.save_for_backward(norm_weight, norm_bias, *params)
+            return x.clone()
+        plist = [tuple(params[i:i + 3]) for i in range(0, len(params), 3)]
+        y, saved = _loop_forward(plist, norm_weight, norm_bias, x.contiguous(), *ctx.cfg, float(ln_eps), True,
+                                 any(ctx.needs_input_grad))
+        ctx.nparams = 2 + len(params)
+        _save_loop(ctx, (norm_weight, norm_bias, *params), saved)
+        return y
 
     @staticmethod
     def backward(ctx, grad_out):
-        inner, outer, block, activation, nparams, shared = ctx.cfg
-        saved = ctx.saved_tensors
-        gamma, beta = saved[:2]
-        params = saved[2:2 + nparams]
-        plist = [tuple(params[:3])] * outer if nparams == 3 else [tuple(params[i:i + 3]) for i in range(0, 3 * outer, 3)]
-        inputs, stats = saved[2 + nparams:2 + nparams + outer], saved[2 + nparams + outer:2 + nparams + 2 * outer]
-        stashes, ctx.stashes = list(ctx.stashes), None
-        g = grad_out.contiguous()
-        if outer == 0:
-            return (torch.zeros_like(gamma), torch.zeros_like(beta), g, None, None, None, None, None) + \
-                tuple(torch.zeros_like(t) for t in params)
-        B, M, N, K = g.shape
-        P = M * N * K
-        dev = g.device
-        per_step = [None] * outer
-        total = None
-        gg = gbt = None
-        with torch.cuda.device(dev):
-            st = torch.cuda.current_stream().cuda_stream
-            nws = _workspace(lib.gn_norm_workspace_bytes(B, P), dev)
-            sums = torch.empty(B, 2, dtype=torch.float64, device=dev)
-            for k in reversed(range(outer)):
-                weight, bias, scale = plist[k]
-                h, mr = inputs[k], stats[k]
-                dw, db, ds, gn = (torch.empty_like(t) for t in (weight, bias, scale, h))
-                # the step's input n = layer_norm(h): rebuilt by the backward kernels while they load h (block 8),
-                # else by a pass here
-                if _step_backward_fused_in(weight, bias, scale, h, mr, gamma, beta, g, dw, db, ds, gn, inner, block,
-                                           activation, stashes[k]):
-                    stashes[k] = None
-                else:
-                    n = torch.empty_like(h)
-                    check(lib.gn_norm_apply_f32(h.data_ptr(), gamma.data_ptr(), beta.data_ptr(), mr.data_ptr(), n.data_ptr(),
-                                                B, P, st))
-                    if stashes[k] is not None:
-                        gridnet_cuda.backward_with_stash(weight, bias, scale, n, g, dw, db, ds, gn, inner, block, activation,
-                                                         stashes[k])
-                        stashes[k] = None
-                    else:
-                        gridnet_cuda.backward(weight, bias, scale, n, g, dw, db, ds, gn, inner, block, 1e-5, False, activation)
-                    del n
-                gn -= g  # h' = h + net(n) - n: n also enters with a minus sign
-                gh, dg, dbt = torch.empty_like(h), torch.empty_like(gamma), torch.empty_like(gamma)
-                check(lib.gn_norm_backward_local_sums_f32(h.data_ptr(), gamma.data_ptr(), gn.data_ptr(), mr.data_ptr(),
-                                                          sums.data_ptr(), B, P, nws.data_ptr(), nws.numel(), st))
-                check(lib.gn_norm_backward_apply_f32(h.data_ptr(), gamma.data_ptr(), gn.data_ptr(), mr.data_ptr(),
-                                                     sums.data_ptr(), P, gh.data_ptr(), dg.data_ptr(), dbt.data_ptr(), B, P,
-                                                     nws.data_ptr(), nws.numel(), st))
-                g = g + gh
-                if nparams == 3:
-                    if total is None:
-                        total = [dw, db, ds]
-                    else:
-                        for acc, t in zip(total, (dw, db, ds)):
-                            acc += t
-                else:
-                    per_step[k] = (dw, db, ds)
-                if gg is None:
-                    gg, gbt = dg, dbt
-                else:
-                    gg += dg
-                    gbt += dbt
-        pgrads = tuple(total) if nparams == 3 else tuple(t for grads in per_step for t in grads)
-        return (gg, gbt, g, None, None, None, None, None) + pgrads
-
-
-_STAGGER = 4352  # bytes: 17 x 256, keeps 16-byte alignment
-_STAGGER_FROM = 1 << 30  # only tensors of a GiB and more: measured at 2 GiB (C3); at 128 MiB (C4) it cost 1 %
-
-
-def _staggered_bytes(nbytes: int, device, k: int) -> torch.Tensor:
-    """``nbytes`` of device memory starting ``(k % 7 + 1) * 4352`` bytes into its allocation. The tensors a training
-    step streams side by side (input, output, kept iterations) are each an exact power of two in size at the
-    benchmark's shapes, so fresh allocations start at the same offset inside every 2 MB page; depending on where
-    the driver put the pages, the forward pass of C3 then took anything from 79 to 105 ms. Different offsets make
-    the streams fall on different memory channels whatever the placement."""
-    if nbytes < _STAGGER_FROM:
-        return torch.empty(nbytes, dtype=torch.uint8, device=device)
-    off = (k % 7 + 1) * _STAGGER
-    return torch.empty(nbytes + 8 * _STAGGER, dtype=torch.uint8, device=device)[off:off + nbytes]
-
-
-def _staggered_like(x: torch.Tensor, k: int) -> torch.Tensor:
-    return _staggered_bytes(x.numel() * x.element_size(), x.device, k).view(x.dtype).view(x.shape)
-
-
-def _fused_loop_forward(plist, norm_weight, norm_bias, x, inner_iters, block_size, activation, ln_eps, need_grad):
-    """The fused forward of the model loop with one (weight, bias, residual_scale) per outer step: every step kernel
-    normalises its input while loading it and reduces the statistics of what it writes. Returns the normalised
-    final grid, the raw step outputs, their (mean, rstd) and the kept inner iterations (or None) per step."""
-    B, M, N, K = x.shape
-    P = M * N * K
-    act = activation_id(activation)
-    dev = x.device
-    for weight, bias, residual_scale in plist:
-        _assert_step_args(weight, bias, residual_scale, x, block_size, False)
-        assert norm_weight.shape == bias.shape == norm_bias.shape, f"{norm_weight.shape=} invalid for {bias.shape=}"
-        _require_f32_cuda(weight=weight, bias=bias, residual_scale=residual_scale)
-    _require_f32_cuda(norm_weight=norm_weight, norm_bias=norm_bias, x=x)
-    nparts = int(lib.gn_step_stats_partials(M, N, K, block_size))
-    partials = torch.empty(B, nparts, 2, dtype=torch.float64, device=dev)
-    raws, stats, stashes = [], [], []
-    src, src_stats = x, None
-    with torch.cuda.device(dev):
-        st = torch.cuda.current_stream().cuda_stream
-        # the LAST steps keep their inner iterations: their backward comes first, so their stash is freed first
-        keep = _stash_steps(plist[0][0], x, inner_iters, block_size, len(plist)) if need_grad and plist else 0
-        for k, (weight, bias, residual_scale) in enumerate(plist):
-            dst = _staggered_like(x, k) if need_grad else torch.empty_like(x)
-            stash = None
-            if need_grad and k >= len(plist) - keep:
-                stash = _staggered_bytes(int(lib.gn_step_stash_bytes(B, M, N, K, int(inner_iters), int(block_size))),
-                                         dev, k + 3)
-            check(lib.gn_step_forward_train_f32(
-                weight.data_ptr(), bias.data_ptr(), residual_scale.data_ptr(), src.data_ptr(), dst.data_ptr(),
-                norm_weight.data_ptr(), norm_bias.data_ptr(), None if src_stats is None else src_stats.data_ptr(),
-                partials.data_ptr(), B, M, N, K, int(inner_iters), int(block_size), act,
-                None if stash is None else stash.data_ptr(), 0 if stash is None else stash.numel(), st))
-            mr = torch.empty(B, 2, dtype=torch.float32, device=dev)
-            check(lib.gn_norm_finalize_f32(partials.data_ptr(), nparts, mr.data_ptr(), B, P, float(ln_eps), st))
-            if need_grad:
-                raws.append(dst)
-                stats.append(mr)
-                stashes.append(stash)
-            src, src_stats = dst, mr
-        y = torch.empty_like(x)
-        if plist:
-            check(lib.gn_norm_apply_f32(src.data_ptr(), norm_weight.data_ptr(), norm_bias.data_ptr(),
-                                        src_stats.data_ptr(), y.data_ptr(), B, P, st))
-        else:
-            y.copy_(x)
-    return y, raws, stats, stashes
-
-
-def _step_backward_fused_in(weight, bias, scale, x_raw, mean_rstd, gamma, beta, gy, dw, db, ds, gx, inner, block,
-                            activation, stash) -> bool:
-    """The tuned step backward on an input given as (raw tensor, statistics, norm parameters); False where the
-    library has no such path (the caller then normalises first)."""
-    from ._lib import GN_ERR_UNSUPPORTED
-
-    if int(block) != 8:
-        return False
-    B, M, N, K = x_raw.shape
-    with torch.cuda.device(x_raw.device):
-        if stash is not None:
-            need = int(lib.gn_step_backward_stash_workspace_bytes(B, M, N, K, int(inner), int(block)))
-        else:
-            need = int(lib.gn_step_backward_workspace_bytes(B, M, N, K, int(inner), int(block), 0, 4))
-        if need <= 0:
-            return False
-        ws = torch.empty(need, dtype=torch.uint8, device=x_raw.device)
-        rc = lib.gn_step_backward_fused_in_f32(
-            weight.data_ptr(), bias.data_ptr(), scale.data_ptr(), x_raw.data_ptr(), mean_rstd.data_ptr(), gamma.data_ptr(),
-            beta.data_ptr(), gy.data_ptr(), dw.data_ptr(), db.data_ptr(), ds.data_ptr(), gx.data_ptr(), B, M, N, K,
-            int(inner), int(block), activation_id(activation), None if stash is None else stash.data_ptr(),
-            0 if stash is None else stash.numel(), ws.data_ptr(), ws.numel(), torch.cuda.current_stream().cuda_stream)
-    if rc == GN_ERR_UNSUPPORTED:
-        return False
-    check(rc)
-    return True
-
-
-def _fused_loop_backward(plist, gamma, beta, x, raws, stats, stashes, grad_y, inner, block, activation, sink):
-    """The reverse walk over the steps of :func:`_fused_loop_forward`: the library's LayerNorm backward with the
-    saved statistics, then the tuned step backward on the step's normalised input rebuilt from the saved raw
-    tensor. ``sink(k, (dw, db, ds))`` receives step k's parameter gradients; returns the gradients of the norm
-    weight and bias (summed over the steps) and of x."""
-    outer = len(plist)
-    B, M, N, K = x.shape
-    P = M * N * K
-    dev = x.device
-    g = grad_y.contiguous()
-    gg = gbt = None
-    stashes = list(stashes)
-    with torch.cuda.device(dev):
-        st = torch.cuda.current_stream().cuda_stream
-        nws = _workspace(lib.gn_norm_workspace_bytes(B, P), dev)
-        sums = torch.empty(B, 2, dtype=torch.float64, device=dev)
-        for k in reversed(range(outer)):
-            weight, bias, scale = plist[k]
-            # LayerNorm backward of step k with the statistics saved by the forward pass
-            gs_k, dg, dbt = torch.empty_like(x), torch.empty_like(gamma), torch.empty_like(gamma)
-            check(lib.gn_norm_backward_local_sums_f32(raws[k].data_ptr(), gamma.data_ptr(), g.data_ptr(),
-                                                      stats[k].data_ptr(), sums.data_ptr(), B, P, nws.data_ptr(),
-                                                      nws.numel(), st))
-            check(lib.gn_norm_backward_apply_f32(raws[k].data_ptr(), gamma.data_ptr(), g.data_ptr(), stats[k].data_ptr(),
-                                                 sums.data_ptr(), P, gs_k.data_ptr(), dg.data_ptr(), dbt.data_ptr(), B, P,
-                                                 nws.data_ptr(), nws.numel(), st))
-            dw, db, ds, gx = (torch.empty_like(t) for t in (weight, bias, scale, x))
-            # the step's input: x itself for the first step, else the normalised output of the step before - which
-            # the backward kernels rebuild while loading the raw tensor where they can (block 8), else a pass here
-            if k > 0 and _step_backward_fused_in(weight, bias, scale, raws[k - 1], stats[k - 1], gamma, beta, gs_k, dw, db,
-                                                 ds, gx, inner, block, activation, stashes[k]):
-                stashes[k] = None
-                sink(k, (dw, db, ds))
-                if gg is None:
-                    gg, gbt = dg, dbt
-                else:
-                    gg += dg
-                    gbt += dbt
-                g = gx
-                continue
-            if k == 0:
-                xin = x
-            else:
-                xin = torch.empty_like(x)
-                check(lib.gn_norm_apply_f32(raws[k - 1].data_ptr(), gamma.data_ptr(), beta.data_ptr(),
-                                            stats[k - 1].data_ptr(), xin.data_ptr(), B, P, st))
-            if stashes[k] is not None:
-                gridnet_cuda.backward_with_stash(weight, bias, scale, xin, gs_k, dw, db, ds, gx, inner, block, activation,
-                                                 stashes[k])
-                stashes[k] = None
-            else:
-                gridnet_cuda.backward(weight, bias, scale, xin, gs_k, dw, db, ds, gx, inner, block, 1e-5, False,
-                                      activation)
-            sink(k, (dw, db, ds))
-            if gg is None:
-                gg, gbt = dg, dbt
-            else:
-                gg += dg
-                gbt += dbt
-            g = gx
-    return gg, gbt, g
+        outer = ctx.cfg[1]
+        if not outer:
+            z = [torch.zeros_like(t) for t in ctx.saved_tensors]
+            return (z[0], z[1], grad_out, None, None, None, None, None, *z[2:])
+        params, saved = _restore_loop(ctx, ctx.nparams, outer)
+        plist = [params[i:i + 3] for i in range(2, ctx.nparams, 3)]
+        grads, gg, gb, gx = _loop_backward(plist, *params[:2], saved, grad_out, *ctx.cfg, True)
+        return (gg, gb, gx, None, None, None, None, None) + tuple(t for triple in grads for t in triple)
 
 
 def fused_loop_forward(step_params, norm_weight, norm_bias, x, inner_iters: int, block_size: int,
@@ -618,41 +449,18 @@ def fused_loop_forward(step_params, norm_weight, norm_bias, x, inner_iters: int,
     """The model loop of gridnet/scripts/train_imagenet.py:76-86 without gradients, for the variants that
     :func:`outer_forward` does not take: ``step_params`` is one ``(weight, bias, residual_scale)`` per outer step
     (``separate_params``; repeat one tuple for shared parameters), and with ``outer_residual`` a step is
-    ``n = norm(h); h = h + (net(n) - n)`` instead of ``h = norm(net(h))``. Float32, tuned step kernel
-    (whole 8^3 regions, block 4 or 8). The normalised tensor is never stored: the step kernel normalises while it
-    loads, and either it (plain form) or the combining pass (residual form) reduces the next statistics."""
-    x = x.contiguous()
-    if not outer_residual:
-        with torch.no_grad():
-            return _fused_loop_forward(list(step_params), norm_weight, norm_bias, x, int(inner_iters), int(block_size),
-                                       activation, float(ln_eps), False)[0]
-    B, M, N, K = x.shape
-    P = M * N * K
-    act = activation_id(activation)
-    dev = x.device
-    _require_f32_cuda(norm_weight=norm_weight, norm_bias=norm_bias, x=x)
-    with torch.cuda.device(dev), torch.no_grad():
-        st = torch.cuda.current_stream().cuda_stream
-        nws = _workspace(lib.gn_norm_workspace_bytes(B, P), dev)
-        sums = torch.empty(B, 2, dtype=torch.float64, device=dev)
-        mr = [torch.empty(B, 2, dtype=torch.float32, device=dev) for _ in range(2)]
-        h, y = x, torch.empty_like(x)
-        out = torch.empty_like(x)
-        check(lib.gn_norm_local_sums_f32(h.data_ptr(), sums.data_ptr(), B, P, nws.data_ptr(), nws.numel(), st))
-        check(lib.gn_norm_finalize_f32(sums.data_ptr(), 1, mr[0].data_ptr(), B, P, float(ln_eps), st))
-        for k, (weight, bias, residual_scale) in enumerate(step_params):
-            _assert_step_args(weight, bias, residual_scale, x, block_size, False)
-            _require_f32_cuda(weight=weight, bias=bias, residual_scale=residual_scale)
-            cur, nxt = mr[k & 1], mr[(k + 1) & 1]
-            check(lib.gn_step_forward_train_f32(
-                weight.data_ptr(), bias.data_ptr(), residual_scale.data_ptr(), h.data_ptr(), y.data_ptr(),
-                norm_weight.data_ptr(), norm_bias.data_ptr(), cur.data_ptr(), None, B, M, N, K, int(inner_iters),
-                int(block_size), act, None, 0, st))
-            check(lib.gn_norm_residual_combine_f32(h.data_ptr(), y.data_ptr(), norm_weight.data_ptr(),
-                                                   norm_bias.data_ptr(), cur.data_ptr(), out.data_ptr(), nxt.data_ptr(),
-                                                   B, P, float(ln_eps), nws.data_ptr(), nws.numel(), st))
-            h = out  # the combining pass may write over its own h
-        return h.clone() if h is x else h
+    ``n = norm(h); h = h + (net(n) - n)`` instead of ``h = norm(net(h))``. Float32, whole 8^3 regions, block 4 or 8. The
+    normalised tensor is never stored: the step kernel normalises while it loads, and either it (plain form) or the
+    combining pass (residual form) reduces the next statistics."""
+    plist = [tuple(p) for p in step_params]
+    outer = len(plist)
+    if not outer or not x.shape[0]:
+        return x.clone()
+    if all(t is u for p in plist[1:] for t, u in zip(p, plist[0])):
+        plist = plist[:1]  # shared parameters: re-ordered once
+    with torch.no_grad():
+        return _loop_forward(plist, norm_weight, norm_bias, x.contiguous(), int(inner_iters), outer, int(block_size),
+                             activation, float(ln_eps), bool(outer_residual), False)[0]
 
 
 def device_status(clear: bool = True, device=None) -> bool:

@@ -143,7 +143,7 @@ struct QuadStep {
     const float2 *in_stats;   // [4 Q] or nullptr
     double2 *out_partials;    // [4 Q][nparts] or nullptr; slots 0 .. regions-1 of every row are written
     int nparts;
-    float *save_h, *save_x;   // replay (IL4 tensors, [inner] and [inner - 1] of them) or nullptr
+    float *save_h;            // [inner] IL4 tensors of pre-activations, or nullptr
     int *error_flag;
     int M, N, K, Q, inner, block;
 };
@@ -157,6 +157,43 @@ int launch_to_il4(const float *x, float *il, int B, long long P, cudaStream_t st
 int launch_from_il4(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, long long P,
                     cudaStream_t st);
 int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st);
+
+// ---- step_quad_bwd.cu (backward of the quad kernels; all activation tensors IL4)
+struct QuadReverse {
+    const float *packed_t;     // launch_quad_pack(..., transposed) with (norm weight, scale) in the place of (bias, scale)
+    const float *g;            // gradient of the step's output; with raw: of its normalised output
+    const float *raw;          // the step's output, or nullptr
+    const float2 *stats, *ac;  // with raw
+    const float *h;            // [inner]
+    float *delta, *dsum, *gx;  // [inner], one, one
+    float *dsq;                // [Q][P]
+    int M, N, K, Q, inner, block;
+};
+int launch_quad_reverse(const QuadReverse &a, int act, cudaStream_t st);
+struct QuadWgrad {
+    const float *in_il4;       // the step's input (with in_stats: the raw output of the step before)
+    const float2 *gbt;
+    const float2 *in_stats;
+    const float *delta, *h, *dsq;
+    const float *scale;        // native layout: activations between iterations are rebuilt from h
+    float *gpk;                // quad_grad_floats(...)
+    int accumulate;
+    int *error_flag;
+    int M, N, K, Q, inner, block;
+};
+size_t quad_grad_floats(int M, int N, int K, int Q);
+int launch_quad_wgrad(const QuadWgrad &a, int act, cudaStream_t st);
+int launch_quad_unpack_grads(const float *gpk, float *gw, float *gb, float *gs, int M, int N, int K, int Q, int block, cudaStream_t st);
+int launch_quad_border(const float *w, const float *dsum, float *gx, int M, int N, int K, int Q, int block, cudaStream_t st);
+int quad_norm_parts(long long P);
+int launch_quad_norm_sums(const float *x, const float *g, const float *sub, const float *gamma, const float2 *stats, double2 *partials,
+                          float *ggamma, float *gbeta, int accumulate, float2 *ac, int Q, long long P, cudaStream_t st);
+int launch_quad_norm_residual_apply(const float *h, const float *gn, const float *gu, const float *gamma, const float2 *stats, const float2 *ac,
+                                    float *out, int Q, long long P, cudaStream_t st);
+int quad_combine_parts(long long P);
+int launch_quad_residual_combine(const float *h, const float *y, const float *gamma, const float *beta, const float2 *stats, float *out,
+                                 double2 *partials, int Q, long long P, cudaStream_t st);
+int quad_make_map(CUtensorMap *map, const float *il, int M, int N, int K, int Q, int block);
 
 // ---- status.cu: device address of the per-device status word that kernels set when a bounded wait gives up
 // and the caller passed no flag of its own (nullptr if it cannot be resolved)

@@ -100,6 +100,86 @@ __device__ __forceinline__ void cp_async16(unsigned dst, const void *src)
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+// ---- a lane's 16 cells in an IL4 tensor. base: its first cell row (dz = dy = 0) at x = 4 h, the lower end of its x half;
+// zstr, ystr: floats to the next row in z and (signed) in y. 32 bytes, a whole sector, per access: cells one by one, the
+// two halves of a sector go to memory separately.
+__device__ __forceinline__ void stg256(float *p, u64 a, u64 b, u64 c, u64 d)
+{
+    asm volatile("st.global.v4.b64 [%0], {%1, %2, %3, %4};" ::"l"(p), "l"(a), "l"(b), "l"(c), "l"(d) : "memory");
+}
+__device__ __forceinline__ void ldg256(const float *p, u64 &a, u64 &b, u64 &c, u64 &d)
+{
+    asm volatile("ld.global.v4.b64 {%0, %1, %2, %3}, [%4];" : "=l"(a), "=l"(b), "=l"(c), "=l"(d) : "l"(p) : "memory");
+}
+// two x-neighbours (o = 2 j, 2 j + 1) of neuron row n
+__device__ __forceinline__ void quad_store2(float *base, int n, int j, long long zstr, long long ystr, int h, const u64 (&v)[4][2])
+{
+    float *p = base + (n >> 1) * zstr + (n & 1) * ystr + 8 * (j ^ h);
+    const u64 *lo = v[2 * j], *hi = v[2 * j + 1];
+    stg256(p, h ? hi[0] : lo[0], h ? hi[1] : lo[1], h ? lo[0] : hi[0], h ? lo[1] : hi[1]);
+}
+__device__ __forceinline__ void quad_store(float *base, long long zstr, long long ystr, int h, const u64 (&v)[4][4][2])
+{
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) quad_store2(base, n, j, zstr, ystr, h, v[n]);
+}
+__device__ __forceinline__ void quad_load(const float *base, long long zstr, long long ystr, int h, u64 (&v)[4][4][2])
+{
+#pragma unroll
+    for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            u64 a, b, c, d;
+            ldg256(base + (n >> 1) * zstr + (n & 1) * ystr + 8 * (j ^ h), a, b, c, d);
+            v[n][2 * j][0] = h ? c : a;
+            v[n][2 * j][1] = h ? d : b;
+            v[n][2 * j + 1][0] = h ? a : c;
+            v[n][2 * j + 1][1] = h ? b : d;
+        }
+}
+// ---- a region's 512 cells, staged in shared memory by whole lines: cell (z, y, x) at unit (8 z + y) 8 + (x ^ (y >> 1)) of 16
+// bytes. The swizzle keeps both the copies (8 lanes to a row) and the reads of a lane's own cells free of bank conflicts.
+// src: the region's first cell; cells of planes z0 .. z0 + nz - 1, 4 rows per instruction.
+template <int Z0, int NZ>
+__device__ __forceinline__ void quad_stage(unsigned stage, const float *src, long long zstr, int K, int lane)
+{
+    const int y = lane >> 3, x = lane & 7;
+    const float *s = src + ((long long)y * K + x) * 4 + Z0 * zstr;
+#pragma unroll
+    for (int k = 2 * Z0; k < 2 * (Z0 + NZ); ++k) {
+        const int yy = y + 4 * (k & 1);
+        cp_async16(stage + (unsigned)(((k >> 1) * 8 + yy) * 8 + (x ^ (yy >> 1))) * 16u, s + (k & 1) * 16ll * K + ((k >> 1) - Z0) * zstr);
+    }
+}
+// the same for four planes z0, z0 + dz, ...
+__device__ __forceinline__ void quad_stage4(unsigned stage, const float *src, long long zstr, int K, int lane, int z0, int dz)
+{
+    const int y = lane >> 3, x = lane & 7;
+    const float *s = src + ((long long)y * K + x) * 4 + z0 * zstr;
+    const unsigned d0 = stage + (unsigned)((z0 * 8 + y) * 8 + (x ^ (y >> 1))) * 16u;
+    const unsigned d1 = stage + (unsigned)((z0 * 8 + y + 4) * 8 + (x ^ ((y + 4) >> 1))) * 16u;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        cp_async16(d0 + k * dz * 1024, s + k * dz * zstr);
+        cp_async16(d1 + k * dz * 1024, s + k * dz * zstr + 16ll * K);
+    }
+}
+// offset of a lane's own cell (n = (dz, dy), o) in such a staging area: row(n) + ((o ^ e) * 16)
+template <int SUB>
+struct QuadStage {
+    unsigned row0, e;
+    int ys;
+    __device__ __forceinline__ explicit QuadStage(const QuadLane<SUB> &L)
+    {
+        row0 = (unsigned)(L.z0 * 8 + L.y0) * 128u;
+        e = (L.h ? 7u : 0u) ^ (unsigned)(L.y0 >> 1);
+        ys = L.ysgn * 128;
+    }
+    __device__ __forceinline__ unsigned at(int n, int o) const { return row0 + (n >> 1) * 1024u + (unsigned)((n & 1) * ys) + (((unsigned)o ^ e) << 4); }
+};
+
 // the warps of a team
 template <int TEAM>
 __device__ __forceinline__ void team_sync(int quarter)
@@ -142,15 +222,15 @@ __device__ __forceinline__ void quad_load_params(const float *packed, int role, 
 //   FWD: acc starts at the bias, and done(n, o, scale, centre) is called when a sum is complete - for the neurons of
 //   dy = 0 between the FMAs of the last window rows, so that their activation functions (MUFU) run under them.
 //   Otherwise acc is added to, and done is not called.
-template <int SUB, bool FWD, typename Done>
-__device__ __forceinline__ void quad_stencil(unsigned win, unsigned tm, const QuadLane<SUB> &L, u64 (&acc)[4][4][2], Done done)
+//   rows[ry]: where window row ry of plane 0, column 0 starts; PLANE: cells from one plane to the next; dx: bytes from
+//   one column to the next.
+template <int PLANE, bool FWD, typename Done>
+__device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, unsigned tm, u64 (&acc)[4][4][2], Done done)
 {
-    using G = QuadGeo<SUB>;
-    const int dx = L.xsgn * 16, dy_ = L.ysgn * G::ROW * 16;
     float wb[2][12], sc[2][4];
     auto finish = [&](int n, int o, float s) {
         u64 c0, c1;
-        lds128u(win + (unsigned)((1 + (n & 1)) * dy_ + (1 + o) * dx) + (1 + (n >> 1)) * G::PLANE * 16u, c0, c1);
+        lds128u(rows[1 + (n & 1)] + (unsigned)((1 + o) * dx) + (1 + (n >> 1)) * PLANE * 16u, c0, c1);
         done(n, o, s, c0, c1);
     };
     if (FWD) {
@@ -169,12 +249,12 @@ __device__ __forceinline__ void quad_stencil(unsigned win, unsigned tm, const Qu
     for (int ry = 0; ry < 4; ++ry) {
         unsigned a6[6];
 #pragma unroll
-        for (int j = 0; j < 6; ++j) a6[j] = win + (unsigned)(ry * dy_ + j * dx);
+        for (int j = 0; j < 6; ++j) a6[j] = rows[ry] + (unsigned)(j * dx);
 #pragma unroll
         for (int rz = 0; rz < 4; ++rz) {
             u64 v[6][2];
 #pragma unroll
-            for (int j = 0; j < 6; ++j) lds128u(a6[j] + rz * G::PLANE * 16u, v[j][0], v[j][1]);
+            for (int j = 0; j < 6; ++j) lds128u(a6[j] + rz * PLANE * 16u, v[j][0], v[j][1]);
 #pragma unroll
             for (int n = 0; n < 4; ++n) {
                 const int a = rz - (n >> 1), b = ry - (n & 1);

@@ -1,0 +1,247 @@
+// The model loop with gradients on the quad kernels, as two calls: forward (also without gradients) and backward.
+//
+//   plain     h = x;  repeat: h = layer_norm(step(h))                gridnet/scripts/train_mnist.py:62-64
+//   residual  h = x;  repeat: n = layer_norm(h); h = h + step(n) - n  gridnet/scripts/train_imagenet.py:81-83
+//
+// with one set of step parameters for all outer steps or one per step (train_imagenet.py:54-58). Activations stay in the
+// IL4 layout from the first step to the last; everything that a step needs is queued from here, so an outer step costs the
+// host a few microseconds (as a sequence of library calls and tensor operations from Python it was 30 us forward and
+// 150 us backward, which is what small models took).
+#include "common.cuh"
+#include "kernels.h"
+
+namespace gn {
+
+static size_t up256(size_t v) { return (v + 255) / 256 * 256; }
+
+struct LoopDims {
+    int B, M, N, K, Q, inner, outer, block, nparams, residual;
+    long long P;
+    size_t T4;  // floats of an IL4 tensor
+    int regions;
+};
+
+static LoopDims loop_dims(int B, int M, int N, int K, int inner, int outer, int block, int nparams, int residual)
+{
+    LoopDims d;
+    d.B = B; d.M = M; d.N = N; d.K = K; d.Q = (B + 3) / 4; d.inner = inner; d.outer = outer; d.block = block;
+    d.nparams = nparams; d.residual = residual;
+    d.P = (long long)M * N * K;
+    d.T4 = (size_t)d.Q * d.P * 4;
+    d.regions = (M / 8) * (N / 8) * (K / 8);
+    return d;
+}
+
+struct LoopWs {
+    float *packed, *packed_t, *gpk, *tmp, *g[2], *delta, *dsum, *dsq, *replay;
+    float2 *gbt, *ac;
+    double2 *partials;
+    int *error_flag;
+    size_t bytes;
+};
+
+// replay: some step has no kept iterations, so the backward pass runs the inner iterations again
+static LoopWs carve_loop(void *base, const LoopDims &d, bool backward, bool replay)
+{
+    LoopWs w{};
+    size_t off = 0;
+    unsigned char *p = static_cast<unsigned char *>(base);
+    auto take = [&](size_t bytes) {
+        void *r = p + off;
+        off = up256(off + bytes);
+        return r;
+    };
+    const size_t pk = sizeof(float) * quad_packed_floats(d.M, d.N, d.K), t = sizeof(float) * d.T4;
+    size_t parts = d.regions;
+    if (backward && (size_t)quad_norm_parts(d.P) > parts) parts = quad_norm_parts(d.P);
+    if (d.residual && (size_t)quad_combine_parts(d.P) > parts) parts = quad_combine_parts(d.P);
+    w.error_flag = static_cast<int *>(take(sizeof(int)));
+    w.partials = static_cast<double2 *>(take(sizeof(double2) * parts * 4 * d.Q));
+    w.gbt = static_cast<float2 *>(take(sizeof(float2) * (size_t)d.regions * quad_tile_cells(d.block)));
+    if (!backward || replay) w.packed = static_cast<float *>(take(pk));
+    if (!backward && d.residual) w.tmp = static_cast<float *>(take(t));
+    if (backward) {
+        w.packed_t = static_cast<float *>(take(pk));
+        w.gpk = static_cast<float *>(take(sizeof(float) * quad_grad_floats(d.M, d.N, d.K, d.Q)));
+        w.ac = static_cast<float2 *>(take(sizeof(float2) * 4 * d.Q));
+        for (int i = 0; i < 2; ++i) w.g[i] = static_cast<float *>(take(t));
+        w.delta = static_cast<float *>(take(t * d.inner));
+        w.dsum = static_cast<float *>(take(t));
+        w.dsq = static_cast<float *>(take(t / 4));
+        if (replay) w.replay = static_cast<float *>(take(t * d.inner));
+    }
+    w.bytes = off;
+    return w;
+}
+
+static int loop_check(int B, int M, int N, int K, int inner, int outer, int block, int act, int nparams)
+{
+    if (B <= 0 || M <= 0 || N <= 0 || K <= 0 || outer < 1) return GN_ERR_BAD_SHAPE;
+    if (block != 4 && block != 8) return GN_ERR_BAD_BLOCK;
+    if (inner < 1) return GN_ERR_BAD_INNER;
+    if (act < GN_ACT_RELU || act > GN_ACT_TANH) return GN_ERR_BAD_ACTIVATION;
+    if (nparams != 1 && nparams != outer) return GN_ERR_BAD_SHAPE;
+    if (!quad_applicable(M, N, K, block, inner) || (B + 3) / 4 > 65535) return GN_ERR_UNSUPPORTED;
+    return GN_OK;
+}
+
+#define TRY_(call)                     \
+    do {                               \
+        const int rc_ = (call);        \
+        if (rc_ != GN_OK) return rc_;  \
+    } while (0)
+
+static int clear_flag(int *flag, cudaStream_t st)
+{
+    const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), st);
+    if (e == cudaSuccess) return GN_OK;
+    record_cuda_error(e, "cudaMemsetAsync");
+    return GN_ERR_CUDA;
+}
+
+}  // namespace gn
+
+using namespace gn;
+
+extern "C" {
+
+GN_API int gn_loop_train_supported(int B, int M, int N, int K, int inner, int block)
+{
+    return loop_check(B, M, N, K, inner, 1, block, GN_ACT_RELU, 1) == GN_OK;
+}
+
+GN_API size_t gn_loop_tensor_bytes(int B, int M, int N, int K)
+{
+    if (B <= 0 || M <= 0 || N <= 0 || K <= 0) return 0;
+    return (size_t)((B + 3) / 4) * M * N * K * 16;
+}
+
+GN_API size_t gn_loop_forward_workspace_bytes(int B, int M, int N, int K, int inner, int outer, int block, int residual)
+{
+    if (loop_check(B, M, N, K, inner, outer, block, GN_ACT_RELU, 1) != GN_OK) return 0;
+    return carve_loop(nullptr, loop_dims(B, M, N, K, inner, outer, block, 1, residual), false, false).bytes;
+}
+
+GN_API size_t gn_loop_backward_workspace_bytes(int B, int M, int N, int K, int inner, int outer, int block, int residual, int replay)
+{
+    if (loop_check(B, M, N, K, inner, outer, block, GN_ACT_RELU, 1) != GN_OK) return 0;
+    return carve_loop(nullptr, loop_dims(B, M, N, K, inner, outer, block, 1, residual), true, replay != 0).bytes;
+}
+
+GN_API int gn_loop_forward_f32(const float *const *weights, const float *const *biases, const float *const *scales, int nparams,
+                               const float *gamma, const float *beta, const float *x, float *y, float *x_il4, float *const *outs,
+                               float *stats, float *const *stashes, int B, int M, int N, int K, int inner, int outer, int block,
+                               float ln_eps, int act, int residual, void *workspace, size_t workspace_bytes, void *stream)
+{
+    TRY_(loop_check(B, M, N, K, inner, outer, block, act, nparams));
+    if (!weights || !biases || !scales || !gamma || !beta || !x || !y || !x_il4 || !outs || !stats || !workspace) return GN_ERR_NULL_POINTER;
+    const LoopDims d = loop_dims(B, M, N, K, inner, outer, block, nparams, residual);
+    const LoopWs w = carve_loop(workspace, d, false, false);
+    if (workspace_bytes < w.bytes || reinterpret_cast<uintptr_t>(workspace) % 256) return GN_ERR_WORKSPACE;
+    cudaStream_t st = (cudaStream_t)stream;
+    float2 *const mr = reinterpret_cast<float2 *>(stats);
+    const int S = 4 * d.Q;  // statistics of one step
+    TRY_(clear_flag(w.error_flag, st));
+    TRY_(launch_quad_table(gamma, beta, w.gbt, M, N, K, block, st));
+    TRY_(launch_to_il4(x, x_il4, B, d.P, st));
+    if (residual) {
+        TRY_(launch_quad_residual_combine(x_il4, nullptr, nullptr, nullptr, nullptr, nullptr, w.partials, d.Q, d.P, st));
+        TRY_(launch_norm_finalize(w.partials, quad_combine_parts(d.P), mr, S, d.P, ln_eps, st));
+    }
+    for (int k = 0; k < outer; ++k) {
+        if (k == 0 || nparams > 1) TRY_(launch_quad_pack(weights[k], biases[k], scales[k], w.packed, M, N, K, block, false, st));
+        const float *in = k ? outs[k - 1] : x_il4;
+        QuadStep a{};
+        a.packed = w.packed; a.gbt = w.gbt;
+        a.in_il4 = in;
+        a.out_il4 = residual ? w.tmp : outs[k];
+        a.in_stats = residual ? mr + (size_t)k * S : (k ? mr + (size_t)(k - 1) * S : nullptr);
+        a.out_partials = residual ? nullptr : w.partials;
+        a.nparts = d.regions;
+        if (stashes) a.save_h = stashes[k];
+        a.error_flag = w.error_flag;
+        a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;
+        TRY_(launch_step_fwd_quad(a, act, st));
+        if (residual) {
+            TRY_(launch_quad_residual_combine(in, w.tmp, gamma, beta, mr + (size_t)k * S, outs[k], w.partials, d.Q, d.P, st));
+            if (k + 1 < outer) TRY_(launch_norm_finalize(w.partials, quad_combine_parts(d.P), mr + (size_t)(k + 1) * S, S, d.P, ln_eps, st));
+        } else {
+            TRY_(launch_norm_finalize(w.partials, d.regions, mr + (size_t)k * S, S, d.P, ln_eps, st));
+        }
+    }
+    TRY_(launch_from_il4(outs[outer - 1], residual ? nullptr : mr + (size_t)(outer - 1) * S, gamma, beta, y, B, d.P, st));
+    return launch_propagate_flag(w.error_flag, st);
+}
+
+GN_API int gn_loop_backward_f32(const float *const *weights, const float *const *biases, const float *const *scales, int nparams,
+                                const float *gamma, const float *beta, const float *x_il4, float *const *outs, const float *stats,
+                                float *const *stashes, const float *gy, float *const *gw, float *const *gb, float *const *gs,
+                                float *ggamma, float *gbeta, float *gx, int B, int M, int N, int K, int inner, int outer, int block,
+                                int act, int residual, void *workspace, size_t workspace_bytes, void *stream)
+{
+    TRY_(loop_check(B, M, N, K, inner, outer, block, act, nparams));
+    if (!weights || !biases || !scales || !gamma || !beta || !x_il4 || !outs || !stats || !gy || !gw || !gb || !gs || !ggamma || !gbeta ||
+        !gx || !workspace)
+        return GN_ERR_NULL_POINTER;
+    const LoopDims d = loop_dims(B, M, N, K, inner, outer, block, nparams, residual);
+    bool replay = false;
+    for (int k = 0; k < outer; ++k) replay |= !stashes || !stashes[k];
+    const LoopWs w = carve_loop(workspace, d, true, replay);
+    if (workspace_bytes < w.bytes || reinterpret_cast<uintptr_t>(workspace) % 256) return GN_ERR_WORKSPACE;
+    cudaStream_t st = (cudaStream_t)stream;
+    const float2 *const mr = reinterpret_cast<const float2 *>(stats);
+    const int S = 4 * d.Q;
+    TRY_(clear_flag(w.error_flag, st));
+    TRY_(launch_quad_table(gamma, beta, w.gbt, M, N, K, block, st));
+    int cur = 0;
+    TRY_(launch_to_il4(gy, w.g[0], B, d.P, st));
+    for (int k = outer - 1; k >= 0; --k) {
+        const int kp = nparams > 1 ? k : 0;
+        const bool first = k == outer - 1;  // first to be walked back
+        const float *in = k ? outs[k - 1] : x_il4;
+        const float2 *in_stats = residual ? mr + (size_t)k * S : (k ? mr + (size_t)(k - 1) * S : nullptr);
+        const bool kept = stashes && stashes[k];
+        if (first || nparams > 1) {
+            TRY_(launch_quad_pack(weights[kp], gamma, scales[kp], w.packed_t, M, N, K, block, true, st));
+            if (replay) TRY_(launch_quad_pack(weights[kp], biases[kp], scales[kp], w.packed, M, N, K, block, false, st));
+        }
+        if (!residual)
+            TRY_(launch_quad_norm_sums(outs[k], w.g[cur], nullptr, gamma, mr + (size_t)k * S, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
+        float *const h = kept ? stashes[k] : w.replay;
+        if (!kept) {
+            QuadStep a{};
+            a.packed = w.packed; a.gbt = w.gbt; a.in_il4 = in; a.in_stats = in_stats;
+            a.save_h = h;
+            a.error_flag = w.error_flag;
+            a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;
+            TRY_(launch_step_fwd_quad(a, act, st));
+        }
+        QuadReverse r{};
+        r.packed_t = w.packed_t; r.g = w.g[cur];
+        if (!residual) {
+            r.raw = outs[k]; r.stats = mr + (size_t)k * S; r.ac = w.ac;
+        }
+        r.h = h; r.delta = w.delta; r.dsum = w.dsum; r.gx = w.g[cur ^ 1]; r.dsq = w.dsq;
+        r.M = M; r.N = N; r.K = K; r.Q = d.Q; r.inner = inner; r.block = block;
+        TRY_(launch_quad_reverse(r, act, st));
+        QuadWgrad g{};
+        g.in_il4 = in; g.gbt = w.gbt; g.in_stats = in_stats;
+        g.delta = w.delta; g.h = h; g.scale = scales[kp]; g.dsq = w.dsq; g.gpk = w.gpk;
+        g.accumulate = nparams == 1 && !first;
+        g.error_flag = w.error_flag;
+        g.M = M; g.N = N; g.K = K; g.Q = d.Q; g.inner = inner; g.block = block;
+        TRY_(launch_quad_wgrad(g, act, st));
+        if (nparams > 1 || k == 0) TRY_(launch_quad_unpack_grads(w.gpk, gw[kp], gb[kp], gs[kp], M, N, K, d.Q, block, st));
+        TRY_(launch_quad_border(weights[kp], w.dsum, w.g[cur ^ 1], M, N, K, d.Q, block, st));
+        if (residual) {
+            TRY_(launch_quad_norm_sums(in, w.g[cur ^ 1], w.g[cur], gamma, in_stats, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
+            TRY_(launch_quad_norm_residual_apply(in, w.g[cur ^ 1], w.g[cur], gamma, in_stats, w.ac, w.g[cur], d.Q, d.P, st));
+        } else {
+            cur ^= 1;
+        }
+    }
+    TRY_(launch_from_il4(w.g[cur], nullptr, nullptr, nullptr, gx, B, d.P, st));
+    return launch_propagate_flag(w.error_flag, st);
+}
+
+}  // extern "C"

@@ -43,13 +43,14 @@ struct QuadParams {
     double2 *out_partials;   // [4 Q][nparts]: slot `region` of every row is written; nullptr: not wanted
     int nparts;
     float *y;                // IL4; nullptr: not wanted (replay)
-    float *save_h, *save_x;  // replay: [inner][Q][P][4], [inner-1][Q][P][4]
+    float *save_h;           // SAVE: [inner][Q][P][4]
     int *error_flag;
     int M, N, K, Q, inner;
     long long nitems;        // regions * Q
 };
 
-// SAVE (replay for the backward pass): every iteration's pre-activations, and the activations between iterations.
+// SAVE: keep every iteration's pre-activations for the backward pass (which gets the activations in between from them and
+// the step's input).
 template <int SUB, int ACT, bool FUSE_IN, bool SAVE>
 __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     step_fwd_quad(const __grid_constant__ CUtensorMap in_map, const QuadParams p)
@@ -192,16 +193,23 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
             }
 
             const unsigned win = tile + L.cell0 * 16u;  // window cell (0, 0, 0) of this lane
-            // own neurons in an IL4 tensor: (dz, dy, o) at + dz * zstr + dy * ystr + o * xstr
-            const size_t own = ((size_t)q * P + g0 + (L.h ? 3 : 0)) * 4;
+            unsigned rows[4];
+#pragma unroll
+            for (int ry = 0; ry < 4; ++ry) rows[ry] = win + (unsigned)(ry * L.ysgn * G::ROW * 16);
+            const size_t own = ((size_t)q * P + g0) * 4;  // the lane's cells in an IL4 tensor
             const long long zstr = wzs * 4, ystr = wys * 4;
-            const int xstr = L.xsgn * 4;
             for (int t = 0; t < p.inner; ++t) {
                 const bool last = t + 1 == p.inner;
-                u64 acc[4][4][2];
+                u64 acc[4][4][2], hold[2] = {0, 0};
                 float *const sh = SAVE ? p.save_h + (size_t)t * p.Q * P * 4 + own : nullptr;
-                quad_stencil<SUB, true>(win, tm, L, acc, [&](int n, int o, float scale, u64 c0, u64 c1) {
-                    if (SAVE) stg128(sh + (n >> 1) * zstr + (n & 1) * ystr + o * xstr, acc[n][o][0], acc[n][o][1]);
+                quad_stencil<G::PLANE, true>(rows, L.xsgn * 16, tm, acc, [&](int n, int o, float scale, u64 c0, u64 c1) {
+                    if (SAVE) {  // two neighbours at a time
+                        if (o & 1)
+                            stg256(sh + (n >> 1) * zstr + (n & 1) * ystr + 8 * ((o >> 1) ^ L.h), L.h ? acc[n][o][0] : hold[0],
+                                   L.h ? acc[n][o][1] : hold[1], L.h ? hold[0] : acc[n][o][0], L.h ? hold[1] : acc[n][o][1]);
+                        else
+                            hold[0] = acc[n][o][0], hold[1] = acc[n][o][1];
+                    }
                     acc[n][o][0] = act_residual2<ACT>(acc[n][o][0], scale, c0);
                     acc[n][o][1] = act_residual2<ACT>(acc[n][o][1], scale, c1);
                 });
@@ -214,24 +222,11 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                         for (int n = 0; n < 4; ++n)
                             sts128u(a + (unsigned)((n & 1) * L.ysgn * G::ROW * 16) + (n >> 1) * G::PLANE * 16u, acc[n][o][0], acc[n][o][1]);
                     }
-                    if (SAVE) {
-                        float *const sx = p.save_x + (size_t)t * p.Q * P * 4 + own;
-#pragma unroll
-                        for (int n = 0; n < 4; ++n)
-#pragma unroll
-                            for (int o = 0; o < 4; ++o) stg128(sx + (n >> 1) * zstr + (n & 1) * ystr + o * xstr, acc[n][o][0], acc[n][o][1]);
-                    }
                     __syncwarp();
                 } else {
                     if (lane == 0 && i + NBUF < cnt) issue(i + NBUF);  // the tile is dead: fetch the next one
                     __syncwarp();
-                    if (p.y) {
-#pragma unroll
-                        for (int n = 0; n < 4; ++n)
-#pragma unroll
-                            for (int o = 0; o < 4; ++o)
-                                stg128(p.y + own + (n >> 1) * zstr + (n & 1) * ystr + o * xstr, acc[n][o][0], acc[n][o][1]);
-                    }
+                    if (p.y) quad_store(p.y + own, zstr, ystr, L.h, acc);
                     if (p.out_partials) {
                         u64 s2[2] = {0, 0}, q2[2] = {0, 0};
 #pragma unroll
@@ -511,7 +506,7 @@ int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
     p.packed = a.packed;
     p.gbt = a.gbt; p.in_stats = a.in_stats;
     p.out_partials = a.out_partials; p.nparts = a.nparts;
-    p.y = a.out_il4; p.save_h = a.save_h; p.save_x = a.save_x;
+    p.y = a.out_il4; p.save_h = a.save_h;
     p.error_flag = a.error_flag ? a.error_flag : device_status_ptr();
     p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;
     p.nitems = (long long)(a.M / 8) * (a.N / 8) * (a.K / 8) * a.Q;

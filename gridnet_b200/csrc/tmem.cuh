@@ -59,6 +59,11 @@ __device__ __forceinline__ void tmem_use8(float *r)
 {
     asm volatile("" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]));
 }
+__device__ __forceinline__ void tmem_use12(float *r)
+{
+    asm volatile("" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]), "+f"(r[8]),
+                 "+f"(r[9]), "+f"(r[10]), "+f"(r[11]));
+}
 __device__ __forceinline__ void tmem_use16(float *r)
 {
     asm volatile("" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]), "+f"(r[8]),

@@ -462,6 +462,41 @@ GN_API int gn_outer_forward_flags_f32(const float *weight, const float *bias, co
                                int activation, void *workspace, size_t workspace_bytes, int flags,
                                void *stream);
 
+/* ------------------------------------------------------ the model loop with gradients
+ * The loop of gridnet/scripts/train_mnist.py:62-64 (residual = 0: h = layer_norm(step(h))) or of
+ * train_imagenet.py:81-83 (residual = 1: n = layer_norm(h), h = h + step(n) - n), float32, per-block normalisation off,
+ * as one call forward and one backward. nparams = 1: one set of step parameters for all outer steps, or nparams =
+ * outer: one per step (train_imagenet.py:54-58); weights, biases, scales are host arrays of nparams device pointers.
+ *
+ * Activations inside the loop are interleaved by four samples ("IL4": [ceil(B/4)][M][N][K][4], missing samples zero);
+ * gn_loop_tensor_bytes is the size of one such tensor. The forward call fills, for the backward call:
+ *   x_il4    the input, one tensor;
+ *   outs     host array of `outer` device pointers, one tensor each: the step outputs before normalisation (residual: the
+ *            next h). Without a backward pass two tensors may take turns.
+ *   stats    [outer][4 ceil(B/4)][2] floats: (mean, 1/sqrt(var + eps)) of outs[k] (residual: of the input of step k);
+ *   stashes  NULL, or a host array of `outer` device pointers, each NULL or `inner` tensors: the pre-activations of the
+ *            inner iterations for the backward pass, which otherwise runs them again.
+ * Workspaces: 256-byte aligned, sizes from the two functions (replay = 1: some step has no stash). gn_loop_backward_f32
+ * overwrites all gradients: gw, gb, gs are host arrays of nparams device pointers, gx is the gradient of x. Needs M, N, K
+ * multiples of 8, inner >= 1, outer >= 1 (gn_loop_train_supported). A bounded wait that gave up is reported through
+ * gn_device_status. */
+GN_API int gn_loop_train_supported(int B, int M, int N, int K, int inner, int block);
+GN_API size_t gn_loop_tensor_bytes(int B, int M, int N, int K);
+GN_API size_t gn_loop_forward_workspace_bytes(int B, int M, int N, int K, int inner, int outer, int block, int residual);
+GN_API size_t gn_loop_backward_workspace_bytes(int B, int M, int N, int K, int inner, int outer, int block, int residual,
+                                        int replay);
+GN_API int gn_loop_forward_f32(const float *const *weights, const float *const *biases, const float *const *scales,
+                        int nparams, const float *gamma, const float *beta, const float *x, float *y, float *x_il4,
+                        float *const *outs, float *stats, float *const *stashes, int B, int M, int N, int K, int inner,
+                        int outer, int block, float ln_eps, int activation, int residual, void *workspace,
+                        size_t workspace_bytes, void *stream);
+GN_API int gn_loop_backward_f32(const float *const *weights, const float *const *biases, const float *const *scales,
+                         int nparams, const float *gamma, const float *beta, const float *x_il4, float *const *outs,
+                         const float *stats, float *const *stashes, const float *gy, float *const *gw, float *const *gb,
+                         float *const *gs, float *ggamma, float *gbeta, float *gx, int B, int M, int N, int K, int inner,
+                         int outer, int block, int activation, int residual, void *workspace, size_t workspace_bytes,
+                         void *stream);
+
 #ifdef __cplusplus
 }
 #endif
