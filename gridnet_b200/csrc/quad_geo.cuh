@@ -153,19 +153,6 @@ __device__ __forceinline__ void quad_stage(unsigned stage, const float *src, lon
         cp_async16(stage + (unsigned)(((k >> 1) * 8 + yy) * 8 + (x ^ (yy >> 1))) * 16u, s + (k & 1) * 16ll * K + ((k >> 1) - Z0) * zstr);
     }
 }
-// the same for four planes z0, z0 + dz, ...
-__device__ __forceinline__ void quad_stage4(unsigned stage, const float *src, long long zstr, int K, int lane, int z0, int dz)
-{
-    const int y = lane >> 3, x = lane & 7;
-    const float *s = src + ((long long)y * K + x) * 4 + z0 * zstr;
-    const unsigned d0 = stage + (unsigned)((z0 * 8 + y) * 8 + (x ^ (y >> 1))) * 16u;
-    const unsigned d1 = stage + (unsigned)((z0 * 8 + y + 4) * 8 + (x ^ ((y + 4) >> 1))) * 16u;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        cp_async16(d0 + k * dz * 1024, s + k * dz * zstr);
-        cp_async16(d1 + k * dz * 1024, s + k * dz * zstr + 16ll * K);
-    }
-}
 // offset of a lane's own cell (n = (dz, dy), o) in such a staging area: row(n) + ((o ^ e) * 16)
 template <int SUB>
 struct QuadStage {

@@ -5,10 +5,9 @@
 //            is the 27-tap sum over the delta tile with transposed weights, read from tensor memory. The gradient of the
 //            whole-grid normalisation that follows the step is applied to g on the way in, so the normalised gradient
 //            never exists in memory.
-//   wgrad    quad_wgrad_k: dW[n][t] += x_t[n + o_t] delta_t[n]. The 432 sums per lane live in tensor memory and are
-//            read, added to and written back twelve at a time; a team's two warps work on the same item, each on one half
-//            of the window rows. Sums go to the slot of (region, team) and are added up in team order by
-//            quad_unpack_grads_k: no atomics, the same bits every time.
+//   wgrad    quad_wgrad_k: dW[n][t] += x_t[n + o_t] delta_t[n], accumulated in registers over quads and iterations. Chunks of
+//            the batch leave their sums in parts of their own, which quad_unpack_grads_k adds up in chunk order: no
+//            atomics, the same bits every time.
 //   border   quad_border_k: the part of grad_x that crosses block borders, from the per-neuron sums of deltas.
 //   norms    quad_norm_sums_k: one pass over the step's output and the gradient of its normalised form gives the
 //            per-sample sums of the LayerNorm gradient and the gradients of its weight and bias.
@@ -126,13 +125,6 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
         for (int k = 0; k < 16; ++k)
             cp_async16(tile + (unsigned)(((k >> 1) + 1) * PLANE + (y + 4 * (k & 1)) * ROW + x + 1) * 16u, src + (k & 1) * 16ll * p.K + (k >> 1) * zstr);
     };
-    auto prefetch_rows = [&](const float *t, size_t corner) {  // a region's 64 rows of 128 bytes on their way to L2
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const int r = lane + 32 * k;
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(t + corner + (r >> 3) * zstr + (long long)(r & 7) * p.K * 4));
-        }
-    };
     const size_t to_own = (((size_t)L.z0 * p.N + L.y0) * p.K + 4 * L.h) * 4;  // corner -> this lane's cells
     __syncwarp();
     if (role < cnt) {
@@ -163,44 +155,43 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
             const size_t corner = corner_of(i), own = corner + to_own;
             u64 g[4][4][2], dsum[4][4][2];
             float dsa[4][4];
-            u64 r[4][4][2];
-            if (NORM_IN) quad_load(p.raw + own, zstr, ystr, L.h, r);
-            if (i + TEAM < cnt) {
-                const size_t next = corner_of(i + TEAM);
-                prefetch_rows(p.g, next);
-                if (NORM_IN) prefetch_rows(p.raw, next);
-            }
-            cp_async_wait_all();
-            __syncwarp();
-#pragma unroll
-            for (int n = 0; n < 4; ++n)
-#pragma unroll
-                for (int o = 0; o < 4; ++o) lds128u(own_cell(n, o), g[n][o][0], g[n][o][1]);
-            if (NORM_IN) {
-                // gradient of (x - mean) rstd gamma + beta: rstd (g gamma - a - xhat c)
-                u64 mu[2], rs[2], ma[2], mc[2];
-#pragma unroll
-                for (int k2 = 0; k2 < 2; ++k2) {
-                    const float2 m0 = p.stats[4 * q + 2 * k2], m1 = p.stats[4 * q + 2 * k2 + 1];
-                    const float2 a0 = p.ac[4 * q + 2 * k2], a1 = p.ac[4 * q + 2 * k2 + 1];
-                    mu[k2] = pack2(-m0.x, -m1.x);
-                    rs[k2] = pack2(m0.y, m1.y);
-                    ma[k2] = pack2(-a0.x, -a1.x);
-                    mc[k2] = pack2(-a0.y, -a1.y);
-                }
+            {
+                // everything the item starts with is asked for at once
+                u64 r[4][4][2];
+                float2 m4[4], a4[4];
                 float gm[16];
-                tmem_ld16(tm + COL_BIAS, gm);
-                tmem_wait_ld16(gm);
+                if (NORM_IN) {
+                    quad_load(p.raw + own, zstr, ystr, L.h, r);
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        m4[s] = __ldg(p.stats + 4 * q + s);
+                        a4[s] = __ldg(p.ac + 4 * q + s);
+                    }
+                    tmem_ld16(tm + COL_BIAS, gm);
+                }
+                cp_async_wait_all();
+                if (NORM_IN) tmem_wait_ld16(gm);
+                __syncwarp();
 #pragma unroll
                 for (int n = 0; n < 4; ++n)
 #pragma unroll
-                    for (int o = 0; o < 4; ++o)
+                    for (int o = 0; o < 4; ++o) lds128u(own_cell(n, o), g[n][o][0], g[n][o][1]);
+                if (NORM_IN) {
+                    // gradient of (x - mean) rstd gamma + beta: rstd (g gamma - a - xhat c)
 #pragma unroll
-                        for (int k2 = 0; k2 < 2; ++k2) {
-                            const u64 xh = fmul2(fadd2(r[n][o][k2], mu[k2]), rs[k2]);
-                            const u64 gg = ffma2r(g[n][o][k2], pack2(gm[n * 4 + o], gm[n * 4 + o]), ma[k2]);
-                            g[n][o][k2] = fmul2(ffma2r(xh, mc[k2], gg), rs[k2]);
-                        }
+                    for (int k2 = 0; k2 < 2; ++k2) {
+                        const float2 m0 = m4[2 * k2], m1 = m4[2 * k2 + 1], a0 = a4[2 * k2], a1 = a4[2 * k2 + 1];
+                        const u64 mu = pack2(-m0.x, -m1.x), rs = pack2(m0.y, m1.y), ma = pack2(-a0.x, -a1.x), mc = pack2(-a0.y, -a1.y);
+#pragma unroll
+                        for (int n = 0; n < 4; ++n)
+#pragma unroll
+                            for (int o = 0; o < 4; ++o) {
+                                const u64 xh = fmul2(fadd2(r[n][o][k2], mu), rs);
+                                const u64 gg = ffma2r(g[n][o][k2], pack2(gm[n * 4 + o], gm[n * 4 + o]), ma);
+                                g[n][o][k2] = fmul2(ffma2r(xh, mc, gg), rs);
+                            }
+                    }
+                }
             }
 #pragma unroll
             for (int n = 0; n < 4; ++n)
@@ -215,28 +206,33 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
                 cp_async_wait_all();
                 tmem_wait_ld16(sc);
                 __syncwarp();  // everyone's part of h_t has landed
+                // Row by row: loads, arithmetic and stores of a row of four cells each overlap with themselves (cell by cell,
+                // a load waits for the store before it); more rows at a time spill (0.64 ms by one row, 0.67 by two, 0.71 by
+                // four, at 128^3 with two inner iterations and batch 32).
                 float *const dt = p.delta + (size_t)t * T4 + own;
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
-                    u64 dl[4][2];
+                    u64 h[4][2];
+#pragma unroll
+                    for (int o = 0; o < 4; ++o) lds128u(stage + S.at(n, o), h[o][0], h[o][1]);
 #pragma unroll
                     for (int o = 0; o < 4; ++o) {
-                        u64 h0, h1, f0, f1, d0, d1;
-                        lds128u(stage + S.at(n, o), h0, h1);
-                        act_both2<ACT>(h0, f0, d0);
-                        act_both2<ACT>(h1, f1, d1);
+                        u64 f0, f1, d0, d1;
+                        act_both2<ACT>(h[o][0], f0, d0);
+                        act_both2<ACT>(h[o][1], f1, d1);
                         float s0, s1;
                         unpack2(ffma2r(f0, g[n][o][0], fmul2(f1, g[n][o][1])), s0, s1);
                         dsa[n][o] += s0 + s1;
                         const u64 s2 = pack2(sc[n * 4 + o], sc[n * 4 + o]);
-                        dl[o][0] = fmul2(fmul2(d0, g[n][o][0]), s2);
-                        dl[o][1] = fmul2(fmul2(d1, g[n][o][1]), s2);
-                        dsum[n][o][0] = fadd2(dsum[n][o][0], dl[o][0]);
-                        dsum[n][o][1] = fadd2(dsum[n][o][1], dl[o][1]);
-                        sts128u(own_cell(n, o), dl[o][0], dl[o][1]);
+                        h[o][0] = fmul2(fmul2(d0, g[n][o][0]), s2);
+                        h[o][1] = fmul2(fmul2(d1, g[n][o][1]), s2);
+                        dsum[n][o][0] = fadd2(dsum[n][o][0], h[o][0]);
+                        dsum[n][o][1] = fadd2(dsum[n][o][1], h[o][1]);
                     }
-                    quad_store2(dt, n, 0, zstr, ystr, L.h, dl);
-                    quad_store2(dt, n, 1, zstr, ystr, L.h, dl);
+#pragma unroll
+                    for (int o = 0; o < 4; ++o) sts128u(own_cell(n, o), h[o][0], h[o][1]);
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) quad_store2(dt, n, j, zstr, ystr, L.h, h);
                 }
                 __syncwarp();  // the delta tile is complete, h_t has been read
                 if (t > 0) fetch_h(corner, t - 1);
@@ -264,16 +260,45 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
 }
 
 // ---------------------------------------------------------------------------------------- weight gradients
-// What a team has in shared memory: tiles of the step's input with its halo (block 8: two, which take turns over the
-// inner iterations so that one barrier per iteration is enough; block 4: one, updated in place between two), two staging
-// areas for deltas and one for pre-activations.
+// One CTA of 128 threads per region and chunk of quads. A thread owns a 2 x 2 x 1 (z, y, x) patch and keeps its 4 x 27 sums
+// in registers from the first quad to the last; a quarter-warp reads whole rows of cells, so every shared-memory access is
+// free of bank conflicts. Per iteration and quad 48 cells serve 4 x 27 x 4 FMAs: 2.25 per wavefront, half of what the
+// 2 x 2 x 4 patches of the other kernels get, but those would need their 432 sums in tensor memory, and reading, adding to
+// and writing back sums there was 3 to 4 times slower than this (128^3, two inner iterations, batch 32: 0.77 - 0.97 ms).
+// The step's input tile arrives by bulk tensor copy and is normalised in place; activations between iterations are rebuilt
+// from it and the pre-activations. Block 8: two tiles take turns over the iterations, one barrier each; block 4: one tile,
+// updated in place between two barriers. Deltas and pre-activations arrive an iteration ahead, each thread its own.
 namespace quadwg {
-constexpr int TEAM = 2, STAGE_BYTES = 512 * 16;
+constexpr int CTAS = 2;  // per SM: 255 registers (three with 168 spill, and are no faster)
+constexpr int THREADS = 128, OWN = 4 * THREADS * 16;  // bytes of one staging area: a thread's four cells
+constexpr int GRAD_F = (27 * 4 + 8) * THREADS;        // floats per region and chunk: weights, biases, scales
 template <int SUB>
 struct Lay {
     static constexpr int NT = SUB == 8 ? 2 : 1;
-    static constexpr int TEAM_BYTES = NT * QuadGeo<SUB>::BUF_BYTES + 3 * STAGE_BYTES;
-    static constexpr int SMEM = 4 * TEAM_BYTES;
+    static constexpr int TILE = (QuadGeo<SUB>::BUF_BYTES + 127) / 128 * 128;
+    static constexpr int GB = NT * TILE + 3 * OWN;  // normalise-on-load: the region's (gamma, beta) table
+    static constexpr int smem(bool fuse) { return GB + (fuse ? QuadGeo<SUB>::CELLS * 8 : 0); }
+};
+// thread -> patch. Block 8: lanes of a quarter-warp are the eight x; block 4: four x and two y patches (two rows of six
+// cells further is four banks further)
+template <int SUB>
+struct Patch {
+    int x, yp, zp, cell0;
+    __device__ __forceinline__ explicit Patch(int tid)
+    {
+        using G = QuadGeo<SUB>;
+        const int l = tid & 31;
+        zp = tid >> 5;
+        if (SUB == 8) {
+            x = l & 7;
+            yp = l >> 3;
+            cell0 = 2 * zp * G::PLANE + 2 * yp * G::ROW + x;
+        } else {
+            x = (l & 3) | ((l >> 3) & 1) << 2;
+            yp = ((l >> 2) & 1) | (l >> 4) << 1;
+            cell0 = (((zp >> 1) * 2 + (yp >> 1)) * 2 + (x >> 2)) * 216 + 2 * (zp & 1) * G::PLANE + 2 * (yp & 1) * G::ROW + (x & 3);
+        }
+    }
 };
 }  // namespace quadwg
 
@@ -283,190 +308,42 @@ struct QuadWgradParams {
     const float *delta, *h;  // [inner] IL4
     const float *scale;      // [M][N][K]
     const float *dsq;        // [Q][P]
-    float *gpk;              // [slots][regions][PACK_F]
-    int accumulate;          // add to what the slots hold
+    float *gpk;              // [chunks][regions][GRAD_F]
+    int accumulate;          // add to what is there
     int *error_flag;
-    int M, N, K, Q, inner, regions;
-    long long nitems;
+    int M, N, K, Q, inner, qpc;
 };
 
-// first team that works on an item >= n, when nitems items are cut into nteams contiguous ranges
-__host__ __device__ __forceinline__ long long quad_team_of(long long n, long long nitems, long long nteams)
-{
-    return ((n + 1) * nteams - 1) / nitems;
-}
-
-// The sums of a warp: half of the window rows. In the two inner row pairs (ry = 1, 2) a window row is read by both neuron
-// rows dy = 0, 1: their sums are neighbours in tensor memory ("pair units", 24 columns: [c][o][dy]) and take packed FMAs
-// with the cell's value as the scalar operand. The outer rows (ry = 0, 3) serve one neuron row ("single units", 12
-// columns: [c][o]). Half 0: six single units, then six pair units; half 1 the other way round.
-template <int COLS>
-__device__ __forceinline__ void quad_ld_cols(unsigned a, float *r)
-{
-    if (COLS == 24) {
-        tmem_ld16(a, r);
-        tmem_ld8(a + 16, r + 16);
-    } else {
-        tmem_ld8(a, r);
-        tmem_ld4(a + 8, r + 8);
-    }
-}
-
-// One iteration: every sum += window cell * delta, four samples. dp[dz][o][s]: deltas of (dy = 0, dy = 1).
-// Bound by FMA issue: 288 packed and 288 scalar FMAs per warp. Three register buffers per unit in flight: a unit's sums
-// are asked for while the one before is worked on and are still being written back while the next one is.
-template <int PLANE, int HALF>
-__device__ __forceinline__ void quad_wgrad_rows(const unsigned (&rows)[4], int dx, unsigned tm, const u64 (&dp)[2][4][4])
-{
-    const unsigned t0 = tm + HALF * 216;
-    float wb[2][24];
-    tmem_wait_st();  // the previous iteration's sums are in place
-    if (HALF == 0) quad_ld_cols<12>(t0, wb[0]);
-    else quad_ld_cols<24>(t0, wb[0]);
-    int unit = 0, col = 0;
-#pragma unroll
-    for (int ry = 2 * HALF; ry < 2 * HALF + 2; ++ry) {
-        const bool pair = ry == 1 || ry == 2;
-        unsigned a6[6];
-#pragma unroll
-        for (int j = 0; j < 6; ++j) a6[j] = rows[ry] + (unsigned)(j * dx);
-#pragma unroll
-        for (int rz = 0; rz < 4; ++rz) {
-            float4 v[6];
-#pragma unroll
-            for (int j = 0; j < 6; ++j) v[j] = lds128(a6[j] + rz * PLANE * 16u);
-#pragma unroll
-            for (int dz = 0; dz < 2; ++dz) {
-                if (rz - dz < 0 || rz - dz > 2) continue;
-                float *wp = wb[unit % 2], *wn = wb[(unit + 1) % 2];
-                const int cols = pair ? 24 : 12, next = col + cols;
-                tmem_wait_ld12(wp);
-                if (pair) tmem_use12(wp + 12);
-                if (unit + 1 < 12) {
-                    const bool next_pair = HALF == 0 ? unit + 1 >= 6 : unit + 1 < 6;
-                    if (next_pair) quad_ld_cols<24>(t0 + next, wn);
-                    else quad_ld_cols<12>(t0 + next, wn);
-                }
-                if (pair) {
-                    u64 acc[12];
-#pragma unroll
-                    for (int k = 0; k < 12; ++k) acc[k] = pack2(wp[2 * k], wp[2 * k + 1]);
-#pragma unroll
-                    for (int s = 0; s < 4; ++s)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c)
-#pragma unroll
-                            for (int o = 0; o < 4; ++o) {
-                                const float4 &vv = v[o + c];
-                                const float x = s == 0 ? vv.x : (s == 1 ? vv.y : (s == 2 ? vv.z : vv.w));
-                                ffma2(acc[c * 4 + o], dp[dz][o][s], pack2(x, x));
-                            }
-#pragma unroll
-                    for (int k = 0; k < 12; ++k) unpack2(acc[k], wp[2 * k], wp[2 * k + 1]);
-                    tmem_st16(t0 + col, wp);
-                    tmem_st8(t0 + col + 16, wp + 16);
-                } else {
-#pragma unroll
-                    for (int s = 0; s < 4; ++s)
-#pragma unroll
-                        for (int c = 0; c < 3; ++c)
-#pragma unroll
-                            for (int o = 0; o < 4; ++o) {
-                                const float4 &vv = v[o + c];
-                                const float x = s == 0 ? vv.x : (s == 1 ? vv.y : (s == 2 ? vv.z : vv.w));
-                                float lo, hi;
-                                unpack2(dp[dz][o][s], lo, hi);
-                                wp[c * 4 + o] = fmaf(x, HALF == 0 ? lo : hi, wp[c * 4 + o]);
-                            }
-                    tmem_st8(t0 + col, wp);
-                    tmem_st4(t0 + col + 8, wp + 8);
-                }
-                ++unit;
-                col = next;
-            }
-        }
-    }
-}
-
-// 72 of a warp's 216 sums (six single units, or three pair units) -> (or onto) 18 vectors of the packed gradient
-template <bool PAIR>
-__device__ __forceinline__ void quad_flush72(float4 *o, unsigned col, bool accumulate)
-{
-    float r[72];
-    float4 old[18];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) quad_ld_cols<24>(col + k * 24, r + k * 24);
-#pragma unroll
-    for (int v = 0; v < 18; ++v) old[v] = accumulate ? o[v * 32] : make_float4(0.f, 0.f, 0.f, 0.f);
-    tmem_wait_ld12(r);
-#pragma unroll
-    for (int k = 1; k < 6; ++k) tmem_use12(r + 12 * k);
-#pragma unroll
-    for (int v = 0; v < 18; ++v) {
-        // pair unit j: vectors 6 j + 3 dy + c, columns 24 j + (4 c + o) 2 + dy
-        const int j = v / 6, dy = v % 6 / 3, c = v % 3;
-        float e[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) e[i] = PAIR ? r[24 * j + (4 * c + i) * 2 + dy] : r[4 * v + i];
-        o[v * 32] = make_float4(e[0] + old[v].x, e[1] + old[v].y, e[2] + old[v].z, e[3] + old[v].w);
-    }
-}
-
 template <int SUB, int ACT, bool FUSE_IN>
-__global__ void __launch_bounds__(256, 1) quad_wgrad_k(const __grid_constant__ CUtensorMap in_map, const QuadWgradParams p)
+__global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(const __grid_constant__ CUtensorMap in_map, const QuadWgradParams p)
 {
-    using namespace quad;
+    using namespace quadwg;
     using G = QuadGeo<SUB>;
-    using Y = quadwg::Lay<SUB>;
-    constexpr int TEAM = quadwg::TEAM, NT = Y::NT, SB = quadwg::STAGE_BYTES;
+    using Y = Lay<SUB>;
+    constexpr int NT = Y::NT;
+    constexpr unsigned kSpin = quad::kSpinLimit;
     extern __shared__ __align__(1024) unsigned char smem[];
-    __shared__ __align__(8) unsigned long long bars[QUARTERS * NT];
-    __shared__ unsigned tmem_slot;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int quarter = warp & 3, role = warp >> 2;
-    if (warp == 0) tmem_alloc_all(&tmem_slot);
+    __shared__ __align__(8) unsigned long long bars[NT];
+    const int tid = threadIdx.x;
     if (tid == 0) {
-        for (int i = 0; i < QUARTERS * NT; ++i) mbar_init(smem_u32(&bars[i]), 1);
+        for (int i = 0; i < NT; ++i) mbar_init(smem_u32(&bars[i]), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();
     }
-    tmem_fence_before();
     __syncthreads();
-    tmem_fence_after();
-    const unsigned tm = tmem_slot + ((unsigned)(quarter * 32) << 16);
-
-    const QuadLane<SUB> L(lane);
-    const QuadStage<SUB> S(L);
-    const int nbx = p.K >> 3, nby = p.N >> 3;
+    const Patch<SUB> T(tid);
+    const int nbx = p.K >> 3, nby = p.N >> 3, blk = blockIdx.x;
+    const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t P = (size_t)p.M * p.N * p.K, T4 = (size_t)p.Q * P * 4;
-    const long long nteams = (long long)gridDim.x * QUARTERS, team = (long long)blockIdx.x * QUARTERS + quarter;
-    const long long n0 = p.nitems * team / nteams;
-    const int cnt = (int)(p.nitems * (team + 1) / nteams - n0);
-    const unsigned tiles = smem_u32(smem) + quarter * Y::TEAM_BYTES;
-    const unsigned stage_d = tiles + NT * G::BUF_BYTES, stage_h = stage_d + 2 * SB;
-    const unsigned bar0 = smem_u32(&bars[quarter * NT]);
-    const long long wzs = (long long)p.N * p.K, wys = (long long)L.ysgn * p.K, zstr = wzs * 4;
-    const int dx = L.xsgn * 16;
-    const unsigned own0 = (unsigned)(L.cell0 * 16 + dx + L.ysgn * G::ROW * 16) + G::PLANE * 16u;  // own cell (0, 0, 0) in a tile
+    const unsigned tiles = smem_u32(smem), stage_d = tiles + NT * Y::TILE + tid * 16, stage_h = stage_d + 2 * OWN;
+    const unsigned bar0 = smem_u32(bars);
+    const size_t g0 = ((size_t)(bz * 8 + 2 * T.zp) * p.N + (by * 8 + 2 * T.yp)) * p.K + bx * 8 + T.x;
+    const size_t zs = (size_t)p.N * p.K;
+    const int q0 = blockIdx.y * p.qpc, q1 = min(p.Q, q0 + p.qpc);
     bool failed = false;
 
-    // normalise pass: this thread's cells are first, first + 64, ...; which of them are halo (kept in both tiles)
-    const int first = role * 32 + lane;
-    constexpr int STEPS = (G::CELLS + 63) / 64;
-    unsigned halo = 0;
-    if (NT == 2) {
-        for (int c = 0; c < STEPS; ++c) {
-            int cz, cy, cx;
-            G::cell(first + 64 * c, cz, cy, cx);
-            if (cz == 0 || cz == 9 || cy == 0 || cy == 9 || cx == 0 || cx == 9) halo |= 1u << c;
-        }
-    }
-
-    auto issue = [&](int i, int buf) {  // one lane: tile of item i
-        const long long n = n0 + i;
-        const int blk = (int)(n / p.Q), q = (int)(n - (long long)blk * p.Q);
-        const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
-        const unsigned tile = tiles + buf * G::BUF_BYTES, bar = bar0 + 8 * buf;
+    auto issue = [&](int q, int buf) {
+        const unsigned tile = tiles + buf * Y::TILE, bar = bar0 + 8 * buf;
         fence_proxy_async();
         mbar_expect_tx(bar, G::CELLS * 16);
         if (SUB == 8) {
@@ -477,278 +354,225 @@ __global__ void __launch_bounds__(256, 1) quad_wgrad_k(const __grid_constant__ C
                             bz * 8 + (sub >> 2) * 4 - 1, q);
         }
     };
-    auto corner_of = [&](int i) {
-        const long long n = n0 + i;
-        const int blk = (int)(n / p.Q), q = (int)(n - (long long)blk * p.Q);
-        const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
-        return ((size_t)q * P + ((size_t)(bz * 8) * p.N + by * 8) * p.K + bx * 8) * 4;
+    auto fetch = [&](unsigned dst, const float *src) {  // this thread's four cells
+#pragma unroll
+        for (int n = 0; n < 4; ++n) cp_async16(dst + n * (THREADS * 16), src + ((n >> 1) * zs + (n & 1) * (size_t)p.K) * 4);
     };
-    // Deltas of iteration t -> staging area `buf`: each warp brings half of the planes, the team barrier shares them.
-    // Pre-activations h_t: each warp the planes whose neurons it updates (dz = role), for itself alone.
-    auto fetch_d = [&](size_t corner, int t, int buf) {
-        quad_stage4(stage_d + buf * SB, p.delta + (size_t)t * T4 + corner, zstr, p.K, lane, role * 4, 1);
-    };
-    auto fetch_h = [&](size_t corner, int t) {
-        quad_stage4(stage_h, p.h + (size_t)t * T4 + corner, zstr, p.K, lane, role, 2);
-    };
-    int buf_x = 0, buf_d = 0;     // tile and delta area of the iteration at hand
-    unsigned landed[NT] = {};     // phases of the tile barriers
-    if (cnt > 0) {
-        if (role == 0 && lane == 0) issue(0, 0);
-        __syncwarp();
-        fetch_d(corner_of(0), 0, 0);
-        if (p.inner > 1) fetch_h(corner_of(0), 0);
+    auto at = [&](const float *t, int q, int it) { return t + (size_t)it * T4 + ((size_t)q * P + g0) * 4; };
+
+    // sums: sg[dy = 0 at ry = 0, dy = 1 at ry = 3][dz][a][c], sp[ry = 1, 2][dz][a][c] = (dy = 0, dy = 1)
+    float sg[2][2][3][3];
+    u64 sp[2][2][3][3];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int a = 0; a < 3; ++a)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    sg[i][j][a][c] = 0.0f;
+                    sp[i][j][a][c] = 0;
+                }
+    u64 db[2] = {0, 0}, ds[2] = {0, 0};  // [dz]: (dy = 0, dy = 1)
+
+    int buf_x = 0, buf_d = 0;
+    unsigned landed = 0;  // bit b: phase of tile b's barrier
+    const float2 *const gbs = reinterpret_cast<const float2 *>(smem + Y::GB);
+    if (FUSE_IN) {
+        const unsigned char *src = reinterpret_cast<const unsigned char *>(p.gbt + (size_t)blk * G::CELLS);
+        for (int c = tid; c < G::CELLS / 2; c += THREADS) cp_async16(tiles + Y::GB + c * 16, src + c * 16);
+        cp_async_wait_all();
+        __syncthreads();
     }
+    if (tid == 0) issue(q0, 0);
+    fetch(stage_d, at(p.delta, q0, 0));
+    if (p.inner > 1) fetch(stage_h, at(p.h, q0, 0));
+    const unsigned own0 = (unsigned)(T.cell0 + G::PLANE + G::ROW + 1) * 16u;
 
-    int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
-    for (int i0 = 0; i0 < cnt;) {
-        const int here = min(cnt - i0, p.Q - q0);
-        const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
-        const size_t g0 = ((size_t)(bz * 8 + L.z0) * p.N + (by * 8 + L.y0)) * p.K + bx * 8 + (L.h ? 7 : 0);
-        {
-            float z[16];
+    for (int q = q0; q < q1; ++q) {
+        {  // scale terms of this quad
+            const float *s = p.dsq + (size_t)q * P + g0;
 #pragma unroll
-            for (int k = 0; k < 16; ++k) z[k] = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 13; ++k) tmem_st16(tm + role * 216 + k * 16, z);
-            tmem_st8(tm + role * 216 + 208, z);
+            for (int dz = 0; dz < 2; ++dz) ds[dz] = fadd2(ds[dz], pack2(__ldg(s + dz * zs), __ldg(s + dz * zs + p.K)));
         }
-        float dacc[4][4];  // role 0: bias gradient, role 1: gradient of the residual scale
-        float sc[2][4];    // scales of the neurons this warp updates between iterations
+        if (!mbar_wait_bounded(bar0 + 8 * buf_x, (landed >> buf_x) & 1u, kSpin)) failed = true;
+        landed ^= 1u << buf_x;
+        const bool two = NT == 2 && p.inner > 1;
+        if (two) __syncthreads();  // nobody reads the other tile any more: it gets the new halo
+        if (FUSE_IN || two) {
+            const unsigned tile = tiles + buf_x * Y::TILE, other = tiles + (buf_x ^ 1) * Y::TILE;
+            u64 na[2], nb[2];
+            if (FUSE_IN) {
+                float2 mr[4];
 #pragma unroll
-        for (int n = 0; n < 4; ++n)
+                for (int s = 0; s < 4; ++s) mr[s] = __ldg(p.in_stats + 4 * q + s);
+                na[0] = pack2(mr[0].y, mr[1].y);
+                na[1] = pack2(mr[2].y, mr[3].y);
+                nb[0] = pack2(-mr[0].x * mr[0].y, -mr[1].x * mr[1].y);
+                nb[1] = pack2(-mr[2].x * mr[2].y, -mr[3].x * mr[3].y);
+            }
+            constexpr int STEPS = (G::CELLS + THREADS - 1) / THREADS, BATCH = SUB == 8 ? 8 : 7;
+#pragma unroll 1
+            for (int c0 = 0; c0 < STEPS; c0 += BATCH) {
+                u64 v[BATCH][2];
+                float2 g2[BATCH];
 #pragma unroll
-            for (int o = 0; o < 4; ++o) dacc[n][o] = 0.0f;
-        if (p.inner > 1) {
+                for (int c = 0; c < BATCH; ++c) {
+                    const int i = (c0 + c) * THREADS + tid;
+                    if (i < G::CELLS) {
+                        if (FUSE_IN) g2[c] = gbs[i];
+                        lds128u(tile + i * 16, v[c][0], v[c][1]);
+                    }
+                }
 #pragma unroll
-            for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-                for (int o = 0; o < 4; ++o) sc[dy][o] = __ldg(p.scale + g0 + role * wzs + dy * wys + o * L.xsgn);
+                for (int c = 0; c < BATCH; ++c) {
+                    const int i = (c0 + c) * THREADS + tid;
+                    if (i < G::CELLS) {
+                        if (FUSE_IN) {
+                            const u64 gg = pack2(g2[c].x, g2[c].x), bb = pack2(g2[c].y, g2[c].y);
+                            v[c][0] = ffma2r(ffma2r(v[c][0], na[0], nb[0]), gg, bb);
+                            v[c][1] = ffma2r(ffma2r(v[c][1], na[1], nb[1]), gg, bb);
+                            sts128u(tile + i * 16, v[c][0], v[c][1]);
+                        }
+                        if (two) {
+                            int cz, cy, cx;
+                            G::cell(i, cz, cy, cx);
+                            if (cz == 0 || cz == 9 || cy == 0 || cy == 9 || cx == 0 || cx == 9) sts128u(other + i * 16, v[c][0], v[c][1]);
+                        }
+                    }
+                }
+            }
         }
-
-        for (int k = 0; k < here; ++k) {
-            const int i = i0 + k, q = q0 + k;
-            const size_t corner = corner_of(i);
-            if (role == 1) {
-                const float *dq = p.dsq + corner / 4 + ((size_t)L.z0 * p.N + L.y0) * p.K + 4 * L.h;
+        for (int t = 0; t < p.inner; ++t) {
+            const bool last = t + 1 == p.inner;
+            const unsigned tile = tiles + buf_x * Y::TILE;
+            cp_async_wait_all();
+            __syncthreads();  // the tile is complete; nobody is an iteration behind
+            u64 dp[2][4];     // deltas [dz][sample]: (dy = 0, dy = 1)
+#pragma unroll
+            for (int dz = 0; dz < 2; ++dz) {
+                const float4 a = lds128(stage_d + buf_d * OWN + (2 * dz) * (THREADS * 16)), b = lds128(stage_d + buf_d * OWN + (2 * dz + 1) * (THREADS * 16));
+                dp[dz][0] = pack2(a.x, b.x);
+                dp[dz][1] = pack2(a.y, b.y);
+                dp[dz][2] = pack2(a.z, b.z);
+                dp[dz][3] = pack2(a.w, b.w);
+            }
+            // block 8: the activations of iteration t + 1 -> the other tile; block 4: those of iteration t, in place
+            if (NT == 2 ? !last : t > 0) {
+                const unsigned to = NT == 2 ? tiles + (buf_x ^ 1) * Y::TILE : tile;
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
-                    const float4 v = *reinterpret_cast<const float4 *>(dq + (n >> 1) * wzs + (n & 1) * wys);
-                    dacc[n][0] += L.h ? v.w : v.x;
-                    dacc[n][1] += L.h ? v.z : v.y;
-                    dacc[n][2] += L.h ? v.y : v.z;
-                    dacc[n][3] += L.h ? v.x : v.w;
+                    const unsigned c = own0 + (unsigned)((n >> 1) * G::PLANE + (n & 1) * G::ROW) * 16u;
+                    const float sc = __ldg(p.scale + g0 + (n >> 1) * zs + (n & 1) * (size_t)p.K);
+                    u64 h0, h1, x0, x1;
+                    lds128u(stage_h + n * (THREADS * 16), h0, h1);
+                    lds128u(tile + c, x0, x1);
+                    sts128u(to + c, act_residual2<ACT>(h0, sc, x0), act_residual2<ACT>(h1, sc, x1));
                 }
             }
-            {
-                const unsigned tile = tiles + buf_x * G::BUF_BYTES, other = tiles + (buf_x ^ 1) * G::BUF_BYTES;
-                constexpr int BATCH = SUB == 8 ? 16 : 14;
-                float2 g2[FUSE_IN ? BATCH : 1];
-                const float2 *gp = FUSE_IN ? p.gbt + (size_t)blk * G::CELLS + first : nullptr;
-                u64 na[2], nb[2];
-                if (FUSE_IN) {  // (gamma, beta) of the first batch: in flight while the tile is waited for
-#pragma unroll
-                    for (int c = 0; c < BATCH; ++c)
-                        if (c * 64 + first < G::CELLS) g2[c] = ld_pinned2(reinterpret_cast<const float *>(gp + c * 64));
-                    float2 mr[4];
-#pragma unroll
-                    for (int s = 0; s < 4; ++s) mr[s] = p.in_stats[4 * q + s];
-                    na[0] = pack2(mr[0].y, mr[1].y);
-                    na[1] = pack2(mr[2].y, mr[3].y);
-                    nb[0] = pack2(-mr[0].x * mr[0].y, -mr[1].x * mr[1].y);
-                    nb[1] = pack2(-mr[2].x * mr[2].y, -mr[3].x * mr[3].y);
-                }
-                if (!mbar_wait_bounded(bar0 + 8 * buf_x, landed[buf_x] & 1u, kSpinLimit)) failed = true;
-                if (NT == 1 || buf_x == 0) ++landed[0];
-                else ++landed[NT - 1];
-                __syncwarp();
-                if (NT == 2 && p.inner > 1) team_sync<TEAM>(quarter);  // nobody reads the other tile any more: it gets the new halo
-                if (FUSE_IN || (NT == 2 && p.inner > 1)) {
-#pragma unroll 1
-                    for (int c0 = 0; c0 < STEPS; c0 += BATCH) {
-                        const unsigned a = (unsigned)(c0 * 64 + first) * 16u;
-                        u64 v[BATCH][2];
-#pragma unroll
-                        for (int c = 0; c < BATCH; ++c)
-                            if ((c0 + c) * 64 + first < G::CELLS) {
-                                if (FUSE_IN && c0 > 0) g2[c] = ld_pinned2(reinterpret_cast<const float *>(gp + (c0 + c) * 64));
-                                lds128u(tile + a + c * 1024, v[c][0], v[c][1]);
-                            }
-#pragma unroll
-                        for (int c = 0; c < BATCH; ++c)
-                            if ((c0 + c) * 64 + first < G::CELLS) {
-                                if (FUSE_IN) {
-                                    const u64 gg = pack2(g2[c].x, g2[c].x), bb = pack2(g2[c].y, g2[c].y);
-                                    v[c][0] = ffma2r(ffma2r(v[c][0], na[0], nb[0]), gg, bb);
-                                    v[c][1] = ffma2r(ffma2r(v[c][1], na[1], nb[1]), gg, bb);
-                                    sts128u(tile + a + c * 1024, v[c][0], v[c][1]);
-                                }
-                                if (NT == 2 && p.inner > 1 && (halo >> (c0 + c) & 1u)) sts128u(other + a + c * 1024, v[c][0], v[c][1]);
-                            }
-                    }
-                }
+            if (NT == 1 && t > 0) __syncthreads();  // the tile is complete
+            // the next iteration's data
+            if (!last) {
+                fetch(stage_d + (buf_d ^ 1) * OWN, at(p.delta, q, t + 1));
+                if (NT == 1 || t + 2 < p.inner) fetch(stage_h, at(p.h, q, NT == 2 ? t + 1 : t));
+            } else if (q + 1 < q1) {
+                fetch(stage_d + (buf_d ^ 1) * OWN, at(p.delta, q + 1, 0));
+                if (NT == 2 && p.inner > 1) fetch(stage_h, at(p.h, q + 1, 0));
+                if (NT == 2 && tid == 0) issue(q + 1, buf_x ^ 1);
             }
-            for (int t = 0; t < p.inner; ++t) {
-                const bool last = t + 1 == p.inner;
-                const unsigned tile = tiles + buf_x * G::BUF_BYTES;
-                cp_async_wait_all();
-                __syncwarp();
-                team_sync<TEAM>(quarter);  // staged data and the tile's new values are visible; nobody is an iteration behind
-                u64 dp[2][4][4];
 #pragma unroll
-                for (int dz = 0; dz < 2; ++dz)
+            for (int dz = 0; dz < 2; ++dz) db[dz] = fadd2(db[dz], fadd2(fadd2(dp[dz][0], dp[dz][1]), fadd2(dp[dz][2], dp[dz][3])));
+            const unsigned win = tile + T.cell0 * 16u;
 #pragma unroll
-                    for (int o = 0; o < 4; ++o) {
-                        const float4 a = lds128(stage_d + buf_d * SB + S.at(dz * 2, o)), b = lds128(stage_d + buf_d * SB + S.at(dz * 2 + 1, o));
-                        dp[dz][o][0] = pack2(a.x, b.x);
-                        dp[dz][o][1] = pack2(a.y, b.y);
-                        dp[dz][o][2] = pack2(a.z, b.z);
-                        dp[dz][o][3] = pack2(a.w, b.w);
-                    }
-                // the activations that this warp's neurons turn into: block 8 those of iteration t + 1, into the other tile;
-                // block 4 those of iteration t, in place
-                if (NT == 2 ? !last : t > 0) {
-                    const unsigned to = NT == 2 ? tiles + (buf_x ^ 1) * G::BUF_BYTES : tile;
+            for (int rz = 0; rz < 4; ++rz)
 #pragma unroll
-                    for (int dy = 0; dy < 2; ++dy)
+                for (int ry = 0; ry < 4; ++ry)
 #pragma unroll
-                        for (int o = 0; o < 4; ++o) {
-                            const unsigned c = own0 + (unsigned)(dy * L.ysgn * G::ROW * 16 + o * dx) + role * (G::PLANE * 16u);
-                            u64 h0, h1, x0, x1;
-                            lds128u(stage_h + S.at(role * 2 + dy, o), h0, h1);
-                            lds128u(tile + c, x0, x1);
-                            sts128u(to + c, act_residual2<ACT>(h0, sc[dy][o], x0), act_residual2<ACT>(h1, sc[dy][o], x1));
-                        }
-                    __syncwarp();
-                }
-                if (NT == 1) team_sync<TEAM>(quarter);  // the tile is complete
-                // next iteration's data
-                if (!last) {
-                    fetch_d(corner, t + 1, buf_d ^ 1);
-                    if (NT == 2 ? t + 2 < p.inner : true) fetch_h(corner, NT == 2 ? t + 1 : t);
-                } else if (i + 1 < cnt) {
-                    const size_t next = corner_of(i + 1);
-                    fetch_d(next, 0, buf_d ^ 1);
-                    if (NT == 2 && p.inner > 1) fetch_h(next, 0);
-                    if (NT == 2 && role == 0 && lane == 0) issue(i + 1, buf_x ^ 1);
-                    __syncwarp();
-                }
-                unsigned rows[4];
+                    for (int c = 0; c < 3; ++c) {
+                        const float4 v = lds128(win + (unsigned)(rz * G::PLANE + ry * G::ROW + c) * 16u);
+                        const float vs[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-                for (int ry = 0; ry < 4; ++ry) rows[ry] = tile + (unsigned)(L.cell0 * 16 + ry * L.ysgn * G::ROW * 16);
-                if (role == 0) {
-#pragma unroll
-                    for (int n = 0; n < 4; ++n)
-#pragma unroll
-                        for (int o = 0; o < 4; ++o) {
-                            float e[4];
+                        for (int dz = 0; dz < 2; ++dz) {
+                            const int a = rz - dz;
+                            if (a < 0 || a > 2) continue;
 #pragma unroll
                             for (int s = 0; s < 4; ++s) {
-                                float lo, hi;
-                                unpack2(dp[n >> 1][o][s], lo, hi);
-                                e[s] = n & 1 ? hi : lo;
+                                if (ry == 1 || ry == 2) {
+                                    ffma2(sp[ry - 1][dz][a][c], dp[dz][s], pack2(vs[s], vs[s]));
+                                } else {
+                                    float lo, hi;
+                                    unpack2(dp[dz][s], lo, hi);
+                                    sg[ry ? 1 : 0][dz][a][c] = fmaf(vs[s], ry ? hi : lo, sg[ry ? 1 : 0][dz][a][c]);
+                                }
                             }
-                            dacc[n][o] += (e[0] + e[1]) + (e[2] + e[3]);
                         }
-                    quad_wgrad_rows<G::PLANE, 0>(rows, dx, tm, dp);
-                } else {
-                    quad_wgrad_rows<G::PLANE, 1>(rows, dx, tm, dp);
+                    }
+            if (NT == 2) buf_x ^= 1;
+            buf_d ^= 1;
+        }
+        if (NT == 1 && q + 1 < q1) {
+            __syncthreads();
+            if (tid == 0) issue(q + 1, 0);
+        }
+    }
+    // ---- sums -> this chunk's part: [tap][n] then [bias | scale][n], 128 threads each
+    float *const dst = p.gpk + ((size_t)blockIdx.y * gridDim.x + blk) * GRAD_F + tid;
+    auto put = [&](int k, float v) { dst[k * THREADS] = p.accumulate ? dst[k * THREADS] + v : v; };
+#pragma unroll
+    for (int dz = 0; dz < 2; ++dz)
+#pragma unroll
+        for (int a = 0; a < 3; ++a)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                // window row ry is tap row b = ry - dy of neuron row dy
+                put((a * 9 + 0 + c) * 4 + dz * 2 + 0, sg[0][dz][a][c]);
+                put((a * 9 + 6 + c) * 4 + dz * 2 + 1, sg[1][dz][a][c]);
+#pragma unroll
+                for (int r = 0; r < 2; ++r) {
+                    float lo, hi;
+                    unpack2(sp[r][dz][a][c], lo, hi);
+                    put((a * 9 + (r + 1) * 3 + c) * 4 + dz * 2 + 0, lo);
+                    put((a * 9 + r * 3 + c) * 4 + dz * 2 + 1, hi);
                 }
-                __syncwarp();
-                if (NT == 2) buf_x ^= 1;
-                buf_d ^= 1;
             }
-            if (NT == 1) {
-                team_sync<TEAM>(quarter);
-                if (role == 0 && lane == 0 && i + 1 < cnt) issue(i + 1, 0);
-                __syncwarp();
-            }
-        }
-
-        // ---- the region's sums -> this team's slot
-        const long long slot = team - quad_team_of((long long)blk * p.Q, p.nitems, nteams);
-        float4 *dst = reinterpret_cast<float4 *>(p.gpk + ((size_t)slot * p.regions + blk) * PACK_F) + lane;
-        tmem_wait_st();
-        // half 0: single units first, half 1: last
-        quad_flush72<false>(dst + role * 90 * 32, tm + role * 360, p.accumulate);
-#pragma unroll 1
-        for (int b = 0; b < 2; ++b) {
-            const int at = 1 + role * 2 + b;  // in batches of 72 columns, 18 vectors
-            quad_flush72<true>(dst + at * 18 * 32, tm + at * 72, p.accumulate);
-        }
-        float4 *o4 = dst + (108 + role * 4) * 32, old[4];
-        if (p.accumulate) {
 #pragma unroll
-            for (int n = 0; n < 4; ++n) old[n] = o4[n * 32];
-        }
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            float4 x = make_float4(dacc[n][0], dacc[n][1], dacc[n][2], dacc[n][3]);
-            if (p.accumulate) x.x += old[n].x, x.y += old[n].y, x.z += old[n].z, x.w += old[n].w;
-            o4[n * 32] = x;
-        }
-        __syncwarp();
-        i0 += here;
-        q0 = 0;
-        ++blk;
+    for (int dz = 0; dz < 2; ++dz) {
+        float lo, hi;
+        unpack2(db[dz], lo, hi);
+        put(108 + dz * 2, lo);
+        put(109 + dz * 2, hi);
+        unpack2(ds[dz], lo, hi);
+        put(112 + dz * 2, lo);
+        put(113 + dz * 2, hi);
     }
     if (failed && p.error_flag) *p.error_flag = 1;
-    tmem_fence_before();
-    __syncthreads();
-    if (warp == 0) tmem_free_all(tmem_slot);
 }
 
-// Sums of the teams' slots in team order -> gradients in the layout of the parameters. One CTA per region.
+// The chunks' sums in chunk order -> gradients in the layout of the parameters. Four CTAs per region.
+constexpr int kUnpack = 29;  // of the 116 values per thread
 template <int SUB>
-__global__ void __launch_bounds__(256) quad_unpack_grads_k(const float *__restrict__ gpk, float *__restrict__ gw, float *__restrict__ gb,
-                                                           float *__restrict__ gs, int M, int N, int K, int Q, long long nteams)
+__global__ void __launch_bounds__(128) quad_unpack_grads_k(const float *__restrict__ gpk, float *__restrict__ gw, float *__restrict__ gb,
+                                                           float *__restrict__ gs, int M, int N, int K, int chunks)
 {
-    __shared__ unsigned char uses[36];
-    if (threadIdx.x == 0) {
-        int k = 0;
-        for (int ry = 0; ry < 4; ++ry)
-            for (int rz = 0; rz < 4; ++rz)
-                for (int n = 0; n < 4; ++n) {
-                    const int a = rz - (n >> 1), bb = ry - (n & 1);
-                    if (a >= 0 && a <= 2 && bb >= 0 && bb <= 2) uses[k++] = (unsigned char)((a * 3 + bb) | n << 4);
-                }
-    }
-    __syncthreads();
-    const int lane = threadIdx.x & 31;
-    const QuadLane<SUB> L(lane);
-    const int nbx = K >> 3, nby = N >> 3, blk = blockIdx.x, regions = gridDim.x;
+    using namespace quadwg;
+    const int tid = threadIdx.x;
+    const Patch<SUB> T(tid);
+    const int nbx = K >> 3, nby = N >> 3, blk = blockIdx.x;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t P = (size_t)M * N * K;
-    const size_t g0 = ((size_t)(bz * 8 + L.z0) * N + (by * 8 + L.y0)) * K + bx * 8 + 4 * L.h;
-    const long long zs = (long long)N * K, ys = (long long)L.ysgn * K;
-    const long long nitems = (long long)regions * Q;
-    const int slots = (int)(quad_team_of((long long)(blk + 1) * Q - 1, nitems, nteams) - quad_team_of((long long)blk * Q, nitems, nteams)) + 1;
-#pragma unroll 2
-    for (int v = threadIdx.x >> 5; v < quad::VECS; v += 8) {
-        const float4 *src = reinterpret_cast<const float4 *>(gpk + (size_t)blk * quad::PACK_F) + v * 32 + lane;
-        float4 r = *src;
-        for (int k = 1; k < slots; ++k) {
-            const float4 e = src[(size_t)k * regions * (quad::PACK_F / 4)];
-            r.x += e.x, r.y += e.y, r.z += e.z, r.w += e.w;
-        }
-        if (L.h) r = make_float4(r.w, r.z, r.y, r.x);
-        int n;
-        float *dst;
-        if (v < 108) {
-            const int u = uses[v / 3], c = v % 3;
-            n = u >> 4;
-            const int tb = (u & 15) % 3;
-            dst = gw + (size_t)((u & 15) / 3 * 9 + (L.ysgn < 0 ? 2 - tb : tb) * 3 + (L.h ? 2 - c : c)) * P;
-        } else {
-            n = v & 3;
-            dst = v < 112 ? gb : gs;
-        }
-        dst += g0 + (n >> 1) * zs + (n & 1) * ys;
-        if ((reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-            *reinterpret_cast<float4 *>(dst) = r;
-        } else {
-            dst[0] = r.x, dst[1] = r.y, dst[2] = r.z, dst[3] = r.w;
-        }
+    const size_t g0 = ((size_t)(bz * 8 + 2 * T.zp) * N + (by * 8 + 2 * T.yp)) * K + bx * 8 + T.x;
+    const float *src = gpk + (size_t)blk * GRAD_F + tid;
+    const size_t step = (size_t)gridDim.x * GRAD_F;
+    const int k0 = blockIdx.y * kUnpack;
+#pragma unroll
+    for (int i = 0; i < kUnpack; ++i) {
+        const int k = k0 + i;
+        float v = src[k * THREADS];
+        for (int c = 1; c < chunks; ++c) v += src[c * step + k * THREADS];
+        const int n = k & 3;
+        float *dst = k < 108 ? gw + (size_t)(k >> 2) * P : (k < 112 ? gb : gs);
+        dst[g0 + (size_t)(n >> 1) * N * K + (size_t)(n & 1) * K] = v;
     }
 }
 
@@ -765,7 +589,7 @@ __device__ __forceinline__ float4 fma4(float w, float4 v, float4 a)
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
 namespace quadborder {
-constexpr int TS = 1000;
+constexpr int TS = 1000, RING = 3;
 }
 
 __global__ void __launch_bounds__(384) quad_border8_k(const float *__restrict__ w, const float4 *__restrict__ dsum, float4 *__restrict__ gx,
@@ -774,15 +598,15 @@ __global__ void __launch_bounds__(384) quad_border8_k(const float *__restrict__ 
     using namespace quadborder;
     constexpr int THREADS = 384, SLOTS = 3;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4 *const tile = reinterpret_cast<float4 *>(smem_raw);                   // [2][TS]
-    float4 *const part = reinterpret_cast<float4 *>(smem_raw) + 2 * TS;          // [2][3][128]
+    float4 *const tile = reinterpret_cast<float4 *>(smem_raw);                   // [RING][TS]
+    float4 *const part = reinterpret_cast<float4 *>(smem_raw) + RING * TS;       // [2][3][128]
     const int tid = threadIdx.x;
     const int nbx = K >> 3, nby = N >> 3;
     const unsigned blk = blockIdx.x;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t P = (size_t)M * N * K;
     const long long origin = ((long long)(bz * 8 - 1) * N + (by * 8 - 1)) * K + (bx * 8 - 1);
-    for (int i = tid; i < 2 * TS; i += THREADS) tile[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = tid; i < RING * TS; i += THREADS) tile[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     // shell cells this thread fetches: tile offset and offset from the tile's origin
     int tof[SLOTS], rel[SLOTS];
 #pragma unroll
@@ -844,28 +668,32 @@ __global__ void __launch_bounds__(384) quad_border8_k(const float *__restrict__ 
     const int px = (sx == 0 || sx == 7) ? (sx / 7) * 64 + sz * 8 + sy : -1;
 
     const int q0 = blockIdx.y * qpc, q1 = min(Q, q0 + qpc);
-    float4 pf[SLOTS], gnext = make_float4(0.f, 0.f, 0.f, 0.f);
+    const unsigned tile0 = smem_u32(tile);
+    // two quads ahead: the shell by asynchronous copies, the surface cell by an ordinary load
     auto fetch = [&](int q) {
         if (q < q1) {
             const float4 *src = dsum + (size_t)q * P + origin;
 #pragma unroll
             for (int j = 0; j < SLOTS; ++j)
-                if (tof[j] >= 0) pf[j] = __ldg(src + rel[j]);
+                if (tof[j] >= 0) cp_async16(tile0 + (unsigned)((q % RING) * TS + tof[j]) * 16u, src + rel[j]);
         }
+        asm volatile("cp.async.commit_group;" ::: "memory");
     };
+    float4 g1 = make_float4(0.f, 0.f, 0.f, 0.f), g2 = g1;
+    __syncthreads();  // tiles are zeroed
     fetch(q0);
-    if (active && q0 < q1) gnext = gx[(size_t)q0 * P + c];
-    __syncthreads();
+    fetch(q0 + 1);
+    if (active && q0 < q1) g1 = gx[(size_t)q0 * P + c];
+    if (active && q0 + 1 < q1) g2 = gx[(size_t)(q0 + 1) * P + c];
     for (int q = q0; q < q1; ++q) {
         const int par = q & 1;
-        float4 *tl = tile + par * TS;
-#pragma unroll
-        for (int j = 0; j < SLOTS; ++j)
-            if (tof[j] >= 0) tl[tof[j]] = pf[j];
-        fetch(q + 1);
-        float4 acc = gnext;
-        if (active && q + 1 < q1) gnext = gx[(size_t)(q + 1) * P + c];
-        __syncthreads();
+        const float4 *tl = tile + (q % RING) * TS;
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();  // quad q has landed; the tile of quad q - 1 has been read
+        fetch(q + 2);
+        float4 acc = g1;
+        g1 = g2;
+        if (active && q + 2 < q1) g2 = gx[(size_t)(q + 2) * P + c];
         {
             float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -1181,54 +1009,48 @@ int launch_quad_reverse(const QuadReverse &a, int act, cudaStream_t st)
     return a.block == 8 ? launch_reverse_sub<8>(p, (unsigned)ctas, act, st) : launch_reverse_sub<4>(p, (unsigned)ctas, act, st);
 }
 
-// CTAs of the weight-gradient kernel: every team writes (or adds to) 59 KB per region it touches, so small problems use
-// teams of at least two items
-static unsigned wgrad_ctas(long long nitems)
+// Into how many chunks the quads of a region go: as many as fill three CTAs per SM evenly. A chunk costs its CTA about
+// two quads' time (tile latency, sums out) and its part of the gradient, 59 KB, is written and added up once.
+static int wgrad_chunks(long long regions, int Q)
 {
-    long long ctas = (nitems + 2 * quad::QUARTERS - 1) / (2 * quad::QUARTERS);
-    if (ctas > sm_count()) ctas = sm_count();
-    return (unsigned)(ctas < 1 ? 1 : ctas);
+    const int c = pick_batch_chunks_balanced(regions, Q, quadwg::CTAS, 2.0, 16);
+    const int qpc = (Q + c - 1) / c;
+    return (Q + qpc - 1) / qpc;
 }
 
 size_t quad_grad_floats(int M, int N, int K, int Q)
 {
-    const long long regions = regions_of(M, N, K), nitems = regions * Q;
-    const long long nteams = (long long)wgrad_ctas(nitems) * quad::QUARTERS;
-    long long slots = 1;
-    for (long long r = 0; r < regions; ++r) {
-        const long long s = quad_team_of((r + 1) * Q - 1, nitems, nteams) - quad_team_of(r * Q, nitems, nteams) + 1;
-        if (s > slots) slots = s;
-    }
-    return (size_t)slots * regions * quad::PACK_F;
+    const long long regions = regions_of(M, N, K);
+    return (size_t)wgrad_chunks(regions, Q) * regions * quadwg::GRAD_F;
 }
 
 template <int SUB, int ACT>
-static int launch_wgrad_one(const CUtensorMap &map, const QuadWgradParams &p, unsigned ctas, cudaStream_t st)
+static int launch_wgrad_one(const CUtensorMap &map, const QuadWgradParams &p, dim3 grid, cudaStream_t st)
 {
     static unsigned long long done[2] = {};
-    constexpr int smem = quadwg::Lay<SUB>::SMEM;
-    static_assert(smem <= 232448 - 2048, "shared memory budget of one SM");
     int rc;
     if (p.in_stats) {
+        constexpr int smem = quadwg::Lay<SUB>::smem(true);
         rc = smem_once(quad_wgrad_k<SUB, ACT, true>, smem, &done[1], "cudaFuncSetAttribute(quad_wgrad_k)");
         if (rc != GN_OK) return rc;
-        quad_wgrad_k<SUB, ACT, true><<<ctas, 256, smem, st>>>(map, p);
+        quad_wgrad_k<SUB, ACT, true><<<grid, quadwg::THREADS, smem, st>>>(map, p);
     } else {
+        constexpr int smem = quadwg::Lay<SUB>::smem(false);
         rc = smem_once(quad_wgrad_k<SUB, ACT, false>, smem, &done[0], "cudaFuncSetAttribute(quad_wgrad_k)");
         if (rc != GN_OK) return rc;
-        quad_wgrad_k<SUB, ACT, false><<<ctas, 256, smem, st>>>(map, p);
+        quad_wgrad_k<SUB, ACT, false><<<grid, quadwg::THREADS, smem, st>>>(map, p);
     }
     return check_launch("quad_wgrad");
 }
 
 template <int SUB>
-static int launch_wgrad_sub(const CUtensorMap &map, const QuadWgradParams &p, unsigned ctas, int act, cudaStream_t st)
+static int launch_wgrad_sub(const CUtensorMap &map, const QuadWgradParams &p, dim3 grid, int act, cudaStream_t st)
 {
     switch (act) {
-    case GN_ACT_RELU: return launch_wgrad_one<SUB, GN_ACT_RELU>(map, p, ctas, st);
-    case GN_ACT_LEAKY_RELU: return launch_wgrad_one<SUB, GN_ACT_LEAKY_RELU>(map, p, ctas, st);
-    case GN_ACT_SILU: return launch_wgrad_one<SUB, GN_ACT_SILU>(map, p, ctas, st);
-    default: return launch_wgrad_one<SUB, GN_ACT_TANH>(map, p, ctas, st);
+    case GN_ACT_RELU: return launch_wgrad_one<SUB, GN_ACT_RELU>(map, p, grid, st);
+    case GN_ACT_LEAKY_RELU: return launch_wgrad_one<SUB, GN_ACT_LEAKY_RELU>(map, p, grid, st);
+    case GN_ACT_SILU: return launch_wgrad_one<SUB, GN_ACT_SILU>(map, p, grid, st);
+    default: return launch_wgrad_one<SUB, GN_ACT_TANH>(map, p, grid, st);
     }
 }
 
@@ -1243,31 +1065,32 @@ int launch_quad_wgrad(const QuadWgrad &a, int act, cudaStream_t st)
     p.accumulate = a.accumulate;
     p.error_flag = a.error_flag ? a.error_flag : device_status_ptr();
     p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;
-    p.regions = (int)regions_of(a.M, a.N, a.K);
-    p.nitems = (long long)p.regions * a.Q;
-    const unsigned ctas = wgrad_ctas(p.nitems);
-    return a.block == 8 ? launch_wgrad_sub<8>(map, p, ctas, act, st) : launch_wgrad_sub<4>(map, p, ctas, act, st);
+    const long long regions = regions_of(a.M, a.N, a.K);
+    const int chunks = wgrad_chunks(regions, a.Q);
+    p.qpc = (a.Q + chunks - 1) / chunks;
+    const dim3 grid((unsigned)regions, (unsigned)chunks);
+    return a.block == 8 ? launch_wgrad_sub<8>(map, p, grid, act, st) : launch_wgrad_sub<4>(map, p, grid, act, st);
 }
 
 int launch_quad_unpack_grads(const float *gpk, float *gw, float *gb, float *gs, int M, int N, int K, int Q, int block, cudaStream_t st)
 {
     const long long regions = regions_of(M, N, K);
-    const long long nteams = (long long)wgrad_ctas(regions * Q) * quad::QUARTERS;
-    if (block == 8) quad_unpack_grads_k<8><<<(unsigned)regions, 256, 0, st>>>(gpk, gw, gb, gs, M, N, K, Q, nteams);
-    else quad_unpack_grads_k<4><<<(unsigned)regions, 256, 0, st>>>(gpk, gw, gb, gs, M, N, K, Q, nteams);
+    const int chunks = wgrad_chunks(regions, Q);
+    if (block == 8) quad_unpack_grads_k<8><<<dim3((unsigned)regions, 116 / kUnpack), 128, 0, st>>>(gpk, gw, gb, gs, M, N, K, chunks);
+    else quad_unpack_grads_k<4><<<dim3((unsigned)regions, 116 / kUnpack), 128, 0, st>>>(gpk, gw, gb, gs, M, N, K, chunks);
     return check_launch("quad_unpack_grads");
 }
 
 int launch_quad_border(const float *w, const float *dsum, float *gx, int M, int N, int K, int Q, int block, cudaStream_t st)
 {
     const long long nb = regions_of(M, N, K);
-    const int ctas_per_sm = block == 8 ? 4 : 3;
+    const int ctas_per_sm = 3;
     const int chunks = pick_batch_chunks_balanced(nb, Q, ctas_per_sm, 4.0, 32);
     const int qpc = (Q + chunks - 1) / chunks;
     dim3 grid((unsigned)nb, (unsigned)((Q + qpc - 1) / qpc));
     static unsigned long long done[2] = {};
     if (block == 8) {
-        constexpr int smem = (2 * quadborder::TS + 2 * 3 * 128) * 16;
+        constexpr int smem = (quadborder::RING * quadborder::TS + 2 * 3 * 128) * 16;
         const int rc = smem_once(quad_border8_k, smem, &done[0], "cudaFuncSetAttribute(quad_border8_k)");
         if (rc != GN_OK) return rc;
         quad_border8_k<<<grid, 384, smem, st>>>(w, reinterpret_cast<const float4 *>(dsum), reinterpret_cast<float4 *>(gx), Q, M, N, K, qpc);
