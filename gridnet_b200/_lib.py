@@ -76,6 +76,10 @@ SIGNATURES = {
                                             c_int, c_int, c_int, c_int, c_int, _P, _P]),
     "gn_norm_finalize_f32": (c_int, [_P, c_int, _P, c_int, c_longlong, c_float, _P]),
     "gn_norm_apply_f32": (c_int, [_P] * 5 + [c_int, c_longlong, _P]),
+    "gn_step_kept_bytes": (c_size_t, [c_int] * 7),
+    "gn_step_kept_workspace_bytes": (c_size_t, [c_int] * 9),
+    "gn_step_forward_kept_f32": (c_int, [_P] * 5 + _geom + [c_int, c_int, c_float, c_int, c_int, _P, c_size_t, _P, c_size_t, _P]),
+    "gn_step_backward_kept_f32": (c_int, [_P] * 9 + _geom + [c_int, c_int, c_float, c_int, c_int, _P, c_size_t, _P, c_size_t, _P]),
     "gn_loop_train_supported": (c_int, [c_int] * 6),
     "gn_loop_tensor_bytes": (c_size_t, [c_int] * 4),
     "gn_loop_forward_workspace_bytes": (c_size_t, [c_int] * 8),

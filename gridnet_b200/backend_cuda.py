@@ -15,6 +15,8 @@ models run between steps (gridnet/scripts/train_mnist.py:54,62-64):
 from __future__ import annotations
 
 import ctypes
+import functools
+import threading
 
 import torch
 
@@ -57,18 +59,64 @@ def keep_forward_stash(enabled):
     return previous
 
 
-def _stash_wanted(weight, init_activations, inner_iters: int, block_size: int) -> bool:
-    if _keep_forward_stash is not None:
-        return _keep_forward_stash
-    B, M, N, K = init_activations.shape
-    need = int(lib.gn_step_stash_bytes(B, M, N, K, int(inner_iters), int(block_size)))
-    if need <= 0:
-        return False
-    dev = weight.device
-    free, _ = torch.cuda.mem_get_info(dev)
-    # what torch's caching allocator holds but has not handed out counts as free too
-    free += torch.cuda.memory_reserved(dev) - torch.cuda.memory_allocated(dev)
-    return need * 10 <= free
+class _Kept:
+    """``nbytes`` of device memory that a step keeps for its backward pass. Knows how much all of them hold together, which
+    is what makes it unnecessary to ask the driver for the free memory (half a millisecond) before every small step."""
+
+    _lock, _held = threading.Lock(), 0
+
+    def __init__(self, nbytes: int, device):
+        self.buffer = torch.empty(nbytes, dtype=torch.uint8, device=device)
+        self.nbytes = nbytes
+        with _Kept._lock:
+            _Kept._held += nbytes
+
+    def __del__(self):
+        if hasattr(self, "nbytes"):
+            with _Kept._lock:
+                _Kept._held -= self.nbytes
+
+    @staticmethod
+    def room_for(need: int, device) -> bool:
+        """As :func:`keep_forward_stash` says; otherwise while all steps together keep less than 2 GiB, and beyond that while
+        ``need`` is at most a tenth of the free device memory."""
+        if _keep_forward_stash is not None:
+            return _keep_forward_stash
+        if _Kept._held + need <= 2 << 30:
+            return True
+        free, _ = torch.cuda.mem_get_info(device)
+        # what torch's caching allocator holds but has not handed out counts as free too
+        free += torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
+        return need * 10 <= free
+
+
+# Time of a step forward and backward in microseconds, measured over 16 x 32 x 24 .. 96^3 grids, batches of 2 to 128 and one to
+# five inner iterations: max(host, fixed + per neuron * P + B * P * (a + b * inner)). The kernels of forward_kept re-order 27 weights per
+# neuron three times but do a sample in a half to two thirds of the time (a seventh against the general kernels, which are the
+# others' choice for normalised blocks of 4).
+_STEP_COST_KEPT = {False: (195, 0, 4.2e-4, 14e-6, 6e-6), True: (195, 0, 4.2e-4, 18e-6, 8e-6)}  # by normalize
+_STEP_COST_OTHER = {(8, False): (175, 85, 5e-5, 11e-6, 10.5e-6), (8, True): (170, 100, 7e-5, 20e-6, 19.7e-6),
+                    (4, False): (175, 60, 6e-5, 12e-6, 15.5e-6), (4, True): (152, 45, 0, 0, 120e-6)}
+
+
+def _step_cost(c, P: int, B: int, inner: int) -> float:
+    host, fixed, per_neuron, a, b = c
+    return max(host, fixed + per_neuron * P + B * P * (a + b * inner))
+
+
+@functools.lru_cache(maxsize=512)
+def _kept_is_faster(shape, inner: int, block: int, normalize: bool) -> bool:
+    B, M, N, K = shape
+    P = M * N * K
+    return (block, normalize) in _STEP_COST_OTHER and _step_cost(_STEP_COST_KEPT[normalize], P, 4 * ((B + 3) // 4), inner) < _step_cost(
+        _STEP_COST_OTHER[block, normalize], P, B, inner)
+
+
+def _quad_step(weight, x, inner_iters: int, block_size: int, normalize: bool):
+    """What :func:`gridnet_cuda.step_bytes` says if the step should run on the kernels of :func:`gridnet_cuda.forward_kept`."""
+    if weight.dtype != torch.float32 or not _kept_is_faster(x.shape, int(inner_iters), int(block_size), bool(normalize)):
+        return None
+    return gridnet_cuda.step_bytes(weight, x, inner_iters, block_size, normalize)
 
 
 class GridnetCudaOp(torch.autograd.Function):
@@ -82,15 +130,29 @@ class GridnetCudaOp(torch.autograd.Function):
             return init_activations.clone()
         ctx.save_for_backward(weight, bias, residual_scale, init_activations)
         ctx.cfg = (inner_iters, block_size, eps, normalize, activation)
-        ctx.stash = None
+        ctx.kept = None
         outputs = torch.empty_like(init_activations)
-        if (not normalize and weight.dtype == torch.float32 and any(ctx.needs_input_grad[:4])
-                and _stash_wanted(weight, init_activations, inner_iters, block_size)):
-            ctx.stash = gridnet_cuda.forward_with_stash(weight, bias, residual_scale, init_activations, outputs,
-                                                        inner_iters, block_size, activation)
-            return outputs
-        gridnet_cuda.forward(weight, bias, residual_scale, init_activations, outputs, inner_iters, block_size,
-                             eps, normalize, activation)
+        args = (weight, bias, residual_scale, init_activations, outputs, inner_iters, block_size)
+        quad = _quad_step(weight, init_activations, inner_iters, block_size, normalize)
+        ctx.quad = quad is not None
+        need = 0
+        if weight.dtype == torch.float32 and any(ctx.needs_input_grad[:4]):
+            if quad is not None:
+                need = quad[0]
+            elif not normalize:
+                need = int(lib.gn_step_stash_bytes(*init_activations.shape, int(inner_iters), int(block_size)))
+        if need and _Kept.room_for(need, weight.device):
+            try:
+                ctx.kept = _Kept(need, weight.device)
+            except torch.cuda.OutOfMemoryError:
+                pass  # the backward pass runs the step again
+        if ctx.quad:
+            gridnet_cuda.forward_kept(*args, eps, normalize, activation, None if ctx.kept is None else ctx.kept.buffer)
+        elif ctx.kept is not None:
+            if gridnet_cuda.forward_with_stash(*args, activation, ctx.kept.buffer) is None:
+                ctx.kept = None
+        else:
+            gridnet_cuda.forward(*args, eps, normalize, activation)
         return outputs
 
     @staticmethod
@@ -98,20 +160,16 @@ class GridnetCudaOp(torch.autograd.Function):
         weight, bias, residual_scale, init_activations = ctx.saved_tensors
         inner_iters, block_size, eps, normalize, activation = ctx.cfg
         # every gradient buffer is written in full by the library: no zero fill
-        weight_grad = torch.empty_like(weight)
-        bias_grad = torch.empty_like(bias)
-        scale_grad = torch.empty_like(residual_scale)
-        act_grad = torch.empty_like(init_activations)
-        if ctx.stash is not None:
-            stash, ctx.stash = ctx.stash, None
-            gridnet_cuda.backward_with_stash(weight, bias, residual_scale, init_activations, grad_output.contiguous(),
-                                             weight_grad, bias_grad, scale_grad, act_grad, inner_iters, block_size,
-                                             activation, stash)
-            return weight_grad, bias_grad, scale_grad, act_grad, None, None, None, None, None
-        gridnet_cuda.backward(weight, bias, residual_scale, init_activations, grad_output.contiguous(),
-                              weight_grad, bias_grad, scale_grad, act_grad, inner_iters, block_size, eps,
-                              normalize, activation)
-        return weight_grad, bias_grad, scale_grad, act_grad, None, None, None, None, None
+        grads = [torch.empty_like(t) for t in ctx.saved_tensors]
+        args = (weight, bias, residual_scale, init_activations, grad_output.contiguous(), *grads, inner_iters, block_size)
+        kept, ctx.kept = ctx.kept, None
+        if ctx.quad:
+            gridnet_cuda.backward_kept(*args, eps, normalize, activation, None if kept is None else kept.buffer)
+        elif kept is not None:
+            gridnet_cuda.backward_with_stash(*args, activation, kept.buffer)
+        else:
+            gridnet_cuda.backward(*args, eps, normalize, activation)
+        return (*grads, None, None, None, None, None)
 
 
 class GatedGridnetCudaOp(torch.autograd.Function):

@@ -1021,13 +1021,13 @@ static int outer_forward_impl(const float *w, const float *b, const float *s, co
             record_cuda_error(cudaGetLastError(), "cudaMemsetAsync");
             return GN_ERR_CUDA;
         }
+        QuadPrepare r{};
         if (!(flags & GN_OUTER_PARAMS_UNCHANGED)) {
-            rc = launch_quad_pack(w, b, s, ws.qpacked, M, N, K, block, false, st);
-            if (rc != GN_OK) return rc;
-            rc = launch_quad_table(gamma, beta, ws.gbt, M, N, K, block, st);
-            if (rc != GN_OK) return rc;
+            r.w = w; r.b = b; r.s = s; r.packed = ws.qpacked;
+            r.gamma = gamma; r.beta = beta; r.gbt = ws.gbt;
         }
-        rc = launch_to_il4(x, ws.buf[0], B, P, st);
+        r.x = x; r.il = ws.buf[0]; r.B = B;
+        rc = launch_quad_prepare(r, M, N, K, block, st);
         if (rc != GN_OK) return rc;
         for (int o = 0; o < outer; ++o) {
             QuadStep a{};

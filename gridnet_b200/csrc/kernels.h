@@ -136,34 +136,53 @@ int launch_from_il64(const float *il, const float2 *stats, const float *gamma, c
 // ---- step_quad.cu (weights in tensor memory, four samples per lane; activations in the IL4 layout [quad][z][y][x][4
 // samples], blocks of 8 and 4; B need not be a multiple of 4, the missing samples are zeros)
 struct QuadStep {
-    const float *packed;      // from launch_quad_pack
-    const float2 *gbt;        // from launch_quad_table; used when in_stats is set
+    const float *packed;      // from launch_quad_prepare
+    const float2 *gbt;        // from launch_quad_prepare; used when in_stats is set
     const float *in_il4;
     float *out_il4;           // or nullptr
     const float2 *in_stats;   // [4 Q] or nullptr
     double2 *out_partials;    // [4 Q][nparts] or nullptr; slots 0 .. regions-1 of every row are written
     int nparts;
     float *save_h;            // [inner] IL4 tensors of pre-activations, or nullptr
+    const float *wsum;        // from launch_quad_prepare: per-block normalisation; nullptr: off
+    float4 *tile_stats;       // with wsum and save_h: quad_stats_vectors(...) vectors
+    float eps;
     int *error_flag;
     int M, N, K, Q, inner, block;
 };
 bool quad_applicable(int M, int N, int K, int block, int inner);
 size_t quad_packed_floats(int M, int N, int K);
-int launch_quad_pack(const float *w, const float *b, const float *s, float *packed, int M, int N, int K, int block, bool transposed,
-                     cudaStream_t st);
+size_t quad_tiles(int M, int N, int K, int block);
+size_t quad_stats_vectors(int M, int N, int K, int Q, int inner, int block);
 int quad_tile_cells(int block);  // float2 entries per region of the (gamma, beta) table
-int launch_quad_table(const float *gamma, const float *beta, float2 *gbt, int M, int N, int K, int block, cudaStream_t st);
-int launch_to_il4(const float *x, float *il, int B, long long P, cudaStream_t st);
+// What is re-ordered ahead of a step or a loop; jobs whose destination is nullptr are left out.
+struct QuadPrepare {
+    const float *w, *b, *s;
+    float *packed;             // quad_packed_floats(...): weights, b, s in the order of the forward sums
+    const float *b_t;
+    float *packed_t;           // the same for the backward sums: transposed weights, b_t, s
+    float *wsum;               // M N K floats: the neurons' weight sums
+    const float *gamma, *beta;
+    float2 *gbt;               // regions x quad_tile_cells(block)
+    const float *x;
+    float *il;                 // x [B, P] -> IL4
+    int B;
+};
+int launch_quad_prepare(const QuadPrepare &a, int M, int N, int K, int block, cudaStream_t st);
 int launch_from_il4(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, long long P,
                     cudaStream_t st);
 int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st);
 
 // ---- step_quad_bwd.cu (backward of the quad kernels; all activation tensors IL4)
 struct QuadReverse {
-    const float *packed_t;     // launch_quad_pack(..., transposed) with (norm weight, scale) in the place of (bias, scale)
+    const float *packed_t;     // launch_quad_prepare; whole-grid norm: with the norm's weight as b_t
     const float *g;            // gradient of the step's output; with raw: of its normalised output
     const float *raw;          // the step's output, or nullptr
-    const float2 *stats, *ac;  // with raw
+    const float2 *stats, *ac;  // with raw, unless:
+    const float *wsum;         // per-block normalisation: the forward pass's, and
+    const float4 *tile_stats;  //   its statistics; nullptr: off
+    float4 *hterm;             // with tile_stats: [Q][tiles][2]
+    int B;                     // samples that are real
     const float *h;            // [inner]
     float *delta, *dsum, *gx;  // [inner], one, one
     float *dsq;                // [Q][P]
@@ -177,14 +196,19 @@ struct QuadWgrad {
     const float *delta, *h, *dsq;
     const float *scale;        // native layout: activations between iterations are rebuilt from h
     float *gpk;                // quad_grad_floats(...)
+    const float4 *tile_stats;  // per-block normalisation, or nullptr
     int accumulate;
     int *error_flag;
     int M, N, K, Q, inner, block;
 };
 size_t quad_grad_floats(int M, int N, int K, int Q);
 int launch_quad_wgrad(const QuadWgrad &a, int act, cudaStream_t st);
-int launch_quad_unpack_grads(const float *gpk, float *gw, float *gb, float *gs, int M, int N, int K, int Q, int block, cudaStream_t st);
-int launch_quad_border(const float *w, const float *dsum, float *gx, int M, int N, int K, int Q, int block, cudaStream_t st);
+// gradients of the parameters out of gpk and, with il, il (IL4) -> x [B, P]
+int launch_quad_finish(const float *gpk, float *gw, float *gb, float *gs, const float *il, float *x, int B, int M, int N, int K, int block,
+                       cudaStream_t st);
+// hterm (from launch_quad_reverse) and the step's input: per-block normalisation, or nullptr
+int launch_quad_border(const float *w, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K, int Q,
+                       int block, cudaStream_t st);
 int quad_norm_parts(long long P);
 int launch_quad_norm_sums(const float *x, const float *g, const float *sub, const float *gamma, const float2 *stats, double2 *partials,
                           float *ggamma, float *gbeta, int accumulate, float2 *ac, int Q, long long P, cudaStream_t st);

@@ -10,8 +10,10 @@ namespace gn {
 namespace quad {
 constexpr int QUARTERS = 4;
 constexpr unsigned kSpinLimit = 1u << 20;
-// columns of tensor memory: 36 uses of 12 weights, then 16 biases, 16 scales
-constexpr int COL_BIAS = 432, COL_SCALE = 448;
+// columns of tensor memory: 36 uses of 12 weights, then 16 biases, 16 scales, 16 weight sums (per-block normalisation)
+constexpr int COL_BIAS = 432, COL_SCALE = 448, COL_WSUM = 464;
+// what the 27-tap sums start from: what is there (backward), the bias, or minus the tile's mean times the weight sum
+enum Mode { ADD, BIAS, NORMED };
 }  // namespace quad
 
 // A region's tile buffer, in cells of 16 bytes (four samples).
@@ -205,29 +207,49 @@ __device__ __forceinline__ void quad_load_params(const float *packed, int role, 
     quad_move<29>(src + 29 * 32, tm + role * 232 + 116);
 }
 
+// the weight sums of per-block normalisation (quad_wsum_k), by one warp of the team
+__device__ __forceinline__ void quad_load_wsum(const float *wsum, int region, int lane, unsigned tm)
+{
+    const float4 *src = reinterpret_cast<const float4 *>(wsum) + (size_t)region * 128 + lane;
+    float r[16];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 v = __ldg(src + k * 32);
+        r[4 * k + 0] = v.x, r[4 * k + 1] = v.y, r[4 * k + 2] = v.z, r[4 * k + 3] = v.w;
+    }
+    tmem_st16(tm + quad::COL_WSUM, r);
+}
+
 // The 27-tap sums of the lane's 16 neurons for four samples, acc[n = (dz, dy)][o][sample pair] += sum.
-//   FWD: acc starts at the bias, and done(n, o, scale, centre) is called when a sum is complete - for the neurons of
-//   dy = 0 between the FMAs of the last window rows, so that their activation functions (MUFU) run under them.
-//   Otherwise acc is added to, and done is not called.
+//   BIAS: acc starts at the bias, and done(n, o, scale, bias, centre) is called when a sum is complete - for the neurons
+//   of dy = 0 between the FMAs of the last window rows, so that their activation functions (MUFU) run under them.
+//   NORMED: the same, but acc starts at negm (minus the mean of the tile) times the sum of the neuron's weights, and the
+//   bias is left to done. ADD: acc is added to, and done is not called.
 //   rows[ry]: where window row ry of plane 0, column 0 starts; PLANE: cells from one plane to the next; dx: bytes from
 //   one column to the next.
-template <int PLANE, bool FWD, typename Done>
-__device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, unsigned tm, u64 (&acc)[4][4][2], Done done)
+template <int PLANE, quad::Mode MODE, typename Done>
+__device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, unsigned tm, u64 (&acc)[4][4][2], const u64 (&negm)[2],
+                                             Done done)
 {
-    float wb[2][12], sc[2][4];
-    auto finish = [&](int n, int o, float s) {
+    constexpr bool FWD = MODE != quad::ADD, NORMED = MODE == quad::NORMED;
+    float wb[2][12], sc[2][4], bi[2][4];
+    auto finish = [&](int n, int o, float s, float b) {
         u64 c0, c1;
         lds128u(rows[1 + (n & 1)] + (unsigned)((1 + o) * dx) + (1 + (n >> 1)) * PLANE * 16u, c0, c1);
-        done(n, o, s, c0, c1);
+        done(n, o, s, b, c0, c1);
     };
     if (FWD) {
-        float bias[16];
-        tmem_ld16(tm + quad::COL_BIAS, bias);
-        tmem_wait_ld16(bias);
+        float first[16];
+        tmem_ld16(tm + (NORMED ? quad::COL_WSUM : quad::COL_BIAS), first);
+        tmem_wait_ld16(first);
 #pragma unroll
         for (int n = 0; n < 4; ++n)
 #pragma unroll
-            for (int o = 0; o < 4; ++o) acc[n][o][0] = acc[n][o][1] = pack2(bias[n * 4 + o], bias[n * 4 + o]);
+            for (int o = 0; o < 4; ++o) {
+                const u64 f2 = pack2(first[n * 4 + o], first[n * 4 + o]);
+#pragma unroll
+                for (int k = 0; k < 2; ++k) acc[n][o][k] = NORMED ? fmul2(f2, negm[k]) : f2;
+            }
     }
     tmem_ld8(tm, wb[0]);
     tmem_ld4(tm + 8, wb[0] + 8);
@@ -249,6 +271,7 @@ __device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, 
                 float *wp = wb[use & 1];
                 tmem_wait_ld12(wp);
                 if (FWD && use == 30) tmem_use8(sc[0]);  // asked for before: that wait covered it
+                if (NORMED && use == 30) tmem_use8(bi[0]);
                 if (use + 1 < 36) {
                     tmem_ld8(tm + (use + 1) * 12, wb[(use & 1) ^ 1]);
                     tmem_ld4(tm + (use + 1) * 12 + 8, wb[(use & 1) ^ 1] + 8);
@@ -256,6 +279,10 @@ __device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, 
                 if (FWD && use == 29) {
                     tmem_ld4(tm + quad::COL_SCALE, sc[0]);
                     tmem_ld4(tm + quad::COL_SCALE + 8, sc[1]);
+                    if (NORMED) {
+                        tmem_ld4(tm + quad::COL_BIAS, bi[0]);
+                        tmem_ld4(tm + quad::COL_BIAS + 8, bi[1]);
+                    }
                 }
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
@@ -268,16 +295,22 @@ __device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, 
                 ++use;
                 if (FWD && ry == 3)
 #pragma unroll
-                    for (int e = (use - 30) * 8 / 6; fin < e; ++fin) finish((fin >> 2) * 2, fin & 3, sc[fin >> 2][fin & 3]);
+                    for (int e = (use - 30) * 8 / 6; fin < e; ++fin)
+                        finish((fin >> 2) * 2, fin & 3, sc[fin >> 2][fin & 3], NORMED ? bi[fin >> 2][fin & 3] : 0.0f);
             }
         }
     }
     if (FWD) {
         tmem_ld4(tm + quad::COL_SCALE + 4, sc[0]);
         tmem_ld4(tm + quad::COL_SCALE + 12, sc[1]);
+        if (NORMED) {
+            tmem_ld4(tm + quad::COL_BIAS + 4, bi[0]);
+            tmem_ld4(tm + quad::COL_BIAS + 12, bi[1]);
+        }
         tmem_wait_ld8(sc[0]);
+        if (NORMED) tmem_use8(bi[0]);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) finish((e >> 2) * 2 + 1, e & 3, sc[e >> 2][e & 3]);
+        for (int e = 0; e < 8; ++e) finish((e >> 2) * 2 + 1, e & 3, sc[e >> 2][e & 3], NORMED ? bi[e >> 2][e & 3] : 0.0f);
     }
 }
 
@@ -295,5 +328,34 @@ __device__ __forceinline__ float quad_reduce8(const float (&v)[8], int lane)
     c += __shfl_xor_sync(0xffffffffu, c, 1);
     return c;
 }
+
+// Adds eight values over the lanes that share a tile (block 8: the warp, block 4: the four lanes of a sub-block); every
+// lane gets all eight sums.
+template <int SUB>
+__device__ __forceinline__ void quad_tile_sum8(float (&v)[8], int lane)
+{
+    if (SUB == 8) {
+        const float r = quad_reduce8(v, lane);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) v[k] = __shfl_sync(0xffffffffu, r, 4 * k);
+    } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            v[k] += __shfl_xor_sync(0xffffffffu, v[k], 2);
+            v[k] += __shfl_xor_sync(0xffffffffu, v[k], 8);
+        }
+    }
+}
+// The tile of a lane among all blocks of the grid (block 8: the region, block 4: eight per region), and the lane that
+// writes what the lanes of a tile have in common.
+template <int SUB>
+__device__ __forceinline__ int quad_tile_of(const QuadLane<SUB> &L, int region)
+{
+    return SUB == 8 ? region : region * 8 + ((L.z0 >> 2) * 2 + (L.y0 >> 2)) * 2 + L.h;
+}
+template <int SUB>
+__device__ __forceinline__ bool quad_tile_leader(int lane) { return SUB == 8 ? lane == 0 : (lane & 10) == 0; }
+// Per-block normalisation keeps, for every iteration, quad and tile, four vectors over the quad's samples
+enum QuadStat { QS_MEAN, QS_INV /* 1 / (std + eps) */, QS_STD, QS_STDEPS, QS_COUNT };
 
 }  // namespace gn

@@ -36,7 +36,6 @@ struct LoopWs {
     float *packed, *packed_t, *gpk, *tmp, *g[2], *delta, *dsum, *dsq, *replay;
     float2 *gbt, *ac;
     double2 *partials;
-    int *error_flag;
     size_t bytes;
 };
 
@@ -55,7 +54,6 @@ static LoopWs carve_loop(void *base, const LoopDims &d, bool backward, bool repl
     size_t parts = d.regions;
     if (backward && (size_t)quad_norm_parts(d.P) > parts) parts = quad_norm_parts(d.P);
     if (d.residual && (size_t)quad_combine_parts(d.P) > parts) parts = quad_combine_parts(d.P);
-    w.error_flag = static_cast<int *>(take(sizeof(int)));
     w.partials = static_cast<double2 *>(take(sizeof(double2) * parts * 4 * d.Q));
     w.gbt = static_cast<float2 *>(take(sizeof(float2) * (size_t)d.regions * quad_tile_cells(d.block)));
     if (!backward || replay) w.packed = static_cast<float *>(take(pk));
@@ -90,14 +88,6 @@ static int loop_check(int B, int M, int N, int K, int inner, int outer, int bloc
         const int rc_ = (call);        \
         if (rc_ != GN_OK) return rc_;  \
     } while (0)
-
-static int clear_flag(int *flag, cudaStream_t st)
-{
-    const cudaError_t e = cudaMemsetAsync(flag, 0, sizeof(int), st);
-    if (e == cudaSuccess) return GN_OK;
-    record_cuda_error(e, "cudaMemsetAsync");
-    return GN_ERR_CUDA;
-}
 
 }  // namespace gn
 
@@ -141,15 +131,23 @@ GN_API int gn_loop_forward_f32(const float *const *weights, const float *const *
     cudaStream_t st = (cudaStream_t)stream;
     float2 *const mr = reinterpret_cast<float2 *>(stats);
     const int S = 4 * d.Q;  // statistics of one step
-    TRY_(clear_flag(w.error_flag, st));
-    TRY_(launch_quad_table(gamma, beta, w.gbt, M, N, K, block, st));
-    TRY_(launch_to_il4(x, x_il4, B, d.P, st));
+    {
+        QuadPrepare a{};
+        a.w = weights[0]; a.b = biases[0]; a.s = scales[0]; a.packed = w.packed;
+        a.gamma = gamma; a.beta = beta; a.gbt = w.gbt;
+        a.x = x; a.il = x_il4; a.B = B;
+        TRY_(launch_quad_prepare(a, M, N, K, block, st));
+    }
     if (residual) {
         TRY_(launch_quad_residual_combine(x_il4, nullptr, nullptr, nullptr, nullptr, nullptr, w.partials, d.Q, d.P, st));
         TRY_(launch_norm_finalize(w.partials, quad_combine_parts(d.P), mr, S, d.P, ln_eps, st));
     }
     for (int k = 0; k < outer; ++k) {
-        if (k == 0 || nparams > 1) TRY_(launch_quad_pack(weights[k], biases[k], scales[k], w.packed, M, N, K, block, false, st));
+        if (k > 0 && nparams > 1) {
+            QuadPrepare a{};
+            a.w = weights[k]; a.b = biases[k]; a.s = scales[k]; a.packed = w.packed;
+            TRY_(launch_quad_prepare(a, M, N, K, block, st));
+        }
         const float *in = k ? outs[k - 1] : x_il4;
         QuadStep a{};
         a.packed = w.packed; a.gbt = w.gbt;
@@ -159,7 +157,6 @@ GN_API int gn_loop_forward_f32(const float *const *weights, const float *const *
         a.out_partials = residual ? nullptr : w.partials;
         a.nparts = d.regions;
         if (stashes) a.save_h = stashes[k];
-        a.error_flag = w.error_flag;
         a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;
         TRY_(launch_step_fwd_quad(a, act, st));
         if (residual) {
@@ -169,8 +166,7 @@ GN_API int gn_loop_forward_f32(const float *const *weights, const float *const *
             TRY_(launch_norm_finalize(w.partials, d.regions, mr + (size_t)k * S, S, d.P, ln_eps, st));
         }
     }
-    TRY_(launch_from_il4(outs[outer - 1], residual ? nullptr : mr + (size_t)(outer - 1) * S, gamma, beta, y, B, d.P, st));
-    return launch_propagate_flag(w.error_flag, st);
+    return launch_from_il4(outs[outer - 1], residual ? nullptr : mr + (size_t)(outer - 1) * S, gamma, beta, y, B, d.P, st);
 }
 
 GN_API int gn_loop_backward_f32(const float *const *weights, const float *const *biases, const float *const *scales, int nparams,
@@ -191,10 +187,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
     cudaStream_t st = (cudaStream_t)stream;
     const float2 *const mr = reinterpret_cast<const float2 *>(stats);
     const int S = 4 * d.Q;
-    TRY_(clear_flag(w.error_flag, st));
-    TRY_(launch_quad_table(gamma, beta, w.gbt, M, N, K, block, st));
     int cur = 0;
-    TRY_(launch_to_il4(gy, w.g[0], B, d.P, st));
     for (int k = outer - 1; k >= 0; --k) {
         const int kp = nparams > 1 ? k : 0;
         const bool first = k == outer - 1;  // first to be walked back
@@ -202,8 +195,14 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
         const float2 *in_stats = residual ? mr + (size_t)k * S : (k ? mr + (size_t)(k - 1) * S : nullptr);
         const bool kept = stashes && stashes[k];
         if (first || nparams > 1) {
-            TRY_(launch_quad_pack(weights[kp], gamma, scales[kp], w.packed_t, M, N, K, block, true, st));
-            if (replay) TRY_(launch_quad_pack(weights[kp], biases[kp], scales[kp], w.packed, M, N, K, block, false, st));
+            QuadPrepare a{};
+            a.w = weights[kp]; a.b = biases[kp]; a.s = scales[kp]; a.b_t = gamma; a.packed_t = w.packed_t;
+            if (replay) a.packed = w.packed;
+            if (first) {
+                a.gamma = gamma; a.beta = beta; a.gbt = w.gbt;
+                a.x = gy; a.il = w.g[0]; a.B = B;
+            }
+            TRY_(launch_quad_prepare(a, M, N, K, block, st));
         }
         if (!residual)
             TRY_(launch_quad_norm_sums(outs[k], w.g[cur], nullptr, gamma, mr + (size_t)k * S, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
@@ -212,8 +211,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
             QuadStep a{};
             a.packed = w.packed; a.gbt = w.gbt; a.in_il4 = in; a.in_stats = in_stats;
             a.save_h = h;
-            a.error_flag = w.error_flag;
-            a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;
+                a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;
             TRY_(launch_step_fwd_quad(a, act, st));
         }
         QuadReverse r{};
@@ -228,11 +226,10 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
         g.in_il4 = in; g.gbt = w.gbt; g.in_stats = in_stats;
         g.delta = w.delta; g.h = h; g.scale = scales[kp]; g.dsq = w.dsq; g.gpk = w.gpk;
         g.accumulate = nparams == 1 && !first;
-        g.error_flag = w.error_flag;
         g.M = M; g.N = N; g.K = K; g.Q = d.Q; g.inner = inner; g.block = block;
         TRY_(launch_quad_wgrad(g, act, st));
-        if (nparams > 1 || k == 0) TRY_(launch_quad_unpack_grads(w.gpk, gw[kp], gb[kp], gs[kp], M, N, K, d.Q, block, st));
-        TRY_(launch_quad_border(weights[kp], w.dsum, w.g[cur ^ 1], M, N, K, d.Q, block, st));
+        if (nparams > 1 && k > 0) TRY_(launch_quad_finish(w.gpk, gw[kp], gb[kp], gs[kp], nullptr, nullptr, B, M, N, K, block, st));
+        TRY_(launch_quad_border(weights[kp], w.dsum, w.g[cur ^ 1], nullptr, nullptr, M, N, K, d.Q, block, st));
         if (residual) {
             TRY_(launch_quad_norm_sums(in, w.g[cur ^ 1], w.g[cur], gamma, in_stats, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
             TRY_(launch_quad_norm_residual_apply(in, w.g[cur ^ 1], w.g[cur], gamma, in_stats, w.ac, w.g[cur], d.Q, d.P, st));
@@ -240,8 +237,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
             cur ^= 1;
         }
     }
-    TRY_(launch_from_il4(w.g[cur], nullptr, nullptr, nullptr, gx, B, d.P, st));
-    return launch_propagate_flag(w.error_flag, st);
+    return launch_quad_finish(w.gpk, gw[0], gb[0], gs[0], w.g[cur], gx, B, M, N, K, block, st);
 }
 
 }  // extern "C"

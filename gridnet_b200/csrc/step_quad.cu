@@ -42,6 +42,9 @@ struct QuadParams {
     const float2 *in_stats;  // FUSE_IN: [4 Q] (mean, rstd)
     double2 *out_partials;   // [4 Q][nparts]: slot `region` of every row is written; nullptr: not wanted
     int nparts;
+    const float *wsum;       // NORM: the neurons' weight sums, [regions][4][32] vectors
+    float4 *tile_stats;      // NORM: [inner][Q][tiles][QS_COUNT]; nullptr: not wanted
+    float eps;
     float *y;                // IL4; nullptr: not wanted (replay)
     float *save_h;           // SAVE: [inner][Q][P][4]
     int *error_flag;
@@ -51,7 +54,13 @@ struct QuadParams {
 
 // SAVE: keep every iteration's pre-activations for the backward pass (which gets the activations in between from them and
 // the step's input).
-template <int SUB, int ACT, bool FUSE_IN, bool SAVE>
+// NORM: per-block normalisation (the reference's normalize=True, gridnet/backend_torch.py:92-97): the input of an
+// iteration's sums is (tile - mean) / (std + eps) over all cells of the block's tile, the residual stays as it is. A tile
+// belongs to one warp, so the statistics need only shuffles. The landed tile is read once for its mean c and once more
+// to subtract it and to take the sums over its halo, which no iteration changes; from then on the tile holds v - c, so
+// that neither the variance nor sum w v - mean sum w cancels. Each iteration adds up the values it has just computed
+// while they are still in registers.
+template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM>
 __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     step_fwd_quad(const __grid_constant__ CUtensorMap in_map, const QuadParams p)
 {
@@ -80,8 +89,23 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     __syncthreads();
     tmem_fence_after();
     const unsigned tm = tmem_slot + ((unsigned)(quarter * 32) << 16);
+    static_assert(!(NORM && FUSE_IN), "per-block normalisation takes plain input");
 
     const QuadLane<SUB> L(lane);
+    // NORM: the lane's share of its tile's cells, first + STRIDE k; four lanes share a block-4 tile, and the first two
+    // bits of a quarter-warp's tiles are spread over the banks. Bit k of inside: cell k is no halo.
+    constexpr int TILE_CELLS = SUB == 8 ? G::CELLS : 216, STRIDE = SUB == 8 ? 32 : 4, SHARE = (TILE_CELLS + STRIDE - 1) / STRIDE;
+    const int my = L.ysgn < 0, turn = SUB == 8 ? 0 : 2 * (2 * my + L.h);
+    const int first = SUB == 8 ? lane : ((lane >> 1) & 1) + ((lane >> 3) & 1) * 2 + turn;
+    const unsigned tile_off = SUB == 8 ? 0u : (unsigned)(((L.z0 >> 2) * 2 + (L.y0 >> 2)) * 2 + L.h) * (TILE_CELLS * 16u);
+    unsigned long long inside = 0;
+    if (NORM)
+        for (int k = 0; k < SHARE; ++k) {
+            int c = first + STRIDE * k;
+            if (SUB == 4 && c >= TILE_CELLS) c -= TILE_CELLS;
+            const int cx = c % G::SIDE, cy = c / G::SIDE % G::SIDE, cz = c / G::SIDE / G::SIDE;
+            if (cx > 0 && cx < G::SIDE - 1 && cy > 0 && cy < G::SIDE - 1 && cz > 0 && cz < G::SIDE - 1) inside |= 1ull << k;
+        }
     const int nbx = p.K >> 3, nby = p.N >> 3;
     const size_t P = (size_t)p.M * p.N * p.K;
     const long long worker = (long long)blockIdx.x * QUARTERS + quarter, nworkers = (long long)gridDim.x * QUARTERS;
@@ -139,6 +163,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
             __syncwarp();  // tensor memory instructions want the whole warp together
         }
         quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm);
+        if (NORM && role == 0) quad_load_wsum(p.wsum, blk, lane, tm);
         tmem_wait_st();
         if (GB_SMEM) cp_async_wait_all();
         tmem_fence_before();
@@ -192,17 +217,142 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                 wait_tile(i);
             }
 
+            u64 piv[2] = {0, 0}, negm[2], inv[2];
+            float halo[8], fresh[8];  // per sample: sum, sum of squares, relative to the pivot
+            if (NORM) {
+                const unsigned t0 = tile + tile_off;
+                constexpr int BATCH = SUB == 8 ? 16 : 18;
+                auto cell = [&](int k) {
+                    int c = first + STRIDE * k;
+                    if (SUB == 4 && c >= TILE_CELLS) c -= TILE_CELLS;
+                    return t0 + (unsigned)c * 16u;
+                };
+                auto mine = [&](int k) { return SUB == 4 || first + STRIDE * k < TILE_CELLS; };
+                u64 s2[2] = {0, 0}, q2[2] = {0, 0};
+#pragma unroll 1
+                for (int k0 = 0; k0 < SHARE; k0 += BATCH) {
+                    u64 v[BATCH][2];
+#pragma unroll
+                    for (int k = 0; k < BATCH; ++k) {
+                        v[k][0] = v[k][1] = 0;
+                        if (mine(k0 + k)) lds128u(cell(k0 + k), v[k][0], v[k][1]);
+                    }
+#pragma unroll
+                    for (int k = 0; k < BATCH; ++k) {
+                        s2[0] = fadd2(s2[0], v[k][0]);
+                        s2[1] = fadd2(s2[1], v[k][1]);
+                    }
+                }
+                auto spread = [&]() {
+                    unpack2(s2[0], halo[0], halo[1]);
+                    unpack2(s2[1], halo[2], halo[3]);
+                    unpack2(q2[0], halo[4], halo[5]);
+                    unpack2(q2[1], halo[6], halo[7]);
+                    quad_tile_sum8<SUB>(halo, lane);
+                };
+                spread();
+                constexpr float per_cell = 1.0f / TILE_CELLS;
+                piv[0] = pack2(halo[0] * per_cell, halo[1] * per_cell);
+                piv[1] = pack2(halo[2] * per_cell, halo[3] * per_cell);
+                const u64 neg[2] = {fmul2(piv[0], pack2(-1.0f, -1.0f)), fmul2(piv[1], pack2(-1.0f, -1.0f))};
+                s2[0] = s2[1] = 0;
+#pragma unroll 1
+                for (int k0 = 0; k0 < SHARE; k0 += BATCH) {
+                    u64 v[BATCH][2];
+                    const unsigned in = (unsigned)(inside >> k0);
+#pragma unroll
+                    for (int k = 0; k < BATCH; ++k)
+                        if (mine(k0 + k)) lds128u(cell(k0 + k), v[k][0], v[k][1]);
+#pragma unroll
+                    for (int k = 0; k < BATCH; ++k)
+                        if (mine(k0 + k)) {
+                            const float f = in >> k & 1 ? 0.0f : 1.0f;
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) {
+                                v[k][j] = fadd2(v[k][j], neg[j]);
+                                const u64 m = fmul2(v[k][j], pack2(f, f));
+                                s2[j] = fadd2(s2[j], m);
+                                ffma2(q2[j], m, v[k][j]);
+                            }
+                            sts128u(cell(k0 + k), v[k][0], v[k][1]);
+                        }
+                }
+                spread();
+                __syncwarp();
+            }
+
             const unsigned win = tile + L.cell0 * 16u;  // window cell (0, 0, 0) of this lane
             unsigned rows[4];
 #pragma unroll
             for (int ry = 0; ry < 4; ++ry) rows[ry] = win + (unsigned)(ry * L.ysgn * G::ROW * 16);
             const size_t own = ((size_t)q * P + g0) * 4;  // the lane's cells in an IL4 tensor
             const long long zstr = wzs * 4, ystr = wys * 4;
+            // NORM: the sums over the lane's own cells -> over the tile's interior
+            auto sum_fresh = [&](const u64 (&v)[4][4][2]) {
+                u64 s2[2] = {0, 0}, q2[2] = {0, 0};
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int o = 0; o < 4; ++o)
+#pragma unroll
+                        for (int k2 = 0; k2 < 2; ++k2) {
+                            s2[k2] = fadd2(s2[k2], v[n][o][k2]);
+                            ffma2(q2[k2], v[n][o][k2], v[n][o][k2]);
+                        }
+                unpack2(s2[0], fresh[0], fresh[1]);
+                unpack2(s2[1], fresh[2], fresh[3]);
+                unpack2(q2[0], fresh[4], fresh[5]);
+                unpack2(q2[1], fresh[6], fresh[7]);
+                quad_tile_sum8<SUB>(fresh, lane);
+            };
+            auto own_cell = [&](int n, int o) {
+                return win + (unsigned)((1 + o) * L.xsgn * 16 + (1 + (n & 1)) * L.ysgn * G::ROW * 16) + (1 + (n >> 1)) * G::PLANE * 16u;
+            };
+            if (NORM) {
+                u64 v[4][4][2];
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int o = 0; o < 4; ++o) lds128u(own_cell(n, o), v[n][o][0], v[n][o][1]);
+                sum_fresh(v);
+            }
             for (int t = 0; t < p.inner; ++t) {
                 const bool last = t + 1 == p.inner;
+                if (NORM) {
+                    constexpr float per_cell = 1.0f / TILE_CELLS;
+                    float m[4], sd[4], rs[4];
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        m[s] = (halo[s] + fresh[s]) * per_cell;
+                        const float var = fmaxf(fmaf(-m[s], m[s], (halo[4 + s] + fresh[4 + s]) * per_cell), 0.0f);
+                        // approximate square root and reciprocal: a few ulp
+                        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(sd[s]) : "f"(var));
+                        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rs[s]) : "f"(sd[s] + p.eps));
+                    }
+                    negm[0] = pack2(-m[0], -m[1]);
+                    negm[1] = pack2(-m[2], -m[3]);
+                    inv[0] = pack2(rs[0], rs[1]);
+                    inv[1] = pack2(rs[2], rs[3]);
+                    if (SAVE && quad_tile_leader<SUB>(lane)) {
+                        const size_t ntiles = (size_t)nbx * nby * (p.M >> 3) * (SUB == 8 ? 1 : 8);
+                        float4 *to = p.tile_stats + (((size_t)t * p.Q + q) * ntiles + quad_tile_of(L, blk)) * QS_COUNT;
+                        float c[4];
+                        unpack2(piv[0], c[0], c[1]);
+                        unpack2(piv[1], c[2], c[3]);
+                        to[QS_MEAN] = make_float4(c[0] + m[0], c[1] + m[1], c[2] + m[2], c[3] + m[3]);
+                        to[QS_INV] = make_float4(rs[0], rs[1], rs[2], rs[3]);
+                        to[QS_STD] = make_float4(sd[0], sd[1], sd[2], sd[3]);
+                        to[QS_STDEPS] = make_float4(sd[0] + p.eps, sd[1] + p.eps, sd[2] + p.eps, sd[3] + p.eps);
+                    }
+                    __syncwarp();
+                }
                 u64 acc[4][4][2], hold[2] = {0, 0};
                 float *const sh = SAVE ? p.save_h + (size_t)t * p.Q * P * 4 + own : nullptr;
-                quad_stencil<G::PLANE, true>(rows, L.xsgn * 16, tm, acc, [&](int n, int o, float scale, u64 c0, u64 c1) {
+                quad_stencil<G::PLANE, NORM ? NORMED : BIAS>(rows, L.xsgn * 16, tm, acc, negm, [&](int n, int o, float scale, float bias, u64 c0, u64 c1) {
+                    if (NORM) {
+                        acc[n][o][0] = ffma2r(acc[n][o][0], inv[0], pack2(bias, bias));
+                        acc[n][o][1] = ffma2r(acc[n][o][1], inv[1], pack2(bias, bias));
+                    }
                     if (SAVE) {  // two neighbours at a time
                         if (o & 1)
                             stg256(sh + (n >> 1) * zstr + (n & 1) * ystr + 8 * ((o >> 1) ^ L.h), L.h ? acc[n][o][0] : hold[0],
@@ -216,16 +366,21 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                 __syncwarp();  // every lane has read its window
                 if (!last) {
 #pragma unroll
-                    for (int o = 0; o < 4; ++o) {
-                        const unsigned a = win + (unsigned)((1 + o) * L.xsgn * 16) + (unsigned)(L.ysgn * G::ROW * 16) + G::PLANE * 16u;
+                    for (int o = 0; o < 4; ++o)
 #pragma unroll
-                        for (int n = 0; n < 4; ++n)
-                            sts128u(a + (unsigned)((n & 1) * L.ysgn * G::ROW * 16) + (n >> 1) * G::PLANE * 16u, acc[n][o][0], acc[n][o][1]);
-                    }
+                        for (int n = 0; n < 4; ++n) sts128u(own_cell(n, o), acc[n][o][0], acc[n][o][1]);
+                    if (NORM) sum_fresh(acc);
                     __syncwarp();
                 } else {
                     if (lane == 0 && i + NBUF < cnt) issue(i + NBUF);  // the tile is dead: fetch the next one
                     __syncwarp();
+                    if (NORM)
+#pragma unroll
+                        for (int n = 0; n < 4; ++n)
+#pragma unroll
+                            for (int o = 0; o < 4; ++o)
+#pragma unroll
+                                for (int k2 = 0; k2 < 2; ++k2) acc[n][o][k2] = fadd2(acc[n][o][k2], piv[k2]);
                     if (p.y) quad_store(p.y + own, zstr, ystr, L.h, acc);
                     if (p.out_partials) {
                         u64 s2[2] = {0, 0}, q2[2] = {0, 0};
@@ -263,19 +418,6 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
 }
 
 // ---- layout conversion at the ends of a loop --------------------------------------------------------------
-// [B, P] -> [Q][P][4]; samples beyond B are zero. One cell per thread and step: four coalesced 4-byte reads, one
-// coalesced 16-byte write.
-__global__ void __launch_bounds__(256) to_il4_k(const float *__restrict__ x, float4 *__restrict__ il, int B, size_t P)
-{
-    const size_t c = (size_t)blockIdx.x * 256 + threadIdx.x;
-    if (c >= P) return;
-    const int q = blockIdx.y;
-    float v[4];
-#pragma unroll
-    for (int s = 0; s < 4; ++s) v[s] = 4 * q + s < B ? x[(size_t)(4 * q + s) * P + c] : 0.0f;
-    il[(size_t)q * P + c] = make_float4(v[0], v[1], v[2], v[3]);
-}
-
 // IL4 -> [B, P], normalised on the way when statistics are given
 __global__ void __launch_bounds__(256) from_il4_k(const float4 *__restrict__ il, const float2 *__restrict__ stats,
                                                   const float *__restrict__ gamma, const float *__restrict__ beta,
@@ -302,14 +444,27 @@ __global__ void __launch_bounds__(256) from_il4_k(const float4 *__restrict__ il,
         }
 }
 
+// [B, P] -> [Q][P][4]; samples beyond B are zero. One cell per thread and step: four coalesced 4-byte reads, one
+// coalesced 16-byte write.
+__device__ __forceinline__ void to_il4(const float *__restrict__ x, float4 *__restrict__ il, int B, size_t P, int q, size_t part)
+{
+    const size_t c = part * 256 + threadIdx.x;
+    if (c >= P) return;
+    float v[4];
+#pragma unroll
+    for (int s = 0; s < 4; ++s) v[s] = 4 * q + s < B ? x[(size_t)(4 * q + s) * P + c] : 0.0f;
+    il[(size_t)q * P + c] = make_float4(v[0], v[1], v[2], v[3]);
+}
+
 // Parameters in the order of the stencil: vector v of a region is, for every lane, the four x-neighbouring weights of
 // one (neuron row, tap), v = 0 .. 107 in the order of the uses in quad_stencil (three x-taps each), then the four rows
 // of b, then of s. TRANS: the weights of the backward sum, in which a cell collects from the neurons of its own block
-// that read it: the neuron at tap t sees the cell through its tap 26 - t; zero across the block's border. One CTA per
-// region; reads are 16-byte pieces, writes whole lines.
+// that read it: the neuron at tap t sees the cell through its tap 26 - t; zero across the block's border. Four CTAs of 256 threads per
+// region, so that small grids fill the GPU; reads are 16-byte pieces, writes whole lines.
+constexpr int kPackCtas = 4;
 template <int SUB, bool TRANS>
-__global__ void __launch_bounds__(256) quad_pack_k(const float *__restrict__ w, const float *__restrict__ b, const float *__restrict__ s,
-                                                   float *__restrict__ packed, int M, int N, int K)
+__device__ __forceinline__ void quad_pack(const float *__restrict__ w, const float *__restrict__ b, const float *__restrict__ s,
+                                          float *__restrict__ packed, int M, int N, int K, int cta)
 {
     __shared__ unsigned char uses[36];  // (a * 3 + b) | n << 4
     if (threadIdx.x == 0) {
@@ -324,14 +479,16 @@ __global__ void __launch_bounds__(256) quad_pack_k(const float *__restrict__ w, 
     __syncthreads();
     const int lane = threadIdx.x & 31;
     const QuadLane<SUB> L(lane);
-    const int nbx = K >> 3, nby = N >> 3, blk = blockIdx.x;
+    const int nbx = K >> 3, nby = N >> 3, blk = cta / kPackCtas;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t P = (size_t)M * N * K;
     const size_t g0 = ((size_t)(bz * 8 + L.z0) * N + (by * 8 + L.y0)) * K + bx * 8 + 4 * L.h;
     const long long zs = (long long)N * K, ys = (long long)L.ysgn * K;
     float4 *out = reinterpret_cast<float4 *>(packed + (size_t)blk * quad::PACK_F) + lane;
-#pragma unroll 4
-    for (int v = threadIdx.x >> 5; v < quad::VECS; v += 8) {
+#pragma unroll
+    for (int i = 0; i < (quad::VECS + 8 * kPackCtas - 1) / (8 * kPackCtas); ++i) {
+        const int v = (i * kPackCtas + cta % kPackCtas) * 8 + (threadIdx.x >> 5);
+        if (v >= quad::VECS) break;
         int n;
         float4 r;
         if (v < 108) {
@@ -369,13 +526,37 @@ __global__ void __launch_bounds__(256) quad_pack_k(const float *__restrict__ w, 
     }
 }
 
+// The sum of every neuron's 27 weights, for per-block normalisation: vector n of a region is, for every lane, its neuron
+// row n. One warp per row, two
+// regions per CTA.
+template <int SUB>
+__device__ __forceinline__ void quad_wsum(const float *__restrict__ w, float4 *__restrict__ wsum, int M, int N, int K, int cta)
+{
+    const int lane = threadIdx.x & 31, n = (threadIdx.x >> 5) & 3;
+    const QuadLane<SUB> L(lane);
+    const int nbx = K >> 3, nby = N >> 3, blk = 2 * cta + (threadIdx.x >> 7);
+    if (blk >= (M >> 3) * nby * nbx) return;
+    const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
+    const size_t P = (size_t)M * N * K;
+    const float *src = w + ((size_t)(bz * 8 + L.z0 + (n >> 1)) * N + (by * 8 + L.y0 + L.ysgn * (n & 1))) * K + bx * 8 + 4 * L.h;
+    const bool al = (reinterpret_cast<uintptr_t>(w) & 15) == 0;
+    float4 r = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int t = 0; t < 27; ++t) {
+        const float *a = src + (size_t)t * P;
+        const float4 v = al ? *reinterpret_cast<const float4 *>(a) : make_float4(a[0], a[1], a[2], a[3]);
+        r.x += v.x, r.y += v.y, r.z += v.z, r.w += v.w;
+    }
+    wsum[(size_t)blk * 128 + (threadIdx.x & 127)] = L.h ? make_float4(r.w, r.z, r.y, r.x) : r;
+}
+
 // (gamma, beta) of every tile cell of every region, in the order of the tile buffer
 template <int SUB>
-__global__ void __launch_bounds__(256) quad_table_k(const float *__restrict__ gamma, const float *__restrict__ beta,
-                                                    float2 *__restrict__ gbt, int M, int N, int K)
+__device__ __forceinline__ void quad_table(const float *__restrict__ gamma, const float *__restrict__ beta, float2 *__restrict__ gbt, int M,
+                                           int N, int K, int cta)
 {
     using G = QuadGeo<SUB>;
-    const int nbx = K >> 3, nby = N >> 3, blk = blockIdx.x;
+    const int nbx = K >> 3, nby = N >> 3, blk = cta;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     for (int c = threadIdx.x; c < G::CELLS; c += 256) {
         int cz, cy, cx;
@@ -388,6 +569,26 @@ __global__ void __launch_bounds__(256) quad_table_k(const float *__restrict__ ga
         }
         gbt[(size_t)blk * G::CELLS + c] = gb;
     }
+}
+
+// Everything that has to be re-ordered before a step or a loop, in one launch (a launch costs the host as much as the
+// kernel of a small grid takes): CTAs first .. first + n of job j do that job.
+struct PrepareArgs {
+    QuadPrepare a;
+    int M, N, K;
+    unsigned end[5];  // last CTA + 1 of: pack, transposed pack, weight sums, table, conversion
+    unsigned parts;   // conversion: CTAs per quad
+};
+template <int SUB>
+__global__ void __launch_bounds__(256) quad_prepare_k(const PrepareArgs p)
+{
+    const unsigned c = blockIdx.x;
+    const QuadPrepare &a = p.a;
+    if (c < p.end[0]) quad_pack<SUB, false>(a.w, a.b, a.s, a.packed, p.M, p.N, p.K, (int)c);
+    else if (c < p.end[1]) quad_pack<SUB, true>(a.w, a.b_t, a.s, a.packed_t, p.M, p.N, p.K, (int)(c - p.end[0]));
+    else if (c < p.end[2]) quad_wsum<SUB>(a.w, reinterpret_cast<float4 *>(a.wsum), p.M, p.N, p.K, (int)(c - p.end[1]));
+    else if (c < p.end[3]) quad_table<SUB>(a.gamma, a.beta, a.gbt, p.M, p.N, p.K, (int)(c - p.end[2]));
+    else to_il4(a.x, reinterpret_cast<float4 *>(a.il), a.B, (size_t)p.M * p.N * p.K, (int)((c - p.end[3]) / p.parts), (c - p.end[3]) % p.parts);
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------
@@ -422,13 +623,6 @@ int quad_make_map(CUtensorMap *map, const float *il, int M, int N, int K, int Q,
     return GN_OK;
 }
 
-int launch_to_il4(const float *x, float *il, int B, long long P, cudaStream_t st)
-{
-    dim3 grid((unsigned)((P + 255) / 256), (unsigned)((B + 3) / 4));
-    to_il4_k<<<grid, 256, 0, st>>>(x, reinterpret_cast<float4 *>(il), B, (size_t)P);
-    return check_launch("to_il4");
-}
-
 int launch_from_il4(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, long long P,
                     cudaStream_t st)
 {
@@ -437,32 +631,34 @@ int launch_from_il4(const float *il, const float2 *stats, const float *gamma, co
     return check_launch("from_il4");
 }
 
+size_t quad_tiles(int M, int N, int K, int block) { return (size_t)(M / block) * (N / block) * (K / block); }
+size_t quad_stats_vectors(int M, int N, int K, int Q, int inner, int block) { return (size_t)inner * Q * quad_tiles(M, N, K, block) * QS_COUNT; }
 size_t quad_packed_floats(int M, int N, int K) { return (size_t)(M / 8) * (N / 8) * (K / 8) * quad::PACK_F; }
 
-int launch_quad_pack(const float *w, const float *b, const float *s, float *packed, int M, int N, int K, int block, bool transposed,
-                     cudaStream_t st)
+int launch_quad_prepare(const QuadPrepare &a, int M, int N, int K, int block, cudaStream_t st)
 {
     const unsigned regions = (unsigned)((M / 8) * (N / 8) * (K / 8));
-    if (block == 8 && transposed) quad_pack_k<8, true><<<regions, 256, 0, st>>>(w, b, s, packed, M, N, K);
-    else if (block == 8) quad_pack_k<8, false><<<regions, 256, 0, st>>>(w, b, s, packed, M, N, K);
-    else if (transposed) quad_pack_k<4, true><<<regions, 256, 0, st>>>(w, b, s, packed, M, N, K);
-    else quad_pack_k<4, false><<<regions, 256, 0, st>>>(w, b, s, packed, M, N, K);
-    return check_launch("quad_pack");
+    PrepareArgs p{a, M, N, K, {}, (unsigned)(((long long)M * N * K + 255) / 256)};
+    const unsigned long long jobs[5] = {a.packed ? regions * kPackCtas : 0u, a.packed_t ? regions * kPackCtas : 0u,
+                                        a.wsum ? (regions + 1) / 2 : 0u, a.gbt ? regions : 0u,
+                                        a.il ? (unsigned long long)p.parts * ((a.B + 3) / 4) : 0u};
+    unsigned long long n = 0;
+    for (int j = 0; j < 5; ++j) {
+        n += jobs[j];
+        if (n >= 1ull << 31) return GN_ERR_UNSUPPORTED;
+        p.end[j] = (unsigned)n;
+    }
+    if (n == 0) return GN_OK;
+    if (block == 8) quad_prepare_k<8><<<(unsigned)n, 256, 0, st>>>(p);
+    else quad_prepare_k<4><<<(unsigned)n, 256, 0, st>>>(p);
+    return check_launch("quad_prepare");
 }
 
-int launch_quad_table(const float *gamma, const float *beta, float2 *gbt, int M, int N, int K, int block, cudaStream_t st)
-{
-    const unsigned regions = (unsigned)((M / 8) * (N / 8) * (K / 8));
-    if (block == 8) quad_table_k<8><<<regions, 256, 0, st>>>(gamma, beta, gbt, M, N, K);
-    else quad_table_k<4><<<regions, 256, 0, st>>>(gamma, beta, gbt, M, N, K);
-    return check_launch("quad_table");
-}
-
-template <int SUB, int ACT, bool FUSE_IN, bool SAVE>
+template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM = false>
 static int launch_quad_one(const CUtensorMap &map, const QuadParams &p, unsigned ctas, cudaStream_t st)
 {
     using G = QuadGeo<SUB>;
-    auto kern = step_fwd_quad<SUB, ACT, FUSE_IN, SAVE>;
+    auto kern = step_fwd_quad<SUB, ACT, FUSE_IN, SAVE, NORM>;
     // tiles; block 8 with normalise-on-load also a (gamma, beta) table per team
     constexpr int smem = quad::QUARTERS * G::NBUF * G::BUF_BYTES + (SUB == 8 && FUSE_IN ? quad::QUARTERS * G::CELLS * 8 : 0);
     static_assert(smem <= 232448 - 1024 - 256, "shared memory budget of one SM");
@@ -481,6 +677,7 @@ static int launch_quad_one(const CUtensorMap &map, const QuadParams &p, unsigned
 template <int SUB, int ACT>
 static int launch_quad_act(const CUtensorMap &map, const QuadParams &p, unsigned ctas, cudaStream_t st)
 {
+    if (p.wsum) return p.save_h ? launch_quad_one<SUB, ACT, false, true, true>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, false, true>(map, p, ctas, st);
     if (p.save_h) return p.in_stats ? launch_quad_one<SUB, ACT, true, true>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, true>(map, p, ctas, st);
     return p.in_stats ? launch_quad_one<SUB, ACT, true, false>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, false>(map, p, ctas, st);
 }
@@ -498,6 +695,7 @@ static int launch_quad_sub(const CUtensorMap &map, const QuadParams &p, unsigned
 
 int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
 {
+    if (a.wsum && (a.in_stats || !a.save_h != !a.tile_stats)) return GN_ERR_UNSUPPORTED;
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
     const int rc = quad_make_map(&map, a.in_il4, a.M, a.N, a.K, a.Q, a.block);
@@ -506,6 +704,7 @@ int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
     p.packed = a.packed;
     p.gbt = a.gbt; p.in_stats = a.in_stats;
     p.out_partials = a.out_partials; p.nparts = a.nparts;
+    p.wsum = a.wsum; p.tile_stats = a.tile_stats; p.eps = a.eps;
     p.y = a.out_il4; p.save_h = a.save_h;
     p.error_flag = a.error_flag ? a.error_flag : device_status_ptr();
     p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;

@@ -29,17 +29,29 @@ namespace gn {
 namespace quadrev {
 // delta tile of a region: 10 planes of 8 rows of 10 cells. The outer planes and columns are zero; rows beyond the region
 // are read as the nearest row and meet zero weights.
-// Before an item, the gradient of its output is fetched into the tile's own cells; pre-activations arrive in a staging area.
-constexpr int ROW = 10, PLANE = 80, CELLS = 800, TILE_BYTES = CELLS * 16, STAGE_BYTES = 512 * 16;
-constexpr int WARP_BYTES = TILE_BYTES + STAGE_BYTES, TEAM = 2;
-constexpr int SMEM_BYTES = 4 * TEAM * WARP_BYTES;
+// Before an item, the gradient of its output is fetched into the tile's own cells; pre-activations arrive in a staging area,
+// with per-block normalisation the activations in a second one and the iteration's statistics behind it. The tiles of
+// neighbouring warps share a zero plane, without which that would not fit.
+constexpr int ROW = 10, PLANE = 80, CELLS = 800, TILE_BYTES = 9 * PLANE * 16, STAGE_BYTES = 512 * 16, TEAM = 2, WARPS = 4 * TEAM;
+constexpr int TILES_BYTES = WARPS * TILE_BYTES + PLANE * 16;
+constexpr int STATS_BYTES = 8 * QS_COUNT * 16;  // block 4: eight tiles
+enum In { PLAIN, GRID_NORM /* the output went through a whole-grid norm */, BLOCK_NORM /* the sums' inputs were normalised per block */ };
+template <In IN>
+struct Bytes {
+    static constexpr int STAGE = IN == BLOCK_NORM ? 2 * STAGE_BYTES + STATS_BYTES : STAGE_BYTES, SMEM = TILES_BYTES + WARPS * STAGE;
+    static_assert(SMEM <= 232448 - 1024, "shared memory of one SM");
+};
 }  // namespace quadrev
 
 struct QuadRevParams {
-    const float *packed;           // transposed weights; NORM_IN: the norm's weight in the place of the biases
-    const float *g;                // gradient of the step's output (NORM_IN: of its normalised output), IL4
-    const float *raw;              // NORM_IN: the step's output, IL4
-    const float2 *stats, *ac;      // NORM_IN: [4 Q] (mean, rstd) and (sum g gamma, sum g gamma xhat) / P
+    const float *packed;           // transposed weights; GRID_NORM: the norm's weight in the place of the biases
+    const float *g;                // gradient of the step's output (GRID_NORM: of its normalised output), IL4
+    const float *raw;              // GRID_NORM, BLOCK_NORM: the step's output, IL4
+    const float2 *stats, *ac;      // GRID_NORM: [4 Q] (mean, rstd) and (sum g gamma, sum g gamma xhat) / P
+    const float *wsum;             // BLOCK_NORM: as in step_fwd_quad
+    const float4 *tile_stats;      // BLOCK_NORM: [inner][Q][tiles][QS_COUNT]
+    float4 *hterm;                 // BLOCK_NORM: [Q][tiles][2] F, E
+    int B;
     const float *h;                // [inner] pre-activations, IL4
     float *delta, *dsum, *gx;      // [inner], one, one IL4 tensors
     float *dsq;                    // [Q][P] gradient terms of the residual scale, summed over the quad and the iterations
@@ -72,17 +84,27 @@ __device__ __forceinline__ void act_both2(u64 h, u64 &f, u64 &d)
     d = pack2(d0, d1);
 }
 
-template <int SUB, int ACT, bool NORM_IN>
+// BLOCK_NORM: the input of iteration t's sums was (tile - mean) inv with inv = 1 / (std + eps). With Gin the gradient of that
+// input, a tile cell's gradient is inv Gin - P1 - P2 (x - mean), P1 = inv sum(Gin) / cells, P2 = inv sum(Gin in) /
+// (cells std), and both sums are sums over the block's neurons: sum(Gin) = sum raw W (W the neuron's weights added up), sum(Gin
+// in) = sum raw (h - bias), raw the delta before it is scaled by inv. The deltas that are stored and summed are the scaled
+// ones, so the other kernels see inv Gin. The lanes that share a tile add the two sums up by shuffles; what the halo
+// cells owe, F + E x with F = sum_t (P1 - P2 mean), E = sum_t P2, goes (negated) to the border kernel. The activations x_t are
+// walked back from the step's output, x_t = x_(t+1) - scale act(h_t).
+template <int SUB, int ACT, quadrev::In IN>
 __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
 {
     using namespace quad;
     using namespace quadrev;
+    constexpr bool NORM_IN = IN == GRID_NORM, BN = IN == BLOCK_NORM;
+    constexpr float PER_CELL = SUB == 8 ? 1.0f / 1000 : 1.0f / 216;
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ unsigned tmem_slot;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int quarter = warp & 3, role = warp >> 2;
     if (warp == 0) tmem_alloc_all(&tmem_slot);
-    const unsigned tile = smem_u32(smem) + warp * WARP_BYTES, stage = tile + TILE_BYTES;
+    const unsigned tile = smem_u32(smem) + warp * TILE_BYTES, stage = smem_u32(smem) + TILES_BYTES + warp * Bytes<IN>::STAGE;
+    const unsigned stage_x = stage + STAGE_BYTES, stage_s = stage_x + STAGE_BYTES;  // BN
     for (int c = lane; c < CELLS; c += 32) sts128u(tile + c * 16, 0, 0);
     tmem_fence_before();
     __syncthreads();
@@ -117,7 +139,18 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
         const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
         return ((size_t)q * P + ((size_t)(bz * 8) * p.N + by * 8) * p.K + bx * 8) * 4;
     };
-    auto fetch_h = [&](size_t corner, int t) { quad_stage<0, 8>(stage, p.h + (size_t)t * T4 + corner, zstr, p.K, lane); };
+    const size_t ntiles = (size_t)nbx * nby * (p.M >> 3) * (SUB == 8 ? 1 : 8);
+    // pre-activations of iteration t of the team's item i (BN: and the statistics of its tiles)
+    auto fetch_h = [&](int i, size_t corner, int t) {
+        quad_stage<0, 8>(stage, p.h + (size_t)t * T4 + corner, zstr, p.K, lane);
+        if (BN) {
+            const long long n = n0 + i;
+            const int blk = (int)(n / p.Q), q = (int)(n - (long long)blk * p.Q);
+            const float4 *src = p.tile_stats + (((size_t)t * p.Q + q) * ntiles + (size_t)blk * (SUB == 8 ? 1 : 8)) * QS_COUNT;
+            if (lane < (SUB == 8 ? 1 : 8) * QS_COUNT) cp_async16(stage_s + lane * 16, src + lane);
+        }
+    };
+    auto fetch_x = [&](size_t corner) { quad_stage<0, 8>(stage_x, p.raw + corner, zstr, p.K, lane); };
     auto fetch_g = [&](size_t corner) {
         const int y = lane >> 3, x = lane & 7;
         const float *src = p.g + corner + ((long long)y * p.K + x) * 4;
@@ -129,7 +162,8 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
     __syncwarp();
     if (role < cnt) {
         fetch_g(corner_of(role));
-        fetch_h(corner_of(role), p.inner - 1);
+        fetch_h(role, corner_of(role), p.inner - 1);
+        if (BN) fetch_x(corner_of(role));
     }
 
     int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
@@ -141,6 +175,7 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
             tmem_fence_after();
         }
         quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm);
+        if (BN && role == 0) quad_load_wsum(p.wsum, blk, lane, tm);
         tmem_wait_st();
         tmem_fence_before();
         team_sync<TEAM>(quarter);
@@ -150,6 +185,7 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
             for (int c = role * 32 + lane; c < PACK_F * 4 / 128; c += 32 * TEAM) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + c * 128));
             __syncwarp();
         }
+        const unsigned my_stats = stage_s + (SUB == 8 ? 0 : (unsigned)quad_tile_of(L, 0)) * (QS_COUNT * 16);
         for (int k = (role + TEAM - i0 % TEAM) % TEAM; k < here; k += TEAM) {
             const int i = i0 + k, q = q0 + k;
             const size_t corner = corner_of(i), own = corner + to_own;
@@ -200,21 +236,38 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
                     dsum[n][o][0] = dsum[n][o][1] = 0;
                     dsa[n][o] = 0.0f;
                 }
+            u64 hf[2] = {0, 0}, he[2] = {0, 0};  // BN: F and E
             for (int t = p.inner - 1; t >= 0; --t) {
                 float sc[16];
-                tmem_ld16(tm + COL_SCALE, sc);
+                if (!BN) tmem_ld16(tm + COL_SCALE, sc);
                 cp_async_wait_all();
-                tmem_wait_ld16(sc);
+                if (!BN) tmem_wait_ld16(sc);
                 __syncwarp();  // everyone's part of h_t has landed
+                u64 inv[2] = {0, 0}, pa[2] = {0, 0}, pc[2] = {0, 0};
+                if (BN) lds128u(my_stats + QS_INV * 16, inv[0], inv[1]);
                 // Row by row: loads, arithmetic and stores of a row of four cells each overlap with themselves (cell by cell,
                 // a load waits for the store before it); more rows at a time spill (0.64 ms by one row, 0.67 by two, 0.71 by
                 // four, at 128^3 with two inner iterations and batch 32).
                 float *const dt = p.delta + (size_t)t * T4 + own;
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
-                    u64 h[4][2];
+                    u64 h[4][2], x[4][2];
+                    float bw[16];  // BN: bias and scale, weight sum
+                    if (BN) {
+                        tmem_ld4(tm + COL_BIAS + n * 4, bw);
+                        tmem_ld4(tm + COL_SCALE + n * 4, bw + 4);
+                        tmem_ld4(tm + COL_WSUM + n * 4, bw + 8);
+                    }
 #pragma unroll
-                    for (int o = 0; o < 4; ++o) lds128u(stage + S.at(n, o), h[o][0], h[o][1]);
+                    for (int o = 0; o < 4; ++o) {
+                        lds128u(stage + S.at(n, o), h[o][0], h[o][1]);
+                        if (BN) lds128u(stage_x + S.at(n, o), x[o][0], x[o][1]);
+                    }
+                    if (BN) {
+                        tmem_wait_ld12(bw);
+#pragma unroll
+                        for (int o = 0; o < 4; ++o) sc[n * 4 + o] = bw[4 + o];
+                    }
 #pragma unroll
                     for (int o = 0; o < 4; ++o) {
                         u64 f0, f1, d0, d1;
@@ -224,8 +277,22 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
                         unpack2(ffma2r(f0, g[n][o][0], fmul2(f1, g[n][o][1])), s0, s1);
                         dsa[n][o] += s0 + s1;
                         const u64 s2 = pack2(sc[n * 4 + o], sc[n * 4 + o]);
-                        h[o][0] = fmul2(fmul2(d0, g[n][o][0]), s2);
-                        h[o][1] = fmul2(fmul2(d1, g[n][o][1]), s2);
+                        if (BN) {
+                            const u64 nb = pack2(-bw[o], -bw[o]), w2 = pack2(bw[8 + o], bw[8 + o]), ns = pack2(-sc[n * 4 + o], -sc[n * 4 + o]);
+                            const u64 r0 = fmul2(fmul2(d0, g[n][o][0]), s2), r1 = fmul2(fmul2(d1, g[n][o][1]), s2);
+                            ffma2(pa[0], r0, w2);
+                            ffma2(pa[1], r1, w2);
+                            ffma2(pc[0], r0, fadd2(h[o][0], nb));
+                            ffma2(pc[1], r1, fadd2(h[o][1], nb));
+                            ffma2(x[o][0], f0, ns);
+                            ffma2(x[o][1], f1, ns);
+                            sts128u(stage_x + S.at(n, o), x[o][0], x[o][1]);
+                            h[o][0] = fmul2(r0, inv[0]);
+                            h[o][1] = fmul2(r1, inv[1]);
+                        } else {
+                            h[o][0] = fmul2(fmul2(d0, g[n][o][0]), s2);
+                            h[o][1] = fmul2(fmul2(d1, g[n][o][1]), s2);
+                        }
                         dsum[n][o][0] = fadd2(dsum[n][o][0], h[o][0]);
                         dsum[n][o][1] = fadd2(dsum[n][o][1], h[o][1]);
                     }
@@ -234,13 +301,64 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
 #pragma unroll
                     for (int j = 0; j < 2; ++j) quad_store2(dt, n, j, zstr, ystr, L.h, h);
                 }
+                if (BN) {
+                    u64 mean[2], sd[2];
+                    lds128u(my_stats + QS_MEAN * 16, mean[0], mean[1]);
+                    lds128u(my_stats + QS_STD * 16, sd[0], sd[1]);
+                    float v[8];
+                    unpack2(pa[0], v[0], v[1]);
+                    unpack2(pa[1], v[2], v[3]);
+                    unpack2(pc[0], v[4], v[5]);
+                    unpack2(pc[1], v[6], v[7]);
+                    quad_tile_sum8<SUB>(v, lane);
+                    u64 np1[2], np2[2];  // -(P1 - P2 mean), -P2
+#pragma unroll
+                    for (int j = 0; j < 2; ++j) {
+                        float i0, i1, s0, s1;
+                        unpack2(inv[j], i0, i1);
+                        unpack2(sd[j], s0, s1);
+                        // samples that only fill up the quad have no deviation to divide by
+                        const float e0 = 4 * q + 2 * j < p.B ? -v[4 + 2 * j] * i0 / (s0 * (1.0f / PER_CELL)) : 0.0f;
+                        const float e1 = 4 * q + 2 * j + 1 < p.B ? -v[5 + 2 * j] * i1 / (s1 * (1.0f / PER_CELL)) : 0.0f;
+                        np2[j] = pack2(e0, e1);
+                        const u64 p1 = pack2(v[2 * j] * i0 * -PER_CELL, v[2 * j + 1] * i1 * -PER_CELL);
+                        np1[j] = ffma2r(fmul2(np2[j], pack2(-1.0f, -1.0f)), mean[j], p1);
+                        hf[j] = fadd2(hf[j], np1[j]);
+                        he[j] = fadd2(he[j], np2[j]);
+                    }
+#pragma unroll
+                    for (int n = 0; n < 4; ++n) {
+                        u64 x[4][2];
+#pragma unroll
+                        for (int o = 0; o < 4; ++o) lds128u(stage_x + S.at(n, o), x[o][0], x[o][1]);
+#pragma unroll
+                        for (int o = 0; o < 4; ++o)
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) g[n][o][j] = fadd2(g[n][o][j], ffma2r(x[o][j], np2[j], np1[j]));
+                    }
+                }
                 __syncwarp();  // the delta tile is complete, h_t has been read
-                if (t > 0) fetch_h(corner, t - 1);
-                else if (i + TEAM < cnt) fetch_h(corner_of(i + TEAM), p.inner - 1);
-                quad_stencil<PLANE, false>(rows, dx, tm, g, [](int, int, float, u64, u64) {});
+                if (t > 0) {
+                    fetch_h(i, corner, t - 1);
+                } else if (i + TEAM < cnt) {
+                    fetch_h(i + TEAM, corner_of(i + TEAM), p.inner - 1);
+                    if (BN) fetch_x(corner_of(i + TEAM));
+                }
+                quad_stencil<PLANE, ADD>(rows, dx, tm, g, inv, [](int, int, float, float, u64, u64) {});
                 __syncwarp();  // ... and has been read
             }
             if (i + TEAM < cnt) fetch_g(corner_of(i + TEAM));
+            if (BN && quad_tile_leader<SUB>(lane)) {
+                float4 *to = p.hterm + ((size_t)q * ntiles + quad_tile_of(L, blk)) * 2;
+                float v[8];
+                unpack2(hf[0], v[0], v[1]);
+                unpack2(hf[1], v[2], v[3]);
+                unpack2(he[0], v[4], v[5]);
+                unpack2(he[1], v[6], v[7]);
+                to[0] = make_float4(v[0], v[1], v[2], v[3]);
+                to[1] = make_float4(v[4], v[5], v[6], v[7]);
+            }
+            __syncwarp();
             quad_store(p.gx + own, zstr, ystr, L.h, g);
             quad_store(p.dsum + own, zstr, ystr, L.h, dsum);
             // four x-neighbours at a time, in ascending order
@@ -277,7 +395,8 @@ struct Lay {
     static constexpr int NT = SUB == 8 ? 2 : 1;
     static constexpr int TILE = (QuadGeo<SUB>::BUF_BYTES + 127) / 128 * 128;
     static constexpr int GB = NT * TILE + 3 * OWN;  // normalise-on-load: the region's (gamma, beta) table
-    static constexpr int smem(bool fuse) { return GB + (fuse ? QuadGeo<SUB>::CELLS * 8 : 0); }
+    static constexpr int NSTAT = (SUB == 8 ? 1 : 8) * QS_COUNT;  // per-block normalisation, there: two iterations' statistics
+    static constexpr int smem(bool fuse, bool norm) { return GB + (fuse ? QuadGeo<SUB>::CELLS * 8 : 0) + (norm ? 2 * NSTAT * 16 : 0); }
 };
 // thread -> patch. Block 8: lanes of a quarter-warp are the eight x; block 4: four x and two y patches (two rows of six
 // cells further is four banks further)
@@ -308,13 +427,17 @@ struct QuadWgradParams {
     const float *delta, *h;  // [inner] IL4
     const float *scale;      // [M][N][K]
     const float *dsq;        // [Q][P]
+    const float4 *tile_stats;  // NORM: [inner][Q][tiles][QS_COUNT]
     float *gpk;              // [chunks][regions][GRAD_F]
     int accumulate;          // add to what is there
     int *error_flag;
     int M, N, K, Q, inner, qpc;
 };
 
-template <int SUB, int ACT, bool FUSE_IN>
+// NORM: per-block normalisation. The deltas are already scaled by 1 / (std + eps). The tile is kept relative to its mean before the
+// first iteration, v - c, and sum delta (v - mean_t) = sum delta (v - c) - sum delta (mean_t - c): the second sum is one
+// number per neuron, taken off all its 27 sums at the end. The bias gradient wants the unscaled delta back.
+template <int SUB, int ACT, bool FUSE_IN, bool NORM>
 __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(const __grid_constant__ CUtensorMap in_map, const QuadWgradParams p)
 {
     using namespace quadwg;
@@ -358,6 +481,12 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
 #pragma unroll
         for (int n = 0; n < 4; ++n) cp_async16(dst + n * (THREADS * 16), src + ((n >> 1) * zs + (n & 1) * (size_t)p.K) * 4);
     };
+    const unsigned stats0 = tiles + Y::GB;  // NORM: [2][tile][QS_COUNT]
+    const unsigned my_tile = SUB == 8 ? 0u : (unsigned)(((T.zp >> 1) * 2 + (T.yp >> 1)) * 2 + (T.x >> 2)) * (QS_COUNT * 16);
+    auto fetch_stats = [&](int buf, int q, int it) {
+        if (NORM && tid < Y::NSTAT)
+            cp_async16(stats0 + buf * (Y::NSTAT * 16) + tid * 16, p.tile_stats + (((size_t)it * p.Q + q) * gridDim.x + blk) * Y::NSTAT + tid);
+    };
     auto at = [&](const float *t, int q, int it) { return t + (size_t)it * T4 + ((size_t)q * P + g0) * 4; };
 
     // sums: sg[dy = 0 at ry = 0, dy = 1 at ry = 3][dz][a][c], sp[ry = 1, 2][dz][a][c] = (dy = 0, dy = 1)
@@ -375,6 +504,7 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                     sp[i][j][a][c] = 0;
                 }
     u64 db[2] = {0, 0}, ds[2] = {0, 0};  // [dz]: (dy = 0, dy = 1)
+    u64 off[2] = {0, 0};                 // NORM: sum delta (mean_t - c)
 
     int buf_x = 0, buf_d = 0;
     unsigned landed = 0;  // bit b: phase of tile b's barrier
@@ -387,6 +517,7 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
     }
     if (tid == 0) issue(q0, 0);
     fetch(stage_d, at(p.delta, q0, 0));
+    fetch_stats(0, q0, 0);
     if (p.inner > 1) fetch(stage_h, at(p.h, q0, 0));
     const unsigned own0 = (unsigned)(T.cell0 + G::PLANE + G::ROW + 1) * 16u;
 
@@ -399,8 +530,11 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
         if (!mbar_wait_bounded(bar0 + 8 * buf_x, (landed >> buf_x) & 1u, kSpin)) failed = true;
         landed ^= 1u << buf_x;
         const bool two = NT == 2 && p.inner > 1;
-        if (two) __syncthreads();  // nobody reads the other tile any more: it gets the new halo
-        if (FUSE_IN || two) {
+        if (NORM) cp_async_wait_all();  // the first iteration's statistics
+        if (two || NORM) __syncthreads();  // nobody reads the other tile any more: it gets the new halo
+        float4 pivot = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (NORM) pivot = lds128(stats0 + buf_d * (Y::NSTAT * 16) + my_tile + QS_MEAN * 16);
+        if (FUSE_IN || two || NORM) {
             const unsigned tile = tiles + buf_x * Y::TILE, other = tiles + (buf_x ^ 1) * Y::TILE;
             u64 na[2], nb[2];
             if (FUSE_IN) {
@@ -435,6 +569,13 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                             v[c][1] = ffma2r(ffma2r(v[c][1], na[1], nb[1]), gg, bb);
                             sts128u(tile + i * 16, v[c][0], v[c][1]);
                         }
+                        if (NORM) {
+                            u64 m0, m1;
+                            lds128u(stats0 + buf_d * (Y::NSTAT * 16) + (SUB == 8 ? 0 : i / 216 * (QS_COUNT * 16)) + QS_MEAN * 16, m0, m1);
+                            v[c][0] = ffma2r(m0, pack2(-1.0f, -1.0f), v[c][0]);
+                            v[c][1] = ffma2r(m1, pack2(-1.0f, -1.0f), v[c][1]);
+                            sts128u(tile + i * 16, v[c][0], v[c][1]);
+                        }
                         if (two) {
                             int cz, cy, cx;
                             G::cell(i, cz, cy, cx);
@@ -458,6 +599,13 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                 dp[dz][2] = pack2(a.z, b.z);
                 dp[dz][3] = pack2(a.w, b.w);
             }
+            float4 unscale = make_float4(1.f, 1.f, 1.f, 1.f), shift = unscale;  // NORM
+            if (NORM) {
+                const unsigned st = stats0 + buf_d * (Y::NSTAT * 16) + my_tile;
+                unscale = lds128(st + QS_STDEPS * 16);
+                shift = lds128(st + QS_MEAN * 16);
+                shift.x -= pivot.x, shift.y -= pivot.y, shift.z -= pivot.z, shift.w -= pivot.w;
+            }
             // block 8: the activations of iteration t + 1 -> the other tile; block 4: those of iteration t, in place
             if (NT == 2 ? !last : t > 0) {
                 const unsigned to = NT == 2 ? tiles + (buf_x ^ 1) * Y::TILE : tile;
@@ -475,14 +623,27 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
             // the next iteration's data
             if (!last) {
                 fetch(stage_d + (buf_d ^ 1) * OWN, at(p.delta, q, t + 1));
+                fetch_stats(buf_d ^ 1, q, t + 1);
                 if (NT == 1 || t + 2 < p.inner) fetch(stage_h, at(p.h, q, NT == 2 ? t + 1 : t));
             } else if (q + 1 < q1) {
                 fetch(stage_d + (buf_d ^ 1) * OWN, at(p.delta, q + 1, 0));
+                fetch_stats(buf_d ^ 1, q + 1, 0);
                 if (NT == 2 && p.inner > 1) fetch(stage_h, at(p.h, q + 1, 0));
                 if (NT == 2 && tid == 0) issue(q + 1, buf_x ^ 1);
             }
 #pragma unroll
-            for (int dz = 0; dz < 2; ++dz) db[dz] = fadd2(db[dz], fadd2(fadd2(dp[dz][0], dp[dz][1]), fadd2(dp[dz][2], dp[dz][3])));
+            for (int dz = 0; dz < 2; ++dz) {
+                if (NORM) {
+                    const float us[4] = {unscale.x, unscale.y, unscale.z, unscale.w}, sh[4] = {shift.x, shift.y, shift.z, shift.w};
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) {
+                        ffma2(db[dz], dp[dz][s], pack2(us[s], us[s]));
+                        ffma2(off[dz], dp[dz][s], pack2(sh[s], sh[s]));
+                    }
+                } else {
+                    db[dz] = fadd2(db[dz], fadd2(fadd2(dp[dz][0], dp[dz][1]), fadd2(dp[dz][2], dp[dz][3])));
+                }
+            }
             const unsigned win = tile + T.cell0 * 16u;
 #pragma unroll
             for (int rz = 0; rz < 4; ++rz)
@@ -520,22 +681,25 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
     float *const dst = p.gpk + ((size_t)blockIdx.y * gridDim.x + blk) * GRAD_F + tid;
     auto put = [&](int k, float v) { dst[k * THREADS] = p.accumulate ? dst[k * THREADS] + v : v; };
 #pragma unroll
-    for (int dz = 0; dz < 2; ++dz)
+    for (int dz = 0; dz < 2; ++dz) {
+        float off0 = 0.0f, off1 = 0.0f;
+        if (NORM) unpack2(off[dz], off0, off1);
 #pragma unroll
         for (int a = 0; a < 3; ++a)
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
                 // window row ry is tap row b = ry - dy of neuron row dy
-                put((a * 9 + 0 + c) * 4 + dz * 2 + 0, sg[0][dz][a][c]);
-                put((a * 9 + 6 + c) * 4 + dz * 2 + 1, sg[1][dz][a][c]);
+                put((a * 9 + 0 + c) * 4 + dz * 2 + 0, sg[0][dz][a][c] - off0);
+                put((a * 9 + 6 + c) * 4 + dz * 2 + 1, sg[1][dz][a][c] - off1);
 #pragma unroll
                 for (int r = 0; r < 2; ++r) {
                     float lo, hi;
                     unpack2(sp[r][dz][a][c], lo, hi);
-                    put((a * 9 + (r + 1) * 3 + c) * 4 + dz * 2 + 0, lo);
-                    put((a * 9 + r * 3 + c) * 4 + dz * 2 + 1, hi);
+                    put((a * 9 + (r + 1) * 3 + c) * 4 + dz * 2 + 0, lo - off0);
+                    put((a * 9 + r * 3 + c) * 4 + dz * 2 + 1, hi - off1);
                 }
             }
+    }
 #pragma unroll
     for (int dz = 0; dz < 2; ++dz) {
         float lo, hi;
@@ -549,22 +713,37 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
     if (failed && p.error_flag) *p.error_flag = 1;
 }
 
-// The chunks' sums in chunk order -> gradients in the layout of the parameters. Four CTAs per region.
+// The chunks' sums in chunk order -> gradients in the layout of the parameters. Two regions per CTA
+// of 256 threads, four CTAs side by side; the CTAs after those put the input's gradient back into the grid's own layout.
 constexpr int kUnpack = 29;  // of the 116 values per thread
 template <int SUB>
-__global__ void __launch_bounds__(128) quad_unpack_grads_k(const float *__restrict__ gpk, float *__restrict__ gw, float *__restrict__ gb,
-                                                           float *__restrict__ gs, int M, int N, int K, int chunks)
+__global__ void __launch_bounds__(256) quad_finish_k(const float *__restrict__ gpk, float *__restrict__ gw, float *__restrict__ gb,
+                                                     float *__restrict__ gs, const float4 *__restrict__ il, float *__restrict__ x, int B, int M,
+                                                     int N, int K, int chunks, unsigned grads, unsigned parts)
 {
     using namespace quadwg;
-    const int tid = threadIdx.x;
+    if (blockIdx.x >= grads) {
+        const unsigned i = blockIdx.x - grads;
+        const size_t P = (size_t)M * N * K, c = (size_t)(i % parts) * 256 + threadIdx.x;
+        const int q = i / parts;
+        if (c >= P) return;
+        const float4 v = il[(size_t)q * P + c];
+        const float vs[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int s = 0; s < 4; ++s)
+            if (4 * q + s < B) x[(size_t)(4 * q + s) * P + c] = vs[s];
+        return;
+    }
+    const int tid = threadIdx.x & 127, regions = (M >> 3) * (N >> 3) * (K >> 3);
     const Patch<SUB> T(tid);
-    const int nbx = K >> 3, nby = N >> 3, blk = blockIdx.x;
+    const int nbx = K >> 3, nby = N >> 3, blk = blockIdx.x / (116 / kUnpack) * 2 + (threadIdx.x >> 7);
+    if (blk >= regions) return;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t P = (size_t)M * N * K;
     const size_t g0 = ((size_t)(bz * 8 + 2 * T.zp) * N + (by * 8 + 2 * T.yp)) * K + bx * 8 + T.x;
     const float *src = gpk + (size_t)blk * GRAD_F + tid;
-    const size_t step = (size_t)gridDim.x * GRAD_F;
-    const int k0 = blockIdx.y * kUnpack;
+    const size_t step = (size_t)regions * GRAD_F;
+    const int k0 = blockIdx.x % (116 / kUnpack) * kUnpack;
 #pragma unroll
     for (int i = 0; i < kUnpack; ++i) {
         const int k = k0 + i;
@@ -581,78 +760,118 @@ __global__ void __launch_bounds__(128) quad_unpack_grads_k(const float *__restri
 // x faces use half of every sector they touch.
 // Block 8: three groups of 128 threads, one per axis; a thread owns one cell of the two faces and the nine taps that cross
 // that face (a tap that crosses several faces belongs to the first axis in the order z, y, x); then one thread per surface
-// cell adds the up to three partial sums to grad_x in that order.
+// cell adds the up to three partial sums to grad_x in that order. Only the shell of 488 cells around the region is fetched,
+// face by face: what a group reads is dense, so there are no bank conflicts and a thread needs one base address. Bound by
+// memory latency: everything a quad needs is asked for two quads ahead by asynchronous copies, which need no registers,
+// so that three CTAs fit on an SM (with the 10^3 tile and register prefetch two did: 72 us, now 40, at 64^3, batch 64).
 __device__ __forceinline__ float4 fma4(float w, float4 v, float4 a)
 {
     return make_float4(fmaf(w, v.x, a.x), fmaf(w, v.y, a.y), fmaf(w, v.z, a.z), fmaf(w, v.w, a.w));
 }
 __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 
+// NORM (per-block normalisation): a cell also owes F + E x to the statistics of every tile that it is a halo cell of
+// (quad_reverse_k). The (negated) terms of the surrounding tiles, 3^3 regions or 4^3 blocks of 4, come with the quad.
 namespace quadborder {
-constexpr int TS = 1000, RING = 3;
-}
+constexpr int TS = 1000;               // block 4: cells of a tile
+constexpr int SHELL = 500, RING = 3;   // block 8: cells of a shell, padded for taps that do not count; quads in flight
+constexpr int SURFACE = 296, DIRS = 27;
+template <int SUB>
+struct Terms {
+    static constexpr int SIDE = SUB == 8 ? 3 : 4, COUNT = SIDE * SIDE * SIDE;
+    // the tile this thread fetches, -1: none, or outside the grid
+    __device__ static int tile(int slot, int bx, int by, int bz, int M, int N, int K)
+    {
+        if (slot >= COUNT) return -1;
+        const int tx = bx * (8 / SUB) + slot % SIDE - 1, ty = by * (8 / SUB) + slot / SIDE % SIDE - 1, tz = bz * (8 / SUB) + slot / SIDE / SIDE - 1;
+        if (tx < 0 || ty < 0 || tz < 0 || tx >= K / SUB || ty >= N / SUB || tz >= M / SUB) return -1;
+        if (SUB == 8) return (tz * (N / 8) + ty) * (K / 8) + tx;
+        return (((tz >> 1) * (N / 8) + (ty >> 1)) * (K / 8) + (tx >> 1)) * 8 + ((tz & 1) * 2 + (ty & 1)) * 2 + (tx & 1);
+    }
+    // sum over the tiles that contain a cell of tile `own` as halo, the cell lying on the faces (dz, dy, dx)
+    __device__ static float4 along(const float4 *t, int own, int dz, int dy, int dx)
+    {
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int m = 1; m < 8; ++m)
+            if ((!(m & 4) || dz) && (!(m & 2) || dy) && (!(m & 1) || dx)) {
+                const float4 f = t[2 * (own + ((m & 4 ? dz : 0) * SIDE + (m & 2 ? dy : 0)) * SIDE + (m & 1 ? dx : 0))];
+                a.x += f.x, a.y += f.y, a.z += f.z, a.w += f.w;
+            }
+        return a;
+    }
+    // F + E v of the region's cell (z, y, x)
+    __device__ static float4 sum(const float4 *t, int z, int y, int x, float4 v)
+    {
+        const int qz = z % SUB, qy = y % SUB, qx = x % SUB;
+        const int dz = qz == 0 ? -1 : (qz == SUB - 1 ? 1 : 0), dy = qy == 0 ? -1 : (qy == SUB - 1 ? 1 : 0), dx = qx == 0 ? -1 : (qx == SUB - 1 ? 1 : 0);
+        const int own = ((z / SUB + 1) * SIDE + y / SUB + 1) * SIDE + x / SUB + 1;
+        const float4 f = along(t, own, dz, dy, dx), e = along(t + 1, own, dz, dy, dx);
+        return make_float4(fmaf(e.x, v.x, f.x), fmaf(e.y, v.y, f.y), fmaf(e.z, v.z, f.z), fmaf(e.w, v.w, f.w));
+    }
+};
+}  // namespace quadborder
 
-__global__ void __launch_bounds__(384) quad_border8_k(const float *__restrict__ w, const float4 *__restrict__ dsum, float4 *__restrict__ gx,
-                                                      int Q, int M, int N, int K, int qpc)
+template <bool NORM>
+__global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict__ w, const float4 *__restrict__ dsum, float4 *__restrict__ gx,
+                                                         const float4 *__restrict__ x, const float4 *__restrict__ hterm, int Q, int M, int N,
+                                                         int K, int qpc)
 {
     using namespace quadborder;
-    constexpr int THREADS = 384, SLOTS = 3;
+    using T = Terms<8>;
+    constexpr int THREADS = 384;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4 *const tile = reinterpret_cast<float4 *>(smem_raw);                   // [RING][TS]
-    float4 *const part = reinterpret_cast<float4 *>(smem_raw) + RING * TS;       // [2][3][128]
+    float4 *const shell = reinterpret_cast<float4 *>(smem_raw);  // [RING][SHELL]
+    float4 *const part = shell + RING * SHELL;                   // [2][3][128]
+    float4 *const mine = part + 2 * 3 * 128;                     // [RING][SURFACE] grad_x, NORM: then x
+    __shared__ float4 terms[NORM ? RING : 1][2 * T::COUNT], dirs[NORM ? 2 : 1][2 * DIRS];
     const int tid = threadIdx.x;
     const int nbx = K >> 3, nby = N >> 3;
     const unsigned blk = blockIdx.x;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t P = (size_t)M * N * K;
     const long long origin = ((long long)(bz * 8 - 1) * N + (by * 8 - 1)) * K + (bx * 8 - 1);
-    for (int i = tid; i < RING * TS; i += THREADS) tile[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    // shell cells this thread fetches: tile offset and offset from the tile's origin
-    int tof[SLOTS], rel[SLOTS];
+    for (int i = tid; i < RING * SHELL; i += THREADS) shell[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    // shell cells this thread fetches: z faces 2 x 10 x 10, then y faces 2 x 8 x 10, then x faces 2 x 8 x 8
+    int rel[2];
 #pragma unroll
-    for (int j = 0; j < SLOTS; ++j) {
+    for (int j = 0; j < 2; ++j) {
         const int i = tid + j * THREADS;
-        tof[j] = -1;
-        rel[j] = 0;
-        if (i < TS) {
-            const int cx = i % 10, cy = (i / 10) % 10, cz = i / 100;
-            const int gz = bz * 8 + cz - 1, gy = by * 8 + cy - 1, gxx = bx * 8 + cx - 1;
-            const bool shell = cx == 0 || cx == 9 || cy == 0 || cy == 9 || cz == 0 || cz == 9;
-            if (shell && gz >= 0 && gz < M && gy >= 0 && gy < N && gxx >= 0 && gxx < K) {
-                tof[j] = i;
-                rel[j] = (cz * N + cy) * K + cx;
-            }
+        int cz, cy, cx;
+        if (i < 200) {
+            cz = i / 100 * 9, cy = i % 100 / 10, cx = i % 10;
+        } else if (i < 360) {
+            const int e = i - 200;
+            cz = 1 + e % 80 / 10, cy = e / 80 * 9, cx = e % 10;
+        } else {
+            const int e = i - 360;
+            cz = 1 + e % 64 / 8, cy = 1 + e % 8, cx = e / 64 * 9;
         }
+        const int gz = bz * 8 + cz - 1, gy = by * 8 + cy - 1, gxx = bx * 8 + cx - 1;
+        const bool in = i < 488 && gz >= 0 && gz < M && gy >= 0 && gy < N && gxx >= 0 && gxx < K;
+        rel[j] = in ? (cz * N + cy) * K + cx : -1;
     }
-    // role 1: one cell of one face
+    // role 1: one cell of one face, (u, v) its coordinates along the other two axes
     const int axis = tid >> 7, fc = tid & 127, side = fc >> 6, u = (fc >> 3) & 7, v = fc & 7;
-    int l[3];
-    l[axis] = side * 7;
-    l[axis == 0 ? 1 : 0] = u;
-    l[axis == 2 ? 1 : 2] = v;
-    const int dcross = side == 0 ? 1 : -1;
+    const int across = side == 0 ? 1 : -1;
     float wf[9];
-    int toff[9];
+    {
+        const int lz = axis == 0 ? side * 7 : u, ly = axis == 0 ? u : (axis == 1 ? side * 7 : v), lx = axis == 2 ? side * 7 : v;
 #pragma unroll
-    for (int q = 0; q < 9; ++q) {
-        int d[3];
-        d[axis] = dcross;
-        d[axis == 0 ? 1 : 0] = q / 3 - 1;
-        d[axis == 2 ? 1 : 2] = q % 3 - 1;
-        bool owned = true;
-        for (int a = 0; a < axis; ++a) {
-            const int s = l[a] - d[a];
-            if (s < 0 || s > 7) owned = false;
+        for (int e = 0; e < 9; ++e) {
+            const int d1 = e / 3 - 1, d2 = e % 3 - 1;
+            const int dz = axis == 0 ? across : d1, dy = axis == 0 ? d1 : (axis == 1 ? across : d2), dx = axis == 2 ? across : d2;
+            const bool owned = (axis == 0 || (u - d1 >= 0 && u - d1 < 8)) && (axis < 2 || (v - d2 >= 0 && v - d2 < 8));
+            const int nz = bz * 8 + lz - dz, ny = by * 8 + ly - dy, nx = bx * 8 + lx - dx;
+            const bool ok = owned && nz >= 0 && nz < M && ny >= 0 && ny < N && nx >= 0 && nx < K;
+            wf[e] = ok ? w[(size_t)((dz + 1) * 9 + (dy + 1) * 3 + dx + 1) * P + ((size_t)nz * N + ny) * K + nx] : 0.0f;
         }
-        const int nz = bz * 8 + l[0] - d[0], ny = by * 8 + l[1] - d[1], nx = bx * 8 + l[2] - d[2];
-        const bool ok = owned && nz >= 0 && nz < M && ny >= 0 && ny < N && nx >= 0 && nx < K;
-        const int t = (d[0] + 1) * 9 + (d[1] + 1) * 3 + (d[2] + 1);
-        wf[q] = ok ? w[(size_t)t * P + ((size_t)nz * N + ny) * K + nx] : 0.0f;
-        toff[q] = (l[0] + 1 - d[0]) * 100 + (l[1] + 1 - d[1]) * 10 + (l[2] + 1 - d[2]);
     }
+    const int row = axis == 2 ? 8 : 10;
+    const int base = axis == 0 ? side * 100 + (u + 1) * 10 + v + 1 : (axis == 1 ? 200 + side * 80 + u * 10 + v + 1 : 360 + side * 64 + u * 8 + v);
     // role 2: one surface cell
     int sz = 0, sy = 0, sx = 0;
-    const bool active = tid < 296;
+    const bool active = tid < SURFACE;
     if (tid < 128) {
         sz = (tid >> 6) * 7; sy = (tid >> 3) & 7; sx = tid & 7;
     } else if (tid < 224) {
@@ -663,57 +882,73 @@ __global__ void __launch_bounds__(384) quad_border8_k(const float *__restrict__ 
         sx = (j / 36) * 7; sz = 1 + (j % 36) / 6; sy = 1 + j % 6;
     }
     const size_t c = ((size_t)(bz * 8 + sz) * N + by * 8 + sy) * K + bx * 8 + sx;
-    const int pz = (sz == 0 || sz == 7) ? (sz / 7) * 64 + sy * 8 + sx : -1;
-    const int py = (sy == 0 || sy == 7) ? (sy / 7) * 64 + sz * 8 + sx : -1;
-    const int px = (sx == 0 || sx == 7) ? (sx / 7) * 64 + sz * 8 + sy : -1;
+    const bool on_z = sz == 0 || sz == 7, on_y = sy == 0 || sy == 7, on_x = sx == 0 || sx == 7;
+    const int pz = (sz / 7) * 64 + sy * 8 + sx, py = 128 + (sy / 7) * 64 + sz * 8 + sx, px = 256 + (sx / 7) * 64 + sz * 8 + sy;
+    const int my_dir = ((on_z ? sz / 7 * 2 : 1) * 3 + (on_y ? sy / 7 * 2 : 1)) * 3 + (on_x ? sx / 7 * 2 : 1);
 
     const int q0 = blockIdx.y * qpc, q1 = min(Q, q0 + qpc);
-    const unsigned tile0 = smem_u32(tile);
-    // two quads ahead: the shell by asynchronous copies, the surface cell by an ordinary load
-    auto fetch = [&](int q) {
+    const unsigned shell0 = smem_u32(shell) + tid * 16, mine0 = smem_u32(mine) + tid * 16;
+    const int my_term = NORM ? T::tile(tid >> 1, bx, by, bz, M, N, K) : -1;
+    if (NORM && tid < 2 * T::COUNT)
+        for (int r = 0; r < RING; ++r) terms[r][tid] = make_float4(0.f, 0.f, 0.f, 0.f);
+    int slot = 0;  // ring slot of the quad in work
+    auto fetch = [&](int q, int r) {
         if (q < q1) {
             const float4 *src = dsum + (size_t)q * P + origin;
 #pragma unroll
-            for (int j = 0; j < SLOTS; ++j)
-                if (tof[j] >= 0) cp_async16(tile0 + (unsigned)((q % RING) * TS + tof[j]) * 16u, src + rel[j]);
+            for (int j = 0; j < 2; ++j)
+                if (rel[j] >= 0) cp_async16(shell0 + (unsigned)(r * SHELL + j * THREADS) * 16u, src + rel[j]);
+            if (active) {
+                cp_async16(mine0 + (unsigned)(r * SURFACE) * 16u, gx + (size_t)q * P + c);
+                if (NORM) cp_async16(mine0 + (unsigned)((RING + r) * SURFACE) * 16u, x + (size_t)q * P + c);
+            }
+            if (NORM && my_term >= 0) cp_async16(smem_u32(&terms[r][tid]), hterm + ((size_t)q * gridDim.x + my_term) * 2 + (tid & 1));
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    float4 g1 = make_float4(0.f, 0.f, 0.f, 0.f), g2 = g1;
-    __syncthreads();  // tiles are zeroed
-    fetch(q0);
-    fetch(q0 + 1);
-    if (active && q0 < q1) g1 = gx[(size_t)q0 * P + c];
-    if (active && q0 + 1 < q1) g2 = gx[(size_t)(q0 + 1) * P + c];
+    __syncthreads();  // the shells are zeroed
+    fetch(q0, 0);
+    fetch(q0 + 1, 1);
     for (int q = q0; q < q1; ++q) {
         const int par = q & 1;
-        const float4 *tl = tile + (q % RING) * TS;
         asm volatile("cp.async.wait_group 1;" ::: "memory");
-        __syncthreads();  // quad q has landed; the tile of quad q - 1 has been read
-        fetch(q + 2);
-        float4 acc = g1;
-        g1 = g2;
-        if (active && q + 2 < q1) g2 = gx[(size_t)(q + 2) * P + c];
+        __syncthreads();  // quad q has landed; the shell of quad q - 1 has been read
+        fetch(q + 2, slot == 0 ? 2 : slot - 1);
         {
+            const float4 *sh = shell + slot * SHELL + base;
             float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int e = 0; e < 9; ++e) s = fma4(wf[e], tl[toff[e]], s);
-            part[(par * 3 + axis) * 128 + fc] = s;
+            for (int e = 0; e < 9; ++e) s = fma4(wf[e], sh[-(e / 3 - 1) * row - (e % 3 - 1)], s);
+            part[par * 384 + tid] = s;
+        }
+        if (NORM && tid < 2 * DIRS) {
+            const int d = tid >> 1;
+            dirs[par][tid] = T::along(&terms[slot][tid & 1], 13, d / 9 - 1, d / 3 % 3 - 1, d % 3 - 1);
         }
         __syncthreads();
         if (active) {
-            if (pz >= 0) acc = add4(acc, part[(par * 3 + 0) * 128 + pz]);
-            if (py >= 0) acc = add4(acc, part[(par * 3 + 1) * 128 + py]);
-            if (px >= 0) acc = add4(acc, part[(par * 3 + 2) * 128 + px]);
+            float4 acc = mine[slot * SURFACE + tid];
+            if (NORM) {
+                const float4 xv = mine[(RING + slot) * SURFACE + tid], f = dirs[par][2 * my_dir], e = dirs[par][2 * my_dir + 1];
+                acc.x += fmaf(e.x, xv.x, f.x), acc.y += fmaf(e.y, xv.y, f.y), acc.z += fmaf(e.z, xv.z, f.z), acc.w += fmaf(e.w, xv.w, f.w);
+            }
+            if (on_z) acc = add4(acc, part[par * 384 + pz]);
+            if (on_y) acc = add4(acc, part[par * 384 + py]);
+            if (on_x) acc = add4(acc, part[par * 384 + px]);
             gx[(size_t)q * P + c] = acc;
         }
+        slot = slot == RING - 1 ? 0 : slot + 1;
     }
 }
 
 // Block 4: one thread per cell of the region, all 27 taps; sources in the cell's own block carry a zero weight.
-__global__ void __launch_bounds__(512) quad_border4_k(const float *__restrict__ w, const float4 *__restrict__ dsum, float4 *__restrict__ gx,
-                                                      int Q, int M, int N, int K, int qpc)
+template <bool NORM>
+__global__ void __launch_bounds__(512, 2) quad_border4_k(const float *__restrict__ w, const float4 *__restrict__ dsum, float4 *__restrict__ gx,
+                                                      const float4 *__restrict__ x_il4, const float4 *__restrict__ hterm, int Q, int M,
+                                                      int N, int K, int qpc)
 {
+    using T = quadborder::Terms<4>;
+    __shared__ float4 terms[NORM ? 2 : 1][2 * T::COUNT];
     using namespace quadborder;
     constexpr int THREADS = 512, SLOTS = 2;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -756,6 +991,9 @@ __global__ void __launch_bounds__(512) quad_border4_k(const float *__restrict__ 
     }
     const int tbase = (lz + 1) * 100 + (ly + 1) * 10 + (lx + 1);
     const int q0 = blockIdx.y * qpc, q1 = min(Q, q0 + qpc);
+    const int my_term = NORM ? T::tile(tid >> 1, bx, by, bz, M, N, K) : -1;
+    const size_t ntiles = (size_t)gridDim.x * 8;
+    float4 pt = make_float4(0.f, 0.f, 0.f, 0.f), xnext = pt;
     float4 pf[SLOTS], gnext = make_float4(0.f, 0.f, 0.f, 0.f);
     auto fetch = [&](int q) {
         if (q < q1) {
@@ -763,21 +1001,27 @@ __global__ void __launch_bounds__(512) quad_border4_k(const float *__restrict__ 
 #pragma unroll
             for (int j = 0; j < SLOTS; ++j)
                 if (tof[j] >= 0) pf[j] = __ldg(src + rel[j]);
+            if (NORM && my_term >= 0) pt = __ldg(hterm + ((size_t)q * ntiles + my_term) * 2 + (tid & 1));
         }
     };
     fetch(q0);
     if (active && q0 < q1) gnext = gx[(size_t)q0 * P + c];
+    if (NORM && active && q0 < q1) xnext = x_il4[(size_t)q0 * P + c];
     __syncthreads();
     for (int q = q0; q < q1; ++q) {
         float4 *tl = tile + (q & 1) * TS;
 #pragma unroll
         for (int j = 0; j < SLOTS; ++j)
             if (tof[j] >= 0) tl[tof[j]] = pf[j];
+        if (NORM && tid < 2 * T::COUNT) terms[q & 1][tid] = pt;
         fetch(q + 1);
         float4 acc = gnext;
+        const float4 xv = xnext;
         if (active && q + 1 < q1) gnext = gx[(size_t)(q + 1) * P + c];
+        if (NORM && active && q + 1 < q1) xnext = x_il4[(size_t)(q + 1) * P + c];
         __syncthreads();  // the other tile may still be read by slower threads; it is rewritten after the next barrier
         if (active) {
+            if (NORM) acc = add4(acc, T::sum(terms[q & 1], lz, ly, lx, xv));
 #pragma unroll
             for (int t = 0; t < 27; ++t) {
                 const int dz = t / 9 - 1, dy = (t / 3) % 3 - 1, dx = t % 3 - 1;
@@ -969,21 +1213,21 @@ static int smem_once(Kern kern, int bytes, unsigned long long *mask, const char 
 
 static long long regions_of(int M, int N, int K) { return (long long)(M / 8) * (N / 8) * (K / 8); }
 
+template <int SUB, int ACT, quadrev::In IN>
+static int launch_reverse_in(const QuadRevParams &p, unsigned ctas, cudaStream_t st)
+{
+    constexpr int smem = quadrev::Bytes<IN>::SMEM;
+    static unsigned long long done = 0;
+    const int rc = smem_once(quad_reverse_k<SUB, ACT, IN>, smem, &done, "cudaFuncSetAttribute(quad_reverse_k)");
+    if (rc != GN_OK) return rc;
+    quad_reverse_k<SUB, ACT, IN><<<ctas, 256, smem, st>>>(p);
+    return check_launch("quad_reverse");
+}
 template <int SUB, int ACT>
 static int launch_reverse_one(const QuadRevParams &p, unsigned ctas, cudaStream_t st)
 {
-    static unsigned long long done[2] = {};
-    int rc;
-    if (p.raw) {
-        rc = smem_once(quad_reverse_k<SUB, ACT, true>, quadrev::SMEM_BYTES, &done[1], "cudaFuncSetAttribute(quad_reverse_k)");
-        if (rc != GN_OK) return rc;
-        quad_reverse_k<SUB, ACT, true><<<ctas, 256, quadrev::SMEM_BYTES, st>>>(p);
-    } else {
-        rc = smem_once(quad_reverse_k<SUB, ACT, false>, quadrev::SMEM_BYTES, &done[0], "cudaFuncSetAttribute(quad_reverse_k)");
-        if (rc != GN_OK) return rc;
-        quad_reverse_k<SUB, ACT, false><<<ctas, 256, quadrev::SMEM_BYTES, st>>>(p);
-    }
-    return check_launch("quad_reverse");
+    if (p.tile_stats) return launch_reverse_in<SUB, ACT, quadrev::BLOCK_NORM>(p, ctas, st);
+    return p.raw ? launch_reverse_in<SUB, ACT, quadrev::GRID_NORM>(p, ctas, st) : launch_reverse_in<SUB, ACT, quadrev::PLAIN>(p, ctas, st);
 }
 
 template <int SUB>
@@ -1001,6 +1245,7 @@ int launch_quad_reverse(const QuadReverse &a, int act, cudaStream_t st)
 {
     QuadRevParams p{};
     p.packed = a.packed_t; p.g = a.g; p.raw = a.raw; p.stats = a.stats; p.ac = a.ac; p.h = a.h;
+    p.wsum = a.wsum; p.tile_stats = a.tile_stats; p.hterm = a.hterm; p.B = a.B;
     p.delta = a.delta; p.dsum = a.dsum; p.gx = a.gx; p.dsq = a.dsq;
     p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;
     p.nitems = regions_of(a.M, a.N, a.K) * a.Q;
@@ -1024,23 +1269,21 @@ size_t quad_grad_floats(int M, int N, int K, int Q)
     return (size_t)wgrad_chunks(regions, Q) * regions * quadwg::GRAD_F;
 }
 
+template <int SUB, int ACT, bool FUSE_IN, bool NORM>
+static int launch_wgrad_in(const CUtensorMap &map, const QuadWgradParams &p, dim3 grid, cudaStream_t st)
+{
+    constexpr int smem = quadwg::Lay<SUB>::smem(FUSE_IN, NORM);
+    static unsigned long long done = 0;
+    const int rc = smem_once(quad_wgrad_k<SUB, ACT, FUSE_IN, NORM>, smem, &done, "cudaFuncSetAttribute(quad_wgrad_k)");
+    if (rc != GN_OK) return rc;
+    quad_wgrad_k<SUB, ACT, FUSE_IN, NORM><<<grid, quadwg::THREADS, smem, st>>>(map, p);
+    return check_launch("quad_wgrad");
+}
 template <int SUB, int ACT>
 static int launch_wgrad_one(const CUtensorMap &map, const QuadWgradParams &p, dim3 grid, cudaStream_t st)
 {
-    static unsigned long long done[2] = {};
-    int rc;
-    if (p.in_stats) {
-        constexpr int smem = quadwg::Lay<SUB>::smem(true);
-        rc = smem_once(quad_wgrad_k<SUB, ACT, true>, smem, &done[1], "cudaFuncSetAttribute(quad_wgrad_k)");
-        if (rc != GN_OK) return rc;
-        quad_wgrad_k<SUB, ACT, true><<<grid, quadwg::THREADS, smem, st>>>(map, p);
-    } else {
-        constexpr int smem = quadwg::Lay<SUB>::smem(false);
-        rc = smem_once(quad_wgrad_k<SUB, ACT, false>, smem, &done[0], "cudaFuncSetAttribute(quad_wgrad_k)");
-        if (rc != GN_OK) return rc;
-        quad_wgrad_k<SUB, ACT, false><<<grid, quadwg::THREADS, smem, st>>>(map, p);
-    }
-    return check_launch("quad_wgrad");
+    if (p.tile_stats) return launch_wgrad_in<SUB, ACT, false, true>(map, p, grid, st);
+    return p.in_stats ? launch_wgrad_in<SUB, ACT, true, false>(map, p, grid, st) : launch_wgrad_in<SUB, ACT, false, false>(map, p, grid, st);
 }
 
 template <int SUB>
@@ -1058,10 +1301,12 @@ int launch_quad_wgrad(const QuadWgrad &a, int act, cudaStream_t st)
 {
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
+    if (a.tile_stats && a.in_stats) return GN_ERR_UNSUPPORTED;
     const int rc = quad_make_map(&map, a.in_il4, a.M, a.N, a.K, a.Q, a.block);
     if (rc != GN_OK) return rc;
     QuadWgradParams p{};
     p.gbt = a.gbt; p.in_stats = a.in_stats; p.delta = a.delta; p.h = a.h; p.scale = a.scale; p.dsq = a.dsq; p.gpk = a.gpk;
+    p.tile_stats = a.tile_stats;
     p.accumulate = a.accumulate;
     p.error_flag = a.error_flag ? a.error_flag : device_status_ptr();
     p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;
@@ -1072,35 +1317,51 @@ int launch_quad_wgrad(const QuadWgrad &a, int act, cudaStream_t st)
     return a.block == 8 ? launch_wgrad_sub<8>(map, p, grid, act, st) : launch_wgrad_sub<4>(map, p, grid, act, st);
 }
 
-int launch_quad_unpack_grads(const float *gpk, float *gw, float *gb, float *gs, int M, int N, int K, int Q, int block, cudaStream_t st)
+int launch_quad_finish(const float *gpk, float *gw, float *gb, float *gs, const float *il, float *x, int B, int M, int N, int K, int block,
+                       cudaStream_t st)
 {
     const long long regions = regions_of(M, N, K);
-    const int chunks = wgrad_chunks(regions, Q);
-    if (block == 8) quad_unpack_grads_k<8><<<dim3((unsigned)regions, 116 / kUnpack), 128, 0, st>>>(gpk, gw, gb, gs, M, N, K, chunks);
-    else quad_unpack_grads_k<4><<<dim3((unsigned)regions, 116 / kUnpack), 128, 0, st>>>(gpk, gw, gb, gs, M, N, K, chunks);
-    return check_launch("quad_unpack_grads");
+    const int chunks = wgrad_chunks(regions, (B + 3) / 4);
+    const unsigned grads = (unsigned)((regions + 1) / 2) * (116 / kUnpack), parts = (unsigned)(((long long)M * N * K + 255) / 256);
+    const unsigned long long n = grads + (il ? (unsigned long long)parts * ((B + 3) / 4) : 0);
+    if (n >= 1ull << 31) return GN_ERR_UNSUPPORTED;
+    const float4 *const i4 = reinterpret_cast<const float4 *>(il);
+    if (block == 8) quad_finish_k<8><<<(unsigned)n, 256, 0, st>>>(gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, grads, parts);
+    else quad_finish_k<4><<<(unsigned)n, 256, 0, st>>>(gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, grads, parts);
+    return check_launch("quad_finish");
 }
 
-int launch_quad_border(const float *w, const float *dsum, float *gx, int M, int N, int K, int Q, int block, cudaStream_t st)
+template <bool NORM>
+static int launch_border(const float *w, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K, int Q,
+                         int block, cudaStream_t st)
 {
     const long long nb = regions_of(M, N, K);
-    const int ctas_per_sm = 3;
+    const int ctas_per_sm = block == 8 ? 3 : 2;
     const int chunks = pick_batch_chunks_balanced(nb, Q, ctas_per_sm, 4.0, 32);
     const int qpc = (Q + chunks - 1) / chunks;
     dim3 grid((unsigned)nb, (unsigned)((Q + qpc - 1) / qpc));
     static unsigned long long done[2] = {};
+    const float4 *const d4 = reinterpret_cast<const float4 *>(dsum), *const x4 = reinterpret_cast<const float4 *>(x_il4);
+    float4 *const g4 = reinterpret_cast<float4 *>(gx);
     if (block == 8) {
-        constexpr int smem = (quadborder::RING * quadborder::TS + 2 * 3 * 128) * 16;
-        const int rc = smem_once(quad_border8_k, smem, &done[0], "cudaFuncSetAttribute(quad_border8_k)");
+        constexpr int smem = (quadborder::RING * (quadborder::SHELL + (NORM ? 2 : 1) * quadborder::SURFACE) + 2 * 3 * 128) * 16;
+        const int rc = smem_once(quad_border8_k<NORM>, smem, &done[0], "cudaFuncSetAttribute(quad_border8_k)");
         if (rc != GN_OK) return rc;
-        quad_border8_k<<<grid, 384, smem, st>>>(w, reinterpret_cast<const float4 *>(dsum), reinterpret_cast<float4 *>(gx), Q, M, N, K, qpc);
+        quad_border8_k<NORM><<<grid, 384, smem, st>>>(w, d4, g4, x4, hterm, Q, M, N, K, qpc);
     } else {
         constexpr int smem = 2 * quadborder::TS * 16;
-        const int rc = smem_once(quad_border4_k, smem, &done[1], "cudaFuncSetAttribute(quad_border4_k)");
+        const int rc = smem_once(quad_border4_k<NORM>, smem, &done[1], "cudaFuncSetAttribute(quad_border4_k)");
         if (rc != GN_OK) return rc;
-        quad_border4_k<<<grid, 512, smem, st>>>(w, reinterpret_cast<const float4 *>(dsum), reinterpret_cast<float4 *>(gx), Q, M, N, K, qpc);
+        quad_border4_k<NORM><<<grid, 512, smem, st>>>(w, d4, g4, x4, hterm, Q, M, N, K, qpc);
     }
     return check_launch("quad_border");
+}
+
+int launch_quad_border(const float *w, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K, int Q,
+                       int block, cudaStream_t st)
+{
+    return hterm ? launch_border<true>(w, dsum, gx, x_il4, hterm, M, N, K, Q, block, st)
+                 : launch_border<false>(w, dsum, gx, nullptr, nullptr, M, N, K, Q, block, st);
 }
 
 int quad_norm_parts(long long P)

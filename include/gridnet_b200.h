@@ -462,6 +462,22 @@ GN_API int gn_outer_forward_flags_f32(const float *weight, const float *bias, co
                                int activation, void *workspace, size_t workspace_bytes, int flags,
                                void *stream);
 
+/* ---- one step on the kernels that hold the weights in tensor memory, four samples per lane (block 4 or 8, M, N, K multiples
+ * of 8, inner >= 1; anything else: GN_ERR_UNSUPPORTED and sizes of 0). gn_step_forward_kept_f32 computes what
+ * gn_step_forward_f32 does; with `kept` (gn_step_kept_bytes, or NULL) it leaves there what the backward pass would otherwise
+ * compute again. gn_step_backward_kept_f32 computes what gn_step_backward_f32 does; kept from the forward call with the same
+ * arguments, or NULL (then x is read, else it may be NULL). Workspaces: gn_step_kept_workspace_bytes(..., backward, kept
+ * given). kept and workspace: 256-byte aligned. A bounded wait that gave up is reported through gn_device_status. */
+GN_API size_t gn_step_kept_bytes(int B, int M, int N, int K, int inner, int block, int normalize);
+GN_API size_t gn_step_kept_workspace_bytes(int B, int M, int N, int K, int inner, int block, int normalize, int backward, int kept);
+GN_API int gn_step_forward_kept_f32(const float *weight, const float *bias, const float *scale, const float *x, float *y, int B, int M,
+                                    int N, int K, int inner, int block, float eps, int normalize, int act, void *kept,
+                                    size_t kept_bytes, void *workspace, size_t workspace_bytes, void *stream);
+GN_API int gn_step_backward_kept_f32(const float *weight, const float *bias, const float *scale, const float *x, const float *gy,
+                                     float *gw, float *gb, float *gs, float *gx, int B, int M, int N, int K, int inner, int block,
+                                     float eps, int normalize, int act, void *kept, size_t kept_bytes, void *workspace,
+                                     size_t workspace_bytes, void *stream);
+
 /* ------------------------------------------------------ the model loop with gradients
  * The loop of gridnet/scripts/train_mnist.py:62-64 (residual = 0: h = layer_norm(step(h))) or of
  * train_imagenet.py:81-83 (residual = 1: n = layer_norm(h), h = h + step(n) - n), float32, per-block normalisation off,

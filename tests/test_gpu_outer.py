@@ -451,3 +451,29 @@ def test_full_size_step_gradients(name, shape, B, bs, inner):
     two = backward(True, x[idx].contiguous(), gy[idx].contiguous())
     for name_, a, r, n32 in zip(("gw", "gb", "gs", "gx"), two, ref_g, ref_g32):
         assert_close(a.cpu().numpy(), r, n32, f"{name} {name_}, two samples")
+
+
+@pytest.mark.parametrize("normalize", [False, True])
+@pytest.mark.parametrize("block,shape,batch,inner,act", [(8, (8, 16, 24), 5, 1, "relu"), (8, (24, 8, 8), 2, 3, "silu"), (4, (16, 8, 8), 7, 2, "tanh")])
+def test_step_with_weights_in_tensor_memory(block, shape, batch, inner, act, normalize):
+    """One step forward and backward through the kept-activation entry points, with what the forward pass keeps and without,
+    ragged quads included, against the float64 oracle."""
+    from gridnet_b200 import gridnet_cuda as gc
+    from gridnet_b200._lib import lib
+
+    r = np.random.default_rng(7)
+    w = (r.standard_normal((27, *shape)) / np.sqrt(27)).astype(np.float32)
+    b, s = (0.1 * r.standard_normal(shape)).astype(np.float32), (1 + 0.1 * r.standard_normal(shape)).astype(np.float32)
+    x, gy = (3 + r.standard_normal((batch, *shape)).astype(np.float32) for _ in range(2))
+    args64 = [a.astype(np.float64) for a in (w, b, s, x)]
+    ref_y = orc.step_forward(*args64, inner, block, 1e-5, normalize, act)
+    refs = orc.step_backward(*args64, gy.astype(np.float64), inner, block, 1e-5, normalize, act)
+    t = [dev(a) for a in (w, b, s, x)]
+    for keep in (True, False):
+        y, grads = torch.empty_like(t[3]), [torch.empty_like(a) for a in t]
+        kept = torch.empty(lib.gn_step_kept_bytes(batch, *shape, inner, block, normalize), dtype=torch.uint8, device="cuda") if keep else None
+        gc.forward_kept(*t, y, inner, block, 1e-5, normalize, act, kept)
+        gc.backward_kept(*t, dev(gy), *grads, inner, block, 1e-5, normalize, act, kept)
+        assert_close(y.cpu().numpy(), ref_y, None, "y")
+        for g, ref, name in zip(grads, refs, ("weight", "bias", "scale", "x")):
+            assert_close(g.cpu().numpy(), ref, None, f"grad {name}, keep {keep}")
