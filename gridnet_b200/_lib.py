@@ -88,6 +88,9 @@ SIGNATURES = {
                                                                         c_size_t, _P]),
     "gn_loop_backward_f32": (c_int, [_P] * 3 + [c_int] + [_P] * 13 + _geom + [c_int, c_int, c_int, c_int, c_int, _P, c_size_t,
                                                                           _P]),
+    "gn_gated_loop_workspace_bytes": (c_size_t, [c_int] * 8),
+    "gn_gated_loop_forward_f32": (c_int, [_P] * 10 + _geom + [c_int, c_int, c_float, c_int, _P, c_size_t, _P]),
+    "gn_gated_loop_backward_f32": (c_int, [_P] * 14 + _geom + [c_int, c_int, c_int, _P, c_size_t, _P]),
     "gn_outer_forward_plan": (c_int, [c_int] * 7),
     "gn_outer_forward_workspace_bytes": (c_size_t, [c_int] * 5),
     "gn_outer_forward_error_flag_offset": (c_size_t, [c_int] * 5),

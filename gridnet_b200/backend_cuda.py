@@ -287,14 +287,14 @@ def _kept_steps(nbytes_out: int, nbytes_stash: int, outer: int, device) -> int:
 
 
 def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, block: int, activation: str, ln_eps: float,
-                  residual: bool, need_grad: bool):
+                  residual: bool, need_grad: bool, gated: bool = False):
     """The loop forward through ``gn_loop_forward_f32``; ``plist``: one (weight, bias, residual_scale) for all steps, or one
-    per step. Returns the output and the tensors the backward pass needs: (x_il4, stats, outs, stashes)."""
+    per step; gated: one (weight, bias), through ``gn_gated_loop_forward_f32``. Returns the output and the tensors the backward pass needs: (x_il4, stats, outs, stashes)."""
     B, M, N, K = x.shape
     for params in plist:
-        _assert_step_args(*params, x, block, False)
-        assert norm_weight.shape == params[1].shape == norm_bias.shape, f"{norm_weight.shape=} invalid for {params[1].shape=}"
-        _require_f32_cuda(weight=params[0], bias=params[1], residual_scale=params[2])
+        _assert_step_args(*params, *([None] if gated else []), x, block, gated)
+        assert norm_weight.shape == params[1].shape[-3:] == norm_bias.shape, f"{norm_weight.shape=} invalid for {params[1].shape=}"
+        _require_f32_cuda(**dict(zip(("weight", "bias", "residual_scale"), params)))
     _require_f32_cuda(norm_weight=norm_weight, norm_bias=norm_bias, x=x)
     dev = x.device
     one = int(lib.gn_loop_tensor_bytes(B, M, N, K))
@@ -302,13 +302,16 @@ def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, bloc
     stat = (stat + 255) // 256 * 256
     y = torch.empty_like(x)
     with torch.cuda.device(dev):
-        wbytes = int(lib.gn_loop_forward_workspace_bytes(B, M, N, K, inner, outer, block, int(residual)))
+        if gated:
+            wbytes = int(lib.gn_gated_loop_workspace_bytes(B, M, N, K, inner, outer, 0, 0))
+        else:
+            wbytes = int(lib.gn_loop_forward_workspace_bytes(B, M, N, K, inner, outer, block, int(residual)))
         if wbytes == 0:
             raise RuntimeError(f"the fused loop does not cover {tuple(x.shape)}, block {block}, {inner} inner iterations")
         ws = torch.empty(wbytes, dtype=torch.uint8, device=dev)
         stashes = [None] * outer
         if need_grad:
-            stash_bytes = inner * one
+            stash_bytes = (3 if gated else 1) * inner * one
             keep = _kept_steps(one, stash_bytes, outer, dev)
             total = (outer + 1) * one + stat + keep * stash_bytes
             if total < _BIG:  # one allocation, cut up
@@ -337,6 +340,13 @@ def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, bloc
             x_il4 = torch.empty(one, dtype=torch.uint8, device=dev)
             pair = [torch.empty(one, dtype=torch.uint8, device=dev) for _ in range(min(2, outer))]
             outs = [pair[k & 1] for k in range(outer)]
+        if gated:
+            weight, bias = plist[0]
+            check(lib.gn_gated_loop_forward_f32(weight.data_ptr(), bias.data_ptr(), norm_weight.data_ptr(), norm_bias.data_ptr(), x.data_ptr(),
+                                                y.data_ptr(), x_il4.data_ptr(), _pointers(outs), stats.data_ptr(), _pointers(stashes), B, M,
+                                                N, K, inner, outer, ln_eps, activation_id(activation), ws.data_ptr(), ws.numel(),
+                                                torch.cuda.current_stream().cuda_stream))
+            return y, (x_il4, stats, outs, stashes)
         weights, biases, scales = ([p[i] for p in plist] for i in range(3))
         check(lib.gn_loop_forward_f32(_pointers(weights), _pointers(biases), _pointers(scales), len(plist),
                                       norm_weight.data_ptr(), norm_bias.data_ptr(), x.data_ptr(), y.data_ptr(),
@@ -347,7 +357,7 @@ def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, bloc
 
 
 def _loop_backward(plist, norm_weight, norm_bias, saved, grad_y, inner: int, outer: int, block: int, activation: str,
-                   residual: bool):
+                   residual: bool, gated: bool = False):
     """The gradients of :func:`_loop_forward` through ``gn_loop_backward_f32``: one (weight, bias, residual_scale) triple per
     entry of ``plist``, then those of the norm's weight and bias and of x."""
     x_il4, stats, outs, stashes = saved
@@ -358,6 +368,15 @@ def _loop_backward(plist, norm_weight, norm_bias, saved, grad_y, inner: int, out
     gg, gb, gx = torch.empty_like(norm_weight), torch.empty_like(norm_bias), torch.empty_like(g)
     with torch.cuda.device(dev):
         replay = int(any(t is None for t in stashes))
+        if gated:
+            (weight, bias), (gw, gb_) = plist[0], grads[0]
+            ws = torch.empty(int(lib.gn_gated_loop_workspace_bytes(B, M, N, K, inner, outer, 1, replay)), dtype=torch.uint8, device=dev)
+            check(lib.gn_gated_loop_backward_f32(weight.data_ptr(), bias.data_ptr(), norm_weight.data_ptr(), norm_bias.data_ptr(),
+                                                 x_il4.data_ptr(), _pointers(outs), stats.data_ptr(), _pointers(stashes), g.data_ptr(),
+                                                 gw.data_ptr(), gb_.data_ptr(), gg.data_ptr(), gb.data_ptr(), gx.data_ptr(), B, M, N, K,
+                                                 inner, outer, activation_id(activation), ws.data_ptr(), ws.numel(),
+                                                 torch.cuda.current_stream().cuda_stream))
+            return grads, gg, gb, gx
         ws = torch.empty(int(lib.gn_loop_backward_workspace_bytes(B, M, N, K, inner, outer, block, int(residual), replay)),
                          dtype=torch.uint8, device=dev)
         columns = [_pointers([p[i] for p in plist]) for i in range(3)] + [_pointers([p[i] for p in grads]) for i in range(3)]
@@ -423,6 +442,41 @@ class FusedLoopTrainOp(torch.autograd.Function):
             return (*(torch.zeros_like(t) for t in ctx.saved_tensors), grad_y, None, None, None, None, None)
         params, saved = _restore_loop(ctx, 5, outer)
         grads, gg, gb, gx = _loop_backward([params[:3]], *params[3:], saved, grad_y, *ctx.cfg, False)
+        return (*grads[0], gg, gb, gx, None, None, None, None, None)
+
+
+class FusedGatedLoopTrainOp(torch.autograd.Function):
+    """:class:`FusedLoopTrainOp` for the gated step (gridnet/scripts/train_mnist.py:36-44, 62-64), block 8:
+
+        for _ in range(outer_iters):
+            h = layer_norm(gated_gridnet_step(weight, bias, h, ...), norm_weight, norm_bias)
+
+    ``FusedGatedLoopTrainOp.apply(weight, bias, norm_weight, norm_bias, x, inner_iters, outer_iters, block_size, activation,
+    ln_eps)``."""
+
+    @staticmethod
+    def supported(weight, x, inner_iters: int, block_size: int) -> bool:
+        return block_size == 8 and FusedLoopTrainOp.supported(weight, x, inner_iters, block_size)
+
+    @staticmethod
+    def forward(ctx, weight, bias, norm_weight, norm_bias, x, inner_iters: int, outer_iters: int, block_size: int,
+                activation: str, ln_eps: float):
+        ctx.cfg = (int(inner_iters), int(outer_iters), int(block_size), activation)
+        if not ctx.cfg[1]:
+            ctx.save_for_backward(weight, bias, norm_weight, norm_bias)
+            return x.clone()
+        y, saved = _loop_forward([(weight, bias)], norm_weight, norm_bias, x.contiguous(), *ctx.cfg, float(ln_eps), False,
+                                 any(ctx.needs_input_grad[:5]), gated=True)
+        _save_loop(ctx, (weight, bias, norm_weight, norm_bias), saved)
+        return y
+
+    @staticmethod
+    def backward(ctx, grad_y):
+        outer = ctx.cfg[1]
+        if not outer:
+            return (*(torch.zeros_like(t) for t in ctx.saved_tensors), grad_y, None, None, None, None, None)
+        params, saved = _restore_loop(ctx, 4, outer)
+        grads, gg, gb, gx = _loop_backward([params[:2]], *params[2:], saved, grad_y, *ctx.cfg, False, gated=True)
         return (*grads[0], gg, gb, gx, None, None, None, None, None)
 
 

@@ -158,6 +158,7 @@ int quad_tile_cells(int block);  // float2 entries per region of the (gamma, bet
 // What is re-ordered ahead of a step or a loop; jobs whose destination is nullptr are left out.
 struct QuadPrepare {
     const float *w, *b, *s;
+    bool gated;                // w, b, b_t and the packed parameters have two branches; s is not looked at (any M N K floats)
     float *packed;             // quad_packed_floats(...): weights, b, s in the order of the forward sums
     const float *b_t;
     float *packed_t;           // the same for the backward sums: transposed weights, b_t, s
@@ -197,18 +198,19 @@ struct QuadWgrad {
     const float *scale;        // native layout: activations between iterations are rebuilt from h
     float *gpk;                // quad_grad_floats(...)
     const float4 *tile_stats;  // per-block normalisation, or nullptr
+    const float *delta2;       // gated: deltas of the gate; h then holds the activations after each iteration; or nullptr
     int accumulate;
     int *error_flag;
     int M, N, K, Q, inner, block;
 };
-size_t quad_grad_floats(int M, int N, int K, int Q);
+size_t quad_grad_floats(int M, int N, int K, int Q, int branches);
 int launch_quad_wgrad(const QuadWgrad &a, int act, cudaStream_t st);
 // gradients of the parameters out of gpk and, with il, il (IL4) -> x [B, P]
 int launch_quad_finish(const float *gpk, float *gw, float *gb, float *gs, const float *il, float *x, int B, int M, int N, int K, int block,
-                       cudaStream_t st);
-// hterm (from launch_quad_reverse) and the step's input: per-block normalisation, or nullptr
-int launch_quad_border(const float *w, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K, int Q,
-                       int block, cudaStream_t st);
+                       int branches, cudaStream_t st);
+// branches: 2 if w is one branch of [27][2][P]. hterm (from launch_quad_reverse), x_il4 (the step's input): per-block normalisation, or nullptr
+int launch_quad_border(const float *w, int branches, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
+                       int Q, int block, cudaStream_t st);
 int quad_norm_parts(long long P);
 int launch_quad_norm_sums(const float *x, const float *g, const float *sub, const float *gamma, const float2 *stats, double2 *partials,
                           float *ggamma, float *gbeta, int accumulate, float2 *ac, int Q, long long P, cudaStream_t st);
@@ -218,6 +220,29 @@ int quad_combine_parts(long long P);
 int launch_quad_residual_combine(const float *h, const float *y, const float *gamma, const float *beta, const float2 *stats, float *out,
                                  double2 *partials, int Q, long long P, cudaStream_t st);
 int quad_make_map(CUtensorMap *map, const float *il, int M, int N, int K, int Q, int block);
+
+// ---- step_quad_gated.cu (gated update, block 8; all activation tensors IL4)
+struct QuadGated {
+    const float *packed;       // launch_quad_prepare, gated
+    const float2 *gbt;
+    const float *in_il4;
+    float *out_il4;
+    const float2 *in_stats;    // [4 Q] or nullptr
+    double2 *out_partials;     // [4 Q][nparts] or nullptr; slots 0 .. 2 regions-1 of every row are written
+    int nparts;
+    float *hv, *hg, *x;        // [inner] tensors each to keep (pre-activations, activations that went in), or nullptr
+    int M, N, K, Q, inner;
+};
+int launch_quad_gated_fwd(const QuadGated &a, int act, cudaStream_t st);
+struct QuadGatedReverse {
+    const float *packed_t, *gamma, *g, *raw;
+    const float2 *stats, *ac;
+    const float *hv, *hg, *x;
+    float *delta_v, *delta_g;          // [inner]
+    float *dsum_v, *dsum_g, *gx;
+    int M, N, K, Q, inner;
+};
+int launch_quad_gated_reverse(const QuadGatedReverse &a, int act, cudaStream_t st);
 
 // ---- status.cu: device address of the per-device status word that kernels set when a bounded wait gives up
 // and the caller passed no flag of its own (nullptr if it cannot be resolved)

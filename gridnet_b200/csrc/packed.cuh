@@ -63,4 +63,30 @@ __device__ __forceinline__ u64 act_residual2(u64 h, float sc, u64 cen)
     return ffma2r(pack2(Act<ACT, float>::fwd(h0), Act<ACT, float>::fwd(h1)), sc2, cen);
 }
 
+// value and derivative for a pair of samples
+template <int ACT>
+__device__ __forceinline__ void act_both2(u64 h, u64 &f, u64 &d)
+{
+    if (ACT == GN_ACT_SILU) {
+        const u64 t = fmul2(h, pack2(-1.4426950408889634f, -1.4426950408889634f));
+        float t0, t1, e0, e1, r0, r1, d0, d1;
+        unpack2(t, t0, t1);
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(t0));
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(t1));
+        unpack2(fadd2(pack2(e0, e1), pack2(1.0f, 1.0f)), d0, d1);
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d0));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d1));
+        const u64 r = pack2(r0, r1);
+        f = fmul2(h, r);
+        d = ffma2r(f, ffma2r(r, pack2(-1.0f, -1.0f), pack2(1.0f, 1.0f)), r);  // sg (1 + h (1 - sg))
+        return;
+    }
+    float h0, h1, f0, f1, d0, d1;
+    unpack2(h, h0, h1);
+    Act<ACT, float>::both(h0, f0, d0);
+    Act<ACT, float>::both(h1, f1, d1);
+    f = pack2(f0, f1);
+    d = pack2(d0, d1);
+}
+
 }  // namespace gn

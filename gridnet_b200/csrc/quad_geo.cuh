@@ -127,19 +127,21 @@ __device__ __forceinline__ void quad_store(float *base, long long zstr, long lon
 #pragma unroll
         for (int j = 0; j < 2; ++j) quad_store2(base, n, j, zstr, ystr, h, v[n]);
 }
+__device__ __forceinline__ void quad_load2(const float *base, int n, int j, long long zstr, long long ystr, int h, u64 (&v)[4][2])
+{
+    u64 a, b, c, d;
+    ldg256(base + (n >> 1) * zstr + (n & 1) * ystr + 8 * (j ^ h), a, b, c, d);
+    v[2 * j][0] = h ? c : a;
+    v[2 * j][1] = h ? d : b;
+    v[2 * j + 1][0] = h ? a : c;
+    v[2 * j + 1][1] = h ? b : d;
+}
 __device__ __forceinline__ void quad_load(const float *base, long long zstr, long long ystr, int h, u64 (&v)[4][4][2])
 {
 #pragma unroll
     for (int n = 0; n < 4; ++n)
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            u64 a, b, c, d;
-            ldg256(base + (n >> 1) * zstr + (n & 1) * ystr + 8 * (j ^ h), a, b, c, d);
-            v[n][2 * j][0] = h ? c : a;
-            v[n][2 * j][1] = h ? d : b;
-            v[n][2 * j + 1][0] = h ? a : c;
-            v[n][2 * j + 1][1] = h ? b : d;
-        }
+        for (int j = 0; j < 2; ++j) quad_load2(base, n, j, zstr, ystr, h, v[n]);
 }
 // ---- a region's 512 cells, staged in shared memory by whole lines: cell (z, y, x) at unit (8 z + y) 8 + (x ^ (y >> 1)) of 16
 // bytes. The swizzle keeps both the copies (8 lanes to a row) and the reads of a lane's own cells free of bank conflicts.

@@ -464,7 +464,7 @@ __device__ __forceinline__ void to_il4(const float *__restrict__ x, float4 *__re
 constexpr int kPackCtas = 4;
 template <int SUB, bool TRANS>
 __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const float *__restrict__ b, const float *__restrict__ s,
-                                          float *__restrict__ packed, int M, int N, int K, int cta)
+                                          float *__restrict__ packed, size_t tap, int M, int N, int K, int cta)
 {
     __shared__ unsigned char uses[36];  // (a * 3 + b) | n << 4
     if (threadIdx.x == 0) {
@@ -481,7 +481,6 @@ __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const flo
     const QuadLane<SUB> L(lane);
     const int nbx = K >> 3, nby = N >> 3, blk = cta / kPackCtas;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
-    const size_t P = (size_t)M * N * K;
     const size_t g0 = ((size_t)(bz * 8 + L.z0) * N + (by * 8 + L.y0)) * K + bx * 8 + 4 * L.h;
     const long long zs = (long long)N * K, ys = (long long)L.ysgn * K;
     float4 *out = reinterpret_cast<float4 *>(packed + (size_t)blk * quad::PACK_F) + lane;
@@ -499,7 +498,7 @@ __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const flo
             const int t = ta * 9 + tb * 3 + tc;
             const size_t own = g0 + (n >> 1) * zs + (n & 1) * ys;
             if (!TRANS) {
-                const float *src = w + (size_t)t * P + own;
+                const float *src = w + (size_t)t * tap + own;
                 if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) r = *reinterpret_cast<const float4 *>(src);
                 else r = make_float4(src[0], src[1], src[2], src[3]);
             } else {
@@ -507,7 +506,7 @@ __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const flo
                 const int mask = ~(SUB - 1);
                 const bool row = lz >= 0 && lz < 8 && ly >= 0 && ly < 8 && ((lz ^ (L.z0 + (n >> 1))) & mask & 7) == 0 &&
                                  ((ly ^ (L.y0 + L.ysgn * (n & 1))) & mask & 7) == 0;
-                const float *src = w + (size_t)(26 - t) * P + own + (ta - 1) * zs + (long long)(tb - 1) * K + (tc - 1);
+                const float *src = w + (size_t)(26 - t) * tap + own + (ta - 1) * zs + (long long)(tb - 1) * K + (tc - 1);
                 float f[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
@@ -578,17 +577,24 @@ struct PrepareArgs {
     int M, N, K;
     unsigned end[5];  // last CTA + 1 of: pack, transposed pack, weight sums, table, conversion
     unsigned parts;   // conversion: CTAs per quad
+    unsigned pack;    // packing: CTAs per branch
+    int branches;
 };
 template <int SUB>
 __global__ void __launch_bounds__(256) quad_prepare_k(const PrepareArgs p)
 {
     const unsigned c = blockIdx.x;
     const QuadPrepare &a = p.a;
-    if (c < p.end[0]) quad_pack<SUB, false>(a.w, a.b, a.s, a.packed, p.M, p.N, p.K, (int)c);
-    else if (c < p.end[1]) quad_pack<SUB, true>(a.w, a.b_t, a.s, a.packed_t, p.M, p.N, p.K, (int)(c - p.end[0]));
+    const size_t P = (size_t)p.M * p.N * p.K, tap = p.branches * P;
+    if (c < p.end[1]) {  // branch k of a gated network: weights [27][2][P], bias [2][P]
+        const unsigned j = c < p.end[0] ? c : c - p.end[0], k = j / p.pack;
+        const size_t to = (size_t)k * (p.pack / kPackCtas) * quad::PACK_F;
+        if (c < p.end[0]) quad_pack<SUB, false>(a.w + k * P, a.b + k * P, a.s, a.packed + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
+        else quad_pack<SUB, true>(a.w + k * P, a.b_t + k * P, a.s, a.packed_t + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
+    }
     else if (c < p.end[2]) quad_wsum<SUB>(a.w, reinterpret_cast<float4 *>(a.wsum), p.M, p.N, p.K, (int)(c - p.end[1]));
     else if (c < p.end[3]) quad_table<SUB>(a.gamma, a.beta, a.gbt, p.M, p.N, p.K, (int)(c - p.end[2]));
-    else to_il4(a.x, reinterpret_cast<float4 *>(a.il), a.B, (size_t)p.M * p.N * p.K, (int)((c - p.end[3]) / p.parts), (c - p.end[3]) % p.parts);
+    else to_il4(a.x, reinterpret_cast<float4 *>(a.il), a.B, P, (int)((c - p.end[3]) / p.parts), (c - p.end[3]) % p.parts);
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------
@@ -638,8 +644,8 @@ size_t quad_packed_floats(int M, int N, int K) { return (size_t)(M / 8) * (N / 8
 int launch_quad_prepare(const QuadPrepare &a, int M, int N, int K, int block, cudaStream_t st)
 {
     const unsigned regions = (unsigned)((M / 8) * (N / 8) * (K / 8));
-    PrepareArgs p{a, M, N, K, {}, (unsigned)(((long long)M * N * K + 255) / 256)};
-    const unsigned long long jobs[5] = {a.packed ? regions * kPackCtas : 0u, a.packed_t ? regions * kPackCtas : 0u,
+    PrepareArgs p{a, M, N, K, {}, (unsigned)(((long long)M * N * K + 255) / 256), regions * kPackCtas, a.gated ? 2 : 1};
+    const unsigned long long jobs[5] = {a.packed ? p.pack * p.branches : 0u, a.packed_t ? p.pack * p.branches : 0u,
                                         a.wsum ? (regions + 1) / 2 : 0u, a.gbt ? regions : 0u,
                                         a.il ? (unsigned long long)p.parts * ((a.B + 3) / 4) : 0u};
     unsigned long long n = 0;

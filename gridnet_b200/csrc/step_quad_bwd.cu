@@ -59,31 +59,6 @@ struct QuadRevParams {
     long long nitems;
 };
 
-template <int ACT>
-__device__ __forceinline__ void act_both2(u64 h, u64 &f, u64 &d)
-{
-    if (ACT == GN_ACT_SILU) {
-        const u64 t = fmul2(h, pack2(-1.4426950408889634f, -1.4426950408889634f));
-        float t0, t1, e0, e1, r0, r1, d0, d1;
-        unpack2(t, t0, t1);
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e0) : "f"(t0));
-        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e1) : "f"(t1));
-        unpack2(fadd2(pack2(e0, e1), pack2(1.0f, 1.0f)), d0, d1);
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(d0));
-        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r1) : "f"(d1));
-        const u64 r = pack2(r0, r1);
-        f = fmul2(h, r);
-        d = ffma2r(f, ffma2r(r, pack2(-1.0f, -1.0f), pack2(1.0f, 1.0f)), r);  // sg (1 + h (1 - sg))
-        return;
-    }
-    float h0, h1, f0, f1, d0, d1;
-    unpack2(h, h0, h1);
-    Act<ACT, float>::both(h0, f0, d0);
-    Act<ACT, float>::both(h1, f1, d1);
-    f = pack2(f0, f1);
-    d = pack2(d0, d1);
-}
-
 // BLOCK_NORM: the input of iteration t's sums was (tile - mean) inv with inv = 1 / (std + eps). With Gin the gradient of that
 // input, a tile cell's gradient is inv Gin - P1 - P2 (x - mean), P1 = inv sum(Gin) / cells, P2 = inv sum(Gin in) /
 // (cells std), and both sums are sums over the block's neurons: sum(Gin) = sum raw W (W the neuron's weights added up), sum(Gin
@@ -428,6 +403,7 @@ struct QuadWgradParams {
     const float *scale;      // [M][N][K]
     const float *dsq;        // [Q][P]
     const float4 *tile_stats;  // NORM: [inner][Q][tiles][QS_COUNT]
+    const float *delta2;       // GATED: of the gate
     float *gpk;              // [chunks][regions][GRAD_F]
     int accumulate;          // add to what is there
     int *error_flag;
@@ -437,7 +413,8 @@ struct QuadWgradParams {
 // NORM: per-block normalisation. The deltas are already scaled by 1 / (std + eps). The tile is kept relative to its mean before the
 // first iteration, v - c, and sum delta (v - mean_t) = sum delta (v - c) - sum delta (mean_t - c): the second sum is one
 // number per neuron, taken off all its 27 sums at the end. The bias gradient wants the unscaled delta back.
-template <int SUB, int ACT, bool FUSE_IN, bool NORM>
+// GATED: blockIdx.z picks the branch; h holds the activations after each iteration (they were kept), there is no scale.
+template <int SUB, int ACT, bool FUSE_IN, bool NORM, bool GATED>
 __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(const __grid_constant__ CUtensorMap in_map, const QuadWgradParams p)
 {
     using namespace quadwg;
@@ -516,13 +493,14 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
         __syncthreads();
     }
     if (tid == 0) issue(q0, 0);
-    fetch(stage_d, at(p.delta, q0, 0));
+    const float *const delta = GATED && blockIdx.z ? p.delta2 : p.delta;
+    fetch(stage_d, at(delta, q0, 0));
     fetch_stats(0, q0, 0);
     if (p.inner > 1) fetch(stage_h, at(p.h, q0, 0));
     const unsigned own0 = (unsigned)(T.cell0 + G::PLANE + G::ROW + 1) * 16u;
 
     for (int q = q0; q < q1; ++q) {
-        {  // scale terms of this quad
+        if (!GATED) {  // scale terms of this quad
             const float *s = p.dsq + (size_t)q * P + g0;
 #pragma unroll
             for (int dz = 0; dz < 2; ++dz) ds[dz] = fadd2(ds[dz], pack2(__ldg(s + dz * zs), __ldg(s + dz * zs + p.K)));
@@ -612,9 +590,13 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
                     const unsigned c = own0 + (unsigned)((n >> 1) * G::PLANE + (n & 1) * G::ROW) * 16u;
-                    const float sc = __ldg(p.scale + g0 + (n >> 1) * zs + (n & 1) * (size_t)p.K);
                     u64 h0, h1, x0, x1;
                     lds128u(stage_h + n * (THREADS * 16), h0, h1);
+                    if (GATED) {
+                        sts128u(to + c, h0, h1);
+                        continue;
+                    }
+                    const float sc = __ldg(p.scale + g0 + (n >> 1) * zs + (n & 1) * (size_t)p.K);
                     lds128u(tile + c, x0, x1);
                     sts128u(to + c, act_residual2<ACT>(h0, sc, x0), act_residual2<ACT>(h1, sc, x1));
                 }
@@ -622,11 +604,11 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
             if (NT == 1 && t > 0) __syncthreads();  // the tile is complete
             // the next iteration's data
             if (!last) {
-                fetch(stage_d + (buf_d ^ 1) * OWN, at(p.delta, q, t + 1));
+                fetch(stage_d + (buf_d ^ 1) * OWN, at(delta, q, t + 1));
                 fetch_stats(buf_d ^ 1, q, t + 1);
                 if (NT == 1 || t + 2 < p.inner) fetch(stage_h, at(p.h, q, NT == 2 ? t + 1 : t));
             } else if (q + 1 < q1) {
-                fetch(stage_d + (buf_d ^ 1) * OWN, at(p.delta, q + 1, 0));
+                fetch(stage_d + (buf_d ^ 1) * OWN, at(delta, q + 1, 0));
                 fetch_stats(buf_d ^ 1, q + 1, 0);
                 if (NT == 2 && p.inner > 1) fetch(stage_h, at(p.h, q + 1, 0));
                 if (NT == 2 && tid == 0) issue(q + 1, buf_x ^ 1);
@@ -678,7 +660,7 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
         }
     }
     // ---- sums -> this chunk's part: [tap][n] then [bias | scale][n], 128 threads each
-    float *const dst = p.gpk + ((size_t)blockIdx.y * gridDim.x + blk) * GRAD_F + tid;
+    float *const dst = p.gpk + (((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blk) * GRAD_F + tid;
     auto put = [&](int k, float v) { dst[k * THREADS] = p.accumulate ? dst[k * THREADS] + v : v; };
 #pragma unroll
     for (int dz = 0; dz < 2; ++dz) {
@@ -706,6 +688,7 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
         unpack2(db[dz], lo, hi);
         put(108 + dz * 2, lo);
         put(109 + dz * 2, hi);
+        if (GATED) continue;
         unpack2(ds[dz], lo, hi);
         put(112 + dz * 2, lo);
         put(113 + dz * 2, hi);
@@ -714,12 +697,13 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
 }
 
 // The chunks' sums in chunk order -> gradients in the layout of the parameters. Two regions per CTA
-// of 256 threads, four CTAs side by side; the CTAs after those put the input's gradient back into the grid's own layout.
+// of 256 threads, four CTAs side by side, branch after branch;
+// the CTAs after those put the input's gradient back into the grid's own layout.
 constexpr int kUnpack = 29;  // of the 116 values per thread
 template <int SUB>
 __global__ void __launch_bounds__(256) quad_finish_k(const float *__restrict__ gpk, float *__restrict__ gw, float *__restrict__ gb,
                                                      float *__restrict__ gs, const float4 *__restrict__ il, float *__restrict__ x, int B, int M,
-                                                     int N, int K, int chunks, unsigned grads, unsigned parts)
+                                                     int N, int K, int chunks, int branches, unsigned grads, unsigned parts)
 {
     using namespace quadwg;
     if (blockIdx.x >= grads) {
@@ -735,22 +719,24 @@ __global__ void __launch_bounds__(256) quad_finish_k(const float *__restrict__ g
         return;
     }
     const int tid = threadIdx.x & 127, regions = (M >> 3) * (N >> 3) * (K >> 3);
+    const unsigned per = grads / branches, cta = blockIdx.x % per, branch = blockIdx.x / per;
     const Patch<SUB> T(tid);
-    const int nbx = K >> 3, nby = N >> 3, blk = blockIdx.x / (116 / kUnpack) * 2 + (threadIdx.x >> 7);
+    const int nbx = K >> 3, nby = N >> 3, blk = cta / (116 / kUnpack) * 2 + (threadIdx.x >> 7);
     if (blk >= regions) return;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t P = (size_t)M * N * K;
     const size_t g0 = ((size_t)(bz * 8 + 2 * T.zp) * N + (by * 8 + 2 * T.yp)) * K + bx * 8 + T.x;
-    const float *src = gpk + (size_t)blk * GRAD_F + tid;
+    const float *src = gpk + ((size_t)branch * chunks * regions + blk) * GRAD_F + tid;
     const size_t step = (size_t)regions * GRAD_F;
-    const int k0 = blockIdx.x % (116 / kUnpack) * kUnpack;
+    const int k0 = cta % (116 / kUnpack) * kUnpack;
 #pragma unroll
     for (int i = 0; i < kUnpack; ++i) {
         const int k = k0 + i;
         float v = src[k * THREADS];
         for (int c = 1; c < chunks; ++c) v += src[c * step + k * THREADS];
         const int n = k & 3;
-        float *dst = k < 108 ? gw + (size_t)(k >> 2) * P : (k < 112 ? gb : gs);
+        if (branches > 1 && k >= 112) break;  // no scale
+        float *dst = k < 108 ? gw + ((size_t)(k >> 2) * branches + branch) * P : (k < 112 ? gb + branch * P : gs);
         dst[g0 + (size_t)(n >> 1) * N * K + (size_t)(n & 1) * K] = v;
     }
 }
@@ -813,7 +799,7 @@ struct Terms {
 }  // namespace quadborder
 
 template <bool NORM>
-__global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict__ w, const float4 *__restrict__ dsum, float4 *__restrict__ gx,
+__global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict__ w, size_t tap, const float4 *__restrict__ dsum, float4 *__restrict__ gx,
                                                          const float4 *__restrict__ x, const float4 *__restrict__ hterm, int Q, int M, int N,
                                                          int K, int qpc)
 {
@@ -864,7 +850,7 @@ __global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict
             const bool owned = (axis == 0 || (u - d1 >= 0 && u - d1 < 8)) && (axis < 2 || (v - d2 >= 0 && v - d2 < 8));
             const int nz = bz * 8 + lz - dz, ny = by * 8 + ly - dy, nx = bx * 8 + lx - dx;
             const bool ok = owned && nz >= 0 && nz < M && ny >= 0 && ny < N && nx >= 0 && nx < K;
-            wf[e] = ok ? w[(size_t)((dz + 1) * 9 + (dy + 1) * 3 + dx + 1) * P + ((size_t)nz * N + ny) * K + nx] : 0.0f;
+            wf[e] = ok ? w[(size_t)((dz + 1) * 9 + (dy + 1) * 3 + dx + 1) * tap + ((size_t)nz * N + ny) * K + nx] : 0.0f;
         }
     }
     const int row = axis == 2 ? 8 : 10;
@@ -1256,27 +1242,27 @@ int launch_quad_reverse(const QuadReverse &a, int act, cudaStream_t st)
 
 // Into how many chunks the quads of a region go: as many as fill three CTAs per SM evenly. A chunk costs its CTA about
 // two quads' time (tile latency, sums out) and its part of the gradient, 59 KB, is written and added up once.
-static int wgrad_chunks(long long regions, int Q)
+static int wgrad_chunks(long long regions, int Q, int branches)
 {
-    const int c = pick_batch_chunks_balanced(regions, Q, quadwg::CTAS, 2.0, 16);
+    const int c = pick_batch_chunks_balanced(regions * branches, Q, quadwg::CTAS, 2.0, 16);
     const int qpc = (Q + c - 1) / c;
     return (Q + qpc - 1) / qpc;
 }
 
-size_t quad_grad_floats(int M, int N, int K, int Q)
+size_t quad_grad_floats(int M, int N, int K, int Q, int branches)
 {
     const long long regions = regions_of(M, N, K);
-    return (size_t)wgrad_chunks(regions, Q) * regions * quadwg::GRAD_F;
+    return (size_t)branches * wgrad_chunks(regions, Q, branches) * regions * quadwg::GRAD_F;
 }
 
-template <int SUB, int ACT, bool FUSE_IN, bool NORM>
+template <int SUB, int ACT, bool FUSE_IN, bool NORM, bool GATED = false>
 static int launch_wgrad_in(const CUtensorMap &map, const QuadWgradParams &p, dim3 grid, cudaStream_t st)
 {
     constexpr int smem = quadwg::Lay<SUB>::smem(FUSE_IN, NORM);
     static unsigned long long done = 0;
-    const int rc = smem_once(quad_wgrad_k<SUB, ACT, FUSE_IN, NORM>, smem, &done, "cudaFuncSetAttribute(quad_wgrad_k)");
+    const int rc = smem_once(quad_wgrad_k<SUB, ACT, FUSE_IN, NORM, GATED>, smem, &done, "cudaFuncSetAttribute(quad_wgrad_k)");
     if (rc != GN_OK) return rc;
-    quad_wgrad_k<SUB, ACT, FUSE_IN, NORM><<<grid, quadwg::THREADS, smem, st>>>(map, p);
+    quad_wgrad_k<SUB, ACT, FUSE_IN, NORM, GATED><<<grid, quadwg::THREADS, smem, st>>>(map, p);
     return check_launch("quad_wgrad");
 }
 template <int SUB, int ACT>
@@ -1306,33 +1292,38 @@ int launch_quad_wgrad(const QuadWgrad &a, int act, cudaStream_t st)
     if (rc != GN_OK) return rc;
     QuadWgradParams p{};
     p.gbt = a.gbt; p.in_stats = a.in_stats; p.delta = a.delta; p.h = a.h; p.scale = a.scale; p.dsq = a.dsq; p.gpk = a.gpk;
-    p.tile_stats = a.tile_stats;
+    p.tile_stats = a.tile_stats; p.delta2 = a.delta2;
     p.accumulate = a.accumulate;
     p.error_flag = a.error_flag ? a.error_flag : device_status_ptr();
     p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;
     const long long regions = regions_of(a.M, a.N, a.K);
-    const int chunks = wgrad_chunks(regions, a.Q);
+    const int branches = a.delta2 ? 2 : 1, chunks = wgrad_chunks(regions, a.Q, branches);
     p.qpc = (a.Q + chunks - 1) / chunks;
-    const dim3 grid((unsigned)regions, (unsigned)chunks);
+    const dim3 grid((unsigned)regions, (unsigned)chunks, branches);
+    if (a.delta2) {
+        if (a.block != 8 || a.tile_stats) return GN_ERR_UNSUPPORTED;
+        return a.in_stats ? launch_wgrad_in<8, GN_ACT_RELU, true, false, true>(map, p, grid, st)
+                          : launch_wgrad_in<8, GN_ACT_RELU, false, false, true>(map, p, grid, st);
+    }
     return a.block == 8 ? launch_wgrad_sub<8>(map, p, grid, act, st) : launch_wgrad_sub<4>(map, p, grid, act, st);
 }
 
 int launch_quad_finish(const float *gpk, float *gw, float *gb, float *gs, const float *il, float *x, int B, int M, int N, int K, int block,
-                       cudaStream_t st)
+                       int branches, cudaStream_t st)
 {
     const long long regions = regions_of(M, N, K);
-    const int chunks = wgrad_chunks(regions, (B + 3) / 4);
-    const unsigned grads = (unsigned)((regions + 1) / 2) * (116 / kUnpack), parts = (unsigned)(((long long)M * N * K + 255) / 256);
+    const int chunks = wgrad_chunks(regions, (B + 3) / 4, branches);
+    const unsigned grads = (unsigned)(branches * ((regions + 1) / 2) * (116 / kUnpack)), parts = (unsigned)(((long long)M * N * K + 255) / 256);
     const unsigned long long n = grads + (il ? (unsigned long long)parts * ((B + 3) / 4) : 0);
     if (n >= 1ull << 31) return GN_ERR_UNSUPPORTED;
     const float4 *const i4 = reinterpret_cast<const float4 *>(il);
-    if (block == 8) quad_finish_k<8><<<(unsigned)n, 256, 0, st>>>(gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, grads, parts);
-    else quad_finish_k<4><<<(unsigned)n, 256, 0, st>>>(gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, grads, parts);
+    if (block == 8) quad_finish_k<8><<<(unsigned)n, 256, 0, st>>>(gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, branches, grads, parts);
+    else quad_finish_k<4><<<(unsigned)n, 256, 0, st>>>(gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, branches, grads, parts);
     return check_launch("quad_finish");
 }
 
 template <bool NORM>
-static int launch_border(const float *w, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K, int Q,
+static int launch_border(const float *w, size_t tap, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K, int Q,
                          int block, cudaStream_t st)
 {
     const long long nb = regions_of(M, N, K);
@@ -1347,7 +1338,7 @@ static int launch_border(const float *w, const float *dsum, float *gx, const flo
         constexpr int smem = (quadborder::RING * (quadborder::SHELL + (NORM ? 2 : 1) * quadborder::SURFACE) + 2 * 3 * 128) * 16;
         const int rc = smem_once(quad_border8_k<NORM>, smem, &done[0], "cudaFuncSetAttribute(quad_border8_k)");
         if (rc != GN_OK) return rc;
-        quad_border8_k<NORM><<<grid, 384, smem, st>>>(w, d4, g4, x4, hterm, Q, M, N, K, qpc);
+        quad_border8_k<NORM><<<grid, 384, smem, st>>>(w, tap, d4, g4, x4, hterm, Q, M, N, K, qpc);
     } else {
         constexpr int smem = 2 * quadborder::TS * 16;
         const int rc = smem_once(quad_border4_k<NORM>, smem, &done[1], "cudaFuncSetAttribute(quad_border4_k)");
@@ -1357,11 +1348,13 @@ static int launch_border(const float *w, const float *dsum, float *gx, const flo
     return check_launch("quad_border");
 }
 
-int launch_quad_border(const float *w, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K, int Q,
-                       int block, cudaStream_t st)
+int launch_quad_border(const float *w, int branches, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
+                       int Q, int block, cudaStream_t st)
 {
-    return hterm ? launch_border<true>(w, dsum, gx, x_il4, hterm, M, N, K, Q, block, st)
-                 : launch_border<false>(w, dsum, gx, nullptr, nullptr, M, N, K, Q, block, st);
+    const size_t tap = (size_t)M * N * K * branches;
+    if (branches > 1 && block != 8) return GN_ERR_UNSUPPORTED;
+    return hterm ? launch_border<true>(w, tap, dsum, gx, x_il4, hterm, M, N, K, Q, block, st)
+                 : launch_border<false>(w, tap, dsum, gx, nullptr, nullptr, M, N, K, Q, block, st);
 }
 
 int quad_norm_parts(long long P)

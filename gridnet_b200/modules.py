@@ -13,7 +13,7 @@ from typing import Tuple
 import torch
 import torch.nn as nn
 
-from .backend_cuda import FusedLoopTrainOp, GatedGridnetCudaOp, GridnetCudaOp, GridNormOp, outer_forward
+from .backend_cuda import FusedGatedLoopTrainOp, FusedLoopTrainOp, GatedGridnetCudaOp, GridnetCudaOp, GridNormOp, outer_forward
 
 
 def _need_cuda(t: torch.Tensor, what: str) -> None:
@@ -97,14 +97,20 @@ class Readout(nn.Module):
         return self.proj(self.norm(x[:, :, :, -self.output_layers:].flatten(1)))
 
 
+def fused_gated_applies(network: nn.Module, h: torch.Tensor) -> bool:
+    """Whether a loop over a gated network runs as one call (:class:`FusedGatedLoopTrainOp`, with and without gradients)."""
+    return (isinstance(network, GatedGridnet) and h.dtype == torch.float32
+            and FusedGatedLoopTrainOp.supported(network.weight, h, network.inner_iterations, network.block_size))
+
+
 class GridnetModel(nn.Module):
     """The loop of the reference's scripts: ``for _ in range(outer_iters): h = network(h); h = norm(h)``
     (gridnet/scripts/train_mnist.py:62-64), with submodules named ``network`` and ``norm`` as there.
 
     A plain float32 network with per-block normalisation off runs fused: with gradients disabled as ONE call
     (:func:`outer_forward`), with gradients as one autograd node over the whole loop (:class:`FusedLoopTrainOp`:
-    statistics out of the step kernels, normalisation on load, only raw step outputs saved). Everything else is
-    the step-by-step composition of the two autograd ops."""
+    statistics out of the step kernels, normalisation on load, only raw step outputs saved). So does a gated float32 network
+    with blocks of 8 (:class:`FusedGatedLoopTrainOp`). Everything else is the step-by-step composition of the two autograd ops."""
 
     def __init__(self, shape: Tuple[int, int, int], inner_iters: int, outer_iters: int, block_size: int, device,
                  init_scale: float = 1.0, residual_scale: float = 1.0, activation: str = "silu", gated: bool = False,
@@ -131,6 +137,9 @@ class GridnetModel(nn.Module):
             return FusedLoopTrainOp.apply(net.weight, net.bias, net.residual_scale, self.norm.weight, self.norm.bias, h,
                                           net.inner_iterations, self.outer_iters, net.block_size, net.activation,
                                           self.norm.eps)
+        if fused_gated_applies(net, h):
+            return FusedGatedLoopTrainOp.apply(net.weight, net.bias, self.norm.weight, self.norm.bias, h, net.inner_iterations,
+                                               self.outer_iters, net.block_size, net.activation, self.norm.eps)
         for _ in range(self.outer_iters):
             h = self.norm(net(h))
         return h

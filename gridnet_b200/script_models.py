@@ -16,9 +16,9 @@ from __future__ import annotations
 import torch
 import torch.nn as nn
 
-from .backend_cuda import (FusedLoopResidualTrainOp, FusedLoopSeparateTrainOp, FusedLoopTrainOp, fused_loop_forward,
+from .backend_cuda import (FusedGatedLoopTrainOp, FusedLoopResidualTrainOp, FusedLoopSeparateTrainOp, FusedLoopTrainOp, fused_loop_forward,
                            outer_forward)
-from .modules import GatedGridnet, Gridnet, GridNorm, Readout
+from .modules import GatedGridnet, Gridnet, GridNorm, Readout, fused_gated_applies
 
 
 def _wants_grad(module: nn.Module, *tensors: torch.Tensor) -> bool:
@@ -38,6 +38,9 @@ def _plain_loop(network: nn.Module, norm: GridNorm, h: torch.Tensor, outer_iters
         return FusedLoopTrainOp.apply(network.weight, network.bias, network.residual_scale, norm.weight, norm.bias, h,
                                       network.inner_iterations, outer_iters, network.block_size, network.activation,
                                       norm.eps)
+    if fused_gated_applies(network, h):
+        return FusedGatedLoopTrainOp.apply(network.weight, network.bias, norm.weight, norm.bias, h, network.inner_iterations,
+                                           outer_iters, network.block_size, network.activation, norm.eps)
     for _ in range(outer_iters):
         h = norm(network(h))
     return h

@@ -513,6 +513,17 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
                          int outer, int block, int activation, int residual, void *workspace, size_t workspace_bytes,
                          void *stream);
 
+/* The gated loop, h = layer_norm(gated_step(h)), block 8, shared parameters (weight [27][2][M][N][K], bias [2][M][N][K]): as
+ * the plain loop above, with 3 * inner tensors per stash. */
+GN_API size_t gn_gated_loop_workspace_bytes(int B, int M, int N, int K, int inner, int outer, int backward, int replay);
+GN_API int gn_gated_loop_forward_f32(const float *weight, const float *bias, const float *gamma, const float *beta, const float *x, float *y,
+                                     float *x_il4, float *const *outs, float *stats, float *const *stashes, int B, int M, int N, int K,
+                                     int inner, int outer, float ln_eps, int act, void *workspace, size_t workspace_bytes, void *stream);
+GN_API int gn_gated_loop_backward_f32(const float *weight, const float *bias, const float *gamma, const float *beta, const float *x_il4,
+                                      float *const *outs, const float *stats, float *const *stashes, const float *gy, float *gw, float *gb,
+                                      float *ggamma, float *gbeta, float *gx, int B, int M, int N, int K, int inner, int outer, int act,
+                                      void *workspace, size_t workspace_bytes, void *stream);
+
 #ifdef __cplusplus
 }
 #endif

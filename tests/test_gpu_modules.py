@@ -7,6 +7,8 @@ import torch
 
 from oracle import gridnet_oracle as orc
 
+from util import assert_close
+
 pytestmark = pytest.mark.gpu
 
 
@@ -251,3 +253,36 @@ def test_training_configurations_at_their_own_grid_and_depth(name, grid, block, 
     # the float32 oracle's worst error 1.3e-3, ours 3.0e-3, i.e. 7e-7 of max|ref|; 25 against 29 elements outside)
     for label, g, r64, r32 in zip(("weight", "bias", "scale", "gamma", "beta", "input"), grads, want64, want32):
         assert_close(g.cpu().numpy(), r64, r32, f"{name} gradient of {label}", noise_factor=3.0)
+
+
+@pytest.mark.parametrize("keep", [True, False])
+@pytest.mark.parametrize("shape,batch,inner,outer,act", [((8, 16, 24), 5, 1, 2, "tanh"), ((24, 8, 8), 2, 3, 3, "silu"), ((16, 16, 8), 9, 2, 1, "leaky_relu")])
+def test_gated_loop_matches_oracle(shape, batch, inner, outer, act, keep):
+    """The gated loop as one autograd node, ragged quads, kept iterations and replay, against the float64 oracle."""
+    import gridnet_b200 as gb
+
+    r = np.random.default_rng(11)
+    w = (r.standard_normal((27, 2, *shape)) / np.sqrt(27)).astype(np.float32)
+    b, x, gy = ((0.3 * r.standard_normal(n)).astype(np.float32) for n in ((2, *shape), (batch, *shape), (batch, *shape)))
+    ga, be = (1 + 0.1 * r.standard_normal(shape)).astype(np.float32), (0.1 * r.standard_normal(shape)).astype(np.float32)
+    t = [torch.from_numpy(a).cuda().requires_grad_(True) for a in (w, b, ga, be, x)]
+    previous = gb.keep_forward_stash(keep)
+    try:
+        y = gb.FusedGatedLoopTrainOp.apply(*t, inner, outer, 8, act, 1e-5)
+        y.backward(torch.from_numpy(gy).cuda())
+    finally:
+        gb.keep_forward_stash(previous)
+    w, b, ga, be, h, g = (a.astype(np.float64) for a in (w, b, ga, be, x, gy))
+    ins, mids = [], []
+    for _ in range(outer):
+        ins.append(h)
+        mids.append(orc.gated_forward(w, b, h, inner, 8, act))
+        h = orc.layernorm_forward(mids[-1], ga, be)
+    assert_close(y.detach().cpu().numpy(), h, None, "y")
+    sums = [0.0] * 4
+    for k in reversed(range(outer)):
+        g, dga, dbe = orc.layernorm_backward(mids[k], ga, g)
+        dw, db, g = orc.gated_backward(w, b, ins[k], g, inner, 8, act)
+        sums = [s + d for s, d in zip(sums, (dw, db, dga, dbe))]
+    for got, ref, name in zip(t, (*sums, g), ("weight", "bias", "norm.weight", "norm.bias", "x")):
+        assert_close(got.grad.cpu().numpy(), ref, None, f"grad {name}")
