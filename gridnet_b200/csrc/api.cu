@@ -192,6 +192,8 @@ struct OuterWs {
     float *qpacked;     // weights in the quad kernel's order
     float2 *gbt;        // (gamma, beta) per tile cell of every 8^3 region, for the quad kernel
     int *error_flag;
+    unsigned long long *small_sums, *small_cells;  // what the blocks tell each other in the one-kernel loop; right behind the flag
+    size_t small_bytes;
     size_t bytes;
 };
 
@@ -222,7 +224,12 @@ static OuterWs carve_outer(void *base, int B, int M, int N, int K, int block)
     w.gbt = (float2 *)(p + off);
     if (regions) off = align_up(off + sizeof(float2) * (size_t)(M / 8) * (N / 8) * (K / 8) * quad_tile_cells(block), 256);
     w.error_flag = (int *)(p + off);
-    off = align_up(off + sizeof(int), 256);
+    off += 128;
+    w.small_sums = (unsigned long long *)(p + off);
+    const bool small = pair && (long long)B * P <= kOuterSmallMaxCells;
+    w.small_cells = w.small_sums + 2 * kOuterSmallLine * nb * B;
+    w.small_bytes = small ? sizeof(unsigned long long) * (2 * kOuterSmallLine * nb * B + 2 * B * P) : 0;
+    off = align_up(off + w.small_bytes, 256);
     w.bytes = off;
     return w;
 }
@@ -1002,15 +1009,13 @@ static int outer_forward_impl(const float *w, const float *b, const float *s, co
     if (g_outer_kernel == 0 || g_outer_kernel == 3) {
         const int spc = outer_small_spc(B, M, N, K, block, inner, outer, w, b, s, gamma, beta, x, y);
         if (spc > 0) {
-            // the int after the error flag is the counter of the kernel's grid-wide barrier
-            const cudaError_t e = cudaMemsetAsync(ws.error_flag, 0, 2 * sizeof(int), st);
+            const cudaError_t e = cudaMemsetAsync(ws.error_flag, 0, 128 + ws.small_bytes, st);
             if (e != cudaSuccess) {
                 record_cuda_error(e, "cudaMemsetAsync");
                 return GN_ERR_CUDA;
             }
-            return launch_outer_small(w, b, s, gamma, beta, x, y, ws.buf[0], ws.buf[1], ws.partials,
-                                      reinterpret_cast<unsigned *>(ws.error_flag + 1), ws.error_flag, B, M, N, K, inner, outer,
-                                      spc, ln_eps, act, st);
+            return launch_outer_small(w, b, s, gamma, beta, x, y, ws.small_cells, ws.small_sums, ws.error_flag, B, M, N, K,
+                                      inner, outer, spc, ln_eps, act, st);
         }
         if (g_outer_kernel == 3) return GN_ERR_UNSUPPORTED;
     }
