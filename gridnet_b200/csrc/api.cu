@@ -235,13 +235,18 @@ static OuterWs carve_outer(void *base, int B, int M, int N, int K, int block)
 }
 
 // 0 = choose automatically: the one persistent kernel of outer_small.cu for problems so small that launches are what
-// they cost; else the quad kernel of step_quad.cu from two samples up (64^3, 4 x 12 iterations, ms per loop,
-// register-patch / large-batch / quad, the latter two with the parameters re-ordered before: batch 1 0.265 / - / 0.257,
-// 4 0.445 / - / 0.261, 16 0.97 / - / 0.60, 64 2.92 / 1.87 / 1.76; 128^3, 2 x 16, batch 32: 9.85 / - / 6.06; 64^3 block 4,
-// 8 x 4, batch 128: 3.50 / - / 1.80; for one sample the re-ordering, 0.03 ms, costs more than the kernel gains); else the register-patch kernel of step_fast.cu. 1 = always the register-patch kernel, 2 = always the
-// large-batch kernel of step_pair64.cu, 3 = always the persistent kernel, 4 = always the quad kernel.
+// they cost; else the quad kernel of step_quad.cu where it has work for most of its warps; else the register-patch kernel of
+// step_fast.cu. 1 = always the register-patch kernel, 2 = always the large-batch kernel of step_pair64.cu, 3 = always the
+// persistent kernel, 4 = always the quad kernel.
+// A quad warp works on a whole 8^3 region for four samples, so fewer than about three regions x quads per SM leave it
+// idle, and a single sample fills a quarter of a lane. ms per loop, register-patch / quad: 48^3, 2 x 10, batch 3
+// (1.5 per SM) 0.154 / 0.180, batch 8 (2.9) 0.194 / 0.180, batch 32 0.40 / 0.29; 32^3, 2 x 8, batch 12 (1.3) 0.140 / 0.147, batch 32
+// (3.5) 0.190 / 0.155; 64^3, 4 x 12, batch 4 (3.5) 0.45 / 0.29, batch 64 2.92 / 1.70.
 static int g_outer_kernel = 0;
-constexpr int kQuadMinBatch = 2;
+static bool quad_wanted(int B, int M, int N, int K)
+{
+    return B >= 2 && 4LL * (M / 8) * (N / 8) * (K / 8) * ((B + 3) / 4) >= 11LL * sm_count();
+}
 
 static int check_ws(const void *ws, size_t have, size_t need)
 {
@@ -937,7 +942,7 @@ GN_API int gn_outer_forward_plan(int B, int M, int N, int K, int inner, int oute
     if ((g_outer_kernel == 0 || g_outer_kernel == 3) && outer_small_spc(B, M, N, K, block, inner, outer, a, a, a, a, a, a, a) > 0)
         return 3;
     if (g_outer_kernel == 3) return 0;
-    if (((g_outer_kernel == 0 && B >= kQuadMinBatch) || g_outer_kernel == 4) && quad_applicable(M, N, K, block, inner)) return 5;
+    if (((g_outer_kernel == 0 && quad_wanted(B, M, N, K)) || g_outer_kernel == 4) && quad_applicable(M, N, K, block, inner)) return 5;
     if (g_outer_kernel == 4) return 0;
     if (g_outer_kernel == 2) return pair64_applicable(M, N, K, block, inner) ? 2 : 0;
     FastFwdParams p{};
@@ -1020,7 +1025,7 @@ static int outer_forward_impl(const float *w, const float *b, const float *s, co
         if (g_outer_kernel == 3) return GN_ERR_UNSUPPORTED;
     }
     const bool quad_ok = quad_applicable(M, N, K, block, inner);
-    if (quad_ok && ((g_outer_kernel == 0 && B >= kQuadMinBatch) || g_outer_kernel == 4)) {
+    if (quad_ok && ((g_outer_kernel == 0 && quad_wanted(B, M, N, K)) || g_outer_kernel == 4)) {
         const int Q = (B + 3) / 4, regions = (M / 8) * (N / 8) * (K / 8);
         if (cudaMemsetAsync(ws.error_flag, 0, sizeof(int), st) != cudaSuccess) {
             record_cuda_error(cudaGetLastError(), "cudaMemsetAsync");
