@@ -57,7 +57,7 @@ FALLBACK_HBM_GBS = 6650.0
 # DRAM bytes per launch of the dominant kernel (dram__bytes_read.sum + dram__bytes_write.sum): a constant taken
 # from the ncu capture summarised in the named file, not a measurement of this run
 NCU_TRAFFIC = {
-    "step_fwd_pair64": (143.8e6, "profiles/step_fwd_pair64_c2_ncu_full.txt"),
+    "step_fwd_quad": (143.8e6, "profiles/step_fwd_quad_c2_ncu_sections.txt"),
     "step_fwd_fast8": (173.0e6, "profiles/step_fwd_fast8_c2_ncu_full.txt"),
 }
 
@@ -327,7 +327,7 @@ def bench_c2(ctx: Ctx):
     xs = [x.to(device) for x in xs_host]
     ys = [torch.empty_like(x) for x in xs]
     ws = gb.outer_forward_workspace(BATCH, GRID, BLOCK, device)
-    large_batch = bool(lib.gn_pair64_supported(GRID[0], GRID[1], GRID[2], BLOCK, INNER))
+    quad = int(lib.gn_outer_forward_plan(BATCH, *GRID, INNER, OUTER, BLOCK)) == 5
 
     def step(i):
         gb.outer_forward(w, b, s, gamma, beta, xs[i % NSETS], INNER, OUTER, BLOCK, ACT, out=ys[i % NSETS],
@@ -347,55 +347,64 @@ def bench_c2(ctx: Ctx):
     e1.record()
     ctx.barrier()
     ms = ctx.max_over_ranks(e0.elapsed_time(e1))
-    # per outer step: step kernel + statistics finalize; plus, once per forward, the layout conversion in and out
-    # (and the weight re-ordering) of the large-batch kernel, or the final normalisation of the register-patch one
-    launches_per_step = OUTER * 2 + (3 if large_batch else 1)
+    # per outer step: step kernel + statistics finalize; plus, once per forward, re-ordering into and out of the quad
+    # kernel's layout, or the final normalisation of the register-patch one
+    launches_per_step = OUTER * 2 + (2 if quad else 1)
     value = neuron_updates(BATCH) * world * args.steps / (ms * 1e-3)
     failed = gb.outer_forward_failed(ws, BATCH, GRID, BLOCK)
 
     # ---------------- the dominant kernel alone (roofline)
-    nparts = int(lib.gn_pair64_stats_partials(*GRID)) if large_batch else gb.step_stats_partials(GRID, BLOCK)
-    partials = torch.empty(BATCH, nparts, 2, dtype=torch.float64, device=device)
-    stats = torch.empty(BATCH, 2, device=device)
-    # any finite statistics do for timing: mean 0, rstd 1
-    stats[:, 0] = 0.0
-    stats[:, 1] = 1.0
     reps = max(args.steps, 3) * OUTER
-    if large_batch:
-        from gridnet_b200.backend_cuda import pair64_interleave, pair64_pack_weights, pair64_step
+    if quad:
+        # the step kernel has no entry point of its own: what one outer step more costs a loop (step kernel and the
+        # statistics of its output), from loops of 2 and of OUTER steps
+        kernel_name = "step_fwd_quad<silu, fuse_in> (with the finalize of its statistics)"
+        reps = max(args.steps, 3)
 
-        kernel_name = "step_fwd_pair64<silu, fuse_in, stats_out>"
-        packed = pair64_pack_weights(w, b, s, gamma, beta)
-        xi = [pair64_interleave(x) for x in xs]
-        yi = [torch.empty_like(x) for x in xi]
-        flag = torch.zeros(1, dtype=torch.int32, device=device)
+        def loop(i, outer):
+            gb.outer_forward(w, b, s, gamma, beta, xs[i % NSETS], INNER, outer, BLOCK, ACT, out=ys[i % NSETS], workspace=ws)
 
-        def kernel(i):
-            pair64_step(packed, xi[i % NSETS], yi[(i + 1) % NSETS], BATCH, GRID, INNER, ACT, stats, partials, flag)
+        def loop_ms(outer):
+            for i in range(3):
+                loop(i, outer)
+            torch.cuda.synchronize()
+            k0, k1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            k0.record()
+            for i in range(reps):
+                loop(i, outer)
+            k1.record()
+            torch.cuda.synchronize()
+            return k0.elapsed_time(k1) / reps
+
+        kms = (loop_ms(OUTER) - loop_ms(2)) / (OUTER - 2)
     else:
+        nparts = gb.step_stats_partials(GRID, BLOCK)
+        partials = torch.empty(BATCH, nparts, 2, dtype=torch.float64, device=device)
+        stats = torch.empty(BATCH, 2, device=device)
+        # any finite statistics do for timing: mean 0, rstd 1
+        stats[:, 0] = 0.0
+        stats[:, 1] = 1.0
         kernel_name = "step_fwd_fast8<silu, fuse_in, stats_out>"
 
         def kernel(i):
             gb.fused_step(w, b, s, xs[i % NSETS], ys[(i + 1) % NSETS], INNER, BLOCK, ACT, gamma, beta, stats, partials)
 
-    for i in range(6):
-        kernel(i)
-    torch.cuda.synchronize()
-    k0, k1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-    k0.record()
-    for i in range(reps):
-        kernel(i)
-    k1.record()
-    torch.cuda.synchronize()
-    kms = k0.elapsed_time(k1) / reps
-    if large_batch:
-        del xi, yi, packed
+        for i in range(6):
+            kernel(i)
+        torch.cuda.synchronize()
+        k0, k1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        k0.record()
+        for i in range(reps):
+            kernel(i)
+        k1.record()
+        torch.cuda.synchronize()
+        kms = k0.elapsed_time(k1) / reps
     fp32_measured = measure_fp32_peak(torch, device)
     hbm_peak, peak_kind, sm_max_mhz = measured_peaks()
     ach_gbs = algorithmic_bytes_per_launch(BATCH) / (kms * 1e-3) / 1e9
     fp32_nominal = FP32_LANES * 2 * sm_max_mhz * 1e6 / 1e12
     ach_tflops = 2 * algorithmic_fma_per_launch(BATCH) / (kms * 1e-3) / 1e12
-    traffic, traffic_src = NCU_TRAFFIC["step_fwd_pair64" if large_batch else "step_fwd_fast8"]
+    traffic, traffic_src = NCU_TRAFFIC["step_fwd_quad" if quad else "step_fwd_fast8"]
     fp32 = {"bound": "fp32", "achieved": ach_tflops, "peak": fp32_measured, "unit": "TFLOP/s",
             "frac": ach_tflops / fp32_measured,
             "peak_source": "measured in this run: FFMA-only kernel on every SM, CUDA events (gn_probe_fp32_fma)",
@@ -496,7 +505,7 @@ def bench_c2(ctx: Ctx):
         "config": {"workload": WORKLOAD, "global_batch": BATCH * world, "parallelism": f"batch-sharded x{world}",
                    "l2": f"{NSETS} rotating input/output sets (4 x 67 MB each way) plus a 300 MB working set per step, larger than the 126 MB L2",
                    "samples_per_sec": BATCH * world * args.steps / (ms * 1e-3),
-                   "step_kernel": "large-batch (step_pair64.cu)" if large_batch else "register-patch (step_fast.cu)",
+                   "step_kernel": "weights in tensor memory (step_quad.cu)" if quad else "register-patch (step_fast.cu)",
                    "device_failure_flag": failed},
         "roofline": roofline, "e2e": e2e, "cpu_baseline": cpu,
         "gpu_launches": launches_per_step * args.steps, "clocks": clocks,
@@ -931,7 +940,7 @@ def bench_c1(ctx: Ctx):
     from gridnet_b200._lib import lib
 
     plan = int(lib.gn_outer_forward_plan(B, G, G, G, inner, outer, block))
-    launches = {3: 1, 2: 2 * outer + 3, 1: 2 * outer + 1}.get(plan, 4 * outer)
+    launches = {3: 1, 5: 2 * outer + 2, 2: 2 * outer + 3, 1: 2 * outer + 1}.get(plan, 4 * outer)
     if True:
         return ({
             "metric": METRIC, "value": nu / (graph_ms * 1e-3), "unit": UNIT, "n_gpus": 1, "steps": steps,
@@ -940,6 +949,7 @@ def bench_c1(ctx: Ctx):
             "config": {"workload": "C1: 32^3 grid, block 8, 2 inner x 8 outer, batch 8, fp32, forward + whole-grid "
                                    "LayerNorm per outer step; replayed from a CUDA graph",
                        "kernel": {3: "one persistent cooperative kernel over all outer steps (outer_small.cu)",
+                                  5: "quad kernel, one launch per outer step",
                                   2: "large-batch kernel, one launch per outer step",
                                   1: "register-patch kernel, one launch per outer step"}.get(plan, "generic kernels"),
                        "launch_by_launch_ms": eager_ms, "graph_replay_ms": graph_ms,
