@@ -1047,6 +1047,7 @@ static int outer_forward_impl(const float *w, const float *b, const float *s, co
             a.in_stats = o > 0 ? ws.stats : nullptr;
             a.out_partials = ws.partials;
             a.nparts = regions;
+            a.params_old = o > 0;
             a.error_flag = ws.error_flag;
             a.M = M; a.N = N; a.K = K; a.Q = Q; a.inner = inner; a.block = block;
             rc = launch_step_fwd_quad(a, act, st);

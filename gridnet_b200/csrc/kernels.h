@@ -144,6 +144,7 @@ struct QuadStep {
     double2 *out_partials;    // [4 Q][nparts] or nullptr; slots 0 .. regions-1 of every row are written
     int nparts;
     float *save_h;            // [inner] IL4 tensors of pre-activations, or nullptr
+    bool params_old;          // packed and gbt are not what the kernel queued just before writes
     const float *wsum;        // from launch_quad_prepare: per-block normalisation; nullptr: off
     float4 *tile_stats;       // with wsum and save_h: quad_stats_vectors(...) vectors
     float eps;

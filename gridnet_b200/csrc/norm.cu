@@ -53,13 +53,14 @@ __global__ void __launch_bounds__(256) norm_partial_stats_k(const float *__restr
 // grid B; adds nparts partials in a fixed order. One CTA reads a whole row, so what bounds a long row is how many of
 // its loads are in flight: 1024 threads with four each (256 threads with one each took 241 us for 32 rows of 32768 to
 // 131072 partials)
-__global__ void __launch_bounds__(1024) norm_finalize_k(const double2 *__restrict__ partials, int nparts,
-                                                       float2 *__restrict__ stats, long long P, float eps)
+__global__ void __launch_bounds__(1024) norm_finalize_k(const double2 *partials, int nparts, float2 *stats,  // no read-only loads: written just before
+                                                       long long P, float eps)
 {
     __shared__ double red[33];
     const int b = blockIdx.x;
     const double2 *ps = partials + (size_t)b * nparts;
     double s = 0.0, q = 0.0;
+    previous_done();
 #pragma unroll 4
     for (int i = threadIdx.x; i < nparts; i += blockDim.x) {
         const double2 v = ps[i];
@@ -77,13 +78,13 @@ __global__ void __launch_bounds__(1024) norm_finalize_k(const double2 *__restric
 }
 
 // grid B * ceil(P / 1024), one dimension
-__global__ void __launch_bounds__(256) norm_apply_k(const float *__restrict__ x, const float *__restrict__ gamma,
+__global__ void __launch_bounds__(256) norm_apply_k(const float *x, const float *__restrict__ gamma,
                                                     const float *__restrict__ beta,
-                                                    const float2 *__restrict__ stats, float *__restrict__ y,
-                                                    long long P, unsigned chunks)
+                                                    const float2 *stats, float *y, long long P, unsigned chunks)
 {
     const int b = blockIdx.x / chunks;
     const unsigned chunk = blockIdx.x - (unsigned)b * chunks;
+    previous_done();
     const float2 mr = stats[b];
     const float *xs = x + (size_t)b * P;
     float *ys = y + (size_t)b * P;
@@ -268,7 +269,7 @@ int launch_norm_partial_stats(const float *x, double2 *partials, int B, long lon
 int launch_norm_finalize(const double2 *partials, int nparts, float2 *stats, int B, long long P, float eps,
                          cudaStream_t st)
 {
-    norm_finalize_k<<<B, nparts >= 2048 ? 1024 : 256, 0, st>>>(partials, nparts, stats, P, eps);
+    launch_after(norm_finalize_k, B, nparts >= 2048 ? 1024 : 256, 0, st, partials, nparts, stats, P, eps);
     return check_launch("norm_finalize");
 }
 
@@ -276,7 +277,7 @@ int launch_norm_apply(const float *x, const float *gamma, const float *beta, con
                       int B, long long P, cudaStream_t st)
 {
     const unsigned chunks = (unsigned)((P + 1023) / 1024);
-    norm_apply_k<<<(unsigned)B * chunks, 256, 0, st>>>(x, gamma, beta, stats, y, P, chunks);
+    launch_after(norm_apply_k, (unsigned)B * chunks, 256, 0, st, x, gamma, beta, stats, y, P, chunks);
     return check_launch("norm_apply");
 }
 

@@ -208,6 +208,7 @@ GN_API int gn_loop_forward_f32(const float *const *weights, const float *const *
         a.in_stats = residual ? mr + (size_t)k * S : (k ? mr + (size_t)(k - 1) * S : nullptr);
         a.out_partials = residual ? nullptr : w.partials;
         a.nparts = d.regions;
+        a.params_old = k > 0 && nparams == 1;
         if (stashes) a.save_h = stashes[k];
         a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;
         TRY_(launch_step_fwd_quad(a, act, st));

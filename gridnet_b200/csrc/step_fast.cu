@@ -277,9 +277,11 @@ __global__ void __launch_bounds__(fast8::THREADS, fast8::MIN_CTAS)
             fence_proxy_async();
         }
         __syncthreads();
+        previous_done();
         prefetch(s0);
         prefetch(s0 + 1);
     } else {
+        previous_done();
         prefetch(s0);
     }
     load_stats(s0);
@@ -599,7 +601,10 @@ int launch_step_fwd_fast8(FastFwdParams p, int act, cudaStream_t st)
             if (!tma) return GN_ERR_UNSUPPORTED;                                                          \
             if (p.inner == 8) SUB4_(A, FI, SO, 8);                                                        \
             else SUB4_(A, FI, SO, 0);                                                                     \
-        } else if (tma && p.inner == 4) step_fwd_fast8<8, A, FI, SO, true, 4><<<grid, fast8::THREADS, 0, st>>>(map, p);  \
+        } else if (tma && FI && SO && p.inner == 4) launch_after(step_fwd_fast8<8, A, FI, SO, true, 4>, grid, fast8::THREADS, 0, st, map, p); \
+        else if (tma && FI && SO && p.inner == 2) launch_after(step_fwd_fast8<8, A, FI, SO, true, 2>, grid, fast8::THREADS, 0, st, map, p); \
+        else if (tma && FI && SO) launch_after(step_fwd_fast8<8, A, FI, SO, true, 0>, grid, fast8::THREADS, 0, st, map, p); \
+        else if (tma && p.inner == 4) step_fwd_fast8<8, A, FI, SO, true, 4><<<grid, fast8::THREADS, 0, st>>>(map, p);  \
         else if (tma && p.inner == 2) step_fwd_fast8<8, A, FI, SO, true, 2><<<grid, fast8::THREADS, 0, st>>>(map, p); \
         else if (tma) step_fwd_fast8<8, A, FI, SO, true, 0><<<grid, fast8::THREADS, 0, st>>>(map, p);     \
         else step_fwd_fast8<8, A, FI, SO, false, 0><<<grid, fast8::THREADS, 0, st>>>(map, p);             \

@@ -49,6 +49,7 @@ struct QuadParams {
     float *save_h;           // SAVE: [inner][Q][P][4]
     int *error_flag;
     int M, N, K, Q, inner;
+    int params_old;          // the kernel before this one did not write packed or gbt
     long long nitems;        // regions * Q
 };
 
@@ -142,9 +143,13 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
         if (spins >= kSpinLimit || !mbar_wait_bounded(bar0 + 8 * (i % NBUF), (unsigned)(i / NBUF) & 1u, kSpinLimit)) failed = true;
         __syncwarp();
     };
-    if (role == 0 && lane == 0)
-        for (int i = 0; i < NBUF && i < cnt; ++i) issue(i);
-    __syncwarp();
+    auto begin = [&]() {
+        previous_done();
+        if (role == 0 && lane == 0)
+            for (int i = 0; i < NBUF && i < cnt; ++i) issue(i);
+        __syncwarp();
+    };
+    if (!p.params_old || cnt == 0) begin();  // else the first region's parameters come first
 
     int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
     for (int i0 = 0; i0 < cnt;) {
@@ -166,6 +171,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
         if (NORM && role == 0) quad_load_wsum(p.wsum, blk, lane, tm);
         tmem_wait_st();
         if (GB_SMEM) cp_async_wait_all();
+        if (i0 == 0 && p.params_old) begin();
         tmem_fence_before();
         team_sync<TEAM>(quarter);
         tmem_fence_after();
@@ -419,11 +425,12 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
 
 // ---- layout conversion at the ends of a loop --------------------------------------------------------------
 // IL4 -> [B, P], normalised on the way when statistics are given
-__global__ void __launch_bounds__(256) from_il4_k(const float4 *__restrict__ il, const float2 *__restrict__ stats,
+__global__ void __launch_bounds__(256) from_il4_k(const float4 *il, const float2 *stats,
                                                   const float *__restrict__ gamma, const float *__restrict__ beta,
-                                                  float *__restrict__ y, int B, size_t P)
+                                                  float *y, int B, size_t P)
 {
     const size_t c = (size_t)blockIdx.x * 256 + threadIdx.x;
+    previous_done();
     if (c >= P) return;
     const int q = blockIdx.y;
     const float4 v4 = il[(size_t)q * P + c];
@@ -633,7 +640,7 @@ int launch_from_il4(const float *il, const float2 *stats, const float *gamma, co
                     cudaStream_t st)
 {
     dim3 grid((unsigned)((P + 255) / 256), (unsigned)((B + 3) / 4));
-    from_il4_k<<<grid, 256, 0, st>>>(reinterpret_cast<const float4 *>(il), stats, gamma, beta, y, B, (size_t)P);
+    launch_after(from_il4_k, grid, 256, 0, st, reinterpret_cast<const float4 *>(il), stats, gamma, beta, y, B, (size_t)P);
     return check_launch("from_il4");
 }
 
@@ -676,7 +683,7 @@ static int launch_quad_one(const CUtensorMap &map, const QuadParams &p, unsigned
             return GN_ERR_CUDA;
         }
     }
-    kern<<<ctas, 128 * G::TEAM, smem, st>>>(map, p);
+    launch_after(kern, ctas, 128 * G::TEAM, smem, st, map, p);
     return check_launch("step_fwd_quad");
 }
 
@@ -707,7 +714,7 @@ int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
     const int rc = quad_make_map(&map, a.in_il4, a.M, a.N, a.K, a.Q, a.block);
     if (rc != GN_OK) return rc;
     QuadParams p{};
-    p.packed = a.packed;
+    p.packed = a.packed; p.params_old = a.params_old;
     p.gbt = a.gbt; p.in_stats = a.in_stats;
     p.out_partials = a.out_partials; p.nparts = a.nparts;
     p.wsum = a.wsum; p.tile_stats = a.tile_stats; p.eps = a.eps;

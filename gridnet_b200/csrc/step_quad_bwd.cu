@@ -134,6 +134,7 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
             cp_async16(tile + (unsigned)(((k >> 1) + 1) * PLANE + (y + 4 * (k & 1)) * ROW + x + 1) * 16u, src + (k & 1) * 16ll * p.K + (k >> 1) * zstr);
     };
     const size_t to_own = (((size_t)L.z0 * p.N + L.y0) * p.K + 4 * L.h) * 4;  // corner -> this lane's cells
+    previous_done();
     __syncwarp();
     if (role < cnt) {
         fetch_g(corner_of(role));
@@ -492,6 +493,7 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
         cp_async_wait_all();
         __syncthreads();
     }
+    previous_done();
     if (tid == 0) issue(q0, 0);
     const float *const delta = GATED && blockIdx.z ? p.delta2 : p.delta;
     fetch(stage_d, at(delta, q0, 0));
@@ -893,6 +895,7 @@ __global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     __syncthreads();  // the shells are zeroed
+    previous_done();
     fetch(q0, 0);
     fetch(q0 + 1, 1);
     for (int q = q0; q < q1; ++q) {
@@ -1206,7 +1209,7 @@ static int launch_reverse_in(const QuadRevParams &p, unsigned ctas, cudaStream_t
     static unsigned long long done = 0;
     const int rc = smem_once(quad_reverse_k<SUB, ACT, IN>, smem, &done, "cudaFuncSetAttribute(quad_reverse_k)");
     if (rc != GN_OK) return rc;
-    quad_reverse_k<SUB, ACT, IN><<<ctas, 256, smem, st>>>(p);
+    launch_after(quad_reverse_k<SUB, ACT, IN>, ctas, 256, smem, st, p);
     return check_launch("quad_reverse");
 }
 template <int SUB, int ACT>
@@ -1262,7 +1265,7 @@ static int launch_wgrad_in(const CUtensorMap &map, const QuadWgradParams &p, dim
     static unsigned long long done = 0;
     const int rc = smem_once(quad_wgrad_k<SUB, ACT, FUSE_IN, NORM, GATED>, smem, &done, "cudaFuncSetAttribute(quad_wgrad_k)");
     if (rc != GN_OK) return rc;
-    quad_wgrad_k<SUB, ACT, FUSE_IN, NORM, GATED><<<grid, quadwg::THREADS, smem, st>>>(map, p);
+    launch_after(quad_wgrad_k<SUB, ACT, FUSE_IN, NORM, GATED>, grid, quadwg::THREADS, smem, st, map, p);
     return check_launch("quad_wgrad");
 }
 template <int SUB, int ACT>
@@ -1338,7 +1341,7 @@ static int launch_border(const float *w, size_t tap, const float *dsum, float *g
         constexpr int smem = (quadborder::RING * (quadborder::SHELL + (NORM ? 2 : 1) * quadborder::SURFACE) + 2 * 3 * 128) * 16;
         const int rc = smem_once(quad_border8_k<NORM>, smem, &done[0], "cudaFuncSetAttribute(quad_border8_k)");
         if (rc != GN_OK) return rc;
-        quad_border8_k<NORM><<<grid, 384, smem, st>>>(w, tap, d4, g4, x4, hterm, Q, M, N, K, qpc);
+        launch_after(quad_border8_k<NORM>, grid, 384, smem, st, w, tap, d4, g4, x4, hterm, Q, M, N, K, qpc);
     } else {
         constexpr int smem = 2 * quadborder::TS * 16;
         const int rc = smem_once(quad_border4_k<NORM>, smem, &done[1], "cudaFuncSetAttribute(quad_border4_k)");
