@@ -5,10 +5,6 @@
 
 #include "../../include/gridnet_b200.h"
 
-#ifndef GN_ACCURATE_SIGMOID
-#define GN_ACCURATE_SIGMOID 0
-#endif
-
 namespace gn {
 
 constexpr int kNumSMs = 148;  // B200; only the fallback where the device cannot be asked
@@ -19,28 +15,8 @@ void record_cuda_error(cudaError_t e, const char *where);
 int check_launch(const char *where);
 
 // ---------------------------------------------------------------- activations
-// exp(x) for float: ex2.approx on a product whose rounding error is fed back,
-// so the relative error stays at a few ulp for every |x| (a plain
-// __expf(x) loses |x| * 2^-24 in the product).
-__device__ __forceinline__ float exp_f32(float x)
-{
-    const float l2e_hi = 1.4426950216293335f;   // float(log2(e))
-    const float l2e_lo = 1.9259629911266175e-8f; // log2(e) - l2e_hi
-    float t = x * l2e_hi;
-    float r = fmaf(x, l2e_hi, -t);
-    r = fmaf(x, l2e_lo, r);
-    float p;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p) : "f"(t));
-    return fmaf(p, r * 0.6931471805599453f, p);
-}
-
 __device__ __forceinline__ float sigmoid_(float x)
 {
-#if GN_ACCURATE_SIGMOID
-    // 1 / (1 + exp(-x)). The exponent is capped at 87 so that exp stays finite (an overflowed
-    // ex2 would turn the error-feedback term of exp_f32 into inf - inf); sigmoid(-87) = 1.6e-38.
-    return __fdividef(1.0f, 1.0f + exp_f32(fminf(-x, 87.0f)));
-#else
     // 1 / (1 + 2^(-x * log2 e)) in six instructions: FMUL, FMNMX, MUFU.EX2, FADD, MUFU.RCP
     // (+ the caller's multiply). The exponent is capped at 126 so that 1 + 2^t stays finite.
     // Relative error about |x| * 6e-8 from the rounded product plus 2 ulp from each MUFU.
@@ -49,7 +25,6 @@ __device__ __forceinline__ float sigmoid_(float x)
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(t));
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
     return r;
-#endif
 }
 __device__ __forceinline__ double sigmoid_(double x) { return 1.0 / (1.0 + exp(-x)); }
 
