@@ -144,6 +144,7 @@ struct QuadStep {
     double2 *out_partials;    // [4 Q][nparts] or nullptr; slots 0 .. regions-1 of every row are written
     int nparts;
     float *save_h;            // [inner] IL4 tensors of pre-activations, or nullptr
+    bool ordered;             // packed is in the order of the taps (QuadPrepare::ordered); not with wsum, needed with save_h otherwise
     bool params_old;          // packed and gbt are not what the kernel queued just before writes
     const float *wsum;        // from launch_quad_prepare: per-block normalisation; nullptr: off
     float4 *tile_stats;       // with wsum and save_h: quad_stats_vectors(...) vectors
@@ -161,6 +162,7 @@ struct QuadPrepare {
     const float *w, *b, *s;
     bool gated;                // w, b, b_t and the packed parameters have two branches; s is not looked at (any M N K floats)
     float *packed;             // quad_packed_floats(...): weights, b, s in the order of the forward sums
+    bool ordered;              // ... in the order of the taps, for a QuadStep that says so too
     const float *b_t;
     float *packed_t;           // the same for the backward sums: transposed weights, b_t, s
     float *wsum;               // M N K floats: the neurons' weight sums

@@ -185,7 +185,7 @@ GN_API int gn_loop_forward_f32(const float *const *weights, const float *const *
     const int S = 4 * d.Q;  // statistics of one step
     {
         QuadPrepare a{};
-        a.w = weights[0]; a.b = biases[0]; a.s = scales[0]; a.packed = w.packed;
+        a.w = weights[0]; a.b = biases[0]; a.s = scales[0]; a.packed = w.packed; a.ordered = true;
         a.gamma = gamma; a.beta = beta; a.gbt = w.gbt;
         a.x = x; a.il = x_il4; a.B = B;
         TRY_(launch_quad_prepare(a, M, N, K, block, st));
@@ -197,12 +197,12 @@ GN_API int gn_loop_forward_f32(const float *const *weights, const float *const *
     for (int k = 0; k < outer; ++k) {
         if (k > 0 && nparams > 1) {
             QuadPrepare a{};
-            a.w = weights[k]; a.b = biases[k]; a.s = scales[k]; a.packed = w.packed;
+            a.w = weights[k]; a.b = biases[k]; a.s = scales[k]; a.packed = w.packed; a.ordered = true;
             TRY_(launch_quad_prepare(a, M, N, K, block, st));
         }
         const float *in = k ? outs[k - 1] : x_il4;
         QuadStep a{};
-        a.packed = w.packed; a.gbt = w.gbt;
+        a.packed = w.packed; a.gbt = w.gbt; a.ordered = true;
         a.in_il4 = in;
         a.out_il4 = residual ? w.tmp : outs[k];
         a.in_stats = residual ? mr + (size_t)k * S : (k ? mr + (size_t)(k - 1) * S : nullptr);
@@ -251,6 +251,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
             QuadPrepare a{};
             a.w = weights[kp]; a.b = biases[kp]; a.s = scales[kp]; a.b_t = gamma; a.packed_t = w.packed_t;
             if (replay) a.packed = w.packed;
+            a.ordered = true;
             if (first) {
                 a.gamma = gamma; a.beta = beta; a.gbt = w.gbt;
                 a.x = gy; a.il = w.g[0]; a.B = B;
@@ -262,9 +263,10 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
         float *const h = kept ? stashes[k] : w.replay;
         if (!kept) {
             QuadStep a{};
-            a.packed = w.packed; a.gbt = w.gbt; a.in_il4 = in; a.in_stats = in_stats;
+            a.packed = w.packed; a.gbt = w.gbt; a.ordered = true;
+            a.in_il4 = in; a.in_stats = in_stats;
             a.save_h = h;
-                a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;
+            a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;
             TRY_(launch_step_fwd_quad(a, act, st));
         }
         QuadReverse r{};

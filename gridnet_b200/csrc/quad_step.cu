@@ -116,10 +116,12 @@ int run_forward(const float *w, const float *b, const float *s, float *packed, c
     QuadPrepare r{};
     r.w = w; r.b = b; r.s = s; r.packed = packed; r.x = x; r.il = x_il4; r.B = d.B;
     if (d.normalize) r.wsum = wsum;
+    r.ordered = !d.normalize;
     TRY_(launch_quad_prepare(r, d.M, d.N, d.K, d.block, st));
     QuadStep a{};
     a.packed = packed; a.in_il4 = x_il4; a.out_il4 = y;
     if (d.normalize) a.wsum = wsum;
+    a.ordered = !d.normalize;
     a.eps = eps;
     if (k) {
         a.save_h = k->h;

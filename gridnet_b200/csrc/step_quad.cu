@@ -61,7 +61,8 @@ struct QuadParams {
 // to subtract it and to take the sums over its halo, which no iteration changes; from then on the tile holds v - c, so
 // that neither the variance nor sum w v - mean sum w cancels. Each iteration adds up the values it has just computed
 // while they are still in registers.
-template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM>
+// ORDERED: the sums of quad_stencil_ordered, the bits of step_fast.cu: everything that is differentiated.
+template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM, bool ORDERED>
 __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     step_fwd_quad(const __grid_constant__ CUtensorMap in_map, const QuadParams p)
 {
@@ -90,7 +91,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     __syncthreads();
     tmem_fence_after();
     const unsigned tm = tmem_slot + ((unsigned)(quarter * 32) << 16);
-    static_assert(!(NORM && FUSE_IN), "per-block normalisation takes plain input");
+    static_assert(!(NORM && (FUSE_IN || ORDERED)), "per-block normalisation takes plain input, in the order of the walk");
 
     const QuadLane<SUB> L(lane);
     // NORM: the lane's share of its tile's cells, first + STRIDE k; four lanes share a block-4 tile, and the first two
@@ -193,8 +194,8 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                     for (int s = 0; s < 4; ++s) mr[s] = p.in_stats[4 * q + s];
                     na[0] = pack2(mr[0].y, mr[1].y);
                     na[1] = pack2(mr[2].y, mr[3].y);
-                    nb[0] = pack2(-mr[0].x * mr[0].y, -mr[1].x * mr[1].y);
-                    nb[1] = pack2(-mr[2].x * mr[2].y, -mr[3].x * mr[3].y);
+                    nb[0] = pack2(-mr[0].x, -mr[1].x);
+                    nb[1] = pack2(-mr[2].x, -mr[3].x);
                 }
                 wait_tile(i);
                 const float2 *gp = GB_SMEM ? gbs + lane : p.gbt + (size_t)blk * G::CELLS + lane;
@@ -215,7 +216,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                     for (int c = 0; c < BATCH; ++c)
                         if ((c0 + c) * 32 + lane < G::CELLS) {
                             const u64 gg = pack2(g2[c].x, g2[c].x), bb = pack2(g2[c].y, g2[c].y);
-                            sts128u(a + c * 512, ffma2r(ffma2r(v[c][0], na[0], nb[0]), gg, bb), ffma2r(ffma2r(v[c][1], na[1], nb[1]), gg, bb));
+                            sts128u(a + c * 512, ffma2r(fmul2(fadd2(v[c][0], nb[0]), na[0]), gg, bb), ffma2r(fmul2(fadd2(v[c][1], nb[1]), na[1]), gg, bb));
                         }
                 }
                 __syncwarp();
@@ -354,7 +355,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                 }
                 u64 acc[4][4][2], hold[2] = {0, 0};
                 float *const sh = SAVE ? p.save_h + (size_t)t * p.Q * P * 4 + own : nullptr;
-                quad_stencil<G::PLANE, NORM ? NORMED : BIAS>(rows, L.xsgn * 16, tm, acc, negm, [&](int n, int o, float scale, float bias, u64 c0, u64 c1) {
+                auto done = [&](int n, int o, float scale, float bias, u64 c0, u64 c1) {
                     if (NORM) {
                         acc[n][o][0] = ffma2r(acc[n][o][0], inv[0], pack2(bias, bias));
                         acc[n][o][1] = ffma2r(acc[n][o][1], inv[1], pack2(bias, bias));
@@ -368,7 +369,9 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                     }
                     acc[n][o][0] = act_residual2<ACT>(acc[n][o][0], scale, c0);
                     acc[n][o][1] = act_residual2<ACT>(acc[n][o][1], scale, c1);
-                });
+                };
+                if constexpr (ORDERED) quad_stencil_ordered<SUB, G::PLANE>(L, rows, L.xsgn * 16, tm, acc, done);
+                else quad_stencil<G::PLANE, NORM ? NORMED : BIAS>(rows, L.xsgn * 16, tm, acc, negm, done);
                 __syncwarp();  // every lane has read its window
                 if (!last) {
 #pragma unroll
@@ -389,25 +392,8 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                                 for (int k2 = 0; k2 < 2; ++k2) acc[n][o][k2] = fadd2(acc[n][o][k2], piv[k2]);
                     if (p.y) quad_store(p.y + own, zstr, ystr, L.h, acc);
                     if (p.out_partials) {
-                        u64 s2[2] = {0, 0}, q2[2] = {0, 0};
-#pragma unroll
-                        for (int n = 0; n < 4; ++n)
-#pragma unroll
-                            for (int o = 0; o < 4; ++o)
-#pragma unroll
-                                for (int k2 = 0; k2 < 2; ++k2) {
-                                    s2[k2] = fadd2(s2[k2], acc[n][o][k2]);
-                                    ffma2(q2[k2], acc[n][o][k2], acc[n][o][k2]);
-                                }
-                        float v[8];
-                        unpack2(s2[0], v[0], v[1]);
-                        unpack2(s2[1], v[2], v[3]);
-                        unpack2(q2[0], v[4], v[5]);
-                        unpack2(q2[1], v[6], v[7]);
-                        const float r = quad_reduce8(v, lane);
-                        // lane 4 j holds value j: sums of samples 0..3, then sums of squares
-                        if ((lane & 3) == 0)
-                            reinterpret_cast<double *>(p.out_partials + (size_t)(4 * q + ((lane >> 2) & 3)) * p.nparts + blk)[lane >> 4] = (double)r;
+                        const double r = quad_region_sums(L, acc, lane);
+                        if (lane < 8) reinterpret_cast<double *>(p.out_partials + (size_t)(4 * q + (lane & 3)) * p.nparts + blk)[lane >> 2] = r;
                         __syncwarp();
                     }
                 }
@@ -465,23 +451,23 @@ __device__ __forceinline__ void to_il4(const float *__restrict__ x, float4 *__re
 
 // Parameters in the order of the stencil: vector v of a region is, for every lane, the four x-neighbouring weights of
 // one (neuron row, tap), v = 0 .. 107 in the order of the uses in quad_stencil (three x-taps each), then the four rows
-// of b, then of s. TRANS: the weights of the backward sum, in which a cell collects from the neurons of its own block
+// of b, then of s. ORDERED: for quad_stencil_ordered, weights and b in ascending (y, x). TRANS: the weights of the backward sum, in which a cell collects from the neurons of its own block
 // that read it: the neuron at tap t sees the cell through its tap 26 - t; zero across the block's border. Four CTAs of 256 threads per
 // region, so that small grids fill the GPU; reads are 16-byte pieces, writes whole lines.
 constexpr int kPackCtas = 4;
-template <int SUB, bool TRANS>
+template <int SUB, bool TRANS, bool ORDERED>
 __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const float *__restrict__ b, const float *__restrict__ s,
                                           float *__restrict__ packed, size_t tap, int M, int N, int K, int cta)
 {
     __shared__ unsigned char uses[36];  // (a * 3 + b) | n << 4
     if (threadIdx.x == 0) {
         int k = 0;
-        for (int ry = 0; ry < 4; ++ry)
-            for (int rz = 0; rz < 4; ++rz)
-                for (int n = 0; n < 4; ++n) {
-                    const int a = rz - (n >> 1), bb = ry - (n & 1);
-                    if (a >= 0 && a <= 2 && bb >= 0 && bb <= 2) uses[k++] = (unsigned char)((a * 3 + bb) | n << 4);
-                }
+        for (int r = 0; r < 16; ++r)
+            for (int n = 0; n < 4; ++n) {
+                const int rz = ORDERED ? r >> 2 : r & 3, ry = ORDERED ? r & 3 : r >> 2;
+                const int a = rz - (n >> 1), bb = ry - (n & 1);
+                if (a >= 0 && a <= 2 && bb >= 0 && bb <= 2) uses[k++] = (unsigned char)((a * 3 + bb) | n << 4);
+            }
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -489,7 +475,7 @@ __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const flo
     const int nbx = K >> 3, nby = N >> 3, blk = cta / kPackCtas;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t g0 = ((size_t)(bz * 8 + L.z0) * N + (by * 8 + L.y0)) * K + bx * 8 + 4 * L.h;
-    const long long zs = (long long)N * K, ys = (long long)L.ysgn * K;
+    const long long zs = (long long)N * K;
     float4 *out = reinterpret_cast<float4 *>(packed + (size_t)blk * quad::PACK_F) + lane;
 #pragma unroll
     for (int i = 0; i < (quad::VECS + 8 * kPackCtas - 1) / (8 * kPackCtas); ++i) {
@@ -497,13 +483,16 @@ __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const flo
         if (v >= quad::VECS) break;
         int n;
         float4 r;
+        const bool turned = ORDERED && v < 112;                // ascending, whatever the lane's walk
+        const size_t g1 = turned && L.ysgn < 0 ? g0 - K : g0;  // row dy = 0
+        const long long ys = turned ? K : (long long)L.ysgn * K;
         if (v < 108) {
             const int u = uses[v / 3], c = v % 3;
             n = u >> 4;
             // the tap as the grid numbers it (gridnet/backend_torch.py:283-298)
-            const int ta = (u & 15) / 3, tb = L.ysgn < 0 ? 2 - (u & 15) % 3 : (u & 15) % 3, tc = L.h ? 2 - c : c;
+            const int ta = (u & 15) / 3, tb = !turned && L.ysgn < 0 ? 2 - (u & 15) % 3 : (u & 15) % 3, tc = !turned && L.h ? 2 - c : c;
             const int t = ta * 9 + tb * 3 + tc;
-            const size_t own = g0 + (n >> 1) * zs + (n & 1) * ys;
+            const size_t own = g1 + (n >> 1) * zs + (n & 1) * ys;
             if (!TRANS) {
                 const float *src = w + (size_t)t * tap + own;
                 if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) r = *reinterpret_cast<const float4 *>(src);
@@ -524,11 +513,11 @@ __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const flo
             }
         } else {
             n = v & 3;
-            const float *src = (v < 112 ? b : s) + g0 + (n >> 1) * zs + (n & 1) * ys;
+            const float *src = (v < 112 ? b : s) + g1 + (n >> 1) * zs + (n & 1) * ys;
             if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) r = *reinterpret_cast<const float4 *>(src);
             else r = make_float4(src[0], src[1], src[2], src[3]);
         }
-        out[v * 32] = L.h ? make_float4(r.w, r.z, r.y, r.x) : r;
+        out[v * 32] = L.h && !turned ? make_float4(r.w, r.z, r.y, r.x) : r;
     }
 }
 
@@ -587,7 +576,7 @@ struct PrepareArgs {
     unsigned pack;    // packing: CTAs per branch
     int branches;
 };
-template <int SUB>
+template <int SUB, bool ORDERED>
 __global__ void __launch_bounds__(256) quad_prepare_k(const PrepareArgs p)
 {
     const unsigned c = blockIdx.x;
@@ -596,8 +585,8 @@ __global__ void __launch_bounds__(256) quad_prepare_k(const PrepareArgs p)
     if (c < p.end[1]) {  // branch k of a gated network: weights [27][2][P], bias [2][P]
         const unsigned j = c < p.end[0] ? c : c - p.end[0], k = j / p.pack;
         const size_t to = (size_t)k * (p.pack / kPackCtas) * quad::PACK_F;
-        if (c < p.end[0]) quad_pack<SUB, false>(a.w + k * P, a.b + k * P, a.s, a.packed + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
-        else quad_pack<SUB, true>(a.w + k * P, a.b_t + k * P, a.s, a.packed_t + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
+        if (c < p.end[0]) quad_pack<SUB, false, ORDERED>(a.w + k * P, a.b + k * P, a.s, a.packed + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
+        else quad_pack<SUB, true, false>(a.w + k * P, a.b_t + k * P, a.s, a.packed_t + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
     }
     else if (c < p.end[2]) quad_wsum<SUB>(a.w, reinterpret_cast<float4 *>(a.wsum), p.M, p.N, p.K, (int)(c - p.end[1]));
     else if (c < p.end[3]) quad_table<SUB>(a.gamma, a.beta, a.gbt, p.M, p.N, p.K, (int)(c - p.end[2]));
@@ -662,16 +651,18 @@ int launch_quad_prepare(const QuadPrepare &a, int M, int N, int K, int block, cu
         p.end[j] = (unsigned)n;
     }
     if (n == 0) return GN_OK;
-    if (block == 8) quad_prepare_k<8><<<(unsigned)n, 256, 0, st>>>(p);
-    else quad_prepare_k<4><<<(unsigned)n, 256, 0, st>>>(p);
+    if (block == 8 && a.ordered) quad_prepare_k<8, true><<<(unsigned)n, 256, 0, st>>>(p);
+    else if (block == 8) quad_prepare_k<8, false><<<(unsigned)n, 256, 0, st>>>(p);
+    else if (a.ordered) quad_prepare_k<4, true><<<(unsigned)n, 256, 0, st>>>(p);
+    else quad_prepare_k<4, false><<<(unsigned)n, 256, 0, st>>>(p);
     return check_launch("quad_prepare");
 }
 
-template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM = false>
+template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM, bool ORDERED>
 static int launch_quad_one(const CUtensorMap &map, const QuadParams &p, unsigned ctas, cudaStream_t st)
 {
     using G = QuadGeo<SUB>;
-    auto kern = step_fwd_quad<SUB, ACT, FUSE_IN, SAVE, NORM>;
+    auto kern = step_fwd_quad<SUB, ACT, FUSE_IN, SAVE, NORM, ORDERED>;
     // tiles; block 8 with normalise-on-load also a (gamma, beta) table per team
     constexpr int smem = quad::QUARTERS * G::NBUF * G::BUF_BYTES + (SUB == 8 && FUSE_IN ? quad::QUARTERS * G::CELLS * 8 : 0);
     static_assert(smem <= 232448 - 1024 - 256, "shared memory budget of one SM");
@@ -688,27 +679,31 @@ static int launch_quad_one(const CUtensorMap &map, const QuadParams &p, unsigned
 }
 
 template <int SUB, int ACT>
-static int launch_quad_act(const CUtensorMap &map, const QuadParams &p, unsigned ctas, cudaStream_t st)
+static int launch_quad_act(const CUtensorMap &map, const QuadParams &p, bool ordered, unsigned ctas, cudaStream_t st)
 {
-    if (p.wsum) return p.save_h ? launch_quad_one<SUB, ACT, false, true, true>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, false, true>(map, p, ctas, st);
-    if (p.save_h) return p.in_stats ? launch_quad_one<SUB, ACT, true, true>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, true>(map, p, ctas, st);
-    return p.in_stats ? launch_quad_one<SUB, ACT, true, false>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, false>(map, p, ctas, st);
+#define ONE_(FUSE_IN, SAVE, NORM, ORDERED) launch_quad_one<SUB, ACT, FUSE_IN, SAVE, NORM, ORDERED>(map, p, ctas, st)
+    if (p.wsum) return p.save_h ? ONE_(false, true, true, false) : ONE_(false, false, true, false);
+    if (!ordered) return p.in_stats ? ONE_(true, false, false, false) : ONE_(false, false, false, false);
+    if (p.save_h) return p.in_stats ? ONE_(true, true, false, true) : ONE_(false, true, false, true);
+    return p.in_stats ? ONE_(true, false, false, true) : ONE_(false, false, false, true);
+#undef ONE_
 }
 
 template <int SUB>
-static int launch_quad_sub(const CUtensorMap &map, const QuadParams &p, unsigned ctas, int act, cudaStream_t st)
+static int launch_quad_sub(const CUtensorMap &map, const QuadParams &p, bool ordered, unsigned ctas, int act, cudaStream_t st)
 {
     switch (act) {
-    case GN_ACT_RELU: return launch_quad_act<SUB, GN_ACT_RELU>(map, p, ctas, st);
-    case GN_ACT_LEAKY_RELU: return launch_quad_act<SUB, GN_ACT_LEAKY_RELU>(map, p, ctas, st);
-    case GN_ACT_SILU: return launch_quad_act<SUB, GN_ACT_SILU>(map, p, ctas, st);
-    default: return launch_quad_act<SUB, GN_ACT_TANH>(map, p, ctas, st);
+    case GN_ACT_RELU: return launch_quad_act<SUB, GN_ACT_RELU>(map, p, ordered, ctas, st);
+    case GN_ACT_LEAKY_RELU: return launch_quad_act<SUB, GN_ACT_LEAKY_RELU>(map, p, ordered, ctas, st);
+    case GN_ACT_SILU: return launch_quad_act<SUB, GN_ACT_SILU>(map, p, ordered, ctas, st);
+    default: return launch_quad_act<SUB, GN_ACT_TANH>(map, p, ordered, ctas, st);
     }
 }
 
 int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
 {
-    if (a.wsum && (a.in_stats || !a.save_h != !a.tile_stats)) return GN_ERR_UNSUPPORTED;
+    if (a.wsum && (a.in_stats || a.ordered || !a.save_h != !a.tile_stats)) return GN_ERR_UNSUPPORTED;
+    if (!a.wsum && a.save_h && !a.ordered) return GN_ERR_UNSUPPORTED;
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
     const int rc = quad_make_map(&map, a.in_il4, a.M, a.N, a.K, a.Q, a.block);
@@ -724,7 +719,7 @@ int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
     p.nitems = (long long)(a.M / 8) * (a.N / 8) * (a.K / 8) * a.Q;
     long long ctas = (p.nitems + quad::QUARTERS - 1) / quad::QUARTERS;
     if (ctas > sm_count()) ctas = sm_count();
-    return a.block == 8 ? launch_quad_sub<8>(map, p, (unsigned)ctas, act, st) : launch_quad_sub<4>(map, p, (unsigned)ctas, act, st);
+    return a.block == 8 ? launch_quad_sub<8>(map, p, a.ordered, (unsigned)ctas, act, st) : launch_quad_sub<4>(map, p, a.ordered, (unsigned)ctas, act, st);
 }
 
 }  // namespace gn

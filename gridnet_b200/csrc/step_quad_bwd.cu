@@ -1139,13 +1139,15 @@ __global__ void __launch_bounds__(256) quad_norm_residual_apply_k(const float4 *
 }
 
 // Residual form, forward: out = h + (y - norm(h)), and the per-sample partial sums of out (out may be y). With y and out
-// null only the sums of h are taken (the statistics of the loop's first input).
+// null only the sums of h are taken (the statistics of the loop's first input). As in norm_residual_combine_k and
+// norm_partial_stats_k (norm.cu) four x-neighbours are added in float, everything above in double: neighbouring lanes hold
+// neighbouring cells, and of the sums that four lanes then share each goes on with one sample's. P is a multiple of 512.
 __global__ void __launch_bounds__(256) quad_residual_combine_k(const float4 *__restrict__ h, const float4 *y, const float *__restrict__ gamma,
                                                                const float *__restrict__ beta, const float2 *__restrict__ stats, float4 *out,
                                                                double2 *__restrict__ partials, int nparts, size_t P)
 {
     constexpr int CPT = 4;
-    __shared__ float red[8][8];
+    __shared__ double red[8][8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = blockIdx.y;
     const size_t c0 = (size_t)blockIdx.x * (256 * CPT) + tid;
     float2 mr[4];
@@ -1153,36 +1155,48 @@ __global__ void __launch_bounds__(256) quad_residual_combine_k(const float4 *__r
 #pragma unroll
         for (int s = 0; s < 4; ++s) mr[s] = __ldg(stats + 4 * q + s);
     }
-    float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    double sum = 0.0, squares = 0.0;  // of sample lane & 3
 #pragma unroll
     for (int k = 0; k < CPT; ++k) {
         const size_t c = c0 + k * 256;
-        if (c < P) {
-            const size_t i = (size_t)q * P + c;
-            const float4 hv = h[i];
-            float o[4] = {hv.x, hv.y, hv.z, hv.w};
-            if (y) {
-                const float4 yv = y[i];
-                const float ys[4] = {yv.x, yv.y, yv.z, yv.w};
-                const float g = gamma[c], b = beta[c];
+        if (c >= P) continue;  // the whole CTA
+        const size_t i = (size_t)q * P + c;
+        const float4 hv = h[i];
+        float o[4] = {hv.x, hv.y, hv.z, hv.w};
+        if (y) {
+            const float4 yv = y[i];
+            const float ys[4] = {yv.x, yv.y, yv.z, yv.w};
+            const float g = gamma[c], b = beta[c];
 #pragma unroll
-                for (int s = 0; s < 4; ++s) o[s] = o[s] + (ys[s] - fmaf((o[s] - mr[s].x) * mr[s].y, g, b));
-                out[i] = make_float4(o[0], o[1], o[2], o[3]);
-            }
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {
-                v[s] += o[s];
-                v[4 + s] = fmaf(o[s], o[s], v[4 + s]);
-            }
+            for (int s = 0; s < 4; ++s) o[s] = o[s] + (ys[s] - fmaf((o[s] - mr[s].x) * mr[s].y, g, b));
+            out[i] = make_float4(o[0], o[1], o[2], o[3]);
         }
+        float a[4], b[4];
+#pragma unroll
+        for (int s = 0; s < 4; ++s) {
+            const float other = __shfl_xor_sync(0xffffffffu, o[s], 1), lo = lane & 1 ? other : o[s], hi = lane & 1 ? o[s] : other;
+            a[s] = lo + hi;
+            b[s] = fmaf(lo, lo, hi * hi);
+            a[s] += __shfl_xor_sync(0xffffffffu, a[s], 2);
+            b[s] += __shfl_xor_sync(0xffffffffu, b[s], 2);
+        }
+        sum += (double)(lane & 2 ? (lane & 1 ? a[3] : a[2]) : (lane & 1 ? a[1] : a[0]));
+        squares += (double)(lane & 2 ? (lane & 1 ? b[3] : b[2]) : (lane & 1 ? b[1] : b[0]));
     }
-    const float r = quad_reduce8(v, lane);
-    if ((lane & 3) == 0) red[warp][lane >> 2] = r;
+#pragma unroll
+    for (int m = 4; m < 32; m *= 2) {
+        sum += __shfl_xor_sync(0xffffffffu, sum, m);
+        squares += __shfl_xor_sync(0xffffffffu, squares, m);
+    }
+    if (lane < 4) {
+        red[warp][lane] = sum;
+        red[warp][4 + lane] = squares;
+    }
     __syncthreads();
     if (tid < 8) {
         double s = 0.0;
 #pragma unroll
-        for (int w8 = 0; w8 < 8; ++w8) s += (double)red[w8][tid];
+        for (int w8 = 0; w8 < 8; ++w8) s += red[w8][tid];
         reinterpret_cast<double *>(partials + (size_t)(4 * q + (tid & 3)) * nparts + blockIdx.x)[tid >> 2] = s;
     }
 }

@@ -286,3 +286,70 @@ def test_gated_loop_matches_oracle(shape, batch, inner, outer, act, keep):
         sums = [s + d for s, d in zip(sums, (dw, db, dga, dbe))]
     for got, ref, name in zip(t, (*sums, g), ("weight", "bias", "norm.weight", "norm.bias", "x")):
         assert_close(got.grad.cpu().numpy(), ref, None, f"grad {name}")
+
+
+@pytest.mark.parametrize("block,shape,batch,inner,outer,act", [(8, (8, 16, 24), 5, 1, 3, "leaky_relu"), (8, (40, 24, 16), 9, 4, 4, "silu"),
+                                                               (4, (16, 8, 24), 7, 3, 4, "relu"), (4, (24, 24, 24), 4, 8, 6, "silu")])
+def test_loops_with_gradients_give_the_bits_of_the_register_patch_kernels(block, shape, batch, inner, outer, act):
+    """What rounding differs by in a forward pass is amplified in the gradients, without bound where a pre-activation crosses
+    the kink of an activation function. So the loops with gradients, whichever kernels they run on, have the forward pass
+    of the register-patch kernels bit for bit: plain and residual, with the iterations kept and run again, and a single step."""
+    import gridnet_b200 as gb
+    from gridnet_b200 import gridnet_cuda
+    from gridnet_b200._lib import activation_id, check, lib
+
+    g = torch.Generator().manual_seed(23)
+    mk = lambda *sz, scale=1.0, shift=0.0: (shift + scale * torch.randn(*sz, generator=g)).cuda()
+    params = mk(27, *shape, scale=27 ** -0.5), mk(*shape, scale=0.1), mk(*shape, scale=0.1, shift=1.0)
+    gamma, beta, x, gy = mk(*shape, scale=0.1, shift=1.0), mk(*shape, scale=0.1), mk(batch, *shape, shift=2.0), mk(batch, *shape)
+    P, st = x[0].numel(), torch.cuda.current_stream().cuda_stream
+    ptr = lambda t: None if t is None else t.data_ptr()
+    nws = torch.empty(lib.gn_norm_workspace_bytes(batch, P), dtype=torch.uint8, device="cuda")
+
+    def step(h, mr, partials):
+        y = torch.empty_like(h)
+        check(lib.gn_step_forward_train_f32(*map(ptr, params), ptr(h), ptr(y), ptr(gamma), ptr(beta), ptr(mr), ptr(partials), batch, *shape, inner,
+                                            block, activation_id(act), None, 0, st))
+        return y
+
+    def plain(h):
+        n = lib.gn_step_stats_partials(*shape, block)
+        partials, mr = torch.empty(batch, n, 2, dtype=torch.float64, device="cuda"), None
+        for _ in range(outer):
+            h, mr = step(h, mr, partials), torch.empty(batch, 2, device="cuda")
+            check(lib.gn_norm_finalize_f32(ptr(partials), n, ptr(mr), batch, P, 1e-5, st))
+        y = torch.empty_like(h)
+        check(lib.gn_norm_apply_f32(ptr(h), ptr(gamma), ptr(beta), ptr(mr), ptr(y), batch, P, st))
+        return y
+
+    def residual(h):
+        sums, mr = torch.empty(batch, 2, dtype=torch.float64, device="cuda"), torch.empty(batch, 2, device="cuda")
+        check(lib.gn_norm_local_sums_f32(ptr(h), ptr(sums), batch, P, ptr(nws), nws.numel(), st))
+        check(lib.gn_norm_finalize_f32(ptr(sums), 1, ptr(mr), batch, P, 1e-5, st))
+        for _ in range(outer):
+            out, nxt = torch.empty_like(h), torch.empty(batch, 2, device="cuda")
+            check(lib.gn_norm_residual_combine_f32(ptr(h), ptr(step(h, mr, None)), ptr(gamma), ptr(beta), ptr(mr), ptr(out), ptr(nxt), batch, P,
+                                                   1e-5, ptr(nws), nws.numel(), st))
+            h, mr = out, nxt
+        return h
+
+    grads = []
+    for keep in (True, False):
+        previous = gb.keep_forward_stash(keep)
+        try:
+            for form, want in (("plain", plain(x)), ("residual", residual(x))):
+                leaves = [t.clone().requires_grad_(True) for t in (*params, gamma, beta, x)]
+                if form == "plain":
+                    y = gb.FusedLoopTrainOp.apply(*leaves, inner, outer, block, act, 1e-5)
+                else:
+                    y = gb.FusedLoopResidualTrainOp.apply(*leaves[3:], inner, block, act, 1e-5, outer, *leaves[:3])
+                assert torch.equal(y, want), (form, keep, (y - want).abs().max().item())
+                grads.append(torch.autograd.grad(y, leaves, gy))
+        finally:
+            gb.keep_forward_stash(previous)
+    for a, c in zip(grads[0] + grads[1], grads[2] + grads[3]):
+        assert torch.equal(a, c)  # iterations that are run again are the ones that were kept
+    one, two = torch.empty_like(x), torch.empty_like(x)
+    gridnet_cuda.forward(*params, x, one, inner, block, 1e-5, False, act)
+    gridnet_cuda.forward_kept(*params, x, two, inner, block, 1e-5, False, act)
+    assert torch.equal(one, two)
