@@ -1106,6 +1106,7 @@ static int outer_forward_impl(const float *w, const float *b, const float *s, co
             p.in_stats = o > 0 ? ws.stats : nullptr;  // raw output of the previous step: normalise on load
             p.out_partials = ws.partials;
             p.nparts = nparts_fused;
+            p.params_old = o > 0;
             rc = launch_step_fwd_fast8(p, act, st);
             if (rc != GN_OK) return rc;
             rc = launch_norm_finalize(ws.partials, nparts_fused, ws.stats, B, P, ln_eps, st);

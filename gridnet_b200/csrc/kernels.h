@@ -57,6 +57,9 @@ struct FastFwdParams {
     // Replay mode with per-block normalisation: [inner][B][regions] (mean, 1 / (std + eps), std, std + eps) of the
     // tile every iteration normalised, for the backward kernels; nullptr = not wanted.
     float4 *tile_stats;
+    // The kernel queued just before wrote none of w, b, s, gamma, beta: this one may start, and load them, while that one
+    // still runs. Only a loop that queued both knows; after anything else the previous kernel may be the caller's update.
+    bool params_old;
 };
 bool fast8_applicable(const FastFwdParams &p, int block, int normalize);
 extern int g_fast8_spc_override;  // tuning knob: samples per CTA of the tuned forward kernel, 0 = automatic

@@ -269,6 +269,7 @@ __global__ void __launch_bounds__(fast8::THREADS, fast8::MIN_CTAS)
         if (FUSE_IN && smp < s1) pf_mr = p.in_stats[smp];
     };
 
+    // what was read so far is older than the kernel before this one, or that one has completed (FastFwdParams::params_old)
     if (USE_TMA) {
         if (tid == 0) {
             mbar_init(bar_base, 1);
@@ -601,9 +602,9 @@ int launch_step_fwd_fast8(FastFwdParams p, int act, cudaStream_t st)
             if (!tma) return GN_ERR_UNSUPPORTED;                                                          \
             if (p.inner == 8) SUB4_(A, FI, SO, 8);                                                        \
             else SUB4_(A, FI, SO, 0);                                                                     \
-        } else if (tma && FI && SO && p.inner == 4) launch_after(step_fwd_fast8<8, A, FI, SO, true, 4>, grid, fast8::THREADS, 0, st, map, p); \
-        else if (tma && FI && SO && p.inner == 2) launch_after(step_fwd_fast8<8, A, FI, SO, true, 2>, grid, fast8::THREADS, 0, st, map, p); \
-        else if (tma && FI && SO) launch_after(step_fwd_fast8<8, A, FI, SO, true, 0>, grid, fast8::THREADS, 0, st, map, p); \
+        } else if (tma && FI && SO && p.params_old && p.inner == 4) launch_after(step_fwd_fast8<8, A, FI, SO, true, 4>, grid, fast8::THREADS, 0, st, map, p); \
+        else if (tma && FI && SO && p.params_old && p.inner == 2) launch_after(step_fwd_fast8<8, A, FI, SO, true, 2>, grid, fast8::THREADS, 0, st, map, p); \
+        else if (tma && FI && SO && p.params_old) launch_after(step_fwd_fast8<8, A, FI, SO, true, 0>, grid, fast8::THREADS, 0, st, map, p); \
         else if (tma && p.inner == 4) step_fwd_fast8<8, A, FI, SO, true, 4><<<grid, fast8::THREADS, 0, st>>>(map, p);  \
         else if (tma && p.inner == 2) step_fwd_fast8<8, A, FI, SO, true, 2><<<grid, fast8::THREADS, 0, st>>>(map, p); \
         else if (tma) step_fwd_fast8<8, A, FI, SO, true, 0><<<grid, fast8::THREADS, 0, st>>>(map, p);     \

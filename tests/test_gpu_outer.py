@@ -477,3 +477,27 @@ def test_step_with_weights_in_tensor_memory(block, shape, batch, inner, act, nor
         assert_close(y.cpu().numpy(), ref_y, None, "y")
         for g, ref, name in zip(grads, refs, ("weight", "bias", "scale", "x")):
             assert_close(g.cpu().numpy(), ref, None, f"grad {name}, keep {keep}")
+
+
+@pytest.mark.parametrize("inner", [1, 2, 4])
+def test_fused_step_sees_parameters_written_just_before(inner):
+    """A normalise-on-load step with statistics right behind kernels that write its parameters: it must not have read them
+    before those kernels are done (the loop's own launches may start early, this entry point may not)."""
+    from gridnet_b200 import fused_step, step_stats_partials
+
+    B, shape = 2, (64, 64, 64)
+    w, b, s, gamma, beta = (dev(a) for a in model_params(44, shape))
+    x = torch.randn(B, *shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(45))
+    mr = torch.tensor([[0.1, 1.1], [-0.2, 0.9]], device="cuda")
+    params = [torch.zeros_like(t) for t in (w, b, s, gamma, beta)]
+    out, want = torch.empty_like(x), torch.empty_like(x)
+    partials = torch.empty(B, step_stats_partials(shape, 8), 2, dtype=torch.float64, device="cuda")
+    fused_step(w, b, s, x, want, inner, 8, "silu", gamma, beta, mr, partials)
+    for _ in range(5):
+        for t in params:
+            t.zero_()
+        torch.cuda.synchronize()
+        for t, source in zip(params[::-1], (beta, gamma, s, b, w)):
+            t.copy_(source)
+        fused_step(*params[:3], x, out, inner, 8, "silu", *params[3:], mr, partials)
+        assert torch.equal(out, want)
