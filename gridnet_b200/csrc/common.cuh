@@ -68,7 +68,8 @@ struct Act {
 // A kernel launched with launch_after may start while the one before it still runs; previous_done() waits until that one has
 // completed and only then lets the next one start. So when a kernel starts, everything but its direct predecessor is
 // complete: ahead of previous_done() it may read what older kernels (or the caller's program) have written, and write nothing
-// but its own shared and tensor memory. What overlaps is the launch itself and the loading of parameters, 2 to 7 us of a
+// but its own shared and tensor memory; and what the predecessor writes it reads with ordinary loads, not __ldg, whose data
+// must not change while the kernel runs. What overlaps is the launch itself and the loading of parameters, 2 to 7 us of a
 // kernel that takes 10 to 30 on the small grids.
 __device__ __forceinline__ void previous_done()
 {

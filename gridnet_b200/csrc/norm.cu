@@ -78,8 +78,7 @@ __global__ void __launch_bounds__(1024) norm_finalize_k(const double2 *partials,
 }
 
 // grid B * ceil(P / 1024), one dimension
-__global__ void __launch_bounds__(256) norm_apply_k(const float *x, const float *__restrict__ gamma,
-                                                    const float *__restrict__ beta,
+__global__ void __launch_bounds__(256) norm_apply_k(const float *x, const float *gamma, const float *beta,
                                                     const float2 *stats, float *y, long long P, unsigned chunks)
 {
     const int b = blockIdx.x / chunks;

@@ -189,7 +189,7 @@ __device__ __forceinline__ void quad_move(const float4 *src, unsigned col)
     float r[4 * N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
-        const float4 v = __ldg(src + k * 32);
+        const float4 v = src[k * 32];  // not __ldg: the kernel before may be writing it still
         r[4 * k + 0] = v.x, r[4 * k + 1] = v.y, r[4 * k + 2] = v.z, r[4 * k + 3] = v.w;
     }
     int k = 0;
@@ -216,7 +216,7 @@ __device__ __forceinline__ void quad_load_wsum(const float *wsum, int region, in
     float r[16];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        const float4 v = __ldg(src + k * 32);
+        const float4 v = src[k * 32];  // not __ldg: the kernel before may be writing it still
         r[4 * k + 0] = v.x, r[4 * k + 1] = v.y, r[4 * k + 2] = v.z, r[4 * k + 3] = v.w;
     }
     tmem_st16(tm + quad::COL_WSUM, r);

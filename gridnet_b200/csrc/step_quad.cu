@@ -411,8 +411,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
 
 // ---- layout conversion at the ends of a loop --------------------------------------------------------------
 // IL4 -> [B, P], normalised on the way when statistics are given
-__global__ void __launch_bounds__(256) from_il4_k(const float4 *il, const float2 *stats,
-                                                  const float *__restrict__ gamma, const float *__restrict__ beta,
+__global__ void __launch_bounds__(256) from_il4_k(const float4 *il, const float2 *stats, const float *gamma, const float *beta,
                                                   float *y, int B, size_t P)
 {
     const size_t c = (size_t)blockIdx.x * 256 + threadIdx.x;

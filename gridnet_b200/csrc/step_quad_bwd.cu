@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
                     quad_load(p.raw + own, zstr, ystr, L.h, r);
 #pragma unroll
                     for (int s = 0; s < 4; ++s) {
-                        m4[s] = __ldg(p.stats + 4 * q + s);
-                        a4[s] = __ldg(p.ac + 4 * q + s);
+                        m4[s] = p.stats[4 * q + s];
+                        a4[s] = p.ac[4 * q + s];
                     }
                     tmem_ld16(tm + COL_BIAS, gm);
                 }
@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
         if (!GATED) {  // scale terms of this quad
             const float *s = p.dsq + (size_t)q * P + g0;
 #pragma unroll
-            for (int dz = 0; dz < 2; ++dz) ds[dz] = fadd2(ds[dz], pack2(__ldg(s + dz * zs), __ldg(s + dz * zs + p.K)));
+            for (int dz = 0; dz < 2; ++dz) ds[dz] = fadd2(ds[dz], pack2(s[dz * zs], s[dz * zs + p.K]));
         }
         if (!mbar_wait_bounded(bar0 + 8 * buf_x, (landed >> buf_x) & 1u, kSpin)) failed = true;
         landed ^= 1u << buf_x;
@@ -520,7 +520,7 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
             if (FUSE_IN) {
                 float2 mr[4];
 #pragma unroll
-                for (int s = 0; s < 4; ++s) mr[s] = __ldg(p.in_stats + 4 * q + s);
+                for (int s = 0; s < 4; ++s) mr[s] = p.in_stats[4 * q + s];
                 na[0] = pack2(mr[0].y, mr[1].y);
                 na[1] = pack2(mr[2].y, mr[3].y);
                 nb[0] = pack2(-mr[0].x * mr[0].y, -mr[1].x * mr[1].y);
