@@ -1155,26 +1155,40 @@ __global__ void __launch_bounds__(256) quad_residual_combine_k(const float4 *__r
 #pragma unroll
         for (int s = 0; s < 4; ++s) mr[s] = __ldg(stats + 4 * q + s);
     }
+    float o[CPT][4];
+    {
+        float4 hv[CPT], yv[CPT];
+        float g[CPT], b[CPT];
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) {
+            const size_t c = c0 + k * 256, i = (size_t)q * P + c;
+            hv[k] = yv[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+            g[k] = b[k] = 0.0f;
+            if (c < P) {  // the whole CTA
+                hv[k] = h[i];
+                if (y) {
+                    yv[k] = y[i];
+                    g[k] = gamma[c], b[k] = beta[c];
+                }
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < CPT; ++k) {
+            const size_t c = c0 + k * 256;
+            const float hs[4] = {hv[k].x, hv[k].y, hv[k].z, hv[k].w}, ys[4] = {yv[k].x, yv[k].y, yv[k].z, yv[k].w};
+#pragma unroll
+            for (int s = 0; s < 4; ++s) o[k][s] = y ? hs[s] + (ys[s] - fmaf((hs[s] - mr[s].x) * mr[s].y, g[k], b[k])) : hs[s];
+            if (y && c < P) out[(size_t)q * P + c] = make_float4(o[k][0], o[k][1], o[k][2], o[k][3]);
+            if (c >= P) o[k][0] = o[k][1] = o[k][2] = o[k][3] = 0.0f;
+        }
+    }
     double sum = 0.0, squares = 0.0;  // of sample lane & 3
 #pragma unroll
     for (int k = 0; k < CPT; ++k) {
-        const size_t c = c0 + k * 256;
-        if (c >= P) continue;  // the whole CTA
-        const size_t i = (size_t)q * P + c;
-        const float4 hv = h[i];
-        float o[4] = {hv.x, hv.y, hv.z, hv.w};
-        if (y) {
-            const float4 yv = y[i];
-            const float ys[4] = {yv.x, yv.y, yv.z, yv.w};
-            const float g = gamma[c], b = beta[c];
-#pragma unroll
-            for (int s = 0; s < 4; ++s) o[s] = o[s] + (ys[s] - fmaf((o[s] - mr[s].x) * mr[s].y, g, b));
-            out[i] = make_float4(o[0], o[1], o[2], o[3]);
-        }
         float a[4], b[4];
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
-            const float other = __shfl_xor_sync(0xffffffffu, o[s], 1), lo = lane & 1 ? other : o[s], hi = lane & 1 ? o[s] : other;
+            const float other = __shfl_xor_sync(0xffffffffu, o[k][s], 1), lo = lane & 1 ? other : o[k][s], hi = lane & 1 ? o[k][s] : other;
             a[s] = lo + hi;
             b[s] = fmaf(lo, lo, hi * hi);
             a[s] += __shfl_xor_sync(0xffffffffu, a[s], 2);
