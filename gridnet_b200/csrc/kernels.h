@@ -179,6 +179,7 @@ int launch_quad_prepare(const QuadPrepare &a, int M, int N, int K, int block, cu
 int launch_from_il4(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, long long P,
                     cudaStream_t st);
 int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st);
+int launch_step_fwd_taps(const QuadStep &a, int act, cudaStream_t st);  // step_taps.cu: what launch_step_fwd_quad takes for a.ordered
 
 // ---- step_quad_bwd.cu (backward of the quad kernels; all activation tensors IL4)
 struct QuadReverse {
@@ -225,7 +226,7 @@ int launch_quad_norm_residual_apply(const float *h, const float *gn, const float
 int quad_combine_parts(long long P);
 int launch_quad_residual_combine(const float *h, const float *y, const float *gamma, const float *beta, const float2 *stats, float *out,
                                  double2 *partials, int Q, long long P, cudaStream_t st);
-int quad_make_map(CUtensorMap *map, const float *il, int M, int N, int K, int Q, int block);
+int quad_make_map(CUtensorMap *map, const float *il, int M, int N, int K, int Q, int block, int row = 0);
 
 // ---- step_quad_gated.cu (gated update, block 8; all activation tensors IL4)
 struct QuadGated {

@@ -316,130 +316,6 @@ __device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, 
     }
 }
 
-__device__ __forceinline__ void swap_if(bool c, u64 &a, u64 &b)
-{
-    const u64 t = c ? b : a;
-    b = c ? a : b;
-    a = t;
-}
-// A lane's neurons between the order of its walk and ascending (y, x): planes dz = 0 (n = 0, 1) or 1 (n = 2, 3)
-template <int SUB>
-__device__ __forceinline__ void quad_turn(const QuadLane<SUB> &L, int dz, u64 (&acc)[4][4][2])
-{
-#pragma unroll
-    for (int o = 0; o < 4; ++o)
-#pragma unroll
-        for (int k = 0; k < 2; ++k) swap_if(L.ysgn < 0, acc[2 * dz][o][k], acc[2 * dz + 1][o][k]);
-#pragma unroll
-    for (int dy = 0; dy < 2; ++dy)
-#pragma unroll
-        for (int o = 0; o < 2; ++o)
-#pragma unroll
-            for (int k = 0; k < 2; ++k) swap_if(L.h, acc[2 * dz + dy][o][k], acc[2 * dz + dy][3 - o][k]);
-}
-
-// quad_stencil<BIAS> with every neuron's taps added in the order of their numbers, as the register-patch kernels do
-// (step_fast.cu), which makes the sums the same bits. Loops with gradients need that: rounding that differs is amplified
-// from step to step (block 4, 8 x 16 iterations, silu: gradients up to 3e-5 apart in the 2-norm), and where it carries a
-// pre-activation over the kink of (leaky) relu, gradients jump (40 x 56 x 72, 4 x 10 iterations: 1e-4).
-// The walk over the tile stays as it is, it is what keeps the loads free of bank conflicts; the upper halves' rows and cells
-// are turned round in registers (12 selects per cell of a window row). The parameters are packed for it (QuadPrepare::ordered):
-// weights and biases in ascending (y, x), scales in the lane's order, in which `done` sees the neurons.
-template <int SUB, int PLANE, typename Done>
-__device__ __forceinline__ void quad_stencil_ordered(const QuadLane<SUB> &L, const unsigned (&rows)[4], int dx, unsigned tm, u64 (&acc)[4][4][2],
-                                                     Done done)
-{
-    float wb[2][12], sc[2][4];
-    auto finish = [&](int n, int o, float s) {
-        u64 c0, c1;
-        int step = dx;
-        asm volatile("" : "+r"(step));
-        lds128u(rows[1 + (n & 1)] + (unsigned)((1 + o) * step) + (1 + (n >> 1)) * PLANE * 16u, c0, c1);
-        done(n, o, s, 0.0f, c0, c1);
-    };
-    {
-        float first[16];
-        tmem_ld16(tm + quad::COL_BIAS, first);
-        tmem_wait_ld16(first);
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-#pragma unroll
-            for (int o = 0; o < 4; ++o) acc[n][o][0] = acc[n][o][1] = pack2(first[n * 4 + o], first[n * 4 + o]);
-    }
-    tmem_ld8(tm, wb[0]);
-    tmem_ld4(tm + 8, wb[0] + 8);
-    int use = 0, fin = 0;
-#pragma unroll
-    for (int rz = 0; rz < 4; ++rz) {
-        u64 v[4][6][2];
-        int step = dx;
-        asm volatile("" : "+r"(step));  // the cells' addresses are added up again: kept, they would take 24 registers
-        auto load2 = [&](int r0, int r1) {  // two rows that the upper half of the lanes has the other way round
-#pragma unroll
-            for (int j = 0; j < 6; ++j) {
-                lds128u(rows[r0] + (unsigned)(j * step) + rz * PLANE * 16u, v[r0][j][0], v[r0][j][1]);
-                lds128u(rows[r1] + (unsigned)(j * step) + rz * PLANE * 16u, v[r1][j][0], v[r1][j][1]);
-            }
-        };
-        auto turn2 = [&](int r0, int r1) {
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-#pragma unroll
-                for (int j = 0; j < 6; ++j) swap_if(L.ysgn < 0, v[r0][j][k], v[r1][j][k]);
-#pragma unroll
-                for (int j = 0; j < 3; ++j) {
-                    swap_if(L.h, v[r0][j][k], v[r0][5 - j][k]);
-                    swap_if(L.h, v[r1][j][k], v[r1][5 - j][k]);
-                }
-            }
-        };
-        load2(0, 3);
-        turn2(0, 3);
-        if (rz == 3) quad_turn(L, 0, acc);
-#pragma unroll
-        for (int ry = 0; ry < 4; ++ry) {
-            if (ry == 1) {
-                load2(1, 2);
-                turn2(1, 2);
-            }
-#pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                const int a = rz - (n >> 1), b = ry - (n & 1);
-                if (a < 0 || a > 2 || b < 0 || b > 2) continue;
-                float *wp = wb[use & 1];
-                tmem_wait_ld12(wp);
-                if (use == 30) tmem_use8(sc[0]);  // asked for before: that wait covered it
-                if (use + 1 < 36) {
-                    tmem_ld8(tm + (use + 1) * 12, wb[(use & 1) ^ 1]);
-                    tmem_ld4(tm + (use + 1) * 12 + 8, wb[(use & 1) ^ 1] + 8);
-                }
-                if (use == 29) {
-                    tmem_ld4(tm + quad::COL_SCALE, sc[0]);
-                    tmem_ld4(tm + quad::COL_SCALE + 4, sc[1]);
-                }
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-#pragma unroll
-                    for (int o = 0; o < 4; ++o) {
-                        const u64 ww = pack2(wp[c * 4 + o], wp[c * 4 + o]);
-                        ffma2(acc[n][o][0], v[ry][o + c][0], ww);
-                        ffma2(acc[n][o][1], v[ry][o + c][1], ww);
-                    }
-                ++use;
-                if (rz == 3)
-#pragma unroll
-                    for (int e = (use - 30) * 8 / 6; fin < e; ++fin) finish(fin >> 2, fin & 3, sc[fin >> 2][fin & 3]);
-            }
-        }
-    }
-    quad_turn(L, 1, acc);
-    tmem_ld4(tm + quad::COL_SCALE + 8, sc[0]);
-    tmem_ld4(tm + quad::COL_SCALE + 12, sc[1]);
-    tmem_wait_ld8(sc[0]);
-#pragma unroll
-    for (int e = 0; e < 8; ++e) finish(2 + (e >> 2), e & 3, sc[e >> 2][e & 3]);
-}
-
 // Adds eight values over the warp; afterwards lanes 4 j .. 4 j + 3 all hold the sum of value j.
 __device__ __forceinline__ float quad_reduce8(const float (&v)[8], int lane)
 {
@@ -455,6 +331,12 @@ __device__ __forceinline__ float quad_reduce8(const float (&v)[8], int lane)
     return c;
 }
 
+__device__ __forceinline__ void swap_if(bool c, u64 &a, u64 &b)
+{
+    const u64 t = c ? b : a;
+    b = c ? a : b;
+    a = t;
+}
 // The sum (j = 0) and the sum of squares (j = 1) of a region's values for the quad's samples s = 0 .. 3, in lane 4 j + s. As in
 // step_fast.cu the 128 values of two planes are added in float, in that kernel's order (four by four, then over z, y and
 // x), and the four pairs of planes in double: the statistics of a step are the same whichever kernel ran it.

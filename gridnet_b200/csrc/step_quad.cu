@@ -32,6 +32,7 @@
 #include "kernels.h"
 #include "packed.cuh"
 #include "quad_geo.cuh"
+#include "taps_geo.cuh"
 #include "tmem.cuh"
 
 namespace gn {
@@ -61,8 +62,7 @@ struct QuadParams {
 // to subtract it and to take the sums over its halo, which no iteration changes; from then on the tile holds v - c, so
 // that neither the variance nor sum w v - mean sum w cancels. Each iteration adds up the values it has just computed
 // while they are still in registers.
-// ORDERED: the sums of quad_stencil_ordered, the bits of step_fast.cu: everything that is differentiated.
-template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM, bool ORDERED>
+template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM>
 __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     step_fwd_quad(const __grid_constant__ CUtensorMap in_map, const QuadParams p)
 {
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     __syncthreads();
     tmem_fence_after();
     const unsigned tm = tmem_slot + ((unsigned)(quarter * 32) << 16);
-    static_assert(!(NORM && (FUSE_IN || ORDERED)), "per-block normalisation takes plain input, in the order of the walk");
+    static_assert(!(NORM && FUSE_IN), "per-block normalisation takes plain input");
 
     const QuadLane<SUB> L(lane);
     // NORM: the lane's share of its tile's cells, first + STRIDE k; four lanes share a block-4 tile, and the first two
@@ -370,8 +370,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                     acc[n][o][0] = act_residual2<ACT>(acc[n][o][0], scale, c0);
                     acc[n][o][1] = act_residual2<ACT>(acc[n][o][1], scale, c1);
                 };
-                if constexpr (ORDERED) quad_stencil_ordered<SUB, G::PLANE>(L, rows, L.xsgn * 16, tm, acc, done);
-                else quad_stencil<G::PLANE, NORM ? NORMED : BIAS>(rows, L.xsgn * 16, tm, acc, negm, done);
+                quad_stencil<G::PLANE, NORM ? NORMED : BIAS>(rows, L.xsgn * 16, tm, acc, negm, done);
                 __syncwarp();  // every lane has read its window
                 if (!last) {
 #pragma unroll
@@ -450,23 +449,23 @@ __device__ __forceinline__ void to_il4(const float *__restrict__ x, float4 *__re
 
 // Parameters in the order of the stencil: vector v of a region is, for every lane, the four x-neighbouring weights of
 // one (neuron row, tap), v = 0 .. 107 in the order of the uses in quad_stencil (three x-taps each), then the four rows
-// of b, then of s. ORDERED: for quad_stencil_ordered, weights and b in ascending (y, x). TRANS: the weights of the backward sum, in which a cell collects from the neurons of its own block
+// of b, then of s. TRANS: the weights of the backward sum, in which a cell collects from the neurons of its own block
 // that read it: the neuron at tap t sees the cell through its tap 26 - t; zero across the block's border. Four CTAs of 256 threads per
 // region, so that small grids fill the GPU; reads are 16-byte pieces, writes whole lines.
 constexpr int kPackCtas = 4;
-template <int SUB, bool TRANS, bool ORDERED>
+template <int SUB, bool TRANS>
 __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const float *__restrict__ b, const float *__restrict__ s,
                                           float *__restrict__ packed, size_t tap, int M, int N, int K, int cta)
 {
     __shared__ unsigned char uses[36];  // (a * 3 + b) | n << 4
     if (threadIdx.x == 0) {
         int k = 0;
-        for (int r = 0; r < 16; ++r)
-            for (int n = 0; n < 4; ++n) {
-                const int rz = ORDERED ? r >> 2 : r & 3, ry = ORDERED ? r & 3 : r >> 2;
-                const int a = rz - (n >> 1), bb = ry - (n & 1);
-                if (a >= 0 && a <= 2 && bb >= 0 && bb <= 2) uses[k++] = (unsigned char)((a * 3 + bb) | n << 4);
-            }
+        for (int ry = 0; ry < 4; ++ry)
+            for (int rz = 0; rz < 4; ++rz)
+                for (int n = 0; n < 4; ++n) {
+                    const int a = rz - (n >> 1), bb = ry - (n & 1);
+                    if (a >= 0 && a <= 2 && bb >= 0 && bb <= 2) uses[k++] = (unsigned char)((a * 3 + bb) | n << 4);
+                }
     }
     __syncthreads();
     const int lane = threadIdx.x & 31;
@@ -474,7 +473,7 @@ __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const flo
     const int nbx = K >> 3, nby = N >> 3, blk = cta / kPackCtas;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t g0 = ((size_t)(bz * 8 + L.z0) * N + (by * 8 + L.y0)) * K + bx * 8 + 4 * L.h;
-    const long long zs = (long long)N * K;
+    const long long zs = (long long)N * K, ys = (long long)L.ysgn * K;
     float4 *out = reinterpret_cast<float4 *>(packed + (size_t)blk * quad::PACK_F) + lane;
 #pragma unroll
     for (int i = 0; i < (quad::VECS + 8 * kPackCtas - 1) / (8 * kPackCtas); ++i) {
@@ -482,16 +481,13 @@ __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const flo
         if (v >= quad::VECS) break;
         int n;
         float4 r;
-        const bool turned = ORDERED && v < 112;                // ascending, whatever the lane's walk
-        const size_t g1 = turned && L.ysgn < 0 ? g0 - K : g0;  // row dy = 0
-        const long long ys = turned ? K : (long long)L.ysgn * K;
         if (v < 108) {
             const int u = uses[v / 3], c = v % 3;
             n = u >> 4;
             // the tap as the grid numbers it (gridnet/backend_torch.py:283-298)
-            const int ta = (u & 15) / 3, tb = !turned && L.ysgn < 0 ? 2 - (u & 15) % 3 : (u & 15) % 3, tc = !turned && L.h ? 2 - c : c;
+            const int ta = (u & 15) / 3, tb = L.ysgn < 0 ? 2 - (u & 15) % 3 : (u & 15) % 3, tc = L.h ? 2 - c : c;
             const int t = ta * 9 + tb * 3 + tc;
-            const size_t own = g1 + (n >> 1) * zs + (n & 1) * ys;
+            const size_t own = g0 + (n >> 1) * zs + (n & 1) * ys;
             if (!TRANS) {
                 const float *src = w + (size_t)t * tap + own;
                 if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) r = *reinterpret_cast<const float4 *>(src);
@@ -512,11 +508,45 @@ __device__ __forceinline__ void quad_pack(const float *__restrict__ w, const flo
             }
         } else {
             n = v & 3;
-            const float *src = (v < 112 ? b : s) + g1 + (n >> 1) * zs + (n & 1) * ys;
+            const float *src = (v < 112 ? b : s) + g0 + (n >> 1) * zs + (n & 1) * ys;
             if ((reinterpret_cast<uintptr_t>(src) & 15) == 0) r = *reinterpret_cast<const float4 *>(src);
             else r = make_float4(src[0], src[1], src[2], src[3]);
         }
-        out[v * 32] = L.h && !turned ? make_float4(r.w, r.z, r.y, r.x) : r;
+        out[v * 32] = L.h ? make_float4(r.w, r.z, r.y, r.x) : r;
+    }
+}
+
+// The same for tap_stencil (step_taps.cu): its order of uses and its lanes, whose rows of four lie along x as they are.
+template <int SUB>
+__device__ __forceinline__ void tap_pack(const float *__restrict__ w, const float *__restrict__ b, const float *__restrict__ s,
+                                         float *__restrict__ packed, size_t tap, int N, int K, int cta)
+{
+    __shared__ unsigned char uses[36];  // (a * 3 + b) | n << 4
+    if (threadIdx.x == 0) {
+        int k = 0;
+        for (int rz = 0; rz < 6; ++rz)
+            for (int bb = 0; bb < 3; ++bb)
+                for (int n = 0; n < 4; ++n)
+                    if (rz - n >= 0 && rz - n <= 2) uses[k++] = (unsigned char)(((rz - n) * 3 + bb) | n << 4);
+    }
+    __syncthreads();
+    const TapLane L(threadIdx.x & 31);
+    const int nbx = K >> 3, nby = N >> 3, blk = cta / kPackCtas;
+    const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
+    const size_t g0 = ((size_t)(bz * 8 + 4 * L.zp) * N + (by * 8 + L.y)) * K + bx * 8 + 4 * L.h, zs = (size_t)N * K;
+    float4 *out = reinterpret_cast<float4 *>(packed + (size_t)blk * quad::PACK_F) + (threadIdx.x & 31);
+#pragma unroll
+    for (int i = 0; i < (quad::VECS + 8 * kPackCtas - 1) / (8 * kPackCtas); ++i) {
+        const int v = (i * kPackCtas + cta % kPackCtas) * 8 + (threadIdx.x >> 5);
+        if (v >= quad::VECS) break;
+        const float *src;
+        if (v < 108) {
+            const int u = uses[v / 3];
+            src = w + (size_t)((u & 15) * 3 + v % 3) * tap + g0 + (u >> 4) * zs;
+        } else {
+            src = (v < 112 ? b : s) + g0 + (v & 3) * zs;
+        }
+        out[v * 32] = (reinterpret_cast<uintptr_t>(src) & 15) == 0 ? *reinterpret_cast<const float4 *>(src) : make_float4(src[0], src[1], src[2], src[3]);
     }
 }
 
@@ -584,8 +614,11 @@ __global__ void __launch_bounds__(256) quad_prepare_k(const PrepareArgs p)
     if (c < p.end[1]) {  // branch k of a gated network: weights [27][2][P], bias [2][P]
         const unsigned j = c < p.end[0] ? c : c - p.end[0], k = j / p.pack;
         const size_t to = (size_t)k * (p.pack / kPackCtas) * quad::PACK_F;
-        if (c < p.end[0]) quad_pack<SUB, false, ORDERED>(a.w + k * P, a.b + k * P, a.s, a.packed + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
-        else quad_pack<SUB, true, false>(a.w + k * P, a.b_t + k * P, a.s, a.packed_t + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
+        if (c < p.end[0]) {
+            if (ORDERED) tap_pack<SUB>(a.w + k * P, a.b + k * P, a.s, a.packed + to, tap, p.N, p.K, (int)(j % p.pack));
+            else quad_pack<SUB, false>(a.w + k * P, a.b + k * P, a.s, a.packed + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
+        }
+        else quad_pack<SUB, true>(a.w + k * P, a.b_t + k * P, a.s, a.packed_t + to, tap, p.M, p.N, p.K, (int)(j % p.pack));
     }
     else if (c < p.end[2]) quad_wsum<SUB>(a.w, reinterpret_cast<float4 *>(a.wsum), p.M, p.N, p.K, (int)(c - p.end[1]));
     else if (c < p.end[3]) quad_table<SUB>(a.gamma, a.beta, a.gbt, p.M, p.N, p.K, (int)(c - p.end[2]));
@@ -602,16 +635,17 @@ bool quad_applicable(int M, int N, int K, int block, int inner)
     return encode_tiled_fn() != nullptr;
 }
 
-// tensor map over an IL4 buffer, box = one tile (10^3 or 6^3 cells)
-int quad_make_map(CUtensorMap *map, const float *il, int M, int N, int K, int Q, int block)
+// tensor map over an IL4 buffer, box = one tile (10^3 or 6^3 cells), or with rows of `row` cells
+int quad_make_map(CUtensorMap *map, const float *il, int M, int N, int K, int Q, int block, int row)
 {
-    MapKey key{il, block == 8 ? 40 : 24, 0, {M, N, K, Q}};
+    const cuuint32_t side = block == 8 ? 10 : 6;
+    if (row == 0) row = (int)side;
+    MapKey key{il, 4 * row, 0, {M, N, K, Q}};
     (void)cudaGetDevice(&key.dev);
     if (tensor_map_cache_get(key, map)) return GN_OK;
     const cuuint64_t dims[4] = {(cuuint64_t)K * 4, (cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)Q};
     const cuuint64_t strides[3] = {(cuuint64_t)K * 16, (cuuint64_t)N * K * 16, (cuuint64_t)M * N * K * 16};
-    const cuuint32_t side = block == 8 ? 10 : 6;
-    const cuuint32_t box[4] = {4 * side, side, side, 1};
+    const cuuint32_t box[4] = {4 * (cuuint32_t)row, side, side, 1};
     const cuuint32_t estr[4] = {1, 1, 1, 1};
     const CUresult r = encode_tiled_fn()(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float *>(il), dims, strides, box, estr,
                                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
@@ -657,11 +691,11 @@ int launch_quad_prepare(const QuadPrepare &a, int M, int N, int K, int block, cu
     return check_launch("quad_prepare");
 }
 
-template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM, bool ORDERED>
+template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM>
 static int launch_quad_one(const CUtensorMap &map, const QuadParams &p, unsigned ctas, cudaStream_t st)
 {
     using G = QuadGeo<SUB>;
-    auto kern = step_fwd_quad<SUB, ACT, FUSE_IN, SAVE, NORM, ORDERED>;
+    auto kern = step_fwd_quad<SUB, ACT, FUSE_IN, SAVE, NORM>;
     // tiles; block 8 with normalise-on-load also a (gamma, beta) table per team
     constexpr int smem = quad::QUARTERS * G::NBUF * G::BUF_BYTES + (SUB == 8 && FUSE_IN ? quad::QUARTERS * G::CELLS * 8 : 0);
     static_assert(smem <= 232448 - 1024 - 256, "shared memory budget of one SM");
@@ -678,31 +712,28 @@ static int launch_quad_one(const CUtensorMap &map, const QuadParams &p, unsigned
 }
 
 template <int SUB, int ACT>
-static int launch_quad_act(const CUtensorMap &map, const QuadParams &p, bool ordered, unsigned ctas, cudaStream_t st)
+static int launch_quad_act(const CUtensorMap &map, const QuadParams &p, unsigned ctas, cudaStream_t st)
 {
-#define ONE_(FUSE_IN, SAVE, NORM, ORDERED) launch_quad_one<SUB, ACT, FUSE_IN, SAVE, NORM, ORDERED>(map, p, ctas, st)
-    if (p.wsum) return p.save_h ? ONE_(false, true, true, false) : ONE_(false, false, true, false);
-    if (!ordered) return p.in_stats ? ONE_(true, false, false, false) : ONE_(false, false, false, false);
-    if (p.save_h) return p.in_stats ? ONE_(true, true, false, true) : ONE_(false, true, false, true);
-    return p.in_stats ? ONE_(true, false, false, true) : ONE_(false, false, false, true);
-#undef ONE_
+    if (p.wsum) return p.save_h ? launch_quad_one<SUB, ACT, false, true, true>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, false, true>(map, p, ctas, st);
+    return p.in_stats ? launch_quad_one<SUB, ACT, true, false, false>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, false, false>(map, p, ctas, st);
 }
 
 template <int SUB>
-static int launch_quad_sub(const CUtensorMap &map, const QuadParams &p, bool ordered, unsigned ctas, int act, cudaStream_t st)
+static int launch_quad_sub(const CUtensorMap &map, const QuadParams &p, unsigned ctas, int act, cudaStream_t st)
 {
     switch (act) {
-    case GN_ACT_RELU: return launch_quad_act<SUB, GN_ACT_RELU>(map, p, ordered, ctas, st);
-    case GN_ACT_LEAKY_RELU: return launch_quad_act<SUB, GN_ACT_LEAKY_RELU>(map, p, ordered, ctas, st);
-    case GN_ACT_SILU: return launch_quad_act<SUB, GN_ACT_SILU>(map, p, ordered, ctas, st);
-    default: return launch_quad_act<SUB, GN_ACT_TANH>(map, p, ordered, ctas, st);
+    case GN_ACT_RELU: return launch_quad_act<SUB, GN_ACT_RELU>(map, p, ctas, st);
+    case GN_ACT_LEAKY_RELU: return launch_quad_act<SUB, GN_ACT_LEAKY_RELU>(map, p, ctas, st);
+    case GN_ACT_SILU: return launch_quad_act<SUB, GN_ACT_SILU>(map, p, ctas, st);
+    default: return launch_quad_act<SUB, GN_ACT_TANH>(map, p, ctas, st);
     }
 }
 
 int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
 {
     if (a.wsum && (a.in_stats || a.ordered || !a.save_h != !a.tile_stats)) return GN_ERR_UNSUPPORTED;
-    if (!a.wsum && a.save_h && !a.ordered) return GN_ERR_UNSUPPORTED;
+    if (a.ordered) return launch_step_fwd_taps(a, act, st);
+    if (!a.wsum && a.save_h) return GN_ERR_UNSUPPORTED;
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
     const int rc = quad_make_map(&map, a.in_il4, a.M, a.N, a.K, a.Q, a.block);
@@ -718,7 +749,7 @@ int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
     p.nitems = (long long)(a.M / 8) * (a.N / 8) * (a.K / 8) * a.Q;
     long long ctas = (p.nitems + quad::QUARTERS - 1) / quad::QUARTERS;
     if (ctas > sm_count()) ctas = sm_count();
-    return a.block == 8 ? launch_quad_sub<8>(map, p, a.ordered, (unsigned)ctas, act, st) : launch_quad_sub<4>(map, p, a.ordered, (unsigned)ctas, act, st);
+    return a.block == 8 ? launch_quad_sub<8>(map, p, (unsigned)ctas, act, st) : launch_quad_sub<4>(map, p, (unsigned)ctas, act, st);
 }
 
 }  // namespace gn

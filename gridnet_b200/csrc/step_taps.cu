@@ -1,0 +1,346 @@
+// Float forward of the block-local update on the quad layout (block 8 and 4, per-block normalisation off), weights in tensor
+// memory and four samples per lane as in step_quad.cu, every neuron's taps added in the order of their numbers: the same
+// bits as the register-patch kernel (step_fast.cu), statistics included. Loops with gradients need that: rounding that
+// differs is amplified from step to step (block 4, 8 x 16 iterations, silu: gradients up to 3e-5 apart in the 2-norm), and
+// where it carries a pre-activation over the kink of (leaky) relu gradients jump (40 x 56 x 72, 4 x 10 iterations: 1e-4).
+//
+// What differs from step_quad.cu is the split of a region over the lanes and the layout of the tile (taps_geo.cuh). Items,
+// teams, parameters in tensor memory, normalise-on-load and the overlap of launches are as described there.
+// Block 8: tiles by bulk tensor copy. Block 4: each warp fetches its own next tile, cell by cell and asynchronously; its
+// eight small tiles have to lie an odd number of cells apart, which bulk tensor copies cannot do.
+#include <string.h>
+
+#include "common.cuh"
+#include "kernels.h"
+#include "packed.cuh"
+#include "taps_geo.cuh"
+#include "tmem.cuh"
+
+namespace gn {
+
+namespace {
+
+using namespace quad;
+constexpr int TEAM = 2;  // warps per quarter of tensor memory
+constexpr int TABLE8 = QuadGeo<8>::CELLS;  // entries per region of the (gamma, beta) table, kept in shared memory (block 8)
+
+struct TapParams {
+    const float *packed;     // [regions][PACK_F], QuadPrepare::ordered
+    const float2 *gbt;       // FUSE_IN: (gamma, beta) per tile cell of every region, in the order of QuadGeo
+    const float2 *in_stats;  // FUSE_IN: [4 Q] (mean, rstd)
+    const float *in;         // block 4: IL4
+    double2 *out_partials;   // [4 Q][nparts]: slot `region` of every row is written; nullptr: not wanted
+    int nparts;
+    float *y;                // IL4; nullptr: not wanted (replay)
+    float *save_h;           // SAVE: [inner][Q][P][4]
+    int *error_flag;
+    int M, N, K, Q, inner;
+    int params_old;          // the kernel before this one did not write packed or gbt
+    long long nitems;        // regions * Q
+};
+
+// 16 bytes to shared memory, asynchronously; zeros where !inside (src is then not read)
+__device__ __forceinline__ void cp_async16_or_zero(unsigned dst, const float *src, bool inside)
+{
+    const int n = inside ? 16 : 0;
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+
+// Block 4: the eight tiles of region (bx, by, bz), quad q. Four lanes per tile: first the 36 rows' inner cells, whole sectors,
+// then the two outer cells of two rows at a time.
+__device__ __forceinline__ void fetch_tiles4(unsigned tile, const TapParams &p, int bx, int by, int bz, int q, int lane)
+{
+    using G = TapGeo<4>;
+    const int slot = lane >> 2, r = lane & 3;
+    const int z0 = bz * 8 + (slot >> 2) * 4 - 1, x0 = bx * 8 + ((slot >> 1) & 1) * 4 - 1, y0 = by * 8 + (slot & 1) * 4 - 1;
+    const bool zlo = z0 >= 0, zhi = z0 + 5 < p.M, ylo = y0 >= 0, yhi = y0 + 5 < p.N, xlo = x0 >= 0, xhi = x0 + 5 < p.K;
+    const long long zstr = 4ll * p.N * p.K, ystr = 4ll * p.K;
+    const float *const corner = p.in + ((long long)q * p.M + z0) * zstr + y0 * ystr + 4ll * x0;  // may lie outside, then not read
+    const unsigned to = tile + (unsigned)(slot * G::TILE) * 16u;
+    const int rr = r >> 1, side = (r & 1) * 5;
+    const bool x_in = side ? xhi : xlo;
+#pragma unroll
+    for (int cz = 0; cz < 6; ++cz) {
+        const bool z_in = cz == 0 ? zlo : (cz == 5 ? zhi : true);
+        const float *const plane = corner + cz * zstr;
+#pragma unroll
+        for (int cy = 0; cy < 6; ++cy) {
+            const bool in = z_in && (cy == 0 ? ylo : (cy == 5 ? yhi : true));
+            const float *src = plane + cy * ystr + 4 * (1 + r);
+            cp_async16_or_zero(to + (unsigned)(cz * G::PLANE + cy * G::ROW + 1 + r) * 16u, in ? src : p.in, in);
+        }
+#pragma unroll
+        for (int c2 = 0; c2 < 6; c2 += 2) {
+            const bool in = z_in && x_in && (c2 + rr == 0 ? ylo : (c2 + rr == 5 ? yhi : true));
+            const float *src = plane + (c2 + rr) * ystr + 4 * side;
+            cp_async16_or_zero(to + (unsigned)(cz * G::PLANE + (c2 + rr) * G::ROW + side) * 16u, in ? src : p.in, in);
+        }
+    }
+}
+
+template <int SUB, int ACT, bool FUSE_IN, bool SAVE>
+__global__ void __launch_bounds__(128 * TEAM, 1) step_fwd_taps(const __grid_constant__ CUtensorMap in_map, const TapParams p)
+{
+    using G = TapGeo<SUB>;
+    constexpr int NBUF = G::NBUF;
+    static_assert(SUB == 8 || NBUF == TEAM, "block 4: a buffer per warp");
+    extern __shared__ __align__(1024) unsigned char smem[];
+    __shared__ __align__(8) unsigned long long bars[QUARTERS * NBUF];
+    __shared__ int issued[QUARTERS * NBUF];  // which item's copy into this buffer has been started last
+    __shared__ unsigned tmem_slot;
+
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int quarter = warp & 3, role = warp >> 2;
+    if (warp == 0) tmem_alloc_all(&tmem_slot);
+    if (tid == 0) {
+        for (int i = 0; i < QUARTERS * NBUF; ++i) {
+            mbar_init(smem_u32(&bars[i]), 1);
+            issued[i] = -1;
+        }
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        fence_proxy_async();
+    }
+    float2 *const gbs = reinterpret_cast<float2 *>(smem + QUARTERS * NBUF * G::BUF_BYTES) + quarter * TABLE8;
+    tmem_fence_before();
+    __syncthreads();
+    tmem_fence_after();
+    const unsigned tm = tmem_slot + ((unsigned)(quarter * 32) << 16);
+
+    const TapLane L(lane);
+    const int nbx = p.K >> 3, nby = p.N >> 3;
+    const size_t P = (size_t)p.M * p.N * p.K;
+    const long long worker = (long long)blockIdx.x * QUARTERS + quarter, nworkers = (long long)gridDim.x * QUARTERS;
+    const long long n0 = p.nitems * worker / nworkers;
+    const int cnt = (int)(p.nitems * (worker + 1) / nworkers - n0);
+    const unsigned bar0 = smem_u32(&bars[quarter * NBUF]), issued0 = smem_u32(&issued[quarter * NBUF]);
+    const unsigned tiles = smem_u32(smem) + quarter * (NBUF * G::BUF_BYTES);
+    const long long zstr = 4ll * p.N * p.K;
+    bool failed = false;
+
+    // fetch the tile of the team's item i into its buffer: one lane (block 8), the whole warp (block 4)
+    auto issue = [&](int i) {
+        const long long n = n0 + i;
+        const int blk = (int)(n / p.Q), q = (int)(n - (long long)blk * p.Q);
+        const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
+        const unsigned tile = tiles + (i % NBUF) * G::BUF_BYTES, bar = bar0 + 8 * (i % NBUF);
+        if constexpr (SUB == 8) {
+            fence_proxy_async();  // earlier accesses to the buffer precede the bulk copy's writes
+            mbar_expect_tx(bar, G::CELLS * 16);
+            tma_load_4d(tile, &in_map, bar, (bx * 8 - 1) * 4, by * 8 - 1, bz * 8 - 1, q);
+            st_release_shared(issued0 + 4 * (i % NBUF), i);
+        } else {
+            fetch_tiles4(tile, p, bx, by, bz, q, lane);
+        }
+    };
+    auto wait_tile = [&](int i) {
+        if constexpr (SUB == 8) {  // see step_fwd_quad
+            unsigned spins = 0;
+            while (ld_acquire_shared(issued0 + 4 * (i % NBUF)) != i && ++spins < kSpinLimit) {}
+            if (spins >= kSpinLimit || !mbar_wait_bounded(bar0 + 8 * (i % NBUF), (unsigned)(i / NBUF) & 1u, kSpinLimit)) failed = true;
+        } else {
+            cp_async_wait_all();
+        }
+        __syncwarp();
+    };
+    auto begin = [&]() {
+        previous_done();
+        if constexpr (SUB == 8) {
+            if (role == 0 && lane == 0)
+                for (int i = 0; i < NBUF && i < cnt; ++i) issue(i);
+        } else {
+            if (role < cnt) issue(role);
+        }
+        __syncwarp();
+    };
+    if (!p.params_old || cnt == 0) begin();  // else the first region's parameters come first
+
+    int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
+    for (int i0 = 0; i0 < cnt;) {
+        const int here = min(cnt - i0, p.Q - q0);  // items of this region
+        const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
+        const size_t g0 = ((size_t)(bz * 8 + 4 * L.zp) * p.N + (by * 8 + L.y)) * p.K + bx * 8 + 4 * L.h;  // own patch
+        if (i0 > 0) {
+            tmem_fence_before();
+            team_sync<TEAM>(quarter);  // the other warp no longer reads the old region's weights
+            tmem_fence_after();
+        }
+        if (FUSE_IN && SUB == 8) {
+            const unsigned char *src = reinterpret_cast<const unsigned char *>(p.gbt + (size_t)blk * TABLE8);
+            const unsigned dst = smem_u32(gbs);
+            for (int c = role * 32 + lane; c < TABLE8 / 2; c += 32 * TEAM) cp_async16(dst + c * 16, src + c * 16);
+            __syncwarp();  // tensor memory instructions want the whole warp together
+        }
+        quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm);
+        tmem_wait_st();
+        if (FUSE_IN && SUB == 8) cp_async_wait_all();
+        if (i0 == 0 && p.params_old) begin();
+        tmem_fence_before();
+        team_sync<TEAM>(quarter);
+        tmem_fence_after();
+        if (i0 + here < cnt) {  // the next region's parameters on their way to L2
+            const unsigned char *nx = reinterpret_cast<const unsigned char *>(p.packed + (size_t)(blk + 1) * PACK_F);
+            for (int c = role * 32 + lane; c < PACK_F * 4 / 128; c += 32 * TEAM) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + c * 128));
+            __syncwarp();
+        }
+
+        // item i goes to warp i mod TEAM
+        for (int k = (role + TEAM - i0 % TEAM) % TEAM; k < here; k += TEAM) {
+            const int i = i0 + k, q = q0 + k;
+            const unsigned tile = tiles + (i % NBUF) * G::BUF_BYTES;
+            if (FUSE_IN) {
+                u64 rs[2], mu[2];  // rstd, -mean
+                {
+                    float2 mr[4];
+#pragma unroll
+                    for (int s = 0; s < 4; ++s) mr[s] = p.in_stats[4 * q + s];
+                    rs[0] = pack2(mr[0].y, mr[1].y);
+                    rs[1] = pack2(mr[2].y, mr[3].y);
+                    mu[0] = pack2(-mr[0].x, -mr[1].x);
+                    mu[1] = pack2(-mr[2].x, -mr[3].x);
+                }
+                wait_tile(i);
+                // step c: cell 32 c + lane of the tile (block 8), 4 c + r of the lane's small tile (block 4; the second
+                // tile of a pair is walked three cells ahead, which puts a quarter-warp on eight banks)
+                constexpr int STEPS = SUB == 8 ? 32 : 54, BATCH = SUB == 8 ? 16 : 18;
+                const int slot = lane >> 2, l0 = (lane & 3) + 3 * (slot & 1);
+                const unsigned sub = tile + (unsigned)(slot * 217) * 16u;
+                const float2 *const table = p.gbt + (size_t)blk * QuadGeo<4>::CELLS + ((slot >> 2) * 4 + (slot & 1) * 2 + ((slot >> 1) & 1)) * 216;
+                auto cell = [&](int c) { return SUB == 8 ? c * 32 + lane : (l0 + 4 * c >= 216 ? l0 + 4 * c - 216 : l0 + 4 * c); };
+                auto address = [&](int l) { return SUB == 8 ? tile + (unsigned)(l + l / 10) * 16u : sub + (unsigned)l * 16u; };
+#pragma unroll 1
+                for (int c0 = 0; c0 < STEPS; c0 += BATCH) {
+                    u64 v[BATCH][2];
+                    float2 g2[BATCH];
+#pragma unroll
+                    for (int c = 0; c < BATCH; ++c) {
+                        const int l = cell(c0 + c);
+                        if (SUB == 4 || l < TABLE8) {
+                            g2[c] = SUB == 8 ? gbs[l] : table[l];
+                            lds128u(address(l), v[c][0], v[c][1]);
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < BATCH; ++c) {
+                        const int l = cell(c0 + c);
+                        if (SUB == 4 || l < TABLE8) {
+                            const u64 gg = pack2(g2[c].x, g2[c].x), bb = pack2(g2[c].y, g2[c].y);
+                            sts128u(address(l), ffma2r(fmul2(fadd2(v[c][0], mu[0]), rs[0]), gg, bb), ffma2r(fmul2(fadd2(v[c][1], mu[1]), rs[1]), gg, bb));
+                        }
+                    }
+                }
+                __syncwarp();
+            } else {
+                wait_tile(i);
+            }
+
+            const unsigned win = tile + (unsigned)G::corner(L) * 16u;
+            const unsigned mine = win + (unsigned)(G::PLANE + G::ROW + 1) * 16u;  // own cell (0, 0)
+            const size_t own = ((size_t)q * P + g0) * 4;                           // the lane's cells in an IL4 tensor
+            for (int t = 0; t < p.inner; ++t) {
+                u64 acc[4][4][2], hold[2] = {0, 0};
+                float *const sh = SAVE ? p.save_h + (size_t)t * p.Q * P * 4 + own : nullptr;
+                tap_stencil<SUB>(win, tm, acc, [&](int n, int o, float scale, u64 c0, u64 c1) {
+                    if (SAVE) {  // two neighbours at a time
+                        if (o & 1) stg256(sh + n * zstr + 8 * (o >> 1), hold[0], hold[1], acc[n][o][0], acc[n][o][1]);
+                        else hold[0] = acc[n][o][0], hold[1] = acc[n][o][1];
+                    }
+                    acc[n][o][0] = act_residual2<ACT>(acc[n][o][0], scale, c0);
+                    acc[n][o][1] = act_residual2<ACT>(acc[n][o][1], scale, c1);
+                });
+                __syncwarp();  // every lane has read its window
+                if (t + 1 < p.inner) {
+#pragma unroll
+                    for (int n = 0; n < 4; ++n)
+#pragma unroll
+                        for (int o = 0; o < 4; ++o) sts128u(mine + (unsigned)(n * G::PLANE + o) * 16u, acc[n][o][0], acc[n][o][1]);
+                    __syncwarp();
+                } else {
+                    // the tile is dead: fetch the next one
+                    if (i + NBUF < cnt && (SUB == 4 || lane == 0)) issue(i + NBUF);
+                    __syncwarp();
+                    if (p.y)
+#pragma unroll
+                        for (int n = 0; n < 4; ++n)
+#pragma unroll
+                            for (int o = 0; o < 4; o += 2)
+                                stg256(p.y + own + n * zstr + 4 * o, acc[n][o][0], acc[n][o][1], acc[n][o + 1][0], acc[n][o + 1][1]);
+                    if (p.out_partials) {
+                        const double r = tap_region_sums(acc, lane);
+                        if ((lane & 20) == 0)
+                            reinterpret_cast<double *>(p.out_partials + (size_t)(4 * q + (lane & 2) + (lane >> 3)) * p.nparts + blk)[lane & 1] = r;
+                        __syncwarp();
+                    }
+                }
+            }
+        }
+        i0 += here;
+        q0 = 0;
+        ++blk;
+    }
+    if (failed && p.error_flag) *p.error_flag = 1;
+    tmem_fence_before();
+    __syncthreads();
+    if (warp == 0) tmem_free_all(tmem_slot);
+}
+
+template <int SUB, int ACT, bool FUSE_IN, bool SAVE>
+int launch_one(const CUtensorMap &map, const TapParams &p, unsigned ctas, cudaStream_t st)
+{
+    using G = TapGeo<SUB>;
+    auto kern = step_fwd_taps<SUB, ACT, FUSE_IN, SAVE>;
+    constexpr int smem = QUARTERS * G::NBUF * G::BUF_BYTES + (SUB == 8 && FUSE_IN ? QUARTERS * TABLE8 * 8 : 0);
+    static_assert(smem <= 232448 - 1024 - 256, "shared memory budget of one SM");
+    static unsigned long long attr_set = 0;
+    if (first_use_on_device(&attr_set)) {
+        const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        if (e != cudaSuccess) {
+            record_cuda_error(e, "cudaFuncSetAttribute(step_fwd_taps)");
+            return GN_ERR_CUDA;
+        }
+    }
+    launch_after(kern, ctas, 128 * TEAM, smem, st, map, p);
+    return check_launch("step_fwd_taps");
+}
+
+template <int SUB, int ACT>
+int launch_act(const CUtensorMap &map, const TapParams &p, unsigned ctas, cudaStream_t st)
+{
+    if (p.save_h) return p.in_stats ? launch_one<SUB, ACT, true, true>(map, p, ctas, st) : launch_one<SUB, ACT, false, true>(map, p, ctas, st);
+    return p.in_stats ? launch_one<SUB, ACT, true, false>(map, p, ctas, st) : launch_one<SUB, ACT, false, false>(map, p, ctas, st);
+}
+
+template <int SUB>
+int launch_sub(const CUtensorMap &map, const TapParams &p, unsigned ctas, int act, cudaStream_t st)
+{
+    switch (act) {
+    case GN_ACT_RELU: return launch_act<SUB, GN_ACT_RELU>(map, p, ctas, st);
+    case GN_ACT_LEAKY_RELU: return launch_act<SUB, GN_ACT_LEAKY_RELU>(map, p, ctas, st);
+    case GN_ACT_SILU: return launch_act<SUB, GN_ACT_SILU>(map, p, ctas, st);
+    default: return launch_act<SUB, GN_ACT_TANH>(map, p, ctas, st);
+    }
+}
+
+}  // namespace
+
+int launch_step_fwd_taps(const QuadStep &a, int act, cudaStream_t st)
+{
+    CUtensorMap map;
+    memset(&map, 0, sizeof(map));
+    if (a.block == 8) {
+        const int rc = quad_make_map(&map, a.in_il4, a.M, a.N, a.K, a.Q, 8, TapGeo<8>::ROW);
+        if (rc != GN_OK) return rc;
+    }
+    TapParams p{};
+    p.packed = a.packed; p.params_old = a.params_old;
+    p.gbt = a.gbt; p.in_stats = a.in_stats; p.in = a.in_il4;
+    p.out_partials = a.out_partials; p.nparts = a.nparts;
+    p.y = a.out_il4; p.save_h = a.save_h;
+    p.error_flag = a.error_flag ? a.error_flag : device_status_ptr();
+    p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;
+    p.nitems = (long long)(a.M / 8) * (a.N / 8) * (a.K / 8) * a.Q;
+    long long ctas = (p.nitems + QUARTERS - 1) / QUARTERS;
+    if (ctas > sm_count()) ctas = sm_count();
+    return a.block == 8 ? launch_sub<8>(map, p, (unsigned)ctas, act, st) : launch_sub<4>(map, p, (unsigned)ctas, act, st);
+}
+
+}  // namespace gn

@@ -59,6 +59,7 @@ __device__ __forceinline__ void tmem_use8(float *r)
 {
     asm volatile("" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]));
 }
+__device__ __forceinline__ void tmem_use4(float *r) { asm volatile("" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3])); }
 __device__ __forceinline__ void tmem_use12(float *r)
 {
     asm volatile("" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]), "+f"(r[8]),
@@ -76,6 +77,10 @@ __device__ __forceinline__ void tmem_wait_ld16(float *r)
     asm volatile("tcgen05.wait::ld.sync.aligned;"
                  : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]), "+f"(r[4]), "+f"(r[5]), "+f"(r[6]), "+f"(r[7]), "+f"(r[8]),
                    "+f"(r[9]), "+f"(r[10]), "+f"(r[11]), "+f"(r[12]), "+f"(r[13]), "+f"(r[14]), "+f"(r[15]));
+}
+__device__ __forceinline__ void tmem_wait_ld4(float *r)
+{
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+f"(r[0]), "+f"(r[1]), "+f"(r[2]), "+f"(r[3]));
 }
 __device__ __forceinline__ void tmem_wait_ld8(float *r)
 {
