@@ -1033,7 +1033,7 @@ static int outer_forward_impl(const float *w, const float *b, const float *s, co
         }
         QuadPrepare r{};
         if (!(flags & GN_OUTER_PARAMS_UNCHANGED)) {
-            r.w = w; r.b = b; r.s = s; r.packed = ws.qpacked;
+            r.w = w; r.b = b; r.s = s; r.packed = ws.qpacked; r.ordered = true;
             r.gamma = gamma; r.beta = beta; r.gbt = ws.gbt;
         }
         r.x = x; r.il = ws.buf[0]; r.B = B;

@@ -139,7 +139,7 @@ int launch_from_il64(const float *il, const float2 *stats, const float *gamma, c
 // ---- step_quad.cu (weights in tensor memory, four samples per lane; activations in the IL4 layout [quad][z][y][x][4
 // samples], blocks of 8 and 4; B need not be a multiple of 4, the missing samples are zeros)
 struct QuadStep {
-    const float *packed;      // from launch_quad_prepare
+    const float *packed;      // from launch_quad_prepare; without wsum in the order of the taps (QuadPrepare::ordered)
     const float2 *gbt;        // from launch_quad_prepare; used when in_stats is set
     const float *in_il4;
     float *out_il4;           // or nullptr
@@ -147,7 +147,6 @@ struct QuadStep {
     double2 *out_partials;    // [4 Q][nparts] or nullptr; slots 0 .. regions-1 of every row are written
     int nparts;
     float *save_h;            // [inner] IL4 tensors of pre-activations, or nullptr
-    bool ordered;             // packed is in the order of the taps (QuadPrepare::ordered); not with wsum, needed with save_h otherwise
     bool params_old;          // packed and gbt are not what the kernel queued just before writes
     const float *wsum;        // from launch_quad_prepare: per-block normalisation; nullptr: off
     float4 *tile_stats;       // with wsum and save_h: quad_stats_vectors(...) vectors
@@ -165,7 +164,7 @@ struct QuadPrepare {
     const float *w, *b, *s;
     bool gated;                // w, b, b_t and the packed parameters have two branches; s is not looked at (any M N K floats)
     float *packed;             // quad_packed_floats(...): weights, b, s in the order of the forward sums
-    bool ordered;              // ... in the order of the taps, for a QuadStep that says so too
+    bool ordered;              // ... in the order of the taps: for a QuadStep without wsum
     const float *b_t;
     float *packed_t;           // the same for the backward sums: transposed weights, b_t, s
     float *wsum;               // M N K floats: the neurons' weight sums
@@ -179,7 +178,7 @@ int launch_quad_prepare(const QuadPrepare &a, int M, int N, int K, int block, cu
 int launch_from_il4(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, long long P,
                     cudaStream_t st);
 int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st);
-int launch_step_fwd_taps(const QuadStep &a, int act, cudaStream_t st);  // step_taps.cu: what launch_step_fwd_quad takes for a.ordered
+int launch_step_fwd_taps(const QuadStep &a, int act, cudaStream_t st);  // step_taps.cu: what launch_step_fwd_quad takes without wsum
 
 // ---- step_quad_bwd.cu (backward of the quad kernels; all activation tensors IL4)
 struct QuadReverse {

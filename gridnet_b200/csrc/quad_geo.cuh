@@ -1,4 +1,4 @@
-// Geometry and building blocks shared by the quad kernels (step_quad.cu): how the 32 lanes of a warp split an 8^3
+// Geometry and building blocks shared by the quad kernels (step_quad.cu, step_quad_bwd.cu, step_quad_gated.cu): how the 32 lanes of a warp split an 8^3
 // region of the grid, where a lane's window lies in the tile, the order of the weights in tensor memory, and the
 // 27-tap sum itself.
 #pragma once
@@ -12,8 +12,8 @@ constexpr int QUARTERS = 4;
 constexpr unsigned kSpinLimit = 1u << 20;
 // columns of tensor memory: 36 uses of 12 weights, then 16 biases, 16 scales, 16 weight sums (per-block normalisation)
 constexpr int COL_BIAS = 432, COL_SCALE = 448, COL_WSUM = 464;
-// what the 27-tap sums start from: what is there (backward), the bias, or minus the tile's mean times the weight sum
-enum Mode { ADD, BIAS, NORMED };
+// what the 27-tap sums start from: what is there, or minus the tile's mean times the weight sum
+enum Mode { ADD, NORMED };
 }  // namespace quad
 
 // A region's tile buffer, in cells of 16 bytes (four samples).
@@ -223,26 +223,25 @@ __device__ __forceinline__ void quad_load_wsum(const float *wsum, int region, in
 }
 
 // The 27-tap sums of the lane's 16 neurons for four samples, acc[n = (dz, dy)][o][sample pair] += sum.
-//   BIAS: acc starts at the bias, and done(n, o, scale, bias, centre) is called when a sum is complete - for the neurons
-//   of dy = 0 between the FMAs of the last window rows, so that their activation functions (MUFU) run under them.
-//   NORMED: the same, but acc starts at negm (minus the mean of the tile) times the sum of the neuron's weights, and the
-//   bias is left to done. ADD: acc is added to, and done is not called.
+//   NORMED: acc starts at negm (minus the mean of the tile) times the sum of the neuron's weights, and done(n, o, scale, bias,
+//   centre), which adds the bias, is called when a sum is complete - for the neurons of dy = 0 between the FMAs of the last
+//   window rows, so that their activation functions (MUFU) run under them. ADD: acc is added to, and done is not called.
 //   rows[ry]: where window row ry of plane 0, column 0 starts; PLANE: cells from one plane to the next; dx: bytes from
 //   one column to the next.
 template <int PLANE, quad::Mode MODE, typename Done>
 __device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, unsigned tm, u64 (&acc)[4][4][2], const u64 (&negm)[2],
                                              Done done)
 {
-    constexpr bool FWD = MODE != quad::ADD, NORMED = MODE == quad::NORMED;
+    constexpr bool NORMED = MODE == quad::NORMED;
     float wb[2][12], sc[2][4], bi[2][4];
     auto finish = [&](int n, int o, float s, float b) {
         u64 c0, c1;
         lds128u(rows[1 + (n & 1)] + (unsigned)((1 + o) * dx) + (1 + (n >> 1)) * PLANE * 16u, c0, c1);
         done(n, o, s, b, c0, c1);
     };
-    if (FWD) {
+    if (NORMED) {
         float first[16];
-        tmem_ld16(tm + (NORMED ? quad::COL_WSUM : quad::COL_BIAS), first);
+        tmem_ld16(tm + quad::COL_WSUM, first);
         tmem_wait_ld16(first);
 #pragma unroll
         for (int n = 0; n < 4; ++n)
@@ -250,7 +249,7 @@ __device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, 
             for (int o = 0; o < 4; ++o) {
                 const u64 f2 = pack2(first[n * 4 + o], first[n * 4 + o]);
 #pragma unroll
-                for (int k = 0; k < 2; ++k) acc[n][o][k] = NORMED ? fmul2(f2, negm[k]) : f2;
+                for (int k = 0; k < 2; ++k) acc[n][o][k] = fmul2(f2, negm[k]);
             }
     }
     tmem_ld8(tm, wb[0]);
@@ -272,19 +271,19 @@ __device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, 
                 if (a < 0 || a > 2 || b < 0 || b > 2) continue;
                 float *wp = wb[use & 1];
                 tmem_wait_ld12(wp);
-                if (FWD && use == 30) tmem_use8(sc[0]);  // asked for before: that wait covered it
-                if (NORMED && use == 30) tmem_use8(bi[0]);
+                if (NORMED && use == 30) {  // asked for before: that wait covered it
+                    tmem_use8(sc[0]);
+                    tmem_use8(bi[0]);
+                }
                 if (use + 1 < 36) {
                     tmem_ld8(tm + (use + 1) * 12, wb[(use & 1) ^ 1]);
                     tmem_ld4(tm + (use + 1) * 12 + 8, wb[(use & 1) ^ 1] + 8);
                 }
-                if (FWD && use == 29) {
+                if (NORMED && use == 29) {
                     tmem_ld4(tm + quad::COL_SCALE, sc[0]);
                     tmem_ld4(tm + quad::COL_SCALE + 8, sc[1]);
-                    if (NORMED) {
-                        tmem_ld4(tm + quad::COL_BIAS, bi[0]);
-                        tmem_ld4(tm + quad::COL_BIAS + 8, bi[1]);
-                    }
+                    tmem_ld4(tm + quad::COL_BIAS, bi[0]);
+                    tmem_ld4(tm + quad::COL_BIAS + 8, bi[1]);
                 }
 #pragma unroll
                 for (int c = 0; c < 3; ++c)
@@ -295,24 +294,22 @@ __device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, 
                         ffma2(acc[n][o][1], v[o + c][1], ww);
                     }
                 ++use;
-                if (FWD && ry == 3)
+                if (NORMED && ry == 3)
 #pragma unroll
                     for (int e = (use - 30) * 8 / 6; fin < e; ++fin)
-                        finish((fin >> 2) * 2, fin & 3, sc[fin >> 2][fin & 3], NORMED ? bi[fin >> 2][fin & 3] : 0.0f);
+                        finish((fin >> 2) * 2, fin & 3, sc[fin >> 2][fin & 3], bi[fin >> 2][fin & 3]);
             }
         }
     }
-    if (FWD) {
+    if (NORMED) {
         tmem_ld4(tm + quad::COL_SCALE + 4, sc[0]);
         tmem_ld4(tm + quad::COL_SCALE + 12, sc[1]);
-        if (NORMED) {
-            tmem_ld4(tm + quad::COL_BIAS + 4, bi[0]);
-            tmem_ld4(tm + quad::COL_BIAS + 12, bi[1]);
-        }
+        tmem_ld4(tm + quad::COL_BIAS + 4, bi[0]);
+        tmem_ld4(tm + quad::COL_BIAS + 12, bi[1]);
         tmem_wait_ld8(sc[0]);
-        if (NORMED) tmem_use8(bi[0]);
+        tmem_use8(bi[0]);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) finish((e >> 2) * 2 + 1, e & 3, sc[e >> 2][e & 3], NORMED ? bi[e >> 2][e & 3] : 0.0f);
+        for (int e = 0; e < 8; ++e) finish((e >> 2) * 2 + 1, e & 3, sc[e >> 2][e & 3], bi[e >> 2][e & 3]);
     }
 }
 
@@ -329,62 +326,6 @@ __device__ __forceinline__ float quad_reduce8(const float (&v)[8], int lane)
     c += __shfl_xor_sync(0xffffffffu, c, 2);
     c += __shfl_xor_sync(0xffffffffu, c, 1);
     return c;
-}
-
-__device__ __forceinline__ void swap_if(bool c, u64 &a, u64 &b)
-{
-    const u64 t = c ? b : a;
-    b = c ? a : b;
-    a = t;
-}
-// The sum (j = 0) and the sum of squares (j = 1) of a region's values for the quad's samples s = 0 .. 3, in lane 4 j + s. As in
-// step_fast.cu the 128 values of two planes are added in float, in that kernel's order (four by four, then over z, y and
-// x), and the four pairs of planes in double: the statistics of a step are the same whichever kernel ran it.
-template <int SUB>
-__device__ __forceinline__ double quad_region_sums(const QuadLane<SUB> &L, const u64 (&v)[4][4][2], int lane)
-{
-    u64 s[2][2][2];  // [sum | squares][x pair, ascending][sample pair]
-#pragma unroll
-    for (int p = 0; p < 2; ++p)
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            u64 a[4], b[4];
-#pragma unroll
-            for (int n = 0; n < 4; ++n) {
-                u64 lo = v[n][2 * p][k], hi = v[n][2 * p + 1][k];
-                a[n] = fadd2(lo, hi);
-                swap_if(L.h, lo, hi);
-                b[n] = ffma2r(lo, lo, fmul2(hi, hi));
-            }
-            s[0][p][k] = fadd2(fadd2(a[0], a[1]), fadd2(a[2], a[3]));
-            s[1][p][k] = fadd2(fadd2(b[0], b[1]), fadd2(b[2], b[3]));
-        }
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int k = 0; k < 2; ++k) swap_if(L.h, s[j][0][k], s[j][1][k]);
-    // over y (rows two patches apart first, then neighbours) and the x halves; every level halves what a lane still holds
-    const bool my = lane & 4, e = lane & 2, h = lane & 1;
-    float f[2][2][4], a[2][4], b[2][2], c[2];
-#pragma unroll
-    for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int p = 0; p < 2; ++p) {
-            unpack2(s[j][p][0], f[j][p][0], f[j][p][1]);
-            unpack2(s[j][p][1], f[j][p][2], f[j][p][3]);
-        }
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-#pragma unroll
-        for (int i = 0; i < 4; ++i) a[p][i] = (my ? f[1][p][i] : f[0][p][i]) + __shfl_xor_sync(0xffffffffu, my ? f[0][p][i] : f[1][p][i], 6);
-#pragma unroll
-        for (int i = 0; i < 2; ++i) b[p][i] = (e ? a[p][i + 2] : a[p][i]) + __shfl_xor_sync(0xffffffffu, e ? a[p][i] : a[p][i + 2], 2);
-        c[p] = (h ? b[p][1] : b[p][0]) + __shfl_xor_sync(0xffffffffu, h ? b[p][0] : b[p][1], 1);
-    }
-    double d = (double)(c[0] + c[1]);
-    d += __shfl_xor_sync(0xffffffffu, d, 8);
-    d += __shfl_xor_sync(0xffffffffu, d, 16);
-    return d;
 }
 
 // Adds eight values over the lanes that share a tile (block 8: the warp, block 4: the four lanes of a sub-block); every

@@ -202,7 +202,7 @@ GN_API int gn_loop_forward_f32(const float *const *weights, const float *const *
         }
         const float *in = k ? outs[k - 1] : x_il4;
         QuadStep a{};
-        a.packed = w.packed; a.gbt = w.gbt; a.ordered = true;
+        a.packed = w.packed; a.gbt = w.gbt;
         a.in_il4 = in;
         a.out_il4 = residual ? w.tmp : outs[k];
         a.in_stats = residual ? mr + (size_t)k * S : (k ? mr + (size_t)(k - 1) * S : nullptr);
@@ -263,7 +263,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
         float *const h = kept ? stashes[k] : w.replay;
         if (!kept) {
             QuadStep a{};
-            a.packed = w.packed; a.gbt = w.gbt; a.ordered = true;
+            a.packed = w.packed; a.gbt = w.gbt;
             a.in_il4 = in; a.in_stats = in_stats;
             a.save_h = h;
             a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;

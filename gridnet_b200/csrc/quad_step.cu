@@ -121,7 +121,6 @@ int run_forward(const float *w, const float *b, const float *s, float *packed, c
     QuadStep a{};
     a.packed = packed; a.in_il4 = x_il4; a.out_il4 = y;
     if (d.normalize) a.wsum = wsum;
-    a.ordered = !d.normalize;
     a.eps = eps;
     if (k) {
         a.save_h = k->h;

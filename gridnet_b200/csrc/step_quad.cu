@@ -1,18 +1,19 @@
-// "Quad" kernels: float forward of the block-local update (block 8 and 4, per-block normalisation off) with the
-// weights in tensor memory and four samples per lane.
+// "Quad" kernels: float forward of the block-local update (block 8 and 4) with the weights in tensor memory and four
+// samples per lane. This file has the step with per-block normalisation and what all quad kernels share: re-ordering of
+// parameters and activations. step_taps.cu has the step without it.
 //
 // The register-patch kernel (step_fast.cu) keeps 108 weights per thread in registers and pays 2.25 FMAs per
 // shared-memory wavefront; the large-batch kernel (step_pair64.cu) fetches the weights from shared memory and pays
 // about 2.9. Here the weights do not touch the shared-memory data pipe at all: a warp handles a whole 8^3 region for
 // four samples, a lane owns a 2 x 2 x 4 (z, y, x) patch of neurons, and its 16 x 27 weights, biases and scales are
-// 464 of the 512 words that tensor memory has per lane. They are read back in steps of 24 words, a stencil step
+// 464 of the 512 words that tensor memory has per lane. They are read back in steps of 12 words, a stencil step
 // ahead, and each is used for the lane's four samples. A window is 4 x 4 x 6 cells for 16 neurons: 4.5 FMAs per
 // wavefront, the most that any split of an 8^3 region over 32 lanes gives.
 //
 //   * Layout ("IL4"): activations between the steps are interleaved by four samples, [B/4][M][N][K][4], so that a
 //     cell of a quad is one 128-bit access and FMAs are packed (fma.rn.f32x2) over sample pairs; a weight is the
 //     scalar operand of both.
-//   * A warp is on its own: its tile (10 x 10 x 10 cells, rows of 11) is read and written by no other warp, so the
+//   * A warp is on its own: its tile (10 x 10 x 10 cells) is read and written by no other warp, so the
 //     inner iterations need no barrier beyond __syncwarp, and new values go back into the tile in place.
 //   * Bank conflicts: none, see QuadLane in quad_geo.cuh.
 //   * Two warps (w, w + 4) share a quarter of tensor memory and therefore a region: they take its quads in turn. Each
@@ -22,9 +23,7 @@
 //   * Tiles arrive by bulk tensor copy (zero fill outside the grid) into three buffers per team (block 4: two), so a
 //     tile is under way while the two before it are worked on.
 //
-// Fusion as in step_fast.cu: FUSE_IN normalises the landed tile in place with the whole-grid statistics of the
-// previous step and a per-region (gamma, beta) table; every launch can reduce (sum, sum of squares) per sample and
-// region of what it writes. Reference semantics: gridnet/backend_torch.py:61-142; the kernel it stands in for is
+// Reference semantics: gridnet/backend_torch.py:61-142; the kernel it stands in for is
 // gridnet_cuda_forward_kernel, src/gridnet_cuda_kernels.cu:101-200.
 #include <string.h>
 
@@ -39,37 +38,31 @@ namespace gn {
 
 struct QuadParams {
     const float *packed;     // [regions][quad::PACK_F]
-    const float2 *gbt;       // FUSE_IN: (gamma, beta) per tile cell, [regions][CELLS], zero outside the grid
-    const float2 *in_stats;  // FUSE_IN: [4 Q] (mean, rstd)
-    double2 *out_partials;   // [4 Q][nparts]: slot `region` of every row is written; nullptr: not wanted
-    int nparts;
-    const float *wsum;       // NORM: the neurons' weight sums, [regions][4][32] vectors
-    float4 *tile_stats;      // NORM: [inner][Q][tiles][QS_COUNT]; nullptr: not wanted
+    const float *wsum;       // the neurons' weight sums, [regions][4][32] vectors
+    float4 *tile_stats;      // SAVE: [inner][Q][tiles][QS_COUNT]
     float eps;
     float *y;                // IL4; nullptr: not wanted (replay)
     float *save_h;           // SAVE: [inner][Q][P][4]
     int *error_flag;
     int M, N, K, Q, inner;
-    int params_old;          // the kernel before this one did not write packed or gbt
     long long nitems;        // regions * Q
 };
 
 // SAVE: keep every iteration's pre-activations for the backward pass (which gets the activations in between from them and
 // the step's input).
-// NORM: per-block normalisation (the reference's normalize=True, gridnet/backend_torch.py:92-97): the input of an
+// Per-block normalisation (the reference's normalize=True, gridnet/backend_torch.py:92-97): the input of an
 // iteration's sums is (tile - mean) / (std + eps) over all cells of the block's tile, the residual stays as it is. A tile
 // belongs to one warp, so the statistics need only shuffles. The landed tile is read once for its mean c and once more
 // to subtract it and to take the sums over its halo, which no iteration changes; from then on the tile holds v - c, so
 // that neither the variance nor sum w v - mean sum w cancels. Each iteration adds up the values it has just computed
 // while they are still in registers.
-template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM>
+template <int SUB, int ACT, bool SAVE>
 __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     step_fwd_quad(const __grid_constant__ CUtensorMap in_map, const QuadParams p)
 {
     using namespace quad;
     using G = QuadGeo<SUB>;
     constexpr int TEAM = G::TEAM, NBUF = G::NBUF;
-    constexpr bool GB_SMEM = FUSE_IN && SUB == 8;  // the (gamma, beta) table of the team's region is in shared memory
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) unsigned long long bars[QUARTERS * G::NBUF];
     __shared__ int issued[QUARTERS * G::NBUF];  // which item's copy into this buffer has been started last
@@ -86,28 +79,25 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();
     }
-    float2 *const gbs = reinterpret_cast<float2 *>(smem + QUARTERS * G::NBUF * G::BUF_BYTES) + quarter * G::CELLS;
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
     const unsigned tm = tmem_slot + ((unsigned)(quarter * 32) << 16);
-    static_assert(!(NORM && FUSE_IN), "per-block normalisation takes plain input");
 
     const QuadLane<SUB> L(lane);
-    // NORM: the lane's share of its tile's cells, first + STRIDE k; four lanes share a block-4 tile, and the first two
+    // The lane's share of its tile's cells, first + STRIDE k; four lanes share a block-4 tile, and the first two
     // bits of a quarter-warp's tiles are spread over the banks. Bit k of inside: cell k is no halo.
     constexpr int TILE_CELLS = SUB == 8 ? G::CELLS : 216, STRIDE = SUB == 8 ? 32 : 4, SHARE = (TILE_CELLS + STRIDE - 1) / STRIDE;
     const int my = L.ysgn < 0, turn = SUB == 8 ? 0 : 2 * (2 * my + L.h);
     const int first = SUB == 8 ? lane : ((lane >> 1) & 1) + ((lane >> 3) & 1) * 2 + turn;
     const unsigned tile_off = SUB == 8 ? 0u : (unsigned)(((L.z0 >> 2) * 2 + (L.y0 >> 2)) * 2 + L.h) * (TILE_CELLS * 16u);
     unsigned long long inside = 0;
-    if (NORM)
-        for (int k = 0; k < SHARE; ++k) {
-            int c = first + STRIDE * k;
-            if (SUB == 4 && c >= TILE_CELLS) c -= TILE_CELLS;
-            const int cx = c % G::SIDE, cy = c / G::SIDE % G::SIDE, cz = c / G::SIDE / G::SIDE;
-            if (cx > 0 && cx < G::SIDE - 1 && cy > 0 && cy < G::SIDE - 1 && cz > 0 && cz < G::SIDE - 1) inside |= 1ull << k;
-        }
+    for (int k = 0; k < SHARE; ++k) {
+        int c = first + STRIDE * k;
+        if (SUB == 4 && c >= TILE_CELLS) c -= TILE_CELLS;
+        const int cx = c % G::SIDE, cy = c / G::SIDE % G::SIDE, cz = c / G::SIDE / G::SIDE;
+        if (cx > 0 && cx < G::SIDE - 1 && cy > 0 && cy < G::SIDE - 1 && cz > 0 && cz < G::SIDE - 1) inside |= 1ull << k;
+    }
     const int nbx = p.K >> 3, nby = p.N >> 3;
     const size_t P = (size_t)p.M * p.N * p.K;
     const long long worker = (long long)blockIdx.x * QUARTERS + quarter, nworkers = (long long)gridDim.x * QUARTERS;
@@ -144,13 +134,10 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
         if (spins >= kSpinLimit || !mbar_wait_bounded(bar0 + 8 * (i % NBUF), (unsigned)(i / NBUF) & 1u, kSpinLimit)) failed = true;
         __syncwarp();
     };
-    auto begin = [&]() {
-        previous_done();
-        if (role == 0 && lane == 0)
-            for (int i = 0; i < NBUF && i < cnt; ++i) issue(i);
-        __syncwarp();
-    };
-    if (!p.params_old || cnt == 0) begin();  // else the first region's parameters come first
+    previous_done();
+    if (role == 0 && lane == 0)
+        for (int i = 0; i < NBUF && i < cnt; ++i) issue(i);
+    __syncwarp();
 
     int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
     for (int i0 = 0; i0 < cnt;) {
@@ -162,17 +149,9 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
             team_sync<TEAM>(quarter);  // the other warps no longer read the old region's weights
             tmem_fence_after();
         }
-        if (GB_SMEM) {
-            const unsigned char *src = reinterpret_cast<const unsigned char *>(p.gbt + (size_t)blk * G::CELLS);
-            const unsigned dst = smem_u32(gbs);
-            for (int c = role * 32 + lane; c < G::CELLS / 2; c += 32 * TEAM) cp_async16(dst + c * 16, src + c * 16);
-            __syncwarp();  // tensor memory instructions want the whole warp together
-        }
         quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm);
-        if (NORM && role == 0) quad_load_wsum(p.wsum, blk, lane, tm);
+        if (role == 0) quad_load_wsum(p.wsum, blk, lane, tm);
         tmem_wait_st();
-        if (GB_SMEM) cp_async_wait_all();
-        if (i0 == 0 && p.params_old) begin();
         tmem_fence_before();
         team_sync<TEAM>(quarter);
         tmem_fence_after();
@@ -186,47 +165,11 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
         for (int k = (role + TEAM - i0 % TEAM) % TEAM; k < here; k += TEAM) {
             const int i = i0 + k, q = q0 + k;
             const unsigned tile = tiles + (i % NBUF) * G::BUF_BYTES;
-            if (FUSE_IN) {
-                u64 na[2], nb[2];
-                {
-                    float2 mr[4];
-#pragma unroll
-                    for (int s = 0; s < 4; ++s) mr[s] = p.in_stats[4 * q + s];
-                    na[0] = pack2(mr[0].y, mr[1].y);
-                    na[1] = pack2(mr[2].y, mr[3].y);
-                    nb[0] = pack2(-mr[0].x, -mr[1].x);
-                    nb[1] = pack2(-mr[2].x, -mr[3].x);
-                }
-                wait_tile(i);
-                const float2 *gp = GB_SMEM ? gbs + lane : p.gbt + (size_t)blk * G::CELLS + lane;
-                constexpr int STEPS = (G::CELLS + 31) / 32;
-                constexpr int BATCH = SUB == 8 ? 16 : 18;  // loads of a batch are in flight together
-#pragma unroll 1
-                for (int c0 = 0; c0 < STEPS; c0 += BATCH) {
-                    const unsigned a = tile + (unsigned)(c0 * 32 + lane) * 16u;
-                    u64 v[BATCH][2];
-                    float2 g2[BATCH];
-#pragma unroll
-                    for (int c = 0; c < BATCH; ++c)
-                        if ((c0 + c) * 32 + lane < G::CELLS) {
-                            g2[c] = gp[(c0 + c) * 32];
-                            lds128u(a + c * 512, v[c][0], v[c][1]);
-                        }
-#pragma unroll
-                    for (int c = 0; c < BATCH; ++c)
-                        if ((c0 + c) * 32 + lane < G::CELLS) {
-                            const u64 gg = pack2(g2[c].x, g2[c].x), bb = pack2(g2[c].y, g2[c].y);
-                            sts128u(a + c * 512, ffma2r(fmul2(fadd2(v[c][0], nb[0]), na[0]), gg, bb), ffma2r(fmul2(fadd2(v[c][1], nb[1]), na[1]), gg, bb));
-                        }
-                }
-                __syncwarp();
-            } else {
-                wait_tile(i);
-            }
+            wait_tile(i);
 
-            u64 piv[2] = {0, 0}, negm[2], inv[2];
+            u64 piv[2], negm[2], inv[2];
             float halo[8], fresh[8];  // per sample: sum, sum of squares, relative to the pivot
-            if (NORM) {
+            {
                 const unsigned t0 = tile + tile_off;
                 constexpr int BATCH = SUB == 8 ? 16 : 18;
                 auto cell = [&](int k) {
@@ -294,7 +237,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
             for (int ry = 0; ry < 4; ++ry) rows[ry] = win + (unsigned)(ry * L.ysgn * G::ROW * 16);
             const size_t own = ((size_t)q * P + g0) * 4;  // the lane's cells in an IL4 tensor
             const long long zstr = wzs * 4, ystr = wys * 4;
-            // NORM: the sums over the lane's own cells -> over the tile's interior
+            // The sums over the lane's own cells -> over the tile's interior
             auto sum_fresh = [&](const u64 (&v)[4][4][2]) {
                 u64 s2[2] = {0, 0}, q2[2] = {0, 0};
 #pragma unroll
@@ -315,7 +258,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
             auto own_cell = [&](int n, int o) {
                 return win + (unsigned)((1 + o) * L.xsgn * 16 + (1 + (n & 1)) * L.ysgn * G::ROW * 16) + (1 + (n >> 1)) * G::PLANE * 16u;
             };
-            if (NORM) {
+            {
                 u64 v[4][4][2];
 #pragma unroll
                 for (int n = 0; n < 4; ++n)
@@ -325,7 +268,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
             }
             for (int t = 0; t < p.inner; ++t) {
                 const bool last = t + 1 == p.inner;
-                if (NORM) {
+                {
                     constexpr float per_cell = 1.0f / TILE_CELLS;
                     float m[4], sd[4], rs[4];
 #pragma unroll
@@ -355,11 +298,9 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                 }
                 u64 acc[4][4][2], hold[2] = {0, 0};
                 float *const sh = SAVE ? p.save_h + (size_t)t * p.Q * P * 4 + own : nullptr;
-                auto done = [&](int n, int o, float scale, float bias, u64 c0, u64 c1) {
-                    if (NORM) {
-                        acc[n][o][0] = ffma2r(acc[n][o][0], inv[0], pack2(bias, bias));
-                        acc[n][o][1] = ffma2r(acc[n][o][1], inv[1], pack2(bias, bias));
-                    }
+                quad_stencil<G::PLANE, NORMED>(rows, L.xsgn * 16, tm, acc, negm, [&](int n, int o, float scale, float bias, u64 c0, u64 c1) {
+                    acc[n][o][0] = ffma2r(acc[n][o][0], inv[0], pack2(bias, bias));
+                    acc[n][o][1] = ffma2r(acc[n][o][1], inv[1], pack2(bias, bias));
                     if (SAVE) {  // two neighbours at a time
                         if (o & 1)
                             stg256(sh + (n >> 1) * zstr + (n & 1) * ystr + 8 * ((o >> 1) ^ L.h), L.h ? acc[n][o][0] : hold[0],
@@ -369,32 +310,25 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                     }
                     acc[n][o][0] = act_residual2<ACT>(acc[n][o][0], scale, c0);
                     acc[n][o][1] = act_residual2<ACT>(acc[n][o][1], scale, c1);
-                };
-                quad_stencil<G::PLANE, NORM ? NORMED : BIAS>(rows, L.xsgn * 16, tm, acc, negm, done);
+                });
                 __syncwarp();  // every lane has read its window
                 if (!last) {
 #pragma unroll
                     for (int o = 0; o < 4; ++o)
 #pragma unroll
                         for (int n = 0; n < 4; ++n) sts128u(own_cell(n, o), acc[n][o][0], acc[n][o][1]);
-                    if (NORM) sum_fresh(acc);
+                    sum_fresh(acc);
                     __syncwarp();
                 } else {
                     if (lane == 0 && i + NBUF < cnt) issue(i + NBUF);  // the tile is dead: fetch the next one
                     __syncwarp();
-                    if (NORM)
 #pragma unroll
-                        for (int n = 0; n < 4; ++n)
+                    for (int n = 0; n < 4; ++n)
 #pragma unroll
-                            for (int o = 0; o < 4; ++o)
+                        for (int o = 0; o < 4; ++o)
 #pragma unroll
-                                for (int k2 = 0; k2 < 2; ++k2) acc[n][o][k2] = fadd2(acc[n][o][k2], piv[k2]);
+                            for (int k2 = 0; k2 < 2; ++k2) acc[n][o][k2] = fadd2(acc[n][o][k2], piv[k2]);
                     if (p.y) quad_store(p.y + own, zstr, ystr, L.h, acc);
-                    if (p.out_partials) {
-                        const double r = quad_region_sums(L, acc, lane);
-                        if (lane < 8) reinterpret_cast<double *>(p.out_partials + (size_t)(4 * q + (lane & 3)) * p.nparts + blk)[lane >> 2] = r;
-                        __syncwarp();
-                    }
                 }
             }
         }
@@ -691,13 +625,12 @@ int launch_quad_prepare(const QuadPrepare &a, int M, int N, int K, int block, cu
     return check_launch("quad_prepare");
 }
 
-template <int SUB, int ACT, bool FUSE_IN, bool SAVE, bool NORM>
+template <int SUB, int ACT, bool SAVE>
 static int launch_quad_one(const CUtensorMap &map, const QuadParams &p, unsigned ctas, cudaStream_t st)
 {
     using G = QuadGeo<SUB>;
-    auto kern = step_fwd_quad<SUB, ACT, FUSE_IN, SAVE, NORM>;
-    // tiles; block 8 with normalise-on-load also a (gamma, beta) table per team
-    constexpr int smem = quad::QUARTERS * G::NBUF * G::BUF_BYTES + (SUB == 8 && FUSE_IN ? quad::QUARTERS * G::CELLS * 8 : 0);
+    auto kern = step_fwd_quad<SUB, ACT, SAVE>;
+    constexpr int smem = quad::QUARTERS * G::NBUF * G::BUF_BYTES;
     static_assert(smem <= 232448 - 1024 - 256, "shared memory budget of one SM");
     static unsigned long long attr_set = 0;
     if (first_use_on_device(&attr_set)) {
@@ -714,8 +647,7 @@ static int launch_quad_one(const CUtensorMap &map, const QuadParams &p, unsigned
 template <int SUB, int ACT>
 static int launch_quad_act(const CUtensorMap &map, const QuadParams &p, unsigned ctas, cudaStream_t st)
 {
-    if (p.wsum) return p.save_h ? launch_quad_one<SUB, ACT, false, true, true>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, false, true>(map, p, ctas, st);
-    return p.in_stats ? launch_quad_one<SUB, ACT, true, false, false>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false, false, false>(map, p, ctas, st);
+    return p.save_h ? launch_quad_one<SUB, ACT, true>(map, p, ctas, st) : launch_quad_one<SUB, ACT, false>(map, p, ctas, st);
 }
 
 template <int SUB>
@@ -731,17 +663,14 @@ static int launch_quad_sub(const CUtensorMap &map, const QuadParams &p, unsigned
 
 int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
 {
-    if (a.wsum && (a.in_stats || a.ordered || !a.save_h != !a.tile_stats)) return GN_ERR_UNSUPPORTED;
-    if (a.ordered) return launch_step_fwd_taps(a, act, st);
-    if (!a.wsum && a.save_h) return GN_ERR_UNSUPPORTED;
+    if (!a.wsum) return launch_step_fwd_taps(a, act, st);
+    if (a.in_stats || a.out_partials || !a.save_h != !a.tile_stats) return GN_ERR_UNSUPPORTED;
     CUtensorMap map;
     memset(&map, 0, sizeof(map));
     const int rc = quad_make_map(&map, a.in_il4, a.M, a.N, a.K, a.Q, a.block);
     if (rc != GN_OK) return rc;
     QuadParams p{};
-    p.packed = a.packed; p.params_old = a.params_old;
-    p.gbt = a.gbt; p.in_stats = a.in_stats;
-    p.out_partials = a.out_partials; p.nparts = a.nparts;
+    p.packed = a.packed;
     p.wsum = a.wsum; p.tile_stats = a.tile_stats; p.eps = a.eps;
     p.y = a.out_il4; p.save_h = a.save_h;
     p.error_flag = a.error_flag ? a.error_flag : device_status_ptr();

@@ -1,11 +1,18 @@
 // Float forward of the block-local update on the quad layout (block 8 and 4, per-block normalisation off), weights in tensor
-// memory and four samples per lane as in step_quad.cu, every neuron's taps added in the order of their numbers: the same
+// memory and four samples per lane as described in step_quad.cu, every neuron's taps added in the order of their numbers: the same
 // bits as the register-patch kernel (step_fast.cu), statistics included. Loops with gradients need that: rounding that
 // differs is amplified from step to step (block 4, 8 x 16 iterations, silu: gradients up to 3e-5 apart in the 2-norm), and
 // where it carries a pre-activation over the kink of (leaky) relu gradients jump (40 x 56 x 72, 4 x 10 iterations: 1e-4).
 //
-// What differs from step_quad.cu is the split of a region over the lanes and the layout of the tile (taps_geo.cuh). Items,
-// teams, parameters in tensor memory, normalise-on-load and the overlap of launches are as described there.
+// What differs from step_quad.cu is the split of a region over the lanes and the layout of the tile (taps_geo.cuh), and two
+// buffers per team (a third does not fit beside the (gamma, beta) tables; with three and the tables read from L2 256^3 x 32 took
+// 110.7 ms instead of 96.6). Fusion as in step_fast.cu: FUSE_IN normalises the landed tile in place with the whole-grid
+// statistics of the previous step and a per-region (gamma, beta) table; every launch can reduce (sum, sum of squares) per
+// sample and region of what it writes.
+// Measured against the 2 x 2 x 4 patches of step_quad.cu, whose sums come in another order: a step of 64^3 x 16, two inner
+// iterations, with the pre-activations kept 36.9 us against 37.5; the inference loop 64^3 x 64, 4 x 12, 1649 us against
+// 1652; 256^3 x 32, 2 x 32, 97.2 ms against 98.4; 40 x 56 x 72 x 37, 3 x 6, 314 us against 299, where a warp has two or three
+// items and waits for each tile.
 // Block 8: tiles by bulk tensor copy. Block 4: each warp fetches its own next tile, cell by cell and asynchronously; its
 // eight small tiles have to lie an odd number of cells apart, which bulk tensor copies cannot do.
 #include <string.h>
