@@ -80,7 +80,7 @@ static int loop_check(int B, int M, int N, int K, int inner, int outer, int bloc
     if (inner < 1) return GN_ERR_BAD_INNER;
     if (act < GN_ACT_RELU || act > GN_ACT_TANH) return GN_ERR_BAD_ACTIVATION;
     if (nparams != 1 && nparams != outer) return GN_ERR_BAD_SHAPE;
-    if (!quad_applicable(M, N, K, block, inner) || (B + 3) / 4 > 65535) return GN_ERR_UNSUPPORTED;
+    if (!quad_applicable(M, N, K, block, inner)) return GN_ERR_UNSUPPORTED;
     return GN_OK;
 }
 

@@ -99,7 +99,7 @@ int step_check(int B, int M, int N, int K, int inner, int block, int act)
     if (block != 4 && block != 8) return GN_ERR_BAD_BLOCK;
     if (inner < 1) return GN_ERR_BAD_INNER;
     if (act < GN_ACT_RELU || act > GN_ACT_TANH) return GN_ERR_BAD_ACTIVATION;
-    if (!quad_applicable(M, N, K, block, inner) || (B + 3) / 4 > 65535) return GN_ERR_UNSUPPORTED;
+    if (!quad_applicable(M, N, K, block, inner)) return GN_ERR_UNSUPPORTED;
     return GN_OK;
 }
 

@@ -343,14 +343,15 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
 }
 
 // ---- layout conversion at the ends of a loop --------------------------------------------------------------
-// IL4 -> [B, P], normalised on the way when statistics are given
+// IL4 -> [B, P], normalised on the way when statistics are given. grid ceil(B / 4) * parts, one dimension: gridDim.y
+// ends at 65535
 __global__ void __launch_bounds__(256) from_il4_k(const float4 *il, const float2 *stats, const float *gamma, const float *beta,
-                                                  float *y, int B, size_t P)
+                                                  float *y, int B, size_t P, unsigned parts)
 {
-    const size_t c = (size_t)blockIdx.x * 256 + threadIdx.x;
+    const unsigned q = blockIdx.x / parts;
+    const size_t c = (size_t)(blockIdx.x - q * parts) * 256 + threadIdx.x;
     previous_done();
     if (c >= P) return;
-    const int q = blockIdx.y;
     const float4 v4 = il[(size_t)q * P + c];
     float v[4] = {v4.x, v4.y, v4.z, v4.w};
     float g = 1.0f, b = 0.0f;
@@ -595,8 +596,10 @@ int quad_make_map(CUtensorMap *map, const float *il, int M, int N, int K, int Q,
 int launch_from_il4(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, long long P,
                     cudaStream_t st)
 {
-    dim3 grid((unsigned)((P + 255) / 256), (unsigned)((B + 3) / 4));
-    launch_after(from_il4_k, grid, 256, 0, st, reinterpret_cast<const float4 *>(il), stats, gamma, beta, y, B, (size_t)P);
+    const unsigned parts = (unsigned)((P + 255) / 256);
+    const unsigned long long n = (unsigned long long)parts * ((B + 3) / 4);
+    if (n >= 1ull << 31) return GN_ERR_UNSUPPORTED;
+    launch_after(from_il4_k, (unsigned)n, 256, 0, st, reinterpret_cast<const float4 *>(il), stats, gamma, beta, y, B, (size_t)P, parts);
     return check_launch("from_il4");
 }
 

@@ -1119,11 +1119,11 @@ __global__ void __launch_bounds__(256) quad_norm_ac_k(const double2 *__restrict_
 // out = gu + rstd ((gn - gu) gamma - a - xhat c), gu = gradient of h'. out may be gu.
 __global__ void __launch_bounds__(256) quad_norm_residual_apply_k(const float4 *__restrict__ h, const float4 *__restrict__ gn, const float4 *gu,
                                                                   const float *__restrict__ gamma, const float2 *__restrict__ stats,
-                                                                  const float2 *__restrict__ ac, float4 *out, size_t P)
+                                                                  const float2 *__restrict__ ac, float4 *out, size_t P, unsigned parts)
 {
-    const size_t c = (size_t)blockIdx.x * 256 + threadIdx.x;
+    const unsigned q = blockIdx.x / parts;
+    const size_t c = (size_t)(blockIdx.x - q * parts) * 256 + threadIdx.x;
     if (c >= P) return;
-    const int q = blockIdx.y;
     const size_t i = (size_t)q * P + c;
     const float gm = gamma[c];
     const float4 hv = h[i], nv = gn[i], uv = gu[i];
@@ -1144,12 +1144,13 @@ __global__ void __launch_bounds__(256) quad_norm_residual_apply_k(const float4 *
 // neighbouring cells, and of the sums that four lanes then share each goes on with one sample's. P is a multiple of 512.
 __global__ void __launch_bounds__(256) quad_residual_combine_k(const float4 *__restrict__ h, const float4 *y, const float *__restrict__ gamma,
                                                                const float *__restrict__ beta, const float2 *__restrict__ stats, float4 *out,
-                                                               double2 *__restrict__ partials, int nparts, size_t P)
+                                                               double2 *__restrict__ partials, unsigned nparts, size_t P)
 {
     constexpr int CPT = 4;
     __shared__ double red[8][8];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, q = blockIdx.y;
-    const size_t c0 = (size_t)blockIdx.x * (256 * CPT) + tid;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned q = blockIdx.x / nparts, part = blockIdx.x - q * nparts;
+    const size_t c0 = (size_t)part * (256 * CPT) + tid;
     float2 mr[4];
     if (y) {
 #pragma unroll
@@ -1211,7 +1212,7 @@ __global__ void __launch_bounds__(256) quad_residual_combine_k(const float4 *__r
         double s = 0.0;
 #pragma unroll
         for (int w8 = 0; w8 < 8; ++w8) s += red[w8][tid];
-        reinterpret_cast<double *>(partials + (size_t)(4 * q + (tid & 3)) * nparts + blockIdx.x)[tid >> 2] = s;
+        reinterpret_cast<double *>(partials + (size_t)(4 * q + (tid & 3)) * nparts + part)[tid >> 2] = s;
     }
 }
 
@@ -1413,9 +1414,10 @@ int launch_quad_norm_sums(const float *x, const float *g, const float *sub, cons
 int launch_quad_norm_residual_apply(const float *h, const float *gn, const float *gu, const float *gamma, const float2 *stats, const float2 *ac,
                                     float *out, int Q, long long P, cudaStream_t st)
 {
-    dim3 grid((unsigned)((P + 255) / 256), (unsigned)Q);
-    quad_norm_residual_apply_k<<<grid, 256, 0, st>>>(reinterpret_cast<const float4 *>(h), reinterpret_cast<const float4 *>(gn),
-                                                     reinterpret_cast<const float4 *>(gu), gamma, stats, ac, reinterpret_cast<float4 *>(out), (size_t)P);
+    const unsigned parts = (unsigned)((P + 255) / 256);
+    if ((unsigned long long)parts * Q >= 1ull << 31) return GN_ERR_UNSUPPORTED;
+    quad_norm_residual_apply_k<<<parts * (unsigned)Q, 256, 0, st>>>(reinterpret_cast<const float4 *>(h), reinterpret_cast<const float4 *>(gn),
+                                                     reinterpret_cast<const float4 *>(gu), gamma, stats, ac, reinterpret_cast<float4 *>(out), (size_t)P, parts);
     return check_launch("quad_norm_residual_apply");
 }
 
@@ -1424,9 +1426,10 @@ int quad_combine_parts(long long P) { return (int)((P + 1023) / 1024); }
 int launch_quad_residual_combine(const float *h, const float *y, const float *gamma, const float *beta, const float2 *stats, float *out,
                                  double2 *partials, int Q, long long P, cudaStream_t st)
 {
-    dim3 grid((unsigned)quad_combine_parts(P), (unsigned)Q);
-    quad_residual_combine_k<<<grid, 256, 0, st>>>(reinterpret_cast<const float4 *>(h), reinterpret_cast<const float4 *>(y), gamma, beta, stats,
-                                                  reinterpret_cast<float4 *>(out), partials, quad_combine_parts(P), (size_t)P);
+    const unsigned parts = (unsigned)quad_combine_parts(P);
+    if ((unsigned long long)parts * Q >= 1ull << 31) return GN_ERR_UNSUPPORTED;
+    quad_residual_combine_k<<<parts * (unsigned)Q, 256, 0, st>>>(reinterpret_cast<const float4 *>(h), reinterpret_cast<const float4 *>(y), gamma, beta, stats,
+                                                  reinterpret_cast<float4 *>(out), partials, parts, (size_t)P);
     return check_launch("quad_residual_combine");
 }
 

@@ -501,3 +501,36 @@ def test_fused_step_sees_parameters_written_just_before(inner):
             t.copy_(source)
         fused_step(*params[:3], x, out, inner, 8, "silu", *params[3:], mr, partials)
         assert torch.equal(out, want)
+
+
+def test_batches_beyond_the_second_grid_dimension():
+    """262144 quads and more: one CTA row per quad in gridDim.y (at most 65535) would refuse batches above 262140. Inference and a
+    training step of the residual and the plain loop on a single block; samples from both ends against a batch of those alone."""
+    import gridnet_b200 as gb
+    from gridnet_b200._lib import lib
+
+    B, shape, inner, outer = 262149, (8, 8, 8), 1, 2
+    params = [dev(a) for a in model_params(51, shape)]
+    x = torch.randn(B, *shape, device="cuda", generator=torch.Generator(device="cuda").manual_seed(52))
+    idx = torch.tensor([0, 1, 131071, 262139, 262140, 262143, B - 1], device="cuda")
+    assert lib.gn_outer_forward_plan(B, *shape, inner, outer, 8) == 5
+    y = gb.outer_forward(*params, x, inner, outer, 8)
+    want = gb.outer_forward(*params, x[idx].contiguous(), inner, outer, 8)
+    assert torch.allclose(y[idx], want, rtol=1e-5, atol=1e-6)
+    del y
+    for form in ("plain", "residual"):
+        grads = []
+        for t in (x, x[idx].contiguous()):
+            leaves = [p.clone().requires_grad_(True) for p in params] + [t.detach().requires_grad_(True)]
+            assert gb.FusedLoopTrainOp.supported(leaves[0], leaves[5], inner, 8)
+            if form == "plain":
+                y = gb.FusedLoopTrainOp.apply(*leaves, inner, outer, 8, "silu", 1e-5)
+            else:
+                y = gb.FusedLoopResidualTrainOp.apply(*leaves[3:], inner, 8, "silu", 1e-5, outer, *leaves[:3])
+            grads.append(torch.autograd.grad(y, leaves[5], torch.ones_like(y))[0])
+        assert torch.allclose(grads[0][idx], grads[1], rtol=1e-4, atol=1e-5), form
+    one = torch.empty_like(x)
+    gb.gridnet_cuda.forward_kept(*params[:3], x, one, inner, 8, 1e-5, True, "silu")
+    two = torch.empty_like(x[idx])
+    gb.gridnet_cuda.forward_kept(*params[:3], x[idx].contiguous(), two, inner, 8, 1e-5, True, "silu")
+    assert torch.allclose(one[idx], two, rtol=1e-5, atol=1e-6)
