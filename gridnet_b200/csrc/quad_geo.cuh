@@ -314,9 +314,10 @@ __device__ __forceinline__ void quad_stencil(const unsigned (&rows)[4], int dx, 
 }
 
 // Adds eight values over the warp; afterwards lanes 4 j .. 4 j + 3 all hold the sum of value j.
-__device__ __forceinline__ float quad_reduce8(const float (&v)[8], int lane)
+template <typename T>
+__device__ __forceinline__ T quad_reduce8(const T (&v)[8], int lane)
 {
-    float a[4], b[2], c;
+    T a[4], b[2], c;
     const bool h16 = lane & 16, h8 = lane & 8, h4 = lane & 4;
 #pragma unroll
     for (int k = 0; k < 4; ++k) a[k] = (h16 ? v[k + 4] : v[k]) + __shfl_xor_sync(0xffffffffu, h16 ? v[k] : v[k + 4], 16);
@@ -329,19 +330,23 @@ __device__ __forceinline__ float quad_reduce8(const float (&v)[8], int lane)
 }
 
 // Adds eight values over the lanes that share a tile (block 8: the warp, block 4: the four lanes of a sub-block); every
-// lane gets all eight sums.
-template <int SUB>
-__device__ __forceinline__ void quad_tile_sum8(float (&v)[8], int lane)
+// lane gets all eight sums. T: what the lanes' values are added in.
+template <int SUB, typename T = float>
+__device__ __forceinline__ void quad_tile_sum8(float (&f)[8], int lane)
 {
-    if (SUB == 8) {
-        const float r = quad_reduce8(v, lane);
+    T v[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) v[k] = __shfl_sync(0xffffffffu, r, 4 * k);
+    for (int k = 0; k < 8; ++k) v[k] = (T)f[k];
+    if (SUB == 8) {
+        const float r = (float)quad_reduce8(v, lane);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) f[k] = __shfl_sync(0xffffffffu, r, 4 * k);
     } else {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
             v[k] += __shfl_xor_sync(0xffffffffu, v[k], 2);
             v[k] += __shfl_xor_sync(0xffffffffu, v[k], 8);
+            f[k] = (float)v[k];
         }
     }
 }

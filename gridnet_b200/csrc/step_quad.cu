@@ -198,9 +198,9 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                     unpack2(s2[1], halo[2], halo[3]);
                     unpack2(q2[0], halo[4], halo[5]);
                     unpack2(q2[1], halo[6], halo[7]);
-                    quad_tile_sum8<SUB>(halo, lane);
                 };
                 spread();
+                quad_tile_sum8<SUB>(halo, lane);  // any pivot near the mean will do
                 constexpr float per_cell = 1.0f / TILE_CELLS;
                 piv[0] = pack2(halo[0] * per_cell, halo[1] * per_cell);
                 piv[1] = pack2(halo[2] * per_cell, halo[3] * per_cell);
@@ -228,6 +228,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                         }
                 }
                 spread();
+                quad_tile_sum8<SUB, double>(halo, lane);  // enters every iteration
                 __syncwarp();
             }
 
@@ -238,7 +239,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
             const size_t own = ((size_t)q * P + g0) * 4;  // the lane's cells in an IL4 tensor
             const long long zstr = wzs * 4, ystr = wys * 4;
             // The sums over the lane's own cells -> over the tile's interior
-            auto sum_fresh = [&](const u64 (&v)[4][4][2]) {
+            auto sum_fresh = [&](const u64 (&v)[4][4][2], auto add) {
                 u64 s2[2] = {0, 0}, q2[2] = {0, 0};
 #pragma unroll
                 for (int n = 0; n < 4; ++n)
@@ -253,7 +254,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                 unpack2(s2[1], fresh[2], fresh[3]);
                 unpack2(q2[0], fresh[4], fresh[5]);
                 unpack2(q2[1], fresh[6], fresh[7]);
-                quad_tile_sum8<SUB>(fresh, lane);
+                quad_tile_sum8<SUB, decltype(add)>(fresh, lane);
             };
             auto own_cell = [&](int n, int o) {
                 return win + (unsigned)((1 + o) * L.xsgn * 16 + (1 + (n & 1)) * L.ysgn * G::ROW * 16) + (1 + (n >> 1)) * G::PLANE * 16u;
@@ -264,7 +265,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                 for (int n = 0; n < 4; ++n)
 #pragma unroll
                     for (int o = 0; o < 4; ++o) lds128u(own_cell(n, o), v[n][o][0], v[n][o][1]);
-                sum_fresh(v);
+                sum_fresh(v, 0.0);  // the step's input: added in double above the lane
             }
             for (int t = 0; t < p.inner; ++t) {
                 const bool last = t + 1 == p.inner;
@@ -275,9 +276,13 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                     for (int s = 0; s < 4; ++s) {
                         m[s] = (halo[s] + fresh[s]) * per_cell;
                         const float var = fmaxf(fmaf(-m[s], m[s], (halo[4 + s] + fresh[4 + s]) * per_cell), 0.0f);
-                        // approximate square root and reciprocal: a few ulp
-                        asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(sd[s]) : "f"(var));
-                        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rs[s]) : "f"(sd[s] + p.eps));
+                        if (SUB == 4) {  // as the kernel that blocks of 4 had before
+                            sd[s] = __fsqrt_rn(var);
+                            rs[s] = __frcp_rn(sd[s] + p.eps);
+                        } else {  // as step_fast.cu: approximate square root and reciprocal, a few ulp
+                            asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(sd[s]) : "f"(var));
+                            asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(rs[s]) : "f"(sd[s] + p.eps));
+                        }
                     }
                     negm[0] = pack2(-m[0], -m[1]);
                     negm[1] = pack2(-m[2], -m[3]);
@@ -317,7 +322,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                     for (int o = 0; o < 4; ++o)
 #pragma unroll
                         for (int n = 0; n < 4; ++n) sts128u(own_cell(n, o), acc[n][o][0], acc[n][o][1]);
-                    sum_fresh(acc);
+                    sum_fresh(acc, 0.0f);
                     __syncwarp();
                 } else {
                     if (lane == 0 && i + NBUF < cnt) issue(i + NBUF);  // the tile is dead: fetch the next one

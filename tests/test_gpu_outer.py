@@ -534,3 +534,25 @@ def test_batches_beyond_the_second_grid_dimension():
     two = torch.empty_like(x[idx])
     gb.gridnet_cuda.forward_kept(*params[:3], x[idx].contiguous(), two, inner, 8, 1e-5, True, "silu")
     assert torch.allclose(one[idx], two, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("offset", [100, 1000])
+@pytest.mark.parametrize("block,shape,inner", [(8, (16, 16, 24), 1), (8, (16, 16, 24), 4), (4, (16, 16, 8), 5)])
+def test_normalised_step_keeps_its_digits_with_a_large_offset(block, shape, inner, offset):
+    """Per-block normalisation where the mean is 100 and 1000 deviations away, on the kernels with the weights in tensor memory:
+    the output within two roundings of the float64 oracle (2-norm), gradients within eight."""
+    from gridnet_b200 import gridnet_cuda as gc
+
+    r = np.random.default_rng(7)
+    w = (r.standard_normal((27, *shape)) / np.sqrt(27)).astype(np.float32)
+    b, s = (0.1 * r.standard_normal(shape)).astype(np.float32), (1 + 0.1 * r.standard_normal(shape)).astype(np.float32)
+    x, gy = (offset + r.standard_normal((6, *shape))).astype(np.float32), r.standard_normal((6, *shape)).astype(np.float32)
+    args64 = [a.astype(np.float64) for a in (w, b, s, x)]
+    want = orc.step_forward(*args64, inner, block, 1e-5, True, "silu"), *orc.step_backward(*args64, gy.astype(np.float64), inner, block, 1e-5, True, "silu")
+    t = [dev(a) for a in (w, b, s, x)]
+    got = [torch.empty_like(t[3])] + [torch.empty_like(a) for a in t]
+    gc.forward_kept(*t, got[0], inner, block, 1e-5, True, "silu")
+    gc.backward_kept(*t, dev(gy), *got[1:], inner, block, 1e-5, True, "silu")
+    for a, ref, name, roundings in zip(got, want, ("y", "weight", "bias", "scale", "x"), (2, 8, 8, 8, 8)):
+        off = np.linalg.norm(a.cpu().numpy().astype(np.float64) - ref) / np.linalg.norm(ref)
+        assert off <= roundings * 2.0 ** -24, (name, off)
