@@ -523,8 +523,8 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                 for (int s = 0; s < 4; ++s) mr[s] = p.in_stats[4 * q + s];
                 na[0] = pack2(mr[0].y, mr[1].y);
                 na[1] = pack2(mr[2].y, mr[3].y);
-                nb[0] = pack2(-mr[0].x * mr[0].y, -mr[1].x * mr[1].y);
-                nb[1] = pack2(-mr[2].x * mr[2].y, -mr[3].x * mr[3].y);
+                nb[0] = pack2(-mr[0].x, -mr[1].x);
+                nb[1] = pack2(-mr[2].x, -mr[3].x);
             }
             constexpr int STEPS = (G::CELLS + THREADS - 1) / THREADS, BATCH = SUB == 8 ? 8 : 7;
 #pragma unroll 1
@@ -545,8 +545,8 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                     if (i < G::CELLS) {
                         if (FUSE_IN) {
                             const u64 gg = pack2(g2[c].x, g2[c].x), bb = pack2(g2[c].y, g2[c].y);
-                            v[c][0] = ffma2r(ffma2r(v[c][0], na[0], nb[0]), gg, bb);
-                            v[c][1] = ffma2r(ffma2r(v[c][1], na[1], nb[1]), gg, bb);
+                            v[c][0] = ffma2r(fmul2(fadd2(v[c][0], nb[0]), na[0]), gg, bb);
+                            v[c][1] = ffma2r(fmul2(fadd2(v[c][1], nb[1]), na[1]), gg, bb);
                             sts128u(tile + i * 16, v[c][0], v[c][1]);
                         }
                         if (NORM) {

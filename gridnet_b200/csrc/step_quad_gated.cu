@@ -165,8 +165,8 @@ __global__ void __launch_bounds__(256, 1) quad_gated_fwd_k(const __grid_constant
                     for (int s = 0; s < 4; ++s) mr[s] = p.in_stats[4 * q + s];
                     na[0] = pack2(mr[0].y, mr[1].y);
                     na[1] = pack2(mr[2].y, mr[3].y);
-                    nb[0] = pack2(-mr[0].x * mr[0].y, -mr[1].x * mr[1].y);
-                    nb[1] = pack2(-mr[2].x * mr[2].y, -mr[3].x * mr[3].y);
+                    nb[0] = pack2(-mr[0].x, -mr[1].x);
+                    nb[1] = pack2(-mr[2].x, -mr[3].x);
                 }
                 wait_tile(i);
                 u64 v[16][2];
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256, 1) quad_gated_fwd_k(const __grid_constant
                 for (int c = 0; c < 16; ++c)
                     if (c0 + c * 64 < G::CELLS) {
                         const u64 gg = pack2(g2[c].x, g2[c].x), bb = pack2(g2[c].y, g2[c].y);
-                        sts128u(tile + (c0 + c * 64) * 16, ffma2r(ffma2r(v[c][0], na[0], nb[0]), gg, bb), ffma2r(ffma2r(v[c][1], na[1], nb[1]), gg, bb));
+                        sts128u(tile + (c0 + c * 64) * 16, ffma2r(fmul2(fadd2(v[c][0], nb[0]), na[0]), gg, bb), ffma2r(fmul2(fadd2(v[c][1], nb[1]), na[1]), gg, bb));
                     }
                 pair_sync(pair);
             } else {
@@ -264,25 +264,27 @@ __global__ void __launch_bounds__(256, 1) quad_gated_fwd_k(const __grid_constant
 #pragma unroll
                         for (int j = 0; j < 2; ++j) quad_store2(to, r, j, zstr, ystr, L.h, x[r]);
                     if (p.out_partials) {
-                        u64 s2[2] = {0, 0}, q2[2] = {0, 0};
+                        // four x-neighbours in float, everything above in double, as norm_partial_stats_k (norm.cu)
+                        double v[8];
 #pragma unroll
-                        for (int r = 0; r < 2; ++r)
+                        for (int k2 = 0; k2 < 2; ++k2) {
+                            float f[2][2][2];  // [row][sum | squares][sample]
 #pragma unroll
-                            for (int o = 0; o < 4; ++o)
+                            for (int r = 0; r < 2; ++r) {
+                                u64 a[4];
 #pragma unroll
-                                for (int k2 = 0; k2 < 2; ++k2) {
-                                    s2[k2] = fadd2(s2[k2], x[r][o][k2]);
-                                    ffma2(q2[k2], x[r][o][k2], x[r][o][k2]);
-                                }
-                        float v[8];
-                        unpack2(s2[0], v[0], v[1]);
-                        unpack2(s2[1], v[2], v[3]);
-                        unpack2(q2[0], v[4], v[5]);
-                        unpack2(q2[1], v[6], v[7]);
-                        const float r = quad_reduce8(v, lane);
+                                for (int o = 0; o < 4; ++o) a[o] = x[r][L.h ? 3 - o : o][k2];
+                                unpack2(fadd2(fadd2(a[0], a[1]), fadd2(a[2], a[3])), f[r][0][0], f[r][0][1]);
+                                unpack2(fadd2(ffma2r(a[0], a[0], fmul2(a[1], a[1])), ffma2r(a[2], a[2], fmul2(a[3], a[3]))), f[r][1][0], f[r][1][1]);
+                            }
+#pragma unroll
+                            for (int j = 0; j < 2; ++j)
+#pragma unroll
+                                for (int i = 0; i < 2; ++i) v[4 * j + 2 * k2 + i] = (double)f[0][j][i] + (double)f[1][j][i];
+                        }
+                        const double r = quad_reduce8(v, lane);
                         if ((lane & 3) == 0)
-                            reinterpret_cast<double *>(p.out_partials + (size_t)(4 * q + ((lane >> 2) & 3)) * p.nparts + 2 * blk + branch)[lane >> 4] =
-                                (double)r;
+                            reinterpret_cast<double *>(p.out_partials + (size_t)(4 * q + ((lane >> 2) & 3)) * p.nparts + 2 * blk + branch)[lane >> 4] = r;
                     }
                     pair_sync(pair);  // the tile is dead
                     if (branch == 0 && lane == 0 && i + NBUF < cnt) issue(i + NBUF);

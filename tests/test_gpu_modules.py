@@ -353,3 +353,29 @@ def test_loops_with_gradients_give_the_bits_of_the_register_patch_kernels(block,
     gridnet_cuda.forward(*params, x, one, inner, block, 1e-5, False, act)
     gridnet_cuda.forward_kept(*params, x, two, inner, block, 1e-5, False, act)
     assert torch.equal(one, two)
+
+
+def test_gated_loop_takes_its_statistics_as_the_norm_op_does():
+    """Step outputs whose mean is 300 deviations from zero: the statistics that the gated loop's kernel takes from them are those
+    that the norm op's kernels take (floats of four values, doubles above), to a rounding of the result."""
+    import gridnet_b200 as gb
+    from gridnet_b200 import backend_cuda
+    from gridnet_b200._lib import check, lib
+
+    shape, batch = (16, 8, 24), 6
+    P = shape[0] * shape[1] * shape[2]
+    g = torch.Generator().manual_seed(3)
+    w = torch.zeros(27, 2, *shape, device="cuda")
+    b = torch.stack([300 + torch.randn(shape, generator=g), torch.randn(shape, generator=g)]).cuda()
+    x = (300 + torch.randn(batch, *shape, generator=g)).cuda()
+    gamma, beta = torch.ones(shape, device="cuda"), torch.zeros(shape, device="cuda")
+    _, (_, stats, outs, _) = backend_cuda._loop_forward([(w, b)], gamma, beta, x, 2, 1, 8, "silu", 1e-5, False, True, gated=True)
+    raw = outs[0].view(torch.float32).view(-1, P, 4).permute(0, 2, 1).reshape(-1, P)[:batch].contiguous()
+    got = stats.view(torch.float32).view(-1, 2)[:batch]
+    sums, want = torch.empty(batch, 2, dtype=torch.float64, device="cuda"), torch.empty(batch, 2, device="cuda")
+    ws = torch.empty(lib.gn_norm_workspace_bytes(batch, P), dtype=torch.uint8, device="cuda")
+    st = torch.cuda.current_stream().cuda_stream
+    check(lib.gn_norm_local_sums_f32(raw.data_ptr(), sums.data_ptr(), batch, P, ws.data_ptr(), ws.numel(), st))
+    check(lib.gn_norm_finalize_f32(sums.data_ptr(), 1, want.data_ptr(), batch, P, 1e-5, st))
+    assert raw.mean() / raw.std() > 200
+    assert torch.allclose(got, want, rtol=2.0 ** -22, atol=0), (got, want)
