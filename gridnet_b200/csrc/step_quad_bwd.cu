@@ -1023,8 +1023,8 @@ __global__ void __launch_bounds__(512, 2) quad_border4_k(const float *__restrict
 
 // ------------------------------------------------------------------------------------------ whole-grid norm
 // Gradient of y = (x - mean) rstd gamma + beta, first pass: per sample a = sum g gamma and c = sum g gamma xhat, and the
-// gradients of gamma and beta, which need no second look at the batch. A thread owns CPT cells and walks the quads; the
-// eight sums of a quad are added over the warp in float (32 CPT values), above that in double. SUB_G: the gradient is
+// gradients of gamma and beta, which need no second look at the batch. A thread owns CPT cells and walks the quads. The
+// eight sums of a quad are added in double from the single value on, as in norm_bwd_partial_k (norm.cu). SUB_G: the gradient is
 // g - sub (residual form of the loop).
 template <int CPT, bool SUB_G>
 __global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *__restrict__ x, const float4 *__restrict__ g,
@@ -1034,7 +1034,7 @@ __global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *__restrict
                                                         size_t P)
 {
     constexpr int QB = 16;  // quads between two block-wide sums
-    __shared__ float red[QB][8][8];
+    __shared__ double red[QB][8][8];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t c0 = (size_t)blockIdx.x * (256 * CPT) + tid;
     float gm[CPT], dg[CPT], db[CPT];
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *__restrict
                     }
                 }
             }
-            float v[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            double v[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
             float2 mr[4];
 #pragma unroll
             for (int s = 0; s < 4; ++s) mr[s] = __ldg(stats + 4 * q + s);
@@ -1071,20 +1071,20 @@ __global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *__restrict
 #pragma unroll
                 for (int s = 0; s < 4; ++s) {
                     const float xh = (xs[s] - mr[s].x) * mr[s].y, gg = gs[s] * gm[k];
-                    v[s] += gg;
-                    v[4 + s] = fmaf(gg, xh, v[4 + s]);
+                    v[s] += (double)gg;
+                    v[4 + s] += (double)(gg * xh);
                     dg[k] = fmaf(gs[s], xh, dg[k]);
                     db[k] += gs[s];
                 }
             }
-            const float r = quad_reduce8(v, lane);
+            const double r = quad_reduce8(v, lane);
             if ((lane & 3) == 0) red[q - qb][warp][lane >> 2] = r;
         }
         __syncthreads();
         for (int e = tid; e < (qe - qb) * 8; e += 256) {
             double s = 0.0;
 #pragma unroll
-            for (int w8 = 0; w8 < 8; ++w8) s += (double)red[e >> 3][w8][e & 7];
+            for (int w8 = 0; w8 < 8; ++w8) s += red[e >> 3][w8][e & 7];
             const int j = e & 7;  // value j: a of samples 0..3, then c
             reinterpret_cast<double *>(partials + (size_t)(4 * (qb + (e >> 3)) + (j & 3)) * nparts + blockIdx.x)[j >> 2] = s;
         }
