@@ -633,14 +633,18 @@ def outer_forward(weight, bias, residual_scale, norm_weight, norm_bias, init_act
     if workspace is None:
         ws = torch.empty(_outer_workspace_bytes(weight.device.index, B, M, N, K, block_size), dtype=torch.uint8, device=weight.device)
     else:
-        # A caller-owned workspace keeps the parameters re-ordered for the large-batch kernel between calls. They are
-        # rebuilt unless this very workspace tensor was used by the previous call with the same parameter tensors and
-        # neither they nor the workspace have been written to through torch since (torch counts in-place writes).
+        # A caller-owned workspace keeps the parameters re-ordered for the quad or the large-batch kernel between calls. They
+        # are rebuilt unless this very workspace tensor was used by the previous call with the same parameter tensors, by the
+        # same of these two kernels, and neither they nor the workspace have been written to through torch since (torch
+        # counts in-place writes).
         ws = workspace
-        params = (weight, bias, residual_scale, norm_weight, norm_bias)
-        key = (tuple((t.data_ptr(), t._version) for t in params), (B, M, N, K, int(block_size)))
-        if getattr(ws, "_gn_packed_for", None) == (key, ws._version):
-            flags = 1  # GN_OUTER_PARAMS_UNCHANGED
+        with torch.cuda.device(weight.device):
+            plan = int(lib.gn_outer_forward_plan(B, M, N, K, int(inner_iters), int(outer_iters), int(block_size)))
+        if plan in (2, 5):
+            params = (weight, bias, residual_scale, norm_weight, norm_bias)
+            key = (plan, tuple((t.data_ptr(), t._version) for t in params), (B, M, N, K, int(block_size)))
+            if getattr(ws, "_gn_packed_for", None) == (key, ws._version):
+                flags = 1  # GN_OUTER_PARAMS_UNCHANGED
     with torch.cuda.device(weight.device):
         check(lib.gn_outer_forward_flags_f32(weight.data_ptr(), bias.data_ptr(), residual_scale.data_ptr(),
                                              norm_weight.data_ptr(), norm_bias.data_ptr(),
@@ -649,7 +653,7 @@ def outer_forward(weight, bias, residual_scale, norm_weight, norm_bias, init_act
                                              activation_id(activation), ws.data_ptr(), ws.numel(), flags,
                                              gridnet_cuda._stream(weight)))
     if workspace is not None:
-        ws._gn_packed_for = (key, ws._version)
+        ws._gn_packed_for = None if key is None else (key, ws._version)
     return y
 
 

@@ -452,7 +452,8 @@ GN_API int gn_outer_forward_f32(const float *weight, const float *bias, const fl
                          float ln_eps, int activation, void *workspace,
                          size_t workspace_bytes, void *stream);
 /* gn_outer_forward_f32 with flags. GN_OUTER_PARAMS_UNCHANGED: the previous call with this workspace had the same
- * weight, bias, scale, gamma and beta (same values, same shape) and nothing else has written to the workspace
+ * weight, bias, scale, gamma and beta (same values, same shape), ran on the same kernel (gn_outer_forward_plan; 2 and 5 keep
+ * parameters, and a plan that says 2 or 5 holds whatever the alignment) and nothing else has written to the workspace
  * since, so the re-ordered copy of the parameters that the quad and large-batch kernels keep there is still good and is
  * not rebuilt (an inference server calls the loop many times between weight updates). */
 #define GN_OUTER_PARAMS_UNCHANGED 1

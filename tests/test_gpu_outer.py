@@ -556,3 +556,39 @@ def test_normalised_step_keeps_its_digits_with_a_large_offset(block, shape, inne
     for a, ref, name, roundings in zip(got, want, ("y", "weight", "bias", "scale", "x"), (2, 8, 8, 8, 8)):
         off = np.linalg.norm(a.cpu().numpy().astype(np.float64) - ref) / np.linalg.norm(ref)
         assert off <= roundings * 2.0 ** -24, (name, off)
+
+
+@pytest.mark.parametrize("shape,B,block", [((16, 16, 16), 64, 8), ((24, 8, 16), 9, 4)])
+def test_reused_workspace_follows_parameters_and_kernel(shape, B, block):
+    """The kernels that keep re-ordered parameters in a reused workspace: rebuilt when a parameter changes in place or is another
+    tensor, and when the call before ran on another kernel, which left none or others there."""
+    from gridnet_b200 import outer_forward, outer_forward_workspace
+    from gridnet_b200._lib import lib
+
+    inner, outer = 2, 2
+    w, b, s, gamma, beta = (dev(a) for a in model_params(71, shape))
+    x = dev(face_input(72, B, shape))
+    kernels = (4, 2) if block == 8 else (4,)
+    plan = {4: 5, 2: 2, 1: 1}
+
+    def run(kernel, *params, ws=None):
+        assert lib.gn_config_set(b"outer_kernel", kernel) == 0
+        assert lib.gn_outer_forward_plan(B, *shape, inner, outer, block) == plan[kernel]
+        return outer_forward(*params, x, inner, outer, block, workspace=ws)
+
+    try:
+        for kernel in kernels:
+            ws = outer_forward_workspace(B, shape, block, x.device)
+            ws.fill_(255)  # what is not written reads as NaN
+            for first in (1, kernel, *kernels, 1):  # what runs ahead of the call under test
+                run(first, w, b, s, gamma, beta, ws=ws)
+                got = run(kernel, w, b, s, gamma, beta, ws=ws)
+                assert torch.equal(got, run(kernel, w, b, s, gamma, beta)), (kernel, first)
+                with torch.no_grad():
+                    w.mul_(1.05)
+                changed = run(kernel, w, b, s, gamma, beta, ws=ws)
+                assert torch.equal(changed, run(kernel, w, b, s, gamma, beta)) and not torch.equal(changed, got), (kernel, first)
+                other = run(kernel, w, b, s, gamma * 0.5, beta, ws=ws)
+                assert torch.equal(other, run(kernel, w, b, s, gamma * 0.5, beta)), (kernel, first)
+    finally:
+        lib.gn_config_set(b"outer_kernel", 0)
