@@ -217,12 +217,13 @@ static OuterWs carve_outer(void *base, int B, int M, int N, int K, int block)
     off = align_up(off + sizeof(double2) * Bp * nb * 4, 256);
     w.stats = (float2 *)(p + off);
     off = align_up(off + sizeof(float2) * Bp, 256);
-    w.packed = (float *)(p + off);
-    if (pair) off = align_up(off + sizeof(float) * pair64_packed_floats(M, N, K), 256);
-    w.qpacked = (float *)(p + off);
+    // one call runs on one of the two kernels: their parameters share their place
+    w.packed = w.qpacked = (float *)(p + off);
+    const size_t pair_end = pair ? align_up(off + sizeof(float) * pair64_packed_floats(M, N, K), 256) : off;
     if (regions) off = align_up(off + sizeof(float) * quad_packed_floats(M, N, K), 256);
     w.gbt = (float2 *)(p + off);
     if (regions) off = align_up(off + sizeof(float2) * (size_t)(M / 8) * (N / 8) * (K / 8) * quad_tile_cells(block), 256);
+    if (off < pair_end) off = pair_end;
     w.error_flag = (int *)(p + off);
     off += 128;
     w.small_sums = (unsigned long long *)(p + off);

@@ -431,9 +431,9 @@ GN_API int gn_norm_apply_f32(const float *x, const float *gamma, const float *be
  * per-sample statistics of what it writes, and the next step applies
  * (x - mean) * rstd * gamma + beta while it loads its tiles; only the last
  * step's output is normalised by a separate kernel into y.
- * workspace: two [B rounded up to 64 (block 4: 4), M,N,K] float buffers, the statistics partials, the weights
- * re-ordered for the quad kernel (29/27 of the weight tensor) and for the large-batch kernel (block 8), and a
- * (gamma, beta) table.
+ * workspace: two [B rounded up to 64 (block 4: 4), M,N,K] float buffers, the statistics partials, and the
+ * weights re-ordered for the quad kernel (29/27 of the weight tensor) with a (gamma, beta) table, or in the same place for
+ * the large-batch kernel (block 8).
  * With the quad kernel the activations stay interleaved by four samples between steps, [quad][M][N][K][4]; with the
  * large-batch kernel (see gn_step_forward_pair64_f32 below) by groups of 64, [group][M][N][K][64]. */
 /* Which kernel gn_outer_forward_f32 would take for this problem with suitably aligned buffers: 3 = the whole loop

@@ -90,3 +90,14 @@ def test_no_fallback_when_library_is_missing(tmp_path, monkeypatch):
     with pytest.raises(ImportError):
         _lib._load()
     importlib.reload(_lib)
+
+
+def test_inference_workspace_holds_one_set_of_parameters():
+    """The loop's workspace: two activation buffers, and ONE re-ordered copy of the parameters, whichever kernel runs (a second one
+    would be 1.9 GB at 256^3)."""
+    from gridnet_b200._lib import lib
+
+    B, side = 64, 256
+    buffers = 2 * 4 * B * side ** 3
+    weights = 4 * 27 * side ** 3
+    assert lib.gn_outer_forward_workspace_bytes(B, side, side, side, 8) < buffers + 1.35 * weights
