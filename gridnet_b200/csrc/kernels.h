@@ -189,7 +189,6 @@ struct QuadReverse {
     const float *wsum;         // per-block normalisation: the forward pass's, and
     const float4 *tile_stats;  //   its statistics; nullptr: off
     float4 *hterm;             // with tile_stats: [Q][tiles][2]
-    int B;                     // samples that are real
     const float *h;            // [inner]
     float *delta, *dsum, *gx;  // [inner], one, one
     float *dsq;                // [Q][P]

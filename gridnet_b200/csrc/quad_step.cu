@@ -189,7 +189,6 @@ GN_API int gn_step_backward_kept_f32(const float *w, const float *b, const float
     if (normalize) {
         r.raw = k.y; r.wsum = k.wsum; r.tile_stats = k.stats; r.hterm = ws.hterm;
     }
-    r.B = B;
     r.delta = ws.delta; r.dsum = ws.dsum; r.gx = ws.gout; r.dsq = ws.dsq;
     r.M = M; r.N = N; r.K = K; r.Q = d.Q; r.inner = inner; r.block = block;
     TRY_(launch_quad_reverse(r, act, st));

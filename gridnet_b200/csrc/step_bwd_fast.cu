@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(bwd8::THREADS, 3) bwd_reverse8(const BwdParams
                 }
             if (NORM) {
                 const float p1 = ts.y * red_a * (1.0f / Geo::CELLS);
-                const float p2 = red_c * ts.y / ((float)Geo::CELLS * ts.z);
+                const float p2 = ts.z > 0.0f ? red_c * ts.y / ((float)Geo::CELLS * ts.z) : 0.0f;  // a constant tile: x - mean is zero
                 hF += fmaf(-p2, ts.x, p1);
                 hE += p2;
 #pragma unroll

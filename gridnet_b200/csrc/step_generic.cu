@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(BS *BS *BS)
                 for (int i = tid; i < T; i += NT) {
                     const int pi = Geo<BS>::pad(i);
                     R v = Gin[pi] * inv - sg * inv / R(T);
-                    v += dsd * (tile[pi] - mu) / (R(T) * sd);
+                    if (sd > R(0)) v += dsd * (tile[pi] - mu) / (R(T) * sd);  // a constant tile: nothing, not 0 / 0
                     G[pi] += v;
                     Gin[pi] = R(0);
                 }

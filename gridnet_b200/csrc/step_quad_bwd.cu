@@ -51,7 +51,6 @@ struct QuadRevParams {
     const float *wsum;             // BLOCK_NORM: as in step_fwd_quad
     const float4 *tile_stats;      // BLOCK_NORM: [inner][Q][tiles][QS_COUNT]
     float4 *hterm;                 // BLOCK_NORM: [Q][tiles][2] F, E
-    int B;
     const float *h;                // [inner] pre-activations, IL4
     float *delta, *dsum, *gx;      // [inner], one, one IL4 tensors
     float *dsq;                    // [Q][P] gradient terms of the residual scale, summed over the quad and the iterations
@@ -293,9 +292,9 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
                         float i0, i1, s0, s1;
                         unpack2(inv[j], i0, i1);
                         unpack2(sd[j], s0, s1);
-                        // samples that only fill up the quad have no deviation to divide by
-                        const float e0 = 4 * q + 2 * j < p.B ? -v[4 + 2 * j] * i0 / (s0 * (1.0f / PER_CELL)) : 0.0f;
-                        const float e1 = 4 * q + 2 * j + 1 < p.B ? -v[5 + 2 * j] * i1 / (s1 * (1.0f / PER_CELL)) : 0.0f;
+                        // a constant tile has no deviation to divide by, and nothing is as far from its mean as to need it
+                        const float e0 = s0 > 0.0f ? -v[4 + 2 * j] * i0 / (s0 * (1.0f / PER_CELL)) : 0.0f;
+                        const float e1 = s1 > 0.0f ? -v[5 + 2 * j] * i1 / (s1 * (1.0f / PER_CELL)) : 0.0f;
                         np2[j] = pack2(e0, e1);
                         const u64 p1 = pack2(v[2 * j] * i0 * -PER_CELL, v[2 * j + 1] * i1 * -PER_CELL);
                         np1[j] = ffma2r(fmul2(np2[j], pack2(-1.0f, -1.0f)), mean[j], p1);
@@ -1263,7 +1262,7 @@ int launch_quad_reverse(const QuadReverse &a, int act, cudaStream_t st)
 {
     QuadRevParams p{};
     p.packed = a.packed_t; p.g = a.g; p.raw = a.raw; p.stats = a.stats; p.ac = a.ac; p.h = a.h;
-    p.wsum = a.wsum; p.tile_stats = a.tile_stats; p.hterm = a.hterm; p.B = a.B;
+    p.wsum = a.wsum; p.tile_stats = a.tile_stats; p.hterm = a.hterm;
     p.delta = a.delta; p.dsum = a.dsum; p.gx = a.gx; p.dsq = a.dsq;
     p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;
     p.nitems = regions_of(a.M, a.N, a.K) * a.Q;

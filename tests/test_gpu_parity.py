@@ -634,3 +634,28 @@ def test_backward_on_a_raw_input_with_statistics(with_stash):
     assert lib.gn_step_backward_fused_in_f32(
         tw.data_ptr(), tb.data_ptr(), ts.data_ptr(), tx.data_ptr(), mr.data_ptr(), tga.data_ptr(), tbe.data_ptr(),
         tgy.data_ptr(), *(t.data_ptr() for t in g), B, M, N, K, inner, 4, 2, None, 0, ws.data_ptr(), ws.numel(), st) == -8
+
+
+@pytest.mark.parametrize("block,shape,dtype", [(8, (8, 16, 24), "float32"), (4, (8, 16, 8), "float32"), (8, (8, 8, 16), "float64")])
+def test_constant_tiles_have_finite_gradients(block, shape, dtype):
+    """Per-block normalisation of an input that is zero away from its first face, as a model's is: blocks whose tile is constant have no
+    deviation to divide by. Gradients as torch has them (that of a deviation of zero is zero), on every kernel of the step."""
+    from gridnet_b200 import gridnet_cuda as gc
+
+    r = np.random.default_rng(12)
+    f = np.dtype(dtype)
+    w, b, s = (r.standard_normal((27, *shape)) / np.sqrt(27)).astype(f), (0.1 * r.standard_normal(shape)).astype(f), np.ones(shape, f)
+    x, gy = np.zeros((5, *shape), f), r.standard_normal((5, *shape)).astype(f)
+    x[..., 0] = r.standard_normal(x.shape[:-1])
+    args64 = [a.astype(np.float64) for a in (w, b, s, x)]
+    want = orc.step_backward(*args64, gy.astype(np.float64), 2, block, 1e-2, True, "silu")
+    assert all(np.isfinite(a).all() for a in want)
+    t = [torch.from_numpy(a).cuda() for a in (w, b, s, x)]
+    ways = [gc.backward] + ([gc.backward_kept] if dtype == "float32" else [])
+    for way in ways:
+        got = [torch.empty_like(a) for a in t]
+        way(*t, torch.from_numpy(gy).cuda(), *got, 2, block, 1e-2, True, "silu")
+        for a, ref, name in zip(got, want, ("weight", "bias", "scale", "x")):
+            a = a.cpu().numpy().astype(np.float64)
+            # constant tiles: gradients are large (1 / eps) sums that cancel, so the bound is on the 2-norm
+            assert np.isfinite(a).all() and np.linalg.norm(a - ref) <= 1e-5 * np.linalg.norm(ref), (way.__name__, name)
