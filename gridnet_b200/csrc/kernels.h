@@ -137,7 +137,8 @@ int launch_from_il64(const float *il, const float2 *stats, const float *gamma, c
                      long long P, cudaStream_t st);
 
 // ---- step_quad.cu (weights in tensor memory, four samples per lane; activations in the IL4 layout [quad][z][y][x][4
-// samples], blocks of 8 and 4; B need not be a multiple of 4, the missing samples are zeros)
+// samples], blocks of 8 and 4; B need not be a multiple of 4: what fills up the last quad has the last sample's activations
+// and zero gradients)
 struct QuadStep {
     const float *packed;      // from launch_quad_prepare; without wsum in the order of the taps (QuadPrepare::ordered)
     const float2 *gbt;        // from launch_quad_prepare; used when in_stats is set
@@ -173,6 +174,7 @@ struct QuadPrepare {
     const float *x;
     float *il;                 // x [B, P] -> IL4
     int B;
+    bool gradient;             // samples that fill up the last quad: zeros; else copies of the last sample
 };
 int launch_quad_prepare(const QuadPrepare &a, int M, int N, int K, int block, cudaStream_t st);
 int launch_from_il4(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, long long P,

@@ -254,7 +254,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
             a.ordered = true;
             if (first) {
                 a.gamma = gamma; a.beta = beta; a.gbt = w.gbt;
-                a.x = gy; a.il = w.g[0]; a.B = B;
+                a.x = gy; a.il = w.g[0]; a.B = B; a.gradient = true;
             }
             TRY_(launch_quad_prepare(a, M, N, K, block, st));
         }
@@ -347,7 +347,7 @@ GN_API int gn_gated_loop_backward_f32(const float *weight, const float *bias, co
         a.w = weight; a.b = bias; a.s = weight; a.b_t = bias; a.gated = true; a.packed_t = w.packed_t;
         if (replay) a.packed = w.packed;
         a.gamma = gamma; a.beta = beta; a.gbt = w.gbt;
-        a.x = gy; a.il = w.g[0]; a.B = B;
+        a.x = gy; a.il = w.g[0]; a.B = B; a.gradient = true;
         TRY_(launch_quad_prepare(a, M, N, K, 8, st));
     }
     float *const delta_v = w.delta, *const delta_g = w.delta + inner * d.T4, *const dsum_v = w.dsum, *const dsum_g = w.dsum + d.T4;

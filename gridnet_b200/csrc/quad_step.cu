@@ -182,7 +182,7 @@ GN_API int gn_step_backward_kept_f32(const float *w, const float *b, const float
     cudaStream_t st = (cudaStream_t)stream;
     if (!kept) TRY_(run_forward(w, b, s, ws.packed, x, k.x, k.y, k.wsum, &k, eps, act, d, st));
     QuadPrepare a{};
-    a.w = w; a.b_t = b; a.s = s; a.packed_t = ws.packed_t; a.x = gy; a.il = ws.gin; a.B = B;
+    a.w = w; a.b_t = b; a.s = s; a.packed_t = ws.packed_t; a.x = gy; a.il = ws.gin; a.B = B; a.gradient = true;
     TRY_(launch_quad_prepare(a, M, N, K, block, st));
     QuadReverse r{};
     r.packed_t = ws.packed_t; r.g = ws.gin; r.h = k.h;

@@ -375,15 +375,16 @@ __global__ void __launch_bounds__(256) from_il4_k(const float4 *il, const float2
         }
 }
 
-// [B, P] -> [Q][P][4]; samples beyond B are zero. One cell per thread and step: four coalesced 4-byte reads, one
-// coalesced 16-byte write.
-__device__ __forceinline__ void to_il4(const float *__restrict__ x, float4 *__restrict__ il, int B, size_t P, int q, size_t part)
+// [B, P] -> [Q][P][4]. One cell per thread and step: four coalesced 4-byte reads, one coalesced 16-byte write. Samples
+// beyond B: zeros if these are gradients; activations are copies of sample B - 1. Zeros there could end in infinities or NaN where no
+// sample does (a constant block or grid and an eps of zero), and zero gradients do not keep those out of the parameters' sums.
+__device__ __forceinline__ void to_il4(const float *__restrict__ x, float4 *__restrict__ il, int B, size_t P, int q, size_t part, bool gradient)
 {
     const size_t c = part * 256 + threadIdx.x;
     if (c >= P) return;
     float v[4];
 #pragma unroll
-    for (int s = 0; s < 4; ++s) v[s] = 4 * q + s < B ? x[(size_t)(4 * q + s) * P + c] : 0.0f;
+    for (int s = 0; s < 4; ++s) v[s] = 4 * q + s < B || !gradient ? x[(size_t)min(4 * q + s, B - 1) * P + c] : 0.0f;
     il[(size_t)q * P + c] = make_float4(v[0], v[1], v[2], v[3]);
 }
 
@@ -562,7 +563,7 @@ __global__ void __launch_bounds__(256) quad_prepare_k(const PrepareArgs p)
     }
     else if (c < p.end[2]) quad_wsum<SUB>(a.w, reinterpret_cast<float4 *>(a.wsum), p.M, p.N, p.K, (int)(c - p.end[1]));
     else if (c < p.end[3]) quad_table<SUB>(a.gamma, a.beta, a.gbt, p.M, p.N, p.K, (int)(c - p.end[2]));
-    else to_il4(a.x, reinterpret_cast<float4 *>(a.il), a.B, P, (int)((c - p.end[3]) / p.parts), (c - p.end[3]) % p.parts);
+    else to_il4(a.x, reinterpret_cast<float4 *>(a.il), a.B, P, (int)((c - p.end[3]) / p.parts), (c - p.end[3]) % p.parts, a.gradient);
 }
 
 // ---- host side -----------------------------------------------------------------------------------------------

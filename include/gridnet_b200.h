@@ -485,7 +485,7 @@ GN_API int gn_step_backward_kept_f32(const float *weight, const float *bias, con
  * as one call forward and one backward. nparams = 1: one set of step parameters for all outer steps, or nparams =
  * outer: one per step (train_imagenet.py:54-58); weights, biases, scales are host arrays of nparams device pointers.
  *
- * Activations inside the loop are interleaved by four samples ("IL4": [ceil(B/4)][M][N][K][4], missing samples zero);
+ * Activations inside the loop are interleaved by four samples ("IL4": [ceil(B/4)][M][N][K][4], missing samples copies of the last one);
  * gn_loop_tensor_bytes is the size of one such tensor. The forward call fills, for the backward call:
  *   x_il4    the input, one tensor;
  *   outs     host array of `outer` device pointers, one tensor each: the step outputs before normalisation (residual: the

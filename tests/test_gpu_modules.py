@@ -379,3 +379,42 @@ def test_gated_loop_takes_its_statistics_as_the_norm_op_does():
     check(lib.gn_norm_finalize_f32(sums.data_ptr(), 1, want.data_ptr(), batch, P, 1e-5, st))
     assert raw.mean() / raw.std() > 200
     assert torch.allclose(got, want, rtol=2.0 ** -22, atol=0), (got, want)
+
+
+@pytest.mark.parametrize("batch", [1, 3, 4, 6])
+def test_samples_that_fill_up_a_quad_leave_no_trace(batch):
+    """The quad kernels work on four samples at a time. With an eps of zero a constant grid or block divides by zero; where no
+    sample of the batch is constant, what fills up the last quad must not be either."""
+    import gridnet_b200 as gb
+    from gridnet_b200 import gridnet_cuda as gc
+
+    g = torch.Generator().manual_seed(9)
+    shape, inner, outer = (8, 16, 8), 2, 2
+    mk = lambda *sz, scale=1.0, shift=0.0: (shift + scale * torch.randn(*sz, generator=g)).cuda()
+    w, b, s = mk(27, *shape, scale=27 ** -0.5), torch.zeros(shape, device="cuda"), torch.ones(shape, device="cuda")
+    gamma, beta, x, gy = mk(*shape, scale=0.1, shift=1.0), mk(*shape, scale=0.1), mk(batch, *shape), mk(batch, *shape)
+    w2, b2 = mk(27, 2, *shape, scale=27 ** -0.5), torch.zeros(2, *shape, device="cuda")
+
+    def plain(step):
+        def f(w, b, *rest):
+            *s, ga, be, h = rest
+            for _ in range(outer):
+                h = torch.nn.functional.layer_norm(step(w, b, *s, h), shape, ga, be, 0.0)
+            return h
+        return f
+
+    def check(f, ref, leaves):
+        a, c = ([t.clone().requires_grad_(True) for t in leaves] for _ in range(2))
+        got, want = torch.autograd.grad(f(*a), a, gy), torch.autograd.grad(ref(*c), c, gy)
+        for i, (p, q) in enumerate(zip(got, want)):
+            assert torch.isfinite(q).all() and torch.allclose(p, q, rtol=1e-3, atol=1e-4 * (1 + q.abs().max().item())), i
+
+    check(lambda *t: gb.FusedLoopTrainOp.apply(*t, inner, outer, 8, "silu", 0.0),
+          plain(lambda w, b, s, h: gb.GridnetCudaOp.apply(w, b, s, h, inner, 8, 1e-5, False, "silu")), (w, b, s, gamma, beta, x))
+    check(lambda *t: gb.FusedGatedLoopTrainOp.apply(*t, inner, outer, 8, "tanh", 0.0),
+          plain(lambda w, b, h: gb.GatedGridnetCudaOp.apply(w, b, h, inner, 8, "tanh")), (w2, b2, gamma, beta, x))
+    got, want = ([torch.empty_like(t) for t in (w, b, s, x)] for _ in range(2))
+    gc.backward_kept(w, b, s, x, gy, *got, inner, 8, 0.0, True, "silu")
+    gc.backward(w, b, s, x, gy, *want, inner, 8, 0.0, True, "silu")
+    for i, (p, q) in enumerate(zip(got, want)):
+        assert torch.isfinite(q).all() and torch.allclose(p, q, rtol=1e-3, atol=1e-4 * (1 + q.abs().max().item())), i
