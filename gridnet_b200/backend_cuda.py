@@ -16,7 +16,6 @@ from __future__ import annotations
 
 import ctypes
 import functools
-import threading
 
 import torch
 
@@ -46,48 +45,55 @@ _keep_forward_stash = None  # None: decide per call from the free device memory
 
 
 def keep_forward_stash(enabled):
-    """Trade memory for time in training: a :class:`GridnetCudaOp` forward that will be differentiated
-    (float32, per-block normalisation off, tuned path) can also keep every inner iteration's pre-activations
-    and intermediate activations, ``(2 * inner_iters - 1)`` extra activation tensors per call, so that its
-    backward skips recomputing them (about a quarter of the backward time; same gradient bits). The reference
-    always recomputes. ``True`` / ``False`` force the choice; ``None`` (the default) keeps them whenever they
-    take at most a tenth of the device memory that is free at that moment, and recomputes otherwise, call by
-    call; the fused training loop (:class:`FusedLoopTrainOp`) decides once per loop how many of its LAST outer
-    steps keep them: as many as fit into 70 % of the free memory. Returns the previous setting."""
+    """Trade memory for time in training: a forward pass of a step or a loop that will be differentiated (float32) can also keep
+    what its inner iterations computed, so that its backward skips computing that again (about a quarter of the backward time;
+    same gradient bits): of a step (:class:`GridnetCudaOp`) ``inner_iters`` to ``2 * inner_iters - 1`` extra activation tensors,
+    two and the statistics of the blocks more with per-block normalisation; of a loop ``inner_iters`` per outer step (gated:
+    three times that). The reference always recomputes. ``True`` / ``False`` force the choice; ``None`` (the default)
+    decides by memory. Steps keep it while all steps alive keep less than 2 GiB on the device together, and beyond that while it
+    is at most a tenth of the device memory that is free at that moment. The loops decide once per loop how many of their LAST
+    outer steps keep theirs: all where the loop holds less than a GiB, else as many as fit into 70 % of the free memory.
+    What cannot be allocated after all is recomputed. Returns the previous setting."""
     global _keep_forward_stash
     previous, _keep_forward_stash = _keep_forward_stash, (None if enabled is None else bool(enabled))
     return previous
 
 
-class _Kept:
-    """``nbytes`` of device memory that a step keeps for its backward pass. Knows how much all of them hold together, which
-    is what makes it unnecessary to ask the driver for the free memory (half a millisecond) before every small step."""
+def _free_bytes(device) -> int:
+    """Free memory of the device as a caller of torch sees it: what the caching allocator holds but has not handed out
+    counts. Asks the driver, half a millisecond."""
+    free, _ = torch.cuda.mem_get_info(device)
+    return free + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
 
-    _lock, _held = threading.Lock(), 0
+
+class _Kept:
+    """``nbytes`` of device memory that a step keeps for its backward pass. Knows how much all of them hold together on a
+    device, which is what makes it unnecessary to ask the driver for the free memory before every small step."""
+
+    # device index -> {id: bytes} of the objects alive. Single dict operations only, no lock: __del__ may run in the middle
+    # of __init__ of another one, on the same thread, when the garbage collector decides so
+    _alive = {}
+    UNASKED = 2 << 30
 
     def __init__(self, nbytes: int, device):
         self.buffer = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        self.nbytes = nbytes
-        with _Kept._lock:
-            _Kept._held += nbytes
+        self.alive = _Kept._alive.setdefault(self.buffer.device.index, {})
+        self.alive[id(self)] = nbytes
 
     def __del__(self):
-        if hasattr(self, "nbytes"):
-            with _Kept._lock:
-                _Kept._held -= self.nbytes
+        alive = getattr(self, "alive", None)
+        if alive is not None:
+            alive.pop(id(self), None)
 
     @staticmethod
     def room_for(need: int, device) -> bool:
-        """As :func:`keep_forward_stash` says; otherwise while all steps together keep less than 2 GiB, and beyond that while
-        ``need`` is at most a tenth of the free device memory."""
+        """As :func:`keep_forward_stash` says; otherwise while all steps together keep less than 2 GiB on the device, and
+        beyond that while ``need`` is at most a tenth of its free memory."""
         if _keep_forward_stash is not None:
             return _keep_forward_stash
-        if _Kept._held + need <= 2 << 30:
+        if sum(list(_Kept._alive.get(device.index, {}).values())) + need <= _Kept.UNASKED:
             return True
-        free, _ = torch.cuda.mem_get_info(device)
-        # what torch's caching allocator holds but has not handed out counts as free too
-        free += torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
-        return need * 10 <= free
+        return need * 10 <= _free_bytes(device)
 
 
 # Time of a step forward and backward in microseconds, measured over 16 x 32 x 24 .. 96^3 grids, batches of 2 to 128 and one to
@@ -280,10 +286,7 @@ def _kept_steps(nbytes_out: int, nbytes_stash: int, outer: int, device) -> int:
     per_step = nbytes_out + nbytes_stash
     if per_step * outer < _BIG:
         return outer
-    free, _ = torch.cuda.mem_get_info(device)
-    # what torch's caching allocator holds but has not handed out counts as free too
-    free += torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
-    return max(0, min(outer, int(0.7 * free) // per_step))
+    return max(0, min(outer, int(0.7 * _free_bytes(device)) // per_step))
 
 
 def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, block: int, activation: str, ln_eps: float,
@@ -312,12 +315,14 @@ def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, bloc
         stashes = [None] * outer
         if need_grad:
             stash_bytes = (3 if gated else 1) * inner * one
-            keep = _kept_steps(one, stash_bytes, outer, dev)
+            keep, keep_all = _kept_steps(one, stash_bytes, outer, dev), _keep_forward_stash is True
             total = (outer + 1) * one + stat + keep * stash_bytes
             if total < _BIG:  # one allocation, cut up
                 try:
                     pool = torch.empty(total, dtype=torch.uint8, device=dev)
                 except torch.cuda.OutOfMemoryError:
+                    if keep_all:
+                        raise
                     keep = 0
                     pool = torch.empty((outer + 1) * one + stat, dtype=torch.uint8, device=dev)
                 sizes = [stat] + [one] * (outer + 1) + [stash_bytes] * keep
@@ -330,11 +335,18 @@ def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, bloc
             else:
                 stats = torch.empty(stat, dtype=torch.uint8, device=dev)
                 x_il4 = _staggered(one, dev, 6)
-                outs = []
-                for k in range(outer):
-                    outs.append(_staggered(one, dev, k))
-                    if k >= outer - keep:
+                outs = [_staggered(one, dev, k) for k in range(outer)]
+                try:
+                    for k in reversed(range(outer - keep, outer)):  # the last ones first: where memory ends, the others go without
                         stashes[k] = _staggered(stash_bytes, dev, k + 3)
+                except torch.cuda.OutOfMemoryError:
+                    if keep_all:
+                        raise
+                    # what is left free is the backward pass's: give back what it takes to run iterations again
+                    for k in range(outer):
+                        if stashes[k] is not None:
+                            stashes[k] = None
+                            break
         else:
             stats = torch.empty(stat, dtype=torch.uint8, device=dev)
             x_il4 = torch.empty(one, dtype=torch.uint8, device=dev)

@@ -418,3 +418,57 @@ def test_samples_that_fill_up_a_quad_leave_no_trace(batch):
     gc.backward(w, b, s, x, gy, *want, inner, 8, 0.0, True, "silu")
     for i, (p, q) in enumerate(zip(got, want)):
         assert torch.isfinite(q).all() and torch.allclose(p, q, rtol=1e-3, atol=1e-4 * (1 + q.abs().max().item())), i
+
+
+def test_what_does_not_fit_is_recomputed(monkeypatch):
+    """The bookkeeping of kept iterations: per device, without a lock that a finaliser could meet held, and a loop that runs out of
+    memory while it allocates them goes on with those it has (allocation made to fail here; the gradients are the same bits)."""
+    import gc
+
+    import gridnet_b200 as gb
+    from gridnet_b200 import backend_cuda
+
+    kept = backend_cuda._Kept
+    device = torch.device("cuda", torch.cuda.current_device())
+    held = lambda: sum(kept._alive.get(device.index, {}).values())
+    base = held()
+    a, b = kept(1 << 20, device), kept(2 << 20, device)
+    assert held() == base + (3 << 20)
+    b.itself = b  # a cycle: its finaliser runs inside a collection, whenever that is
+    del b
+    gc.collect()
+    assert held() == base + (1 << 20)
+    monkeypatch.setattr(kept, "UNASKED", held() + 100)
+    assert kept.room_for(100, device)
+    monkeypatch.setattr(backend_cuda, "_free_bytes", lambda d: 5000)
+    assert kept.room_for(500, device) and not kept.room_for(501, device)
+    monkeypatch.setitem(kept._alive, device.index + 1, {1: 1 << 40})  # another device's does not count
+    assert kept.room_for(100, device)
+    del a
+
+    monkeypatch.undo()
+    g = torch.Generator().manual_seed(2)
+    shape, batch, inner, outer = (16, 8, 8), 5, 2, 4
+    mk = lambda *sz, scale=1.0: (scale * torch.randn(*sz, generator=g)).cuda()
+    leaves = [mk(27, *shape, scale=27 ** -0.5), mk(*shape, scale=0.1), mk(*shape), mk(*shape), mk(*shape), mk(batch, *shape)]
+    gy = mk(batch, *shape)
+
+    def grads():
+        t = [u.clone().requires_grad_(True) for u in leaves]
+        return torch.autograd.grad(gb.FusedLoopTrainOp.apply(*t, inner, outer, 8, "silu", 1e-5), t, gy)
+
+    want = grads()
+    monkeypatch.setattr(backend_cuda, "_BIG", 0)  # the path of loops that hold more than a GiB
+    real, calls = backend_cuda._staggered, []
+
+    def scarce(nbytes, dev, k):
+        calls.append(nbytes)
+        if len(calls) > 1 + outer + 2:  # the input, the outputs and two steps' iterations
+            raise torch.cuda.OutOfMemoryError("out of memory")
+        return real(nbytes, dev, k)
+
+    for f in (real, scarce):
+        monkeypatch.setattr(backend_cuda, "_staggered", f)
+        for u, v in zip(grads(), want):
+            assert torch.equal(u, v)
+    assert len(calls) == 1 + outer + 3
