@@ -125,7 +125,18 @@ def _quad_step(weight, x, inner_iters: int, block_size: int, normalize: bool):
     return gridnet_cuda.step_bytes(weight, x, inner_iters, block_size, normalize)
 
 
-class GridnetCudaOp(torch.autograd.Function):
+class _Op(torch.autograd.Function):
+    """An op that keeps things for its backward pass. Where gradients are off there is none, but a parameter still says that it
+    requires one (``ctx.needs_input_grad``), so it comes detached."""
+
+    @classmethod
+    def apply(cls, *args):
+        if not torch.is_grad_enabled():
+            args = [a.detach() if isinstance(a, torch.Tensor) else a for a in args]
+        return super().apply(*args)
+
+
+class GridnetCudaOp(_Op):
     """One outer-loop step of the plain gridnet (gridnet/backend_cuda.py:5-108)."""
 
     @staticmethod
@@ -413,7 +424,7 @@ def _restore_loop(ctx, nparams: int, outer: int):
     return params, (rest[0], rest[1], outs, [next(kept) if k else None for k in ctx.kept])
 
 
-class FusedLoopTrainOp(torch.autograd.Function):
+class FusedLoopTrainOp(_Op):
     """The model loop of the reference's scripts with gradients:
 
         h = x
@@ -457,7 +468,7 @@ class FusedLoopTrainOp(torch.autograd.Function):
         return (*grads[0], gg, gb, gx, None, None, None, None, None)
 
 
-class FusedGatedLoopTrainOp(torch.autograd.Function):
+class FusedGatedLoopTrainOp(_Op):
     """:class:`FusedLoopTrainOp` for the gated step (gridnet/scripts/train_mnist.py:36-44, 62-64), block 8:
 
         for _ in range(outer_iters):
@@ -492,7 +503,7 @@ class FusedGatedLoopTrainOp(torch.autograd.Function):
         return (*grads[0], gg, gb, gx, None, None, None, None, None)
 
 
-class FusedLoopSeparateTrainOp(torch.autograd.Function):
+class FusedLoopSeparateTrainOp(_Op):
     """:class:`FusedLoopTrainOp` for a loop in which every outer step has its own network
     (``separate_params`` of gridnet/scripts/train_imagenet.py:54-58,76-79): the same fused forward and the same
     reverse walk, each step's parameter gradients going to that step's parameters.
@@ -525,7 +536,7 @@ class FusedLoopSeparateTrainOp(torch.autograd.Function):
         return (gg, gb, gx, None, None, None, None) + tuple(t for triple in grads for t in triple)
 
 
-class FusedLoopResidualTrainOp(torch.autograd.Function):
+class FusedLoopResidualTrainOp(_Op):
     """The residual form of the model loop with gradients (gridnet/scripts/train_imagenet.py:81-83):
 
         for net in nets:  n = layer_norm(h);  h = h + (net(n) - n)
