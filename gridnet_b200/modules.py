@@ -97,9 +97,16 @@ class Readout(nn.Module):
         return self.proj(self.norm(x[:, :, :, -self.output_layers:].flatten(1)))
 
 
-def fused_gated_applies(network: nn.Module, h: torch.Tensor) -> bool:
-    """Whether a loop over a gated network runs as one call (:class:`FusedGatedLoopTrainOp`, with and without gradients)."""
-    return (isinstance(network, GatedGridnet) and h.dtype == torch.float32
+def _called_as_defined(module: nn.Module, cls: type) -> bool:
+    """Whether calling ``module`` is calling ``cls.forward`` and nothing else: no subclass's own, no hooks."""
+    return (type(module).forward is cls.forward and "forward" not in vars(module)
+            and not any((module._forward_hooks, module._forward_pre_hooks, module._backward_hooks, module._backward_pre_hooks)))
+
+
+def fused_gated_applies(network: nn.Module, norm: nn.Module, h: torch.Tensor) -> bool:
+    """Whether a loop over a gated network and a norm runs as one call (:class:`FusedGatedLoopTrainOp`, with and without
+    gradients), which does not call the modules: not where somebody listens to them or has redefined them."""
+    return (_called_as_defined(network, GatedGridnet) and _called_as_defined(norm, GridNorm) and h.dtype == torch.float32
             and FusedGatedLoopTrainOp.supported(network.weight, h, network.inner_iterations, network.block_size))
 
 
@@ -137,7 +144,7 @@ class GridnetModel(nn.Module):
             return FusedLoopTrainOp.apply(net.weight, net.bias, net.residual_scale, self.norm.weight, self.norm.bias, h,
                                           net.inner_iterations, self.outer_iters, net.block_size, net.activation,
                                           self.norm.eps)
-        if fused_gated_applies(net, h):
+        if fused_gated_applies(net, self.norm, h):
             return FusedGatedLoopTrainOp.apply(net.weight, net.bias, self.norm.weight, self.norm.bias, h, net.inner_iterations,
                                                self.outer_iters, net.block_size, net.activation, self.norm.eps)
         for _ in range(self.outer_iters):

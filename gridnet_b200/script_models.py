@@ -38,7 +38,7 @@ def _plain_loop(network: nn.Module, norm: GridNorm, h: torch.Tensor, outer_iters
         return FusedLoopTrainOp.apply(network.weight, network.bias, network.residual_scale, norm.weight, norm.bias, h,
                                       network.inner_iterations, outer_iters, network.block_size, network.activation,
                                       norm.eps)
-    if fused_gated_applies(network, h):
+    if fused_gated_applies(network, norm, h):
         return FusedGatedLoopTrainOp.apply(network.weight, network.bias, norm.weight, norm.bias, h, network.inner_iterations,
                                            outer_iters, network.block_size, network.activation, norm.eps)
     for _ in range(outer_iters):

@@ -500,3 +500,32 @@ def test_nothing_is_kept_where_gradients_are_off(kind):
     assert not y.requires_grad and torch.equal(y, want)
     # output, input and output of a step in the kernels' layout, parameters re-ordered
     assert torch.cuda.max_memory_allocated() - base < 5 * one + 3 * 4 * 54 * 32 ** 3, kind
+
+
+def test_gated_loop_calls_modules_that_are_listened_to():
+    """Forward hooks on the gated network or its norm, and a network with a forward of its own, see every outer step."""
+    import gridnet_b200 as gb
+
+    shape, outer = (8, 8, 16), 3
+    device = torch.device("cuda")
+    torch.manual_seed(4)
+    model = gb.GridnetModel(shape, 2, outer, 8, device, activation="tanh", gated=True)
+    x = torch.randn(5, *shape, device=device)
+    want = model(x)
+    for module in (model.network, model.norm):
+        seen = []
+        handle = module.register_forward_hook(lambda m, args, out: seen.append(out))
+        y = model(x)
+        handle.remove()
+        assert len(seen) == outer
+        assert torch.allclose(y, want, rtol=1e-4, atol=1e-5)
+
+    class Doubled(gb.GatedGridnet):
+        def forward(self, h):
+            return 2 * super().forward(h)
+
+    model.network.__class__ = Doubled
+    h = x
+    for _ in range(outer):
+        h = model.norm(model.network(h))
+    assert torch.equal(model(x), h)
