@@ -498,8 +498,8 @@ def test_nothing_is_kept_where_gradients_are_off(kind):
     with torch.no_grad():
         y = model(x)
     assert not y.requires_grad and torch.equal(y, want)
-    # output, input and output of a step in the kernels' layout, parameters re-ordered
-    assert torch.cuda.max_memory_allocated() - base < 5 * one + 3 * 4 * 54 * 32 ** 3, kind
+    # the output, input and outputs of a step in the kernels' layout, and at most 8.2 MB of parameters in another order
+    assert torch.cuda.max_memory_allocated() - base < 4 * one + 10e6, kind
 
 
 def test_gated_loop_calls_modules_that_are_listened_to():
