@@ -19,7 +19,7 @@ import functools
 
 import torch
 
-from . import gridnet_cuda
+from . import gridnet_cuda, patch_loop
 from ._lib import activation_id, check, lib
 
 
@@ -300,6 +300,49 @@ def _kept_steps(nbytes_out: int, nbytes_stash: int, outer: int, device) -> int:
     return max(0, min(outer, int(0.7 * _free_bytes(device)) // per_step))
 
 
+def _allocate_stashes(outer: int, keep: int, nbytes: int, device):
+    """Room for the iterations of the last ``keep`` of ``outer`` steps, None for the others."""
+    stashes = [None] * outer
+    try:
+        for k in reversed(range(outer - keep, outer)):  # the last ones first: where memory ends, the others go without
+            stashes[k] = _staggered(nbytes, device, k + 3)
+    except torch.cuda.OutOfMemoryError:
+        if _keep_forward_stash:
+            raise
+        # what is left free is the backward pass's: give back what it takes to run iterations again
+        for k in range(outer):
+            if stashes[k] is not None:
+                stashes[k] = None
+                break
+    return stashes
+
+
+def on_patches(B: int, M: int, N: int, K: int) -> bool:
+    """Whether a loop with gradients runs on the register-patch kernels (gated, one sample: as its steps and norms one by one).
+    The quad kernels compute, keep and walk back four samples whatever the batch. On small grids they are faster all the same
+    (one sample, 2 x 8 iterations: 64^3 0.71 ms against 2.9, 128^3 4.5 against 4.5); beyond 128^3 one sample, beyond twice that two
+    are better off with the other kernels, which also hold no more activations than there are. ms and GB, quad / patches: 160^3,
+    2 x 8, one sample 8.5, 4.1 / 7.8, 2.6, two 8.4 / 8.9; 256^3, 2 x 4, one 17.8, 13.5 / 14.7, 9.5, two 18.1, 13.8 / 17.0, 11.0,
+    three 17.9 / 19.8; blocks of 4, 4 x 4, one 24.5, 16.4 / 18.9, 10.6, two 24.4, 16.6 / 24.2, 13.2; gated 160^3, 2 x 4, one 8.1,
+    6.4 / 7.5, 3.1, two 8.1 / 8.9."""
+    return B <= 2 and M * N * K > B << 21
+
+
+def _patch_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, block: int, activation: str, ln_eps: float,
+                   residual: bool, need_grad: bool):
+    """:func:`_loop_forward` where :func:`on_patches`: x, outs and stashes are in the grid's own layout, x in float32."""
+    one, dev = x.numel() * 4, x.device
+    with torch.cuda.device(dev):
+        stash = patch_loop.stash_bytes(x, inner, block)
+        keep = _kept_steps(one, stash, outer, dev) if need_grad and stash else 0
+        stats = torch.empty(outer, x.shape[0], 2, dtype=torch.float32, device=dev)
+        outs = [_staggered(one, dev, k).view(torch.float32).view(x.shape) for k in range(outer if need_grad else min(2, outer))]
+        stashes = _allocate_stashes(outer, keep, stash, dev)
+        y = patch_loop.forward(plist, norm_weight, norm_bias, x, inner, outer, block, activation, ln_eps, residual,
+                               [outs[k % len(outs)] for k in range(outer)], stats, stashes)
+    return y, (x, stats, outs, stashes)
+
+
 def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, block: int, activation: str, ln_eps: float,
                   residual: bool, need_grad: bool, gated: bool = False):
     """The loop forward through ``gn_loop_forward_f32``; ``plist``: one (weight, bias, residual_scale) for all steps, or one
@@ -310,6 +353,9 @@ def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, bloc
         assert norm_weight.shape == params[1].shape[-3:] == norm_bias.shape, f"{norm_weight.shape=} invalid for {params[1].shape=}"
         _require_f32_cuda(**dict(zip(("weight", "bias", "residual_scale"), params)))
     _require_f32_cuda(norm_weight=norm_weight, norm_bias=norm_bias, x=x)
+    # the register-patch kernels read by bulk tensor copies and in pairs
+    if not gated and on_patches(B, M, N, K) and all(t.data_ptr() % 16 == 0 for t in (x, norm_weight, norm_bias, *(t for p in plist for t in p))):
+        return _patch_forward(plist, norm_weight, norm_bias, x, inner, outer, block, activation, ln_eps, residual, need_grad)
     dev = x.device
     one = int(lib.gn_loop_tensor_bytes(B, M, N, K))
     stat = outer * 4 * ((B + 3) // 4) * 8
@@ -326,13 +372,13 @@ def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, bloc
         stashes = [None] * outer
         if need_grad:
             stash_bytes = (3 if gated else 1) * inner * one
-            keep, keep_all = _kept_steps(one, stash_bytes, outer, dev), _keep_forward_stash is True
+            keep = _kept_steps(one, stash_bytes, outer, dev)
             total = (outer + 1) * one + stat + keep * stash_bytes
             if total < _BIG:  # one allocation, cut up
                 try:
                     pool = torch.empty(total, dtype=torch.uint8, device=dev)
                 except torch.cuda.OutOfMemoryError:
-                    if keep_all:
+                    if _keep_forward_stash:
                         raise
                     keep = 0
                     pool = torch.empty((outer + 1) * one + stat, dtype=torch.uint8, device=dev)
@@ -347,17 +393,7 @@ def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, bloc
                 stats = torch.empty(stat, dtype=torch.uint8, device=dev)
                 x_il4 = _staggered(one, dev, 6)
                 outs = [_staggered(one, dev, k) for k in range(outer)]
-                try:
-                    for k in reversed(range(outer - keep, outer)):  # the last ones first: where memory ends, the others go without
-                        stashes[k] = _staggered(stash_bytes, dev, k + 3)
-                except torch.cuda.OutOfMemoryError:
-                    if keep_all:
-                        raise
-                    # what is left free is the backward pass's: give back what it takes to run iterations again
-                    for k in range(outer):
-                        if stashes[k] is not None:
-                            stashes[k] = None
-                            break
+                stashes = _allocate_stashes(outer, keep, stash_bytes, dev)
         else:
             stats = torch.empty(stat, dtype=torch.uint8, device=dev)
             x_il4 = torch.empty(one, dtype=torch.uint8, device=dev)
@@ -387,6 +423,9 @@ def _loop_backward(plist, norm_weight, norm_bias, saved, grad_y, inner: int, out
     g = grad_y.contiguous()
     B, M, N, K = g.shape
     dev = g.device
+    if x_il4.dtype == torch.float32:  # _patch_forward
+        with torch.cuda.device(dev):
+            return patch_loop.backward(plist, norm_weight, norm_bias, x_il4, outs, stats, stashes, g, inner, outer, block, activation, residual)
     grads = [tuple(torch.empty_like(t) for t in params) for params in plist]
     gg, gb, gx = torch.empty_like(norm_weight), torch.empty_like(norm_bias), torch.empty_like(g)
     with torch.cuda.device(dev):
@@ -432,7 +471,8 @@ class FusedLoopTrainOp(_Op):
             h = layer_norm(gridnet_step(weight, bias, residual_scale, h, ..., normalize=False), norm_weight, norm_bias)
 
     (gridnet/scripts/train_mnist.py:62-64) as ONE autograd node, float32, shared parameters, on the quad kernels
-    (``gn_loop_forward_f32`` / ``gn_loop_backward_f32``): every step kernel reduces the statistics of what it writes and
+    (``gn_loop_forward_f32`` / ``gn_loop_backward_f32``) or, for one or two samples of a large grid, on the register-patch
+    kernels (:func:`on_patches`): every step kernel reduces the statistics of what it writes and
     normalises its input while loading it, so between steps only the RAW step outputs (and their statistics) exist and are
     saved - half the activations that the step-by-step composition saves. The last steps also keep their inner iterations
     for the backward pass, as many as the memory allows (:func:`keep_forward_stash`).
@@ -479,7 +519,8 @@ class FusedGatedLoopTrainOp(_Op):
 
     @staticmethod
     def supported(weight, x, inner_iters: int, block_size: int) -> bool:
-        return block_size == 8 and FusedLoopTrainOp.supported(weight, x, inner_iters, block_size)
+        return block_size == 8 and not (x.shape[0] == 1 and on_patches(*x.shape)) and FusedLoopTrainOp.supported(weight, x, inner_iters,
+                                                                                                                  block_size)
 
     @staticmethod
     def forward(ctx, weight, bias, norm_weight, norm_bias, x, inner_iters: int, outer_iters: int, block_size: int,

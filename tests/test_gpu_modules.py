@@ -529,3 +529,56 @@ def test_gated_loop_calls_modules_that_are_listened_to():
     for _ in range(outer):
         h = model.norm(model.network(h))
     assert torch.equal(model(x), h)
+
+
+@pytest.mark.parametrize("block,batch", [(8, 1), (8, 2), (4, 1)])
+def test_loops_on_patches_match_the_quad_kernels(block, batch, monkeypatch):
+    """Loops with gradients of one or two samples of a large grid run on the register-patch kernels: the same output bits, and
+    gradients, as on the quad kernels; plain, per-step parameters and residual; iterations kept and run again. On a small grid
+    that the rule is made to cover; an input that these kernels cannot read stays on the quad kernels."""
+    import gridnet_b200 as gb
+    from gridnet_b200 import backend_cuda
+
+    for n, first in ((1, (128, 128, 136)), (2, (128, 136, 256))):
+        assert backend_cuda.on_patches(n, *first) and not backend_cuda.on_patches(n, 128, 128, n * 128)
+    assert not backend_cuda.on_patches(3, 256, 256, 256)
+    g = torch.Generator().manual_seed(31)
+    shape, inner, outer = (16, 24, 8), 3, 3
+    mk = lambda *sz, scale=1.0, shift=0.0: (shift + scale * torch.randn(*sz, generator=g)).cuda()
+    plist = [(mk(27, *shape, scale=27 ** -0.5), mk(*shape, scale=0.1), mk(*shape, scale=0.1, shift=1.0)) for _ in range(outer)]
+    gamma, beta, x, gy = mk(*shape, scale=0.1, shift=1.0), mk(*shape, scale=0.1), mk(batch, *shape), mk(batch, *shape)
+
+    def run(form, keep, x=x):
+        ps = [tuple(t.clone().requires_grad_(True) for t in p) for p in (plist if form == "separate" else plist[:1])]
+        ga, be, xl = gamma.clone().requires_grad_(True), beta.clone().requires_grad_(True), x.detach().requires_grad_(True)
+        flat = [t for p in ps for t in p]
+        previous = gb.keep_forward_stash(keep)
+        try:
+            if form == "plain":
+                y = gb.FusedLoopTrainOp.apply(*flat, ga, be, xl, inner, outer, block, "silu", 1e-5)
+            elif form == "separate":
+                y = gb.FusedLoopSeparateTrainOp.apply(ga, be, xl, inner, block, "silu", 1e-5, *flat)
+            else:
+                y = gb.FusedLoopResidualTrainOp.apply(ga, be, xl, inner, block, "silu", 1e-5, outer, *flat)
+            return [y] + list(torch.autograd.grad(y, [ga, be, xl] + flat, gy))
+        finally:
+            gb.keep_forward_stash(previous)
+
+    def inference(form):
+        with torch.no_grad():
+            return gb.fused_loop_forward(plist if form == "separate" else plist[:1] * outer, gamma, beta, x, inner, block, "silu", 1e-5, form == "residual")
+
+    for form in ("plain", "separate", "residual"):
+        want = run(form, True)
+        assert torch.equal(inference(form), want[0])
+        with monkeypatch.context() as m:
+            m.setattr(backend_cuda, "on_patches", lambda *a: True)
+            for keep in (True, False):
+                got = run(form, keep)
+                assert torch.equal(got[0], want[0]), (form, keep)
+                for i, (a, c) in enumerate(zip(got[1:], want[1:])):
+                    assert torch.allclose(a, c, rtol=1e-3, atol=1e-5 * (1 + c.abs().max().item())), (form, keep, i)
+            assert torch.equal(inference(form), want[0])
+            shifted = torch.empty(x.numel() + 1, device="cuda")[1:].view(x.shape).copy_(x)
+            for a, c in zip(run(form, True, shifted), want):
+                assert torch.equal(a, c), form
