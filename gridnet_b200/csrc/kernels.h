@@ -136,7 +136,7 @@ int launch_to_il64(const float *x, float *il, int B, int G, long long P, cudaStr
 int launch_from_il64(const float *il, const float2 *stats, const float *gamma, const float *beta, float *y, int B, int G,
                      long long P, cudaStream_t st);
 
-// ---- step_quad.cu (weights in tensor memory, four samples per lane; activations in the IL4 layout [quad][z][y][x][4
+// ---- step_quad.cu, step_taps.cu (weights in tensor memory, four samples per lane; activations in the IL4 layout [quad][z][y][x][4
 // samples], blocks of 8 and 4; B need not be a multiple of 4: what fills up the last quad has the last sample's activations
 // and zero gradients)
 struct QuadStep {

@@ -20,7 +20,7 @@ enum Mode { ADD, NORMED };
 template <int SUB>
 struct QuadGeo;
 
-// TEAM: warps per quarter of tensor memory; NBUF: tile buffers per team. Block 8: the region is one block, its tile
+// TEAM: warps per quarter of tensor memory; NBUF: tile buffers per team of step_quad.cu. Block 8: the region is one block, its tile
 // 10 x 10 x 10 cells.
 template <>
 struct QuadGeo<8> {
@@ -178,7 +178,7 @@ __device__ __forceinline__ void team_sync(int quarter)
     asm volatile("bar.sync %0, %1;" ::"r"(quarter + 1), "n"(32 * TEAM) : "memory");
 }
 
-// Parameters of a region, packed in the order quad_stencil uses them (quad_pack_k): 116 vectors of four words per
+// Parameters of a region, packed in the order quad_stencil uses them (quad_pack; tap_stencil: tap_pack): 116 vectors of four words per
 // lane, lane-contiguous (512 bytes per vector and warp).
 namespace quad {
 constexpr int VECS = 116, PACK_F = VECS * 128;  // floats per region
@@ -209,7 +209,7 @@ __device__ __forceinline__ void quad_load_params(const float *packed, int role, 
     quad_move<29>(src + 29 * 32, tm + role * 232 + 116);
 }
 
-// the weight sums of per-block normalisation (quad_wsum_k), by one warp of the team
+// the weight sums of per-block normalisation (quad_wsum), by one warp of the team
 __device__ __forceinline__ void quad_load_wsum(const float *wsum, int region, int lane, unsigned tm)
 {
     const float4 *src = reinterpret_cast<const float4 *>(wsum) + (size_t)region * 128 + lane;

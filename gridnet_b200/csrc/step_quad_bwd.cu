@@ -1,4 +1,4 @@
-// Backward of the block-local update with the quad mapping (float, block 8 and 4, per-block normalisation off): the
+// Backward of the block-local update with the quad mapping (float, block 8 and 4, with and without per-block normalisation): the
 // decomposition of step_bwd_fast.cu on the layout and the work split of step_quad.cu.
 //
 //   reverse  quad_reverse_k: walks the inner iterations backwards. delta_t = act'(h_t) g s; what flows back inside a block
@@ -6,13 +6,13 @@
 //            whole-grid normalisation that follows the step is applied to g on the way in, so the normalised gradient
 //            never exists in memory.
 //   wgrad    quad_wgrad_k: dW[n][t] += x_t[n + o_t] delta_t[n], accumulated in registers over quads and iterations. Chunks of
-//            the batch leave their sums in parts of their own, which quad_unpack_grads_k adds up in chunk order: no
+//            the batch leave their sums in parts of their own, which quad_finish_k adds up in chunk order: no
 //            atomics, the same bits every time.
 //   border   quad_border_k: the part of grad_x that crosses block borders, from the per-neuron sums of deltas.
 //   norms    quad_norm_sums_k: one pass over the step's output and the gradient of its normalised form gives the
 //            per-sample sums of the LayerNorm gradient and the gradients of its weight and bias.
 //
-// Reference semantics: the gradient of gridnet/backend_torch.py:61-142 with normalize=False and of
+// Reference semantics: the gradient of gridnet/backend_torch.py:61-142 and of
 // torch.nn.LayerNorm((M,N,K)) (gridnet/scripts/train_mnist.py:54,62-64); the kernel this stands in for is
 // gridnet_cuda_backward_kernel, src/gridnet_cuda_kernels.cu:202-450.
 #include <string.h>
@@ -1271,7 +1271,7 @@ int launch_quad_reverse(const QuadReverse &a, int act, cudaStream_t st)
     return a.block == 8 ? launch_reverse_sub<8>(p, (unsigned)ctas, act, st) : launch_reverse_sub<4>(p, (unsigned)ctas, act, st);
 }
 
-// Into how many chunks the quads of a region go: as many as fill three CTAs per SM evenly. A chunk costs its CTA about
+// Into how many chunks the quads of a region go: as many as fill the two CTAs that an SM holds evenly. A chunk costs its CTA about
 // two quads' time (tile latency, sums out) and its part of the gradient, 59 KB, is written and added up once.
 static int wgrad_chunks(long long regions, int Q, int branches)
 {
