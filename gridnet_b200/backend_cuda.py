@@ -307,8 +307,6 @@ def _allocate_stashes(outer: int, keep: int, nbytes: int, device):
         for k in reversed(range(outer - keep, outer)):  # the last ones first: where memory ends, the others go without
             stashes[k] = _staggered(nbytes, device, k + 3)
     except torch.cuda.OutOfMemoryError:
-        if _keep_forward_stash:
-            raise
         # what is left free is the backward pass's: give back what it takes to run iterations again
         for k in range(outer):
             if stashes[k] is not None:
@@ -378,8 +376,6 @@ def _loop_forward(plist, norm_weight, norm_bias, x, inner: int, outer: int, bloc
                 try:
                     pool = torch.empty(total, dtype=torch.uint8, device=dev)
                 except torch.cuda.OutOfMemoryError:
-                    if _keep_forward_stash:
-                        raise
                     keep = 0
                     pool = torch.empty((outer + 1) * one + stat, dtype=torch.uint8, device=dev)
                 sizes = [stat] + [one] * (outer + 1) + [stash_bytes] * keep
