@@ -12,7 +12,8 @@
 // What an outer step costs at this size is the way of its results to the other CTAs, and fences and flags are the longest part
 // of it (a fence by the writer is 0.7 us here, an acquire by the reader 2.5). So there are none: every 64-bit word that a CTA
 // leaves for another carries the number of the step, a cell as (value, step), a block's sum and sum of squares as doubles
-// whose low eight bits hold it, and the reader looks at the word until the step is right. A further warp per sample publishes
+// whose low eight bits hold it (44 bits are left, twenty more than the added values have), and the reader looks at the word
+// until the step is right. A further warp per sample publishes
 // the block's sums and watches for those of the other blocks of that sample; while it does, the other four warps work on
 // the CTA's other sample. All CTAs of a sample add the same sums in the same order, hence get the same bits. The words
 // are zeroed before the launch (step numbers start at 1), and steps alternate between two sets of them: a block can be at
