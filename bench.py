@@ -57,7 +57,7 @@ FALLBACK_HBM_GBS = 6650.0
 # DRAM bytes per launch of the dominant kernel (dram__bytes_read.sum + dram__bytes_write.sum): a constant taken
 # from the ncu capture summarised in the named file, not a measurement of this run
 NCU_TRAFFIC = {
-    "step_fwd_quad": (178.2e6, "profiles/step_fwd_quad_c2_ncu_sections.txt"),
+    "step_fwd_taps": (180.7e6, "profiles/step_fwd_taps_c2_ncu_sections.txt"),
     "step_fwd_fast8": (173.0e6, "profiles/step_fwd_fast8_c2_ncu_full.txt"),
 }
 
@@ -358,7 +358,7 @@ def bench_c2(ctx: Ctx):
     if quad:
         # the step kernel has no entry point of its own: what one outer step more costs a loop (step kernel and the
         # statistics of its output), from loops of 2 and of OUTER steps
-        kernel_name = "step_fwd_quad<silu, fuse_in> (with the finalize of its statistics)"
+        kernel_name = "step_fwd_taps<silu, fuse_in> (with the finalize of its statistics)"
         reps = max(args.steps, 3)
 
         def loop(i, outer):
@@ -404,7 +404,7 @@ def bench_c2(ctx: Ctx):
     ach_gbs = algorithmic_bytes_per_launch(BATCH) / (kms * 1e-3) / 1e9
     fp32_nominal = FP32_LANES * 2 * sm_max_mhz * 1e6 / 1e12
     ach_tflops = 2 * algorithmic_fma_per_launch(BATCH) / (kms * 1e-3) / 1e12
-    traffic, traffic_src = NCU_TRAFFIC["step_fwd_quad" if quad else "step_fwd_fast8"]
+    traffic, traffic_src = NCU_TRAFFIC["step_fwd_taps" if quad else "step_fwd_fast8"]
     fp32 = {"bound": "fp32", "achieved": ach_tflops, "peak": fp32_measured, "unit": "TFLOP/s",
             "frac": ach_tflops / fp32_measured,
             "peak_source": "measured in this run: FFMA-only kernel on every SM, CUDA events (gn_probe_fp32_fma)",
@@ -505,7 +505,7 @@ def bench_c2(ctx: Ctx):
         "config": {"workload": WORKLOAD, "global_batch": BATCH * world, "parallelism": f"batch-sharded x{world}",
                    "l2": f"{NSETS} rotating input/output sets (4 x 67 MB each way) plus a 300 MB working set per step, larger than the 126 MB L2",
                    "samples_per_sec": BATCH * world * args.steps / (ms * 1e-3),
-                   "step_kernel": "weights in tensor memory (step_quad.cu)" if quad else "register-patch (step_fast.cu)",
+                   "step_kernel": "weights in tensor memory (step_taps.cu)" if quad else "register-patch (step_fast.cu)",
                    "device_failure_flag": failed},
         "roofline": roofline, "e2e": e2e, "cpu_baseline": cpu,
         "gpu_launches": launches_per_step * args.steps, "clocks": clocks,
@@ -875,7 +875,7 @@ def bench_train(ctx: Ctx, name: str, stash=None, microbatches=None, steps_cap: i
                                  "peak_source": hbm_src + " (MEASURED_PEAKS.json hbm_gbs)" if hbm_src == "measured"
                                  else "fallback"},
                          "traffic": None,
-                         "traffic_source": "not captured for the training step (many kernels; see profiles/train_step_c3_launch_list.txt for their shares)"},
+                         "traffic_source": "not captured for the training step (many kernels; see profiles/train_step_kernels.txt for their shares)"},
             "clocks": clocks,
         })
     gb.keep_forward_stash(previous_stash)

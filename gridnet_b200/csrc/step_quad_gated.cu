@@ -11,7 +11,8 @@
 // two pairs that share a region take its quads in turn, one's exchange under the other's sums.
 //
 // Bound by the shared-memory pipe like the plain kernel (4.5 FMAs per wavefront of the window). At 32^3, two inner
-// iterations, batch 64: forward 34 us with what the backward pass needs written out (register-patch kernel: 38), reverse sweep 53 us (57).
+// iterations, batch 64: forward 38 us with what the backward pass needs written out and statistics in double above four values (34 with
+// floats of 256; register-patch kernel: 38), reverse sweep 53 us (57).
 #include <string.h>
 
 #include "common.cuh"
