@@ -940,7 +940,8 @@ GN_API int gn_outer_forward_plan(int B, int M, int N, int K, int inner, int oute
     if (B <= 0 || M <= 0 || N <= 0 || K <= 0 || inner < 1 || outer < 1 || (block != 4 && block != 8)) return 0;
     alignas(16) static const double aligned[2] = {0.0, 0.0};  // any 16-byte aligned address: only alignment is looked at
     const void *a = aligned;
-    if ((g_outer_kernel == 0 || g_outer_kernel == 3) && outer_small_spc(B, M, N, K, block, inner, outer, a, a, a, a, a, a, a) > 0)
+    if ((g_outer_kernel == 0 || g_outer_kernel == 3) && (outer_small_spc(B, M, N, K, block, inner, outer, a, a, a, a, a, a, a) > 0 ||
+                                                         outer_held_spc(B, M, N, K, block, inner, outer, a, a, a, a, a, a, a) > 0))
         return 3;
     if (g_outer_kernel == 3) return 0;
     if (((g_outer_kernel == 0 && quad_wanted(B, M, N, K)) || g_outer_kernel == 4) && quad_applicable(M, N, K, block, inner)) return 5;
@@ -1014,12 +1015,16 @@ static int outer_forward_impl(const float *w, const float *b, const float *s, co
 
     if (g_outer_kernel == 0 || g_outer_kernel == 3) {
         const int spc = outer_small_spc(B, M, N, K, block, inner, outer, w, b, s, gamma, beta, x, y);
-        if (spc > 0) {
+        const int held = spc > 0 ? 0 : outer_held_spc(B, M, N, K, block, inner, outer, w, b, s, gamma, beta, x, y);
+        if (spc > 0 || held > 0) {
             const cudaError_t e = cudaMemsetAsync(ws.error_flag, 0, 128 + ws.small_bytes, st);
             if (e != cudaSuccess) {
                 record_cuda_error(e, "cudaMemsetAsync");
                 return GN_ERR_CUDA;
             }
+            if (held > 0)
+                return launch_outer_held(w, b, s, gamma, beta, x, y, ws.small_cells, ws.small_sums, ws.error_flag, B, M, N, K, inner, outer, held,
+                                         ln_eps, act, st);
             return launch_outer_small(w, b, s, gamma, beta, x, y, ws.small_cells, ws.small_sums, ws.error_flag, B, M, N, K,
                                       inner, outer, spc, ln_eps, act, st);
         }

@@ -281,6 +281,13 @@ int launch_outer_small(const float *w, const float *b, const float *s, const flo
                        float *y, unsigned long long *cells, unsigned long long *sums, int *error_flag, int B, int M, int N, int K,
                        int inner, int outer, int spc, float eps, int act, cudaStream_t st);  // cells: 2 B M N K, sums: 2 B blocks lines, zeroed
 
+// ---- outer_held.cu (the same with the weights in tensor memory: grids of up to four blocks per SM); arguments as above
+int outer_held_spc(int B, int M, int N, int K, int block, int inner, int outer, const void *w, const void *b, const void *s, const void *gamma,
+                   const void *beta, const void *x, const void *y);
+int launch_outer_held(const float *w, const float *b, const float *s, const float *gamma, const float *beta, const float *x, float *y,
+                      unsigned long long *cells, unsigned long long *sums, int *error_flag, int B, int M, int N, int K, int inner, int outer,
+                      int spc, float eps, int act, cudaStream_t st);
+
 // ---- norm.cu
 constexpr int kNormMaxParts = 64;
 // per-sample (sum, sum of squares) of x in double, `parts` slices per sample

@@ -27,6 +27,7 @@
 
 #include "common.cuh"
 #include "kernels.h"
+#include "outer_words.cuh"
 #include "patch_geo.cuh"
 
 namespace gn {
@@ -52,24 +53,6 @@ struct OuterSmallParams {
     int B, M, N, K, inner, outer, spc;
     float eps;
 };
-
-__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
-__device__ __forceinline__ unsigned long long ld_word(const unsigned long long *p)
-{
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ void ld_words(const unsigned long long *p, unsigned long long &a, unsigned long long &b)
-{
-    asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
-}
-__device__ __forceinline__ void st_words(unsigned long long *p, unsigned long long a, unsigned long long b)
-{
-    asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(a), "l"(b) : "memory");
-}
-__device__ __forceinline__ unsigned long long cell_word(float v, unsigned step) { return (unsigned long long)step << 32 | __float_as_uint(v); }
 
 template <int ACT>
 __global__ void __launch_bounds__(small8::THREADS, 2) outer_small_k(const OuterSmallParams p)
@@ -111,35 +94,7 @@ __global__ void __launch_bounds__(small8::THREADS, 2) outer_small_k(const OuterS
                          ((unsigned long long)__double_as_longlong(sq) & ~0xffull) | tag);
             }
             __syncwarp();
-            // Everything down to the result is done at every look, not only at the last: after some thousand cycles without
-            // double-precision work the first such instructions take 4500 cycles, which then keeps all blocks waiting for each other.
-            float2 result;
-            for (unsigned spins = 0;;) {
-                double sm = 0.0, sq = 0.0;
-                bool there = true;
-                for (int i = lane; i < p.nblocks; i += 64) {  // two blocks at a time
-                    const bool two = i + 32 < p.nblocks;
-                    unsigned long long v[4] = {tag, tag, tag, tag};
-                    ld_words(sums + kOuterSmallLine * i, v[0], v[1]);
-                    if (two) ld_words(sums + kOuterSmallLine * (i + 32), v[2], v[3]);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) there &= (v[e] & 0xff) == tag;
-                    sm += __longlong_as_double((long long)(v[0] & ~0xffull));
-                    sq += __longlong_as_double((long long)(v[1] & ~0xffull));
-                    if (two) {
-                        sm += __longlong_as_double((long long)(v[2] & ~0xffull));
-                        sq += __longlong_as_double((long long)(v[3] & ~0xffull));
-                    }
-                }
-                sm = warp_sum(sm);
-                sq = warp_sum(sq);
-                const double mean = sm * per_cell;
-                double var = fma(-mean, mean, sq * per_cell);
-                if (var < 0.0) var = 0.0;
-                result = make_float2((float)mean, (float)rsqrt(var + (double)p.eps));
-                if (__all_sync(0xffffffffu, there) || gave_up) break;
-                gave_up = ++spins > kSpinLimit;
-            }
+            const float2 result = watch_sums(sums, p.nblocks, kOuterSmallLine, tag, per_cell, p.eps, lane, kSpinLimit, gave_up);
             if (lane == 0) mstats[q] = result;
             __syncwarp();
             bar_arrive(B_STATS + q, WATCHED);

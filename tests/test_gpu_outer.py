@@ -224,6 +224,41 @@ def test_persistent_kernel_matches_step_by_step_loop_and_oracle(B, shape, inner,
     assert_close(got.cpu().numpy(), orc.outer_forward(*a64, inner, outer, 8, activation=act), None, f"persistent kernel B={B}")
 
 
+@pytest.mark.parametrize("B,shape,inner,outer,act", [
+    (1, (16, 296, 64), 1, 2, "relu"),        # 592 blocks, four for every SM
+    (2, (64, 64, 64), 2, 3, "silu"),         # two samples per CTA
+    (1, (40, 56, 72), 3, 2, "tanh"),         # 315 blocks: the last CTA has three
+    (5, (32, 40, 64), 2, 2, "leaky_relu"),   # three chunks of two samples, the last one with one
+    (1, (64, 64, 64), 2, 300, "silu"),       # more steps than the eight bits that mark the sums
+])
+def test_persistent_kernel_with_weights_in_tensor_memory(B, shape, inner, outer, act):
+    """Loops whose blocks do not fit into registers (outer_held.cu) against the loop of one launch per outer step and, where that is
+    affordable, the oracle; two runs give the same bits."""
+    from gridnet_b200 import outer_forward, outer_forward_failed, outer_forward_workspace
+    from gridnet_b200._lib import lib
+
+    w, b, s, gamma, beta = model_params(85, shape)
+    x = face_input(86, B, shape)
+    args = [dev(a) for a in (w, b, s, gamma, beta, x)]
+    ws = outer_forward_workspace(B, shape, 8, args[0].device)
+    assert lib.gn_outer_forward_plan(B, *shape, inner, outer, 8) == 3
+    try:
+        assert lib.gn_config_set(b"outer_kernel", 1) == 0
+        base = outer_forward(*args, inner, outer, 8, act)
+    finally:
+        lib.gn_config_set(b"outer_kernel", 0)
+    got = outer_forward(*args, inner, outer, 8, act, workspace=ws)
+    again = outer_forward(*args, inner, outer, 8, act, workspace=ws)
+    assert not outer_forward_failed(ws, B, shape, 8)
+    assert torch.equal(got, again)
+    if outer > 10:  # rounding of the statistics grows from step to step
+        assert torch.allclose(got, base, rtol=1e-3, atol=1e-3), (got - base).abs().max().item()
+        return
+    assert torch.allclose(got, base, rtol=2e-5, atol=2e-6), (got - base).abs().max().item()
+    a64 = [a.astype(np.float64) for a in (w, b, s, gamma, beta, x)]
+    assert_close(got.cpu().numpy(), orc.outer_forward(*a64, inner, outer, 8, activation=act), None, f"weights in tensor memory B={B}")
+
+
 @pytest.mark.parametrize("B,shape,block,inner,outer,act", [
     (1, (8, 8, 8), 8, 1, 1, "relu"),        # one region, one sample of a quad
     (5, (8, 16, 24), 8, 3, 2, "tanh"),      # a ragged second quad, non-cubic grid
