@@ -24,14 +24,14 @@ struct QuadGeo;
 // 10 x 10 x 10 cells.
 template <>
 struct QuadGeo<8> {
-    static constexpr int SIDE = 10, ROW = 10, PLANE = 100, CELLS = 1000, BUF_BYTES = 16000, TEAM = 2, NBUF = 3;
+    static constexpr int SIDE = 10, ROW = 10, PLANE = 100, CELLS = 1000, BUF_BYTES = 16000, TEAM = 2, NBUF = 2;
     __device__ static void cell(int c, int &cz, int &cy, int &cx)
     {
         cx = c % 10, cy = (c / 10) % 10, cz = c / 100;
     }
 };
 
-// Block 4: eight blocks, each with its own 6^3 tile (no room for a third buffer)
+// Block 4: eight blocks, each with its own 6^3 tile
 template <>
 struct QuadGeo<4> {
     static constexpr int SIDE = 6, ROW = 6, PLANE = 36, SUBCELLS = 216, CELLS = 8 * SUBCELLS, BUF_BYTES = CELLS * 16, TEAM = 2, NBUF = 2;
@@ -184,14 +184,17 @@ namespace quad {
 constexpr int VECS = 116, PACK_F = VECS * 128;  // floats per region
 }
 template <int N>
-__device__ __forceinline__ void quad_move(const float4 *src, unsigned col)
+__device__ __forceinline__ void quad_fetch(const float4 *src, float (&r)[4 * N])
 {
-    float r[4 * N];
 #pragma unroll
     for (int k = 0; k < N; ++k) {
         const float4 v = src[k * 32];  // not __ldg: the kernel before may be writing it still
         r[4 * k + 0] = v.x, r[4 * k + 1] = v.y, r[4 * k + 2] = v.z, r[4 * k + 3] = v.w;
     }
+}
+template <int N>
+__device__ __forceinline__ void quad_put(unsigned col, const float (&r)[4 * N])
+{
     int k = 0;
 #pragma unroll
     for (; k + 4 <= N; k += 4) tmem_st16(col + 4 * k, r + 4 * k);
@@ -201,12 +204,31 @@ __device__ __forceinline__ void quad_move(const float4 *src, unsigned col)
     }
     if (N & 1) tmem_st4(col + 4 * k, r + 4 * k);
 }
-// -> tensor memory. Each warp of a team moves half of the vectors, 29 loads in flight per lane.
+// -> tensor memory, by the TEAM warps of a quarter, each its share of the vectors in two goes: the loads of the first, then
+// between(), after which the region before may be overwritten, then the rest.
+template <int TEAM = 2, typename Between>
+__device__ __forceinline__ void quad_load_params(const float *packed, int role, int lane, unsigned tm, Between between)
+{
+    static_assert(TEAM == 2 || TEAM == 3, "");
+    constexpr int N = TEAM == 2 ? 29 : 20, LAST = quad::VECS - N * (2 * TEAM - 1);  // 29, 16
+    const float4 *src = reinterpret_cast<const float4 *>(packed) + role * (2 * N) * 32 + lane;
+    tm += role * (8 * N);
+    float r[4 * N];
+    quad_fetch<N>(src, r);
+    between();
+    quad_put<N>(tm, r);
+    if (LAST == N || role < TEAM - 1) {
+        quad_fetch<N>(src + N * 32, r);
+        quad_put<N>(tm + 4 * N, r);
+    } else {
+        float last[4 * LAST];
+        quad_fetch<LAST>(src + N * 32, last);
+        quad_put<LAST>(tm + 4 * N, last);
+    }
+}
 __device__ __forceinline__ void quad_load_params(const float *packed, int role, int lane, unsigned tm)
 {
-    const float4 *src = reinterpret_cast<const float4 *>(packed) + role * 58 * 32 + lane;
-    quad_move<29>(src, tm + role * 232);
-    quad_move<29>(src + 29 * 32, tm + role * 232 + 116);
+    quad_load_params<2>(packed, role, lane, tm, [] {});
 }
 
 // the weight sums of per-block normalisation (quad_wsum), by one warp of the team

@@ -4,15 +4,19 @@
 // differs is amplified from step to step (block 4, 8 x 16 iterations, silu: gradients up to 3e-5 apart in the 2-norm), and
 // where it carries a pre-activation over the kink of (leaky) relu gradients jump (40 x 56 x 72, 4 x 10 iterations: 1e-4).
 //
-// What differs from step_quad.cu is the split of a region over the lanes and the layout of the tile (taps_geo.cuh), and two
-// buffers per team (a third does not fit beside the (gamma, beta) tables; with three and the tables read from L2 256^3 x 32 took
-// 110.7 ms instead of 96.6). Fusion as in step_fast.cu: FUSE_IN normalises the landed tile in place with the whole-grid
-// statistics of the previous step and a per-region (gamma, beta) table; every launch can reduce (sum, sum of squares) per
-// sample and region of what it writes.
-// Measured against the 2 x 2 x 4 patches of step_quad.cu, whose sums come in another order: a step of 64^3 x 16, two inner
-// iterations, with the pre-activations kept 36.9 us against 37.5; the inference loop 64^3 x 64, 4 x 12, 1649 us against
-// 1652; 256^3 x 32, 2 x 32, 97.2 ms against 98.4; 40 x 56 x 72 x 37, 3 x 6, 314 us against 299, where a warp has two or three
-// items and waits for each tile.
+// What differs from step_quad.cu is the split of a region over the lanes and the layout of the tile (taps_geo.cuh). Fusion as in
+// step_fast.cu: FUSE_IN normalises the landed tile in place with the whole-grid statistics of the previous step and a per-region
+// (gamma, beta) table; every launch can reduce (sum, sum of squares) per sample and region of what it writes.
+// What bounds it: an iteration of an item takes 2820 cycles where two warps share a scheduler (3100 alone), 2270 of them the 864
+// packed FMAs, which get their operands from the register file at 2.6 cycles each instead of 2.0, the rest activation functions.
+// Around the iterations an item waits for its tile, normalises it and leaves sums and results. For that:
+//   - A lane's own cells stay in registers from their normalisation to the last iteration (92 instead of 124 shared loads per
+//     iteration). Only the halo's 488 entries of the (gamma, beta) table are in shared memory, a lane's own in tensor memory.
+//   - A warp takes the next item of its quarter when it is free (64^3: 1597 -> 1553 us), and asks for the first half of the
+//     next region's parameters before it waits for the other warp.
+// Measured before and after: 64^3 x 64, 4 x 12 iterations 1652 -> 1553 us; 40 x 56 x 72 x 37, 3 x 6 315 -> 290 us; 256^3 x 32, 2 x 32 91.8 ->
+// 90.4 ms (at 1.77 GHz); 64^3 x 128, block 4, 8 x 16 with gradients 41.3 -> 40.7 ms. Letting one or two warps of a quarter at a time into
+// the 27-tap sums, so that the rest of an item overlaps with another's, was slower (1754 and 1721 us).
 // Block 8: tiles by bulk tensor copy. Block 4: each warp fetches its own next tile, cell by cell and asynchronously; its
 // eight small tiles have to lie an odd number of cells apart, which bulk tensor copies cannot do.
 #include <string.h>
@@ -28,8 +32,9 @@ namespace gn {
 namespace {
 
 using namespace quad;
-constexpr int TEAM = 2;  // warps per quarter of tensor memory
-constexpr int TABLE8 = QuadGeo<8>::CELLS;  // entries per region of the (gamma, beta) table, kept in shared memory (block 8)
+// block 8: halo cells of a tile, whose (gamma, beta) are kept in shared memory; those of a lane's own cells and the places of its
+// halo cells are in the columns of tensor memory that parameters leave free
+constexpr int HALO8 = 488, COL_GAMMA = 464, COL_BETA = 480, COL_PLACE = 496;
 
 struct TapParams {
     const float *packed;     // [regions][PACK_F], QuadPrepare::ordered
@@ -85,15 +90,28 @@ __device__ __forceinline__ void fetch_tiles4(unsigned tile, const TapParams &p, 
     }
 }
 
+// Block 8: halo cell j = 0 .. 487 of a tile, as its index among the 10^3 cells: two z faces of 100, then two y faces of 8 x 10,
+// then two x faces of 8 x 8
+__device__ __forceinline__ int halo_cell(int j)
+{
+    if (j < 200) return j + (j >= 100 ? 800 : 0);
+    if (j < 360) {
+        const int e = j - 200, s = e >= 80 ? e - 80 : e;
+        return (1 + s / 10) * 100 + (e >= 80 ? 90 : 0) + s % 10;
+    }
+    const int e = j - 360, s = e & 63;
+    return (1 + (s >> 3)) * 100 + (1 + (s & 7)) * 10 + (e >= 64 ? 9 : 0);
+}
+
 template <int SUB, int ACT, bool FUSE_IN, bool SAVE>
-__global__ void __launch_bounds__(128 * TEAM, 1) step_fwd_taps(const __grid_constant__ CUtensorMap in_map, const TapParams p)
+__global__ void __launch_bounds__(128 * TapGeo<SUB>::TEAM, 1) step_fwd_taps(const __grid_constant__ CUtensorMap in_map, const TapParams p)
 {
     using G = TapGeo<SUB>;
-    constexpr int NBUF = G::NBUF;
-    static_assert(SUB == 8 || NBUF == TEAM, "block 4: a buffer per warp");
+    constexpr int TEAM = G::TEAM, NBUF = G::NBUF;
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) unsigned long long bars[QUARTERS * NBUF];
     __shared__ int issued[QUARTERS * NBUF];  // which item's copy into this buffer has been started last
+    __shared__ int claimed[QUARTERS];        // items of the team that warps have taken
     __shared__ unsigned tmem_slot;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -104,10 +122,11 @@ __global__ void __launch_bounds__(128 * TEAM, 1) step_fwd_taps(const __grid_cons
             mbar_init(smem_u32(&bars[i]), 1);
             issued[i] = -1;
         }
+        for (int i = 0; i < QUARTERS; ++i) claimed[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();
     }
-    float2 *const gbs = reinterpret_cast<float2 *>(smem + QUARTERS * NBUF * G::BUF_BYTES) + quarter * TABLE8;
+    float2 *const gbs = reinterpret_cast<float2 *>(smem + QUARTERS * NBUF * G::BUF_BYTES) + quarter * HALO8;
     tmem_fence_before();
     __syncthreads();
     tmem_fence_after();
@@ -117,8 +136,10 @@ __global__ void __launch_bounds__(128 * TEAM, 1) step_fwd_taps(const __grid_cons
     const int nbx = p.K >> 3, nby = p.N >> 3;
     const size_t P = (size_t)p.M * p.N * p.K;
     const long long worker = (long long)blockIdx.x * QUARTERS + quarter, nworkers = (long long)gridDim.x * QUARTERS;
-    const long long n0 = p.nitems * worker / nworkers;
-    const int cnt = (int)(p.nitems * (worker + 1) / nworkers - n0);
+    // whole rounds of the team per region where there are such (64^3 x 64: 14 items are 7 rounds instead of up to 8)
+    const long long even = p.Q % TEAM == 0 ? TEAM : 1;
+    const unsigned n0 = (unsigned)(p.nitems / even * worker / nworkers * even);
+    const int cnt = (int)(p.nitems / even * (worker + 1) / nworkers * even - n0);
     const unsigned bar0 = smem_u32(&bars[quarter * NBUF]), issued0 = smem_u32(&issued[quarter * NBUF]);
     const unsigned tiles = smem_u32(smem) + quarter * (NBUF * G::BUF_BYTES);
     const long long zstr = 4ll * p.N * p.K;
@@ -126,28 +147,40 @@ __global__ void __launch_bounds__(128 * TEAM, 1) step_fwd_taps(const __grid_cons
 
     // fetch the tile of the team's item i into its buffer: one lane (block 8), the whole warp (block 4)
     auto issue = [&](int i) {
-        const long long n = n0 + i;
-        const int blk = (int)(n / p.Q), q = (int)(n - (long long)blk * p.Q);
+        const unsigned n = n0 + i, blk = n / (unsigned)p.Q, buf = (unsigned)i % NBUF;
+        const int q = (int)(n - blk * p.Q);
         const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
-        const unsigned tile = tiles + (i % NBUF) * G::BUF_BYTES, bar = bar0 + 8 * (i % NBUF);
+        const unsigned tile = tiles + buf * G::BUF_BYTES;
         if constexpr (SUB == 8) {
             fence_proxy_async();  // earlier accesses to the buffer precede the bulk copy's writes
-            mbar_expect_tx(bar, G::CELLS * 16);
-            tma_load_4d(tile, &in_map, bar, (bx * 8 - 1) * 4, by * 8 - 1, bz * 8 - 1, q);
-            st_release_shared(issued0 + 4 * (i % NBUF), i);
+            mbar_expect_tx(bar0 + 8 * buf, G::CELLS * 16);
+            tma_load_4d(tile, &in_map, bar0 + 8 * buf, (bx * 8 - 1) * 4, by * 8 - 1, bz * 8 - 1, q);
+            st_release_shared(issued0 + 4 * buf, i);
         } else {
             fetch_tiles4(tile, p, bx, by, bz, q, lane);
         }
     };
     auto wait_tile = [&](int i) {
         if constexpr (SUB == 8) {  // see step_fwd_quad
+            const unsigned buf = (unsigned)i % NBUF;
             unsigned spins = 0;
-            while (ld_acquire_shared(issued0 + 4 * (i % NBUF)) != i && ++spins < kSpinLimit) {}
-            if (spins >= kSpinLimit || !mbar_wait_bounded(bar0 + 8 * (i % NBUF), (unsigned)(i / NBUF) & 1u, kSpinLimit)) failed = true;
+            while (ld_acquire_shared(issued0 + 4 * buf) != i && ++spins < kSpinLimit) {}
+            if (spins >= kSpinLimit || !mbar_wait_bounded(bar0 + 8 * buf, (unsigned)i / NBUF & 1u, kSpinLimit)) failed = true;
         } else {
             cp_async_wait_all();
         }
         __syncwarp();
+    };
+    // the warp's next item. Block 8: whoever is free takes it, its tile has been asked for already. Block 4: item i is fetched
+    // by the warp that works on it, i mod TEAM.
+    auto claim = [&](int last) {
+        if constexpr (SUB == 8) {
+            int i = 0;
+            if (lane == 0) i = atomicAdd(&claimed[quarter], 1);
+            return __shfl_sync(0xffffffffu, i, 0);
+        } else {
+            return last < 0 ? role : last + TEAM;
+        }
     };
     auto begin = [&]() {
         previous_done();
@@ -159,27 +192,61 @@ __global__ void __launch_bounds__(128 * TEAM, 1) step_fwd_taps(const __grid_cons
         }
         __syncwarp();
     };
+    if (FUSE_IN && SUB == 8 && role == 0) {
+        float place[16];
+#pragma unroll
+        for (int c = 0; c < 16; ++c) {
+            const int l = halo_cell(min(c * 32 + lane, HALO8 - 1));
+            place[c] = __int_as_float((l + l / 10) * 16);
+        }
+        tmem_st16(tm + COL_PLACE, place);
+    }
     if (!p.params_old || cnt == 0) begin();  // else the first region's parameters come first
 
-    int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
+    int blk = (int)(n0 / (unsigned)p.Q), q0 = (int)(n0 - (unsigned)blk * p.Q);
+    int i = claim(-1);
     for (int i0 = 0; i0 < cnt;) {
         const int here = min(cnt - i0, p.Q - q0);  // items of this region
         const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
         const size_t g0 = ((size_t)(bz * 8 + 4 * L.zp) * p.N + (by * 8 + L.y)) * p.K + bx * 8 + 4 * L.h;  // own patch
-        if (i0 > 0) {
-            tmem_fence_before();
-            team_sync<TEAM>(quarter);  // the other warp no longer reads the old region's weights
-            tmem_fence_after();
-        }
+        quad_load_params<TEAM>(p.packed + (size_t)blk * PACK_F, role, lane, tm, [&] {
+            if (i0 > 0) {
+                tmem_fence_before();
+                team_sync<TEAM>(quarter);  // the other warps no longer read the old region's weights
+                tmem_fence_after();
+            }
+        });
         if (FUSE_IN && SUB == 8) {
-            const unsigned char *src = reinterpret_cast<const unsigned char *>(p.gbt + (size_t)blk * TABLE8);
-            const unsigned dst = smem_u32(gbs);
-            for (int c = role * 32 + lane; c < TABLE8 / 2; c += 32 * TEAM) cp_async16(dst + c * 16, src + c * 16);
+            const float2 *const table = p.gbt + (size_t)blk * QuadGeo<8>::CELLS;
+            constexpr int STEPS = (16 + TEAM - 1) / TEAM;
+            float2 gh[STEPS], go[8];
+            const int n = 2 * role;  // planes whose own cells this warp looks after
+#pragma unroll
+            for (int c = 0; c < STEPS; ++c) {
+                const int j = (c * TEAM + role) * 32 + lane;
+                if (j < HALO8) gh[c] = table[halo_cell(j)];
+            }
+            if (role < 2)
+#pragma unroll
+                for (int c = 0; c < 8; ++c) go[c] = table[(4 * L.zp + n + (c >> 2) + 1) * 100 + (L.y + 1) * 10 + 4 * L.h + (c & 3) + 1];
+#pragma unroll
+            for (int c = 0; c < STEPS; ++c) {
+                const int j = (c * TEAM + role) * 32 + lane;
+                if (j < HALO8) gbs[j] = gh[c];
+            }
             __syncwarp();  // tensor memory instructions want the whole warp together
+            if (role < 2) {
+                float ga[8], be[8];
+#pragma unroll
+                for (int c = 0; c < 8; ++c) {
+                    ga[c] = go[c].x;
+                    be[c] = go[c].y;
+                }
+                tmem_st8(tm + COL_GAMMA + 4 * n, ga);
+                tmem_st8(tm + COL_BETA + 4 * n, be);
+            }
         }
-        quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm);
         tmem_wait_st();
-        if (FUSE_IN && SUB == 8) cp_async_wait_all();
         if (i0 == 0 && p.params_old) begin();
         tmem_fence_before();
         team_sync<TEAM>(quarter);
@@ -187,13 +254,20 @@ __global__ void __launch_bounds__(128 * TEAM, 1) step_fwd_taps(const __grid_cons
         if (i0 + here < cnt) {  // the next region's parameters on their way to L2
             const unsigned char *nx = reinterpret_cast<const unsigned char *>(p.packed + (size_t)(blk + 1) * PACK_F);
             for (int c = role * 32 + lane; c < PACK_F * 4 / 128; c += 32 * TEAM) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + c * 128));
+            if (FUSE_IN) {
+                constexpr int BYTES = QuadGeo<SUB>::CELLS * 8;
+                const unsigned char *ng = reinterpret_cast<const unsigned char *>(p.gbt) + (size_t)(blk + 1) * BYTES;
+                for (int c = role * 32 + lane; c < BYTES / 128; c += 32 * TEAM) asm volatile("prefetch.global.L2 [%0];" ::"l"(ng + c * 128));
+            }
             __syncwarp();
         }
 
-        // item i goes to warp i mod TEAM
-        for (int k = (role + TEAM - i0 % TEAM) % TEAM; k < here; k += TEAM) {
-            const int i = i0 + k, q = q0 + k;
-            const unsigned tile = tiles + (i % NBUF) * G::BUF_BYTES;
+        for (int next; i < i0 + here; i = next) {
+            const int q = q0 + i - i0;
+            const unsigned tile = tiles + (unsigned)i % NBUF * G::BUF_BYTES;
+            const unsigned win = tile + (unsigned)G::corner(L) * 16u;
+            const unsigned mine = win + (unsigned)(G::PLANE + G::ROW + 1) * 16u;  // own cell (0, 0)
+            u64 own[4][4][2];
             if (FUSE_IN) {
                 u64 rs[2], mu[2];  // rstd, -mean
                 {
@@ -205,74 +279,110 @@ __global__ void __launch_bounds__(128 * TEAM, 1) step_fwd_taps(const __grid_cons
                     mu[0] = pack2(-mr[0].x, -mr[1].x);
                     mu[1] = pack2(-mr[2].x, -mr[3].x);
                 }
-                wait_tile(i);
-                // step c: cell 32 c + lane of the tile (block 8), 4 c + r of the lane's small tile (block 4; the second
-                // tile of a pair is walked three cells ahead, which puts a quarter-warp on eight banks)
-                constexpr int STEPS = SUB == 8 ? 32 : 54, BATCH = SUB == 8 ? 16 : 18;
-                const int slot = lane >> 2, l0 = (lane & 3) + 3 * (slot & 1);
-                const unsigned sub = tile + (unsigned)(slot * 217) * 16u;
-                const float2 *const table = p.gbt + (size_t)blk * QuadGeo<4>::CELLS + ((slot >> 2) * 4 + (slot & 1) * 2 + ((slot >> 1) & 1)) * 216;
-                auto cell = [&](int c) { return SUB == 8 ? c * 32 + lane : (l0 + 4 * c >= 216 ? l0 + 4 * c - 216 : l0 + 4 * c); };
-                auto address = [&](int l) { return SUB == 8 ? tile + (unsigned)(l + l / 10) * 16u : sub + (unsigned)l * 16u; };
-#pragma unroll 1
-                for (int c0 = 0; c0 < STEPS; c0 += BATCH) {
-                    u64 v[BATCH][2];
-                    float2 g2[BATCH];
+                auto normed = [&](u64 v, int k2, float gm, float bt) {
+                    return ffma2r(fmul2(fadd2(v, mu[k2]), rs[k2]), pack2(gm, gm), pack2(bt, bt));
+                };
+                if constexpr (SUB == 8) {
+                    float place[16];
+                    tmem_ld16(tm + COL_PLACE, place);
+                    wait_tile(i);
+                    tmem_wait_ld16(place);
 #pragma unroll
-                    for (int c = 0; c < BATCH; ++c) {
-                        const int l = cell(c0 + c);
-                        if (SUB == 4 || l < TABLE8) {
-                            g2[c] = SUB == 8 ? gbs[l] : table[l];
-                            lds128u(address(l), v[c][0], v[c][1]);
+                    for (int c0 = 0; c0 < 16; c0 += 8) {
+                        u64 v[8][2];
+                        float2 g2[8];
+#pragma unroll
+                        for (int c = 0; c < 8; ++c) {
+                            g2[c] = gbs[min((c0 + c) * 32 + lane, HALO8 - 1)];
+                            lds128u(tile + __float_as_int(place[c0 + c]), v[c][0], v[c][1]);
                         }
+#pragma unroll
+                        for (int c = 0; c < 8; ++c)
+                            if (c0 + c < 15 || lane < HALO8 - 15 * 32)
+                                sts128u(tile + __float_as_int(place[c0 + c]), normed(v[c][0], 0, g2[c].x, g2[c].y), normed(v[c][1], 1, g2[c].x, g2[c].y));
                     }
 #pragma unroll
-                    for (int c = 0; c < BATCH; ++c) {
-                        const int l = cell(c0 + c);
-                        if (SUB == 4 || l < TABLE8) {
-                            const u64 gg = pack2(g2[c].x, g2[c].x), bb = pack2(g2[c].y, g2[c].y);
-                            sts128u(address(l), ffma2r(fmul2(fadd2(v[c][0], mu[0]), rs[0]), gg, bb), ffma2r(fmul2(fadd2(v[c][1], mu[1]), rs[1]), gg, bb));
+                    for (int n = 0; n < 4; n += 2) {
+                        float gb[16];  // of two planes
+                        u64 v[2][4][2];
+                        tmem_ld8(tm + COL_GAMMA + 4 * n, gb);
+                        tmem_ld8(tm + COL_BETA + 4 * n, gb + 8);
+#pragma unroll
+                        for (int o = 0; o < 8; ++o) lds128u(mine + (unsigned)((n + (o >> 2)) * G::PLANE + (o & 3)) * 16u, v[o >> 2][o & 3][0], v[o >> 2][o & 3][1]);
+                        tmem_wait_ld16(gb);
+#pragma unroll
+                        for (int o = 0; o < 8; ++o) {
+                            const u64 a = normed(v[o >> 2][o & 3][0], 0, gb[o], gb[8 + o]), b = normed(v[o >> 2][o & 3][1], 1, gb[o], gb[8 + o]);
+                            sts128u(mine + (unsigned)((n + (o >> 2)) * G::PLANE + (o & 3)) * 16u, a, b);
+                            own[n + (o >> 2)][o & 3][0] = a, own[n + (o >> 2)][o & 3][1] = b;
                         }
+                    }
+                } else {
+                    wait_tile(i);
+                    // step c: cell 4 c + r of the lane's small tile; the second tile of a pair is walked three cells ahead,
+                    // which puts a quarter-warp on eight banks
+                    constexpr int STEPS = 54, BATCH = 18;
+                    const int slot = lane >> 2, l0 = (lane & 3) + 3 * (slot & 1);
+                    const unsigned sub = tile + (unsigned)(slot * G::TILE) * 16u;
+                    const float2 *const table = p.gbt + (size_t)blk * QuadGeo<4>::CELLS + ((slot >> 2) * 4 + (slot & 1) * 2 + ((slot >> 1) & 1)) * 216;
+                    auto cell = [&](int c) { return l0 + 4 * c >= 216 ? l0 + 4 * c - 216 : l0 + 4 * c; };
+#pragma unroll 1
+                    for (int c0 = 0; c0 < STEPS; c0 += BATCH) {
+                        u64 v[BATCH][2];
+                        float2 g2[BATCH];
+#pragma unroll
+                        for (int c = 0; c < BATCH; ++c) {
+                            const int l = cell(c0 + c);
+                            g2[c] = table[l];
+                            lds128u(sub + (unsigned)l * 16u, v[c][0], v[c][1]);
+                        }
+#pragma unroll
+                        for (int c = 0; c < BATCH; ++c)
+                            sts128u(sub + (unsigned)cell(c0 + c) * 16u, normed(v[c][0], 0, g2[c].x, g2[c].y), normed(v[c][1], 1, g2[c].x, g2[c].y));
                     }
                 }
                 __syncwarp();
             } else {
                 wait_tile(i);
             }
+            if (!(FUSE_IN && SUB == 8))
+#pragma unroll
+                for (int n = 0; n < 4; ++n)
+#pragma unroll
+                    for (int o = 0; o < 4; ++o) lds128u(mine + (unsigned)(n * G::PLANE + o) * 16u, own[n][o][0], own[n][o][1]);
 
-            const unsigned win = tile + (unsigned)G::corner(L) * 16u;
-            const unsigned mine = win + (unsigned)(G::PLANE + G::ROW + 1) * 16u;  // own cell (0, 0)
-            const size_t own = ((size_t)q * P + g0) * 4;                           // the lane's cells in an IL4 tensor
+            const size_t at = ((size_t)q * P + g0) * 4;  // the lane's cells in an IL4 tensor
             for (int t = 0; t < p.inner; ++t) {
                 u64 acc[4][4][2], hold[2] = {0, 0};
-                float *const sh = SAVE ? p.save_h + (size_t)t * p.Q * P * 4 + own : nullptr;
-                tap_stencil<SUB>(win, tm, acc, [&](int n, int o, float scale, u64 c0, u64 c1) {
+                float *const sh = SAVE ? p.save_h + (size_t)t * p.Q * P * 4 + at : nullptr;
+                tap_stencil<SUB>(win, tm, acc, own, [&](int n, int o, float scale) {
                     if (SAVE) {  // two neighbours at a time
                         if (o & 1) stg256(sh + n * zstr + 8 * (o >> 1), hold[0], hold[1], acc[n][o][0], acc[n][o][1]);
                         else hold[0] = acc[n][o][0], hold[1] = acc[n][o][1];
                     }
-                    acc[n][o][0] = act_residual2<ACT>(acc[n][o][0], scale, c0);
-                    acc[n][o][1] = act_residual2<ACT>(acc[n][o][1], scale, c1);
+                    own[n][o][0] = act_residual2<ACT>(acc[n][o][0], scale, own[n][o][0]);
+                    own[n][o][1] = act_residual2<ACT>(acc[n][o][1], scale, own[n][o][1]);
                 });
                 __syncwarp();  // every lane has read its window
                 if (t + 1 < p.inner) {
 #pragma unroll
                     for (int n = 0; n < 4; ++n)
 #pragma unroll
-                        for (int o = 0; o < 4; ++o) sts128u(mine + (unsigned)(n * G::PLANE + o) * 16u, acc[n][o][0], acc[n][o][1]);
+                        for (int o = 0; o < 4; ++o) sts128u(mine + (unsigned)(n * G::PLANE + o) * 16u, own[n][o][0], own[n][o][1]);
                     __syncwarp();
                 } else {
                     // the tile is dead: fetch the next one
                     if (i + NBUF < cnt && (SUB == 4 || lane == 0)) issue(i + NBUF);
                     __syncwarp();
+                    next = claim(i);
                     if (p.y)
 #pragma unroll
                         for (int n = 0; n < 4; ++n)
 #pragma unroll
                             for (int o = 0; o < 4; o += 2)
-                                stg256(p.y + own + n * zstr + 4 * o, acc[n][o][0], acc[n][o][1], acc[n][o + 1][0], acc[n][o + 1][1]);
+                                stg256(p.y + at + n * zstr + 4 * o, own[n][o][0], own[n][o][1], own[n][o + 1][0], own[n][o + 1][1]);
                     if (p.out_partials) {
-                        const double r = tap_region_sums(acc, lane);
+                        const double r = tap_region_sums(own, lane);
                         if ((lane & 20) == 0)
                             reinterpret_cast<double *>(p.out_partials + (size_t)(4 * q + (lane & 2) + (lane >> 3)) * p.nparts + blk)[lane & 1] = r;
                         __syncwarp();
@@ -295,7 +405,7 @@ int launch_one(const CUtensorMap &map, const TapParams &p, unsigned ctas, cudaSt
 {
     using G = TapGeo<SUB>;
     auto kern = step_fwd_taps<SUB, ACT, FUSE_IN, SAVE>;
-    constexpr int smem = QUARTERS * G::NBUF * G::BUF_BYTES + (SUB == 8 && FUSE_IN ? QUARTERS * TABLE8 * 8 : 0);
+    constexpr int smem = QUARTERS * G::NBUF * G::BUF_BYTES + (SUB == 8 && FUSE_IN ? QUARTERS * HALO8 * 8 : 0);
     static_assert(smem <= 232448 - 1024 - 256, "shared memory budget of one SM");
     static unsigned long long attr_set = 0;
     if (first_use_on_device(&attr_set)) {
@@ -305,7 +415,7 @@ int launch_one(const CUtensorMap &map, const TapParams &p, unsigned ctas, cudaSt
             return GN_ERR_CUDA;
         }
     }
-    launch_after(kern, ctas, 128 * TEAM, smem, st, map, p);
+    launch_after(kern, ctas, 128 * G::TEAM, smem, st, map, p);
     return check_launch("step_fwd_taps");
 }
 

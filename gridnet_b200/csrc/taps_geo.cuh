@@ -17,10 +17,13 @@ struct TapLane {
 template <int SUB>
 struct TapGeo;
 
-// Block 8: rows of 11 cells, the last one beyond the tile (11 y mod 8 takes eight values), fetched by bulk tensor copy
+// TEAM: warps per quarter of tensor memory; NBUF: tile buffers per team. A third buffer fits but leaves nothing of the SM's memory
+// for the first-level cache (64^3 x 64, 4 x 12: 1616 us with three, 1553 with two).
+// Block 8: rows of 11 cells, the last one beyond the tile (11 y mod 8 takes eight values), fetched by bulk tensor copy. A third
+// warp, with 168 registers, brought nothing: two keep the FMA pipe as busy as its operands allow (64^3 x 64, 4 x 12: 1667 us).
 template <>
 struct TapGeo<8> {
-    static constexpr int ROW = 11, PLANE = 110, CELLS = 1100, BUF_BYTES = 17664, NBUF = 2;
+    static constexpr int ROW = 11, PLANE = 110, CELLS = 1100, BUF_BYTES = 17664, TEAM = 2, NBUF = 2;
     __device__ static int corner(const TapLane &L) { return 4 * L.zp * PLANE + L.y * ROW + 4 * L.h; }
 };
 
@@ -28,7 +31,7 @@ struct TapGeo<8> {
 // the two tiles along y by 1. Bulk tensor copies go to multiples of 8 cells only, so these are fetched cell by cell.
 template <>
 struct TapGeo<4> {
-    static constexpr int ROW = 6, PLANE = 36, TILE = 217, BUF_BYTES = 8 * TILE * 16, NBUF = 2;
+    static constexpr int ROW = 6, PLANE = 36, TILE = 217, BUF_BYTES = 8 * TILE * 16, TEAM = 2, NBUF = 2;
     __device__ static int corner(const TapLane &L) { return ((L.zp * 2 + L.h) * 2 + (L.y >> 2)) * TILE + (L.y & 3) * ROW; }
 };
 
@@ -37,7 +40,7 @@ struct TapGeo<4> {
 // done(n, o, scale, centre) is called when neuron (n, o) has its sum, between the FMAs of the planes that follow, so that the
 // activation functions (MUFU) run under them.
 template <int SUB, typename Done>
-__device__ __forceinline__ void tap_stencil(unsigned win, unsigned tm, u64 (&acc)[4][4][2], Done done)
+__device__ __forceinline__ void tap_stencil(unsigned win, unsigned tm, u64 (&acc)[4][4][2], const u64 (&own)[4][4][2], Done done)
 {
     using G = TapGeo<SUB>;
     float wb[2][12], sc[2][4];
@@ -50,11 +53,6 @@ __device__ __forceinline__ void tap_stencil(unsigned win, unsigned tm, u64 (&acc
 #pragma unroll
             for (int o = 0; o < 4; ++o) acc[n][o][0] = acc[n][o][1] = pack2(first[n * 4 + o], first[n * 4 + o]);
     }
-    auto finish = [&](int n, int o, float s) {
-        u64 c0, c1;
-        lds128u(win + (unsigned)((n + 1) * G::PLANE + G::ROW + 1 + o) * 16u, c0, c1);
-        done(n, o, s, c0, c1);
-    };
     tmem_ld8(tm, wb[0]);
     tmem_ld4(tm + 8, wb[0] + 8);
     int use = 0;
@@ -66,7 +64,10 @@ __device__ __forceinline__ void tap_stencil(unsigned win, unsigned tm, u64 (&acc
         for (int b = 0; b < 3; ++b) {
             u64 v[6][2];
 #pragma unroll
-            for (int j = 0; j < 6; ++j) lds128u(win + (unsigned)(rz * G::PLANE + b * G::ROW + j) * 16u, v[j][0], v[j][1]);
+            for (int j = 0; j < 6; ++j) {
+                if (b == 1 && rz >= 1 && rz <= 4 && j >= 1 && j <= 4) v[j][0] = own[rz - 1][j - 1][0], v[j][1] = own[rz - 1][j - 1][1];
+                else lds128u(win + (unsigned)(rz * G::PLANE + b * G::ROW + j) * 16u, v[j][0], v[j][1]);
+            }
 #pragma unroll
             for (int n = 0; n < 4; ++n) {
                 const int a = rz - n;
@@ -90,13 +91,13 @@ __device__ __forceinline__ void tap_stencil(unsigned win, unsigned tm, u64 (&acc
                     }
                 if (rz >= 3)
 #pragma unroll
-                    for (int e = 4 * at / uses; fin < e; ++fin) finish(rz - 3, fin, sc[rz & 1][fin]);
+                    for (int e = 4 * at / uses; fin < e; ++fin) done(rz - 3, fin, sc[rz & 1][fin]);
             }
         }
     }
     tmem_wait_ld4(sc[0]);
 #pragma unroll
-    for (int o = 0; o < 4; ++o) finish(3, o, sc[0][o]);
+    for (int o = 0; o < 4; ++o) done(3, o, sc[0][o]);
 }
 
 // The sum (j = 0) and the sum of squares (j = 1) of a region's values for the quad's samples s = 0 .. 3: on return lanes with
