@@ -77,19 +77,27 @@ __device__ __forceinline__ void previous_done()
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 template <typename... P, typename... A>
-inline void launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+inline void launch_after_cluster(unsigned cluster_y, void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
 {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = attr[1].val.clusterDim.z = 1;
+    attr[1].val.clusterDim.y = cluster_y;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = cluster_y > 1 ? 2 : 1;
     (void)cudaLaunchKernelEx(&cfg, kern, P(args)...);  // check_launch sees the error
+}
+template <typename... P, typename... A>
+inline void launch_after(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args)
+{
+    launch_after_cluster(1, kern, grid, block, smem, st, args...);
 }
 
 // ------------------------------------------------------------------ reductions

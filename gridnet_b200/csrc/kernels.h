@@ -195,6 +195,7 @@ struct QuadReverse {
     float *delta, *dsum, *gx;  // [inner], one, one
     float *dsq;                // [Q][P]
     int M, N, K, Q, inner, block;
+    int params_old;            // the kernel queued before this one did not write packed_t or wsum: it may load them while that one runs
 };
 int launch_quad_reverse(const QuadReverse &a, int act, cudaStream_t st);
 struct QuadWgrad {
@@ -215,8 +216,8 @@ int launch_quad_wgrad(const QuadWgrad &a, int act, cudaStream_t st);
 // gradients of the parameters out of gpk and, with il, il (IL4) -> x [B, P]
 int launch_quad_finish(const float *gpk, float *gw, float *gb, float *gs, const float *il, float *x, int B, int M, int N, int K, int block,
                        int branches, cudaStream_t st);
-// branches: 2 if w is one branch of [27][2][P]. hterm (from launch_quad_reverse), x_il4 (the step's input): per-block normalisation, or nullptr
-int launch_quad_border(const float *w, int branches, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
+// dsum2: of the gate, w is then [27][2][P]; or nullptr. hterm (from launch_quad_reverse), x_il4 (the step's input): per-block normalisation, or nullptr
+int launch_quad_border(const float *w, const float *dsum, const float *dsum2, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
                        int Q, int block, cudaStream_t st);
 int quad_norm_parts(long long P);
 int launch_quad_norm_sums(const float *x, const float *g, const float *sub, const float *gamma, const float2 *stats, double2 *partials,
@@ -239,6 +240,7 @@ struct QuadGated {
     int nparts;
     float *hv, *hg, *x;        // [inner] tensors each to keep (pre-activations, activations that went in), or nullptr
     int M, N, K, Q, inner;
+    int params_old;            // the kernel queued before this one did not write packed or gbt
 };
 int launch_quad_gated_fwd(const QuadGated &a, int act, cudaStream_t st);
 struct QuadGatedReverse {

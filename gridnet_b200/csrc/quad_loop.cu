@@ -128,11 +128,11 @@ static GatedWs carve_gated(void *base, const LoopDims &d, bool backward, bool re
 }
 
 // one step; kept: [3][inner] tensors (the two pre-activations, the activations that went in), or nullptr
-static int gated_step(const GatedWs &w, const LoopDims &d, const float *in, const float2 *in_stats, float *out, double2 *partials, float *kept, int act,
-                      cudaStream_t st)
+static int gated_step(const GatedWs &w, const LoopDims &d, const float *in, const float2 *in_stats, float *out, double2 *partials, float *kept,
+                      int params_old, int act, cudaStream_t st)
 {
     QuadGated a{};
-    a.packed = w.packed; a.gbt = w.gbt; a.in_il4 = in; a.out_il4 = out; a.in_stats = in_stats;
+    a.packed = w.packed; a.gbt = w.gbt; a.params_old = params_old; a.in_il4 = in; a.out_il4 = out; a.in_stats = in_stats;
     a.out_partials = partials; a.nparts = 2 * d.regions;
     if (kept) {
         a.hv = kept; a.hg = kept + d.inner * d.T4; a.x = kept + 2 * d.inner * d.T4;
@@ -271,6 +271,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
         }
         QuadReverse r{};
         r.packed_t = w.packed_t; r.g = w.g[cur];
+        r.params_old = !residual || !kept || (!first && nparams == 1);  // something ran since they were re-ordered
         if (!residual) {
             r.raw = outs[k]; r.stats = mr + (size_t)k * S; r.ac = w.ac;
         }
@@ -284,7 +285,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
         g.M = M; g.N = N; g.K = K; g.Q = d.Q; g.inner = inner; g.block = block;
         TRY_(launch_quad_wgrad(g, act, st));
         if (nparams > 1 && k > 0) TRY_(launch_quad_finish(w.gpk, gw[kp], gb[kp], gs[kp], nullptr, nullptr, B, M, N, K, block, 1, st));
-        TRY_(launch_quad_border(weights[kp], 1, w.dsum, w.g[cur ^ 1], nullptr, nullptr, M, N, K, d.Q, block, st));
+        TRY_(launch_quad_border(weights[kp], w.dsum, nullptr, w.g[cur ^ 1], nullptr, nullptr, M, N, K, d.Q, block, st));
         if (residual) {
             TRY_(launch_quad_norm_sums(in, w.g[cur ^ 1], w.g[cur], gamma, in_stats, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
             TRY_(launch_quad_norm_residual_apply(in, w.g[cur ^ 1], w.g[cur], gamma, in_stats, w.ac, w.g[cur], d.Q, d.P, st));
@@ -320,7 +321,7 @@ GN_API int gn_gated_loop_forward_f32(const float *weight, const float *bias, con
     TRY_(launch_quad_prepare(a, M, N, K, 8, st));
     for (int k = 0; k < outer; ++k) {
         TRY_(gated_step(w, d, k ? outs[k - 1] : x_il4, k ? mr + (size_t)(k - 1) * S : nullptr, outs[k], w.partials, stashes ? stashes[k] : nullptr,
-                        act, st));
+                        k > 0, act, st));
         TRY_(launch_norm_finalize(w.partials, 2 * d.regions, mr + (size_t)k * S, S, d.P, ln_eps, st));
     }
     return launch_from_il4(outs[outer - 1], mr + (size_t)(outer - 1) * S, gamma, beta, y, B, d.P, st);
@@ -361,7 +362,7 @@ GN_API int gn_gated_loop_backward_f32(const float *weight, const float *bias, co
         if (!kept) {
             // the step's output is computed once more, into the buffer that receives the gradient afterwards
             kept = w.replay;
-            TRY_(gated_step(w, d, in, in_stats, w.g[cur ^ 1], nullptr, kept, act, st));
+            TRY_(gated_step(w, d, in, in_stats, w.g[cur ^ 1], nullptr, kept, 1, act, st));
         }
         QuadGatedReverse r{};
         r.packed_t = w.packed_t; r.gamma = gamma; r.g = w.g[cur]; r.raw = outs[k]; r.stats = mr + (size_t)k * S; r.ac = w.ac;
@@ -375,8 +376,7 @@ GN_API int gn_gated_loop_backward_f32(const float *weight, const float *bias, co
         g.accumulate = !first;
         g.M = M; g.N = N; g.K = K; g.Q = d.Q; g.inner = inner; g.block = 8;
         TRY_(launch_quad_wgrad(g, act, st));
-        TRY_(launch_quad_border(weight, 2, dsum_v, w.g[cur ^ 1], nullptr, nullptr, M, N, K, d.Q, 8, st));
-        TRY_(launch_quad_border(weight + d.P, 2, dsum_g, w.g[cur ^ 1], nullptr, nullptr, M, N, K, d.Q, 8, st));
+        TRY_(launch_quad_border(weight, dsum_v, dsum_g, w.g[cur ^ 1], nullptr, nullptr, M, N, K, d.Q, 8, st));
     }
     return launch_quad_finish(w.gpk, gw, gb, nullptr, w.g[cur], gx, B, M, N, K, 8, 2, st);
 }

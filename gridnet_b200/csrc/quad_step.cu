@@ -196,7 +196,7 @@ GN_API int gn_step_backward_kept_f32(const float *w, const float *b, const float
     g.in_il4 = k.x; g.delta = ws.delta; g.h = k.h; g.scale = s; g.dsq = ws.dsq; g.gpk = ws.gpk; g.tile_stats = k.stats;
     g.M = M; g.N = N; g.K = K; g.Q = d.Q; g.inner = inner; g.block = block;
     TRY_(launch_quad_wgrad(g, act, st));
-    TRY_(launch_quad_border(w, 1, ws.dsum, ws.gout, k.x, ws.hterm, M, N, K, d.Q, block, st));
+    TRY_(launch_quad_border(w, ws.dsum, nullptr, ws.gout, k.x, ws.hterm, M, N, K, d.Q, block, st));
     return launch_quad_finish(ws.gpk, gw, gb, gs, ws.gout, gx, B, M, N, K, block, 1, st);
 }
 

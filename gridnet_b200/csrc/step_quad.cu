@@ -66,6 +66,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) unsigned long long bars[QUARTERS * G::NBUF];
     __shared__ int issued[QUARTERS * G::NBUF];  // which item's copy into this buffer has been started last
+    __shared__ int claimed[QUARTERS];           // items of the team that warps have taken
     __shared__ unsigned tmem_slot;
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -76,6 +77,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
             mbar_init(smem_u32(&bars[i]), 1);
             issued[i] = -1;
         }
+        for (int i = 0; i < QUARTERS; ++i) claimed[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         fence_proxy_async();
     }
@@ -101,8 +103,9 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     const int nbx = p.K >> 3, nby = p.N >> 3;
     const size_t P = (size_t)p.M * p.N * p.K;
     const long long worker = (long long)blockIdx.x * QUARTERS + quarter, nworkers = (long long)gridDim.x * QUARTERS;
-    const long long n0 = p.nitems * worker / nworkers;
-    const int cnt = (int)(p.nitems * (worker + 1) / nworkers - n0);
+    const long long even = p.Q % TEAM == 0 ? TEAM : 1;  // whole rounds of the team per region
+    const unsigned n0 = (unsigned)(p.nitems / even * worker / nworkers * even);
+    const int cnt = (int)(p.nitems / even * (worker + 1) / nworkers * even - n0);
     const unsigned bar0 = smem_u32(&bars[quarter * NBUF]), issued0 = smem_u32(&issued[quarter * NBUF]);
     const unsigned tiles = smem_u32(smem) + quarter * (NBUF * G::BUF_BYTES);
     const long long wzs = (long long)p.N * p.K, wys = (long long)L.ysgn * p.K;
@@ -110,8 +113,8 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
 
     // one lane: fetch the tile of the team's item i into its buffer
     auto issue = [&](int i) {
-        const long long n = n0 + i;
-        const int blk = (int)(n / p.Q), q = (int)(n - (long long)blk * p.Q);
+        const unsigned n = n0 + i, blk = n / (unsigned)p.Q;
+        const int q = (int)(n - blk * p.Q);
         const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
         const unsigned tile = tiles + (i % NBUF) * G::BUF_BYTES, bar = bar0 + 8 * (i % NBUF);
         fence_proxy_async();  // earlier accesses to the buffer precede the bulk copies' writes
@@ -134,22 +137,29 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
         if (spins >= kSpinLimit || !mbar_wait_bounded(bar0 + 8 * (i % NBUF), (unsigned)(i / NBUF) & 1u, kSpinLimit)) failed = true;
         __syncwarp();
     };
+    auto claim = [&]() {  // the next item, for whichever warp is free
+        int i = 0;
+        if (lane == 0) i = atomicAdd(&claimed[quarter], 1);
+        return __shfl_sync(0xffffffffu, i, 0);
+    };
     previous_done();
     if (role == 0 && lane == 0)
         for (int i = 0; i < NBUF && i < cnt; ++i) issue(i);
     __syncwarp();
+    int i = claim();
 
-    int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
+    int blk = (int)(n0 / (unsigned)p.Q), q0 = (int)(n0 - (unsigned)blk * p.Q);
     for (int i0 = 0; i0 < cnt;) {
         const int here = min(cnt - i0, p.Q - q0);  // items of this region
         const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
         const size_t g0 = ((size_t)(bz * 8 + L.z0) * p.N + (by * 8 + L.y0)) * p.K + bx * 8 + 4 * L.h;  // own patch, native layout
-        if (i0 > 0) {
-            tmem_fence_before();
-            team_sync<TEAM>(quarter);  // the other warps no longer read the old region's weights
-            tmem_fence_after();
-        }
-        quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm);
+        quad_load_params<TEAM>(p.packed + (size_t)blk * PACK_F, role, lane, tm, [&] {
+            if (i0 > 0) {
+                tmem_fence_before();
+                team_sync<TEAM>(quarter);  // the other warp no longer reads the old region's weights
+                tmem_fence_after();
+            }
+        });
         if (role == 0) quad_load_wsum(p.wsum, blk, lane, tm);
         tmem_wait_st();
         tmem_fence_before();
@@ -161,9 +171,8 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
             __syncwarp();
         }
 
-        // item i goes to warp i mod TEAM
-        for (int k = (role + TEAM - i0 % TEAM) % TEAM; k < here; k += TEAM) {
-            const int i = i0 + k, q = q0 + k;
+        for (int next = 0; i < i0 + here; i = next) {
+            const int q = q0 + i - i0;
             const unsigned tile = tiles + (i % NBUF) * G::BUF_BYTES;
             wait_tile(i);
 
@@ -327,6 +336,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
                 } else {
                     if (lane == 0 && i + NBUF < cnt) issue(i + NBUF);  // the tile is dead: fetch the next one
                     __syncwarp();
+                    next = claim();
 #pragma unroll
                     for (int n = 0; n < 4; ++n)
 #pragma unroll

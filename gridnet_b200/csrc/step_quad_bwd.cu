@@ -15,6 +15,7 @@
 // Reference semantics: the gradient of gridnet/backend_torch.py:61-142 and of
 // torch.nn.LayerNorm((M,N,K)) (gridnet/scripts/train_mnist.py:54,62-64); the kernel this stands in for is
 // gridnet_cuda_backward_kernel, src/gridnet_cuda_kernels.cu:202-450.
+#include <cooperative_groups.h>
 #include <string.h>
 
 #include "common.cuh"
@@ -55,6 +56,7 @@ struct QuadRevParams {
     float *delta, *dsum, *gx;      // [inner], one, one IL4 tensors
     float *dsq;                    // [Q][P] gradient terms of the residual scale, summed over the quad and the iterations
     int M, N, K, Q, inner;
+    int params_old;                // the kernel before this one did not write packed (or wsum)
     long long nitems;
 };
 
@@ -74,9 +76,11 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
     constexpr float PER_CELL = SUB == 8 ? 1.0f / 1000 : 1.0f / 216;
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ unsigned tmem_slot;
+    __shared__ int claimed[QUARTERS];  // items of the team that warps have taken
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int quarter = warp & 3, role = warp >> 2;
     if (warp == 0) tmem_alloc_all(&tmem_slot);
+    if (tid < QUARTERS) claimed[tid] = 0;
     const unsigned tile = smem_u32(smem) + warp * TILE_BYTES, stage = smem_u32(smem) + TILES_BYTES + warp * Bytes<IN>::STAGE;
     const unsigned stage_x = stage + STAGE_BYTES, stage_s = stage_x + STAGE_BYTES;  // BN
     for (int c = lane; c < CELLS; c += 32) sts128u(tile + c * 16, 0, 0);
@@ -89,8 +93,9 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
     const int nbx = p.K >> 3, nby = p.N >> 3;
     const size_t P = (size_t)p.M * p.N * p.K, T4 = (size_t)p.Q * P * 4;  // floats of an IL4 tensor
     const long long worker = (long long)blockIdx.x * QUARTERS + quarter, nworkers = (long long)gridDim.x * QUARTERS;
-    const long long n0 = p.nitems * worker / nworkers;
-    const int cnt = (int)(p.nitems * (worker + 1) / nworkers - n0);
+    const long long even = p.Q % TEAM == 0 ? TEAM : 1;  // whole rounds of the team per region
+    const unsigned n0 = (unsigned)(p.nitems / even * worker / nworkers * even);
+    const int cnt = (int)(p.nitems / even * (worker + 1) / nworkers * even - n0);
     const long long wzs = (long long)p.N * p.K, wys = (long long)L.ysgn * p.K;
     const long long zstr = wzs * 4, ystr = wys * 4;
     const int dx = L.xsgn * 16;
@@ -108,8 +113,7 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
     auto own_cell = [&](int n, int o) { return mine + (unsigned)((n & 1) * L.ysgn * ROW * 16 + o * dx) + (n >> 1) * PLANE * 16u; };
     // first cell of the region of the team's item i in an IL4 tensor
     auto corner_of = [&](int i) {
-        const long long n = n0 + i;
-        const int blk = (int)(n / p.Q), q = (int)(n - (long long)blk * p.Q);
+        const unsigned n = n0 + i, blk = n / (unsigned)p.Q, q = n - blk * p.Q;
         const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
         return ((size_t)q * P + ((size_t)(bz * 8) * p.N + by * 8) * p.K + bx * 8) * 4;
     };
@@ -118,8 +122,7 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
     auto fetch_h = [&](int i, size_t corner, int t) {
         quad_stage<0, 8>(stage, p.h + (size_t)t * T4 + corner, zstr, p.K, lane);
         if (BN) {
-            const long long n = n0 + i;
-            const int blk = (int)(n / p.Q), q = (int)(n - (long long)blk * p.Q);
+            const unsigned n = n0 + i, blk = n / (unsigned)p.Q, q = n - blk * p.Q;
             const float4 *src = p.tile_stats + (((size_t)t * p.Q + q) * ntiles + (size_t)blk * (SUB == 8 ? 1 : 8)) * QS_COUNT;
             if (lane < (SUB == 8 ? 1 : 8) * QS_COUNT) cp_async16(stage_s + lane * 16, src + lane);
         }
@@ -132,26 +135,47 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
         for (int k = 0; k < 16; ++k)
             cp_async16(tile + (unsigned)(((k >> 1) + 1) * PLANE + (y + 4 * (k & 1)) * ROW + x + 1) * 16u, src + (k & 1) * 16ll * p.K + (k >> 1) * zstr);
     };
+    // what an item starts with, 64 lines each, on its way to L2
+    auto expect = [&](size_t corner) {
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const size_t row = corner + ((lane >> 3) + 4 * k) * zstr + (lane & 7) * 4ll * p.K;
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.g + row));
+            if (NORM_IN) asm volatile("prefetch.global.L2 [%0];" ::"l"(p.raw + row));
+        }
+    };
+    auto claim = [&]() {
+        int i = 0;
+        if (lane == 0) i = atomicAdd(&claimed[quarter], 1);
+        return __shfl_sync(0xffffffffu, i, 0);
+    };
     const size_t to_own = (((size_t)L.z0 * p.N + L.y0) * p.K + 4 * L.h) * 4;  // corner -> this lane's cells
-    previous_done();
-    __syncwarp();
-    if (role < cnt) {
-        fetch_g(corner_of(role));
-        fetch_h(role, corner_of(role), p.inner - 1);
-        if (BN) fetch_x(corner_of(role));
-    }
+    int i = claim();  // the item in work
+    auto begin = [&]() {
+        previous_done();
+        __syncwarp();
+        if (i < cnt) {
+            fetch_g(corner_of(i));
+            fetch_h(i, corner_of(i), p.inner - 1);
+            if (BN) fetch_x(corner_of(i));
+            if (NORM_IN) expect(corner_of(i));
+        }
+    };
+    if (!p.params_old || cnt == 0) begin();  // else the first region's parameters come first
 
-    int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
+    int blk = (int)(n0 / (unsigned)p.Q), q0 = (int)(n0 - (unsigned)blk * p.Q);
     for (int i0 = 0; i0 < cnt;) {
         const int here = min(cnt - i0, p.Q - q0);
-        if (i0 > 0) {
-            tmem_fence_before();
-            team_sync<TEAM>(quarter);
-            tmem_fence_after();
-        }
-        quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm);
+        quad_load_params<TEAM>(p.packed + (size_t)blk * PACK_F, role, lane, tm, [&] {
+            if (i0 > 0) {
+                tmem_fence_before();
+                team_sync<TEAM>(quarter);  // the other warp no longer reads the old region's weights
+                tmem_fence_after();
+            }
+        });
         if (BN && role == 0) quad_load_wsum(p.wsum, blk, lane, tm);
         tmem_wait_st();
+        if (i0 == 0 && p.params_old) begin();
         tmem_fence_before();
         team_sync<TEAM>(quarter);
         tmem_fence_after();
@@ -161,8 +185,8 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
             __syncwarp();
         }
         const unsigned my_stats = stage_s + (SUB == 8 ? 0 : (unsigned)quad_tile_of(L, 0)) * (QS_COUNT * 16);
-        for (int k = (role + TEAM - i0 % TEAM) % TEAM; k < here; k += TEAM) {
-            const int i = i0 + k, q = q0 + k;
+        for (int next = 0; i < i0 + here; i = next) {
+            const int q = q0 + i - i0;
             const size_t corner = corner_of(i), own = corner + to_own;
             u64 g[4][4][2], dsum[4][4][2];
             float dsa[4][4];
@@ -212,6 +236,7 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
                     dsa[n][o] = 0.0f;
                 }
             u64 hf[2] = {0, 0}, he[2] = {0, 0};  // BN: F and E
+            size_t ahead = 0;                    // corner of the next item
             for (int t = p.inner - 1; t >= 0; --t) {
                 float sc[16];
                 if (!BN) tmem_ld16(tm + COL_SCALE, sc);
@@ -315,14 +340,19 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
                 __syncwarp();  // the delta tile is complete, h_t has been read
                 if (t > 0) {
                     fetch_h(i, corner, t - 1);
-                } else if (i + TEAM < cnt) {
-                    fetch_h(i + TEAM, corner_of(i + TEAM), p.inner - 1);
-                    if (BN) fetch_x(corner_of(i + TEAM));
+                } else {
+                    next = claim();
+                    if (next < cnt) {
+                        ahead = corner_of(next);
+                        fetch_h(next, ahead, p.inner - 1);
+                        if (BN) fetch_x(ahead);
+                        expect(ahead);
+                    }
                 }
                 quad_stencil<PLANE, ADD>(rows, dx, tm, g, inv, [](int, int, float, float, u64, u64) {});
                 __syncwarp();  // ... and has been read
             }
-            if (i + TEAM < cnt) fetch_g(corner_of(i + TEAM));
+            if (next < cnt) fetch_g(ahead);
             if (BN && quad_tile_leader<SUB>(lane)) {
                 float4 *to = p.hterm + ((size_t)q * ntiles + quad_tile_of(L, blk)) * 2;
                 float v[8];
@@ -702,11 +732,11 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
 // the CTAs after those put the input's gradient back into the grid's own layout.
 constexpr int kUnpack = 29;  // of the 116 values per thread
 template <int SUB>
-__global__ void __launch_bounds__(256) quad_finish_k(const float *__restrict__ gpk, float *__restrict__ gw, float *__restrict__ gb,
-                                                     float *__restrict__ gs, const float4 *__restrict__ il, float *__restrict__ x, int B, int M,
+__global__ void __launch_bounds__(256) quad_finish_k(const float *gpk, float *gw, float *gb, float *gs, const float4 *il, float *x, int B, int M,
                                                      int N, int K, int chunks, int branches, unsigned grads, unsigned parts)
 {
     using namespace quadwg;
+    previous_done();
     if (blockIdx.x >= grads) {
         const unsigned i = blockIdx.x - grads;
         const size_t P = (size_t)M * N * K, c = (size_t)(i % parts) * 256 + threadIdx.x;
@@ -730,15 +760,21 @@ __global__ void __launch_bounds__(256) quad_finish_k(const float *__restrict__ g
     const float *src = gpk + ((size_t)branch * chunks * regions + blk) * GRAD_F + tid;
     const size_t step = (size_t)regions * GRAD_F;
     const int k0 = cta % (116 / kUnpack) * kUnpack;
+    // chunk after chunk, so that a thread has 29 loads in flight
+    float v[kUnpack];
+#pragma unroll
+    for (int i = 0; i < kUnpack; ++i) v[i] = src[(k0 + i) * THREADS];
+    for (int c = 1; c < chunks; ++c) {
+        src += step;
+#pragma unroll
+        for (int i = 0; i < kUnpack; ++i) v[i] += src[(k0 + i) * THREADS];
+    }
 #pragma unroll
     for (int i = 0; i < kUnpack; ++i) {
-        const int k = k0 + i;
-        float v = src[k * THREADS];
-        for (int c = 1; c < chunks; ++c) v += src[c * step + k * THREADS];
-        const int n = k & 3;
+        const int k = k0 + i, n = k & 3;
         if (branches > 1 && k >= 112) break;  // no scale
         float *dst = k < 108 ? gw + ((size_t)(k >> 2) * branches + branch) * P : (k < 112 ? gb + branch * P : gs);
-        dst[g0 + (size_t)(n >> 1) * N * K + (size_t)(n & 1) * K] = v;
+        dst[g0 + (size_t)(n >> 1) * N * K + (size_t)(n & 1) * K] = v[i];
     }
 }
 
@@ -799,18 +835,19 @@ struct Terms {
 };
 }  // namespace quadborder
 
-template <bool NORM>
-__global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict__ w, size_t tap, const float4 *__restrict__ dsum, float4 *__restrict__ gx,
-                                                         const float4 *__restrict__ x, const float4 *__restrict__ hterm, int Q, int M, int N,
-                                                         int K, int qpc)
+template <bool NORM, int BR>
+__global__ void __launch_bounds__(384, BR == 1 ? 3 : 2) quad_border8_k(const float *__restrict__ w, size_t branch, const float4 *__restrict__ dsum,
+                                                                       const float4 *__restrict__ dsum2, float4 *__restrict__ gx,
+                                                                       const float4 *__restrict__ x, const float4 *__restrict__ hterm, int Q,
+                                                                       int M, int N, int K, int qpc)
 {
     using namespace quadborder;
     using T = Terms<8>;
     constexpr int THREADS = 384;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    float4 *const shell = reinterpret_cast<float4 *>(smem_raw);  // [RING][SHELL]
-    float4 *const part = shell + RING * SHELL;                   // [2][3][128]
-    float4 *const mine = part + 2 * 3 * 128;                     // [RING][SURFACE] grad_x, NORM: then x
+    float4 *const shell = reinterpret_cast<float4 *>(smem_raw);  // [RING][BR][SHELL]
+    float4 *const part = shell + RING * BR * SHELL;              // [2][BR][3][128]
+    float4 *const mine = part + 2 * BR * 3 * 128;                // [RING][SURFACE] grad_x, NORM: then x
     __shared__ float4 terms[NORM ? RING : 1][2 * T::COUNT], dirs[NORM ? 2 : 1][2 * DIRS];
     const int tid = threadIdx.x;
     const int nbx = K >> 3, nby = N >> 3;
@@ -818,7 +855,7 @@ __global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t P = (size_t)M * N * K;
     const long long origin = ((long long)(bz * 8 - 1) * N + (by * 8 - 1)) * K + (bx * 8 - 1);
-    for (int i = tid; i < RING * SHELL; i += THREADS) shell[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int i = tid; i < RING * BR * SHELL; i += THREADS) shell[i] = make_float4(0.f, 0.f, 0.f, 0.f);
     // shell cells this thread fetches: z faces 2 x 10 x 10, then y faces 2 x 8 x 10, then x faces 2 x 8 x 8
     int rel[2];
 #pragma unroll
@@ -841,7 +878,7 @@ __global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict
     // role 1: one cell of one face, (u, v) its coordinates along the other two axes
     const int axis = tid >> 7, fc = tid & 127, side = fc >> 6, u = (fc >> 3) & 7, v = fc & 7;
     const int across = side == 0 ? 1 : -1;
-    float wf[9];
+    float wf[BR][9];
     {
         const int lz = axis == 0 ? side * 7 : u, ly = axis == 0 ? u : (axis == 1 ? side * 7 : v), lx = axis == 2 ? side * 7 : v;
 #pragma unroll
@@ -851,7 +888,9 @@ __global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict
             const bool owned = (axis == 0 || (u - d1 >= 0 && u - d1 < 8)) && (axis < 2 || (v - d2 >= 0 && v - d2 < 8));
             const int nz = bz * 8 + lz - dz, ny = by * 8 + ly - dy, nx = bx * 8 + lx - dx;
             const bool ok = owned && nz >= 0 && nz < M && ny >= 0 && ny < N && nx >= 0 && nx < K;
-            wf[e] = ok ? w[(size_t)((dz + 1) * 9 + (dy + 1) * 3 + dx + 1) * tap + ((size_t)nz * N + ny) * K + nx] : 0.0f;
+#pragma unroll
+            for (int k = 0; k < BR; ++k)
+                wf[k][e] = ok ? w[((size_t)((dz + 1) * 9 + (dy + 1) * 3 + dx + 1) * BR + k) * branch + ((size_t)nz * N + ny) * K + nx] : 0.0f;
         }
     }
     const int row = axis == 2 ? 8 : 10;
@@ -881,10 +920,13 @@ __global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict
     int slot = 0;  // ring slot of the quad in work
     auto fetch = [&](int q, int r) {
         if (q < q1) {
-            const float4 *src = dsum + (size_t)q * P + origin;
 #pragma unroll
-            for (int j = 0; j < 2; ++j)
-                if (rel[j] >= 0) cp_async16(shell0 + (unsigned)(r * SHELL + j * THREADS) * 16u, src + rel[j]);
+            for (int k = 0; k < BR; ++k) {
+                const float4 *src = (k ? dsum2 : dsum) + (size_t)q * P + origin;
+#pragma unroll
+                for (int j = 0; j < 2; ++j)
+                    if (rel[j] >= 0) cp_async16(shell0 + (unsigned)((r * BR + k) * SHELL + j * THREADS) * 16u, src + rel[j]);
+            }
             if (active) {
                 cp_async16(mine0 + (unsigned)(r * SURFACE) * 16u, gx + (size_t)q * P + c);
                 if (NORM) cp_async16(mine0 + (unsigned)((RING + r) * SURFACE) * 16u, x + (size_t)q * P + c);
@@ -902,12 +944,13 @@ __global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict
         asm volatile("cp.async.wait_group 1;" ::: "memory");
         __syncthreads();  // quad q has landed; the shell of quad q - 1 has been read
         fetch(q + 2, slot == 0 ? 2 : slot - 1);
-        {
-            const float4 *sh = shell + slot * SHELL + base;
+#pragma unroll
+        for (int k = 0; k < BR; ++k) {
+            const float4 *sh = shell + (slot * BR + k) * SHELL + base;
             float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
-            for (int e = 0; e < 9; ++e) s = fma4(wf[e], sh[-(e / 3 - 1) * row - (e % 3 - 1)], s);
-            part[par * 384 + tid] = s;
+            for (int e = 0; e < 9; ++e) s = fma4(wf[k][e], sh[-(e / 3 - 1) * row - (e % 3 - 1)], s);
+            part[(par * BR + k) * 384 + tid] = s;
         }
         if (NORM && tid < 2 * DIRS) {
             const int d = tid >> 1;
@@ -920,9 +963,13 @@ __global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict
                 const float4 xv = mine[(RING + slot) * SURFACE + tid], f = dirs[par][2 * my_dir], e = dirs[par][2 * my_dir + 1];
                 acc.x += fmaf(e.x, xv.x, f.x), acc.y += fmaf(e.y, xv.y, f.y), acc.z += fmaf(e.z, xv.z, f.z), acc.w += fmaf(e.w, xv.w, f.w);
             }
-            if (on_z) acc = add4(acc, part[par * 384 + pz]);
-            if (on_y) acc = add4(acc, part[par * 384 + py]);
-            if (on_x) acc = add4(acc, part[par * 384 + px]);
+#pragma unroll
+            for (int k = 0; k < BR; ++k) {
+                const float4 *from = part + (par * BR + k) * 384;
+                if (on_z) acc = add4(acc, from[pz]);
+                if (on_y) acc = add4(acc, from[py]);
+                if (on_x) acc = add4(acc, from[px]);
+            }
             gx[(size_t)q * P + c] = acc;
         }
         slot = slot == RING - 1 ? 0 : slot + 1;
@@ -931,9 +978,8 @@ __global__ void __launch_bounds__(384, 3) quad_border8_k(const float *__restrict
 
 // Block 4: one thread per cell of the region, all 27 taps; sources in the cell's own block carry a zero weight.
 template <bool NORM>
-__global__ void __launch_bounds__(512, 2) quad_border4_k(const float *__restrict__ w, const float4 *__restrict__ dsum, float4 *__restrict__ gx,
-                                                      const float4 *__restrict__ x_il4, const float4 *__restrict__ hterm, int Q, int M,
-                                                      int N, int K, int qpc)
+__global__ void __launch_bounds__(512, 2) quad_border4_k(const float *__restrict__ w, const float4 *dsum, float4 *gx, const float4 *x_il4,
+                                                         const float4 *hterm, int Q, int M, int N, int K, int qpc)
 {
     using T = quadborder::Terms<4>;
     __shared__ float4 terms[NORM ? 2 : 1][2 * T::COUNT];
@@ -988,10 +1034,11 @@ __global__ void __launch_bounds__(512, 2) quad_border4_k(const float *__restrict
             const float4 *src = dsum + (size_t)q * P + origin;
 #pragma unroll
             for (int j = 0; j < SLOTS; ++j)
-                if (tof[j] >= 0) pf[j] = __ldg(src + rel[j]);
-            if (NORM && my_term >= 0) pt = __ldg(hterm + ((size_t)q * ntiles + my_term) * 2 + (tid & 1));
+                if (tof[j] >= 0) pf[j] = src[rel[j]];
+            if (NORM && my_term >= 0) pt = hterm[((size_t)q * ntiles + my_term) * 2 + (tid & 1)];
         }
     };
+    previous_done();
     fetch(q0);
     if (active && q0 < q1) gnext = gx[(size_t)q0 * P + c];
     if (NORM && active && q0 < q1) xnext = x_il4[(size_t)q0 * P + c];
@@ -1025,25 +1072,28 @@ __global__ void __launch_bounds__(512, 2) quad_border4_k(const float *__restrict
 // gradients of gamma and beta, which need no second look at the batch. A thread owns CPT cells and walks the quads. The
 // eight sums of a quad are added in double from the single value on, as in norm_bwd_partial_k (norm.cu). SUB_G: the gradient is
 // g - sub (residual form of the loop).
+// On a small grid the quads are split over the CTAs of a cluster, which add up their gradients of gamma and beta in
+// the order of their ranks (32^3 x 64: with its launch 14.1 us with one CTA for 16 quads, 11.6 with a cluster of eight that starts early).
 template <int CPT, bool SUB_G>
-__global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *__restrict__ x, const float4 *__restrict__ g,
-                                                        const float4 *__restrict__ sub, const float *__restrict__ gamma,
-                                                        const float2 *__restrict__ stats, double2 *__restrict__ partials, int nparts,
-                                                        float *__restrict__ ggamma, float *__restrict__ gbeta, int accumulate, int Q,
-                                                        size_t P)
+__global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *x, const float4 *g, const float4 *sub, const float *gamma, const float2 *stats,
+                                                        double2 *partials, int nparts, float *ggamma, float *gbeta, int accumulate, int Q,
+                                                        int qpc, size_t P)
 {
     constexpr int QB = 16;  // quads between two block-wide sums
     __shared__ double red[QB][8][8];
+    __shared__ float part[2][CPT * 256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const size_t c0 = (size_t)blockIdx.x * (256 * CPT) + tid;
     float gm[CPT], dg[CPT], db[CPT];
+    previous_done();
 #pragma unroll
     for (int k = 0; k < CPT; ++k) {
         gm[k] = c0 + k * 256 < P ? gamma[c0 + k * 256] : 0.0f;
         dg[k] = db[k] = 0.0f;
     }
-    for (int qb = 0; qb < Q; qb += QB) {
-        const int qe = min(Q, qb + QB);
+    const int q0 = blockIdx.y * qpc, q1 = min(Q, q0 + qpc);
+    for (int qb = q0; qb < q1; qb += QB) {
+        const int qe = min(q1, qb + QB);
 #pragma unroll 2
         for (int q = qb; q < qe; ++q) {
             float4 xv[CPT], gv[CPT];
@@ -1063,7 +1113,7 @@ __global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *__restrict
             double v[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
             float2 mr[4];
 #pragma unroll
-            for (int s = 0; s < 4; ++s) mr[s] = __ldg(stats + 4 * q + s);
+            for (int s = 0; s < 4; ++s) mr[s] = stats[4 * q + s];
 #pragma unroll
             for (int k = 0; k < CPT; ++k) {
                 const float xs[4] = {xv[k].x, xv[k].y, xv[k].z, xv[k].w}, gs[4] = {gv[k].x, gv[k].y, gv[k].z, gv[k].w};
@@ -1089,18 +1139,37 @@ __global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *__restrict
         }
         __syncthreads();
     }
+    auto put = [&](size_t c, float *to, float v) {
+        if (c < P) to[c] = accumulate ? to[c] + v : v;
+    };
+    if (gridDim.y == 1) {
 #pragma unroll
-    for (int k = 0; k < CPT; ++k)
-        if (c0 + k * 256 < P) {
-            ggamma[c0 + k * 256] = accumulate ? ggamma[c0 + k * 256] + dg[k] : dg[k];
-            gbeta[c0 + k * 256] = accumulate ? gbeta[c0 + k * 256] + db[k] : db[k];
+        for (int k = 0; k < CPT; ++k) {
+            put(c0 + k * 256, ggamma, dg[k]);
+            put(c0 + k * 256, gbeta, db[k]);
         }
+        return;
+    }
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+#pragma unroll
+    for (int k = 0; k < CPT; ++k) {
+        part[0][k * 256 + tid] = dg[k];
+        part[1][k * 256 + tid] = db[k];
+    }
+    cluster.sync();
+    for (unsigned i = blockIdx.y * 256 + tid; i < 2 * CPT * 256; i += gridDim.y * 256) {
+        float v = 0.0f;
+        for (unsigned r = 0; r < gridDim.y; ++r) v += *cluster.map_shared_rank(&part[0][0] + i, r);
+        put((size_t)blockIdx.x * (256 * CPT) + i % (CPT * 256), i < CPT * 256 ? ggamma : gbeta, v);
+    }
+    cluster.sync();  // nobody leaves while its part is being read
 }
 
 // grid 4 Q: (a, c) / P from the partial sums, in a fixed order
-__global__ void __launch_bounds__(256) quad_norm_ac_k(const double2 *__restrict__ partials, int nparts, float2 *__restrict__ ac, size_t P)
+__global__ void __launch_bounds__(256) quad_norm_ac_k(const double2 *partials, int nparts, float2 *ac, size_t P)
 {
     __shared__ double red[33];
+    previous_done();
     const double2 *ps = partials + (size_t)blockIdx.x * nparts;
     double a = 0.0, c = 0.0;
 #pragma unroll 4
@@ -1116,10 +1185,10 @@ __global__ void __launch_bounds__(256) quad_norm_ac_k(const double2 *__restrict_
 
 // Residual form of the loop, backward: n = norm(h), h' = h + net(n) - n. gn = gradient that the step sent back to n;
 // out = gu + rstd ((gn - gu) gamma - a - xhat c), gu = gradient of h'. out may be gu.
-__global__ void __launch_bounds__(256) quad_norm_residual_apply_k(const float4 *__restrict__ h, const float4 *__restrict__ gn, const float4 *gu,
-                                                                  const float *__restrict__ gamma, const float2 *__restrict__ stats,
-                                                                  const float2 *__restrict__ ac, float4 *out, size_t P, unsigned parts)
+__global__ void __launch_bounds__(256) quad_norm_residual_apply_k(const float4 *h, const float4 *gn, const float4 *gu, const float *gamma,
+                                                                  const float2 *stats, const float2 *ac, float4 *out, size_t P, unsigned parts)
 {
+    previous_done();
     const unsigned q = blockIdx.x / parts;
     const size_t c = (size_t)(blockIdx.x - q * parts) * 256 + threadIdx.x;
     if (c >= P) return;
@@ -1130,7 +1199,7 @@ __global__ void __launch_bounds__(256) quad_norm_residual_apply_k(const float4 *
     float o[4];
 #pragma unroll
     for (int s = 0; s < 4; ++s) {
-        const float2 mr = __ldg(stats + 4 * q + s), k = __ldg(ac + 4 * q + s);
+        const float2 mr = stats[4 * q + s], k = ac[4 * q + s];
         const float xh = (hs[s] - mr.x) * mr.y;
         o[s] = us[s] + mr.y * ((ns[s] - us[s]) * gm - k.x - xh * k.y);
     }
@@ -1141,9 +1210,8 @@ __global__ void __launch_bounds__(256) quad_norm_residual_apply_k(const float4 *
 // null only the sums of h are taken (the statistics of the loop's first input). As in norm_residual_combine_k and
 // norm_partial_stats_k (norm.cu) four x-neighbours are added in float, everything above in double: neighbouring lanes hold
 // neighbouring cells, and of the sums that four lanes then share each goes on with one sample's. P is a multiple of 512.
-__global__ void __launch_bounds__(256) quad_residual_combine_k(const float4 *__restrict__ h, const float4 *y, const float *__restrict__ gamma,
-                                                               const float *__restrict__ beta, const float2 *__restrict__ stats, float4 *out,
-                                                               double2 *__restrict__ partials, unsigned nparts, size_t P)
+__global__ void __launch_bounds__(256) quad_residual_combine_k(const float4 *h, const float4 *y, const float *gamma, const float *beta,
+                                                               const float2 *stats, float4 *out, double2 *partials, unsigned nparts, size_t P)
 {
     constexpr int CPT = 4;
     __shared__ double red[8][8];
@@ -1151,9 +1219,10 @@ __global__ void __launch_bounds__(256) quad_residual_combine_k(const float4 *__r
     const unsigned q = blockIdx.x / nparts, part = blockIdx.x - q * nparts;
     const size_t c0 = (size_t)part * (256 * CPT) + tid;
     float2 mr[4];
+    previous_done();
     if (y) {
 #pragma unroll
-        for (int s = 0; s < 4; ++s) mr[s] = __ldg(stats + 4 * q + s);
+        for (int s = 0; s < 4; ++s) mr[s] = stats[4 * q + s];
     }
     float o[CPT][4];
     {
@@ -1261,7 +1330,7 @@ static int launch_reverse_sub(const QuadRevParams &p, unsigned ctas, int act, cu
 int launch_quad_reverse(const QuadReverse &a, int act, cudaStream_t st)
 {
     QuadRevParams p{};
-    p.packed = a.packed_t; p.g = a.g; p.raw = a.raw; p.stats = a.stats; p.ac = a.ac; p.h = a.h;
+    p.packed = a.packed_t; p.params_old = a.params_old; p.g = a.g; p.raw = a.raw; p.stats = a.stats; p.ac = a.ac; p.h = a.h;
     p.wsum = a.wsum; p.tile_stats = a.tile_stats; p.hterm = a.hterm;
     p.delta = a.delta; p.dsum = a.dsum; p.gx = a.gx; p.dsq = a.dsq;
     p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;
@@ -1348,44 +1417,47 @@ int launch_quad_finish(const float *gpk, float *gw, float *gb, float *gs, const 
     const unsigned long long n = grads + (il ? (unsigned long long)parts * ((B + 3) / 4) : 0);
     if (n >= 1ull << 31) return GN_ERR_UNSUPPORTED;
     const float4 *const i4 = reinterpret_cast<const float4 *>(il);
-    if (block == 8) quad_finish_k<8><<<(unsigned)n, 256, 0, st>>>(gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, branches, grads, parts);
-    else quad_finish_k<4><<<(unsigned)n, 256, 0, st>>>(gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, branches, grads, parts);
+    if (block == 8) launch_after(quad_finish_k<8>, (unsigned)n, 256, 0, st, gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, branches, grads, parts);
+    else launch_after(quad_finish_k<4>, (unsigned)n, 256, 0, st, gpk, gw, gb, gs, i4, x, B, M, N, K, chunks, branches, grads, parts);
     return check_launch("quad_finish");
 }
 
-template <bool NORM>
-static int launch_border(const float *w, size_t tap, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K, int Q,
-                         int block, cudaStream_t st)
+template <bool NORM, int BR>
+static int launch_border(const float *w, const float *dsum, const float *dsum2, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
+                         int Q, int block, cudaStream_t st)
 {
     const long long nb = regions_of(M, N, K);
-    const int ctas_per_sm = block == 8 ? 3 : 2;
+    const int ctas_per_sm = block == 8 && BR == 1 ? 3 : 2;
     const int chunks = pick_batch_chunks_balanced(nb, Q, ctas_per_sm, 4.0, 32);
     const int qpc = (Q + chunks - 1) / chunks;
     dim3 grid((unsigned)nb, (unsigned)((Q + qpc - 1) / qpc));
     static unsigned long long done[2] = {};
-    const float4 *const d4 = reinterpret_cast<const float4 *>(dsum), *const x4 = reinterpret_cast<const float4 *>(x_il4);
+    const float4 *const d4 = reinterpret_cast<const float4 *>(dsum), *const e4 = reinterpret_cast<const float4 *>(dsum2);
+    const float4 *const x4 = reinterpret_cast<const float4 *>(x_il4);
     float4 *const g4 = reinterpret_cast<float4 *>(gx);
     if (block == 8) {
-        constexpr int smem = (quadborder::RING * (quadborder::SHELL + (NORM ? 2 : 1) * quadborder::SURFACE) + 2 * 3 * 128) * 16;
-        const int rc = smem_once(quad_border8_k<NORM>, smem, &done[0], "cudaFuncSetAttribute(quad_border8_k)");
+        constexpr int smem = (quadborder::RING * (BR * quadborder::SHELL + (NORM ? 2 : 1) * quadborder::SURFACE) + 2 * BR * 3 * 128) * 16;
+        const int rc = smem_once(quad_border8_k<NORM, BR>, smem, &done[0], "cudaFuncSetAttribute(quad_border8_k)");
         if (rc != GN_OK) return rc;
-        launch_after(quad_border8_k<NORM>, grid, 384, smem, st, w, tap, d4, g4, x4, hterm, Q, M, N, K, qpc);
+        launch_after(quad_border8_k<NORM, BR>, grid, 384, smem, st, w, (size_t)M * N * K, d4, e4, g4, x4, hterm, Q, M, N, K, qpc);
     } else {
         constexpr int smem = 2 * quadborder::TS * 16;
         const int rc = smem_once(quad_border4_k<NORM>, smem, &done[1], "cudaFuncSetAttribute(quad_border4_k)");
         if (rc != GN_OK) return rc;
-        quad_border4_k<NORM><<<grid, 512, smem, st>>>(w, d4, g4, x4, hterm, Q, M, N, K, qpc);
+        launch_after(quad_border4_k<NORM>, grid, 512, smem, st, w, d4, g4, x4, hterm, Q, M, N, K, qpc);
     }
     return check_launch("quad_border");
 }
 
-int launch_quad_border(const float *w, int branches, const float *dsum, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
+int launch_quad_border(const float *w, const float *dsum, const float *dsum2, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
                        int Q, int block, cudaStream_t st)
 {
-    const size_t tap = (size_t)M * N * K * branches;
-    if (branches > 1 && block != 8) return GN_ERR_UNSUPPORTED;
-    return hterm ? launch_border<true>(w, tap, dsum, gx, x_il4, hterm, M, N, K, Q, block, st)
-                 : launch_border<false>(w, tap, dsum, gx, nullptr, nullptr, M, N, K, Q, block, st);
+    if (dsum2) {
+        if (block != 8 || hterm) return GN_ERR_UNSUPPORTED;
+        return launch_border<false, 2>(w, dsum, dsum2, gx, nullptr, nullptr, M, N, K, Q, block, st);
+    }
+    return hterm ? launch_border<true, 1>(w, dsum, nullptr, gx, x_il4, hterm, M, N, K, Q, block, st)
+                 : launch_border<false, 1>(w, dsum, nullptr, gx, nullptr, nullptr, M, N, K, Q, block, st);
 }
 
 int quad_norm_parts(long long P)
@@ -1400,13 +1472,19 @@ int launch_quad_norm_sums(const float *x, const float *g, const float *sub, cons
     const int nparts = quad_norm_parts(P);
     const float4 *x4 = reinterpret_cast<const float4 *>(x), *g4 = reinterpret_cast<const float4 *>(g), *s4 = reinterpret_cast<const float4 *>(sub);
     const bool wide = (long long)nparts * 256 < P;
-#define SUMS_(C, S) quad_norm_sums_k<C, S><<<nparts, 256, 0, st>>>(x4, g4, s4, gamma, stats, partials, nparts, ggamma, gbeta, accumulate, Q, (size_t)P)
+    // enough CTAs for a few per SM, by splitting the quads where the cells do not give them
+    int chunks = 1;
+    while (chunks < 8 && 2 * chunks <= Q && (long long)nparts * chunks < 4LL * sm_count()) chunks *= 2;
+    const int qpc = (Q + chunks - 1) / chunks;
+#define SUMS_(C, S)                                                                                                                     \
+    launch_after_cluster(chunks, quad_norm_sums_k<C, S>, dim3(nparts, chunks), 256, 0, st, x4, g4, s4, gamma, stats, partials, nparts, \
+                         ggamma, gbeta, accumulate, Q, qpc, (size_t)P)
     if (wide && sub) SUMS_(4, true);
     else if (wide) SUMS_(4, false);
     else if (sub) SUMS_(1, true);
     else SUMS_(1, false);
 #undef SUMS_
-    quad_norm_ac_k<<<4 * Q, 256, 0, st>>>(partials, nparts, ac, (size_t)P);
+    launch_after(quad_norm_ac_k, 4 * Q, 256, 0, st, partials, nparts, ac, (size_t)P);
     return check_launch("quad_norm_sums");
 }
 
@@ -1415,8 +1493,8 @@ int launch_quad_norm_residual_apply(const float *h, const float *gn, const float
 {
     const unsigned parts = (unsigned)((P + 255) / 256);
     if ((unsigned long long)parts * Q >= 1ull << 31) return GN_ERR_UNSUPPORTED;
-    quad_norm_residual_apply_k<<<parts * (unsigned)Q, 256, 0, st>>>(reinterpret_cast<const float4 *>(h), reinterpret_cast<const float4 *>(gn),
-                                                     reinterpret_cast<const float4 *>(gu), gamma, stats, ac, reinterpret_cast<float4 *>(out), (size_t)P, parts);
+    launch_after(quad_norm_residual_apply_k, parts * (unsigned)Q, 256, 0, st, reinterpret_cast<const float4 *>(h), reinterpret_cast<const float4 *>(gn),
+                 reinterpret_cast<const float4 *>(gu), gamma, stats, ac, reinterpret_cast<float4 *>(out), (size_t)P, parts);
     return check_launch("quad_norm_residual_apply");
 }
 
@@ -1427,8 +1505,8 @@ int launch_quad_residual_combine(const float *h, const float *y, const float *ga
 {
     const unsigned parts = (unsigned)quad_combine_parts(P);
     if ((unsigned long long)parts * Q >= 1ull << 31) return GN_ERR_UNSUPPORTED;
-    quad_residual_combine_k<<<parts * (unsigned)Q, 256, 0, st>>>(reinterpret_cast<const float4 *>(h), reinterpret_cast<const float4 *>(y), gamma, beta, stats,
-                                                  reinterpret_cast<float4 *>(out), partials, parts, (size_t)P);
+    launch_after(quad_residual_combine_k, parts * (unsigned)Q, 256, 0, st, reinterpret_cast<const float4 *>(h), reinterpret_cast<const float4 *>(y), gamma,
+                 beta, stats, reinterpret_cast<float4 *>(out), partials, parts, (size_t)P);
     return check_launch("quad_residual_combine");
 }
 

@@ -71,6 +71,7 @@ struct QuadGateParams {
     float *save_v, *save_g, *save_x;  // SAVE: [inner] IL4 tensors: the two pre-activations, the activations that went in
     int *error_flag;
     int M, N, K, Q, inner;
+    int params_old;         // the kernel before this one did not write packed or gbt
     long long nitems;
 };
 
@@ -129,9 +130,13 @@ __global__ void __launch_bounds__(256, 1) quad_gated_fwd_k(const __grid_constant
         if (spins >= kSpinLimit || !mbar_wait_bounded(bar0 + 8 * (i % NBUF), (unsigned)(i / NBUF) & 1u, kSpinLimit)) failed = true;
         __syncwarp();
     };
-    if (branch == 0 && role == 0 && lane == 0)
-        for (int i = 0; i < NBUF && i < cnt; ++i) issue(i);
-    __syncwarp();
+    auto begin = [&]() {
+        previous_done();
+        if (branch == 0 && role == 0 && lane == 0)
+            for (int i = 0; i < NBUF && i < cnt; ++i) issue(i);
+        __syncwarp();
+    };
+    if (!p.params_old || cnt == 0) begin();  // else the first region's parameters come first
 
     int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
     for (int i0 = 0; i0 < cnt;) {
@@ -151,6 +156,7 @@ __global__ void __launch_bounds__(256, 1) quad_gated_fwd_k(const __grid_constant
         quad_load_params(p.packed + (branch * regions + blk) * PACK_F, role, lane, tm);
         tmem_wait_st();
         if (FUSE_IN) cp_async_wait_all();
+        if (i0 == 0 && p.params_old) begin();
         tmem_fence_before();
         gate_team_sync(team);
         tmem_fence_after();
@@ -378,9 +384,6 @@ __global__ void __launch_bounds__(256, 1) quad_gated_reverse_k(const QuadGateRev
         fetch_half(stage + HALF, p.hg + t * T4 + corner);
         fetch_half(stage + 2 * HALF, p.x + t * T4 + corner);
     };
-    if (role < cnt) fetch(corner_of(role), p.inner - 1);
-    __syncwarp();
-
     int blk = (int)(n0 / p.Q), q0 = (int)(n0 - (long long)blk * p.Q);
     for (int i0 = 0; i0 < cnt;) {
         const int here = min(cnt - i0, p.Q - q0);
@@ -391,8 +394,13 @@ __global__ void __launch_bounds__(256, 1) quad_gated_reverse_k(const QuadGateRev
             gate_team_sync(team);
             tmem_fence_after();
         }
-        quad_load_params(p.packed + (branch * regions + blk) * PACK_F, role, lane, tm);
+        quad_load_params(p.packed + (branch * regions + blk) * PACK_F, role, lane, tm);  // at least two kernels old
         tmem_wait_st();
+        if (i0 == 0) {
+            previous_done();
+            if (role < cnt) fetch(corner_of(role), p.inner - 1);
+            __syncwarp();
+        }
         tmem_fence_before();
         gate_team_sync(team);
         tmem_fence_after();
@@ -413,12 +421,12 @@ __global__ void __launch_bounds__(256, 1) quad_gated_reverse_k(const QuadGateRev
                         quad_load2(p.raw + own, r, j, zstr, ystr, L.h, y[r]);
                     }
 #pragma unroll
-                    for (int o = 0; o < 4; ++o) gm[r][o] = __ldg(p.gamma + g0 + r * wys + (L.h ? 3 - o : o));
+                    for (int o = 0; o < 4; ++o) gm[r][o] = p.gamma[g0 + r * wys + (L.h ? 3 - o : o)];
                 }
 #pragma unroll
                 for (int s = 0; s < 4; ++s) {
-                    m4[s] = __ldg(p.stats + 4 * q + s);
-                    a4[s] = __ldg(p.ac + 4 * q + s);
+                    m4[s] = p.stats[4 * q + s];
+                    a4[s] = p.ac[4 * q + s];
                 }
 #pragma unroll
                 for (int k2 = 0; k2 < 2; ++k2) {
@@ -549,7 +557,7 @@ static int launch_fwd_one(const CUtensorMap &map, const QuadGateParams &p, cudaS
     static unsigned long long done = 0;
     const int rc = set_smem(quad_gated_fwd_k<ACT, FUSE_IN, SAVE>, smem, &done);
     if (rc != GN_OK) return rc;
-    quad_gated_fwd_k<ACT, FUSE_IN, SAVE><<<gate_ctas(p.nitems), 256, smem, st>>>(map, p);
+    launch_after(quad_gated_fwd_k<ACT, FUSE_IN, SAVE>, gate_ctas(p.nitems), 256, smem, st, map, p);
     return check_launch("quad_gated_fwd");
 }
 template <int ACT>
@@ -566,7 +574,7 @@ int launch_quad_gated_fwd(const QuadGated &a, int act, cudaStream_t st)
     const int rc = quad_make_map(&map, a.in_il4, a.M, a.N, a.K, a.Q, 8);
     if (rc != GN_OK) return rc;
     QuadGateParams p{};
-    p.packed = a.packed; p.gbt = a.gbt; p.in_stats = a.in_stats; p.out_partials = a.out_partials; p.nparts = a.nparts; p.y = a.out_il4;
+    p.packed = a.packed; p.params_old = a.params_old; p.gbt = a.gbt; p.in_stats = a.in_stats; p.out_partials = a.out_partials; p.nparts = a.nparts; p.y = a.out_il4;
     p.save_v = a.hv; p.save_g = a.hg; p.save_x = a.x;
     p.error_flag = device_status_ptr();
     p.M = a.M; p.N = a.N; p.K = a.K; p.Q = a.Q; p.inner = a.inner;
@@ -585,7 +593,7 @@ static int launch_rev_act(const QuadGateRevParams &p, cudaStream_t st)
     static unsigned long long done = 0;
     const int rc = set_smem(quad_gated_reverse_k<ACT>, quadgate::REV_SMEM, &done);
     if (rc != GN_OK) return rc;
-    quad_gated_reverse_k<ACT><<<gate_ctas(p.nitems), 256, quadgate::REV_SMEM, st>>>(p);
+    launch_after(quad_gated_reverse_k<ACT>, gate_ctas(p.nitems), 256, quadgate::REV_SMEM, st, p);
     return check_launch("quad_gated_reverse");
 }
 
