@@ -389,17 +389,20 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
 // 2 x 2 x 4 patches of the other kernels get, but those would need their 432 sums in tensor memory, and reading, adding to
 // and writing back sums there was 3 to 4 times slower than this (128^3, two inner iterations, batch 32: 0.77 - 0.97 ms).
 // The step's input tile arrives by bulk tensor copy and is normalised in place; activations between iterations are rebuilt
-// from it and the pre-activations. Block 8: two tiles take turns over the iterations, one barrier each; block 4: one tile,
-// updated in place between two barriers. Deltas and pre-activations arrive an iteration ahead, each thread its own.
+// from it and the pre-activations. Two tiles take turns over the iterations, one barrier each (block 4 with one tile, updated in
+// place between two barriers: 39.9 ms for 64^3 x 128, 8 x 16 with gradients, now 38.8). Deltas and pre-activations arrive
+// an iteration ahead, what else a quad needs a quad ahead, each thread its own (128^3 x 32, 2 x 16: 30.35 -> 30.05 ms).
 namespace quadwg {
 constexpr int CTAS = 2;  // per SM: 255 registers (three with 168 spill, and are no faster)
 constexpr int THREADS = 128, OWN = 4 * THREADS * 16;  // bytes of one staging area: a thread's four cells
 constexpr int GRAD_F = (27 * 4 + 8) * THREADS;        // floats per region and chunk: weights, biases, scales
 template <int SUB>
 struct Lay {
-    static constexpr int NT = SUB == 8 ? 2 : 1;
+    static constexpr int NT = 2;  // tiles
     static constexpr int TILE = (QuadGeo<SUB>::BUF_BYTES + 127) / 128 * 128;
-    static constexpr int GB = NT * TILE + 3 * OWN;  // normalise-on-load: the region's (gamma, beta) table
+    static constexpr int DSQ = NT * TILE + 3 * OWN;  // a quad's terms of the scale gradient, each thread its own four
+    static constexpr int IST = DSQ + THREADS * 16;   // and, each warp its own copy, its statistics
+    static constexpr int GB = IST + THREADS;         // normalise-on-load: the region's (gamma, beta) table
     static constexpr int NSTAT = (SUB == 8 ? 1 : 8) * QS_COUNT;  // per-block normalisation, there: two iterations' statistics
     static constexpr int smem(bool fuse, bool norm) { return GB + (fuse ? QuadGeo<SUB>::CELLS * 8 : 0) + (norm ? 2 * NSTAT * 16 : 0); }
 };
@@ -471,6 +474,12 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
     const size_t zs = (size_t)p.N * p.K;
     const int q0 = blockIdx.y * p.qpc, q1 = min(p.Q, q0 + p.qpc);
     bool failed = false;
+    constexpr int STEPS = (G::CELLS + THREADS - 1) / THREADS;
+    unsigned halo = 0;  // bit c: cell c * THREADS + tid of the tile is a halo cell
+    for (int c = 0; c < STEPS; ++c) {
+        const int l = (c * THREADS + tid) % (SUB == 8 ? 1000 : 216), x = l % G::SIDE, y = l / G::SIDE % G::SIDE, z = l / G::SIDE / G::SIDE;
+        if (z == 0 || z == G::SIDE - 1 || y == 0 || y == G::SIDE - 1 || x == 0 || x == G::SIDE - 1) halo |= 1u << c;
+    }
 
     auto issue = [&](int q, int buf) {
         const unsigned tile = tiles + buf * Y::TILE, bar = bar0 + 8 * buf;
@@ -495,6 +504,17 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
             cp_async16(stats0 + buf * (Y::NSTAT * 16) + tid * 16, p.tile_stats + (((size_t)it * p.Q + q) * gridDim.x + blk) * Y::NSTAT + tid);
     };
     auto at = [&](const float *t, int q, int it) { return t + (size_t)it * T4 + ((size_t)q * P + g0) * 4; };
+    // what a quad starts with, a quad ahead: its scale terms and statistics
+    const unsigned my_dsq = tiles + Y::DSQ + tid * 16, my_ist = tiles + Y::IST + (tid >> 5) * 32;
+    auto fetch_quad = [&](int q) {
+        if (!GATED) {
+            const float *s = p.dsq + (size_t)q * P + g0;
+#pragma unroll
+            for (int n = 0; n < 4; ++n) cp_async4(my_dsq + 4 * n, s + (n >> 1) * zs + (n & 1) * (size_t)p.K);
+        }
+        // two lanes: asynchronous copies of one address by all lanes are a request each (128^3: the step three times as long)
+        if (FUSE_IN && (tid & 31) < 2) cp_async16(my_ist + (tid & 31) * 16, p.in_stats + 4 * q + (tid & 31) * 2);
+    };
 
     // sums: sg[dy = 0 at ry = 0, dy = 1 at ry = 3][dz][a][c], sp[ry = 1, 2][dz][a][c] = (dy = 0, dy = 1)
     float sg[2][2][3][3];
@@ -524,6 +544,7 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
     }
     previous_done();
     if (tid == 0) issue(q0, 0);
+    fetch_quad(q0);
     const float *const delta = GATED && blockIdx.z ? p.delta2 : p.delta;
     fetch(stage_d, at(delta, q0, 0));
     fetch_stats(0, q0, 0);
@@ -531,15 +552,11 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
     const unsigned own0 = (unsigned)(T.cell0 + G::PLANE + G::ROW + 1) * 16u;
 
     for (int q = q0; q < q1; ++q) {
-        if (!GATED) {  // scale terms of this quad
-            const float *s = p.dsq + (size_t)q * P + g0;
-#pragma unroll
-            for (int dz = 0; dz < 2; ++dz) ds[dz] = fadd2(ds[dz], pack2(s[dz * zs], s[dz * zs + p.K]));
-        }
         if (!mbar_wait_bounded(bar0 + 8 * buf_x, (landed >> buf_x) & 1u, kSpin)) failed = true;
         landed ^= 1u << buf_x;
-        const bool two = NT == 2 && p.inner > 1;
-        if (NORM) cp_async_wait_all();  // the first iteration's statistics
+        const bool two = p.inner > 1;
+        cp_async_wait_all();  // the quad's statistics, the first iteration's
+        if (FUSE_IN) __syncwarp();
         if (two || NORM) __syncthreads();  // nobody reads the other tile any more: it gets the new halo
         float4 pivot = make_float4(0.f, 0.f, 0.f, 0.f);
         if (NORM) pivot = lds128(stats0 + buf_d * (Y::NSTAT * 16) + my_tile + QS_MEAN * 16);
@@ -547,15 +564,13 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
             const unsigned tile = tiles + buf_x * Y::TILE, other = tiles + (buf_x ^ 1) * Y::TILE;
             u64 na[2], nb[2];
             if (FUSE_IN) {
-                float2 mr[4];
-#pragma unroll
-                for (int s = 0; s < 4; ++s) mr[s] = p.in_stats[4 * q + s];
-                na[0] = pack2(mr[0].y, mr[1].y);
-                na[1] = pack2(mr[2].y, mr[3].y);
-                nb[0] = pack2(-mr[0].x, -mr[1].x);
-                nb[1] = pack2(-mr[2].x, -mr[3].x);
+                const float4 m01 = lds128(my_ist), m23 = lds128(my_ist + 16);
+                na[0] = pack2(m01.y, m01.w);
+                na[1] = pack2(m23.y, m23.w);
+                nb[0] = pack2(-m01.x, -m01.z);
+                nb[1] = pack2(-m23.x, -m23.z);
             }
-            constexpr int STEPS = (G::CELLS + THREADS - 1) / THREADS, BATCH = SUB == 8 ? 8 : 7;
+            constexpr int BATCH = SUB == 8 ? 8 : 7;
 #pragma unroll 1
             for (int c0 = 0; c0 < STEPS; c0 += BATCH) {
                 u64 v[BATCH][2];
@@ -585,11 +600,7 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                             v[c][1] = ffma2r(m1, pack2(-1.0f, -1.0f), v[c][1]);
                             sts128u(tile + i * 16, v[c][0], v[c][1]);
                         }
-                        if (two) {
-                            int cz, cy, cx;
-                            G::cell(i, cz, cy, cx);
-                            if (cz == 0 || cz == 9 || cy == 0 || cy == 9 || cx == 0 || cx == 9) sts128u(other + i * 16, v[c][0], v[c][1]);
-                        }
+                        if (two && (halo >> (c0 + c) & 1)) sts128u(other + i * 16, v[c][0], v[c][1]);
                     }
                 }
             }
@@ -615,9 +626,8 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                 shift = lds128(st + QS_MEAN * 16);
                 shift.x -= pivot.x, shift.y -= pivot.y, shift.z -= pivot.z, shift.w -= pivot.w;
             }
-            // block 8: the activations of iteration t + 1 -> the other tile; block 4: those of iteration t, in place
-            if (NT == 2 ? !last : t > 0) {
-                const unsigned to = NT == 2 ? tiles + (buf_x ^ 1) * Y::TILE : tile;
+            if (!last) {  // the activations of iteration t + 1 -> the other tile
+                const unsigned to = tiles + (buf_x ^ 1) * Y::TILE;
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
                     const unsigned c = own0 + (unsigned)((n >> 1) * G::PLANE + (n & 1) * G::ROW) * 16u;
@@ -632,17 +642,24 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                     sts128u(to + c, act_residual2<ACT>(h0, sc, x0), act_residual2<ACT>(h1, sc, x1));
                 }
             }
-            if (NT == 1 && t > 0) __syncthreads();  // the tile is complete
+            if (t == 0) {
+                if (!GATED) {
+                    const float4 v = lds128(my_dsq);
+                    ds[0] = fadd2(ds[0], pack2(v.x, v.y));
+                    ds[1] = fadd2(ds[1], pack2(v.z, v.w));
+                }
+                if (q + 1 < q1) fetch_quad(q + 1);  // every warp has passed a barrier since it read the quad's statistics
+            }
             // the next iteration's data
             if (!last) {
                 fetch(stage_d + (buf_d ^ 1) * OWN, at(delta, q, t + 1));
                 fetch_stats(buf_d ^ 1, q, t + 1);
-                if (NT == 1 || t + 2 < p.inner) fetch(stage_h, at(p.h, q, NT == 2 ? t + 1 : t));
+                if (t + 2 < p.inner) fetch(stage_h, at(p.h, q, t + 1));
             } else if (q + 1 < q1) {
                 fetch(stage_d + (buf_d ^ 1) * OWN, at(delta, q + 1, 0));
                 fetch_stats(buf_d ^ 1, q + 1, 0);
-                if (NT == 2 && p.inner > 1) fetch(stage_h, at(p.h, q + 1, 0));
-                if (NT == 2 && tid == 0) issue(q + 1, buf_x ^ 1);
+                if (p.inner > 1) fetch(stage_h, at(p.h, q + 1, 0));
+                if (tid == 0) issue(q + 1, buf_x ^ 1);
             }
 #pragma unroll
             for (int dz = 0; dz < 2; ++dz) {
@@ -682,12 +699,8 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                             }
                         }
                     }
-            if (NT == 2) buf_x ^= 1;
+            buf_x ^= 1;
             buf_d ^= 1;
-        }
-        if (NT == 1 && q + 1 < q1) {
-            __syncthreads();
-            if (tid == 0) issue(q + 1, 0);
         }
     }
     // ---- sums -> this chunk's part: [tap][n] then [bias | scale][n], 128 threads each
