@@ -216,9 +216,23 @@ int launch_quad_wgrad(const QuadWgrad &a, int act, cudaStream_t st);
 // gradients of the parameters out of gpk and, with il, il (IL4) -> x [B, P]
 int launch_quad_finish(const float *gpk, float *gw, float *gb, float *gs, const float *il, float *x, int B, int M, int N, int K, int block,
                        int branches, cudaStream_t st);
-// dsum2: of the gate, w is then [27][2][P]; or nullptr. hterm (from launch_quad_reverse), x_il4 (the step's input): per-block normalisation, or nullptr
-int launch_quad_border(const float *w, const float *dsum, const float *dsum2, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
-                       int Q, int block, cudaStream_t st);
+struct QuadBorder {
+    const float *w;            // dsum2: [27][2][P], else [27][P]
+    const float *dsum, *dsum2; // from launch_quad_reverse; dsum2: of the gate, block 8, or nullptr
+    float *gx;                 // added to
+    const float *x_il4;        // with hterm: the step's input; with gamma: what the norm normalised
+    const float4 *hterm;       // per-block normalisation (launch_quad_reverse), or nullptr
+    // with gamma (block 8, no hterm): the sums of launch_quad_norm_sums over the finished gx as well; arguments as there
+    const float *gamma;
+    const float2 *stats;
+    double2 *partials;         // [4 Q][regions]
+    float *ggamma, *gbeta;
+    float2 *ac;
+    int accumulate;
+    int M, N, K, Q, block;
+};
+bool quad_border_takes_sums(int M, int N, int K, int block);
+int launch_quad_border(const QuadBorder &a, cudaStream_t st);
 int quad_norm_parts(long long P);
 int launch_quad_norm_sums(const float *x, const float *g, const float *sub, const float *gamma, const float2 *stats, double2 *partials,
                           float *ggamma, float *gbeta, int accumulate, float2 *ac, int Q, long long P, cudaStream_t st);

@@ -240,6 +240,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
     cudaStream_t st = (cudaStream_t)stream;
     const float2 *const mr = reinterpret_cast<const float2 *>(stats);
     const int S = 4 * d.Q;
+    const bool with_border = !residual && quad_border_takes_sums(M, N, K, block);
     int cur = 0;
     for (int k = outer - 1; k >= 0; --k) {
         const int kp = nparams > 1 ? k : 0;
@@ -258,7 +259,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
             }
             TRY_(launch_quad_prepare(a, M, N, K, block, st));
         }
-        if (!residual)
+        if (!residual && (first || !with_border))  // else taken with the border of the step after
             TRY_(launch_quad_norm_sums(outs[k], w.g[cur], nullptr, gamma, mr + (size_t)k * S, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
         float *const h = kept ? stashes[k] : w.replay;
         if (!kept) {
@@ -285,7 +286,14 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
         g.M = M; g.N = N; g.K = K; g.Q = d.Q; g.inner = inner; g.block = block;
         TRY_(launch_quad_wgrad(g, act, st));
         if (nparams > 1 && k > 0) TRY_(launch_quad_finish(w.gpk, gw[kp], gb[kp], gs[kp], nullptr, nullptr, B, M, N, K, block, 1, st));
-        TRY_(launch_quad_border(weights[kp], w.dsum, nullptr, w.g[cur ^ 1], nullptr, nullptr, M, N, K, d.Q, block, st));
+        QuadBorder o{};
+        o.w = weights[kp]; o.dsum = w.dsum; o.gx = w.g[cur ^ 1];
+        if (with_border && k > 0) {  // with the sums of the norm that made this step's input
+            o.x_il4 = in; o.stats = in_stats; o.gamma = gamma; o.partials = w.partials; o.ggamma = ggamma; o.gbeta = gbeta; o.ac = w.ac;
+            o.accumulate = 1;
+        }
+        o.M = M; o.N = N; o.K = K; o.Q = d.Q; o.block = block;
+        TRY_(launch_quad_border(o, st));
         if (residual) {
             TRY_(launch_quad_norm_sums(in, w.g[cur ^ 1], w.g[cur], gamma, in_stats, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
             TRY_(launch_quad_norm_residual_apply(in, w.g[cur ^ 1], w.g[cur], gamma, in_stats, w.ac, w.g[cur], d.Q, d.P, st));
@@ -351,13 +359,15 @@ GN_API int gn_gated_loop_backward_f32(const float *weight, const float *bias, co
         a.x = gy; a.il = w.g[0]; a.B = B; a.gradient = true;
         TRY_(launch_quad_prepare(a, M, N, K, 8, st));
     }
+    const bool with_border = quad_border_takes_sums(M, N, K, 8);
     float *const delta_v = w.delta, *const delta_g = w.delta + inner * d.T4, *const dsum_v = w.dsum, *const dsum_g = w.dsum + d.T4;
     int cur = 0;
     for (int k = outer - 1; k >= 0; --k, cur ^= 1) {
         const bool first = k == outer - 1;
         const float *in = k ? outs[k - 1] : x_il4;
         const float2 *in_stats = k ? mr + (size_t)(k - 1) * S : nullptr;
-        TRY_(launch_quad_norm_sums(outs[k], w.g[cur], nullptr, gamma, mr + (size_t)k * S, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
+        if (first || !with_border)  // else taken with the border of the step after
+            TRY_(launch_quad_norm_sums(outs[k], w.g[cur], nullptr, gamma, mr + (size_t)k * S, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
         float *kept = stashes ? stashes[k] : nullptr;
         if (!kept) {
             // the step's output is computed once more, into the buffer that receives the gradient afterwards
@@ -376,7 +386,14 @@ GN_API int gn_gated_loop_backward_f32(const float *weight, const float *bias, co
         g.accumulate = !first;
         g.M = M; g.N = N; g.K = K; g.Q = d.Q; g.inner = inner; g.block = 8;
         TRY_(launch_quad_wgrad(g, act, st));
-        TRY_(launch_quad_border(weight, dsum_v, dsum_g, w.g[cur ^ 1], nullptr, nullptr, M, N, K, d.Q, 8, st));
+        QuadBorder o{};
+        o.w = weight; o.dsum = dsum_v; o.dsum2 = dsum_g; o.gx = w.g[cur ^ 1];
+        if (with_border && k > 0) {  // with the sums of the norm that made this step's input
+            o.x_il4 = in; o.stats = in_stats; o.gamma = gamma; o.partials = w.partials; o.ggamma = ggamma; o.gbeta = gbeta; o.ac = w.ac;
+            o.accumulate = 1;
+        }
+        o.M = M; o.N = N; o.K = K; o.Q = d.Q; o.block = 8;
+        TRY_(launch_quad_border(o, st));
     }
     return launch_quad_finish(w.gpk, gw, gb, nullptr, w.g[cur], gx, B, M, N, K, 8, 2, st);
 }

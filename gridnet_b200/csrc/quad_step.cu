@@ -196,7 +196,10 @@ GN_API int gn_step_backward_kept_f32(const float *w, const float *b, const float
     g.in_il4 = k.x; g.delta = ws.delta; g.h = k.h; g.scale = s; g.dsq = ws.dsq; g.gpk = ws.gpk; g.tile_stats = k.stats;
     g.M = M; g.N = N; g.K = K; g.Q = d.Q; g.inner = inner; g.block = block;
     TRY_(launch_quad_wgrad(g, act, st));
-    TRY_(launch_quad_border(w, ws.dsum, nullptr, ws.gout, k.x, ws.hterm, M, N, K, d.Q, block, st));
+    QuadBorder o{};
+    o.w = w; o.dsum = ws.dsum; o.gx = ws.gout; o.x_il4 = k.x; o.hterm = ws.hterm;
+    o.M = M; o.N = N; o.K = K; o.Q = d.Q; o.block = block;
+    TRY_(launch_quad_border(o, st));
     return launch_quad_finish(ws.gpk, gw, gb, gs, ws.gout, gx, B, M, N, K, block, 1, st);
 }
 

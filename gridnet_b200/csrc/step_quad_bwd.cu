@@ -810,7 +810,7 @@ __device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(
 // (quad_reverse_k). The (negated) terms of the surrounding tiles, 3^3 regions or 4^3 blocks of 4, come with the quad.
 namespace quadborder {
 constexpr int TS = 1000;               // block 4: cells of a tile
-constexpr int SHELL = 500, RING = 3;   // block 8: cells of a shell, padded for taps that do not count; quads in flight
+constexpr int SHELL = 500;             // block 8: cells of a shell, padded for taps that do not count
 constexpr int SURFACE = 296, DIRS = 27;
 template <int SUB>
 struct Terms {
@@ -848,22 +848,67 @@ struct Terms {
 };
 }  // namespace quadborder
 
-template <bool NORM, int BR>
-__global__ void __launch_bounds__(384, BR == 1 ? 3 : 2) quad_border8_k(const float *__restrict__ w, size_t branch, const float4 *__restrict__ dsum,
-                                                                       const float4 *__restrict__ dsum2, float4 *__restrict__ gx,
-                                                                       const float4 *__restrict__ x, const float4 *__restrict__ hterm, int Q,
-                                                                       int M, int N, int K, int qpc)
+// SUMS: the sums of the LayerNorm gradient of the step before, whose output is this step's input, in the same pass (see
+// quad_norm_sums_k), since the gradient is in the CTA's hands anyway. A thread has a cell of the surface or
+// the interior, the first 128 a second one; the CTAs of a region are a cluster, which adds up the gradients of gamma and beta
+// in the order of their ranks. When: quad_border_takes_sums.
+enum BorderSums { NO_SUMS, SUMS };
+struct BorderParams {
+    const float *w;
+    const float4 *dsum, *dsum2;  // BR == 2: of the gate
+    float4 *gx;
+    const float4 *x;             // NORM: the step's input; sums: the norm's, IL4
+    const float4 *hterm;         // NORM
+    const float *gamma;
+    const float2 *stats;
+    double2 *partials;           // sums: [4 Q][regions]
+    float *ggamma, *gbeta;
+    int accumulate, Q, M, N, K, qpc;
+};
+// cell s of a region: 0 .. 295 on its surface, then the interior
+__device__ __forceinline__ void border_cell(int s, int &z, int &y, int &x)
+{
+    if (s < 128) {
+        z = (s >> 6) * 7, y = (s >> 3) & 7, x = s & 7;
+    } else if (s < 224) {
+        const int j = s - 128;
+        y = (j / 48) * 7, z = 1 + (j % 48) / 8, x = j & 7;
+    } else if (s < 296) {
+        const int j = s - 224;
+        x = (j / 36) * 7, z = 1 + (j % 36) / 6, y = 1 + j % 6;
+    } else {
+        const int j = s - 296;
+        z = 1 + j / 36, y = 1 + j / 6 % 6, x = 1 + j % 6;
+    }
+}
+namespace quadborder {
+template <bool NORM, int BR, BorderSums S>
+struct Room {
+    static constexpr int RING = S != NO_SUMS && BR == 2 ? 2 : 3;      // quads in flight
+    static constexpr int CELLS = S == NO_SUMS ? SURFACE : 512;        // a quad's grad_x, and as many of each further tensor
+    static constexpr int TENSORS = S == SUMS || NORM ? 2 : 1;
+    static constexpr int BYTES = (RING * (BR * SHELL + TENSORS * CELLS) + 2 * BR * 384) * 16;
+    static constexpr int CTAS = S == NO_SUMS && BR == 1 ? 3 : 2;
+};
+}  // namespace quadborder
+
+template <bool NORM, int BR, BorderSums S>
+__global__ void __launch_bounds__(384, quadborder::Room<NORM, BR, S>::CTAS) quad_border8_k(const BorderParams p)
 {
     using namespace quadborder;
     using T = Terms<8>;
-    constexpr int THREADS = 384;
+    using R = Room<NORM, BR, S>;
+    static_assert(S == NO_SUMS || !NORM, "");
+    constexpr int THREADS = 384, RING = R::RING, CELLS = R::CELLS, AHEAD = RING - 1, QB = 4;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     float4 *const shell = reinterpret_cast<float4 *>(smem_raw);  // [RING][BR][SHELL]
     float4 *const part = shell + RING * BR * SHELL;              // [2][BR][3][128]
-    float4 *const mine = part + 2 * BR * 3 * 128;                // [RING][SURFACE] grad_x, NORM: then x
+    float4 *const mine = part + 2 * BR * 3 * 128;                // [tensor][RING][CELLS] grad_x, then x
     __shared__ float4 terms[NORM ? RING : 1][2 * T::COUNT], dirs[NORM ? 2 : 1][2 * DIRS];
-    const int tid = threadIdx.x;
-    const int nbx = K >> 3, nby = N >> 3;
+    __shared__ double red[S != NO_SUMS ? QB : 1][THREADS / 32][8];
+    __shared__ float4 quad_stats[S != NO_SUMS ? RING : 1][2];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int M = p.M, N = p.N, K = p.K, nbx = K >> 3, nby = N >> 3;
     const unsigned blk = blockIdx.x;
     const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
     const size_t P = (size_t)M * N * K;
@@ -903,29 +948,31 @@ __global__ void __launch_bounds__(384, BR == 1 ? 3 : 2) quad_border8_k(const flo
             const bool ok = owned && nz >= 0 && nz < M && ny >= 0 && ny < N && nx >= 0 && nx < K;
 #pragma unroll
             for (int k = 0; k < BR; ++k)
-                wf[k][e] = ok ? w[((size_t)((dz + 1) * 9 + (dy + 1) * 3 + dx + 1) * BR + k) * branch + ((size_t)nz * N + ny) * K + nx] : 0.0f;
+                wf[k][e] = ok ? p.w[((size_t)((dz + 1) * 9 + (dy + 1) * 3 + dx + 1) * BR + k) * P + ((size_t)nz * N + ny) * K + nx] : 0.0f;
         }
     }
     const int row = axis == 2 ? 8 : 10;
     const int base = axis == 0 ? side * 100 + (u + 1) * 10 + v + 1 : (axis == 1 ? 200 + side * 80 + u * 10 + v + 1 : 360 + side * 64 + u * 8 + v);
-    // role 2: one surface cell
-    int sz = 0, sy = 0, sx = 0;
-    const bool active = tid < SURFACE;
-    if (tid < 128) {
-        sz = (tid >> 6) * 7; sy = (tid >> 3) & 7; sx = tid & 7;
-    } else if (tid < 224) {
-        const int j = tid - 128;
-        sy = (j / 48) * 7; sz = 1 + (j % 48) / 8; sx = j & 7;
-    } else if (active) {
-        const int j = tid - 224;
-        sx = (j / 36) * 7; sz = 1 + (j % 36) / 6; sy = 1 + j % 6;
-    }
-    const size_t c = ((size_t)(bz * 8 + sz) * N + by * 8 + sy) * K + bx * 8 + sx;
-    const bool on_z = sz == 0 || sz == 7, on_y = sy == 0 || sy == 7, on_x = sx == 0 || sx == 7;
+    // role 2: one surface cell; sums: or one of the interior, and the interior's others
+    const bool surface = tid < SURFACE, active = S != NO_SUMS || surface, second = S != NO_SUMS && tid < 512 - THREADS;
+    auto place = [&](int s) {
+        int z, y, x;
+        border_cell(s, z, y, x);
+        return ((size_t)(bz * 8 + z) * N + by * 8 + y) * K + bx * 8 + x;
+    };
+    int sz, sy, sx;
+    border_cell(tid, sz, sy, sx);
+    const size_t c = active ? place(tid) : 0, c2 = second ? place(THREADS + tid) : 0;
+    const bool on_z = surface && (sz == 0 || sz == 7), on_y = surface && (sy == 0 || sy == 7), on_x = surface && (sx == 0 || sx == 7);
     const int pz = (sz / 7) * 64 + sy * 8 + sx, py = 128 + (sy / 7) * 64 + sz * 8 + sx, px = 256 + (sx / 7) * 64 + sz * 8 + sy;
     const int my_dir = ((on_z ? sz / 7 * 2 : 1) * 3 + (on_y ? sy / 7 * 2 : 1)) * 3 + (on_x ? sx / 7 * 2 : 1);
+    float gm[2] = {0.f, 0.f}, dg[2] = {0.f, 0.f}, db[2] = {0.f, 0.f};  // sums: of the two cells
+    if (S != NO_SUMS) {
+        gm[0] = p.gamma[c];
+        if (second) gm[1] = p.gamma[c2];
+    }
 
-    const int q0 = blockIdx.y * qpc, q1 = min(Q, q0 + qpc);
+    const int Q = p.Q, q0 = blockIdx.y * p.qpc, q1 = min(Q, q0 + p.qpc);
     const unsigned shell0 = smem_u32(shell) + tid * 16, mine0 = smem_u32(mine) + tid * 16;
     const int my_term = NORM ? T::tile(tid >> 1, bx, by, bz, M, N, K) : -1;
     if (NORM && tid < 2 * T::COUNT)
@@ -935,28 +982,31 @@ __global__ void __launch_bounds__(384, BR == 1 ? 3 : 2) quad_border8_k(const flo
         if (q < q1) {
 #pragma unroll
             for (int k = 0; k < BR; ++k) {
-                const float4 *src = (k ? dsum2 : dsum) + (size_t)q * P + origin;
+                const float4 *src = (k ? p.dsum2 : p.dsum) + (size_t)q * P + origin;
 #pragma unroll
                 for (int j = 0; j < 2; ++j)
                     if (rel[j] >= 0) cp_async16(shell0 + (unsigned)((r * BR + k) * SHELL + j * THREADS) * 16u, src + rel[j]);
             }
-            if (active) {
-                cp_async16(mine0 + (unsigned)(r * SURFACE) * 16u, gx + (size_t)q * P + c);
-                if (NORM) cp_async16(mine0 + (unsigned)((RING + r) * SURFACE) * 16u, x + (size_t)q * P + c);
+            const float4 *const tensors[2] = {p.gx, p.x};
+#pragma unroll
+            for (int k = 0; k < R::TENSORS; ++k) {
+                if (active) cp_async16(mine0 + (unsigned)((k * RING + r) * CELLS) * 16u, tensors[k] + (size_t)q * P + c);
+                if (second) cp_async16(mine0 + (unsigned)((k * RING + r) * CELLS + THREADS) * 16u, tensors[k] + (size_t)q * P + c2);
             }
-            if (NORM && my_term >= 0) cp_async16(smem_u32(&terms[r][tid]), hterm + ((size_t)q * gridDim.x + my_term) * 2 + (tid & 1));
+            if (NORM && my_term >= 0) cp_async16(smem_u32(&terms[r][tid]), p.hterm + ((size_t)q * gridDim.x + my_term) * 2 + (tid & 1));
+            if (S != NO_SUMS && tid < 2) cp_async16(smem_u32(&quad_stats[r][tid]), p.stats + 4 * q + 2 * tid);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     __syncthreads();  // the shells are zeroed
     previous_done();
-    fetch(q0, 0);
-    fetch(q0 + 1, 1);
+#pragma unroll
+    for (int k = 0; k < AHEAD; ++k) fetch(q0 + k, k);
     for (int q = q0; q < q1; ++q) {
         const int par = q & 1;
-        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        asm volatile("cp.async.wait_group %0;" ::"n"(AHEAD - 1) : "memory");
         __syncthreads();  // quad q has landed; the shell of quad q - 1 has been read
-        fetch(q + 2, slot == 0 ? 2 : slot - 1);
+        fetch(q + AHEAD, slot == 0 ? RING - 1 : slot - 1);
 #pragma unroll
         for (int k = 0; k < BR; ++k) {
             const float4 *sh = shell + (slot * BR + k) * SHELL + base;
@@ -970,10 +1020,11 @@ __global__ void __launch_bounds__(384, BR == 1 ? 3 : 2) quad_border8_k(const flo
             dirs[par][tid] = T::along(&terms[slot][tid & 1], 13, d / 9 - 1, d / 3 % 3 - 1, d % 3 - 1);
         }
         __syncthreads();
-        if (active) {
-            float4 acc = mine[slot * SURFACE + tid];
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (active) acc = mine[slot * CELLS + tid];
+        if (surface) {
             if (NORM) {
-                const float4 xv = mine[(RING + slot) * SURFACE + tid], f = dirs[par][2 * my_dir], e = dirs[par][2 * my_dir + 1];
+                const float4 xv = mine[(RING + slot) * CELLS + tid], f = dirs[par][2 * my_dir], e = dirs[par][2 * my_dir + 1];
                 acc.x += fmaf(e.x, xv.x, f.x), acc.y += fmaf(e.y, xv.y, f.y), acc.z += fmaf(e.z, xv.z, f.z), acc.w += fmaf(e.w, xv.w, f.w);
             }
 #pragma unroll
@@ -983,9 +1034,65 @@ __global__ void __launch_bounds__(384, BR == 1 ? 3 : 2) quad_border8_k(const flo
                 if (on_y) acc = add4(acc, from[py]);
                 if (on_x) acc = add4(acc, from[px]);
             }
-            gx[(size_t)q * P + c] = acc;
+            p.gx[(size_t)q * P + c] = acc;
+        }
+        if constexpr (S != NO_SUMS) {
+            double sum[8] = {0., 0., 0., 0., 0., 0., 0., 0.};
+            const float4 m01 = quad_stats[slot][0], m23 = quad_stats[slot][1];
+            const float mean[4] = {m01.x, m01.z, m23.x, m23.z}, rstd[4] = {m01.y, m01.w, m23.y, m23.w};
+            auto add = [&](int i, float4 g, const float4 *at) {
+                const float4 xv = at[RING * CELLS];
+                const float gs[4] = {g.x, g.y, g.z, g.w}, xs[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+                for (int s = 0; s < 4; ++s) {
+                    const float xh = (xs[s] - mean[s]) * rstd[s], gg = gs[s] * gm[i];
+                    sum[s] += (double)gg;
+                    sum[4 + s] += (double)(gg * xh);
+                    dg[i] = fmaf(gs[s], xh, dg[i]);
+                    db[i] += gs[s];
+                }
+            };
+            add(0, acc, mine + slot * CELLS + tid);
+            if (second) add(1, mine[slot * CELLS + THREADS + tid], mine + slot * CELLS + THREADS + tid);  // whole warps
+            const double r = quad_reduce8(sum, lane);
+            const int b = (q - q0) % QB;
+            if ((lane & 3) == 0) red[b][warp][lane >> 2] = r;
+            if (b == QB - 1 || q + 1 == q1) {
+                __syncthreads();
+                if (tid < (b + 1) * 8) {
+                    double s = 0.0;
+#pragma unroll
+                    for (int k = 0; k < THREADS / 32; ++k) s += red[tid >> 3][k][tid & 7];
+                    const int j = tid & 7;  // value j: a of samples 0..3, then c
+                    reinterpret_cast<double *>(p.partials + (size_t)(4 * (q - b + (tid >> 3)) + (j & 3)) * gridDim.x + blk)[j >> 2] = s;
+                }
+            }
         }
         slot = slot == RING - 1 ? 0 : slot + 1;
+    }
+    if constexpr (S != NO_SUMS) {
+        auto put = [&](size_t at, float *to, float v) { to[at] = p.accumulate ? to[at] + v : v; };
+        if (gridDim.y == 1) {
+            put(c, p.ggamma, dg[0]);
+            put(c, p.gbeta, db[0]);
+            if (second) {
+                put(c2, p.ggamma, dg[1]);
+                put(c2, p.gbeta, db[1]);
+            }
+            return;
+        }
+        cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+        float *const own = reinterpret_cast<float *>(part);  // [2][512]; the partial sums of the borders have been read:
+        __syncthreads();
+        own[tid] = dg[0], own[512 + tid] = db[0];
+        if (second) own[THREADS + tid] = dg[1], own[512 + THREADS + tid] = db[1];
+        cluster.sync();
+        for (unsigned i = blockIdx.y * THREADS + tid; i < 1024; i += gridDim.y * THREADS) {
+            float s = 0.0f;
+            for (unsigned r = 0; r < gridDim.y; ++r) s += *cluster.map_shared_rank(own + i, r);
+            put(place(i & 511), i < 512 ? p.ggamma : p.gbeta, s);
+        }
+        cluster.sync();  // nobody leaves while its sums are being read
     }
 }
 
@@ -1435,42 +1542,61 @@ int launch_quad_finish(const float *gpk, float *gw, float *gb, float *gs, const 
     return check_launch("quad_finish");
 }
 
-template <bool NORM, int BR>
-static int launch_border(const float *w, const float *dsum, const float *dsum2, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
-                         int Q, int block, cudaStream_t st)
+template <bool NORM, int BR, BorderSums S>
+static int launch_border8(BorderParams p, cudaStream_t st)
 {
-    const long long nb = regions_of(M, N, K);
-    const int ctas_per_sm = block == 8 && BR == 1 ? 3 : 2;
-    const int chunks = pick_batch_chunks_balanced(nb, Q, ctas_per_sm, 4.0, 32);
-    const int qpc = (Q + chunks - 1) / chunks;
-    dim3 grid((unsigned)nb, (unsigned)((Q + qpc - 1) / qpc));
-    static unsigned long long done[2] = {};
-    const float4 *const d4 = reinterpret_cast<const float4 *>(dsum), *const e4 = reinterpret_cast<const float4 *>(dsum2);
-    const float4 *const x4 = reinterpret_cast<const float4 *>(x_il4);
-    float4 *const g4 = reinterpret_cast<float4 *>(gx);
-    if (block == 8) {
-        constexpr int smem = (quadborder::RING * (BR * quadborder::SHELL + (NORM ? 2 : 1) * quadborder::SURFACE) + 2 * BR * 3 * 128) * 16;
-        const int rc = smem_once(quad_border8_k<NORM, BR>, smem, &done[0], "cudaFuncSetAttribute(quad_border8_k)");
-        if (rc != GN_OK) return rc;
-        launch_after(quad_border8_k<NORM, BR>, grid, 384, smem, st, w, (size_t)M * N * K, d4, e4, g4, x4, hterm, Q, M, N, K, qpc);
-    } else {
-        constexpr int smem = 2 * quadborder::TS * 16;
-        const int rc = smem_once(quad_border4_k<NORM>, smem, &done[1], "cudaFuncSetAttribute(quad_border4_k)");
-        if (rc != GN_OK) return rc;
-        launch_after(quad_border4_k<NORM>, grid, 512, smem, st, w, d4, g4, x4, hterm, Q, M, N, K, qpc);
-    }
+    using R = quadborder::Room<NORM, BR, S>;
+    const long long nb = regions_of(p.M, p.N, p.K);
+    const int chunks = pick_batch_chunks_balanced(nb, p.Q, R::CTAS, 4.0, S == NO_SUMS ? 32 : 8);  // sums: a cluster
+    p.qpc = (p.Q + chunks - 1) / chunks;
+    const dim3 grid((unsigned)nb, (unsigned)((p.Q + p.qpc - 1) / p.qpc));
+    static unsigned long long done = 0;
+    const int rc = smem_once(quad_border8_k<NORM, BR, S>, R::BYTES, &done, "cudaFuncSetAttribute(quad_border8_k)");
+    if (rc != GN_OK) return rc;
+    launch_after_cluster(S == NO_SUMS ? 1 : grid.y, quad_border8_k<NORM, BR, S>, grid, 384, R::BYTES, st, p);
     return check_launch("quad_border");
 }
 
-int launch_quad_border(const float *w, const float *dsum, const float *dsum2, float *gx, const float *x_il4, const float4 *hterm, int M, int N, int K,
-                       int Q, int block, cudaStream_t st)
+template <bool NORM>
+static int launch_border4(const BorderParams &p, cudaStream_t st)
 {
-    if (dsum2) {
-        if (block != 8 || hterm) return GN_ERR_UNSUPPORTED;
-        return launch_border<false, 2>(w, dsum, dsum2, gx, nullptr, nullptr, M, N, K, Q, block, st);
+    constexpr int smem = 2 * quadborder::TS * 16;
+    const long long nb = regions_of(p.M, p.N, p.K);
+    const int chunks = pick_batch_chunks_balanced(nb, p.Q, 2, 4.0, 32), qpc = (p.Q + chunks - 1) / chunks;
+    const dim3 grid((unsigned)nb, (unsigned)((p.Q + qpc - 1) / qpc));
+    static unsigned long long done = 0;
+    const int rc = smem_once(quad_border4_k<NORM>, smem, &done, "cudaFuncSetAttribute(quad_border4_k)");
+    if (rc != GN_OK) return rc;
+    launch_after(quad_border4_k<NORM>, grid, 512, smem, st, p.w, p.dsum, p.gx, p.x, p.hterm, p.Q, p.M, p.N, p.K, qpc);
+    return check_launch("quad_border");
+}
+
+// Whether the sums are better taken in the border pass: where a region per SM is all there is, a kernel is mostly its launch and its
+// latency. us of a training loop of 2 x 8 iterations, apart / together: 32^3 (64 regions) x 16 460 / 454, x 64 689 / 657, x 128
+// 1130 / 1093, gated x 64 1416 / 1377; 64^3 (512) x 4 636 / 647, x 16 1264 / 1270, x 64 3726 / 3724; 128^3 (4096) x 4 4228 / 4448. Two
+// CTAs per SM instead of three, and eight times the warp sums per cell, are what it costs.
+bool quad_border_takes_sums(int M, int N, int K, int block) { return block == 8 && regions_of(M, N, K) <= sm_count(); }
+
+int launch_quad_border(const QuadBorder &a, cudaStream_t st)
+{
+    BorderParams p{};
+    p.w = a.w; p.dsum = reinterpret_cast<const float4 *>(a.dsum); p.dsum2 = reinterpret_cast<const float4 *>(a.dsum2);
+    p.gx = reinterpret_cast<float4 *>(a.gx); p.x = reinterpret_cast<const float4 *>(a.x_il4); p.hterm = a.hterm;
+    p.gamma = a.gamma; p.stats = a.stats; p.partials = a.partials;
+    p.ggamma = a.ggamma; p.gbeta = a.gbeta; p.accumulate = a.accumulate;
+    p.Q = a.Q; p.M = a.M; p.N = a.N; p.K = a.K;
+    const bool sums = a.gamma != nullptr;
+    if ((a.dsum2 && (a.block != 8 || a.hterm)) || (sums && (a.block != 8 || a.hterm))) return GN_ERR_UNSUPPORTED;
+    if (a.block == 4) return a.hterm ? launch_border4<true>(p, st) : launch_border4<false>(p, st);
+    if (!sums) {
+        if (a.hterm) return launch_border8<true, 1, NO_SUMS>(p, st);
+        return a.dsum2 ? launch_border8<false, 2, NO_SUMS>(p, st) : launch_border8<false, 1, NO_SUMS>(p, st);
     }
-    return hterm ? launch_border<true, 1>(w, dsum, nullptr, gx, x_il4, hterm, M, N, K, Q, block, st)
-                 : launch_border<false, 1>(w, dsum, nullptr, gx, nullptr, nullptr, M, N, K, Q, block, st);
+    const int rc = a.dsum2 ? launch_border8<false, 2, SUMS>(p, st) : launch_border8<false, 1, SUMS>(p, st);
+    if (rc != GN_OK) return rc;
+    const long long P = (long long)a.M * a.N * a.K;
+    launch_after(quad_norm_ac_k, 4 * a.Q, 256, 0, st, (const double2 *)a.partials, (int)regions_of(a.M, a.N, a.K), a.ac, (size_t)P);
+    return check_launch("quad_norm_ac");
 }
 
 int quad_norm_parts(long long P)

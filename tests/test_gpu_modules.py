@@ -420,6 +420,44 @@ def test_samples_that_fill_up_a_quad_leave_no_trace(batch):
         assert torch.isfinite(q).all() and torch.allclose(p, q, rtol=1e-3, atol=1e-4 * (1 + q.abs().max().item())), i
 
 
+@pytest.mark.parametrize("shape,batch", [((8, 8, 8), 129), ((32, 32, 32), 37), ((16, 24, 8), 3), ((32, 40, 64), 5)])
+@pytest.mark.parametrize("gated", [False, True])
+def test_layer_norm_sums_taken_with_the_border_or_apart(shape, batch, gated):
+    """The backward pass of small grids takes the sums of the norm's gradient in the border pass, quads split over a cluster of CTAs
+    (7 of them, 4, 1); 160 regions have them apart. Against the composition of the step op and torch's layer norm. The sums run
+    over at most 2 x 129 x 512 values of order one in another order: 1e-4 of the largest gradient is twenty times their rounding."""
+    import gridnet_b200 as gb
+
+    g = torch.Generator().manual_seed(17)
+    inner, outer = 2, 3
+    mk = lambda *sz, scale=1.0, shift=0.0: (shift + scale * torch.randn(*sz, generator=g)).cuda()
+    params = [mk(27, *([2] if gated else []), *shape, scale=27 ** -0.5), mk(*([2] if gated else []), *shape, scale=0.1)]
+    if not gated:
+        params.append(mk(*shape, scale=0.1, shift=1.0))
+    leaves = params + [mk(*shape, scale=0.1, shift=1.0), mk(*shape, scale=0.1), mk(batch, *shape)]
+    gy = mk(batch, *shape)
+
+    def loop(*t):
+        if gated:
+            return gb.FusedGatedLoopTrainOp.apply(*t, inner, outer, 8, "tanh", 1e-5)
+        return gb.FusedLoopTrainOp.apply(*t, inner, outer, 8, "silu", 1e-5)
+
+    def composed(*t):
+        *p, gamma, beta, h = t
+        for _ in range(outer):
+            h = gb.GatedGridnetCudaOp.apply(*p, h, inner, 8, "tanh") if gated else gb.GridnetCudaOp.apply(*p, h, inner, 8, 1e-5, False, "silu")
+            h = torch.nn.functional.layer_norm(h, shape, gamma, beta, 1e-5)
+        return h
+
+    grads = []
+    for f in (loop, loop, composed):
+        t = [a.clone().requires_grad_(True) for a in leaves]
+        grads.append(torch.autograd.grad(f(*t), t, gy))
+    for i, (a, again, want) in enumerate(zip(*grads)):
+        assert torch.equal(a, again), i
+        assert torch.allclose(a, want, rtol=0, atol=1e-4 * want.abs().max().item()), (i, (a - want).abs().max().item(), want.abs().max().item())
+
+
 def test_what_does_not_fit_is_recomputed(monkeypatch):
     """The bookkeeping of kept iterations: per device, without a lock that a finaliser could meet held, and a loop that runs out of
     memory while it allocates them goes on with those it has (allocation made to fail here; the gradients are the same bits)."""
