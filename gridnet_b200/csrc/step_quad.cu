@@ -165,11 +165,6 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
         tmem_fence_before();
         team_sync<TEAM>(quarter);
         tmem_fence_after();
-        if (i0 + here < cnt) {  // the next region's parameters on their way to L2
-            const unsigned char *nx = reinterpret_cast<const unsigned char *>(p.packed + (size_t)(blk + 1) * PACK_F);
-            for (int c = role * 32 + lane; c < PACK_F * 4 / 128; c += 32 * TEAM) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + c * 128));
-            __syncwarp();
-        }
 
         for (int next = 0; i < i0 + here; i = next) {
             const int q = q0 + i - i0;

@@ -14,8 +14,10 @@
 //     iteration). Only the halo's 488 entries of the (gamma, beta) table are in shared memory, a lane's own in tensor memory.
 //   - A warp takes the next item of its quarter when it is free (64^3: 1597 -> 1553 us), and asks for the first half of the
 //     next region's parameters before it waits for the other warp.
-// Measured before and after: 64^3 x 64, 4 x 12 iterations 1652 -> 1553 us; 40 x 56 x 72 x 37, 3 x 6 315 -> 290 us; 256^3 x 32, 2 x 32 91.8 ->
-// 90.4 ms (at 1.77 GHz); 64^3 x 128, block 4, 8 x 16 with gradients 41.3 -> 40.7 ms. Letting one or two warps of a quarter at a time into
+//   - The next region's parameters are not prefetched to L2: 256^3 x 32 93.5 -> 88.5 ms, 128^3 x 16 with gradients 9.12 -> 8.85 ms, 40 x 56 x 72
+//     290 -> 285 us, at the price of 1554 -> 1565 us at 64^3. Prefetching tiles was slower too (256^3: 99.5 ms).
+// Measured before and after: 64^3 x 64, 4 x 12 iterations 1652 -> 1565 us; 40 x 56 x 72 x 37, 3 x 6 315 -> 285 us; 256^3 x 32, 2 x 32 96.5 ->
+// 88.5 ms (at 1.77 GHz); 64^3 x 128, block 4, 8 x 16 with gradients 41.3 -> 40.4 ms. Letting one or two warps of a quarter at a time into
 // the 27-tap sums, so that the rest of an item overlaps with another's, was slower (1754 and 1721 us).
 // Block 8: tiles by bulk tensor copy. Block 4: each warp fetches its own next tile, cell by cell and asynchronously; its
 // eight small tiles have to lie an odd number of cells apart, which bulk tensor copies cannot do.
@@ -251,16 +253,6 @@ __global__ void __launch_bounds__(128 * TapGeo<SUB>::TEAM, 1) step_fwd_taps(cons
         tmem_fence_before();
         team_sync<TEAM>(quarter);
         tmem_fence_after();
-        if (i0 + here < cnt) {  // the next region's parameters on their way to L2
-            const unsigned char *nx = reinterpret_cast<const unsigned char *>(p.packed + (size_t)(blk + 1) * PACK_F);
-            for (int c = role * 32 + lane; c < PACK_F * 4 / 128; c += 32 * TEAM) asm volatile("prefetch.global.L2 [%0];" ::"l"(nx + c * 128));
-            if (FUSE_IN) {
-                constexpr int BYTES = QuadGeo<SUB>::CELLS * 8;
-                const unsigned char *ng = reinterpret_cast<const unsigned char *>(p.gbt) + (size_t)(blk + 1) * BYTES;
-                for (int c = role * 32 + lane; c < BYTES / 128; c += 32 * TEAM) asm volatile("prefetch.global.L2 [%0];" ::"l"(ng + c * 128));
-            }
-            __syncwarp();
-        }
 
         for (int next; i < i0 + here; i = next) {
             const int q = q0 + i - i0;
