@@ -402,7 +402,8 @@ struct Lay {
     static constexpr int TILE = (QuadGeo<SUB>::BUF_BYTES + 127) / 128 * 128;
     static constexpr int DSQ = NT * TILE + 3 * OWN;  // a quad's terms of the scale gradient, each thread its own four
     static constexpr int IST = DSQ + THREADS * 16;   // and, each warp its own copy, its statistics
-    static constexpr int GB = IST + THREADS;         // normalise-on-load: the region's (gamma, beta) table
+    static constexpr int SCALE = IST + THREADS;      // residual scales, each thread its own four
+    static constexpr int GB = SCALE + THREADS * 16;  // normalise-on-load: the region's (gamma, beta) table
     static constexpr int NSTAT = (SUB == 8 ? 1 : 8) * QS_COUNT;  // per-block normalisation, there: two iterations' statistics
     static constexpr int smem(bool fuse, bool norm) { return GB + (fuse ? QuadGeo<SUB>::CELLS * 8 : 0) + (norm ? 2 * NSTAT * 16 : 0); }
 };
@@ -542,6 +543,11 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
         cp_async_wait_all();
         __syncthreads();
     }
+    const unsigned my_scale = tiles + Y::SCALE + tid * 16;
+    if (!GATED && p.inner > 1) {
+        const float *s = p.scale + g0;
+        sts128(my_scale, make_float4(s[0], s[p.K], s[zs], s[zs + p.K]));
+    }
     previous_done();
     if (tid == 0) issue(q0, 0);
     fetch_quad(q0);
@@ -626,21 +632,25 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
                 shift = lds128(st + QS_MEAN * 16);
                 shift.x -= pivot.x, shift.y -= pivot.y, shift.z -= pivot.z, shift.w -= pivot.w;
             }
-            if (!last) {  // the activations of iteration t + 1 -> the other tile
+            if (!last) {  // the activations of iteration t + 1 -> the other tile. All loads first: a load waits for a store before it
                 const unsigned to = tiles + (buf_x ^ 1) * Y::TILE;
+                auto cell = [&](int n) { return own0 + (unsigned)((n >> 1) * G::PLANE + (n & 1) * G::ROW) * 16u; };
+                u64 h[4][2], x[4][2];
+                float4 sc = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (!GATED) sc = lds128(my_scale);
 #pragma unroll
                 for (int n = 0; n < 4; ++n) {
-                    const unsigned c = own0 + (unsigned)((n >> 1) * G::PLANE + (n & 1) * G::ROW) * 16u;
-                    u64 h0, h1, x0, x1;
-                    lds128u(stage_h + n * (THREADS * 16), h0, h1);
-                    if (GATED) {
-                        sts128u(to + c, h0, h1);
-                        continue;
-                    }
-                    const float sc = __ldg(p.scale + g0 + (n >> 1) * zs + (n & 1) * (size_t)p.K);
-                    lds128u(tile + c, x0, x1);
-                    sts128u(to + c, act_residual2<ACT>(h0, sc, x0), act_residual2<ACT>(h1, sc, x1));
+                    lds128u(stage_h + n * (THREADS * 16), h[n][0], h[n][1]);
+                    if (!GATED) lds128u(tile + cell(n), x[n][0], x[n][1]);
                 }
+                const float s4[4] = {sc.x, sc.y, sc.z, sc.w};
+                if (!GATED)
+#pragma unroll
+                    for (int n = 0; n < 4; ++n)
+#pragma unroll
+                        for (int k = 0; k < 2; ++k) h[n][k] = act_residual2<ACT>(h[n][k], s4[n], x[n][k]);
+#pragma unroll
+                for (int n = 0; n < 4; ++n) sts128u(to + cell(n), h[n][0], h[n][1]);
             }
             if (t == 0) {
                 if (!GATED) {
