@@ -552,9 +552,12 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
     if (tid == 0) issue(q0, 0);
     fetch_quad(q0);
     const float *const delta = GATED && blockIdx.z ? p.delta2 : p.delta;
-    fetch(stage_d, at(delta, q0, 0));
+    // deltas are asked for in the order (quad, iteration), pre-activations likewise without the last iteration
+    const float *d_next = at(delta, q0, 0), *h_next = at(p.h, q0, 0);
+    const long long next_quad = 4 * (long long)P;
+    fetch(stage_d, d_next);
     fetch_stats(0, q0, 0);
-    if (p.inner > 1) fetch(stage_h, at(p.h, q0, 0));
+    if (p.inner > 1) fetch(stage_h, h_next);
     const unsigned own0 = (unsigned)(T.cell0 + G::PLANE + G::ROW + 1) * 16u;
 
     for (int q = q0; q < q1; ++q) {
@@ -662,13 +665,21 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
             }
             // the next iteration's data
             if (!last) {
-                fetch(stage_d + (buf_d ^ 1) * OWN, at(delta, q, t + 1));
+                d_next += T4;
+                fetch(stage_d + (buf_d ^ 1) * OWN, d_next);
                 fetch_stats(buf_d ^ 1, q, t + 1);
-                if (t + 2 < p.inner) fetch(stage_h, at(p.h, q, t + 1));
+                if (t + 2 < p.inner) {
+                    h_next += T4;
+                    fetch(stage_h, h_next);
+                }
             } else if (q + 1 < q1) {
-                fetch(stage_d + (buf_d ^ 1) * OWN, at(delta, q + 1, 0));
+                d_next += next_quad - (p.inner - 1) * (long long)T4;
+                fetch(stage_d + (buf_d ^ 1) * OWN, d_next);
                 fetch_stats(buf_d ^ 1, q + 1, 0);
-                if (p.inner > 1) fetch(stage_h, at(p.h, q + 1, 0));
+                if (p.inner > 1) {
+                    h_next += next_quad - (p.inner - 2) * (long long)T4;
+                    fetch(stage_h, h_next);
+                }
                 if (tid == 0) issue(q + 1, buf_x ^ 1);
             }
 #pragma unroll
