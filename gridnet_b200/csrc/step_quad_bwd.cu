@@ -1220,7 +1220,8 @@ __global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *x, const f
                                                         double2 *partials, int nparts, float *ggamma, float *gbeta, int accumulate, int Q,
                                                         int qpc, size_t P)
 {
-    constexpr int QB = 16;  // quads between two block-wide sums
+    constexpr int QB = 16;                        // quads between two block-wide sums
+    constexpr int AT_ONCE = CPT == 1 ? 4 : 2;     // quads whose loads are in flight
     __shared__ double red[QB][8][8];
     __shared__ float part[2][CPT * 256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1235,7 +1236,7 @@ __global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *x, const f
     const int q0 = blockIdx.y * qpc, q1 = min(Q, q0 + qpc);
     for (int qb = q0; qb < q1; qb += QB) {
         const int qe = min(q1, qb + QB);
-#pragma unroll 2
+#pragma unroll AT_ONCE
         for (int q = qb; q < qe; ++q) {
             float4 xv[CPT], gv[CPT];
 #pragma unroll
@@ -1635,6 +1636,8 @@ int launch_quad_norm_sums(const float *x, const float *g, const float *sub, cons
     // enough CTAs for a few per SM, by splitting the quads where the cells do not give them
     int chunks = 1;
     while (chunks < 8 && 2 * chunks <= Q && (long long)nparts * chunks < 4LL * sm_count()) chunks *= 2;
+    // long walks once more: 64^3 x 128, block 4, with gradients 37.2 -> 37.0 ms; four quads a CTA are better left alone (64^3 x 16: + 3 %)
+    if (chunks < 8 && 16 * chunks <= Q && (long long)nparts * chunks < 12LL * sm_count()) chunks *= 2;
     const int qpc = (Q + chunks - 1) / chunks;
 #define SUMS_(C, S)                                                                                                                     \
     launch_after_cluster(chunks, quad_norm_sums_k<C, S>, dim3(nparts, chunks), 256, 0, st, x4, g4, s4, gamma, stats, partials, nparts, \
