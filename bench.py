@@ -57,7 +57,7 @@ FALLBACK_HBM_GBS = 6650.0
 # DRAM bytes per launch of the dominant kernel (dram__bytes_read.sum + dram__bytes_write.sum): a constant taken
 # from the ncu capture summarised in the named file, not a measurement of this run
 NCU_TRAFFIC = {
-    "step_fwd_taps": (180.7e6, "profiles/step_fwd_taps_c2_ncu_sections.txt"),
+    "step_fwd_taps": (177.5e6, "profiles/step_fwd_taps_c2_ncu_sections.txt"),
     "step_fwd_fast8": (173.0e6, "profiles/step_fwd_fast8_c2_ncu_full.txt"),
 }
 

@@ -236,8 +236,8 @@ static OuterWs carve_outer(void *base, int B, int M, int N, int K, int block)
 }
 
 // 0 = choose automatically: the one persistent kernel of outer_small.cu for problems so small that launches are what
-// they cost; else the quad kernel of step_quad.cu where it has work for most of its warps; else the register-patch kernel of
-// step_fast.cu. 1 = always the register-patch kernel, 2 = always the large-batch kernel of step_pair64.cu, 3 = always the
+// they cost, or of outer_held.cu for a sample or two per four blocks and SM; else the quad kernel of step_quad.cu where it has work for most of its warps; else the register-patch kernel of
+// step_fast.cu. 1 = always the register-patch kernel, 2 = always the large-batch kernel of step_pair64.cu, 3 = always a
 // persistent kernel, 4 = always the quad kernel.
 // A quad warp works on a whole 8^3 region for four samples, so fewer than about three regions x quads per SM leave it
 // idle, and a single sample fills a quarter of a lane. ms per loop, register-patch / quad: 48^3, 2 x 10, batch 3

@@ -1220,8 +1220,8 @@ __global__ void __launch_bounds__(256) quad_norm_sums_k(const float4 *x, const f
                                                         double2 *partials, int nparts, float *ggamma, float *gbeta, int accumulate, int Q,
                                                         int qpc, size_t P)
 {
-    constexpr int QB = 16;                        // quads between two block-wide sums
-    constexpr int AT_ONCE = CPT == 1 ? 4 : 2;     // quads whose loads are in flight
+    constexpr int QB = 16;                     // quads between two block-wide sums
+    constexpr int AT_ONCE = CPT == 1 ? 4 : 2;  // quads whose loads are in flight
     __shared__ double red[QB][8][8];
     __shared__ float part[2][CPT * 256];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;

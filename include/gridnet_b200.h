@@ -70,8 +70,9 @@ GN_API int gn_version(void);
 /* Process-wide tuning switches (not needed for normal use). Keys:
  *   "outer_kernel": which kernel gn_outer_forward_f32 uses: 0 = automatic (default: the whole
  *                   loop as one persistent kernel when the problem is so small that launches are
- *                   what it costs; else the quad kernel; the register-patch kernel where neither
- *                   applies), 1 = the register-patch kernel, 2 = the large-batch kernel, 3 = the
+ *                   what it costs, or its blocks' weights fit into the tensor memory of the chip;
+ *                   else the quad kernel; the register-patch kernel where neither
+ *                   applies), 1 = the register-patch kernel, 2 = the large-batch kernel, 3 = a
  *                   persistent kernel, 4 = the quad kernel (GN_ERR_UNSUPPORTED from gn_outer_forward_f32 when the forced one does not apply).
  *   "forward_samples_per_cta": samples one CTA of the tuned float forward kernel walks through;
  *                   0 = chosen from the grid and batch size (default). */
@@ -437,7 +438,7 @@ GN_API int gn_norm_apply_f32(const float *x, const float *gamma, const float *be
  * With the quad kernel the activations stay interleaved by four samples between steps, [quad][M][N][K][4]; with the
  * large-batch kernel (see gn_step_forward_pair64_f32 below) by groups of 64, [group][M][N][K][64]. */
 /* Which kernel gn_outer_forward_f32 would take for this problem with suitably aligned buffers: 3 = the whole loop
- * as one persistent kernel (1 launch), 5 = the quad kernel (2 launches per outer step + 2), 2 = the large-batch
+ * as one persistent kernel (1 launch; of the two the one that applies), 5 = the quad kernel (2 launches per outer step + 2), 2 = the large-batch
  * kernel (2 per outer step + 3), 1 = the register-patch kernel (2 per outer step + 1), 4 = the step-by-step
  * composition of the generic kernels, 0 = bad arguments or the kernel forced with gn_config_set does not apply. */
 GN_API int gn_outer_forward_plan(int B, int M, int N, int K, int inner, int outer, int block);
