@@ -353,20 +353,29 @@ static int launch_one(const OuterHeldParams &p, int ctas, cudaStream_t st)
     return GN_OK;
 }
 
-// SMs that take part, 0 where the kernel cannot run; asked once per device
+// CTAs of the kernel that are resident at once, one per SM, 0 where it cannot run; asked once per device
 static int usable_sms()
 {
     static std::atomic<int> known[64];  // + 1
-    int dev = 0, coop = 0;
+    int dev = 0, coop = 0, per_sm = 0, n = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     if (dev < 64 && known[dev].load(std::memory_order_relaxed)) return known[dev].load(std::memory_order_relaxed) - 1;
-    const int n = cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop ? sm_count() : 0;
+    auto kern = outer_held_k<GN_ACT_TANH>;
+    if (cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev) == cudaSuccess && coop &&
+        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, held8::SMEM_ALONE) == cudaSuccess &&
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, held8::THREADS, held8::SMEM_ALONE) == cudaSuccess && per_sm > 0)
+        n = sm_count();
+    else (void)cudaGetLastError();  // what could not be set or asked is an answer too
     if (dev < 64) known[dev].store(n + 1, std::memory_order_relaxed);
     return n;
 }
 
 // Samples per CTA, or 0 if the kernel does not apply: block 8, at least one outer step, all blocks of a chunk of samples resident
-// at once, at most MAX_SPC samples per CTA.
+// at once, at most MAX_SPC samples per CTA (each takes 10 KB of shared memory per block and registers for its patch). Wherever it
+// applies it is ahead of the loop of one launch per step, us, step by step / this kernel: 64^3, 4 x 12, one sample 166 / 80, two 217 / 105;
+// 64^3, 1 x 4 54 / 46; 40 x 56 x 72, 3 x 6 87 / 48; 48^3, 4 x 10, four samples 128 / 89; 32^3, 2 x 8, sixteen 101 / 56; 16^3, 2 x 8, 148
+// samples 103 / 52, 5 x 16, 120 samples 306 / 140. Where the blocks' weights fit into registers outer_small.cu is: 32^3, 2 x 8, eight samples
+// 38 there, 41 here.
 int outer_held_spc(int B, int M, int N, int K, int block, int inner, int outer, const void *w, const void *b, const void *s, const void *gamma,
                    const void *beta, const void *x, const void *y)
 {

@@ -67,6 +67,10 @@ struct QuadRevParams {
 // ones, so the other kernels see inv Gin. The lanes that share a tile add the two sums up by shuffles; what the halo
 // cells owe, F + E x with F = sum_t (P1 - P2 mean), E = sum_t P2, goes (negated) to the border kernel. The activations x_t are
 // walked back from the step's output, x_t = x_(t+1) - scale act(h_t).
+// What bounds it: latency. Of 42 k cycles that an item of two iterations takes at 128^3 x 32 the transposed sums are 13 k, deltas 8.5 k, its
+// first loads 8.8 k (asked for to L2 a stencil ahead; a staging area of their own would take the first-level cache's room and was
+// slower), its stores 4.7 k. Warps take the next item when they are free; a region's first half of parameters is loaded ahead of the barrier,
+// the first region's while the kernel before still runs: 626 -> 571 us.
 template <int SUB, int ACT, quadrev::In IN>
 __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
 {
@@ -390,8 +394,12 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
 // and writing back sums there was 3 to 4 times slower than this (128^3, two inner iterations, batch 32: 0.77 - 0.97 ms).
 // The step's input tile arrives by bulk tensor copy and is normalised in place; activations between iterations are rebuilt
 // from it and the pre-activations. Two tiles take turns over the iterations, one barrier each (block 4 with one tile, updated in
-// place between two barriers: 39.9 ms for 64^3 x 128, 8 x 16 with gradients, now 38.8). Deltas and pre-activations arrive
+// place between two barriers: 64^3 x 128, 8 x 16 with gradients 39.9 ms, with two 38.8). Deltas and pre-activations arrive
 // an iteration ahead, what else a quad needs a quad ahead, each thread its own (128^3 x 32, 2 x 16: 30.35 -> 30.05 ms).
+// What bounds it: 61 % of the shared-memory pipe, 1300 of 2900 cycles per iteration in the window sums, the rest deltas, activations and
+// copies between two barriers (block 4: 956 us a step at 64^3 x 128, now 823; 128^3 x 32 518, now 486). Computing the activations under the
+// window sums takes a second copy of these: 1 % faster at 128^3, 2 % slower at 32^3, where kernels are over before their code has
+// arrived.
 namespace quadwg {
 constexpr int CTAS = 2;  // per SM: 255 registers (three with 168 spill, and are no faster)
 constexpr int THREADS = 128, OWN = 4 * THREADS * 16;  // bytes of one staging area: a thread's four cells
