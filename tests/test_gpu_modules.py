@@ -458,6 +458,29 @@ def test_layer_norm_sums_taken_with_the_border_or_apart(shape, batch, gated):
         assert torch.allclose(a, want, rtol=0, atol=1e-4 * want.abs().max().item()), (i, (a - want).abs().max().item(), want.abs().max().item())
 
 
+@pytest.mark.parametrize("gated", [False, True])
+def test_what_a_loop_keeps_survives_being_packed_and_unpacked(gated):
+    """A small loop saves what it keeps as one tensor and finds its pieces by their addresses. Hooks that move saved tensors away and
+    bring back others, and a second walk over the same graph, give the same gradients."""
+    import gridnet_b200 as gb
+
+    g = torch.Generator().manual_seed(23)
+    shape, batch, inner, outer = (16, 8, 24), 5, 2, 3
+    mk = lambda *sz, scale=1.0, shift=0.0: (shift + scale * torch.randn(*sz, generator=g)).cuda()
+    leaves = [mk(27, *([2] if gated else []), *shape, scale=27 ** -0.5), mk(*([2] if gated else []), *shape, scale=0.1)]
+    leaves += ([] if gated else [mk(*shape, scale=0.1, shift=1.0)]) + [mk(*shape, scale=0.1, shift=1.0), mk(*shape, scale=0.1), mk(batch, *shape)]
+    leaves = [t.requires_grad_(True) for t in leaves]
+    op, gy = gb.FusedGatedLoopTrainOp if gated else gb.FusedLoopTrainOp, mk(batch, *shape)
+    y = op.apply(*leaves, inner, outer, 8, "tanh", 1e-5)
+    want = torch.autograd.grad(y, leaves, gy, retain_graph=True)
+    again = torch.autograd.grad(y, leaves, gy)
+    with torch.autograd.graph.save_on_cpu():
+        y = op.apply(*leaves, inner, outer, 8, "tanh", 1e-5)
+    moved = torch.autograd.grad(y, leaves, gy)
+    for a, b, c in zip(want, again, moved):
+        assert torch.equal(a, b) and torch.equal(a, c)
+
+
 def test_what_does_not_fit_is_recomputed(monkeypatch):
     """The bookkeeping of kept iterations: per device, without a lock that a finaliser could meet held, and a loop that runs out of
     memory while it allocates them goes on with those it has (allocation made to fail here; the gradients are the same bits)."""
