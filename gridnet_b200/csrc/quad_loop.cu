@@ -248,6 +248,7 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
         const float *in = k ? outs[k - 1] : x_il4;
         const float2 *in_stats = residual ? mr + (size_t)k * S : (k ? mr + (size_t)(k - 1) * S : nullptr);
         const bool kept = stashes && stashes[k];
+        bool fresh = false;  // the kernel queued last has re-ordered parameters
         if (first || nparams > 1) {
             QuadPrepare a{};
             a.w = weights[kp]; a.b = biases[kp]; a.s = scales[kp]; a.b_t = gamma; a.packed_t = w.packed_t;
@@ -258,9 +259,12 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
                 a.x = gy; a.il = w.g[0]; a.B = B; a.gradient = true;
             }
             TRY_(launch_quad_prepare(a, M, N, K, block, st));
+            fresh = true;
         }
-        if (!residual && (first || !with_border))  // else taken with the border of the step after
+        if (!residual && (first || !with_border)) {  // else taken with the border of the step after
             TRY_(launch_quad_norm_sums(outs[k], w.g[cur], nullptr, gamma, mr + (size_t)k * S, w.partials, ggamma, gbeta, !first, w.ac, d.Q, d.P, st));
+            fresh = false;
+        }
         float *const h = kept ? stashes[k] : w.replay;
         if (!kept) {
             QuadStep a{};
@@ -269,10 +273,11 @@ GN_API int gn_loop_backward_f32(const float *const *weights, const float *const 
             a.save_h = h;
             a.M = M; a.N = N; a.K = K; a.Q = d.Q; a.inner = inner; a.block = block;
             TRY_(launch_step_fwd_quad(a, act, st));
+            fresh = false;
         }
         QuadReverse r{};
         r.packed_t = w.packed_t; r.g = w.g[cur];
-        r.params_old = !residual || !kept || (!first && nparams == 1);  // something ran since they were re-ordered
+        r.params_old = !fresh;
         if (!residual) {
             r.raw = outs[k]; r.stats = mr + (size_t)k * S; r.ac = w.ac;
         }

@@ -481,6 +481,32 @@ def test_what_a_loop_keeps_survives_being_packed_and_unpacked(gated):
         assert torch.equal(a, b) and torch.equal(a, c)
 
 
+def test_separate_networks_of_a_small_grid_kept_and_recomputed():
+    """A network per step on a grid of 64 regions, whose reverse sweeps follow the re-ordering of their parameters directly where the
+    iterations are kept, and a forward pass where they are not: the same gradients, bit for bit, over many repeats."""
+    import gridnet_b200 as gb
+
+    g = torch.Generator().manual_seed(31)
+    shape, batch, inner, outer = (32, 32, 32), 40, 2, 6
+    mk = lambda *sz, scale=1.0, shift=0.0: (shift + scale * torch.randn(*sz, generator=g)).cuda()
+    leaves = [mk(*shape, scale=0.1, shift=1.0), mk(*shape, scale=0.1), mk(batch, *shape)]
+    sets = [t for _ in range(outer) for t in (mk(27, *shape, scale=27 ** -0.5), mk(*shape, scale=0.1), mk(*shape, scale=0.1, shift=1.0))]
+    leaves, sets, gy = [t.requires_grad_(True) for t in leaves], [t.requires_grad_(True) for t in sets], mk(batch, *shape)
+
+    def grads(keep):
+        previous = gb.keep_forward_stash(keep)
+        try:
+            y = gb.FusedLoopSeparateTrainOp.apply(*leaves, inner, 8, "silu", 1e-5, *sets)
+        finally:
+            gb.keep_forward_stash(previous)
+        return torch.autograd.grad(y, leaves + sets, gy)
+
+    want = grads(False)
+    for _ in range(10):
+        for i, (a, b) in enumerate(zip(grads(True), want)):
+            assert torch.equal(a, b), i
+
+
 def test_what_does_not_fit_is_recomputed(monkeypatch):
     """The bookkeeping of kept iterations: per device, without a lock that a finaliser could meet held, and a loop that runs out of
     memory while it allocates them goes on with those it has (allocation made to fail here; the gradients are the same bits)."""
