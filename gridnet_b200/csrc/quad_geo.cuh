@@ -182,6 +182,18 @@ __device__ __forceinline__ void team_sync(int quarter)
     asm volatile("bar.sync %0, %1;" ::"r"(quarter + 1), "n"(32 * TEAM) : "memory");
 }
 
+// Items (regions x quads) are split over the quarters of ctas CTAs in whole multiples of this: two where that leaves the longest quarter
+// no longer. A region that a quarter has an odd number of quads of ends with a warp on its own, at 3100 cycles an iteration instead of
+// 2820 each for two, so pairs that never straddle a change of region gain where the longest quarter has an even number of items
+// (64^3 x 64: 14). Where it has an odd number, pairs make it one item longer, and where there are no more items than quarters they leave
+// half of these without work. us of a training loop of 2 x 8 iterations, one by one / in pairs: 32^3 x 8 348 / 386, x 64 718 / 648,
+// 64^3 x 16 1316 / 1236, x 64 3668 / 3619; of inference, 4 x 8: 32^3 x 32 141 / 173, x 64 222 / 193, x 96 271 / 309, 64^3 x 32 588 / 629.
+inline int quad_split_unit(long long nitems, long long ctas, int Q)
+{
+    const long long quarters = ctas * quad::QUARTERS, longest = (nitems + quarters - 1) / quarters;
+    return Q % 2 == 0 && longest % 2 == 0 ? 2 : 1;
+}
+
 // Parameters of a region, packed in the order quad_stencil uses them (quad_pack; tap_stencil: tap_pack): 116 vectors of four words per
 // lane, lane-contiguous (512 bytes per vector and warp).
 namespace quad {

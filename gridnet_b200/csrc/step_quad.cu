@@ -47,6 +47,7 @@ struct QuadParams {
     int *error_flag;
     int M, N, K, Q, inner;
     long long nitems;        // regions * Q
+    int unit;                // quad_split_unit
 };
 
 // SAVE: keep every iteration's pre-activations for the backward pass (which gets the activations in between from them and
@@ -104,9 +105,8 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
     const int nbx = p.K >> 3, nby = p.N >> 3;
     const size_t P = (size_t)p.M * p.N * p.K;
     const long long worker = (long long)blockIdx.x * QUARTERS + quarter, nworkers = (long long)gridDim.x * QUARTERS;
-    const long long even = p.Q % TEAM == 0 ? TEAM : 1;  // whole rounds of the team per region
-    const unsigned n0 = (unsigned)(p.nitems / even * worker / nworkers * even);
-    const int cnt = (int)(p.nitems / even * (worker + 1) / nworkers * even - n0);
+    const unsigned n0 = (unsigned)(p.nitems / p.unit * worker / nworkers * p.unit);
+    const int cnt = (int)(p.nitems / p.unit * (worker + 1) / nworkers * p.unit - n0);
     const unsigned bar0 = smem_u32(&bars[quarter * NBUF]), issued0 = smem_u32(&issued[quarter * NBUF]);
     const unsigned tiles = smem_u32(smem) + quarter * (NBUF * G::BUF_BYTES);
     const long long wzs = (long long)p.N * p.K, wys = (long long)L.ysgn * p.K;
@@ -693,6 +693,7 @@ int launch_step_fwd_quad(const QuadStep &a, int act, cudaStream_t st)
     p.nitems = (long long)(a.M / 8) * (a.N / 8) * (a.K / 8) * a.Q;
     long long ctas = (p.nitems + quad::QUARTERS - 1) / quad::QUARTERS;
     if (ctas > sm_count()) ctas = sm_count();
+    p.unit = quad_split_unit(p.nitems, ctas, p.Q);
     return a.block == 8 ? launch_quad_sub<8>(map, p, (unsigned)ctas, act, st) : launch_quad_sub<4>(map, p, (unsigned)ctas, act, st);
 }
 

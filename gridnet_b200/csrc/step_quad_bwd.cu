@@ -57,6 +57,7 @@ struct QuadRevParams {
     float *dsq;                    // [Q][P] gradient terms of the residual scale, summed over the quad and the iterations
     int M, N, K, Q, inner;
     int params_old;                // the kernel before this one did not write packed (or wsum)
+    int unit;                      // quad_split_unit
     long long nitems;
 };
 
@@ -97,9 +98,8 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
     const int nbx = p.K >> 3, nby = p.N >> 3;
     const size_t P = (size_t)p.M * p.N * p.K, T4 = (size_t)p.Q * P * 4;  // floats of an IL4 tensor
     const long long worker = (long long)blockIdx.x * QUARTERS + quarter, nworkers = (long long)gridDim.x * QUARTERS;
-    const long long even = p.Q % TEAM == 0 ? TEAM : 1;  // whole rounds of the team per region
-    const unsigned n0 = (unsigned)(p.nitems / even * worker / nworkers * even);
-    const int cnt = (int)(p.nitems / even * (worker + 1) / nworkers * even - n0);
+    const unsigned n0 = (unsigned)(p.nitems / p.unit * worker / nworkers * p.unit);
+    const int cnt = (int)(p.nitems / p.unit * (worker + 1) / nworkers * p.unit - n0);
     const long long wzs = (long long)p.N * p.K, wys = (long long)L.ysgn * p.K;
     const long long zstr = wzs * 4, ystr = wys * 4;
     const int dx = L.xsgn * 16;
@@ -1487,6 +1487,7 @@ int launch_quad_reverse(const QuadReverse &a, int act, cudaStream_t st)
     p.nitems = regions_of(a.M, a.N, a.K) * a.Q;
     long long ctas = (p.nitems + quad::QUARTERS - 1) / quad::QUARTERS;
     if (ctas > sm_count()) ctas = sm_count();
+    p.unit = quad_split_unit(p.nitems, ctas, p.Q);
     return a.block == 8 ? launch_reverse_sub<8>(p, (unsigned)ctas, act, st) : launch_reverse_sub<4>(p, (unsigned)ctas, act, st);
 }
 

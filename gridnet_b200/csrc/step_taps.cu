@@ -51,6 +51,7 @@ struct TapParams {
     int M, N, K, Q, inner;
     int params_old;          // the kernel before this one did not write packed or gbt
     long long nitems;        // regions * Q
+    int unit;                // quad_split_unit
 };
 
 // 16 bytes to shared memory, asynchronously; zeros where !inside (src is then not read)
@@ -138,10 +139,8 @@ __global__ void __launch_bounds__(128 * TapGeo<SUB>::TEAM, 1) step_fwd_taps(cons
     const int nbx = p.K >> 3, nby = p.N >> 3;
     const size_t P = (size_t)p.M * p.N * p.K;
     const long long worker = (long long)blockIdx.x * QUARTERS + quarter, nworkers = (long long)gridDim.x * QUARTERS;
-    // whole rounds of the team per region where there are such (64^3 x 64: 14 items are 7 rounds instead of up to 8)
-    const long long even = p.Q % TEAM == 0 ? TEAM : 1;
-    const unsigned n0 = (unsigned)(p.nitems / even * worker / nworkers * even);
-    const int cnt = (int)(p.nitems / even * (worker + 1) / nworkers * even - n0);
+    const unsigned n0 = (unsigned)(p.nitems / p.unit * worker / nworkers * p.unit);
+    const int cnt = (int)(p.nitems / p.unit * (worker + 1) / nworkers * p.unit - n0);
     const unsigned bar0 = smem_u32(&bars[quarter * NBUF]), issued0 = smem_u32(&issued[quarter * NBUF]);
     const unsigned tiles = smem_u32(smem) + quarter * (NBUF * G::BUF_BYTES);
     const long long zstr = 4ll * p.N * p.K;
@@ -449,6 +448,7 @@ int launch_step_fwd_taps(const QuadStep &a, int act, cudaStream_t st)
     p.nitems = (long long)(a.M / 8) * (a.N / 8) * (a.K / 8) * a.Q;
     long long ctas = (p.nitems + QUARTERS - 1) / QUARTERS;
     if (ctas > sm_count()) ctas = sm_count();
+    p.unit = quad_split_unit(p.nitems, ctas, p.Q);
     return a.block == 8 ? launch_sub<8>(map, p, (unsigned)ctas, act, st) : launch_sub<4>(map, p, (unsigned)ctas, act, st);
 }
 

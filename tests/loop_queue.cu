@@ -3,6 +3,7 @@
 // (previous_done() in common.cuh), and the buffers that it writes.
 //
 //   loop_queue gated|plain|residual  sets of parameters  outer steps  sums in the border pass (0, 1)  steps with kept iterations (bits)
+//   loop_queue split  regions  CTAs  quads      in which units items are split (quad_split_unit), for every grid and batch up to these
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -12,6 +13,7 @@
 
 #include "../gridnet_b200/csrc/common.cuh"
 #include "../gridnet_b200/csrc/kernels.h"
+#include "../gridnet_b200/csrc/quad_geo.cuh"
 
 static bool g_border_sums;
 
@@ -90,6 +92,16 @@ int launch_quad_border(const QuadBorder &a, cudaStream_t)
 
 int main(int argc, char **argv)
 {
+    using namespace gn;
+    if (argc == 5 && !strcmp(argv[1], "split")) {
+        // every batch of up to the given number of quads, grids of up to the given number of regions
+        for (int regions = 1; regions <= atoi(argv[2]); ++regions)
+            for (int Q = 1; Q <= atoi(argv[4]); ++Q) {
+                const long long items = (long long)regions * Q, need = (items + quad::QUARTERS - 1) / quad::QUARTERS, ctas = need < atoi(argv[3]) ? need : atoi(argv[3]);
+                printf("%d %d %lld %d\n", regions, Q, ctas, quad_split_unit(items, ctas, Q));
+            }
+        return 0;
+    }
     if (argc != 6) return 2;
     const bool gated = !strcmp(argv[1], "gated"), residual = !strcmp(argv[1], "residual");
     const int sets = atoi(argv[2]), outer = atoi(argv[3]), B = 4, side = 16, inner = 2;

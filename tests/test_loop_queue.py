@@ -46,3 +46,33 @@ def test_parameters_are_loaded_ahead_wherever_they_may_be(program, form, sets, l
     behind = sum(before == "prepare" and name.endswith("reverse") for (before, _, _), (name, _, _) in zip(kernels, kernels[1:]))
     assert behind == late
     assert sum(name.endswith("reverse") and not ahead for name, ahead, _ in kernels) == late
+
+
+def longest_quarter(items, quads, quarters, unit):
+    """Cycles of an iteration, times the rounds that the slowest quarter needs: two warps share a region, a lone one is faster than two."""
+    worst = 0
+    for w in range(quarters):
+        at, end = items // unit * w // quarters * unit, items // unit * (w + 1) // quarters * unit
+        cost = 0
+        while at < end:
+            here = min(end, (at // quads + 1) * quads) - at  # of one region
+            cost += here // 2 * 2 * 2820 + here % 2 * 3100
+            at += here
+        worst = max(worst, cost)
+    return worst
+
+
+def test_items_are_split_so_that_the_longest_quarter_is_shortest(program):
+    """The rule against a walk through every quarter, on a GPU of 6 SMs: grids of up to 40 regions, batches of up to 18 quads. In pairs or
+    one by one, whichever is over first."""
+    out = subprocess.run([program, "split", "40", "6", "18"], check=True, capture_output=True, text=True).stdout
+    units = set()
+    for line in out.splitlines():
+        regions, quads, ctas, unit = map(int, line.split())
+        items = regions * quads
+        assert unit == 1 or (unit == 2 and quads % 2 == 0), line
+        one = longest_quarter(items, quads, 4 * ctas, 1)
+        best = min(one, longest_quarter(items, quads, 4 * ctas, 2)) if quads % 2 == 0 else one
+        assert longest_quarter(items, quads, 4 * ctas, unit) == best, line
+        units.add(unit)
+    assert units == {1, 2}
