@@ -105,6 +105,10 @@ __device__ __forceinline__ void cp_async4(unsigned dst, const void *src)
 {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
 }
+__device__ __forceinline__ void cp_async8(unsigned dst, const void *src)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
+}
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 // ---- a lane's 16 cells in an IL4 tensor. base: its first cell row (dz = dy = 0) at x = 4 h, the lower end of its x half;
 // zstr, ystr: floats to the next row in z and (signed) in y. 32 bytes, a whole sector, per access: cells one by one, the

@@ -521,8 +521,9 @@ __global__ void __launch_bounds__(quadwg::THREADS, quadwg::CTAS) quad_wgrad_k(co
 #pragma unroll
             for (int n = 0; n < 4; ++n) cp_async4(my_dsq + 4 * n, s + (n >> 1) * zs + (n & 1) * (size_t)p.K);
         }
-        // two lanes: asynchronous copies of one address by all lanes are a request each (128^3: the step three times as long)
-        if (FUSE_IN && (tid & 31) < 2) cp_async16(my_ist + (tid & 31) * 16, p.in_stats + 4 * q + (tid & 31) * 2);
+        // four lanes: asynchronous copies of one address by all lanes are a request each (128^3: the step three times as long). A pair
+        // each: that is how a caller's statistics are aligned
+        if (FUSE_IN && (tid & 31) < 4) cp_async8(my_ist + (tid & 31) * 8, p.in_stats + 4 * q + (tid & 31));
     };
 
     // sums: sg[dy = 0 at ry = 0, dy = 1 at ry = 3][dz][a][c], sp[ry = 1, 2][dz][a][c] = (dy = 0, dy = 1)
@@ -1023,7 +1024,7 @@ __global__ void __launch_bounds__(384, quadborder::Room<NORM, BR, S>::CTAS) quad
                 if (second) cp_async16(mine0 + (unsigned)((k * RING + r) * CELLS + THREADS) * 16u, tensors[k] + (size_t)q * P + c2);
             }
             if (NORM && my_term >= 0) cp_async16(smem_u32(&terms[r][tid]), p.hterm + ((size_t)q * gridDim.x + my_term) * 2 + (tid & 1));
-            if (S != NO_SUMS && tid < 2) cp_async16(smem_u32(&quad_stats[r][tid]), p.stats + 4 * q + 2 * tid);
+            if (S != NO_SUMS && tid < 4) cp_async8(smem_u32(&quad_stats[r][0]) + tid * 8, p.stats + 4 * q + tid);  // a caller's: 8-byte aligned
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };

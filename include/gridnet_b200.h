@@ -491,7 +491,7 @@ GN_API int gn_step_backward_kept_f32(const float *weight, const float *bias, con
  *   x_il4    the input, one tensor;
  *   outs     host array of `outer` device pointers, one tensor each: the step outputs before normalisation (residual: the
  *            next h). Without a backward pass two tensors may take turns.
- *   stats    [outer][4 ceil(B/4)][2] floats: (mean, 1/sqrt(var + eps)) of outs[k] (residual: of the input of step k);
+ *   stats    [outer][4 ceil(B/4)][2] floats, 8-byte aligned: (mean, 1/sqrt(var + eps)) of outs[k] (residual: of the input of step k);
  *   stashes  NULL, or a host array of `outer` device pointers, each NULL or `inner` tensors: the pre-activations of the
  *            inner iterations for the backward pass, which otherwise runs them again.
  * Workspaces: 256-byte aligned, sizes from the two functions (replay = 1: some step has no stash). gn_loop_backward_f32

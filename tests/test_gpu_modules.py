@@ -507,6 +507,29 @@ def test_separate_networks_of_a_small_grid_kept_and_recomputed():
             assert torch.equal(a, b), i
 
 
+@pytest.mark.parametrize("shape,block,gated", [((16, 8, 24), 8, False), ((16, 8, 24), 8, True), ((16, 8, 24), 4, False), ((32, 40, 64), 8, False)])
+def test_statistics_need_no_more_than_their_own_alignment(shape, block, gated):
+    """A caller of the C interface may keep the loop's statistics at any address that pairs of floats may have: 8 bytes off a multiple of
+    16 they give the same bits (with sums in the border pass, of both branches, apart from it, and with blocks of 4)."""
+    from gridnet_b200 import backend_cuda as bc
+
+    g = torch.Generator().manual_seed(37)
+    batch, inner, outer, act = 6, 2, 3, "tanh"
+    mk = lambda *sz, scale=1.0, shift=0.0: (shift + scale * torch.randn(*sz, generator=g)).cuda()
+    two = [2] if gated else []
+    params = [mk(27, *two, *shape, scale=27 ** -0.5), mk(*two, *shape, scale=0.1)] + ([] if gated else [mk(*shape, scale=0.1, shift=1.0)])
+    gamma, beta, x, gy = mk(*shape, scale=0.1, shift=1.0), mk(*shape, scale=0.1), mk(batch, *shape), mk(batch, *shape)
+    _, saved = bc._loop_forward([params], gamma, beta, x, inner, outer, block, act, 1e-5, False, True, gated=gated)
+    x_il4, stats, outs, stashes = saved
+    assert stats.data_ptr() % 16 == 0
+    moved = torch.empty(stats.numel() + 16, dtype=torch.uint8, device="cuda")[8:8 + stats.numel()].copy_(stats)
+    assert moved.data_ptr() % 16 == 8
+    (want, *more), (got, *moved_more) = (bc._loop_backward([params], gamma, beta, (x_il4, s, outs, stashes), gy, inner, outer, block, act, False, gated=gated)
+                                         for s in (stats, moved))
+    for i, (a, b) in enumerate(zip([*want[0], *more], [*got[0], *moved_more])):
+        assert torch.equal(a, b), i
+
+
 def test_what_does_not_fit_is_recomputed(monkeypatch):
     """The bookkeeping of kept iterations: per device, without a lock that a finaliser could meet held, and a loop that runs out of
     memory while it allocates them goes on with those it has (allocation made to fail here; the gradients are the same bits)."""
