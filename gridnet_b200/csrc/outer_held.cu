@@ -29,6 +29,9 @@ constexpr int THREADS = WORKERS + 32 * MAX_SPC;
 constexpr int WATCHED = WORKERS + 32;          // threads that compute, with the warp that watches a sample
 constexpr int HALO = 488, SLOTS = 4;           // halo cells of a tile, per thread
 constexpr unsigned kSpinLimit = 1u << 18;      // polls, about a microsecond each
+// Inner iterations at most. CTAs wait for each other once a step, those with one block for those with four; an iteration takes up to 0.75 us
+// per sample, so nobody waits longer than 6 ms of the 260 that a wait has (at 1.5 million, 8 x 8 x 72, they ran out).
+constexpr int MAX_INNER = 4096;
 constexpr int B_DONE = 1, B_STATS = 1 + MAX_SPC, B_COMPUTE = 1 + 2 * MAX_SPC;  // named barriers; the last kind one per block
 // columns of tensor memory of a block: 9 chunks of 12 weights, then 4 biases, scales, norm weights and norm biases
 constexpr int COLS = 128, COL_REST = 108;
@@ -370,8 +373,8 @@ static int usable_sms()
     return n;
 }
 
-// Samples per CTA, or 0 if the kernel does not apply: block 8, at least one outer step, all blocks of a chunk of samples resident
-// at once, at most MAX_SPC samples per CTA (each takes 10 KB of shared memory per block and registers for its patch). Wherever it
+// Samples per CTA, or 0 if the kernel does not apply: block 8, at least one outer step, at most MAX_INNER inner iterations, all blocks of
+// a chunk of samples resident at once, at most MAX_SPC samples per CTA (each takes 10 KB of shared memory per block and registers for its patch). Wherever it
 // applies it is ahead of the loop of one launch per step, us, step by step / this kernel: 64^3, 4 x 12, one sample 166 / 80, two 217 / 105;
 // 64^3, 1 x 4 54 / 46; 40 x 56 x 72, 3 x 6 87 / 48; 48^3, 4 x 10, four samples 128 / 89; 32^3, 2 x 8, sixteen 101 / 56; 16^3, 2 x 8, 148
 // samples 103 / 52, 5 x 16, 120 samples 306 / 140. Where the blocks' weights fit into registers outer_small.cu is: 32^3, 2 x 8, eight samples
@@ -379,7 +382,7 @@ static int usable_sms()
 int outer_held_spc(int B, int M, int N, int K, int block, int inner, int outer, const void *w, const void *b, const void *s, const void *gamma,
                    const void *beta, const void *x, const void *y)
 {
-    if (block != 8 || inner < 1 || outer < 1 || B < 1 || M % 8 || N % 8 || K % 8) return 0;
+    if (block != 8 || inner < 1 || inner > held8::MAX_INNER || outer < 1 || B < 1 || M % 8 || N % 8 || K % 8) return 0;
     const long long P = (long long)M * N * K;
     if (P >= (1LL << 31) || (long long)B * P > kOuterSmallMaxCells) return 0;
     auto al8 = [](const void *q) { return (reinterpret_cast<uintptr_t>(q) & 7) == 0; };

@@ -259,6 +259,32 @@ def test_persistent_kernel_with_weights_in_tensor_memory(B, shape, inner, outer,
     assert_close(got.cpu().numpy(), orc.outer_forward(*a64, inner, outer, 8, activation=act), None, f"weights in tensor memory B={B}")
 
 
+def test_persistent_kernel_leaves_very_many_inner_iterations_to_the_steps():
+    """Nine blocks are three CTAs, the last with one block: it waits for the others longer the more inner iterations there are, and waits
+    are limited. Up to 4096 iterations the persistent kernel is taken, and no wait runs out; from there the loop goes step by step.
+    4096 roundings of 6e-8, amplified by up to e^4 (scales of 1e-3): 2e-4."""
+    from gridnet_b200 import outer_forward, outer_forward_failed, outer_forward_workspace
+    from gridnet_b200._lib import lib
+
+    B, shape, outer = 1, (8, 8, 72), 2
+    w, b, s, gamma, beta = model_params(87, shape)
+    args = [dev(a) for a in (w, b, (1e-3 * s).astype(np.float32), gamma, beta, face_input(88, B, shape))]
+    plans = [lib.gn_outer_forward_plan(B, *shape, inner, outer, 8) for inner in (4096, 4097, 1500000)]
+    assert plans[0] == 3 and 3 not in plans[1:], plans
+    ws = outer_forward_workspace(B, shape, 8, args[0].device)
+    got = outer_forward(*args, 4096, outer, 8, "tanh", workspace=ws)
+    assert not outer_forward_failed(ws, B, shape, 8)
+    try:
+        assert lib.gn_config_set(b"outer_kernel", 1) == 0
+        base = outer_forward(*args, 4096, outer, 8, "tanh")
+    finally:
+        lib.gn_config_set(b"outer_kernel", 0)
+    assert torch.allclose(got, base, rtol=1e-3, atol=1e-3), (got - base).abs().max().item()
+    got = outer_forward(*args, 4097, outer, 8, "tanh", workspace=ws)
+    assert not outer_forward_failed(ws, B, shape, 8)
+    assert torch.allclose(got, base, rtol=1e-2, atol=1e-2)  # one iteration more, of steps of at most 1e-3
+
+
 @pytest.mark.parametrize("B,shape,block,inner,outer,act", [
     (1, (8, 8, 8), 8, 1, 1, "relu"),        # one region, one sample of a quad
     (5, (8, 16, 24), 8, 3, 2, "tanh"),      # a ragged second quad, non-cubic grid
