@@ -674,7 +674,8 @@ def fused_loop_forward(step_params, norm_weight, norm_bias, x, inner_iters: int,
 
 def device_status(clear: bool = True, device=None) -> bool:
     """True if, since the last clear, a kernel on ``device`` gave up a bounded wait on a bulk tile copy and had
-    no workspace flag to report it in (the results of that call are invalid). Synchronises the device."""
+    no workspace flag to report it in, or a persistent kernel of :func:`outer_forward` one on its other blocks (the results of that
+    call are invalid). Synchronises the device."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     with torch.cuda.device(dev):
         torch.cuda.synchronize(dev)
@@ -686,7 +687,7 @@ def device_status(clear: bool = True, device=None) -> bool:
 
 def outer_forward_failed(workspace: torch.Tensor, batch: int, shape, block_size: int) -> bool:
     """True if the last :func:`outer_forward` that used ``workspace`` recorded a device-side failure
-    (a bounded wait on a bulk tile copy that gave up). Synchronises the device."""
+    (a bounded wait that gave up). Synchronises the device."""
     m, n, k = shape
     off = int(lib.gn_outer_forward_error_flag_offset(batch, m, n, k, block_size))
     torch.cuda.synchronize(workspace.device)

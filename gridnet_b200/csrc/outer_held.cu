@@ -11,7 +11,7 @@
 //
 // The launch is cooperative and there is one CTA per SM (shared memory is asked for that no second kernel with tensor memory can
 // have beside it), so all CTAs are resident, get their tensor memory, and the waits end; should one run out all the same,
-// the kernel sets the error flag and goes on.
+// the kernel sets the error flag and the device's status word and goes on.
 #include <atomic>
 
 #include "common.cuh"
@@ -46,7 +46,7 @@ struct OuterHeldParams {
     float *y;
     unsigned long long *cells;  // [2][B][P] (raw step output, step); zeroed
     unsigned long long *sums;   // [2][B][ctas per sample], a line each: (sum, sum of squares) as doubles, the low 8 bits the step; zeroed
-    int *error_flag;
+    int *error_flag, *status;   // of the call, and device_status_ptr(): callers seldom hold the workspace that the first one is in
     int nblocks, group;         // group: CTAs that work on the same samples
     int B, M, N, K, inner, outer, spc;
     float eps;
@@ -327,7 +327,7 @@ __global__ void __launch_bounds__(held8::THREADS, 1) outer_held_k(const OuterHel
                     make_float2(fmaf((own[q][j][0] - mr.x) * mr.y, gb[2 * j], gb[4 + 2 * j]), fmaf((own[q][j][1] - mr.x) * mr.y, gb[2 * j + 1], gb[5 + 2 * j]));
         }
     }
-    if (gave_up && p.error_flag) *p.error_flag = 1;
+    if (gave_up) report_wait(p.error_flag, p.status);
     tmem_fence_before();
     __syncthreads();
     if (warp == 0) tmem_free_all(tmem_slot);
@@ -400,7 +400,7 @@ int launch_outer_held(const float *w, const float *b, const float *s, const floa
 {
     OuterHeldParams p{};
     p.w = w; p.b = b; p.s = s; p.gamma = gamma; p.beta = beta; p.x = x; p.y = y;
-    p.cells = cells; p.sums = sums; p.error_flag = error_flag;
+    p.cells = cells; p.sums = sums; p.error_flag = error_flag; p.status = device_status_ptr();
     p.nblocks = (M / 8) * (N / 8) * (K / 8);
     p.group = (p.nblocks + held8::SLOTS_PER_CTA - 1) / held8::SLOTS_PER_CTA;
     p.B = B; p.M = M; p.N = N; p.K = K; p.inner = inner; p.outer = outer; p.spc = spc; p.eps = eps;

@@ -22,7 +22,7 @@
 // to a line that all the others read, it was 39 to 50.)
 //
 // The launch is cooperative, so all CTAs are resident and the waits end; should one run out all the same, the kernel
-// sets the error flag and goes on.
+// sets the error flag and the device's status word and goes on.
 #include <atomic>
 
 #include "common.cuh"
@@ -48,7 +48,7 @@ struct OuterSmallParams {
     float *y;
     unsigned long long *cells;    // [2][B][P] (raw step output, step); zeroed
     unsigned long long *sums;     // [2][B][nblocks], a line each: (sum, sum of squares) as doubles, the low 8 bits the step; zeroed
-    int *error_flag;
+    int *error_flag, *status;     // of the call, and device_status_ptr(): callers seldom hold the workspace that the first one is in
     int nblocks;
     int B, M, N, K, inner, outer, spc;
     float eps;
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(small8::THREADS, 2) outer_small_k(const OuterS
             __syncwarp();
             bar_arrive(B_STATS + q, WATCHED);
         }
-        if (gave_up && p.error_flag) *p.error_flag = 1;
+        if (gave_up) report_wait(p.error_flag, p.status);
         return;
     }
 
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(small8::THREADS, 2) outer_small_k(const OuterS
         }
     }
 
-    if (gave_up && p.error_flag) *p.error_flag = 1;
+    if (gave_up) report_wait(p.error_flag, p.status);
     // ---- the last normalisation
 #pragma unroll
     for (int q = 0; q < MAX_SPC; ++q) {
@@ -348,7 +348,7 @@ int launch_outer_small(const float *w, const float *b, const float *s, const flo
 {
     OuterSmallParams p{};
     p.w = w; p.b = b; p.s = s; p.gamma = gamma; p.beta = beta; p.x = x; p.y = y;
-    p.cells = cells; p.sums = sums; p.error_flag = error_flag;
+    p.cells = cells; p.sums = sums; p.error_flag = error_flag; p.status = device_status_ptr();
     p.nblocks = (M / 8) * (N / 8) * (K / 8);
     p.B = B; p.M = M; p.N = N; p.K = K; p.inner = inner; p.outer = outer; p.spc = spc; p.eps = eps;
     const int ctas = p.nblocks * ((B + spc - 1) / spc);

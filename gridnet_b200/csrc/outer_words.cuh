@@ -23,6 +23,13 @@ __device__ __forceinline__ void st_words(unsigned long long *p, unsigned long lo
 }
 __device__ __forceinline__ unsigned long long cell_word(float v, unsigned step) { return (unsigned long long)step << 32 | __float_as_uint(v); }
 
+// a wait ran out
+__device__ __forceinline__ void report_wait(int *error_flag, int *status)
+{
+    if (error_flag) *error_flag = 1;
+    if (status) *status = 1;
+}
+
 // One warp: adds up `count` pairs of doubles, a line each, whose low eight bits are `tag`, looking until all are there (or
 // gave_up), and returns (mean, rstd). Everything down to the result is done at every look, not only at the last: after
 // some thousand cycles without double-precision work the first such instructions take 4500 cycles, which then keeps all blocks

@@ -83,7 +83,7 @@ GN_API int gn_config_set(const char *key, int value);
  * workspace record that in a flag inside the workspace (gn_*_error_flag_offset); entry points without
  * one (gn_step_forward_f32, gn_step_forward_fused_f32, the slab forms, gn_gated_forward_f32,
  * gn_step_forward_pair64_f32 with error_flag == NULL) and the workspace backward set one int per device
- * inside the library instead. gn_device_status(clear) returns 1 if it is set on the current device, 0 if
+ * inside the library instead; the persistent kernels of gn_outer_forward_f32 set both. gn_device_status(clear) returns 1 if it is set on the current device, 0 if
  * not, a negative status on a CUDA error; clear != 0 resets it. It copies the word back with a blocking
  * copy: synchronise the streams you care about first. gn_device_status_set(v) writes the word (tests).
  * No counterpart in the reference, whose kernels never wait. */

@@ -101,3 +101,18 @@ def test_inference_workspace_holds_one_set_of_parameters():
     buffers = 2 * 4 * B * side ** 3
     weights = 4 * 27 * side ** 3
     assert lib.gn_outer_forward_workspace_bytes(B, side, side, side, 8) < buffers + 1.35 * weights
+
+
+def test_persistent_kernels_report_a_lost_result_where_it_can_be_seen():
+    """outer_forward allocates the workspace itself where the caller passes none, and then nobody can look at the flag in it: a wait between
+    the blocks of a persistent kernel that runs out is reported in the device's status word as well. Read off the sources; such a wait does
+    not run out in a test."""
+    csrc = os.path.join(ROOT, "gridnet_b200", "csrc")
+    with open(os.path.join(csrc, "outer_words.cuh")) as f:
+        report = f.read().split("void report_wait(int *error_flag, int *status)", 1)[1].split("\n}\n", 1)[0]
+    assert "*error_flag = 1" in report and "*status = 1" in report
+    for name, waits in (("outer_small.cu", 2), ("outer_held.cu", 1)):
+        with open(os.path.join(csrc, name)) as f:
+            text = f.read()
+        assert text.count("if (gave_up) report_wait(p.error_flag, p.status);") == waits, name
+        assert "*p.error_flag" not in text and "p.status = device_status_ptr();" in text, name
