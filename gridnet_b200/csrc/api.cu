@@ -236,9 +236,9 @@ static OuterWs carve_outer(void *base, int B, int M, int N, int K, int block)
 }
 
 // 0 = choose automatically: the one persistent kernel of outer_small.cu for problems so small that launches are what
-// they cost, or of outer_held.cu for a sample or two per four blocks and SM; else the quad kernel of step_quad.cu where it has work for most of its warps; else the register-patch kernel of
-// step_fast.cu. 1 = always the register-patch kernel, 2 = always the large-batch kernel of step_pair64.cu, 3 = always a
-// persistent kernel, 4 = always the quad kernel.
+// they cost, or of outer_held.cu for a sample or two per four blocks and SM; else the quad kernel of step_quad.cu where it has work for
+// most of its warps; else the register-patch kernel of step_fast.cu. 1 = always the register-patch kernel, 2 = always the large-batch
+// kernel of step_pair64.cu, 3 = always the persistent kernel of outer_small.cu, 4 = always the quad kernel.
 // A quad warp works on a whole 8^3 region for four samples, so fewer than about three regions x quads per SM leave it
 // idle, and a single sample fills a quarter of a lane. ms per loop, register-patch / quad: 48^3, 2 x 10, batch 3
 // (1.5 per SM) 0.154 / 0.180, batch 8 (2.9) 0.194 / 0.180, batch 32 0.40 / 0.29; 32^3, 2 x 8, batch 12 (1.3) 0.140 / 0.147, batch 32
@@ -940,9 +940,8 @@ GN_API int gn_outer_forward_plan(int B, int M, int N, int K, int inner, int oute
     if (B <= 0 || M <= 0 || N <= 0 || K <= 0 || inner < 1 || outer < 1 || (block != 4 && block != 8)) return 0;
     alignas(16) static const double aligned[2] = {0.0, 0.0};  // any 16-byte aligned address: only alignment is looked at
     const void *a = aligned;
-    if ((g_outer_kernel == 0 || g_outer_kernel == 3) && (outer_small_spc(B, M, N, K, block, inner, outer, a, a, a, a, a, a, a) > 0 ||
-                                                         outer_held_spc(B, M, N, K, block, inner, outer, a, a, a, a, a, a, a) > 0))
-        return 3;
+    if ((g_outer_kernel == 0 || g_outer_kernel == 3) && outer_small_spc(B, M, N, K, block, inner, outer, a, a, a, a, a, a, a) > 0) return 3;
+    if (g_outer_kernel == 0 && outer_held_spc(B, M, N, K, block, inner, outer, a, a, a, a, a, a, a) > 0) return 3;
     if (g_outer_kernel == 3) return 0;
     if (((g_outer_kernel == 0 && quad_wanted(B, M, N, K)) || g_outer_kernel == 4) && quad_applicable(M, N, K, block, inner)) return 5;
     if (g_outer_kernel == 4) return 0;
@@ -1015,7 +1014,7 @@ static int outer_forward_impl(const float *w, const float *b, const float *s, co
 
     if (g_outer_kernel == 0 || g_outer_kernel == 3) {
         const int spc = outer_small_spc(B, M, N, K, block, inner, outer, w, b, s, gamma, beta, x, y);
-        const int held = spc > 0 ? 0 : outer_held_spc(B, M, N, K, block, inner, outer, w, b, s, gamma, beta, x, y);
+        const int held = spc > 0 || g_outer_kernel != 0 ? 0 : outer_held_spc(B, M, N, K, block, inner, outer, w, b, s, gamma, beta, x, y);
         if (spc > 0 || held > 0) {
             const cudaError_t e = cudaMemsetAsync(ws.error_flag, 0, 128 + ws.small_bytes, st);
             if (e != cudaSuccess) {

@@ -72,8 +72,8 @@ GN_API int gn_version(void);
  *                   loop as one persistent kernel when the problem is so small that launches are
  *                   what it costs, or its blocks' weights fit into the tensor memory of the chip;
  *                   else the quad kernel; the register-patch kernel where neither
- *                   applies), 1 = the register-patch kernel, 2 = the large-batch kernel, 3 = a
- *                   persistent kernel, 4 = the quad kernel (GN_ERR_UNSUPPORTED from gn_outer_forward_f32 when the forced one does not apply).
+ *                   applies), 1 = the register-patch kernel, 2 = the large-batch kernel, 3 = the
+ *                   persistent kernel for small problems, 4 = the quad kernel (GN_ERR_UNSUPPORTED from gn_outer_forward_f32 when the forced one does not apply).
  *   "forward_samples_per_cta": samples one CTA of the tuned float forward kernel walks through;
  *                   0 = chosen from the grid and batch size (default). */
 GN_API int gn_config_set(const char *key, int value);

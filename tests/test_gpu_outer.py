@@ -259,6 +259,24 @@ def test_persistent_kernel_with_weights_in_tensor_memory(B, shape, inner, outer,
     assert_close(got.cpu().numpy(), orc.outer_forward(*a64, inner, outer, 8, activation=act), None, f"weights in tensor memory B={B}")
 
 
+def test_small_persistent_kernel_by_force_refuses_what_it_does_not_cover():
+    """A sample through 64^3 has more blocks than outer_small.cu holds weights for: automatically the kernel with weights in tensor memory
+    takes it; with the small one forced it is refused, as any other kernel that does not apply."""
+    from gridnet_b200 import outer_forward
+    from gridnet_b200._lib import lib
+
+    B, shape = 1, (64, 64, 64)
+    args = [dev(a) for a in (*model_params(89, shape), face_input(90, B, shape))]
+    assert lib.gn_outer_forward_plan(B, *shape, 2, 2, 8) == 3
+    try:
+        assert lib.gn_config_set(b"outer_kernel", 3) == 0
+        assert lib.gn_outer_forward_plan(B, *shape, 2, 2, 8) == 0
+        with pytest.raises(RuntimeError):
+            outer_forward(*args, 2, 2, 8, "silu")
+    finally:
+        lib.gn_config_set(b"outer_kernel", 0)
+
+
 def test_persistent_kernel_leaves_very_many_inner_iterations_to_the_steps():
     """Nine blocks are three CTAs, the last with one block: it waits for the others longer the more inner iterations there are, and waits
     are limited. Up to 4096 iterations the persistent kernel is taken, and no wait runs out; from there the loop goes step by step.
