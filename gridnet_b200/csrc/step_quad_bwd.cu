@@ -1646,8 +1646,6 @@ int launch_quad_norm_sums(const float *x, const float *g, const float *sub, cons
     // enough CTAs for a few per SM, by splitting the quads where the cells do not give them
     int chunks = 1;
     while (chunks < 8 && 2 * chunks <= Q && (long long)nparts * chunks < 4LL * sm_count()) chunks *= 2;
-    // long walks once more: 64^3 x 128, block 4, with gradients 37.2 -> 37.0 ms; four quads a CTA are better left alone (64^3 x 16: + 3 %)
-    if (chunks < 8 && 16 * chunks <= Q && (long long)nparts * chunks < 12LL * sm_count()) chunks *= 2;
     const int qpc = (Q + chunks - 1) / chunks;
 #define SUMS_(C, S)                                                                                                                     \
     launch_after_cluster(chunks, quad_norm_sums_k<C, S>, dim3(nparts, chunks), 256, 0, st, x4, g4, s4, gamma, stats, partials, nparts, \
