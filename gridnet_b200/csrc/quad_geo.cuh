@@ -224,31 +224,24 @@ __device__ __forceinline__ void quad_put(unsigned col, const float (&r)[4 * N])
     }
     if (N & 1) tmem_st4(col + 4 * k, r + 4 * k);
 }
-// -> tensor memory, by the TEAM warps of a quarter, each its share of the vectors in two goes: the loads of the first, then
+// -> tensor memory, by the two warps of a quarter, each its half of the vectors in two goes: the loads of the first, then
 // between(), after which the region before may be overwritten, then the rest.
-template <int TEAM = 2, typename Between>
+template <typename Between>
 __device__ __forceinline__ void quad_load_params(const float *packed, int role, int lane, unsigned tm, Between between)
 {
-    static_assert(TEAM == 2 || TEAM == 3, "");
-    constexpr int N = TEAM == 2 ? 29 : 20, LAST = quad::VECS - N * (2 * TEAM - 1);  // 29, 16
+    constexpr int N = quad::VECS / 4;
     const float4 *src = reinterpret_cast<const float4 *>(packed) + role * (2 * N) * 32 + lane;
     tm += role * (8 * N);
     float r[4 * N];
     quad_fetch<N>(src, r);
     between();
     quad_put<N>(tm, r);
-    if (LAST == N || role < TEAM - 1) {
-        quad_fetch<N>(src + N * 32, r);
-        quad_put<N>(tm + 4 * N, r);
-    } else {
-        float last[4 * LAST];
-        quad_fetch<LAST>(src + N * 32, last);
-        quad_put<LAST>(tm + 4 * N, last);
-    }
+    quad_fetch<N>(src + N * 32, r);
+    quad_put<N>(tm + 4 * N, r);
 }
 __device__ __forceinline__ void quad_load_params(const float *packed, int role, int lane, unsigned tm)
 {
-    quad_load_params<2>(packed, role, lane, tm, [] {});
+    quad_load_params(packed, role, lane, tm, [] {});
 }
 
 // the weight sums of per-block normalisation (quad_wsum), by one warp of the team

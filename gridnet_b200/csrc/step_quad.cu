@@ -17,9 +17,9 @@
 //     inner iterations need no barrier beyond __syncwarp, and new values go back into the tile in place.
 //   * Bank conflicts: none, see QuadLane in quad_geo.cuh.
 //   * Two warps (w, w + 4) share a quarter of tensor memory and therefore a region: each takes the next of its quads when it
-//     is free. Each such team has its own contiguous range of (region, quad) items, and meets (named barrier) only to exchange the
-//     weights at a new region. The two warps sit on the same scheduler, so one's activation functions (MUFU) overlap
-//     the other's FMAs.
+//     is free (its tile may have to wait for the buffer that the other warp is done with last). Each such team has its own
+//     contiguous range of (region, quad) items, and meets (named barrier) only to exchange the weights at a new region. The
+//     two warps sit on the same scheduler, so one's activation functions (MUFU) overlap the other's FMAs.
 //   * Tiles arrive by bulk tensor copy (zero fill outside the grid) into two buffers per team. With a third one the kernel was
 //     slower, the first-level cache being what is left; so it was with the next region's parameters prefetched to L2 (64^3 x 64,
 //     two iterations, kept for a backward pass: 120 us with both, 114 without).
@@ -154,7 +154,7 @@ __global__ void __launch_bounds__(128 * QuadGeo<SUB>::TEAM, 1)
         const int here = min(cnt - i0, p.Q - q0);  // items of this region
         const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
         const size_t g0 = ((size_t)(bz * 8 + L.z0) * p.N + (by * 8 + L.y0)) * p.K + bx * 8 + 4 * L.h;  // own patch, native layout
-        quad_load_params<TEAM>(p.packed + (size_t)blk * PACK_F, role, lane, tm, [&] {
+        quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm, [&] {
             if (i0 > 0) {
                 tmem_fence_before();
                 team_sync<TEAM>(quarter);  // the other warp no longer reads the old region's weights

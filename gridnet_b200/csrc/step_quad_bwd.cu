@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(256, 1) quad_reverse_k(const QuadRevParams p)
     int blk = (int)(n0 / (unsigned)p.Q), q0 = (int)(n0 - (unsigned)blk * p.Q);
     for (int i0 = 0; i0 < cnt;) {
         const int here = min(cnt - i0, p.Q - q0);
-        quad_load_params<TEAM>(p.packed + (size_t)blk * PACK_F, role, lane, tm, [&] {
+        quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm, [&] {
             if (i0 > 0) {
                 tmem_fence_before();
                 team_sync<TEAM>(quarter);  // the other warp no longer reads the old region's weights

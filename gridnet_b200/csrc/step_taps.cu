@@ -12,8 +12,8 @@
 // Around the iterations an item waits for its tile, normalises it and leaves sums and results. For that:
 //   - A lane's own cells stay in registers from their normalisation to the last iteration (92 instead of 124 shared loads per
 //     iteration). Only the halo's 488 entries of the (gamma, beta) table are in shared memory, a lane's own in tensor memory.
-//   - A warp takes the next item of its quarter when it is free (64^3: 1597 -> 1553 us), and asks for the first half of the
-//     next region's parameters before it waits for the other warp.
+//   - A warp takes the next item of its quarter when it is free (64^3: 1597 -> 1553 us; for its tile it may have to wait for the other
+//     warp's buffer), and asks for the first half of the next region's parameters before it waits for the other warp.
 //   - The next region's parameters are not prefetched to L2: 256^3 x 32 93.5 -> 88.5 ms, 128^3 x 16 with gradients 9.12 -> 8.85 ms, 40 x 56 x 72
 //     290 -> 285 us, at the price of 1554 -> 1565 us at 64^3. Prefetching tiles was slower too (256^3: 99.5 ms).
 // Measured before and after: 64^3 x 64, 4 x 12 iterations 1652 -> 1565 us; 40 x 56 x 72 x 37, 3 x 6 315 -> 285 us; 256^3 x 32, 2 x 32 96.5 ->
@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(128 * TapGeo<SUB>::TEAM, 1) step_fwd_taps(cons
 {
     using G = TapGeo<SUB>;
     constexpr int TEAM = G::TEAM, NBUF = G::NBUF;
+    static_assert(TEAM == 2, "parameters and tables are loaded by two warps");
     extern __shared__ __align__(1024) unsigned char smem[];
     __shared__ __align__(8) unsigned long long bars[QUARTERS * NBUF];
     __shared__ int issued[QUARTERS * NBUF];  // which item's copy into this buffer has been started last
@@ -172,8 +173,9 @@ __global__ void __launch_bounds__(128 * TapGeo<SUB>::TEAM, 1) step_fwd_taps(cons
         }
         __syncwarp();
     };
-    // the warp's next item. Block 8: whoever is free takes it, its tile has been asked for already. Block 4: item i is fetched
-    // by the warp that works on it, i mod TEAM.
+    // the warp's next item. Block 8: whoever is free takes the next one; with as many buffers as warps its tile has been asked for only
+    // if the item two before it is done, else wait_tile waits for the other warp to finish that. Block 4: item i is fetched by the warp
+    // that works on it, i mod TEAM.
     auto claim = [&](int last) {
         if constexpr (SUB == 8) {
             int i = 0;
@@ -210,10 +212,10 @@ __global__ void __launch_bounds__(128 * TapGeo<SUB>::TEAM, 1) step_fwd_taps(cons
         const int here = min(cnt - i0, p.Q - q0);  // items of this region
         const int bx = blk % nbx, by = (blk / nbx) % nby, bz = blk / nbx / nby;
         const size_t g0 = ((size_t)(bz * 8 + 4 * L.zp) * p.N + (by * 8 + L.y)) * p.K + bx * 8 + 4 * L.h;  // own patch
-        quad_load_params<TEAM>(p.packed + (size_t)blk * PACK_F, role, lane, tm, [&] {
+        quad_load_params(p.packed + (size_t)blk * PACK_F, role, lane, tm, [&] {
             if (i0 > 0) {
                 tmem_fence_before();
-                team_sync<TEAM>(quarter);  // the other warps no longer read the old region's weights
+                team_sync<TEAM>(quarter);  // the other warp no longer reads the old region's weights
                 tmem_fence_after();
             }
         });
@@ -227,25 +229,22 @@ __global__ void __launch_bounds__(128 * TapGeo<SUB>::TEAM, 1) step_fwd_taps(cons
                 const int j = (c * TEAM + role) * 32 + lane;
                 if (j < HALO8) gh[c] = table[halo_cell(j)];
             }
-            if (role < 2)
 #pragma unroll
-                for (int c = 0; c < 8; ++c) go[c] = table[(4 * L.zp + n + (c >> 2) + 1) * 100 + (L.y + 1) * 10 + 4 * L.h + (c & 3) + 1];
+            for (int c = 0; c < 8; ++c) go[c] = table[(4 * L.zp + n + (c >> 2) + 1) * 100 + (L.y + 1) * 10 + 4 * L.h + (c & 3) + 1];
 #pragma unroll
             for (int c = 0; c < STEPS; ++c) {
                 const int j = (c * TEAM + role) * 32 + lane;
                 if (j < HALO8) gbs[j] = gh[c];
             }
             __syncwarp();  // tensor memory instructions want the whole warp together
-            if (role < 2) {
-                float ga[8], be[8];
+            float ga[8], be[8];
 #pragma unroll
-                for (int c = 0; c < 8; ++c) {
-                    ga[c] = go[c].x;
-                    be[c] = go[c].y;
-                }
-                tmem_st8(tm + COL_GAMMA + 4 * n, ga);
-                tmem_st8(tm + COL_BETA + 4 * n, be);
+            for (int c = 0; c < 8; ++c) {
+                ga[c] = go[c].x;
+                be[c] = go[c].y;
             }
+            tmem_st8(tm + COL_GAMMA + 4 * n, ga);
+            tmem_st8(tm + COL_BETA + 4 * n, be);
         }
         tmem_wait_st();
         if (i0 == 0 && p.params_old) begin();
