@@ -61,7 +61,7 @@ def keep_forward_stash(enabled):
 
 def _free_bytes(device) -> int:
     """Free memory of the device as a caller of torch sees it: what the caching allocator holds but has not handed out
-    counts. Asks the driver, half a millisecond."""
+    counts. Asks the driver: 0.3 ms on a quiet host, now and then tens or hundreds where other programs use it."""
     free, _ = torch.cuda.mem_get_info(device)
     return free + torch.cuda.memory_reserved(device) - torch.cuda.memory_allocated(device)
 
@@ -274,9 +274,9 @@ _BIG = 1 << 30
 def _staggered(nbytes: int, device, k: int) -> torch.Tensor:
     """``nbytes`` of device memory; from a GiB up starting ``(k % 7 + 1) * 4352`` bytes into its allocation. The tensors a
     training step streams side by side (input, output, kept iterations) are each an exact power of two in size at the
-    benchmark's shapes, so fresh allocations start at the same offset inside every 2 MB page; depending on where
-    the driver put the pages, the forward pass of C3 then took anything from 79 to 105 ms. Different offsets make
-    the streams fall on different memory channels whatever the placement."""
+    benchmark's shapes, so fresh allocations start at the same offset inside every 2 MB page. Different offsets were meant to keep the
+    streams off the same memory channels; with the kernels of today they make no difference (C3's forward pass 51.8 ms with
+    them, 51.4 without, six processes each), and what made single passes longer was :func:`_free_bytes`."""
     if nbytes < _BIG:
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
     off = (k % 7 + 1) * _STAGGER
